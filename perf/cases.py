@@ -208,6 +208,69 @@ def run(s):
     return s["y"]
 
 
+# ---- the same results in 64 bits, in plain torch on the bytes that the state holds ----
+
+def _plain(buf, rows, cols, bits, w_off, s_off, b_off):
+    """A quantised matrix as float64: code * scale + bias, 64 columns to a group, the low nibble first."""
+    groups, nbytes = cols // 64, rows * cols * bits // 8
+    q = buf[w_off:w_off + nbytes].view(rows, -1)
+    if bits == 4:
+        q = torch.stack((q & 15, q >> 4), dim=-1)
+    sb = [buf[o:o + rows * groups * 2].view(torch.bfloat16).view(rows, groups, 1).double() for o in (s_off, b_off)]
+    return (q.reshape(rows, groups, 64).double() * sb[0] + sb[1]).view(rows, cols)
+
+
+def _plain_tensor(t):
+    return _plain(t.buffer, t.rows, t.cols, t.bits, 0, t.s_off, t.b_off)
+
+
+def _plain_mlp(x, gate, up, down):
+    return (torch.nn.functional.gelu(x @ gate.T, approximate="tanh") * (x @ up.T)) @ down.T
+
+
+def _plain_block(layer, x):
+    """(indices, weights, y) of one MoE block for float64 rows."""
+    logits = (x * layer.effective_scale.view(torch.bfloat16).double()) @ _plain_tensor(layer.router).T
+    if layer.logit_bias is not None:
+        logits = logits + layer.logit_bias.double()
+    top, idx = torch.topk(logits, K, dim=-1)
+    weights = torch.softmax(top, dim=-1) * layer.per_expert_scale.view(torch.bfloat16).double()[idx]
+    y = _plain_mlp(x, *(_plain_tensor(t) for t in (layer.shared_gate, layer.shared_up, layer.shared_down)))
+    pool, o = layer.pool, layer.pool.offsets
+    for e in torch.unique(idx).tolist():
+        blob = tf_stack.device_view_u8(pool.ptr(layer.layer_index, e), pool.stride)
+        token, rank = torch.nonzero(idx == e, as_tuple=True)
+        out = _plain_mlp(x[token], _plain(blob, F, D, 4, o.gate_w_off, o.gate_s_off, o.gate_b_off),
+                         _plain(blob, F, D, 4, o.up_w_off, o.up_s_off, o.up_b_off),
+                         _plain(blob, D, F, 4, o.down_w_off, o.down_s_off, o.down_b_off))
+        y.index_add_(0, token, out * weights[token, rank][:, None])
+    return idx, weights, y
+
+
+def exact(case, seed):
+    s = prepare(case, seed)
+    kind, x = case["kind"], s["x"].double()
+    if kind in ("step", "prefill"):
+        if case["tokens"] > 512:
+            return None                 # takes too long in 64 bits
+        model = s["model"]
+        for layer, w in zip(model.layers, model.norm_weights):
+            normed = x * torch.rsqrt(x.square().mean(dim=-1, keepdim=True) + model.eps) * w.view(torch.bfloat16).double()
+            x = x + _plain_block(layer, normed)[2]
+        return x
+    if kind == "block":
+        return _plain_block(s["layer"], x)[2]
+    if kind == "operators":
+        idx, weights, y = _plain_block(s["layer"], x)
+        return {"indices": idx[0].int(), "weights": weights[0], "y": y[0]}
+    w = s["w"]
+    if kind == "lm_head":
+        normed = x * torch.rsqrt(x.square().mean(dim=-1, keepdim=True) + 1e-6) * s["norm"].double()
+        return (_plain_tensor(w) @ normed[0]).argmax().int().view(1)
+    y = x @ _plain_tensor(w).T
+    return y[0] if kind == "gemv" else y
+
+
 def _affine_bytes(rows, cols, bits):
     return rows * cols * bits // 8 + 2 * rows * (cols // 64) * 2
 
