@@ -83,10 +83,9 @@ tf_status tf_context_create(int device, tf_context** out) {
     if (e == cudaSuccess) e = cudaMemset(ctx->peer_error, 0, sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMalloc(&ctx->streamed_scratch, tf::streamed_scratch_bytes());
     if (e == cudaSuccess) e = cudaMalloc(&ctx->group_scratch, sizeof(uint32_t) * 2 * 256 * TF_MAX_ROUTER_EXPERTS);     // counts, then start positions
+    if (e == cudaSuccess) e = cudaMalloc(&ctx->qmm_groups, 2 * 16 * (TF_MAX_ROUTER_EXPERTS + 1));   // routed and dense tables
     if (e == cudaSuccess) e = cudaMalloc(&ctx->grid_barrier, sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMemset(ctx->grid_barrier, 0, sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&ctx->qmm_groups, 2 * 64 * (TF_MAX_ROUTER_EXPERTS + 1));   // routed and dense tables
-    if (e == cudaSuccess) e = cudaMalloc(&ctx->qmm_totals, 4 * sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->side_stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->fork_event, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->join_event, cudaEventDisableTiming);
@@ -109,9 +108,8 @@ void tf_context_destroy(tf_context* ctx) {
     if (ctx->peer_error) cudaFree(ctx->peer_error);
     if (ctx->streamed_scratch) cudaFree(ctx->streamed_scratch);
     if (ctx->group_scratch) cudaFree(ctx->group_scratch);
-    if (ctx->grid_barrier) cudaFree(ctx->grid_barrier);
     if (ctx->qmm_groups) cudaFree(ctx->qmm_groups);
-    if (ctx->qmm_totals) cudaFree(ctx->qmm_totals);
+    if (ctx->grid_barrier) cudaFree(ctx->grid_barrier);
     if (ctx->lm_x) cudaFree(ctx->lm_x);
     if (ctx->lm_logits) cudaFree(ctx->lm_logits);
     if (ctx->lm_best) cudaFree(ctx->lm_best);

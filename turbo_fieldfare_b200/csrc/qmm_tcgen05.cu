@@ -38,52 +38,56 @@
 namespace tf {
 
 constexpr int kQmmTokMax = 128;        // largest N of one MMA: tokens per tile
-constexpr int kQmmBoxRows = 16;        // activation rows per TMA box (2 KB per step)
-constexpr int kQmmRows = 128;          // M of the MMA: weight rows per tile
-constexpr int kQmmK = 128;             // columns per step: two quantisation groups, so that the per-step costs of the
-                                       // single-thread roles (waits, descriptors, commits) are paid once per 128 columns
-constexpr int kQmmRawStages = 4;       // ring of packed-code stages (NMAT x 8 KB each)
-constexpr int kQmmBSlots = 32;         // ring of activation slots (16 rows x 64 columns, 2 KB); a step takes 2, 4, 8 or 16
+constexpr int kQmmRows = 128;          // M of the MMA: weight rows per tile (gate/up: 64 gate rows over 64 up rows)
+constexpr int kQmmRawK = 256;          // columns per packed-code stage: one quantisation group per dequantiser thread
+constexpr int kQmmHalfK = 128;         // columns per operand slot (A in tensor memory, B in shared memory)
+constexpr uint32_t kQmmRawBytes = kQmmRows * (kQmmRawK / 2);        // 16 KB
+constexpr int kQmmRawMax = 4, kQmmBMax = 12, kQmmScMax = 4;         // ring depths (the launch picks them to fit, see QmmPlan)
+constexpr int kQmmASlots = 4;          // TMEM ring of dequantised 128-column slots, 64 TMEM columns each
 constexpr int kQmmFirstDequantWarp = 4, kQmmDequantWarps = 16;      // four threads per weight row
 constexpr int kQmmFirstEpilogueWarp = 20, kQmmEpilogueWarps = 4;
 constexpr int kQmmThreads = (kQmmFirstEpilogueWarp + kQmmEpilogueWarps) * 32;
-constexpr int kQmmTmemCols = 512;      // columns 0..255: accumulators; 256..511: ring of dequantised weight stages
+constexpr int kQmmTmemCols = 512;      // columns 0..255: two accumulator buffers; 256..511: the ring of dequantised slots
 constexpr int kQmmAccCols = 256;
+constexpr uint32_t kQmmStageBytes = 16384;    // output staging of the epilogue
 constexpr uint32_t kQmmSpin = 1u << 22;
 constexpr uint32_t kErrQmmTimeout = 0x7E000000u;
+static_assert(TF_MAX_ROUTER_EXPERTS <= kQmmThreads, "one thread per group");
 static_assert(kQmmFirstEpilogueWarp % 4 == 0 && kQmmFirstDequantWarp % 4 == 0, "warp w touches TMEM lanes 32 * (w % 4)");
 
-struct QmmGroup {
-    const uint16_t* S[2];   // scale / bias planes of the group's matrices
-    const uint16_t* B[2];
-    uint32_t expert;        // third coordinate of the weight tensor maps (0 for a dense matrix)
-    uint32_t row_start;     // first row of the group in the (sorted) activation matrix
-    uint32_t count;         // tokens of the group
-    uint32_t tile_start;    // first token tile of the group in the global tile order
-    uint32_t pad[4];
+// How a launch divides its shared memory (offsets from a 1024-byte aligned base); computed on the host from K.
+struct QmmPlan {
+    uint32_t raw_stages;    // packed-code stages of 16 KB
+    uint32_t b_bytes;       // activation ring
+    uint32_t sc_bufs;       // scale-plane buffers
+    uint32_t plane_bytes;   // one scale or bias plane of a tile (128 / NMAT rows)
+    uint32_t sc_bytes;      // one buffer: NMAT x (scale plane, bias plane)
+    uint32_t tok_max;       // tokens per tile
+    uint32_t off_b, off_sc, off_stage, off_table, off_bars, total;
 };
-static_assert(sizeof(QmmGroup) == 64, "the context allocates 64 bytes per group-table row");
 
 struct QmmArgs {
-    QmmGroup* groups;       // device array, filled by qmm_prepare_kernel
-    uint32_t* totals;       // device: [0] group count, [1] token tiles
-    // routed source (prepare kernel)
-    const uint8_t* pool_base;
+    // planes of matrix m of expert e at S[m] + e * expert_stride bytes (dense: one expert)
+    const uint16_t* S[2];
+    const uint16_t* B[2];
     uint64_t expert_stride;
-    uint32_t s_off[2], b_off[2];
+    // groups of the launch, filled by qmm_prepare_kernel: {first token tile, first row, tokens, expert | tokens per tile << 16},
+    // and {groups, token tiles, largest N}
+    uint4* groups;
+    uint32_t* totals;
+    // their source; routed: what the grouping kernels left on the device; dense (NULL): one group
     const tf_group* route_groups;
     const uint32_t* route_counters;
-    // dense source
-    const uint16_t* dense_S[2];
-    const uint16_t* dense_B[2];
-    uint32_t dense_tokens;
+    uint32_t dense_tokens, dense_per_tile;
     // problem
     uint32_t rows;          // weight rows (output features)
     uint32_t k;             // columns (input features)
     uint16_t* out;          // [tokens, out_stride] fp16
     uint32_t out_stride;
+    uint32_t out_vec;       // rows of out start on 16-byte boundaries
     uint32_t round_gate_up; // shared expert: gate and up rounded to fp16 before the activation
     uint32_t* error;
+    QmmPlan plan;
 };
 
 // ---- PTX wrappers ----
@@ -145,27 +149,20 @@ __device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t (&r)[16]) {
                  : "r"(taddr) : "memory");
 }
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-// 16 consecutive 32-bit columns of this thread's TMEM lane <- 16 registers (four uint4)
-__device__ __forceinline__ void tc_st16(uint32_t taddr, const uint4& a, const uint4& b, const uint4& c, const uint4& d) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-                 "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
-                 ::"r"(taddr), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w),
-                   "r"(c.x), "r"(c.y), "r"(c.z), "r"(c.w), "r"(d.x), "r"(d.y), "r"(d.z), "r"(d.w) : "memory");
-}
-// 8 consecutive 32-bit columns of this thread's TMEM lane <- 8 registers
-__device__ __forceinline__ void tc_st8(uint32_t taddr, const uint4& a, const uint4& b) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
-                 ::"r"(taddr), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w) : "memory");
+// 32 consecutive 32-bit columns of this thread's TMEM lane <- 32 registers (eight uint4)
+__device__ __forceinline__ void tc_st32(uint32_t taddr, const uint4 (&v)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+                 "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
+                 "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
+                 ::"r"(taddr), "r"(v[0].x), "r"(v[0].y), "r"(v[0].z), "r"(v[0].w), "r"(v[1].x), "r"(v[1].y), "r"(v[1].z), "r"(v[1].w),
+                   "r"(v[2].x), "r"(v[2].y), "r"(v[2].z), "r"(v[2].w), "r"(v[3].x), "r"(v[3].y), "r"(v[3].z), "r"(v[3].w),
+                   "r"(v[4].x), "r"(v[4].y), "r"(v[4].z), "r"(v[4].w), "r"(v[5].x), "r"(v[5].y), "r"(v[5].z), "r"(v[5].w),
+                   "r"(v[6].x), "r"(v[6].y), "r"(v[6].z), "r"(v[6].w), "r"(v[7].x), "r"(v[7].y), "r"(v[7].z), "r"(v[7].w) : "memory");
 }
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ uint4 q_lds128(uint32_t addr) {
     uint4 v;
     asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
-    return v;
-}
-__device__ __forceinline__ uint2 q_lds64(uint32_t addr) {
-    uint2 v;
-    asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
     return v;
 }
 __device__ __forceinline__ uint32_t q_lds16(uint32_t addr) {
@@ -183,438 +180,448 @@ __device__ __forceinline__ uint32_t qmm_idesc(uint32_t n) {
     return (1u << 4) | ((n >> 3) << 17) | ((uint32_t)(kQmmRows >> 4) << 24);
 }
 
-// Builds the group table on the device: routed groups from the routing metadata, or one dense group.
-__global__ void qmm_prepare_kernel(QmmArgs a, int nmat, int dense) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    uint32_t ng, tiles = 0;
-    if (dense) {
-        ng = 1;
-        QmmGroup g{};
-        for (int m = 0; m < nmat; ++m) { g.S[m] = a.dense_S[m]; g.B[m] = a.dense_B[m]; }
-        g.expert = 0; g.row_start = 0; g.count = a.dense_tokens; g.tile_start = 0;
-        a.groups[0] = g;
-        tiles = (a.dense_tokens + kQmmTokMax - 1) / kQmmTokMax;
-    } else {
-        ng = a.route_counters[0];
-        for (uint32_t i = 0; i < ng; ++i) {
-            const tf_group rg = a.route_groups[i];
-            const uint8_t* blob = a.pool_base + (uint64_t)rg.expert * a.expert_stride;
-            QmmGroup g{};
-            for (int m = 0; m < nmat; ++m) {
-                g.S[m] = reinterpret_cast<const uint16_t*>(blob + a.s_off[m]);
-                g.B[m] = reinterpret_cast<const uint16_t*>(blob + a.b_off[m]);
-            }
-            g.expert = rg.expert; g.row_start = rg.pair_start; g.count = rg.pair_count; g.tile_start = tiles;
-            a.groups[i] = g;
-            tiles += (rg.pair_count + kQmmTokMax - 1) / kQmmTokMax;
-        }
-    }
-    a.totals[0] = ng;
-    a.totals[1] = tiles;
-}
-
-// Shared-memory plan (offsets from a 1024-byte aligned base).
-template <int NMAT>
-struct QmmSmem {
-    static constexpr uint32_t kRawMat = kQmmRows * (kQmmK / 2);              // 8 KB: 128 rows x 64 packed bytes
-    static constexpr uint32_t kRawStage = NMAT * kRawMat;
-    static constexpr uint32_t kOffRaw = 0;
-    static constexpr uint32_t kOffB = kOffRaw + kQmmRawStages * kRawStage;   // 32 slots x 2 KB
-    static constexpr uint32_t kOffScales = kOffB + kQmmBSlots * kQmmBoxRows * 128;
-    // scale and bias planes of a tile: 128 rows x (K / 64) bf16, two buffers, sized at launch
-    __host__ __device__ static uint32_t plane_bytes(uint32_t k) { return ((kQmmRows * (k / kGroup) * 2u) + 15u) & ~15u; }
-    __host__ __device__ static uint32_t scale_buf_bytes(uint32_t k) { return NMAT * 2 * plane_bytes(k); }
-    __host__ __device__ static uint32_t off_bars(uint32_t k) { return kOffScales + 2 * scale_buf_bytes(k); }
-    __host__ __device__ static uint32_t total(uint32_t k) { return off_bars(k) + 1024 /* barriers */ + 1024 /* alignment slack */; }
-    static constexpr int kAStages = 256 / (NMAT * (kQmmK / 2));              // TMEM ring of dequantised stages: 2 or 4
-};
-
 // Eight packed codes (one 32-bit word) -> eight fp16 weights w = half(q * s + b).
-// Fast form: a nibble moved to bits 4..7 of a half is the subnormal q * 2^-20, so one HFMA2 with s * 2^20
-// gives fma(q, s, b) rounded once (tensorops.metal:60-75 stores half(fma(q, s, b))); s * 2^20 is exact in
-// fp16 (s is a bf16) while |s| < 2^-5. Larger scales take the two-step form (1024 + q) - 1024.
-// Output order: PERMUTED (k0,k4,k1,k5,k2,k6,k3,k7), otherwise natural.
+// A nibble inside the ten mantissa bits of a half is a subnormal: q * 2^-22 at bits 2..5, q * 2^-20 at bits 4..7,
+// q * 2^-18 at bits 6..9, so one HFMA2 with s times the opposite power of two gives fma(q, s, b) rounded once
+// (tensorops.metal:60-75 stores half(fma(q, s, b))); the scaled s is exact in fp16 (s is a bf16) while it is finite.
+// The kernel is bound by the integer pipe, which takes half a warp per clock, so what counts is its instructions per
+// word: permuted order (k0,k4,k1,k5,k2,k6,k3,k7) two shifts and four masks (|s| < 2^-6), natural order one shift, four
+// byte permutes and four masks (|s| < 2^-5). Larger scales take the two-step form (1024 + q) - 1024.
 template <bool NATURAL_K>
-__device__ __forceinline__ uint4 order8(__half2 h0, __half2 h1, __half2 h2, __half2 h3) {
-    const uint32_t u0 = *reinterpret_cast<uint32_t*>(&h0), u1 = *reinterpret_cast<uint32_t*>(&h1);
-    const uint32_t u2 = *reinterpret_cast<uint32_t*>(&h2), u3 = *reinterpret_cast<uint32_t*>(&h3);
-    if (!NATURAL_K) return make_uint4(u0, u1, u2, u3);
-    uint4 o;
-    asm("prmt.b32 %0, %1, %2, 0x5410;" : "=r"(o.x) : "r"(u0), "r"(u1));   // (k0, k1)
-    asm("prmt.b32 %0, %1, %2, 0x5410;" : "=r"(o.y) : "r"(u2), "r"(u3));   // (k2, k3)
-    asm("prmt.b32 %0, %1, %2, 0x7632;" : "=r"(o.z) : "r"(u0), "r"(u1));   // (k4, k5)
-    asm("prmt.b32 %0, %1, %2, 0x7632;" : "=r"(o.w) : "r"(u2), "r"(u3));   // (k6, k7)
-    return o;
+struct FastScale {
+    __half2 lo, hi;      // permuted: s * 2^22, s * 2^18; natural: both s * 2^20
+    static constexpr float kLimit = NATURAL_K ? 0.03125f : 0.015625f;
+    __device__ __forceinline__ explicit FastScale(float s) {
+        if (NATURAL_K) { lo = __float2half2_rn(s * 1048576.0f); hi = lo; }
+        else { lo = __float2half2_rn(s * 4194304.0f); hi = __float2half2_rn(s * 262144.0f); }
+    }
+};
+__device__ __forceinline__ uint32_t q_hfma2(uint32_t a, __half2 s, __half2 b) {
+    const __half2 r = __hfma2(*reinterpret_cast<__half2*>(&a), s, b);
+    return *reinterpret_cast<const uint32_t*>(&r);
 }
 template <bool NATURAL_K>
-__device__ __forceinline__ uint4 dequant8_fast(uint32_t w, __half2 s_fast, __half2 b) {
-    uint32_t t0 = (w << 4) & 0x00F000F0u, t1 = w & 0x00F000F0u, t2 = (w >> 4) & 0x00F000F0u, t3 = (w >> 8) & 0x00F000F0u;
-    return order8<NATURAL_K>(__hfma2(*reinterpret_cast<__half2*>(&t0), s_fast, b),      // (k0, k4)
-                             __hfma2(*reinterpret_cast<__half2*>(&t1), s_fast, b),      // (k1, k5)
-                             __hfma2(*reinterpret_cast<__half2*>(&t2), s_fast, b),      // (k2, k6)
-                             __hfma2(*reinterpret_cast<__half2*>(&t3), s_fast, b));     // (k3, k7)
+__device__ __forceinline__ uint4 dequant8_fast(uint32_t w, const FastScale<NATURAL_K>& s, __half2 b) {
+    if (NATURAL_K) {
+        const uint32_t x = w << 4;
+        uint32_t t0, t1, t2, t3;                                        // low half: nibble of byte i in x, high half: in w
+        asm("prmt.b32 %0, %1, %2, 0x7470;" : "=r"(t0) : "r"(x), "r"(w));
+        asm("prmt.b32 %0, %1, %2, 0x7571;" : "=r"(t1) : "r"(x), "r"(w));
+        asm("prmt.b32 %0, %1, %2, 0x7672;" : "=r"(t2) : "r"(x), "r"(w));
+        asm("prmt.b32 %0, %1, %2, 0x7773;" : "=r"(t3) : "r"(x), "r"(w));
+        return make_uint4(q_hfma2(t0 & 0x00F000F0u, s.lo, b), q_hfma2(t1 & 0x00F000F0u, s.lo, b),
+                          q_hfma2(t2 & 0x00F000F0u, s.lo, b), q_hfma2(t3 & 0x00F000F0u, s.lo, b));
+    }
+    const uint32_t a = w << 2, c = w >> 6;
+    return make_uint4(q_hfma2(a & 0x003C003Cu, s.lo, b), q_hfma2(a & 0x03C003C0u, s.hi, b),      // (k0, k4), (k1, k5)
+                      q_hfma2(c & 0x003C003Cu, s.lo, b), q_hfma2(c & 0x03C003C0u, s.hi, b));     // (k2, k6), (k3, k7)
 }
 template <bool NATURAL_K>
 __device__ __forceinline__ uint4 dequant8_wide(uint32_t w, __half2 s, __half2 b) {
     const __half2 k1024 = __half2half2(__ushort_as_half(0x6400));
-    uint32_t t0 = (w & 0x000F000Fu) | 0x64006400u, t1 = ((w >> 4) & 0x000F000Fu) | 0x64006400u;
-    uint32_t t2 = ((w >> 8) & 0x000F000Fu) | 0x64006400u, t3 = ((w >> 12) & 0x000F000Fu) | 0x64006400u;
-    return order8<NATURAL_K>(__hfma2(__hsub2(*reinterpret_cast<__half2*>(&t0), k1024), s, b),
-                             __hfma2(__hsub2(*reinterpret_cast<__half2*>(&t1), k1024), s, b),
-                             __hfma2(__hsub2(*reinterpret_cast<__half2*>(&t2), k1024), s, b),
-                             __hfma2(__hsub2(*reinterpret_cast<__half2*>(&t3), k1024), s, b));
+    uint32_t t[4], o[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        t[i] = ((w >> (4 * i)) & 0x000F000Fu) | 0x64006400u;
+        const __half2 q = __hsub2(*reinterpret_cast<__half2*>(&t[i]), k1024);
+        o[i] = q_hfma2(*reinterpret_cast<const uint32_t*>(&q), s, b);
+    }
+    if (!NATURAL_K) return make_uint4(o[0], o[1], o[2], o[3]);
+    uint4 r;
+    asm("prmt.b32 %0, %1, %2, 0x5410;" : "=r"(r.x) : "r"(o[0]), "r"(o[1]));   // (k0, k1)
+    asm("prmt.b32 %0, %1, %2, 0x5410;" : "=r"(r.y) : "r"(o[2]), "r"(o[3]));   // (k2, k3)
+    asm("prmt.b32 %0, %1, %2, 0x7632;" : "=r"(r.z) : "r"(o[0]), "r"(o[1]));   // (k4, k5)
+    asm("prmt.b32 %0, %1, %2, 0x7632;" : "=r"(r.w) : "r"(o[2]), "r"(o[3]));   // (k6, k7)
+    return r;
 }
 
 // Position of column k within its eight-column block in the PERMUTED order.
 __device__ __forceinline__ uint32_t permuted_col(uint32_t k) { return (k & ~7u) | ((k & 3u) << 1) | ((k >> 2) & 1u); }
 
-// Accumulator placement in TMEM columns 0..255, two buffers of 128. A tile whose accumulators fit one buffer
-// (one matrix, or two matrices of at most 64 tokens) takes the buffer used less often so far, so consecutive
-// tiles alternate and the epilogue of one overlaps the MMAs of the next; a two-matrix tile of more than 64
-// tokens takes both. The MMA issuer and the epilogue warps replay the same sequence, so they agree.
-struct AccPlan {
-    uint32_t uses0 = 0u, uses1 = 0u;
-    bool both = false;
-    uint32_t buf = 0, col0 = 0, mat_stride = 0;
-    template <int NMAT>
-    __device__ __forceinline__ void next(uint32_t n_mma) {
-        both = NMAT == 2 && n_mma > 64u;
-        buf = both ? 0u : (uses0 <= uses1 ? 0u : 1u);
-        col0 = buf * 128u;
-        mat_stride = both ? 128u : 64u;
+// Tokens per tile of a group: as few tiles as tok_max allows, of equal size (a multiple of 16, the step of the MMA's N).
+// 256 + 14 tokens are three tiles of 96, not 128 + 128 + 14: the weights are dequantised once per tile, and below about
+// 80 tokens that takes longer than the tile's MMAs.
+__host__ __device__ inline uint32_t qmm_tokens_per_tile(uint32_t count, uint32_t tok_max) {
+    const uint32_t tiles = (count + tok_max - 1) / tok_max;
+    return ((count + tiles - 1) / tiles + 15u) & ~15u;
+}
+
+// The group table of a launch: one thread per group, the tile counts scanned over the block. (One thread that walked the
+// groups took 29 us for 128 of them, on the critical path before every routed GEMM; this takes about 2.)
+__global__ void __launch_bounds__(TF_MAX_ROUTER_EXPERTS)
+qmm_prepare_kernel(uint4* __restrict__ groups, uint32_t* __restrict__ totals, const tf_group* __restrict__ route_groups,
+                   const uint32_t* __restrict__ route_counters, uint32_t dense_tokens, uint32_t dense_per_tile, uint32_t tok_max) {
+    __shared__ uint32_t warp_tiles[TF_MAX_ROUTER_EXPERTS / kWarp], warp_top[TF_MAX_ROUTER_EXPERTS / kWarp];
+    const uint32_t warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
+    pdl_launch_dependents();
+    pdl_wait();
+    const uint32_t ngroups = route_groups ? min(route_counters[0], (uint32_t)TF_MAX_ROUTER_EXPERTS) : 1u;
+    uint32_t row = 0, count = 0, expert = 0, per = 16;
+    if (threadIdx.x < ngroups) {
+        if (route_groups) {
+            const tf_group rg = route_groups[threadIdx.x];
+            row = rg.pair_start; count = rg.pair_count; expert = rg.expert;
+            per = qmm_tokens_per_tile(count > 0 ? count : 1u, tok_max);
+        } else {
+            count = dense_tokens; per = dense_per_tile;
+        }
     }
-    __device__ __forceinline__ bool takes(uint32_t b) const { return both || b == buf; }
-    __device__ __forceinline__ uint32_t uses(uint32_t b) const { return b ? uses1 : uses0; }
-    __device__ __forceinline__ void done() {
-        if (both || buf == 0) ++uses0;
-        if (both || buf == 1) ++uses1;
+    const uint32_t tiles = (count + per - 1) / per;
+    uint32_t incl = tiles;
+#pragma unroll
+    for (int o = 1; o < kWarp; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(kFullMask, incl, o);
+        if (lane >= (uint32_t)o) incl += v;
     }
+    const uint32_t top = __reduce_max_sync(kFullMask, min((count + 15u) & ~15u, per));
+    if (lane == kWarp - 1) { warp_tiles[warp] = incl; warp_top[warp] = top; }
+    __syncthreads();
+    uint32_t before = 0, all = 0, n_top = 16;
+#pragma unroll
+    for (uint32_t w = 0; w < TF_MAX_ROUTER_EXPERTS / kWarp; ++w) {
+        before += w < warp ? warp_tiles[w] : 0u;
+        all += warp_tiles[w];
+        n_top = max(n_top, warp_top[w]);
+    }
+    if (threadIdx.x < ngroups) groups[threadIdx.x] = make_uint4(before + incl - tiles, row, count, expert | (per << 16));
+    if (threadIdx.x == 0) { totals[0] = ngroups; totals[1] = all; totals[2] = n_top; }
+}
+
+// A role's place in the CTA's sequence of tiles. Tiles only move forward, so the group is found by stepping through the
+// table in shared memory, not by searching it.
+struct QmmTile {
+    uint32_t gi = 0;            // group
+    uint32_t wt = 0;            // weight-row tile
+    uint32_t row0 = 0;          // first activation / output row
+    uint32_t ntok = 0;          // real tokens
+    uint32_t expert = 0;
+    __device__ __forceinline__ void locate(const uint4* table, uint32_t ngroups, uint32_t wrow_tiles, uint32_t tile) {
+        const uint32_t tglob = tile / wrow_tiles;
+        wt = tile - tglob * wrow_tiles;
+        while (gi + 1 < ngroups && table[gi + 1].x <= tglob) ++gi;
+        const uint4 g = table[gi];                                  // tile start, first row, tokens, expert | tokens per tile << 16
+        const uint32_t per = g.w >> 16, done = (tglob - g.x) * per;
+        expert = g.w & 0xFFFFu;
+        row0 = g.y + done;
+        ntok = g.z - done < per ? g.z - done : per;
+    }
+    __device__ __forceinline__ uint32_t n() const { return (ntok + 15u) & ~15u; }
 };
 
 template <int NMAT, bool NATURAL_K>
 __global__ void __launch_bounds__(kQmmThreads, 1)
-qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap x_map_big,
-                   const __grid_constant__ CUtensorMap w_map0,
-                   const __grid_constant__ CUtensorMap w_map1, const QmmArgs args) {
+qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map16, const __grid_constant__ CUtensorMap x_map32,
+                   const __grid_constant__ CUtensorMap x_map64, const __grid_constant__ CUtensorMap x_map128,
+                   const __grid_constant__ CUtensorMap w_map0, const __grid_constant__ CUtensorMap w_map1, const QmmArgs args) {
     extern __shared__ uint8_t smem_raw[];
-    using L = QmmSmem<NMAT>;
-    constexpr int kAStages = L::kAStages;
+    constexpr uint32_t kMatRows = kQmmRows / NMAT;                     // rows of one matrix in a tile
+    const QmmPlan& plan = args.plan;
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;                      // swizzle atoms need 1024-byte alignment
     uint8_t* base_ptr = smem_raw + (base - raw);
-    const uint32_t plane_bytes = L::plane_bytes(args.k);
-    const uint32_t scale_buf = L::scale_buf_bytes(args.k);
-    const uint32_t bars = base + L::off_bars(args.k);
+    const uint32_t bars = base + plan.off_bars;
     // barrier map (8 bytes each)
-    auto bar_full_raw = [&](uint32_t s) { return bars + s * 8; };                            // 8: TMA tx
-    auto bar_empty_raw = [&](uint32_t s) { return bars + (8 + s) * 8; };                     // 8: dequant warps
-    auto bar_full_b = [&](uint32_t s) { return bars + (16 + s) * 8; };                       // 16: TMA tx
-    auto bar_empty_b = [&](uint32_t s) { return bars + (32 + s) * 8; };                      // 16: tcgen05.commit
-    auto bar_full_a = [&](uint32_t s) { return bars + (48 + s) * 8; };                       // 8: dequant warps
-    auto bar_empty_a = [&](uint32_t s) { return bars + (56 + s) * 8; };                      // 8: tcgen05.commit
-    auto bar_full_sc = [&](uint32_t b) { return bars + (64 + b) * 8; };                      // 2: TMA tx
-    auto bar_empty_sc = [&](uint32_t b) { return bars + (66 + b) * 8; };                     // 2: dequant warps
-    auto bar_acc_full = [&](uint32_t b) { return bars + (68 + b) * 8; };                     // 2: tcgen05.commit
-    auto bar_acc_empty = [&](uint32_t b) { return bars + (70 + b) * 8; };                    // 2: epilogue warps
-    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(base_ptr + L::off_bars(args.k) + 72 * 8);
-    volatile uint32_t* bslots_slot = tmem_slot + 1;
+    auto bar_full_raw = [&](uint32_t s) { return bars + s * 8; };                            // 4: TMA tx
+    auto bar_empty_raw = [&](uint32_t s) { return bars + (4 + s) * 8; };                     // 4: dequant warps
+    auto bar_full_b = [&](uint32_t s) { return bars + (8 + s) * 8; };                        // 12: TMA tx
+    auto bar_empty_b = [&](uint32_t s) { return bars + (20 + s) * 8; };                      // 12: tcgen05.commit
+    auto bar_full_a = [&](uint32_t s) { return bars + (32 + s) * 8; };                       // 4: the dequant warps of a half
+    auto bar_empty_a = [&](uint32_t s) { return bars + (36 + s) * 8; };                      // 4: tcgen05.commit
+    auto bar_full_sc = [&](uint32_t b) { return bars + (40 + b) * 8; };                      // 4: bulk-copy tx
+    auto bar_empty_sc = [&](uint32_t b) { return bars + (44 + b) * 8; };                     // 4: dequant warps
+    auto bar_acc_full = [&](uint32_t b) { return bars + (48 + b) * 8; };                     // 2: tcgen05.commit
+    auto bar_acc_empty = [&](uint32_t b) { return bars + (50 + b) * 8; };                    // 2: epilogue warps
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(base_ptr + plan.off_bars + 52 * 8);   // TMEM base
+    uint4* table = reinterpret_cast<uint4*>(base_ptr + plan.off_table);
 
     const int warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
-    const uint32_t groups_per_row = args.k / kGroup;
-    const uint32_t ksteps = (groups_per_row + 1) / 2;             // an odd last group is padded with zero columns
-    const uint32_t wrow_tiles = (args.rows + kQmmRows - 1) / kQmmRows;
-    const uint32_t ngroups = args.totals[0];
-    const uint32_t total_tiles = args.totals[1] * wrow_tiles;
+    const uint32_t ng = args.k / kGroup;
+    const uint32_t ksteps = (ng + 3) / 4;                              // packed-code stages per tile
+    const uint32_t halves = (ng + 1) / 2;                              // operand slots per tile; the last may hold one group only
+    const uint32_t wrow_tiles = (args.rows + kMatRows - 1) / kMatRows;
 
-    // maps a work item to (group, token tile within the group, weight-row tile)
-    auto locate = [&](uint32_t tile, uint32_t& gi, uint32_t& tt, uint32_t& wt) {
-        const uint32_t tglob = tile / wrow_tiles;
-        wt = tile % wrow_tiles;
-        uint32_t lo = 0, hi = ngroups;                                 // last group with tile_start <= tglob
-        while (hi - lo > 1) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (args.groups[mid].tile_start <= tglob) lo = mid; else hi = mid;
-        }
-        gi = lo;
-        tt = tglob - args.groups[lo].tile_start;
-    };
-    auto tile_tokens = [&](uint32_t count, uint32_t tt) {
-        const uint32_t left = count - tt * kQmmTokMax;
-        return left < (uint32_t)kQmmTokMax ? left : (uint32_t)kQmmTokMax;
-    };
-
+    pdl_launch_dependents();
     if (threadIdx.x == 0) {
-        for (uint32_t s = 0; s < 8; ++s) {
-            q_mbar_init(bar_full_raw(s), 1);
-            q_mbar_init(bar_empty_raw(s), kQmmDequantWarps);
-            q_mbar_init(bar_full_a(s), kQmmDequantWarps);
-            q_mbar_init(bar_empty_a(s), 1);
-        }
-        for (uint32_t s = 0; s < 16; ++s) { q_mbar_init(bar_full_b(s), 1); q_mbar_init(bar_empty_b(s), 1); }
-        for (uint32_t b = 0; b < 2; ++b) {
-            q_mbar_init(bar_full_sc(b), 1);
-            q_mbar_init(bar_empty_sc(b), kQmmDequantWarps);
-            q_mbar_init(bar_acc_full(b), 1);
-            q_mbar_init(bar_acc_empty(b), kQmmEpilogueWarps);
-        }
+        for (uint32_t s = 0; s < (uint32_t)kQmmRawMax; ++s) { q_mbar_init(bar_full_raw(s), 1); q_mbar_init(bar_empty_raw(s), kQmmDequantWarps); }
+        for (uint32_t s = 0; s < (uint32_t)kQmmBMax; ++s) { q_mbar_init(bar_full_b(s), 1); q_mbar_init(bar_empty_b(s), 1); }
+        for (uint32_t s = 0; s < (uint32_t)kQmmASlots; ++s) { q_mbar_init(bar_full_a(s), kQmmDequantWarps / 2); q_mbar_init(bar_empty_a(s), 1); }
+        for (uint32_t b = 0; b < (uint32_t)kQmmScMax; ++b) { q_mbar_init(bar_full_sc(b), 1); q_mbar_init(bar_empty_sc(b), kQmmDequantWarps); }
+        for (uint32_t b = 0; b < 2; ++b) { q_mbar_init(bar_acc_full(b), 1); q_mbar_init(bar_acc_empty(b), kQmmEpilogueWarps); }
         q_fence_async_smem();
-        // Activation slots per step, fixed for this CTA: the largest tile it will meet, rounded up to 1, 2, 4 or 8
-        // boxes of 16 rows, so that a step's rows are contiguous and the ring never has to be re-partitioned.
-        uint32_t max_tok = 1;
-        for (uint32_t tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
-            uint32_t gi, tt, wt;
-            locate(tile, gi, tt, wt);
-            const uint32_t n = tile_tokens(args.groups[gi].count, tt);
-            max_tok = n > max_tok ? n : max_tok;
-        }
-        const uint32_t boxes = (max_tok + kQmmBoxRows - 1) / kQmmBoxRows;
-        *bslots_slot = boxes <= 1 ? 1u : boxes <= 2 ? 2u : boxes <= 4 ? 4u : 8u;
     }
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
                      ::"r"(smem_u32(const_cast<uint32_t*>(tmem_slot))), "r"((uint32_t)kQmmTmemCols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    pdl_wait();                                                        // routes and activations come from the kernels before this one
+    const uint32_t ngroups = args.totals[0], total_tiles = args.totals[1] * wrow_tiles, n_top = args.totals[2];
+    if (threadIdx.x < ngroups) table[threadIdx.x] = args.groups[threadIdx.x];
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    const uint32_t b_slots = *bslots_slot;                            // 16-row boxes per 64-column half of an activation stage
-    const uint32_t b_stages = kQmmBSlots / (2 * b_slots);             // 16, 8, 4 or 2
-    const uint32_t b_half_bytes = b_slots * kQmmBoxRows * 128;        // one 64-column half of a stage
+    // Activation ring: slots of the launch's largest tile, as many as fit.
+    const uint32_t b_half_bytes = n_top * 128;                        // one 64-column block of a slot
+    const uint32_t b_fit = plan.b_bytes / (2 * b_half_bytes);
+    const uint32_t b_stages = b_fit < (uint32_t)kQmmBMax ? b_fit : (uint32_t)kQmmBMax;
     const uint32_t a_ring = tmem_base + kQmmAccCols;
 
     uint32_t fail = 0;
-    uint32_t it = 0;         // running k-step index over all of this CTA's tiles (ring positions)
+    QmmTile tl;
 
     if (warp == 0) {
-        // ===================== copy issuer: packed codes, activation boxes, scale planes =====================
-        uint32_t tile_idx = 0, sb = 0, ub = 0;                     // activation ring position and lap
-        auto issue_scales = [&](uint32_t tile, uint32_t idx) -> bool {
-            const uint32_t buf = idx & 1, n = idx >> 1;
-            if (n > 0 && !q_mbar_wait(bar_empty_sc(buf), (n - 1) & 1)) return false;
-            if (lane == 0) {
-                uint32_t gi, tt, wt;
-                locate(tile, gi, tt, wt);
-                const uint32_t row0 = wt * kQmmRows;
-                const uint32_t nrows = args.rows - row0 < (uint32_t)kQmmRows ? args.rows - row0 : (uint32_t)kQmmRows;
-                const uint32_t bytes = nrows * groups_per_row * 2;        // a multiple of 16: rows are a multiple of 8
-                q_mbar_expect_tx(bar_full_sc(buf), NMAT * 2 * bytes);
-                for (int m = 0; m < NMAT; ++m) {
-                    const uint32_t dst = base + L::kOffScales + buf * scale_buf + m * 2 * plane_bytes;
-                    q_bulk_g2s(dst, args.groups[gi].S[m] + (size_t)row0 * groups_per_row, bytes, bar_full_sc(buf));
-                    q_bulk_g2s(dst + plane_bytes, args.groups[gi].B[m] + (size_t)row0 * groups_per_row, bytes, bar_full_sc(buf));
-                }
-            }
-            __syncwarp();
-            return true;
-        };
-        if (blockIdx.x < total_tiles && !issue_scales(blockIdx.x, 0)) fail = kErrQmmTimeout | 6;
-        for (uint32_t tile = blockIdx.x; tile < total_tiles && !fail; tile += gridDim.x, ++tile_idx) {
-            uint32_t gi, tt, wt;
-            locate(tile, gi, tt, wt);
-            const uint32_t expert = args.groups[gi].expert;
-            const uint32_t row0 = args.groups[gi].row_start + tt * kQmmTokMax;
-            const uint32_t boxes = (tile_tokens(args.groups[gi].count, tt) + kQmmBoxRows - 1) / kQmmBoxRows;
-            // the next tile's scale planes go out once the dequantisers are certainly done with the tile before
-            // this one (they have consumed this tile's first step when its ring slot comes round again)
-            const uint32_t scale_step = ksteps > (uint32_t)kQmmRawStages ? (uint32_t)kQmmRawStages : ksteps - 1;
-            for (uint32_t ks = 0; ks < ksteps; ++ks, ++it) {
-                const uint32_t sr = it % kQmmRawStages, ur = it / kQmmRawStages;
+        // ===================== copy issuer: packed codes =====================
+        uint32_t sr = 0, ur = 0;
+        for (uint32_t tile = blockIdx.x; tile < total_tiles && !fail; tile += gridDim.x) {
+            tl.locate(table, ngroups, wrow_tiles, tile);
+            for (uint32_t ks = 0; ks < ksteps; ++ks) {
                 if (ur > 0 && !q_mbar_wait(bar_empty_raw(sr), (ur - 1) & 1)) { fail = kErrQmmTimeout | 1; break; }
-                const bool leader = elect_one();
-                if (leader) {
-                    q_mbar_expect_tx(bar_full_raw(sr), L::kRawStage);
-                    tma_load_3d(base + L::kOffRaw + sr * L::kRawStage, &w_map0, (int)(ks * (kQmmK / 2)), (int)(wt * kQmmRows), (int)expert, bar_full_raw(sr));
+                if (elect_one()) {
+                    const uint32_t dst = base + sr * kQmmRawBytes;
+                    q_mbar_expect_tx(bar_full_raw(sr), kQmmRawBytes);
+                    tma_load_3d(dst, &w_map0, (int)(ks * (kQmmRawK / 2)), (int)(tl.wt * kMatRows), (int)tl.expert, bar_full_raw(sr));
                     if (NMAT == 2)
-                        tma_load_3d(base + L::kOffRaw + sr * L::kRawStage + L::kRawMat, &w_map1, (int)(ks * (kQmmK / 2)), (int)(wt * kQmmRows), (int)expert, bar_full_raw(sr));
+                        tma_load_3d(dst + kQmmRawBytes / 2, &w_map1, (int)(ks * (kQmmRawK / 2)), (int)(tl.wt * kMatRows), (int)tl.expert, bar_full_raw(sr));
                 }
+                __syncwarp();
+                if (++sr == plan.raw_stages) { sr = 0; ++ur; }
+            }
+        }
+        if (fail)            // the copies already issued land before the CTA's shared memory goes away (bounded)
+            for (uint32_t s = 0; s < plan.raw_stages; ++s) q_mbar_wait(bar_full_raw(s), (s < sr ? ur : ur + 1) & 1);
+    } else if (warp == 2) {
+        // ===================== copy issuer: activations =====================
+        uint32_t sb = 0, ub = 0;
+        for (uint32_t tile = blockIdx.x; tile < total_tiles && !fail; tile += gridDim.x) {
+            tl.locate(table, ngroups, wrow_tiles, tile);
+            const uint32_t n = tl.n();
+            for (uint32_t hs = 0; hs < halves; ++hs) {
                 if (ub > 0 && !q_mbar_wait(bar_empty_b(sb), (ub - 1) & 1)) { fail = kErrQmmTimeout | 7; break; }
-                if (leader) {
-                    if (boxes > 4) {                              // more than 64 tokens: one 128-row box per half
-                        q_mbar_expect_tx(bar_full_b(sb), 2 * kQmmTokMax * 128);
-                        for (uint32_t h = 0; h < 2; ++h)
-                            tma_load_2d(base + L::kOffB + sb * 2 * b_half_bytes + h * b_half_bytes, &x_map_big,
-                                        (int)(ks * kQmmK + h * 64), (int)row0, bar_full_b(sb));
-                    } else {
-                        q_mbar_expect_tx(bar_full_b(sb), 2 * boxes * kQmmBoxRows * 128);
-                        for (uint32_t h = 0; h < 2; ++h)          // columns past K (odd group count) read as zero
-                            for (uint32_t b = 0; b < boxes; ++b)
-                                tma_load_2d(base + L::kOffB + sb * 2 * b_half_bytes + h * b_half_bytes + b * kQmmBoxRows * 128, &x_map,
-                                            (int)(ks * kQmmK + h * 64), (int)(row0 + b * kQmmBoxRows), bar_full_b(sb));
+                if (elect_one()) {
+                    const uint32_t blocks = ng - 2 * hs < 2u ? 1u : 2u;
+                    q_mbar_expect_tx(bar_full_b(sb), blocks * n * 128);
+                    for (uint32_t h = 0; h < blocks; ++h) {
+                        uint32_t dst = base + plan.off_b + (sb * 2 + h) * b_half_bytes;
+                        const int col = (int)(hs * kQmmHalfK + h * 64);
+                        int row = (int)tl.row0;
+                        if (n == 128) {
+                            tma_load_2d(dst, &x_map128, col, row, bar_full_b(sb));
+                        } else {                                  // 16 to 112 rows: boxes of 64, 32 and 16
+                            if (n & 64) { tma_load_2d(dst, &x_map64, col, row, bar_full_b(sb)); dst += 64 * 128; row += 64; }
+                            if (n & 32) { tma_load_2d(dst, &x_map32, col, row, bar_full_b(sb)); dst += 32 * 128; row += 32; }
+                            if (n & 16) tma_load_2d(dst, &x_map16, col, row, bar_full_b(sb));
+                        }
                     }
                 }
                 __syncwarp();
                 if (++sb == b_stages) { sb = 0; ++ub; }
-                if (ks == scale_step && tile + gridDim.x < total_tiles && !issue_scales(tile + gridDim.x, tile_idx + 1)) { fail = kErrQmmTimeout | 6; break; }
             }
         }
+        if (fail)
+            for (uint32_t s = 0; s < b_stages; ++s) q_mbar_wait(bar_full_b(s), (s < sb ? ub : ub + 1) & 1);
+    } else if (warp == 3) {
+        // ===================== copy issuer: scale and bias planes of a tile =====================
+        uint32_t sc = 0, uc = 0;
+        for (uint32_t tile = blockIdx.x; tile < total_tiles && !fail; tile += gridDim.x) {
+            tl.locate(table, ngroups, wrow_tiles, tile);
+            if (uc > 0 && !q_mbar_wait(bar_empty_sc(sc), (uc - 1) & 1)) { fail = kErrQmmTimeout | 6; break; }
+            if (elect_one()) {
+                const uint32_t first = tl.wt * kMatRows;
+                const uint32_t nrows = args.rows - first < kMatRows ? args.rows - first : kMatRows;
+                const uint32_t bytes = nrows * ng * 2;                // a multiple of 16: rows are a multiple of 8
+                const size_t off = (size_t)tl.expert * args.expert_stride + (size_t)first * ng * 2;
+                q_mbar_expect_tx(bar_full_sc(sc), NMAT * 2 * bytes);
+#pragma unroll
+                for (int m = 0; m < NMAT; ++m) {
+                    const uint32_t dst = base + plan.off_sc + sc * plan.sc_bytes + m * 2 * plan.plane_bytes;
+                    q_bulk_g2s(dst, reinterpret_cast<const uint8_t*>(args.S[m]) + off, bytes, bar_full_sc(sc));
+                    q_bulk_g2s(dst + plan.plane_bytes, reinterpret_cast<const uint8_t*>(args.B[m]) + off, bytes, bar_full_sc(sc));
+                }
+            }
+            __syncwarp();
+            if (++sc == plan.sc_bufs) { sc = 0; ++uc; }
+        }
+        if (fail)
+            for (uint32_t s = 0; s < plan.sc_bufs; ++s) q_mbar_wait(bar_full_sc(s), (s < sc ? uc : uc + 1) & 1);
     } else if (warp == 1) {
         // ===================== MMA issuer =====================
-        AccPlan plan;
-        uint32_t sb = 0, ub = 0;                                  // activation ring position and lap
-        const uint64_t b_desc0 = umma_smem_desc(base + L::kOffB);
+        uint32_t sb = 0, ub = 0, sa = 0, ua = 0, buf = 0, uacc = 0;
+        const uint64_t b_desc0 = umma_smem_desc(base + plan.off_b);
         for (uint32_t tile = blockIdx.x; tile < total_tiles && !fail; tile += gridDim.x) {
-            uint32_t gi, tt, wt;
-            locate(tile, gi, tt, wt);
-            const uint32_t n_mma = (tile_tokens(args.groups[gi].count, tt) + 15u) & ~15u;
-            const uint32_t idesc = qmm_idesc(n_mma);
-            plan.next<NMAT>(n_mma);
-#pragma unroll
-            for (uint32_t b = 0; b < 2; ++b) {
-                if (plan.takes(b) && plan.uses(b) > 0 && !q_mbar_wait(bar_acc_empty(b), (plan.uses(b) - 1) & 1))
-                    fail = kErrQmmTimeout | 2;
-            }
-            if (fail) break;
+            tl.locate(table, ngroups, wrow_tiles, tile);
+            const uint32_t idesc = qmm_idesc(tl.n());
+            if (uacc > 0 && !q_mbar_wait(bar_acc_empty(buf), (uacc - 1) & 1)) { fail = kErrQmmTimeout | 2; break; }
             tc_fence_after();
-            const uint32_t acc = tmem_base + plan.col0;
-            for (uint32_t ks = 0; ks < ksteps; ++ks, ++it) {
-                const uint32_t sa = it % kAStages, ua = it / kAStages;
-                if (!q_mbar_wait(bar_full_a(sa), ua & 1) || !q_mbar_wait(bar_full_b(sb), ub & 1)) { fail = kErrQmmTimeout | 3; break; }
+            const uint32_t acc = tmem_base + buf * 128;
+            for (uint32_t hs = 0; hs < halves; ++hs) {
+                if (!q_mbar_wait(bar_full_b(sb), ub & 1) || !q_mbar_wait(bar_full_a(sa), ua & 1)) { fail = kErrQmmTimeout | 3; break; }
                 tc_fence_after();
                 const bool leader = elect_one();
                 const uint64_t b_desc = b_desc0 + (uint64_t)((sb * 2 * b_half_bytes) >> 4);
-                const uint32_t a_stage = a_ring + sa * (NMAT * 64);
-                const uint32_t nj = (2 * ks + 1 < groups_per_row) ? 8u : 4u;     // the padded half of an odd last step is skipped
+                const uint32_t a_slot = a_ring + sa * 64;
+                const bool whole = 2 * hs + 1 < ng;                   // the missing half of an odd last slot is skipped
 #pragma unroll
-                for (int m = 0; m < NMAT; ++m) {
-#pragma unroll
-                    for (int j = 0; j < kQmmK / 16; ++j) {        // 16 columns of K: 8 TMEM columns of A, 32 bytes of B
-                        if ((uint32_t)j < nj && leader)
-                            tc_mma_f16_ts(acc + m * plan.mat_stride, a_stage + m * 64 + j * 8,
-                                          b_desc + (uint64_t)((j >> 2) * (b_half_bytes >> 4) + (j & 3) * 2), idesc, (ks > 0 || j > 0) ? 1u : 0u);
-                    }
+                for (int j = 0; j < kQmmHalfK / 16; ++j) {            // 16 columns of K: 8 TMEM columns of A, 32 bytes of B
+                    if ((j < 4 || whole) && leader)
+                        tc_mma_f16_ts(acc, a_slot + j * 8, b_desc + (uint64_t)((j >> 2) * (b_half_bytes >> 4) + (j & 3) * 2), idesc,
+                                      (hs > 0 || j > 0) ? 1u : 0u);
                 }
                 if (leader) {
-                    tc_commit(bar_empty_a(sa));                   // both rings' stages are free once these MMAs have read them
+                    tc_commit(bar_empty_a(sa));                       // both slots are free once these MMAs have read them
                     tc_commit(bar_empty_b(sb));
-                    if (ks + 1 == ksteps) {
-                        if (plan.both || plan.buf == 0) tc_commit(bar_acc_full(0));
-                        if (plan.both || plan.buf == 1) tc_commit(bar_acc_full(1));
-                    }
+                    if (hs + 1 == halves) tc_commit(bar_acc_full(buf));
                 }
                 __syncwarp();
                 if (++sb == b_stages) { sb = 0; ++ub; }
+                if (++sa == (uint32_t)kQmmASlots) { sa = 0; ++ua; }
             }
-            plan.done();
+            if (++buf == 2) { buf = 0; ++uacc; }
         }
-    } else if (warp >= kQmmFirstDequantWarp && warp < kQmmFirstEpilogueWarp) {
-        // ===================== dequantisers: four threads per weight row =====================
+    } else if (warp < kQmmFirstEpilogueWarp) {
+        // ===================== dequantisers: a thread takes one quantisation group of one weight row per stage =====================
         const uint32_t dw = warp - kQmmFirstDequantWarp;
-        const uint32_t q = dw & 3, qc = dw >> 2;                 // TMEM lane quarter; quarter of the step's 128 columns
+        const uint32_t q = dw & 3, gc = dw >> 2;                 // TMEM lane quarter; group within the stage
+        const uint32_t half = gc >> 1;
         const uint32_t r = q * kWarp + lane;                     // row within the tile = TMEM lane
-        // packed codes of the row: 64 bytes whose 16-byte chunks sit at chunk ^ ((row / 2) % 4) (64-byte TMA swizzle)
-        const uint32_t raw_off = r * 64 + ((qc ^ ((r >> 1) & 3u)) << 4);
-        const uint32_t sc_off = r * groups_per_row * 2;
-        const uint32_t a_lane = a_ring + ((q * kWarp) << 16) + qc * 16;
-        uint32_t tile_idx = 0;
-        for (uint32_t tile = blockIdx.x; tile < total_tiles && !fail; tile += gridDim.x, ++tile_idx) {
-            const uint32_t buf = tile_idx & 1;
-            if (!q_mbar_wait(bar_full_sc(buf), (tile_idx >> 1) & 1)) { fail = kErrQmmTimeout | 8; break; }
-            const uint32_t sc_base = base + L::kOffScales + buf * scale_buf + sc_off;
-            for (uint32_t ks = 0; ks < ksteps; ++ks, ++it) {
-                const uint32_t sr = it % kQmmRawStages, ur = it / kQmmRawStages;
-                const uint32_t sa = it % kAStages, ua = it / kAStages;
-                const uint32_t grp_idx = 2 * ks + (qc >> 1);      // this thread's 32 columns lie in one quantisation group
-                const bool real = grp_idx < groups_per_row;      // the padded group of an odd last step dequantises to zero
+        // packed codes of the row: 128 bytes whose 16-byte chunks sit at chunk ^ (row % 8) (128-byte TMA swizzle)
+        const uint32_t raw_off0 = r * 128 + (((2 * gc) ^ (r & 7u)) << 4), raw_off1 = r * 128 + (((2 * gc + 1) ^ (r & 7u)) << 4);
+        const uint32_t sc_off = base + plan.off_sc + (r / kMatRows) * 2 * plan.plane_bytes + (r % kMatRows) * ng * 2;
+        const uint32_t a_lane = a_ring + ((q * kWarp) << 16) + (gc & 1) * 32;
+        uint32_t sr = 0, ur = 0, sc = 0, uc = 0, slot0 = 0;       // slot0: operand slots of the tiles before this one
+        for (uint32_t tile = blockIdx.x; tile < total_tiles && !fail; tile += gridDim.x, slot0 += halves) {
+            if (!q_mbar_wait(bar_full_sc(sc), uc & 1)) { fail = kErrQmmTimeout | 8; break; }
+            const uint32_t sc_base = sc_off + sc * plan.sc_bytes;
+            for (uint32_t ks = 0; ks < ksteps; ++ks) {
+                const uint32_t grp = 4 * ks + gc, hs = 2 * ks + half;
+                const bool real = grp < ng;                       // a group past K is neither dequantised nor multiplied
+                const float sf = real ? bf16_bits_to_float((uint16_t)q_lds16(sc_base + grp * 2)) : 0.0f;
+                const float bf = real ? bf16_bits_to_float((uint16_t)q_lds16(sc_base + plan.plane_bytes + grp * 2)) : 0.0f;
+                const bool fast = __all_sync(kFullMask, fabsf(sf) < FastScale<NATURAL_K>::kLimit);
                 if (!q_mbar_wait(bar_full_raw(sr), ur & 1)) { fail = kErrQmmTimeout | 4; break; }
-                uint4 codes[NMAT];
-                float sf[NMAT], bf[NMAT];
-                bool fast = true;
-#pragma unroll
-                for (int m = 0; m < NMAT; ++m) {
-                    codes[m] = q_lds128(base + L::kOffRaw + sr * L::kRawStage + m * L::kRawMat + raw_off);
-                    sf[m] = real ? bf16_bits_to_float((uint16_t)q_lds16(sc_base + m * 2 * plane_bytes + grp_idx * 2)) : 0.0f;
-                    bf[m] = real ? bf16_bits_to_float((uint16_t)q_lds16(sc_base + m * 2 * plane_bytes + plane_bytes + grp_idx * 2)) : 0.0f;
-                    fast = fast && fabsf(sf[m]) < 0.03125f;
-                }
-                uint4 out[NMAT][4];
-                if (__all_sync(kFullMask, fast)) {                // one branch per warp and step, both arms straight-line
-#pragma unroll
-                    for (int m = 0; m < NMAT; ++m) {
-                        const __half2 s_fast = __float2half2_rn(sf[m] * 1048576.0f), b2 = __float2half2_rn(bf[m]);
-                        out[m][0] = dequant8_fast<NATURAL_K>(codes[m].x, s_fast, b2);
-                        out[m][1] = dequant8_fast<NATURAL_K>(codes[m].y, s_fast, b2);
-                        out[m][2] = dequant8_fast<NATURAL_K>(codes[m].z, s_fast, b2);
-                        out[m][3] = dequant8_fast<NATURAL_K>(codes[m].w, s_fast, b2);
-                    }
+                const uint4 c0 = q_lds128(base + sr * kQmmRawBytes + raw_off0), c1 = q_lds128(base + sr * kQmmRawBytes + raw_off1);
+                uint4 out[8];
+                if (fast) {                                       // one branch per warp and stage, both arms straight-line
+                    const FastScale<NATURAL_K> s2(sf);
+                    const __half2 b2 = __float2half2_rn(bf);
+                    out[0] = dequant8_fast<NATURAL_K>(c0.x, s2, b2); out[1] = dequant8_fast<NATURAL_K>(c0.y, s2, b2);
+                    out[2] = dequant8_fast<NATURAL_K>(c0.z, s2, b2); out[3] = dequant8_fast<NATURAL_K>(c0.w, s2, b2);
+                    out[4] = dequant8_fast<NATURAL_K>(c1.x, s2, b2); out[5] = dequant8_fast<NATURAL_K>(c1.y, s2, b2);
+                    out[6] = dequant8_fast<NATURAL_K>(c1.z, s2, b2); out[7] = dequant8_fast<NATURAL_K>(c1.w, s2, b2);
                 } else {
-#pragma unroll
-                    for (int m = 0; m < NMAT; ++m) {
-                        const __half2 s2 = __float2half2_rn(sf[m]), b2 = __float2half2_rn(bf[m]);
-                        out[m][0] = dequant8_wide<NATURAL_K>(codes[m].x, s2, b2);
-                        out[m][1] = dequant8_wide<NATURAL_K>(codes[m].y, s2, b2);
-                        out[m][2] = dequant8_wide<NATURAL_K>(codes[m].z, s2, b2);
-                        out[m][3] = dequant8_wide<NATURAL_K>(codes[m].w, s2, b2);
-                    }
+                    const __half2 s2 = __float2half2_rn(sf), b2 = __float2half2_rn(bf);
+                    out[0] = dequant8_wide<NATURAL_K>(c0.x, s2, b2); out[1] = dequant8_wide<NATURAL_K>(c0.y, s2, b2);
+                    out[2] = dequant8_wide<NATURAL_K>(c0.z, s2, b2); out[3] = dequant8_wide<NATURAL_K>(c0.w, s2, b2);
+                    out[4] = dequant8_wide<NATURAL_K>(c1.x, s2, b2); out[5] = dequant8_wide<NATURAL_K>(c1.y, s2, b2);
+                    out[6] = dequant8_wide<NATURAL_K>(c1.z, s2, b2); out[7] = dequant8_wide<NATURAL_K>(c1.w, s2, b2);
                 }
                 __syncwarp();
                 if (lane == 0) q_mbar_arrive(bar_empty_raw(sr));  // the codes are in registers
-                if (ua > 0 && !q_mbar_wait(bar_empty_a(sa), (ua - 1) & 1)) { fail = kErrQmmTimeout | 5; break; }
-                tc_fence_after();
-#pragma unroll
-                for (int m = 0; m < NMAT; ++m) tc_st16(a_lane + sa * (NMAT * 64) + m * 64, out[m][0], out[m][1], out[m][2], out[m][3]);
-                tc_wait_st();
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) q_mbar_arrive(bar_full_a(sa));
+                if (++sr == plan.raw_stages) { sr = 0; ++ur; }
+                if (hs < halves) {
+                    const uint32_t slot = slot0 + hs, sa = slot % kQmmASlots, ua = slot / kQmmASlots;
+                    if (ua > 0 && !q_mbar_wait(bar_empty_a(sa), (ua - 1) & 1)) { fail = kErrQmmTimeout | 5; break; }
+                    tc_fence_after();
+                    if (real) {
+                        tc_st32(a_lane + sa * 64, out);
+                        tc_wait_st();
+                    }
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) q_mbar_arrive(bar_full_a(sa));
+                }
             }
             __syncwarp();
-            if (lane == 0) q_mbar_arrive(bar_empty_sc(buf));      // done with this tile's scale planes
+            if (lane == 0) q_mbar_arrive(bar_empty_sc(sc));       // done with this tile's scale planes
+            if (++sc == plan.sc_bufs) { sc = 0; ++uc; }
         }
-    } else if (warp >= kQmmFirstEpilogueWarp) {
-        // ===================== epilogue: TMEM -> registers -> global =====================
+    } else {
+        // ===================== epilogue: TMEM -> registers -> shared memory -> 16-byte stores =====================
+        // A lane holds one weight row and a register one token, but the output is [token][row]: 32 tokens at a time go
+        // through a staging tile, so that a token's rows leave as whole 16-byte words.
         const uint32_t q = warp & 3;                              // TMEM lane quarter this warp may read
-        const uint32_t r = q * kWarp + lane;                      // weight row within the tile = TMEM lane
-        AccPlan plan;
+        const uint32_t r = q * kWarp + lane;                      // row within the tile = TMEM lane
+        const uint32_t et = threadIdx.x - kQmmFirstEpilogueWarp * kWarp;
+        constexpr uint32_t kTokBytes = kMatRows * 2;              // staged bytes per token
+        const uint32_t xch = base + plan.off_stage;               // gate/up: 32 tokens x 64 rows fp32
+        const uint32_t stage0 = NMAT == 2 ? xch + 8192 : xch;     // two staging tiles of 32 tokens
+        const uint32_t mrow = r % kMatRows;
+        const uint32_t pos = (NMAT == 2 && !NATURAL_K) ? permuted_col(mrow) : mrow;      // the GeGLU output feeds the down GEMM
+        uint32_t buf = 0, uacc = 0, flip = 0;
         for (uint32_t tile = blockIdx.x; tile < total_tiles && !fail; tile += gridDim.x) {
-            uint32_t gi, tt, wt;
-            locate(tile, gi, tt, wt);
-            const QmmGroup grp = args.groups[gi];
-            const uint32_t wrow = wt * kQmmRows + r;
-            const uint32_t out_col = (NMAT == 2 && !NATURAL_K) ? permuted_col(wrow) : wrow;   // the GeGLU output feeds the down GEMM
-            const uint32_t tok0 = tt * kQmmTokMax;
-            const uint32_t ntok = tile_tokens(grp.count, tt);
-            plan.next<NMAT>((ntok + 15u) & ~15u);
-#pragma unroll
-            for (uint32_t b = 0; b < 2; ++b) {
-                if (plan.takes(b) && !q_mbar_wait(bar_acc_full(b), plan.uses(b) & 1)) fail = kErrQmmTimeout | 9;
-            }
-            if (fail) break;
+            tl.locate(table, ngroups, wrow_tiles, tile);
+            const uint32_t first = tl.wt * kMatRows;
+            const uint32_t nrows = args.rows - first < kMatRows ? args.rows - first : kMatRows;
+            if (!q_mbar_wait(bar_acc_full(buf), uacc & 1)) fail = kErrQmmTimeout | 9;
+            // every warp of the role leaves together: the barriers below count all four
+            asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbarrier.red.or.pred q, 1, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                         : "=r"(flip) : "r"(fail) : "memory");
+            if (flip) { if (!fail) fail = kErrQmmTimeout | 9; break; }
             tc_fence_after();
-            const uint32_t acc = tmem_base + ((q * kWarp) << 16) + plan.col0;
-            uint16_t* out_row = args.out + (size_t)(grp.row_start + tok0) * args.out_stride + out_col;
-            for (uint32_t c0 = 0; c0 < ntok; c0 += 16) {
-                uint32_t v0[16], v1[16];
-                tc_ld16(acc + c0, v0);
-                if (NMAT == 2) tc_ld16(acc + plan.mat_stride + c0, v1);
+            const uint32_t acc = tmem_base + ((q * kWarp) << 16) + buf * 128;
+            uint32_t which = 0;
+            for (uint32_t c0 = 0; c0 < tl.ntok; c0 += 32, which ^= 1) {
+                uint32_t va[16], vb[16];
+                tc_ld16(acc + c0, va);
+                tc_ld16(acc + c0 + 16, vb);                       // past the tile's tokens: stale columns of the buffer, never stored
                 tc_wait_ld();
-                if (wrow < args.rows) {
+                if (c0 + 32 >= tl.ntok) {                         // the accumulators are in registers
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) q_mbar_arrive(bar_acc_empty(buf));
+                }
+                const uint32_t stage = stage0 + which * (32 * kTokBytes) + pos * 2;
+                if constexpr (NMAT == 2) {
+                    // lanes 0..63 hold gate rows, 64..127 up rows: each side hands half of the tokens to the other
+                    const bool gate_side = q < 2;
+                    const uint32_t xrow = xch + mrow * 4;
+#pragma unroll
+                    for (int j = 0; j < 16; ++j)
+                        asm volatile("st.shared.b32 [%0], %1;" ::"r"(xrow + (gate_side ? 16 + j : j) * 256), "r"(gate_side ? vb[j] : va[j]) : "memory");
+                    asm volatile("barrier.sync 1, 128;" ::: "memory");
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
-                        const uint32_t tok = c0 + j;
-                        if (tok < ntok) {
-                            float y = __uint_as_float(v0[j]);
-                            if (NMAT == 2) {
-                                float gt = y, up = __uint_as_float(v1[j]);
-                                if (args.round_gate_up) {          // Kernels/MoE/SharedExpertInt4.swift:62-93
-                                    gt = __half2float(__float2half_rn(gt));
-                                    up = __half2float(__float2half_rn(up));
-                                }
-                                y = gelu_tanh(gt) * up;            // prefill.metal:634-636
-                            }
-                            out_row[(size_t)tok * args.out_stride] = __half_as_ushort(__float2half_rn(y));
+                        const uint32_t tok = gate_side ? j : 16 + j;
+                        uint32_t o;
+                        asm volatile("ld.shared.b32 %0, [%1];" : "=r"(o) : "r"(xrow + tok * 256));
+                        float gt = __uint_as_float(gate_side ? va[j] : o), up = __uint_as_float(gate_side ? o : vb[j]);
+                        if (args.round_gate_up) {                 // Kernels/MoE/SharedExpertInt4.swift:62-93
+                            gt = __half2float(__float2half_rn(gt));
+                            up = __half2float(__float2half_rn(up));
+                        }
+                        const uint16_t y = __half_as_ushort(__float2half_rn(gelu_tanh(gt) * up));        // prefill.metal:634-636
+                        asm volatile("st.shared.b16 [%0], %1;" ::"r"(stage + tok * kTokBytes), "h"(y) : "memory");
+                    }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                        const uint16_t y0 = __half_as_ushort(__float2half_rn(__uint_as_float(va[j])));
+                        const uint16_t y1 = __half_as_ushort(__float2half_rn(__uint_as_float(vb[j])));
+                        asm volatile("st.shared.b16 [%0], %1;" ::"r"(stage + j * kTokBytes), "h"(y0) : "memory");
+                        asm volatile("st.shared.b16 [%0], %1;" ::"r"(stage + (16 + j) * kTokBytes), "h"(y1) : "memory");
+                    }
+                }
+                asm volatile("barrier.sync 1, 128;" ::: "memory");
+                // (a staging tile is written again two chunks later, after a barrier that follows these reads)
+                constexpr uint32_t kVecs = kTokBytes / 16;        // 16-byte words per token
+                const uint32_t src = stage0 + which * (32 * kTokBytes);
+#pragma unroll
+                for (uint32_t i = 0; i < 32 * kVecs / 128; ++i) {
+                    const uint32_t v = et + i * 128, tok = v / kVecs, c = v % kVecs;
+                    if (c0 + tok < tl.ntok && c * 8 < nrows) {
+                        const uint4 d = q_lds128(src + tok * kTokBytes + c * 16);
+                        uint16_t* o = args.out + (size_t)(tl.row0 + c0 + tok) * args.out_stride + first + c * 8;
+                        if (args.out_vec) {
+                            *reinterpret_cast<uint4*>(o) = d;
+                        } else {
+                            const uint32_t w4[4] = {d.x, d.y, d.z, d.w};
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) { o[2 * e] = (uint16_t)(w4[e] & 0xFFFFu); o[2 * e + 1] = (uint16_t)(w4[e] >> 16); }
                         }
                     }
                 }
             }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) {
-                if (plan.both || plan.buf == 0) q_mbar_arrive(bar_acc_empty(0));
-                if (plan.both || plan.buf == 1) q_mbar_arrive(bar_acc_empty(1));
-            }
-            plan.done();
+            if (++buf == 2) { buf = 0; ++uacc; }
         }
     }
     if (fail && lane == 0) atomicCAS(args.error, 0u, fail);
@@ -658,49 +665,117 @@ static tf_status make_x_map(tf_context* ctx, CUtensorMap* map, const void* x, ui
     return TF_OK;
 }
 
-// Packed int4 weights as bytes [experts, rows, k / 2]: box = 64 bytes x 128 rows x 1 expert, 64-byte swizzle
-// (the 16-byte chunks of a row are permuted by (row / 2) % 4, which makes the row-per-lane LDS.128 conflict
+// Packed int4 weights as bytes [experts, rows, k / 2]: box = 128 bytes x (128 / NMAT) rows x 1 expert, 128-byte swizzle
+// (the 16-byte chunks of a row are permuted by row % 8, which makes the row-per-lane LDS.128 conflict
 // free); rows past the matrix and bytes past the row read as zero.
 static tf_status make_w_map(tf_context* ctx, CUtensorMap* map, const void* w, uint32_t rows, uint32_t k, uint64_t experts,
-                            uint64_t expert_stride, const char* name) {
+                            uint64_t expert_stride, uint32_t box_rows, const char* name) {
     EncodeTiledFn fn = encode_tiled_fn();
     TF_REQUIRE(ctx, fn != nullptr, TF_ERR_UNSUPPORTED, "%s: cuTensorMapEncodeTiled is not available in this driver", name);
     const cuuint64_t dims[3] = {k / 2, rows, experts};
     const cuuint64_t strides[2] = {(cuuint64_t)(k / 2), expert_stride};
-    const cuuint32_t box[3] = {(cuuint32_t)(kQmmK / 2), (cuuint32_t)kQmmRows, 1};
+    const cuuint32_t box[3] = {(cuuint32_t)(kQmmRawK / 2), (cuuint32_t)box_rows, 1};
     const cuuint32_t estr[3] = {1, 1, 1};
     const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(w), dims, strides, box, estr,
-                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     TF_REQUIRE(ctx, r == CUDA_SUCCESS, TF_ERR_CUDA, "%s: cuTensorMapEncodeTiled(weights) failed (%d)", name, (int)r);
     return TF_OK;
 }
 
-// W[m]: base of matrix m's packed plane for expert 0 (dense: the matrix itself).
+// Divides the 227 KB of shared memory for K columns. Packed codes first (four stages keep 48 to 64 KB in flight, what an
+// SM's share of the HBM rate needs at its latency), the activation ring takes what the scale planes leave: three slots of
+// 128 tokens at K = 2816. Long rows give up stages, then tokens per tile.
+static bool qmm_plan(uint32_t k, uint32_t nmat, QmmPlan* p) {
+    const uint32_t budget = 227u * 1024u - 1024u;                  // less the alignment slack
+    const uint32_t ng = k / kGroup;
+    p->plane_bytes = ((kQmmRows / nmat) * ng * 2u + 15u) & ~15u;
+    p->sc_bytes = nmat * 2 * p->plane_bytes;
+    p->sc_bufs = 4 * p->sc_bytes <= 48u * 1024u ? 4u : 2u;
+    const uint32_t fixed = p->sc_bufs * p->sc_bytes + kQmmStageBytes + TF_MAX_ROUTER_EXPERTS * 16u + 1024u;
+    const uint32_t slot = kQmmTokMax * kQmmHalfK * 2u;              // 32 KB
+    p->raw_stages = 0;
+    for (uint32_t raw = kQmmRawMax; raw >= 2 && !p->raw_stages; --raw)
+        if (fixed + raw * kQmmRawBytes + 2 * slot <= budget) { p->raw_stages = raw; p->tok_max = kQmmTokMax; }
+    if (!p->raw_stages) {                                          // very long rows: two slots of 64 tokens
+        if (fixed + 2 * kQmmRawBytes + slot > budget) return false;
+        p->raw_stages = 2;
+        p->tok_max = kQmmTokMax / 2;
+    }
+    p->b_bytes = (budget - fixed - p->raw_stages * kQmmRawBytes) & ~2047u;
+    p->off_b = p->raw_stages * kQmmRawBytes;
+    p->off_sc = p->off_b + p->b_bytes;
+    p->off_stage = p->off_sc + p->sc_bufs * p->sc_bytes;
+    p->off_table = p->off_stage + kQmmStageBytes;
+    p->off_bars = p->off_table + TF_MAX_ROUTER_EXPERTS * 16u;
+    p->total = p->off_bars + 1024u + 1024u;
+    return true;
+}
+
+// Tokens per tile of a dense launch: rounds of the grid x the time of a tile, which is the larger of its MMAs (four clocks
+// per token and 128 columns) and its dequantisation (about 330 clocks per 128 columns), plus a fixed part.
+static uint32_t qmm_dense_per_tile(uint32_t tokens, uint32_t wrow_tiles, uint32_t halves, uint32_t tok_max, uint32_t sms) {
+    uint32_t best = 16;
+    uint64_t best_cost = ~0ull;
+    for (uint32_t per = tok_max; per >= 16; per -= 16) {
+        const uint64_t tiles = (uint64_t)wrow_tiles * ((tokens + per - 1) / per);
+        const uint64_t step = 4ull * per > 330 ? 4ull * per : 330;
+        const uint64_t cost = ((tiles + sms - 1) / sms) * (halves * step + 1500);
+        if (cost < best_cost) { best_cost = cost; best = per; }
+    }
+    return best;
+}
+
+// W[m]: base of matrix m's packed plane for expert 0 (dense: the matrix itself); a.S, a.B likewise.
 template <int NMAT, bool NATURAL_K>
 static tf_status launch_qmm(tf_context* ctx, void* stream, QmmArgs& a, const void* x, uint64_t x_rows, uint32_t x_stride,
                             const uint8_t* const* W, uint64_t experts, uint64_t expert_stride, bool dense, const char* name) {
     TF_REQUIRE(ctx, a.k % kGroup == 0 && a.k >= (uint32_t)kGroup, TF_ERR_INVALID_ARGUMENT, "%s: K must be a positive multiple of 64", name);
     TF_REQUIRE(ctx, a.rows % 8 == 0 && a.rows > 0, TF_ERR_INVALID_ARGUMENT, "%s: the weight rows must be a positive multiple of 8", name);
     TF_REQUIRE(ctx, aligned(x, 16) && (x_stride * 2) % 16 == 0, TF_ERR_ALIGNMENT, "%s: activation rows must be 16-byte aligned", name);
-    TF_REQUIRE(ctx, ctx->qmm_groups != nullptr, TF_ERR_OUT_OF_MEMORY, "%s: context scratch missing", name);
-    const uint32_t smem = QmmSmem<NMAT>::total(a.k);
-    TF_REQUIRE(ctx, smem <= 227u * 1024u, TF_ERR_UNSUPPORTED, "%s: K=%u needs %u bytes of shared memory for the scale planes", name, a.k, smem);
-    CUtensorMap xmap, xmap_big, wmap[2];
-    if (tf_status s = make_x_map(ctx, &xmap, x, x_rows, a.k, x_stride, kQmmBoxRows, name)) return s;
-    if (tf_status s = make_x_map(ctx, &xmap_big, x, x_rows, a.k, x_stride, kQmmTokMax, name)) return s;
-    for (int m = 0; m < 2; ++m)
-        if (tf_status s = make_w_map(ctx, &wmap[m], W[m < NMAT ? m : 0], a.rows, a.k, experts, dense ? (uint64_t)a.rows * (a.k / 2) : expert_stride, name)) return s;
-    a.groups = static_cast<QmmGroup*>(ctx->qmm_groups) + (dense ? TF_MAX_ROUTER_EXPERTS + 1 : 0);
-    a.totals = ctx->qmm_totals + (dense ? 2 : 0);
+    TF_REQUIRE(ctx, qmm_plan(a.k, NMAT, &a.plan), TF_ERR_UNSUPPORTED, "%s: K=%u needs more shared memory for the scale planes than there is", name, a.k);
+    constexpr uint32_t kMatRows = kQmmRows / NMAT;
+    // Activation boxes of 16, 32, 64 and 128 rows. A dense launch knows its tiles (full ones and a last one) and encodes only
+    // the boxes that those are made of: an encode is most of a microsecond of host time, and small products are bound by it.
+    uint32_t boxes = 16u | 32u | 64u | 128u;
+    if (dense) {
+        a.dense_per_tile = qmm_dense_per_tile(a.dense_tokens, (a.rows + kMatRows - 1) / kMatRows, (a.k + kQmmHalfK - 1) / kQmmHalfK,
+                                              a.plan.tok_max, (uint32_t)ctx->sm_count);
+        const uint32_t rest = (a.dense_tokens % a.dense_per_tile + 15u) & ~15u;
+        boxes = rest | (a.dense_tokens >= a.dense_per_tile ? a.dense_per_tile : 0u);
+    }
+    CUtensorMap xmap[4], wmap[2];
+    int some = -1;
+    for (int i = 0; i < 4; ++i) {
+        if (!(boxes & (16u << i))) continue;
+        if (tf_status s = make_x_map(ctx, &xmap[i], x, x_rows, a.k, x_stride, 16u << i, name)) return s;
+        some = i;
+    }
+    for (int i = 0; i < 4; ++i)
+        if (!(boxes & (16u << i))) xmap[i] = xmap[some];
+    for (int m = 0; m < NMAT; ++m)
+        if (tf_status s = make_w_map(ctx, &wmap[m], W[m], a.rows, a.k, experts, dense ? (uint64_t)a.rows * (a.k / 2) : expert_stride, kMatRows, name)) return s;
+    if (NMAT == 1) wmap[1] = wmap[0];
+    a.expert_stride = dense ? 0 : expert_stride;
+    a.out_vec = aligned(a.out, 16) && a.out_stride % 8 == 0 ? 1u : 0u;
     a.error = ctx->device_error;
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    qmm_prepare_kernel<<<1, 32, 0, st>>>(a, NMAT, dense ? 1 : 0);
+    // one table for routed launches and one for dense ones, which may run on two streams at once
+    TF_REQUIRE(ctx, ctx->qmm_groups != nullptr, TF_ERR_OUT_OF_MEMORY, "%s: context scratch missing", name);
+    a.groups = static_cast<uint4*>(ctx->qmm_groups) + (dense ? TF_MAX_ROUTER_EXPERTS + 1 : 0);
+    a.totals = reinterpret_cast<uint32_t*>(a.groups + TF_MAX_ROUTER_EXPERTS);
+    launch_pdl(qmm_prepare_kernel, dim3(1), dim3(TF_MAX_ROUTER_EXPERTS), 0, static_cast<cudaStream_t>(stream), a.groups, a.totals,
+               a.route_groups, a.route_counters, a.dense_tokens, a.dense_per_tile, a.plan.tok_max);
     if (tf_status s = check_launch(ctx, "qmm_prepare")) return s;
     auto kern = qmm_tcgen05_kernel<NMAT, NATURAL_K>;
     static DeviceSmemCache configured;
-    if (tf_status s = ensure_dynamic_smem(ctx, kern, configured, smem)) return s;
-    kern<<<ctx->sm_count, kQmmThreads, smem, st>>>(xmap, xmap_big, wmap[0], wmap[1], a);
+    if (tf_status s = ensure_dynamic_smem(ctx, kern, configured, a.plan.total)) return s;
+    uint32_t grid = (uint32_t)ctx->sm_count;
+    if (dense) {
+        const uint64_t tiles = (uint64_t)((a.rows + kMatRows - 1) / kMatRows) * ((a.dense_tokens + a.dense_per_tile - 1) / a.dense_per_tile);
+        if (tiles < grid) grid = (uint32_t)tiles;
+    }
+    launch_pdl(kern, dim3(grid), dim3(kQmmThreads), a.plan.total, static_cast<cudaStream_t>(stream), xmap[0], xmap[1], xmap[2], xmap[3],
+               wmap[0], wmap[1], a);
     return check_launch(ctx, name);
 }
 
@@ -727,17 +802,16 @@ tf_status tf_grouped_moe_tensorcore(tf_context* ctx, void* stream, const void* x
     if (x_rows == 0) return TF_OK;
     const uint8_t* pool = static_cast<const uint8_t*>(pool_layer_base);
     tf::QmmArgs a{};
-    a.pool_base = pool; a.expert_stride = expert_stride;
-    a.s_off[0] = offsets->gate_s_off; a.b_off[0] = offsets->gate_b_off;
-    a.s_off[1] = offsets->up_s_off;   a.b_off[1] = offsets->up_b_off;
+    auto plane = [&](uint32_t off) { return reinterpret_cast<const uint16_t*>(pool + off); };
+    a.S[0] = plane(offsets->gate_s_off); a.B[0] = plane(offsets->gate_b_off);
+    a.S[1] = plane(offsets->up_s_off);   a.B[1] = plane(offsets->up_b_off);
     a.route_groups = routes->groups; a.route_counters = routes->counters;
     a.rows = f; a.k = d; a.out = static_cast<uint16_t*>(acts_scratch); a.out_stride = f; a.round_gate_up = 0;
     const uint8_t* w_gu[2] = {pool + offsets->gate_w_off, pool + offsets->up_w_off};
     if (tf_status s = tf::launch_qmm<2, false>(ctx, stream, a, x_sorted, x_rows, d, w_gu, num_experts, expert_stride, false,
                                                 "tf_grouped_moe_tensorcore(gate/up)")) return s;
     tf::QmmArgs b{};
-    b.pool_base = pool; b.expert_stride = expert_stride;
-    b.s_off[0] = offsets->down_s_off; b.b_off[0] = offsets->down_b_off;
+    b.S[0] = plane(offsets->down_s_off); b.B[0] = plane(offsets->down_b_off);
     b.route_groups = routes->groups; b.route_counters = routes->counters;
     b.rows = d; b.k = f; b.out = static_cast<uint16_t*>(out_rows); b.out_stride = d;
     const uint8_t* w_dn[2] = {pool + offsets->down_w_off, pool + offsets->down_w_off};
@@ -776,8 +850,8 @@ tf_status tf_int4_qmm_with_path(tf_context* ctx, void* stream, const void* weigh
     }
     tf::QmmArgs a{};
     const uint8_t* w[2] = {wp, wp};
-    a.dense_S[0] = reinterpret_cast<const uint16_t*>(sp);
-    a.dense_B[0] = reinterpret_cast<const uint16_t*>(bp);
+    a.S[0] = reinterpret_cast<const uint16_t*>(sp);
+    a.B[0] = reinterpret_cast<const uint16_t*>(bp);
     a.dense_tokens = m; a.rows = n; a.k = k;
     a.out = reinterpret_cast<uint16_t*>(yp); a.out_stride = n;
     tf_status s = tf::launch_qmm<1, true>(ctx, stream, a, xp, m, k, w, 1, 0, true, name);
@@ -812,14 +886,14 @@ tf_status tf_shared_expert_int4_tensorcore(tf_context* ctx, void* stream, const 
         TF_REQUIRE(ctx, tf::aligned(W[i], 16) && tf::aligned(S[i], 16) && tf::aligned(B[i], 16), TF_ERR_ALIGNMENT, "%s: planes must be 16-byte aligned", name);
     }
     tf::QmmArgs a{};
-    a.dense_S[0] = S[0]; a.dense_B[0] = B[0];
-    a.dense_S[1] = S[1]; a.dense_B[1] = B[1];
+    a.S[0] = S[0]; a.B[0] = B[0];
+    a.S[1] = S[1]; a.B[1] = B[1];
     a.dense_tokens = rows; a.rows = fs; a.k = d; a.out = static_cast<uint16_t*>(scratch_act); a.out_stride = fs; a.round_gate_up = 1;
     const uint8_t* w_gu[2] = {W[0], W[1]};
     if (tf_status s = tf::launch_qmm<2, true>(ctx, stream, a, x, rows, x_stride_elements, w_gu, 1, 0, true,
                                                "tf_shared_expert_int4_tensorcore(gate/up)")) return s;
     tf::QmmArgs b{};
-    b.dense_S[0] = S[2]; b.dense_B[0] = B[2];
+    b.S[0] = S[2]; b.B[0] = B[2];
     b.dense_tokens = rows; b.rows = d; b.k = fs; b.out = static_cast<uint16_t*>(y); b.out_stride = y_stride_elements;
     const uint8_t* w_dn[2] = {W[2], W[2]};
     return tf::launch_qmm<1, true>(ctx, stream, b, scratch_act, rows, fs, w_dn, 1, 0, true, "tf_shared_expert_int4_tensorcore(down)");
