@@ -40,10 +40,10 @@ namespace tf {
 constexpr int kQmmTokMax = 128;        // largest N of one MMA: tokens per tile
 constexpr int kQmmRows = 128;          // M of the MMA: weight rows per tile (gate/up: 64 gate rows over 64 up rows)
 constexpr int kQmmRawK = 256;          // columns per packed-code stage: one quantisation group per dequantiser thread
-constexpr int kQmmHalfK = 128;         // columns per operand slot (A in tensor memory, B in shared memory)
+constexpr int kQmmHalfK = 128;         // half of a stage; the unit of the activation ring for tiles of more than 64 tokens
 constexpr uint32_t kQmmRawBytes = kQmmRows * (kQmmRawK / 2);        // 16 KB
 constexpr int kQmmRawMax = 4, kQmmBMax = 12, kQmmScMax = 4;         // ring depths (the launch picks them to fit, see QmmPlan)
-constexpr int kQmmASlots = 4;          // TMEM ring of dequantised 128-column slots, 64 TMEM columns each
+constexpr int kQmmASlots = 2;          // TMEM ring of dequantised stages, 128 TMEM columns each
 constexpr int kQmmFirstDequantWarp = 4, kQmmDequantWarps = 16;      // four threads per weight row
 constexpr int kQmmFirstEpilogueWarp = 20, kQmmEpilogueWarps = 4;
 constexpr int kQmmThreads = (kQmmFirstEpilogueWarp + kQmmEpilogueWarps) * 32;
@@ -138,8 +138,8 @@ __device__ __forceinline__ void tc_commit(uint32_t mbar) {
 // D[tmem] (+)= A[tmem] * B[smem descriptor]
 __device__ __forceinline__ void tc_mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-                 ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
+                 "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+                 ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
 __device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
@@ -325,8 +325,8 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map16, const __grid_con
     auto bar_empty_raw = [&](uint32_t s) { return bars + (4 + s) * 8; };                     // 4: dequant warps
     auto bar_full_b = [&](uint32_t s) { return bars + (8 + s) * 8; };                        // 12: TMA tx
     auto bar_empty_b = [&](uint32_t s) { return bars + (20 + s) * 8; };                      // 12: tcgen05.commit
-    auto bar_full_a = [&](uint32_t s) { return bars + (32 + s) * 8; };                       // 4: the dequant warps of a half
-    auto bar_empty_a = [&](uint32_t s) { return bars + (36 + s) * 8; };                      // 4: tcgen05.commit
+    auto bar_full_a = [&](uint32_t s) { return bars + (32 + s) * 8; };                       // 2: dequant warps
+    auto bar_empty_a = [&](uint32_t s) { return bars + (36 + s) * 8; };                      // 2: tcgen05.commit
     auto bar_full_sc = [&](uint32_t b) { return bars + (40 + b) * 8; };                      // 4: bulk-copy tx
     auto bar_empty_sc = [&](uint32_t b) { return bars + (44 + b) * 8; };                     // 4: dequant warps
     auto bar_acc_full = [&](uint32_t b) { return bars + (48 + b) * 8; };                     // 2: tcgen05.commit
@@ -334,17 +334,18 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map16, const __grid_con
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(base_ptr + plan.off_bars + 52 * 8);   // TMEM base
     uint4* table = reinterpret_cast<uint4*>(base_ptr + plan.off_table);
 
-    const int warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
+    // The shuffle makes the warp index uniform for the compiler: the roles' branches and their operands then stay in uniform
+    // registers, where the MMA and copy instructions want them (the MMA issuer's loop was 10 to 15 % slower without).
+    const int warp = __shfl_sync(kFullMask, (int)(threadIdx.x / kWarp), 0), lane = threadIdx.x % kWarp;
     const uint32_t ng = args.k / kGroup;
     const uint32_t ksteps = (ng + 3) / 4;                              // packed-code stages per tile
-    const uint32_t halves = (ng + 1) / 2;                              // operand slots per tile; the last may hold one group only
     const uint32_t wrow_tiles = (args.rows + kMatRows - 1) / kMatRows;
 
     pdl_launch_dependents();
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < (uint32_t)kQmmRawMax; ++s) { q_mbar_init(bar_full_raw(s), 1); q_mbar_init(bar_empty_raw(s), kQmmDequantWarps); }
         for (uint32_t s = 0; s < (uint32_t)kQmmBMax; ++s) { q_mbar_init(bar_full_b(s), 1); q_mbar_init(bar_empty_b(s), 1); }
-        for (uint32_t s = 0; s < (uint32_t)kQmmASlots; ++s) { q_mbar_init(bar_full_a(s), kQmmDequantWarps / 2); q_mbar_init(bar_empty_a(s), 1); }
+        for (uint32_t s = 0; s < (uint32_t)kQmmASlots; ++s) { q_mbar_init(bar_full_a(s), kQmmDequantWarps); q_mbar_init(bar_empty_a(s), 1); }
         for (uint32_t b = 0; b < (uint32_t)kQmmScMax; ++b) { q_mbar_init(bar_full_sc(b), 1); q_mbar_init(bar_empty_sc(b), kQmmDequantWarps); }
         for (uint32_t b = 0; b < 2; ++b) { q_mbar_init(bar_acc_full(b), 1); q_mbar_init(bar_acc_empty(b), kQmmEpilogueWarps); }
         q_fence_async_smem();
@@ -361,9 +362,12 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map16, const __grid_con
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    // Activation ring: slots of the launch's largest tile, as many as fit.
-    const uint32_t b_half_bytes = n_top * 128;                        // one 64-column block of a slot
-    const uint32_t b_fit = plan.b_bytes / (2 * b_half_bytes);
+    // Activation ring: slots of the launch's largest tile, as many as fit. A slot holds a whole stage's columns when two or
+    // more of those fit beside each other with at most 64 tokens (fewer waits and commits per MMA), otherwise half of them.
+    const uint32_t b_block = n_top * 128;                             // 64 columns of a slot
+    const uint32_t b_halves = n_top <= 64 && plan.b_bytes >= 8 * b_block ? 2u : 1u;
+    const uint32_t b_slot = b_halves * 2 * b_block;
+    const uint32_t b_fit = plan.b_bytes / b_slot;
     const uint32_t b_stages = b_fit < (uint32_t)kQmmBMax ? b_fit : (uint32_t)kQmmBMax;
     const uint32_t a_ring = tmem_base + kQmmAccCols;
 
@@ -396,14 +400,14 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map16, const __grid_con
         for (uint32_t tile = blockIdx.x; tile < total_tiles && !fail; tile += gridDim.x) {
             tl.locate(table, ngroups, wrow_tiles, tile);
             const uint32_t n = tl.n();
-            for (uint32_t hs = 0; hs < halves; ++hs) {
+            for (uint32_t g0 = 0; g0 < ng; g0 += 2 * b_halves) {
                 if (ub > 0 && !q_mbar_wait(bar_empty_b(sb), (ub - 1) & 1)) { fail = kErrQmmTimeout | 7; break; }
                 if (elect_one()) {
-                    const uint32_t blocks = ng - 2 * hs < 2u ? 1u : 2u;
+                    const uint32_t left = ng - g0, blocks = left < 2 * b_halves ? left : 2 * b_halves;
                     q_mbar_expect_tx(bar_full_b(sb), blocks * n * 128);
                     for (uint32_t h = 0; h < blocks; ++h) {
-                        uint32_t dst = base + plan.off_b + (sb * 2 + h) * b_half_bytes;
-                        const int col = (int)(hs * kQmmHalfK + h * 64);
+                        uint32_t dst = base + plan.off_b + sb * b_slot + h * b_block;
+                        const int col = (int)((g0 + h) * kGroup);
                         int row = (int)tl.row0;
                         if (n == 128) {
                             tma_load_2d(dst, &x_map128, col, row, bar_full_b(sb));
@@ -454,23 +458,41 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map16, const __grid_con
             if (uacc > 0 && !q_mbar_wait(bar_acc_empty(buf), (uacc - 1) & 1)) { fail = kErrQmmTimeout | 2; break; }
             tc_fence_after();
             const uint32_t acc = tmem_base + buf * 128;
-            for (uint32_t hs = 0; hs < halves; ++hs) {
+            for (uint32_t ks = 0; ks < ksteps; ++ks) {
                 if (!q_mbar_wait(bar_full_b(sb), ub & 1) || !q_mbar_wait(bar_full_a(sa), ua & 1)) { fail = kErrQmmTimeout | 3; break; }
                 tc_fence_after();
+                const uint32_t a_slot = a_ring + sa * 128;
+                const uint32_t groups = ng - 4 * ks;                  // groups left; those past K are skipped
                 const bool leader = elect_one();
-                const uint64_t b_desc = b_desc0 + (uint64_t)((sb * 2 * b_half_bytes) >> 4);
-                const uint32_t a_slot = a_ring + sa * 64;
-                const bool whole = 2 * hs + 1 < ng;                   // the missing half of an odd last slot is skipped
 #pragma unroll
-                for (int j = 0; j < kQmmHalfK / 16; ++j) {            // 16 columns of K: 8 TMEM columns of A, 32 bytes of B
-                    if ((j < 4 || whole) && leader)
-                        tc_mma_f16_ts(acc, a_slot + j * 8, b_desc + (uint64_t)((j >> 2) * (b_half_bytes >> 4) + (j & 3) * 2), idesc,
-                                      (hs > 0 || j > 0) ? 1u : 0u);
+                for (uint32_t h = 0; h < 2; ++h) {
+                    if (h == 1) {
+                        if (groups <= 2) break;
+                        if (b_halves == 1) {                          // the other half has a slot of its own
+                            if (leader) tc_commit(bar_empty_b(sb));
+                            __syncwarp();
+                            if (++sb == b_stages) { sb = 0; ++ub; }
+                            if (!q_mbar_wait(bar_full_b(sb), ub & 1)) { fail = kErrQmmTimeout | 3; break; }
+                        }
+                    }
+                    if (leader) {                                     // 16 columns of K per MMA: 8 TMEM columns of A, 32 bytes of B
+                        const uint64_t b_desc = b_desc0 + (uint64_t)((sb * b_slot + (b_halves == 2 ? h * 2 * b_block : 0u)) >> 4);
+                        const uint32_t a = a_slot + h * 64;
+                        tc_mma_f16_ts(acc, a, b_desc, idesc, (ks > 0 || h > 0) ? 1u : 0u);
+#pragma unroll
+                        for (int j = 1; j < 4; ++j) tc_mma_f16_ts(acc, a + j * 8, b_desc + (uint64_t)(j * 2), idesc, 1u);
+                        if (groups > 2 * h + 1) {
+                            const uint64_t b_desc2 = b_desc + (uint64_t)(b_block >> 4);
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) tc_mma_f16_ts(acc, a + 32 + j * 8, b_desc2 + (uint64_t)(j * 2), idesc, 1u);
+                        }
+                    }
                 }
+                if (fail) break;
                 if (leader) {
                     tc_commit(bar_empty_a(sa));                       // both slots are free once these MMAs have read them
                     tc_commit(bar_empty_b(sb));
-                    if (hs + 1 == halves) tc_commit(bar_acc_full(buf));
+                    if (ks + 1 == ksteps) tc_commit(bar_acc_full(buf));
                 }
                 __syncwarp();
                 if (++sb == b_stages) { sb = 0; ++ub; }
@@ -482,18 +504,17 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map16, const __grid_con
         // ===================== dequantisers: a thread takes one quantisation group of one weight row per stage =====================
         const uint32_t dw = warp - kQmmFirstDequantWarp;
         const uint32_t q = dw & 3, gc = dw >> 2;                 // TMEM lane quarter; group within the stage
-        const uint32_t half = gc >> 1;
         const uint32_t r = q * kWarp + lane;                     // row within the tile = TMEM lane
         // packed codes of the row: 128 bytes whose 16-byte chunks sit at chunk ^ (row % 8) (128-byte TMA swizzle)
         const uint32_t raw_off0 = r * 128 + (((2 * gc) ^ (r & 7u)) << 4), raw_off1 = r * 128 + (((2 * gc + 1) ^ (r & 7u)) << 4);
         const uint32_t sc_off = base + plan.off_sc + (r / kMatRows) * 2 * plan.plane_bytes + (r % kMatRows) * ng * 2;
-        const uint32_t a_lane = a_ring + ((q * kWarp) << 16) + (gc & 1) * 32;
-        uint32_t sr = 0, ur = 0, sc = 0, uc = 0, slot0 = 0;       // slot0: operand slots of the tiles before this one
-        for (uint32_t tile = blockIdx.x; tile < total_tiles && !fail; tile += gridDim.x, slot0 += halves) {
+        const uint32_t a_lane = a_ring + ((q * kWarp) << 16) + gc * 32;
+        uint32_t sr = 0, ur = 0, sc = 0, uc = 0, sa = 0, ua = 0;
+        for (uint32_t tile = blockIdx.x; tile < total_tiles && !fail; tile += gridDim.x) {
             if (!q_mbar_wait(bar_full_sc(sc), uc & 1)) { fail = kErrQmmTimeout | 8; break; }
             const uint32_t sc_base = sc_off + sc * plan.sc_bytes;
             for (uint32_t ks = 0; ks < ksteps; ++ks) {
-                const uint32_t grp = 4 * ks + gc, hs = 2 * ks + half;
+                const uint32_t grp = 4 * ks + gc;
                 const bool real = grp < ng;                       // a group past K is neither dequantised nor multiplied
                 const float sf = real ? bf16_bits_to_float((uint16_t)q_lds16(sc_base + grp * 2)) : 0.0f;
                 const float bf = real ? bf16_bits_to_float((uint16_t)q_lds16(sc_base + plan.plane_bytes + grp * 2)) : 0.0f;
@@ -518,18 +539,16 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map16, const __grid_con
                 __syncwarp();
                 if (lane == 0) q_mbar_arrive(bar_empty_raw(sr));  // the codes are in registers
                 if (++sr == plan.raw_stages) { sr = 0; ++ur; }
-                if (hs < halves) {
-                    const uint32_t slot = slot0 + hs, sa = slot % kQmmASlots, ua = slot / kQmmASlots;
-                    if (ua > 0 && !q_mbar_wait(bar_empty_a(sa), (ua - 1) & 1)) { fail = kErrQmmTimeout | 5; break; }
-                    tc_fence_after();
-                    if (real) {
-                        tc_st32(a_lane + sa * 64, out);
-                        tc_wait_st();
-                    }
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) q_mbar_arrive(bar_full_a(sa));
+                if (ua > 0 && !q_mbar_wait(bar_empty_a(sa), (ua - 1) & 1)) { fail = kErrQmmTimeout | 5; break; }
+                tc_fence_after();
+                if (real) {
+                    tc_st32(a_lane + sa * 128, out);
+                    tc_wait_st();
                 }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) q_mbar_arrive(bar_full_a(sa));
+                if (++sa == (uint32_t)kQmmASlots) { sa = 0; ++ua; }
             }
             __syncwarp();
             if (lane == 0) q_mbar_arrive(bar_empty_sc(sc));       // done with this tile's scale planes
@@ -574,24 +593,31 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map16, const __grid_con
                 if constexpr (NMAT == 2) {
                     // lanes 0..63 hold gate rows, 64..127 up rows: each side hands half of the tokens to the other
                     const bool gate_side = q < 2;
-                    const uint32_t xrow = xch + mrow * 4;
-#pragma unroll
-                    for (int j = 0; j < 16; ++j)
-                        asm volatile("st.shared.b32 [%0], %1;" ::"r"(xrow + (gate_side ? 16 + j : j) * 256), "r"(gate_side ? vb[j] : va[j]) : "memory");
-                    asm volatile("barrier.sync 1, 128;" ::: "memory");
+                    const uint32_t xrow = xch + mrow * 4, give = xrow + (gate_side ? 16 * 256 : 0), take = xrow + (gate_side ? 0 : 16 * 256);
+                    uint32_t own[16], other[16];
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
-                        const uint32_t tok = gate_side ? j : 16 + j;
-                        uint32_t o;
-                        asm volatile("ld.shared.b32 %0, [%1];" : "=r"(o) : "r"(xrow + tok * 256));
-                        float gt = __uint_as_float(gate_side ? va[j] : o), up = __uint_as_float(gate_side ? o : vb[j]);
+                        own[j] = gate_side ? va[j] : vb[j];
+                        asm volatile("st.shared.b32 [%0], %1;" ::"r"(give + j * 256), "r"(gate_side ? vb[j] : va[j]) : "memory");
+                    }
+                    asm volatile("barrier.sync 1, 128;" ::: "memory");
+                    // all loads, then the arithmetic of all sixteen, then the stores: one value at a time is a chain of
+                    // shared-memory and special-function latencies (340 clocks each), longer than a tile's MMAs
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) asm volatile("ld.shared.b32 %0, [%1];" : "=r"(other[j]) : "r"(take + j * 256));
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                        float gt = __uint_as_float(gate_side ? own[j] : other[j]), up = __uint_as_float(gate_side ? other[j] : own[j]);
                         if (args.round_gate_up) {                 // Kernels/MoE/SharedExpertInt4.swift:62-93
                             gt = __half2float(__float2half_rn(gt));
                             up = __half2float(__float2half_rn(up));
                         }
-                        const uint16_t y = __half_as_ushort(__float2half_rn(gelu_tanh(gt) * up));        // prefill.metal:634-636
-                        asm volatile("st.shared.b16 [%0], %1;" ::"r"(stage + tok * kTokBytes), "h"(y) : "memory");
+                        own[j] = __half_as_ushort(__float2half_rn(gelu_tanh(gt) * up));        // prefill.metal:634-636
                     }
+                    const uint32_t out_tok = stage + (gate_side ? 0 : 16) * kTokBytes;
+#pragma unroll
+                    for (int j = 0; j < 16; ++j)
+                        asm volatile("st.shared.b16 [%0], %1;" ::"r"(out_tok + j * kTokBytes), "h"((uint16_t)own[j]) : "memory");
                 } else {
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
@@ -605,16 +631,22 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map16, const __grid_con
                 // (a staging tile is written again two chunks later, after a barrier that follows these reads)
                 constexpr uint32_t kVecs = kTokBytes / 16;        // 16-byte words per token
                 const uint32_t src = stage0 + which * (32 * kTokBytes);
+                constexpr int kPer = 32 * kVecs / 128;
+                uint4 d[kPer];
 #pragma unroll
-                for (uint32_t i = 0; i < 32 * kVecs / 128; ++i) {
+                for (int i = 0; i < kPer; ++i) {
+                    const uint32_t v = et + i * 128;
+                    d[i] = q_lds128(src + (v / kVecs) * kTokBytes + (v % kVecs) * 16);
+                }
+#pragma unroll
+                for (int i = 0; i < kPer; ++i) {
                     const uint32_t v = et + i * 128, tok = v / kVecs, c = v % kVecs;
                     if (c0 + tok < tl.ntok && c * 8 < nrows) {
-                        const uint4 d = q_lds128(src + tok * kTokBytes + c * 16);
                         uint16_t* o = args.out + (size_t)(tl.row0 + c0 + tok) * args.out_stride + first + c * 8;
                         if (args.out_vec) {
-                            *reinterpret_cast<uint4*>(o) = d;
+                            *reinterpret_cast<uint4*>(o) = d[i];
                         } else {
-                            const uint32_t w4[4] = {d.x, d.y, d.z, d.w};
+                            const uint32_t w4[4] = {d[i].x, d[i].y, d[i].z, d[i].w};
 #pragma unroll
                             for (int e = 0; e < 4; ++e) { o[2 * e] = (uint16_t)(w4[e] & 0xFFFFu); o[2 * e + 1] = (uint16_t)(w4[e] >> 16); }
                         }
