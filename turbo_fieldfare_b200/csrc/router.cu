@@ -50,105 +50,6 @@ __device__ __forceinline__ float router_row_logit(const uint8_t* __restrict__ Wr
     return warp_sum(acc);
 }
 
-// Grouping of a small block's routes inside the router launch (the work of group_routes_kernel for at most
-// kRouterSplitRows rows): the block that finishes the last row sorts the (token, rank) pairs by expert, stably in
-// token-major order, and writes offsets, counts, groups and the 8-token chunk table. A pair's place is its expert's
-// offset plus the number of earlier pairs of that expert, counted on a per-expert bitmap over the pairs.
-struct RouterGroupOut {
-    tf_pair* sorted_pairs;          // nullptr: no grouping
-    uint32_t* per_expert_offsets;
-    uint32_t* per_expert_counts;
-    tf_group* groups;
-    uint32_t* chunk_group;
-    uint32_t* chunk_start;
-    uint32_t* counters;
-};
-
-__host__ __device__ inline size_t router_group_smem_bytes(uint32_t n_pairs, uint32_t num_experts) {
-    const uint32_t nw = (n_pairs + 31) / 32;
-    // mask, hist + offs, expert ids, warp totals (3 x 32), weights
-    return (size_t)num_experts * nw * 4 + (size_t)num_experts * 2 * 4 + (size_t)n_pairs * 4 + 96 * 4 + (size_t)((n_pairs + 1) / 2) * 4;
-}
-
-__device__ void group_routes_in_block(const uint32_t* __restrict__ idx, const uint16_t* __restrict__ w, uint32_t T, uint32_t K,
-                                      uint32_t E, const RouterGroupOut& out, uint8_t* smem) {
-    const uint32_t n = T * K, nw = (n + 31) / 32;
-    uint32_t* mask = reinterpret_cast<uint32_t*>(smem);          // [E][nw]
-    uint32_t* hist = mask + (size_t)E * nw;                      // [E]
-    uint32_t* offs = hist + E;                                   // [E]
-    uint32_t* exs = offs + E;                                    // [n]
-    uint32_t* wtot = exs + n;                                    // [3][32]: per-warp totals of the scan
-    uint16_t* wts = reinterpret_cast<uint16_t*>(wtot + 96);      // [n]
-    const uint32_t lane = threadIdx.x % kWarp, warp = threadIdx.x / kWarp, nwarps = blockDim.x / kWarp;
-    // ids and weights (written by other blocks of this launch) travel while the bitmaps are cleared
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-        uint32_t ex = __ldcg(idx + i);
-        if (ex != 0xFFFFFFFFu && ex >= E) ex = E - 1;            // min(id, E-1): Runtime/Inference/RealForwardRunner.swift:955
-        exs[i] = ex;
-        wts[i] = __ldcg(w + i);
-    }
-    for (uint32_t i = threadIdx.x; i < E * nw + E; i += blockDim.x) mask[i] = 0;      // mask and hist are adjacent
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-        const uint32_t ex = exs[i];
-        if (ex != 0xFFFFFFFFu) {
-            atomicAdd(&hist[ex], 1u);
-            atomicOr(&mask[(size_t)ex * nw + i / 32], 1u << (i % 32));
-        }
-    }
-    __syncthreads();
-    // exclusive scans over the experts (pairs, non-empty groups, chunks): every warp scans 32 experts, the warps'
-    // totals meet in shared memory, and rounds of nwarps * 32 experts carry the running totals.
-    uint32_t off = 0, gi = 0, ch = 0;
-    for (uint32_t base = 0; base < E; base += nwarps * kWarp) {
-        const uint32_t e = base + warp * kWarp + lane;
-        const uint32_t cnt = e < E ? hist[e] : 0u;
-        const uint32_t nch = (cnt + (uint32_t)kChunkTokens - 1) / (uint32_t)kChunkTokens;
-        uint32_t i_off = cnt, i_g = cnt ? 1u : 0u, i_ch = nch;
-#pragma unroll
-        for (int o = 1; o < kWarp; o <<= 1) {
-            const uint32_t a = __shfl_up_sync(kFullMask, i_off, o), b2 = __shfl_up_sync(kFullMask, i_g, o),
-                           c = __shfl_up_sync(kFullMask, i_ch, o);
-            if ((int)lane >= o) { i_off += a; i_g += b2; i_ch += c; }
-        }
-        if (lane == kWarp - 1) { wtot[warp] = i_off; wtot[32 + warp] = i_g; wtot[64 + warp] = i_ch; }
-        __syncthreads();
-        uint32_t p_off = off, p_g = gi, p_ch = ch;
-        for (uint32_t v = 0; v < nwarps; ++v) {
-            const uint32_t a = wtot[v], b2 = wtot[32 + v], c = wtot[64 + v];
-            if (v < warp) { p_off += a; p_g += b2; p_ch += c; }
-            off += a; gi += b2; ch += c;
-        }
-        const uint32_t my_off = p_off + i_off - cnt, my_g = p_g + i_g - (cnt ? 1u : 0u), my_ch = p_ch + i_ch - nch;
-        if (e < E) {
-            offs[e] = my_off;
-            out.per_expert_counts[e] = cnt;
-            out.per_expert_offsets[e] = cnt ? my_off : 0xFFFFFFFFu;
-            if (cnt) {
-                out.groups[my_g] = tf_group{e, my_off, cnt};
-                out.chunk_start[my_g] = my_ch;
-                for (uint32_t j = 0; j < nch; ++j) out.chunk_group[my_ch + j] = my_g;
-            }
-        }
-        __syncthreads();                                          // wtot is reused by the next round; offs is read below
-    }
-    if (threadIdx.x == 0) {
-        out.counters[0] = gi;
-        out.counters[1] = ch;
-        out.counters[2] = n;
-        out.counters[3] = off;
-    }
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-        const uint32_t ex = exs[i];
-        if (ex == 0xFFFFFFFFu) continue;
-        const uint32_t* m = mask + (size_t)ex * nw;
-        uint32_t pos = offs[ex];
-        for (uint32_t q = 0; q < i / 32; ++q) pos += __popc(m[q]);
-        pos += __popc(m[i / 32] & ((1u << (i % 32)) - 1u));
-        out.sorted_pairs[pos] = tf_pair{i / K, ex, i % K, (uint32_t)wts[i]};
-    }
-}
-
 // Few rows (decode): grid (rows, experts/4); the block first copies its four expert rows into
 // shared memory with coalesced loads (the per-lane access pattern of the canonical order would
 // otherwise be a chain of 2-byte global loads); the last block to finish a row (self-resetting
@@ -625,6 +526,7 @@ static int tile_router_rows(uint32_t rows, uint32_t slots) {
 // on demand. Growing allocates, which a stream that is being captured must not do: the caller then takes the
 // one-launch kernel.
 static bool router_scratch(tf_context* ctx, cudaStream_t st, uint32_t rows, uint32_t num_experts) {
+    if (rows <= kRouterFusedGroupRows) return ctx->router_approx_few != nullptr;
     const size_t need = (size_t)rows * num_experts * sizeof(float2);
     if (need <= ctx->router_approx_bytes) return true;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -635,11 +537,21 @@ static bool router_scratch(tf_context* ctx, cudaStream_t st, uint32_t rows, uint
     return true;
 }
 
+static RouterGroupOut router_group_out(const tf_device_routes* routes) {
+    return RouterGroupOut{static_cast<tf_pair*>(routes->sorted_pairs), static_cast<uint32_t*>(routes->per_expert_offsets),
+                          static_cast<uint32_t*>(routes->per_expert_counts), static_cast<tf_group*>(routes->groups),
+                          static_cast<uint32_t*>(routes->chunk_group), static_cast<uint32_t*>(routes->chunk_start),
+                          static_cast<uint32_t*>(routes->counters)};
+}
+
+// routes: the tables of the grouping, when it is wanted; *grouped (may be NULL) tells whether a launch of this call fills
+// them (always for at most kRouterSplitRows rows).
 static tf_status launch_router(tf_context* ctx, void* stream, const uint8_t* W, const uint8_t* S, const uint8_t* B,
                                const uint8_t* hidden, tf_dtype hidden_dtype, const uint8_t* eff, const uint8_t* pes,
                                const float* logit_bias, uint32_t* out_idx, uint8_t* out_w, float* out_logits,
                                uint32_t rows, uint32_t num_experts, uint32_t d, uint32_t top_k, uint32_t stride,
-                               const char* name, const tf_device_routes* routes = nullptr) {
+                               const char* name, const tf_device_routes* routes = nullptr, bool* grouped = nullptr) {
+    if (grouped) *grouped = routes != nullptr && rows <= (uint32_t)kRouterSplitRows;
     TF_REQUIRE(ctx, aligned(S, 2) && aligned(B, 2) && aligned(hidden, 2) && aligned(eff, 2) && aligned(pes, 2) &&
                         aligned(out_w, 2) && aligned(out_idx, 4),
                TF_ERR_ALIGNMENT, "%s: 16-bit planes must be 2-byte aligned, indices 4-byte aligned", name);
@@ -661,10 +573,7 @@ static tf_status launch_router(tf_context* ctx, void* stream, const uint8_t* W, 
         size_t smem_rows = (size_t)R * d * 4 + (size_t)kRowsExpertsPerBlock * d + (size_t)kRowsExpertsPerBlock * (d / kGroup) * 4;
         RouterGroupOut grp{};
         if (routes) {
-            grp = RouterGroupOut{static_cast<tf_pair*>(routes->sorted_pairs), static_cast<uint32_t*>(routes->per_expert_offsets),
-                                 static_cast<uint32_t*>(routes->per_expert_counts), static_cast<tf_group*>(routes->groups),
-                                 static_cast<uint32_t*>(routes->chunk_group), static_cast<uint32_t*>(routes->chunk_start),
-                                 static_cast<uint32_t*>(routes->counters)};
+            grp = router_group_out(routes);
             const size_t need = router_group_smem_bytes(rows * top_k, num_experts);
             if (need > smem_rows) smem_rows = need;
         }
@@ -682,10 +591,7 @@ static tf_status launch_router(tf_context* ctx, void* stream, const uint8_t* W, 
         size_t smem_split = (size_t)d * 4 + (size_t)kSplitExpertsPerBlock * d + (size_t)kSplitExpertsPerBlock * (d / kGroup) * 4;
         RouterGroupOut grp{};
         if (routes) {
-            grp = RouterGroupOut{static_cast<tf_pair*>(routes->sorted_pairs), static_cast<uint32_t*>(routes->per_expert_offsets),
-                                 static_cast<uint32_t*>(routes->per_expert_counts), static_cast<tf_group*>(routes->groups),
-                                 static_cast<uint32_t*>(routes->chunk_group), static_cast<uint32_t*>(routes->chunk_start),
-                                 static_cast<uint32_t*>(routes->counters)};
+            grp = router_group_out(routes);
             const size_t need = router_group_smem_bytes(rows * top_k, num_experts);
             if (need > smem_split) smem_split = need;
         }
@@ -696,23 +602,55 @@ static tf_status launch_router(tf_context* ctx, void* stream, const uint8_t* W, 
         return check_launch(ctx, name);
     } else if (rows >= ctx->router_tensorcore_min_rows && !out_logits && vec16 && d % kApxChunk == 0 && aligned(S, 8) && aligned(B, 8) &&
                num_experts <= TF_MAX_ROUTER_EXPERTS && top_k <= (uint32_t)kWarp && top_k <= num_experts &&
-               router_recheck_smem_bytes(d, num_experts) <= 200 * 1024 && router_scratch(ctx, st, rows, num_experts)) {
+               router_recheck_smem_bytes(d, num_experts, kRecheckWarps) <= 200 * 1024 && router_scratch(ctx, st, rows, num_experts)) {
         // logits on the tensor cores, then the canonical logits of the few experts that can reach the top k
-        auto ka = bf ? router_approx_kernel<true> : router_approx_kernel<false>;
+        float2* approx = static_cast<float2*>(rows <= kRouterFusedGroupRows ? ctx->router_approx_few : ctx->router_approx);
+        const uint32_t sms = (uint32_t)ctx->sm_count;
+        // Few rows: blocks of 8 tokens x 32 experts, all of whose operands are in flight at once, as long as they make at
+        // most four rounds of the SMs (a round takes about 6 us, the 16 x 128 blocks 25 us for any row count below 2400).
+        const size_t smem_few = router_approx_few_smem_bytes(d);
+        const dim3 grid_few((rows + kFewTokens - 1) / kFewTokens, (num_experts + kFewExperts - 1) / kFewExperts);
+        if (smem_few <= 224 * 1024 && grid_few.x * grid_few.y <= 4 * sms) {
+            auto ka = bf ? router_approx_few_kernel<true> : router_approx_few_kernel<false>;
+            static DeviceSmemCache configured_few[2];
+            if (tf_status s = ensure_dynamic_smem(ctx, ka, configured_few[bf ? 1 : 0], smem_few)) return s;
+            launch_pdl(ka, grid_few, dim3(kFewThreads), smem_few, st, W, Sp, Bp, hp, stride, ep, approx, rows, num_experts, d);
+        } else {
+            auto ka = bf ? router_approx_kernel<true> : router_approx_kernel<false>;
+            static DeviceSmemCache configured_approx[2];
+            const size_t smem_a = router_approx_smem_bytes();
+            if (tf_status s = ensure_dynamic_smem(ctx, ka, configured_approx[bf ? 1 : 0], smem_a)) return s;
+            launch_pdl(ka, dim3((rows + kApxTokens - 1) / kApxTokens, (num_experts + kApxExperts - 1) / kApxExperts), dim3(kApxThreads),
+                       smem_a, st, W, Sp, Bp, hp, stride, ep, approx, rows, num_experts, d);
+        }
+        if (tf_status s = check_launch(ctx, name)) return s;
         constexpr int kProductionGroups = 2816 / kGroup;          // the recheck keeps an expert's 44 code words in registers
         const bool fixed = d / kGroup == (uint32_t)kProductionGroups;
-        auto kr = fixed ? (bf ? router_recheck_kernel<true, kProductionGroups> : router_recheck_kernel<false, kProductionGroups>)
-                        : (bf ? router_recheck_kernel<true, 0> : router_recheck_kernel<false, 0>);
-        static DeviceSmemCache configured_approx[2], configured_recheck[4];
-        const size_t smem_a = router_approx_smem_bytes(), smem_r = router_recheck_smem_bytes(d, num_experts);
-        if (tf_status s = ensure_dynamic_smem(ctx, ka, configured_approx[bf ? 1 : 0], smem_a)) return s;
-        if (tf_status s = ensure_dynamic_smem(ctx, kr, configured_recheck[(bf ? 1 : 0) + (fixed ? 2 : 0)], smem_r)) return s;
-        float2* approx = reinterpret_cast<float2*>(ctx->router_approx);
-        launch_pdl(ka, dim3((rows + kApxTokens - 1) / kApxTokens, (num_experts + kApxExperts - 1) / kApxExperts), dim3(kApxThreads),
-                   smem_a, st, W, Sp, Bp, hp, stride, ep, approx, rows, num_experts, d);
-        if (tf_status s = check_launch(ctx, name)) return s;
-        launch_pdl(kr, dim3((rows + kRecheckWarps - 1) / kRecheckWarps), dim3(kRecheckWarps * kWarp), smem_r, st, W, Sp, Bp, hp, stride,
-                   ep, pp, logit_bias, static_cast<const float2*>(approx), out_idx, wp, rows, num_experts, d, top_k);
+        // Warps per token: as many as leave the rows in one round of two blocks per SM. A warp that takes all of a token's
+        // candidates one after the other needs about 30 us however few rows there are.
+        const int which = rows <= 2 * sms ? 3 : rows <= 4 * sms ? 2 : rows <= 8 * sms ? 1 : 0;
+        void (*kr)(const uint8_t*, const uint16_t*, const uint16_t*, const uint16_t*, uint32_t, const uint16_t*, const uint16_t*, const float*,
+                   const float2*, uint32_t*, uint16_t*, unsigned int*, RouterGroupOut, uint32_t, uint32_t, uint32_t, uint32_t);
+#define TF_RECHECK(WPT) kr = fixed ? (bf ? router_recheck_kernel<true, kProductionGroups, WPT> : router_recheck_kernel<false, kProductionGroups, WPT>) \
+                                   : (bf ? router_recheck_kernel<true, 0, WPT> : router_recheck_kernel<false, 0, WPT>)
+        if (which == 3) TF_RECHECK(8);
+        else if (which == 2) TF_RECHECK(4);
+        else if (which == 1) TF_RECHECK(2);
+        else TF_RECHECK(1);
+#undef TF_RECHECK
+        const uint32_t per_block = (uint32_t)kRecheckWarps >> which;
+        size_t smem_r = router_recheck_smem_bytes(d, num_experts, per_block);
+        RouterGroupOut grp{};
+        if (routes) {
+            grp = router_group_out(routes);
+            const size_t need = router_group_smem_bytes(rows * top_k, num_experts);
+            if (need > smem_r) smem_r = need;
+        }
+        static DeviceSmemCache configured_recheck[4][4];
+        if (tf_status s = ensure_dynamic_smem(ctx, kr, configured_recheck[which][(bf ? 1 : 0) + (fixed ? 2 : 0)], smem_r)) return s;
+        launch_pdl(kr, dim3((rows + per_block - 1) / per_block), dim3(kRecheckWarps * kWarp), smem_r, st, W, Sp, Bp, hp, stride,
+                   ep, pp, logit_bias, static_cast<const float2*>(approx), out_idx, wp, ctx->router_tickets, grp, rows, num_experts, d, top_k);
+        if (grouped) *grouped = routes != nullptr;
     } else if (rows >= 256 && a2 && (size_t)kTileRouterRows * (d + num_experts) * 4 <= 100 * 1024) {
         const int R = tile_router_rows(rows, (uint32_t)ctx->sm_count * 2u);
         void (*k)(const uint8_t*, const uint16_t*, const uint16_t*, const uint16_t*, uint32_t, const uint16_t*, const uint16_t*, const float*,
@@ -805,15 +743,6 @@ tf_status tf_router_gemma4_block_grouped(tf_context* ctx, void* stream, const vo
     TF_REQUIRE(ctx, routes && routes->sorted_pairs && routes->per_expert_offsets && routes->per_expert_counts && routes->groups &&
                         routes->chunk_group && routes->chunk_start && routes->counters,
                TF_ERR_INVALID_ARGUMENT, "%s: NULL routes buffer", name);
-    if (query_count > (uint32_t)tf::kRouterSplitRows) {
-        // larger blocks: the router kernels for many rows, then the grouping launch
-        tf_status s = tf_router_gemma4_block(ctx, stream, weights, weights_off, scales, scales_off, biases, biases_off, hidden,
-                                             hidden_off, hidden_dtype, effective_scale, effective_scale_off, per_expert_scale,
-                                             per_expert_scale_off, logit_bias, out_indices, 0, out_weights, 0, nullptr,
-                                             query_count, num_experts, d, top_k, hidden_stride_elements);
-        if (s) return s;
-        return tf_group_routes_device(ctx, stream, out_indices, out_weights, query_count, top_k, num_experts, routes);
-    }
     TF_REQUIRE(ctx, weights && scales && biases && hidden && effective_scale && per_expert_scale && out_indices && out_weights,
                TF_ERR_INVALID_ARGUMENT, "%s: NULL buffer", name);
     TF_REQUIRE(ctx, query_count > 0, TF_ERR_INVALID_ARGUMENT, "%s: queryCount must be positive", name);
@@ -824,12 +753,17 @@ tf_status tf_router_gemma4_block_grouped(tf_context* ctx, void* stream, const vo
     TF_REQUIRE(ctx, d > 0 && d % tf::kGroup == 0 && hidden_stride_elements >= d, TF_ERR_INVALID_ARGUMENT,
                "%s: D must be a multiple of 64 and the stride at least D", name);
     TF_REQUIRE(ctx, hidden_dtype == TF_FP16 || hidden_dtype == TF_BF16, TF_ERR_INVALID_ARGUMENT, "%s: bad hidden dtype", name);
-    return tf::launch_router(ctx, stream, tf::byte_ptr(weights, weights_off), tf::byte_ptr(scales, scales_off),
-                             tf::byte_ptr(biases, biases_off), tf::byte_ptr(hidden, hidden_off), hidden_dtype,
-                             tf::byte_ptr(effective_scale, effective_scale_off),
-                             tf::byte_ptr(per_expert_scale, per_expert_scale_off), logit_bias, out_indices,
-                             static_cast<uint8_t*>(out_weights), nullptr, query_count, num_experts, d, top_k,
-                             hidden_stride_elements, name, routes);
+    // Blocks of a few hundred rows group in the router's last launch too (the block that finishes the last row does it);
+    // larger ones group with launches of their own, which many SMs share.
+    bool grouped = false;
+    tf_status s = tf::launch_router(ctx, stream, tf::byte_ptr(weights, weights_off), tf::byte_ptr(scales, scales_off),
+                                    tf::byte_ptr(biases, biases_off), tf::byte_ptr(hidden, hidden_off), hidden_dtype,
+                                    tf::byte_ptr(effective_scale, effective_scale_off),
+                                    tf::byte_ptr(per_expert_scale, per_expert_scale_off), logit_bias, out_indices,
+                                    static_cast<uint8_t*>(out_weights), nullptr, query_count, num_experts, d, top_k,
+                                    hidden_stride_elements, name, query_count <= tf::kRouterFusedGroupRows ? routes : nullptr, &grouped);
+    if (s || grouped) return s;
+    return tf_group_routes_device(ctx, stream, out_indices, out_weights, query_count, top_k, num_experts, routes);
 }
 
 }  // extern "C"

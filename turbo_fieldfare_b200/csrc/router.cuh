@@ -1,5 +1,5 @@
 // Device functions shared by the router kernels and the single-launch decode step: the canonical logit of an
-// expert row staged in shared memory, and the warp-parallel top-k + softmax.
+// expert row staged in shared memory, the warp-parallel top-k + softmax, and the grouping of a small block's routes.
 #pragma once
 
 #include "tf_common.cuh"
@@ -81,6 +81,105 @@ __device__ __forceinline__ float router_row_logit_smem(const uint8_t* Wrow, cons
         acc = __fmaf_rn(b, __fadd_rn(xv.x, xv.y), acc);
     }
     return warp_sum(acc);
+}
+
+// Grouping of a small block's routes inside the router launch (the work of group_routes_kernel for a few
+// hundred rows): the block that finishes the last row sorts the (token, rank) pairs by expert, stably in
+// token-major order, and writes offsets, counts, groups and the 8-token chunk table. A pair's place is its expert's
+// offset plus the number of earlier pairs of that expert, counted on a per-expert bitmap over the pairs.
+struct RouterGroupOut {
+    tf_pair* sorted_pairs;          // nullptr: no grouping
+    uint32_t* per_expert_offsets;
+    uint32_t* per_expert_counts;
+    tf_group* groups;
+    uint32_t* chunk_group;
+    uint32_t* chunk_start;
+    uint32_t* counters;
+};
+
+__host__ __device__ inline size_t router_group_smem_bytes(uint32_t n_pairs, uint32_t num_experts) {
+    const uint32_t nw = (n_pairs + 31) / 32;
+    // mask, hist + offs, expert ids, warp totals (3 x 32), weights
+    return (size_t)num_experts * nw * 4 + (size_t)num_experts * 2 * 4 + (size_t)n_pairs * 4 + 96 * 4 + (size_t)((n_pairs + 1) / 2) * 4;
+}
+
+__device__ inline void group_routes_in_block(const uint32_t* __restrict__ idx, const uint16_t* __restrict__ w, uint32_t T, uint32_t K,
+                                      uint32_t E, const RouterGroupOut& out, uint8_t* smem) {
+    const uint32_t n = T * K, nw = (n + 31) / 32;
+    uint32_t* mask = reinterpret_cast<uint32_t*>(smem);          // [E][nw]
+    uint32_t* hist = mask + (size_t)E * nw;                      // [E]
+    uint32_t* offs = hist + E;                                   // [E]
+    uint32_t* exs = offs + E;                                    // [n]
+    uint32_t* wtot = exs + n;                                    // [3][32]: per-warp totals of the scan
+    uint16_t* wts = reinterpret_cast<uint16_t*>(wtot + 96);      // [n]
+    const uint32_t lane = threadIdx.x % kWarp, warp = threadIdx.x / kWarp, nwarps = blockDim.x / kWarp;
+    // ids and weights (written by other blocks of this launch) travel while the bitmaps are cleared
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+        uint32_t ex = __ldcg(idx + i);
+        if (ex != 0xFFFFFFFFu && ex >= E) ex = E - 1;            // min(id, E-1): Runtime/Inference/RealForwardRunner.swift:955
+        exs[i] = ex;
+        wts[i] = __ldcg(w + i);
+    }
+    for (uint32_t i = threadIdx.x; i < E * nw + E; i += blockDim.x) mask[i] = 0;      // mask and hist are adjacent
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+        const uint32_t ex = exs[i];
+        if (ex != 0xFFFFFFFFu) {
+            atomicAdd(&hist[ex], 1u);
+            atomicOr(&mask[(size_t)ex * nw + i / 32], 1u << (i % 32));
+        }
+    }
+    __syncthreads();
+    // exclusive scans over the experts (pairs, non-empty groups, chunks): every warp scans 32 experts, the warps'
+    // totals meet in shared memory, and rounds of nwarps * 32 experts carry the running totals.
+    uint32_t off = 0, gi = 0, ch = 0;
+    for (uint32_t base = 0; base < E; base += nwarps * kWarp) {
+        const uint32_t e = base + warp * kWarp + lane;
+        const uint32_t cnt = e < E ? hist[e] : 0u;
+        const uint32_t nch = (cnt + (uint32_t)kChunkTokens - 1) / (uint32_t)kChunkTokens;
+        uint32_t i_off = cnt, i_g = cnt ? 1u : 0u, i_ch = nch;
+#pragma unroll
+        for (int o = 1; o < kWarp; o <<= 1) {
+            const uint32_t a = __shfl_up_sync(kFullMask, i_off, o), b2 = __shfl_up_sync(kFullMask, i_g, o),
+                           c = __shfl_up_sync(kFullMask, i_ch, o);
+            if ((int)lane >= o) { i_off += a; i_g += b2; i_ch += c; }
+        }
+        if (lane == kWarp - 1) { wtot[warp] = i_off; wtot[32 + warp] = i_g; wtot[64 + warp] = i_ch; }
+        __syncthreads();
+        uint32_t p_off = off, p_g = gi, p_ch = ch;
+        for (uint32_t v = 0; v < nwarps; ++v) {
+            const uint32_t a = wtot[v], b2 = wtot[32 + v], c = wtot[64 + v];
+            if (v < warp) { p_off += a; p_g += b2; p_ch += c; }
+            off += a; gi += b2; ch += c;
+        }
+        const uint32_t my_off = p_off + i_off - cnt, my_g = p_g + i_g - (cnt ? 1u : 0u), my_ch = p_ch + i_ch - nch;
+        if (e < E) {
+            offs[e] = my_off;
+            out.per_expert_counts[e] = cnt;
+            out.per_expert_offsets[e] = cnt ? my_off : 0xFFFFFFFFu;
+            if (cnt) {
+                out.groups[my_g] = tf_group{e, my_off, cnt};
+                out.chunk_start[my_g] = my_ch;
+                for (uint32_t j = 0; j < nch; ++j) out.chunk_group[my_ch + j] = my_g;
+            }
+        }
+        __syncthreads();                                          // wtot is reused by the next round; offs is read below
+    }
+    if (threadIdx.x == 0) {
+        out.counters[0] = gi;
+        out.counters[1] = ch;
+        out.counters[2] = n;
+        out.counters[3] = off;
+    }
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+        const uint32_t ex = exs[i];
+        if (ex == 0xFFFFFFFFu) continue;
+        const uint32_t* m = mask + (size_t)ex * nw;
+        uint32_t pos = offs[ex];
+        for (uint32_t q = 0; q < i / 32; ++q) pos += __popc(m[q]);
+        pos += __popc(m[i / 32] & ((1u << (i % 32)) - 1u));
+        out.sorted_pairs[pos] = tf_pair{i / K, ex, i % K, (uint32_t)wts[i]};
+    }
 }
 
 }  // namespace tf

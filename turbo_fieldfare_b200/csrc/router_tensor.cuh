@@ -35,13 +35,13 @@ constexpr int kApxXPitch = kApxChunk * 2 + 16;     // bytes per staged activatio
 constexpr int kApxThreads = 256;
 constexpr float kApxPrescale = 1024.0f;            // activations are split as x * 2^10 = hi + lo
 constexpr float kApxRelError = 1.220703125e-04f;   // 2^-13
-constexpr int kRecheckWarps = 8;                   // tokens per block of router_recheck_kernel
+constexpr int kRecheckWarps = 8;                   // warps per block of router_recheck_kernel
 
 __host__ __device__ inline size_t router_approx_smem_bytes() {
     return 2 * (size_t)kApxExperts * kApxWPitch + 2 * (size_t)kApxTokens * kApxXPitch + 2 * 4 * kApxTokens * sizeof(float);
 }
-__host__ __device__ inline size_t router_recheck_smem_bytes(uint32_t d, uint32_t num_experts) {
-    return (size_t)kRecheckWarps * ((size_t)d + num_experts) * sizeof(float);
+__host__ __device__ inline size_t router_recheck_smem_bytes(uint32_t d, uint32_t num_experts, uint32_t tokens_per_block) {
+    return (size_t)tokens_per_block * ((size_t)d + num_experts) * sizeof(float);
 }
 
 __device__ __forceinline__ void cp_async_16(void* smem_dst, const void* global_src) {
@@ -222,6 +222,137 @@ router_approx_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__
     }
 }
 
+// The same for few rows: a block of 8 tokens x 32 experts holds the whole rows of both operands in shared memory, so one
+// round of loads is on its way at once (the weights before the previous kernel has ended) instead of eleven in a row; warp w
+// multiplies expert tile w % 2 over a quarter of the groups (w / 2), and the quarters are added in shared memory. At 200
+// rows the 16 x 128 blocks made 13 blocks that ran 25 us; the sums differ in order only, within the same error bound.
+constexpr int kFewTokens = 8, kFewExperts = 32, kFewThreads = 256, kFewParts = 4;
+__host__ __device__ inline size_t router_approx_few_smem_bytes(uint32_t d) {
+    const size_t groups = d / kGroup;
+    return (size_t)kFewExperts * (d + 64) + 2 * (size_t)kFewTokens * (2 * d + 16) + 2 * groups * kFewTokens * sizeof(float);
+}
+template <bool X_BF16>
+__global__ void __launch_bounds__(kFewThreads, 1)
+router_approx_few_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S, const uint16_t* __restrict__ B,
+                         const uint16_t* __restrict__ hidden, uint32_t hidden_stride, const uint16_t* __restrict__ eff,
+                         float2* __restrict__ out, uint32_t rows, uint32_t num_experts, uint32_t d) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    const uint32_t w_pitch = d + 64, x_pitch = 2 * d + 16;                 // bank-conflict free, as kApxWPitch and kApxXPitch
+    const uint32_t groups = d / kGroup;
+    uint8_t* Ws = smem;                                                    // [32][w_pitch]
+    uint8_t* Hi = Ws + (size_t)kFewExperts * w_pitch;                      // [8][x_pitch]
+    uint8_t* Lo = Hi + (size_t)kFewTokens * x_pitch;
+    float* XS = reinterpret_cast<float*>(Lo + (size_t)kFewTokens * x_pitch);   // [groups][8]: sum of x * 2^10
+    float* XA = XS + groups * kFewTokens;                                  // of |x * 2^10| (+ the split's absolute part)
+    const int tid = threadIdx.x, warp = tid / kWarp, lane = tid % kWarp, g = lane >> 2, t = lane & 3;
+    const uint32_t tok0 = blockIdx.x * kFewTokens, e0 = blockIdx.y * kFewExperts, last = num_experts - 1;
+    pdl_launch_dependents();
+    const uint32_t segs = d / 16;
+    for (uint32_t row = warp; row < (uint32_t)kFewExperts; row += kFewThreads / kWarp) {        // rows past the end repeat the last expert
+        const uint8_t* src = W + (size_t)min(e0 + row, last) * d;
+        for (uint32_t i = lane; i < segs; i += kWarp) cp_async_16(Ws + (size_t)row * w_pitch + i * 16, src + i * 16);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    pdl_wait();
+    {
+        // a warp stages one token, eight columns per lane and step (rows past the end are zeros)
+        const uint32_t tok = tok0 + warp;
+        const uint16_t* hrow = hidden + (size_t)min(tok, rows - 1) * hidden_stride;
+#pragma unroll 4
+        for (uint32_t c = lane * 8; c < d; c += 8 * kWarp) {               // d is a multiple of 256: whole warps
+            const uint4 ev = *reinterpret_cast<const uint4*>(eff + c);
+            uint4 hv = *reinterpret_cast<const uint4*>(hrow + c);
+            if (tok >= rows) hv = make_uint4(0u, 0u, 0u, 0u);
+            const uint32_t hw[4] = {hv.x, hv.y, hv.z, hv.w}, ew[4] = {ev.x, ev.y, ev.z, ev.w};
+            uint32_t hiw[4], low[4];
+            float sum = 0.0f, asum = 0.0f;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const uint16_t h0 = (uint16_t)(hw[j] & 0xFFFFu), h1 = (uint16_t)(hw[j] >> 16);
+                const float y0 = __fmul_rn(X_BF16 ? bf16_bits_to_float(h0) : f16_bits_to_float(h0), bf16_bits_to_float((uint16_t)(ew[j] & 0xFFFFu))) * kApxPrescale;
+                const float y1 = __fmul_rn(X_BF16 ? bf16_bits_to_float(h1) : f16_bits_to_float(h1), bf16_bits_to_float((uint16_t)(ew[j] >> 16))) * kApxPrescale;
+                const __half2 hh = __floats2half2_rn(y0, y1);
+                const float2 hf = __half22float2(hh);
+                const __half2 ll = __floats2half2_rn(y0 - hf.x, y1 - hf.y);
+                hiw[j] = *reinterpret_cast<const uint32_t*>(&hh);
+                low[j] = *reinterpret_cast<const uint32_t*>(&ll);
+                sum += y0 + y1;
+                asum += fabsf(y0) + fabsf(y1);
+            }
+            *reinterpret_cast<uint4*>(Hi + (size_t)warp * x_pitch + c * 2) = make_uint4(hiw[0], hiw[1], hiw[2], hiw[3]);
+            *reinterpret_cast<uint4*>(Lo + (size_t)warp * x_pitch + c * 2) = make_uint4(low[0], low[1], low[2], low[3]);
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) {
+                sum += __shfl_xor_sync(kFullMask, sum, o);
+                asum += __shfl_xor_sync(kFullMask, asum, o);
+            }
+            if ((lane & 7) == 0) {
+                XS[(c / kGroup) * kFewTokens + warp] = sum;
+                XA[(c / kGroup) * kFewTokens + warp] = asum + 0.015625f;   // 64 x 2^-25 / kApxRelError, rounded up
+            }
+        }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    const int tile = warp & 1, part = warp >> 1;
+    const uint32_t e_lo = min(e0 + tile * 16 + g, last), e_hi = min(e0 + tile * 16 + g + 8, last);
+    const uint32_t per = (groups + kFewParts - 1) / kFewParts, g_begin = part * per, g_end = min(g_begin + per, groups);
+    float acc[4] = {}, mag[4] = {};
+#pragma unroll 2
+    for (uint32_t gi = g_begin; gi < g_end; ++gi) {
+        const uint4 a_lo = *reinterpret_cast<const uint4*>(Ws + (size_t)(tile * 16 + g) * w_pitch + gi * 64 + t * 16);
+        const uint4 a_hi = *reinterpret_cast<const uint4*>(Ws + (size_t)(tile * 16 + g + 8) * w_pitch + gi * 64 + t * 16);
+        const float sl = bf16_bits_to_float(__ldg(S + (size_t)e_lo * groups + gi)), sH = bf16_bits_to_float(__ldg(S + (size_t)e_hi * groups + gi));
+        const float bL = bf16_bits_to_float(__ldg(B + (size_t)e_lo * groups + gi)), bH = bf16_bits_to_float(__ldg(B + (size_t)e_hi * groups + gi));
+        const size_t off = (size_t)g * x_pitch + (size_t)(gi * 64 + t * 16) * 2;
+        const uint4 h0 = *reinterpret_cast<const uint4*>(Hi + off), h1 = *reinterpret_cast<const uint4*>(Hi + off + 16);
+        const uint4 l0 = *reinterpret_cast<const uint4*>(Lo + off), l1 = *reinterpret_cast<const uint4*>(Lo + off + 16);
+        const uint32_t alw[4] = {a_lo.x, a_lo.y, a_lo.z, a_lo.w}, ahw[4] = {a_hi.x, a_hi.y, a_hi.z, a_hi.w};
+        const uint32_t bh[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
+        const uint32_t bl[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
+        float P[4] = {};
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+            const uint32_t a0 = bytes_to_half2(alw[s], 0x5140u), a1 = bytes_to_half2(ahw[s], 0x5140u);
+            const uint32_t a2 = bytes_to_half2(alw[s], 0x7362u), a3 = bytes_to_half2(ahw[s], 0x7362u);
+            mma_f16_f32(P, a0, a1, a2, a3, bh[2 * s], bh[2 * s + 1]);
+            mma_f16_f32(P, a0, a1, a2, a3, bl[2 * s], bl[2 * s + 1]);
+        }
+        const float ml = fmaf(255.0f, fabsf(sl), fabsf(bL)), mh = fmaf(255.0f, fabsf(sH), fabsf(bH));
+        const float2 xs = *reinterpret_cast<const float2*>(XS + gi * kFewTokens + 2 * t);
+        const float2 xa = *reinterpret_cast<const float2*>(XA + gi * kFewTokens + 2 * t);
+        acc[0] = fmaf(sl, P[0], fmaf(bL, xs.x, acc[0]));
+        acc[1] = fmaf(sl, P[1], fmaf(bL, xs.y, acc[1]));
+        acc[2] = fmaf(sH, P[2], fmaf(bH, xs.x, acc[2]));
+        acc[3] = fmaf(sH, P[3], fmaf(bH, xs.y, acc[3]));
+        mag[0] = fmaf(ml, xa.x, mag[0]);
+        mag[1] = fmaf(ml, xa.y, mag[1]);
+        mag[2] = fmaf(mh, xa.x, mag[2]);
+        mag[3] = fmaf(mh, xa.y, mag[3]);
+    }
+    __syncthreads();                                  // every fragment has been read: the activations' space holds the partial sums
+    float4* red = reinterpret_cast<float4*>(Hi);      // [warp][lane] x (acc, mag)
+    red[(warp * kWarp + lane) * 2] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    red[(warp * kWarp + lane) * 2 + 1] = make_float4(mag[0], mag[1], mag[2], mag[3]);
+    __syncthreads();
+    if (part != 0) return;
+#pragma unroll
+    for (int p = 1; p < kFewParts; ++p) {
+        const float4 a = red[((warp + 2 * p) * kWarp + lane) * 2], m = red[((warp + 2 * p) * kWarp + lane) * 2 + 1];
+        acc[0] += a.x; acc[1] += a.y; acc[2] += a.z; acc[3] += a.w;
+        mag[0] += m.x; mag[1] += m.y; mag[2] += m.z; mag[3] += m.w;
+    }
+    const float unscale = 1.0f / kApxPrescale;
+    const uint32_t er_lo = e0 + tile * 16 + g, er_hi = er_lo + 8;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        const uint32_t tok = tok0 + 2 * t + c;
+        if (tok >= rows) continue;
+        if (er_lo < num_experts) out[(size_t)tok * num_experts + er_lo] = make_float2(acc[c] * unscale, mag[c] * unscale);
+        if (er_hi < num_experts) out[(size_t)tok * num_experts + er_hi] = make_float2(acc[2 + c] * unscale, mag[2 + c] * unscale);
+    }
+}
+
 // Canonical logits with the expert's codes, scales and biases read from global memory and the row's scaled activations
 // from shared memory (the arithmetic and order of router_row_logit), kLogitChunk groups at a time: the loads of a chunk
 // are issued together, one chunk ahead of the arithmetic (across experts too); lane i holds the scale and bias of the
@@ -307,36 +438,41 @@ __device__ __forceinline__ float router_logit_all(const LogitOperands<GROUPS>& r
     return warp_sum(acc);
 }
 
-// One warp per token: candidates from the approximate logits and their bounds, canonical logits of the candidates,
-// top-k and softmax as in every other router kernel.
-template <bool X_BF16, int GROUPS>          // GROUPS: d / 64 when known at compile time, 0 for any width
+// WPT warps per token: candidates from the approximate logits and their bounds (every warp of the token finds them), canonical
+// logits of the candidates (dealt out to the warps), top-k and softmax as in every other router kernel (one warp). A
+// canonical logit is one long dependent chain, so with few rows a token's eight or nine must not follow one another: one
+// warp per token took 30 us at 333 rows. With grp.sorted_pairs the block that finishes the last row groups all of them.
+template <bool X_BF16, int GROUPS, int WPT>          // GROUPS: d / 64 when known at compile time, 0 for any width
 __global__ void __launch_bounds__(kRecheckWarps * kWarp, 2)
 router_recheck_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S, const uint16_t* __restrict__ B,
                       const uint16_t* __restrict__ hidden, uint32_t hidden_stride, const uint16_t* __restrict__ eff,
                       const uint16_t* __restrict__ per_expert_scale, const float* __restrict__ logit_bias,
-                      const float2* __restrict__ approx, uint32_t* __restrict__ out_idx, uint16_t* __restrict__ out_w,
+                      const float2* __restrict__ approx, uint32_t* out_idx, uint16_t* out_w, unsigned int* tickets, const RouterGroupOut grp,
                       uint32_t rows, uint32_t num_experts, uint32_t d, uint32_t top_k) {
     extern __shared__ __align__(16) uint8_t smem[];
+    constexpr int kTokens = kRecheckWarps / WPT;                    // tokens per block
     const int warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
-    float* xf = reinterpret_cast<float*>(smem) + (size_t)warp * d;
-    float* scores = reinterpret_cast<float*>(smem) + (size_t)kRecheckWarps * d + (size_t)warp * num_experts;
-    const uint32_t row = blockIdx.x * kRecheckWarps + warp;
+    const int slot = warp / WPT, part = warp % WPT;                 // token within the block, warp within the token
+    float* xf = reinterpret_cast<float*>(smem) + (size_t)slot * d;
+    float* scores = reinterpret_cast<float*>(smem) + (size_t)kTokens * d + (size_t)slot * num_experts;
     const uint32_t groups = d / kGroup;
+    // tokens past the end repeat the last one (the same values are written twice); only the first round counts
+    const uint32_t row = min(blockIdx.x * kTokens + slot, rows - 1);
     pdl_launch_dependents();
     pdl_wait();
-    if (row >= rows) return;                     // warps are independent: no block barrier below
     const uint16_t* hrow = hidden + (size_t)row * hidden_stride;
-    for (uint32_t c0 = lane * 2; c0 < d; c0 += 8 * 2 * kWarp) {          // eight independent pairs of loads at a time
+    for (uint32_t e = part * kWarp + lane; e < num_experts; e += WPT * kWarp) scores[e] = -INFINITY;
+    for (uint32_t c0 = (part * kWarp + lane) * 2; c0 < d; c0 += 8 * 2 * kWarp * WPT) {          // eight independent pairs of loads at a time
         uint32_t hv[8], ev[8];
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
-            const uint32_t c = c0 + u * 2 * kWarp;
+            const uint32_t c = c0 + u * 2 * kWarp * WPT;
             hv[u] = c < d ? *reinterpret_cast<const uint32_t*>(hrow + c) : 0u;
             ev[u] = c < d ? *reinterpret_cast<const uint32_t*>(eff + c) : 0u;
         }
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
-            const uint32_t c = c0 + u * 2 * kWarp;
+            const uint32_t c = c0 + u * 2 * kWarp * WPT;
             const uint16_t h0 = (uint16_t)(hv[u] & 0xFFFFu), h1 = (uint16_t)(hv[u] >> 16);
             const float x0 = __fmul_rn(X_BF16 ? bf16_bits_to_float(h0) : f16_bits_to_float(h0), bf16_bits_to_float((uint16_t)(ev[u] & 0xFFFFu)));
             const float x1 = __fmul_rn(X_BF16 ? bf16_bits_to_float(h1) : f16_bits_to_float(h1), bf16_bits_to_float((uint16_t)(ev[u] >> 16)));
@@ -392,11 +528,18 @@ router_recheck_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict_
         const uint32_t e = lane + j * kWarp;
         const bool cand = e < num_experts && (bad || upper[j] >= lb);
         masks[j] = __ballot_sync(kFullMask, cand);
-        if (e < num_experts) scores[e] = -INFINITY;
     }
-    __syncwarp();
+    if (WPT == 1) __syncwarp(); else __syncthreads();             // the row's activations and the cleared scores
+    // this warp's candidates: every WPT-th one
+    auto next_candidate = [&]() {
+        const uint32_t e = pop_candidate(masks);
+#pragma unroll
+        for (int i = 1; i < WPT; ++i) pop_candidate(masks);
+        return e;
+    };
+    for (int i = 0; i < part; ++i) pop_candidate(masks);
     // (expert, chunk) pairs in one software pipeline: the next pair's loads are issued before the current pair is multiplied
-    uint32_t ld_e = pop_candidate(masks), ld_g = 0u;
+    uint32_t ld_e = next_candidate(), ld_g = 0u;
     if constexpr (GROUPS > 0) {
         // two operand sets used in turns: the next candidate's loads are in flight while the current one is multiplied
         LogitOperands<GROUPS> ra, rb;
@@ -407,11 +550,11 @@ router_recheck_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict_
         uint32_t ea = ld_e;
         if (ea != 0xFFFFFFFFu) router_logit_load_all<GROUPS>(W + (size_t)ea * d, S + (size_t)ea * GROUPS, B + (size_t)ea * GROUPS, lane, ra);
         while (ea != 0xFFFFFFFFu) {
-            const uint32_t eb = pop_candidate(masks);
+            const uint32_t eb = next_candidate();
             if (eb != 0xFFFFFFFFu) router_logit_load_all<GROUPS>(W + (size_t)eb * d, S + (size_t)eb * GROUPS, B + (size_t)eb * GROUPS, lane, rb);
             finish(ea, router_logit_all<GROUPS>(ra, xf, lane));
             if (eb == 0xFFFFFFFFu) break;
-            ea = pop_candidate(masks);
+            ea = next_candidate();
             if (ea != 0xFFFFFFFFu) router_logit_load_all<GROUPS>(W + (size_t)ea * d, S + (size_t)ea * GROUPS, B + (size_t)ea * GROUPS, lane, ra);
             finish(eb, router_logit_all<GROUPS>(rb, xf, lane));
         }
@@ -421,7 +564,7 @@ router_recheck_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict_
         float acc = 0.0f;
         auto advance = [&]() {
             ld_g += kLogitChunk;
-            if (ld_g >= groups) { ld_e = pop_candidate(masks); ld_g = 0u; }
+            if (ld_g >= groups) { ld_e = next_candidate(); ld_g = 0u; }
         };
         // multiplies the chunk in (wc, sbc) after requesting the next one into (wn, sbn); true when it was the last one
         auto step = [&](const uint32_t (&wc)[kLogitChunk], uint32_t sbc, uint32_t (&wn)[kLogitChunk], uint32_t& sbn) -> bool {
@@ -447,8 +590,21 @@ router_recheck_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict_
             if (step(wb, sbb, wa, sba)) break;
         }
     }
-    __syncwarp();
-    warp_select_topk(scores, num_experts, top_k, per_expert_scale, out_idx + (size_t)row * top_k, out_w + (size_t)row * top_k, lane);
+    if (WPT == 1) __syncwarp(); else __syncthreads();
+    if (part == 0)
+        warp_select_topk(scores, num_experts, top_k, per_expert_scale, out_idx + (size_t)row * top_k, out_w + (size_t)row * top_k, lane);
+    if (grp.sorted_pairs == nullptr) return;
+    __shared__ bool is_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        is_last = atomicAdd(&tickets[kRouterSplitRows], 1u) == gridDim.x - 1;
+        if (is_last) tickets[kRouterSplitRows] = 0;            // ready for the next launch on this stream
+    }
+    __syncthreads();
+    if (!is_last) return;
+    __threadfence();
+    group_routes_in_block(out_idx, out_w, rows, top_k, num_experts, grp, smem);
 }
 
 }  // namespace tf
