@@ -485,8 +485,8 @@ static tf_status block_routed(tf_context* ctx, void* stream, const tf_moe_layer*
     // The partial dtype follows the workspace's capacity so that one workspace
     // always runs the same arithmetic whatever the call's token count.
     const int f32 = ws->max_tokens <= kF32PartialTokens ? 1 : 0;
-    return tf_grouped_moe_batched(ctx, stream, x, 0, x_stride_elements, layer->pool_layer_base, layer->expert_stride,
-                                  &layer->offsets, &ws->routes, ws->acts, ws->partials, f32, tokens, d, f, K);
+    return grouped_moe_batched(ctx, stream, x, 0, x_stride_elements, layer->pool_layer_base, layer->expert_stride,
+                               &layer->offsets, &ws->routes, ws->acts, ws->partials, f32, tokens, d, f, K, E);
 }
 
 }  // namespace tf

@@ -52,6 +52,12 @@ tf_status launch_decode_step(tf_context* ctx, void* stream, tf_stack* st, void* 
 tf_status group_routes_strided(tf_context* ctx, void* stream, const uint32_t* indices, uint32_t idx_stride, uint32_t* ids_out,
                                const void* weights_f16, uint32_t query_count, uint32_t top_k, uint32_t num_experts,
                                const tf_device_routes* routes, const char* name, const struct PeerWait* peer_wait);
+// grouped.cu: tf_grouped_moe_batched for a caller that knows the experts' number (it decides the tokens per chunk)
+tf_status grouped_moe_batched(tf_context* ctx, void* stream, const void* hidden, uint64_t hidden_off,
+                              uint32_t hidden_stride_elements, const void* pool_layer_base, uint64_t expert_stride,
+                              const tf_expert_offsets* offsets, const tf_device_routes* routes,
+                              void* acts_scratch, void* route_partials, int partials_f32,
+                              uint32_t query_count, uint32_t d, uint32_t f, uint32_t top_k, uint32_t num_experts);
 // block.cu / ep.cu: tf_ep_experts and tf_ep_combine whose first kernel waits (bounded) for the peers' flags
 tf_status ep_experts_waiting(tf_context* ctx, void* stream, const void* pool_layer_base, uint64_t expert_stride,
                              const tf_expert_offsets* offsets, const void* recv_rows, const uint32_t* recv_expert_ids,

@@ -264,6 +264,12 @@ group_place_kernel(const uint32_t* __restrict__ indices, uint32_t idx_stride, co
 // grouped small-batch expert kernels
 // ---------------------------------------------------------------------------
 
+// Chunks of 16 tokens from this many rows per expert on (times two): an item of 16 takes about 1.4 times one of 8, and with
+// a mean of 6.5 rows a quarter of the experts has more than 8.
+constexpr uint32_t kWideRowsX2 = 13;
+// The shared expert takes them from more than 64 rows on: below, half as many items leave SMs without work (at 11 rows the
+// 30-layer step was 12 % slower with them).
+constexpr uint32_t kWideDenseRows = 64;
 constexpr int kGPW = 4;                 // 64-column groups per compute warp
 constexpr int kWStages = 3;             // ring depth (items) of the tile ring (codes + scales)
 // Narrow single-matrix tiles (the routed down projection: 16 rows x 352 bytes) are a few KB each, so three of them in
@@ -372,8 +378,8 @@ __host__ __device__ inline uint32_t ring_row_stride(uint32_t row_bytes) {
     return row_bytes + ((8 + 32 - words) % 32) * 4;
 }
 
-// Shared-memory layout of a CTA with `cw` compute warps.
-template <int NMAT>
+// Shared-memory layout of a CTA with `cw` compute warps and chunks of 8 NT tokens.
+template <int NMAT, int NT>
 struct KSplitSmem {
     uint32_t cw, ng, row_bytes, stages;
     // Rows whose natural stride would put a half warp's four rows on the same banks get 32 bytes of padding per
@@ -391,34 +397,55 @@ struct KSplitSmem {
     __host__ __device__ uint32_t stage_bytes() const { return NMAT * mat_bytes() + NMAT * 2 * sb_plane_bytes(); } // codes, then scales
     __host__ __device__ uint32_t off_sb_in_stage() const { return NMAT * mat_bytes(); }
     __host__ __device__ uint32_t ring_bytes() const { return stages * stage_bytes(); }
-    __host__ __device__ uint32_t red_stage_bytes() const { return cw * NMAT * 128 * 4; }
+    __host__ __device__ uint32_t red_stage_bytes() const { return cw * NMAT * NT * 128 * 4; }
     __host__ __device__ uint32_t red_bytes() const { return kRedStages * red_stage_bytes(); }
     __host__ __device__ uint32_t bar_count() const { return 2 * stages + 2 * kRedStages; }
     __host__ __device__ uint32_t off_red() const { return ring_bytes(); }
     __host__ __device__ uint32_t off_bar() const { return off_red() + red_bytes(); }
-    __host__ __device__ size_t total() const { return (size_t)off_bar() + (size_t)bar_count() * 8; }
+    __host__ __device__ uint32_t off_chunks() const { return off_bar() + bar_count() * 8; }        // NT = 2: first chunk of every group
+    __host__ __device__ size_t total() const { return (size_t)off_chunks() + (NT > 1 ? (TF_MAX_ROUTER_EXPERTS + 1) * 4 : 0); }
 };
 
 // Where a warp is in its CTA's item sequence and what the chunk resolves to.
 template <int NMAT>
 struct ItemCursor {
     uint32_t chunk, tile;
+    uint32_t group;         // NT = 2: the chunk's group (chunks only move forward)
     MatPlanes pl[NMAT];
     uint32_t ntok, row_base;
 };
 
-template <int NMAT, bool DENSE>
-__device__ __forceinline__ void resolve_chunk(const GroupedArgs& args, ItemCursor<NMAT>& c) {
+// The group of a warp's first chunk; from there on resolve_chunk steps forward.
+__device__ __forceinline__ uint32_t find_group(const uint32_t* chunk_first, uint32_t ngroups, uint32_t chunk) {
+    uint32_t lo = 0, hi = ngroups;                                   // last group with chunk_first <= chunk
+    while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (chunk_first[mid] <= chunk) lo = mid; else hi = mid;
+    }
+    return lo;
+}
+// chunk_first: NT = 2, the groups' first chunks of 16 tokens in shared memory (the global tables hold chunks of 8)
+template <int NMAT, bool DENSE, int NT>
+__device__ __forceinline__ void resolve_chunk(const GroupedArgs& args, ItemCursor<NMAT>& c, const uint32_t* chunk_first) {
+    constexpr uint32_t kTokens = (uint32_t)kChunkTokens * NT;
     if constexpr (DENSE) {
 #pragma unroll
         for (int m = 0; m < NMAT; ++m) c.pl[m] = args.dense[m];
-        c.row_base = c.chunk * kChunkTokens;
+        c.row_base = c.chunk * kTokens;
         const uint32_t left = args.dense_tokens - c.row_base;
-        c.ntok = left < (uint32_t)kChunkTokens ? left : (uint32_t)kChunkTokens;
+        c.ntok = left < kTokens ? left : kTokens;
     } else {
-        const uint32_t gi = args.chunk_group[c.chunk];
+        uint32_t gi, first;
+        if constexpr (NT > 1) {
+            while (chunk_first[c.group + 1] <= c.chunk) ++c.group;
+            gi = c.group;
+            first = chunk_first[gi];
+        } else {
+            gi = args.chunk_group[c.chunk];
+            first = args.chunk_start[gi];
+        }
         const tf_group grp = args.groups[gi];
-        const uint32_t cin = c.chunk - args.chunk_start[gi];
+        const uint32_t cin = c.chunk - first;
         const uint8_t* blob = args.pool_base + (uint64_t)grp.expert * args.expert_stride;
 #pragma unroll
         for (int m = 0; m < NMAT; ++m) {
@@ -426,9 +453,9 @@ __device__ __forceinline__ void resolve_chunk(const GroupedArgs& args, ItemCurso
             c.pl[m].S = reinterpret_cast<const uint16_t*>(blob + args.s_off[m]);
             c.pl[m].B = reinterpret_cast<const uint16_t*>(blob + args.b_off[m]);
         }
-        c.row_base = grp.pair_start + cin * kChunkTokens;
-        const uint32_t left = grp.pair_count - cin * kChunkTokens;
-        c.ntok = left < (uint32_t)kChunkTokens ? left : (uint32_t)kChunkTokens;
+        c.row_base = grp.pair_start + cin * kTokens;
+        const uint32_t left = grp.pair_count - cin * kTokens;
+        c.ntok = left < kTokens ? left : kTokens;
     }
 }
 
@@ -436,7 +463,11 @@ __device__ __forceinline__ float bf16_lo(uint32_t v) { return __uint_as_float(v 
 __device__ __forceinline__ float bf16_hi(uint32_t v) { return __uint_as_float(v & 0xFFFF0000u); }
 // KC > 0 fixes the column count at compile time (the production shapes), so that the shared-memory layout, the
 // warp count and every loop bound fold into constants; KC = 0 reads them from the arguments.
-template <int NMAT, bool DENSE, int OUT_MODE, int KC>
+//
+// NT = 2 takes chunks of 16 tokens: a masked code feeds two MMAs, so the integer instructions that bound the kernel are
+// spent once per 16 tokens and an expert with 9 to 16 tokens is streamed once instead of twice. The groups' first chunks are
+// then counted here, per CTA.
+template <int NMAT, bool DENSE, int OUT_MODE, int KC, int NT>
 __global__ void __launch_bounds__((KC ? (KC / kGroup + kGPW - 1) / kGPW : kMaxComputeWarps) * kWarp + kExtraWarps * kWarp)
 grouped_ksplit_kernel(const GroupedArgs args) {
     extern __shared__ __align__(16) uint8_t smem[];
@@ -446,7 +477,7 @@ grouped_ksplit_kernel(const GroupedArgs args) {
     const uint32_t cw = KC ? (ng + kGPW - 1) / kGPW : blockDim.x / kWarp - kExtraWarps;  // compute warps; then the reducers; the last warp loads
     const uint32_t row_bytes = KC ? (uint32_t)(KC / 2) : args.k / 2;
     constexpr uint32_t kSt = ring_stages<NMAT, KC>();
-    const KSplitSmem<NMAT> lay{cw, ng, row_bytes, kSt};
+    const KSplitSmem<NMAT, NT> lay{cw, ng, row_bytes, kSt};
     const uint32_t smem_base = (uint32_t)__cvta_generic_to_shared(smem);
     const uint32_t red_base = smem_base + lay.off_red();
     const uint32_t bar_base = smem_base + lay.off_bar();
@@ -459,7 +490,33 @@ grouped_ksplit_kernel(const GroupedArgs args) {
     const uint32_t tiles = args.rows / kTileRows;
     pdl_launch_dependents();
     pdl_wait();              // routing metadata and activations come from the kernels before this one
-    const uint32_t total_chunks = DENSE ? (args.dense_tokens + kChunkTokens - 1) / kChunkTokens : args.counters[1];
+    constexpr uint32_t kTokens = (uint32_t)kChunkTokens * NT;
+    uint32_t* chunk_first = reinterpret_cast<uint32_t*>(smem + lay.off_chunks());
+    uint32_t total_chunks;
+    if constexpr (DENSE) {
+        total_chunks = (args.dense_tokens + kTokens - 1) / kTokens;
+    } else if constexpr (NT > 1) {
+        // one warp scans the groups' chunk counts, 32 groups at a time
+        const uint32_t ngroups = args.counters[0];
+        if (warp == 0) {
+            uint32_t run = 0;
+            for (uint32_t base = 0; base < ngroups; base += kWarp) {
+                uint32_t incl = base + lane < ngroups ? (args.groups[base + lane].pair_count + kTokens - 1) / kTokens : 0u;
+#pragma unroll
+                for (int o = 1; o < kWarp; o <<= 1) {
+                    const uint32_t v = __shfl_up_sync(kFullMask, incl, o);
+                    if (lane >= o) incl += v;
+                }
+                if (base + lane < ngroups) chunk_first[base + lane + 1] = run + incl;
+                run += __shfl_sync(kFullMask, incl, kWarp - 1);
+            }
+            if (lane == 0) chunk_first[0] = 0u;
+        }
+        __syncthreads();
+        total_chunks = chunk_first[ngroups];
+    } else {
+        total_chunks = args.counters[1];
+    }
     const uint32_t total_items = total_chunks * tiles;
     // contiguous item range per CTA: consecutive items share the chunk, whose activations stay in registers
     const uint32_t item_begin = (uint32_t)((uint64_t)total_items * blockIdx.x / gridDim.x);
@@ -478,7 +535,7 @@ grouped_ksplit_kernel(const GroupedArgs args) {
         if (++c.tile == tiles) {
             c.tile = 0;
             ++c.chunk;
-            if (c.chunk < total_chunks) resolve_chunk<NMAT, DENSE>(args, c);
+            if (c.chunk < total_chunks) resolve_chunk<NMAT, DENSE, NT>(args, c, chunk_first);
         }
     };
 
@@ -499,15 +556,16 @@ grouped_ksplit_kernel(const GroupedArgs args) {
         ItemCursor<NMAT> cur;
         cur.chunk = item_begin / tiles;
         cur.tile = item_begin % tiles;
-        resolve_chunk<NMAT, DENSE>(args, cur);
+        cur.group = !DENSE && NT > 1 ? find_group(chunk_first, args.counters[0], cur.chunk) : 0u;
+        resolve_chunk<NMAT, DENSE, NT>(args, cur, chunk_first);
 
         // Four registers that stay zero: the accumulator input of every group's first MMA (a literal zero makes the
         // compiler clear four fresh registers per MMA).
         float zc[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) asm volatile("mov.f32 %0, 0f00000000;" : "=f"(zc[j]));
-        uint2 xb[kGPW][4];          // B fragments of token g: [group][MMA j] = {b0, b1}
-        float2 xsum[kGPW];          // fp32 sums of the 64 activations of the group for tokens 2t and 2t + 1
+        uint2 xb[NT][kGPW][4];      // B fragments of token 8 n + g: [group][MMA j] = {b0, b1}
+        float2 xsum[NT][kGPW];      // fp32 sums of the 64 activations of the group for tokens 8 n + 2t and 8 n + 2t + 1
         uint32_t loaded_chunk = 0xFFFFFFFFu;
         uint32_t fail = 0;
 
@@ -520,10 +578,12 @@ grouped_ksplit_kernel(const GroupedArgs args) {
                 // odd columns are pre-scaled by 1/16 because their codes sit four mantissa bits higher.
                 loaded_chunk = cur.chunk;
 #pragma unroll
+                for (int n = 0; n < NT; ++n)
+#pragma unroll
                 for (int i = 0; i < kGPW; ++i) {
                     uint32_t r[8];
-                    if ((uint32_t)i < ngw && (uint32_t)g < cur.ntok) {
-                        const uint32_t rr = (DENSE || NMAT == 1) ? cur.row_base + g : args.sorted_pairs[cur.row_base + g].token;
+                    if ((uint32_t)i < ngw && (uint32_t)(n * 8 + g) < cur.ntok) {
+                        const uint32_t rr = (DENSE || NMAT == 1) ? cur.row_base + n * 8 + g : args.sorted_pairs[cur.row_base + n * 8 + g].token;
                         const uint4* p = reinterpret_cast<const uint4*>(args.x + (size_t)rr * args.x_stride + (g0 + i) * kGroup + t * 16);
                         const uint4 lo = __ldg(p), hi = __ldg(p + 1);
                         r[0] = lo.x; r[1] = lo.y; r[2] = lo.z; r[3] = lo.w;
@@ -543,12 +603,12 @@ grouped_ksplit_kernel(const GroupedArgs args) {
                     // The codes enter the MMA as q * 2^-24, so the whole row sum is carried at 2^-24 of its value (the group
                     // sums are scaled to match here, once per chunk) and multiplied back once per item: powers of two, exact.
                     sum *= 5.9604644775390625e-08f;
-                    xsum[i] = make_float2(__shfl_sync(kFullMask, sum, 8 * t), __shfl_sync(kFullMask, sum, 8 * t + 4));
+                    xsum[n][i] = make_float2(__shfl_sync(kFullMask, sum, 8 * t), __shfl_sync(kFullMask, sum, 8 * t + 4));
 #pragma unroll
                     for (int h2 = 0; h2 < 2; ++h2) {
                         const int o = 4 * h2;
-                        xb[i][2 * h2] = make_uint2(prmt(r[o], r[o + 2], 0x5410), prmt(r[o + 1], r[o + 3], 0x5410));
-                        xb[i][2 * h2 + 1] = make_uint2(hmul2_sixteenth(prmt(r[o], r[o + 2], 0x7632)),
+                        xb[n][i][2 * h2] = make_uint2(prmt(r[o], r[o + 2], 0x5410), prmt(r[o + 1], r[o + 3], 0x5410));
+                        xb[n][i][2 * h2 + 1] = make_uint2(hmul2_sixteenth(prmt(r[o], r[o + 2], 0x7632)),
                                                        hmul2_sixteenth(prmt(r[o + 1], r[o + 3], 0x7632)));
                     }
                 }
@@ -557,6 +617,11 @@ grouped_ksplit_kernel(const GroupedArgs args) {
 
             const uint32_t ring_item = smem_base + st * lay.stage_bytes() + lane_code_off;
             const uint32_t sb_item = smem_base + st * lay.stage_bytes() + lay.off_sb_in_stage();
+            // partial sums for the reducer: buffer li % kRedStages, 512 bytes per (warp, matrix, 8 tokens)
+            const uint32_t r = li % kRedStages, ruse = li / kRedStages;
+            const uint32_t red_w = red_base + r * lay.red_stage_bytes() + (warp * NMAT * NT) * 512 + (g * 8 + 2 * t) * 4;
+            if constexpr (NT == 1) {
+            float y[NMAT][4];
             // All codes of the item first, then the MMAs interleaved over the (matrix, group) pairs: the four
             // MMAs of one group form a dependent chain through its accumulator, so consecutive instructions
             // always belong to different chains and the tensor pipe stays full.
@@ -578,30 +643,29 @@ grouped_ksplit_kernel(const GroupedArgs args) {
 #pragma unroll
                 for (int i = 0; i < kGPW; ++i)
                     mma16816_first(c[m][i], wa[m][i].x & 0x000F000Fu, wb[m][i].x & 0x000F000Fu,
-                                   (wa[m][i].x >> 8) & 0x000F000Fu, (wb[m][i].x >> 8) & 0x000F000Fu, xb[i][0], zc);
+                                   (wa[m][i].x >> 8) & 0x000F000Fu, (wb[m][i].x >> 8) & 0x000F000Fu, xb[0][i][0], zc);
             }
 #pragma unroll
             for (int m = 0; m < NMAT; ++m) {
 #pragma unroll
                 for (int i = 0; i < kGPW; ++i)
                     mma16816_acc(c[m][i], wa[m][i].x & 0x00F000F0u, wb[m][i].x & 0x00F000F0u,
-                                 (wa[m][i].x >> 8) & 0x00F000F0u, (wb[m][i].x >> 8) & 0x00F000F0u, xb[i][1]);
+                                 (wa[m][i].x >> 8) & 0x00F000F0u, (wb[m][i].x >> 8) & 0x00F000F0u, xb[0][i][1]);
             }
 #pragma unroll
             for (int m = 0; m < NMAT; ++m) {
 #pragma unroll
                 for (int i = 0; i < kGPW; ++i)
                     mma16816_acc(c[m][i], wa[m][i].y & 0x000F000Fu, wb[m][i].y & 0x000F000Fu,
-                                 (wa[m][i].y >> 8) & 0x000F000Fu, (wb[m][i].y >> 8) & 0x000F000Fu, xb[i][2]);
+                                 (wa[m][i].y >> 8) & 0x000F000Fu, (wb[m][i].y >> 8) & 0x000F000Fu, xb[0][i][2]);
             }
 #pragma unroll
             for (int m = 0; m < NMAT; ++m) {
 #pragma unroll
                 for (int i = 0; i < kGPW; ++i)
                     mma16816_acc(c[m][i], wa[m][i].y & 0x00F000F0u, wb[m][i].y & 0x00F000F0u,
-                                 (wa[m][i].y >> 8) & 0x00F000F0u, (wb[m][i].y >> 8) & 0x00F000F0u, xb[i][3]);
+                                 (wa[m][i].y >> 8) & 0x00F000F0u, (wb[m][i].y >> 8) & 0x00F000F0u, xb[0][i][3]);
             }
-            float y[NMAT][4];
 #pragma unroll
             for (int m = 0; m < NMAT; ++m) {
                 const uint32_t sm_s = sb_item + (m * 2) * lay.sb_plane_bytes(), sm_b = sm_s + lay.sb_plane_bytes();
@@ -631,10 +695,10 @@ grouped_ksplit_kernel(const GroupedArgs args) {
 #pragma unroll
                 for (int i = 0; i < kGPW; ++i) {
                     // c0, c1: weight row g, tokens 2t, 2t+1; c2, c3: weight row g + 8
-                    acc[0] = fmaf(sf[0][i], c[m][i][0], fmaf(bf[0][i], xsum[i].x, acc[0]));
-                    acc[1] = fmaf(sf[0][i], c[m][i][1], fmaf(bf[0][i], xsum[i].y, acc[1]));
-                    acc[2] = fmaf(sf[1][i], c[m][i][2], fmaf(bf[1][i], xsum[i].x, acc[2]));
-                    acc[3] = fmaf(sf[1][i], c[m][i][3], fmaf(bf[1][i], xsum[i].y, acc[3]));
+                    acc[0] = fmaf(sf[0][i], c[m][i][0], fmaf(bf[0][i], xsum[0][i].x, acc[0]));
+                    acc[1] = fmaf(sf[0][i], c[m][i][1], fmaf(bf[0][i], xsum[0][i].y, acc[1]));
+                    acc[2] = fmaf(sf[1][i], c[m][i][2], fmaf(bf[1][i], xsum[0][i].x, acc[2]));
+                    acc[3] = fmaf(sf[1][i], c[m][i][3], fmaf(bf[1][i], xsum[0][i].y, acc[3]));
                 }
 #pragma unroll
                 for (int j = 0; j < 4; ++j) y[m][j] = acc[j] * 16777216.0f;
@@ -642,15 +706,80 @@ grouped_ksplit_kernel(const GroupedArgs args) {
             // this warp is done with the stage (codes and scales are in registers or consumed)
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_empty(st));
-            // hand the partial sums to the reducer
-            const uint32_t r = li % kRedStages, ruse = li / kRedStages;
             if (!mbar_wait(bar_red_free(r), (ruse & 1) ^ 1)) { fail = kErrTimeoutRedFree; break; }
-
-            const uint32_t red_w = red_base + r * lay.red_stage_bytes() + (warp * NMAT) * 512 + (g * 8 + 2 * t) * 4;
 #pragma unroll
             for (int m = 0; m < NMAT; ++m) {
                 sts_f32x2(red_w + m * 512, y[m][0], y[m][1]);
                 sts_f32x2(red_w + m * 512 + 256, y[m][2], y[m][3]);      // weight row g + 8: index (g + 8) * 8 + 2t
+            }
+            } else {
+            // the reducer's buffer is claimed first, so that a matrix's sums leave the registers before the next matrix begins
+            if (!mbar_wait(bar_red_free(r), (ruse & 1) ^ 1)) { fail = kErrTimeoutRedFree; break; }
+#pragma unroll
+            for (int m = 0; m < NMAT; ++m) {
+                const uint32_t sm_s = sb_item + (m * 2) * lay.sb_plane_bytes(), sm_b = sm_s + lay.sb_plane_bytes();
+                uint2 vs0, vs1, vb0, vb1;                 // scale and bias words of rows g and g + 8 (ng a multiple of four)
+                if (sb_vec) { vs0 = lds64(sm_s + sb_row0); vs1 = lds64(sm_s + sb_row1); vb0 = lds64(sm_b + sb_row0); vb1 = lds64(sm_b + sb_row1); }
+                float acc[NT][4];
+#pragma unroll
+                for (int n = 0; n < NT; ++n)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) acc[n][j] = 0.0f;
+                // two groups at a time: 2 NT independent MMA chains, and half of the accumulators alive (the B fragments of 16
+                // tokens take 64 registers; 144 is what the CTA's 14 warps leave a thread)
+#pragma unroll
+                for (int h = 0; h < kGPW; h += 2) {
+                    float c[NT][2][4];
+                    uint2 wa[2], wb[2];
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        wa[i] = lds64(ring_item + m * lay.mat_bytes() + (h + i) * 32);
+                        wb[i] = lds64(ring_item + m * lay.mat_bytes() + row8_off + (h + i) * 32);
+                    }
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+#pragma unroll
+                        for (int i = 0; i < 2; ++i) {
+                            const uint32_t mask = (j & 1) ? 0x00F000F0u : 0x000F000Fu;
+                            const uint32_t wx = j < 2 ? wa[i].x : wa[i].y, wy = j < 2 ? wb[i].x : wb[i].y;
+                            const uint32_t a0 = wx & mask, a1 = wy & mask, a2 = (wx >> 8) & mask, a3 = (wy >> 8) & mask;
+#pragma unroll
+                            for (int n = 0; n < NT; ++n) {
+                                if (j == 0) mma16816_first(c[n][i], a0, a1, a2, a3, xb[n][h + i][0], zc);
+                                else mma16816_acc(c[n][i], a0, a1, a2, a3, xb[n][h + i][j]);
+                            }
+                        }
+                    }
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        float s0, s1, b0, b1;
+                        if (sb_vec) {
+                            const uint32_t ws0 = h ? vs0.y : vs0.x, ws1 = h ? vs1.y : vs1.x, wb0 = h ? vb0.y : vb0.x, wb1 = h ? vb1.y : vb1.x;
+                            s0 = i ? bf16_hi(ws0) : bf16_lo(ws0); s1 = i ? bf16_hi(ws1) : bf16_lo(ws1);
+                            b0 = i ? bf16_hi(wb0) : bf16_lo(wb0); b1 = i ? bf16_hi(wb1) : bf16_lo(wb1);
+                        } else {
+                            const bool ok = (uint32_t)(h + i) < ngw;             // past this warp's range: as in the form above
+                            s0 = ok ? bf16_lo(lds16(sm_s + sb_row0 + (h + i) * 2)) : 0.0f; s1 = ok ? bf16_lo(lds16(sm_s + sb_row1 + (h + i) * 2)) : 0.0f;
+                            b0 = ok ? bf16_lo(lds16(sm_b + sb_row0 + (h + i) * 2)) : 0.0f; b1 = ok ? bf16_lo(lds16(sm_b + sb_row1 + (h + i) * 2)) : 0.0f;
+                        }
+#pragma unroll
+                        for (int n = 0; n < NT; ++n) {
+                            // c0, c1: weight row g, tokens 8 n + 2t, 2t + 1; c2, c3: weight row g + 8
+                            acc[n][0] = fmaf(s0, c[n][i][0], fmaf(b0, xsum[n][h + i].x, acc[n][0]));
+                            acc[n][1] = fmaf(s0, c[n][i][1], fmaf(b0, xsum[n][h + i].y, acc[n][1]));
+                            acc[n][2] = fmaf(s1, c[n][i][2], fmaf(b1, xsum[n][h + i].x, acc[n][2]));
+                            acc[n][3] = fmaf(s1, c[n][i][3], fmaf(b1, xsum[n][h + i].y, acc[n][3]));
+                        }
+                    }
+                }
+#pragma unroll
+                for (int n = 0; n < NT; ++n) {
+                    sts_f32x2(red_w + (m * NT + n) * 512, acc[n][0] * 16777216.0f, acc[n][1] * 16777216.0f);
+                    sts_f32x2(red_w + (m * NT + n) * 512 + 256, acc[n][2] * 16777216.0f, acc[n][3] * 16777216.0f);
+                }
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_empty(st));               // this warp is done with the stage
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_part_full(r));
@@ -662,7 +791,8 @@ grouped_ksplit_kernel(const GroupedArgs args) {
         ItemCursor<NMAT> iss;
         iss.chunk = item_begin / tiles;
         iss.tile = item_begin % tiles;
-        resolve_chunk<NMAT, DENSE>(args, iss);
+        iss.group = !DENSE && NT > 1 ? find_group(chunk_first, args.counters[0], iss.chunk) : 0u;
+        resolve_chunk<NMAT, DENSE, NT>(args, iss, chunk_first);
         const uint32_t plane_bytes = lay.sb_plane_bytes();
         const uint32_t rpc = lay.rows_per_copy();                    // 16: the rows of a tile land as one copy
         const uint32_t tx_bytes = NMAT * kTileRows * row_bytes + NMAT * 2 * plane_bytes;
@@ -706,71 +836,80 @@ grouped_ksplit_kernel(const GroupedArgs args) {
         ItemCursor<NMAT> cur;
         cur.chunk = item_begin / tiles;
         cur.tile = item_begin % tiles;
-        resolve_chunk<NMAT, DENSE>(args, cur);
+        cur.group = !DENSE && NT > 1 ? find_group(chunk_first, args.counters[0], cur.chunk) : 0u;
+        resolve_chunk<NMAT, DENSE, NT>(args, cur, chunk_first);
         if (q < n_items) advance_by(cur, q);
         uint32_t fail = 0;
         const uint32_t row = lay.mma_row(lane >> 1), tok4 = (lane & 1) * 4;      // this lane sums one weight row (MMA row lane / 2) for 4 consecutive tokens
         const uint32_t red_q = red_base + q * lay.red_stage_bytes() + lane * 16;
         uint32_t pair_chunk = 0xFFFFFFFFu;
-        uint32_t pair_base[4] = {0u, 0u, 0u, 0u};                   // (token * top_k + rank) of this lane's 4 tokens
+        uint32_t pair_base[NT][4] = {};                             // (token * top_k + rank) of this lane's 4 tokens per 8
         for (uint32_t li = q; li < n_items; li += kReducers) {
             const uint32_t ruse = li / kRedStages;
             if (OUT_MODE == kOutPartialF16 || OUT_MODE == kOutPartialF32) {
                 if (cur.chunk != pair_chunk) {       // the pair of a token is the same for every tile of the chunk
                     pair_chunk = cur.chunk;
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        if (tok4 + j < cur.ntok) {
-                            const tf_pair pr = args.sorted_pairs[cur.row_base + tok4 + j];
-                            pair_base[j] = pr.token * args.top_k + pr.rank;
+                    for (int n = 0; n < NT; ++n) {
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            if (n * 8 + tok4 + j < cur.ntok) {
+                                const tf_pair pr = args.sorted_pairs[cur.row_base + n * 8 + tok4 + j];
+                                pair_base[n][j] = pr.token * args.top_k + pr.rank;
+                            }
                         }
                     }
                 }
             }
             if (!mbar_wait(bar_part_full(q), ruse & 1)) { fail = kErrTimeoutPartials; break; }
-            float4 acc[NMAT];
-#pragma unroll
-            for (int m = 0; m < NMAT; ++m) {
-                // independent loads first, then the sum in warp order (deterministic)
-                float4 v[kMaxComputeWarps];
-#pragma unroll
-                for (int w2 = 0; w2 < kMaxComputeWarps; ++w2)
-                    v[w2] = (uint32_t)w2 < cw ? lds_f32x4(red_q + (w2 * NMAT + m) * 512) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                acc[m] = v[0];
-#pragma unroll
-                for (int w2 = 1; w2 < kMaxComputeWarps; ++w2) {
-                    if ((uint32_t)w2 < cw) { acc[m].x += v[w2].x; acc[m].y += v[w2].y; acc[m].z += v[w2].z; acc[m].w += v[w2].w; }
-                }
-            }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar_red_free(q));
             const uint32_t out_row = cur.tile * kTileRows + row;
-            const float o0[4] = {acc[0].x, acc[0].y, acc[0].z, acc[0].w};
-            const float o1[4] = {acc[NMAT - 1].x, acc[NMAT - 1].y, acc[NMAT - 1].z, acc[NMAT - 1].w};
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const uint32_t tok = tok4 + j;
-                if (tok < cur.ntok) {
-                    if constexpr (OUT_MODE == kOutActs) {
-                        float gt = o0[j], up = o1[j];
-                        if constexpr (DENSE) {
-                            // shared expert: gate and up are stored as fp16 before the activation
-                            // (Kernels/MoE/SharedExpertInt4.swift:62-93; Metal/Primitives/utility.metal:15-17)
-                            gt = __half2float(__float2half_rn(gt));
-                            up = __half2float(__float2half_rn(up));
+            for (int n = 0; n < NT; ++n) {
+                float4 acc[NMAT];
+#pragma unroll
+                for (int m = 0; m < NMAT; ++m) {
+                    // independent loads first, then the sum in warp order (deterministic)
+                    float4 v[kMaxComputeWarps];
+#pragma unroll
+                    for (int w2 = 0; w2 < kMaxComputeWarps; ++w2)
+                        v[w2] = (uint32_t)w2 < cw ? lds_f32x4(red_q + ((w2 * NMAT + m) * NT + n) * 512) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    acc[m] = v[0];
+#pragma unroll
+                    for (int w2 = 1; w2 < kMaxComputeWarps; ++w2) {
+                        if ((uint32_t)w2 < cw) { acc[m].x += v[w2].x; acc[m].y += v[w2].y; acc[m].z += v[w2].z; acc[m].w += v[w2].w; }
+                    }
+                }
+                if (n == NT - 1) {
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar_red_free(q));
+                }
+                const float o0[4] = {acc[0].x, acc[0].y, acc[0].z, acc[0].w};
+                const float o1[4] = {acc[NMAT - 1].x, acc[NMAT - 1].y, acc[NMAT - 1].z, acc[NMAT - 1].w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const uint32_t tok = n * 8 + tok4 + j;
+                    if (tok < cur.ntok) {
+                        if constexpr (OUT_MODE == kOutActs) {
+                            float gt = o0[j], up = o1[j];
+                            if constexpr (DENSE) {
+                                // shared expert: gate and up are stored as fp16 before the activation
+                                // (Kernels/MoE/SharedExpertInt4.swift:62-93; Metal/Primitives/utility.metal:15-17)
+                                gt = __half2float(__float2half_rn(gt));
+                                up = __half2float(__float2half_rn(up));
+                            }
+                            // routed: act = half(gelu_tanh(gate) * up), gate and up in fp32 (prefill.metal:634-636; moe.metal:368)
+                            static_cast<uint16_t*>(args.out)[(size_t)(cur.row_base + tok) * args.out_stride + out_row] =
+                                __half_as_ushort(__float2half_rn(gelu_tanh(gt) * up));
+                        } else if constexpr (OUT_MODE == kOutDenseF16) {
+                            static_cast<uint16_t*>(args.out)[(size_t)(cur.row_base + tok) * args.out_stride + out_row] =
+                                __half_as_ushort(__float2half_rn(o0[j]));
+                        } else {
+                            const size_t idx = (size_t)pair_base[n][j] * args.out_stride + out_row;
+                            if constexpr (OUT_MODE == kOutPartialF16)       // prefill.metal:666-669
+                                static_cast<uint16_t*>(args.out)[idx] = __half_as_ushort(__float2half_rn(o0[j]));
+                            else
+                                static_cast<float*>(args.out)[idx] = o0[j];
                         }
-                        // routed: act = half(gelu_tanh(gate) * up), gate and up in fp32 (prefill.metal:634-636; moe.metal:368)
-                        static_cast<uint16_t*>(args.out)[(size_t)(cur.row_base + tok) * args.out_stride + out_row] =
-                            __half_as_ushort(__float2half_rn(gelu_tanh(gt) * up));
-                    } else if constexpr (OUT_MODE == kOutDenseF16) {
-                        static_cast<uint16_t*>(args.out)[(size_t)(cur.row_base + tok) * args.out_stride + out_row] =
-                            __half_as_ushort(__float2half_rn(o0[j]));
-                    } else {
-                        const size_t idx = (size_t)pair_base[j] * args.out_stride + out_row;
-                        if constexpr (OUT_MODE == kOutPartialF16)       // prefill.metal:666-669
-                            static_cast<uint16_t*>(args.out)[idx] = __half_as_ushort(__float2half_rn(o0[j]));
-                        else
-                            static_cast<float*>(args.out)[idx] = o0[j];
                     }
                 }
             }
@@ -817,14 +956,14 @@ __global__ void reduce_token_major_kernel(const void* __restrict__ partials, con
     out[(size_t)t * out_stride + d] = __half_as_ushort(__float2half_rn(acc));
 }
 
-template <int NMAT, bool DENSE, int OUT_MODE, int KC>
+template <int NMAT, bool DENSE, int OUT_MODE, int KC, int NT>
 static tf_status launch_grouped_k(tf_context* ctx, void* stream, GroupedArgs& args, const char* name) {
     const uint32_t ng = args.k / kGroup;
     const uint32_t cw = (ng + kGPW - 1) / kGPW;
-    const KSplitSmem<NMAT> lay{cw, ng, args.k / 2, ring_stages<NMAT, KC>()};
+    const KSplitSmem<NMAT, NT> lay{cw, ng, args.k / 2, ring_stages<NMAT, KC>()};
     const size_t smem = lay.total();
     TF_REQUIRE(ctx, smem <= 200 * 1024, TF_ERR_UNSUPPORTED, "%s: K=%u needs %zu bytes of shared memory (limit 200 KB)", name, args.k, smem);
-    auto kern = grouped_ksplit_kernel<NMAT, DENSE, OUT_MODE, KC>;
+    auto kern = grouped_ksplit_kernel<NMAT, DENSE, OUT_MODE, KC, NT>;
     // Attribute and occupancy are queried once per (instantiation, device, warp count) and cached, so
     // steady-state calls are a bare launch (and safe inside stream capture).
     static std::mutex cache_mu;
@@ -845,7 +984,7 @@ static tf_status launch_grouped_k(tf_context* ctx, void* stream, GroupedArgs& ar
     args.error = ctx->device_error;
     uint32_t grid = (uint32_t)ctx->sm_count * (uint32_t)per_sm;
     if (DENSE) {
-        const uint64_t items = (uint64_t)((args.dense_tokens + kChunkTokens - 1) / kChunkTokens) * (args.rows / kTileRows);
+        const uint64_t items = (uint64_t)((args.dense_tokens + kChunkTokens * NT - 1) / (kChunkTokens * NT)) * (args.rows / kTileRows);
         if (items == 0) return TF_OK;
         if (items < grid) grid = (uint32_t)items;
     }
@@ -854,16 +993,18 @@ static tf_status launch_grouped_k(tf_context* ctx, void* stream, GroupedArgs& ar
 }
 
 // KSPEC: the column count this instantiation is specialised for (the Gemma-4 shape of its role); other
-// column counts take the generic kernel.
+// column counts take the generic kernel, which has chunks of 8 tokens only.
+// wide: chunks of 16 tokens, for launches whose experts (or whose dense block) have more than 8 tokens as a rule.
 template <int NMAT, bool DENSE, int OUT_MODE, int KSPEC>
-static tf_status launch_grouped(tf_context* ctx, void* stream, GroupedArgs& args, const char* name) {
+static tf_status launch_grouped(tf_context* ctx, void* stream, GroupedArgs& args, bool wide, const char* name) {
     const uint32_t ng = args.k / kGroup;
     TF_REQUIRE(ctx, ng >= 1 && args.k % kGroup == 0, TF_ERR_INVALID_ARGUMENT, "%s: K must be a positive multiple of 64", name);
     const uint32_t cw = (ng + kGPW - 1) / kGPW;
     TF_REQUIRE(ctx, cw <= (uint32_t)kMaxComputeWarps, TF_ERR_UNSUPPORTED, "%s: K=%u outside the supported range (64..3072)", name, args.k);
     TF_REQUIRE(ctx, args.rows % kTileRows == 0, TF_ERR_UNSUPPORTED, "%s: row count %u must be a multiple of 16", name, args.rows);
-    if (args.k == (uint32_t)KSPEC) return launch_grouped_k<NMAT, DENSE, OUT_MODE, KSPEC>(ctx, stream, args, name);
-    return launch_grouped_k<NMAT, DENSE, OUT_MODE, 0>(ctx, stream, args, name);
+    if (args.k == (uint32_t)KSPEC && wide) return launch_grouped_k<NMAT, DENSE, OUT_MODE, KSPEC, 2>(ctx, stream, args, name);
+    if (args.k == (uint32_t)KSPEC) return launch_grouped_k<NMAT, DENSE, OUT_MODE, KSPEC, 1>(ctx, stream, args, name);
+    return launch_grouped_k<NMAT, DENSE, OUT_MODE, 0, 1>(ctx, stream, args, name);
 }
 
 static tf_status check_blob_alignment(tf_context* ctx, const void* pool, uint64_t stride, const tf_expert_offsets* o, const char* name) {
@@ -986,11 +1127,16 @@ tf_status tf_group_routes_device(tf_context* ctx, void* stream, const uint32_t* 
                                     "tf_group_routes_device", nullptr);
 }
 
-tf_status tf_grouped_moe_batched(tf_context* ctx, void* stream, const void* hidden, uint64_t hidden_off,
-                                 uint32_t hidden_stride_elements, const void* pool_layer_base, uint64_t expert_stride,
-                                 const tf_expert_offsets* offsets, const tf_device_routes* routes,
-                                 void* acts_scratch, void* route_partials, int partials_f32,
-                                 uint32_t query_count, uint32_t d, uint32_t f, uint32_t top_k) {
+}  // extern "C"
+
+namespace tf {
+
+// tf_grouped_moe_batched for a caller that knows the experts' number (0: not known, chunks of 8 tokens).
+tf_status grouped_moe_batched(tf_context* ctx, void* stream, const void* hidden, uint64_t hidden_off,
+                              uint32_t hidden_stride_elements, const void* pool_layer_base, uint64_t expert_stride,
+                              const tf_expert_offsets* offsets, const tf_device_routes* routes,
+                              void* acts_scratch, void* route_partials, int partials_f32,
+                              uint32_t query_count, uint32_t d, uint32_t f, uint32_t top_k, uint32_t num_experts) {
     const char* name = "tf_grouped_moe_batched";
     TF_REQUIRE(ctx, ctx != nullptr, TF_ERR_INVALID_ARGUMENT, "%s: ctx is NULL", name);
     TF_REQUIRE(ctx, hidden && pool_layer_base && routes && acts_scratch && route_partials, TF_ERR_INVALID_ARGUMENT, "%s: NULL argument", name);
@@ -1002,6 +1148,7 @@ tf_status tf_grouped_moe_batched(tf_context* ctx, void* stream, const void* hidd
     TF_REQUIRE(ctx, tf::aligned(hp, 16) && (hidden_stride_elements * 2) % 16 == 0 && tf::aligned(acts_scratch, 16),
                TF_ERR_ALIGNMENT, "%s: hidden rows and acts scratch must be 16-byte aligned", name);
     if (query_count == 0) return TF_OK;
+    const bool wide = num_experts > 0 && (uint64_t)query_count * top_k * 2 >= (uint64_t)num_experts * kWideRowsX2;
     tf::GroupedArgs a{};
     a.pool_base = static_cast<const uint8_t*>(pool_layer_base);
     a.expert_stride = expert_stride;
@@ -1011,7 +1158,7 @@ tf_status tf_grouped_moe_batched(tf_context* ctx, void* stream, const void* hidd
     a.chunk_start = routes->chunk_start; a.counters = routes->counters;
     a.x = reinterpret_cast<const uint16_t*>(hp); a.x_stride = hidden_stride_elements;
     a.out = acts_scratch; a.out_stride = f; a.rows = f; a.k = d; a.top_k = top_k;
-    tf_status s = tf::launch_grouped<2, false, tf::kOutActs, 2816>(ctx, stream, a, "tf_grouped_moe_batched(gate/up)");
+    tf_status s = tf::launch_grouped<2, false, tf::kOutActs, 2816>(ctx, stream, a, wide, "tf_grouped_moe_batched(gate/up)");
     if (s) return s;
 
     tf::GroupedArgs b{};
@@ -1021,8 +1168,21 @@ tf_status tf_grouped_moe_batched(tf_context* ctx, void* stream, const void* hidd
     b.chunk_start = routes->chunk_start; b.counters = routes->counters;
     b.x = static_cast<const uint16_t*>(acts_scratch); b.x_stride = f;
     b.out = route_partials; b.out_stride = d; b.rows = d; b.k = f; b.top_k = top_k;
-    if (partials_f32) return tf::launch_grouped<1, false, tf::kOutPartialF32, 704>(ctx, stream, b, "tf_grouped_moe_batched(down)");
-    return tf::launch_grouped<1, false, tf::kOutPartialF16, 704>(ctx, stream, b, "tf_grouped_moe_batched(down)");
+    if (partials_f32) return tf::launch_grouped<1, false, tf::kOutPartialF32, 704>(ctx, stream, b, wide, "tf_grouped_moe_batched(down)");
+    return tf::launch_grouped<1, false, tf::kOutPartialF16, 704>(ctx, stream, b, wide, "tf_grouped_moe_batched(down)");
+}
+
+}  // namespace tf
+
+extern "C" {
+
+tf_status tf_grouped_moe_batched(tf_context* ctx, void* stream, const void* hidden, uint64_t hidden_off,
+                                 uint32_t hidden_stride_elements, const void* pool_layer_base, uint64_t expert_stride,
+                                 const tf_expert_offsets* offsets, const tf_device_routes* routes,
+                                 void* acts_scratch, void* route_partials, int partials_f32,
+                                 uint32_t query_count, uint32_t d, uint32_t f, uint32_t top_k) {
+    return tf::grouped_moe_batched(ctx, stream, hidden, hidden_off, hidden_stride_elements, pool_layer_base, expert_stride, offsets,
+                                   routes, acts_scratch, route_partials, partials_f32, query_count, d, f, top_k, 0);
 }
 
 }  // extern "C"
@@ -1149,7 +1309,7 @@ tf_status tf_grouped_moe_streamed(tf_context* ctx, void* stream, const void* hid
     a.chunk_start = scratch->chunk_start; a.counters = scratch->counters;
     a.x = reinterpret_cast<const uint16_t*>(hp); a.x_stride = params->hidden_stride_elements;
     a.out = acts; a.out_stride = f; a.rows = f; a.k = d; a.top_k = params->top_k;
-    if (tf_status s = tf::launch_grouped<2, false, tf::kOutActs, 2816>(ctx, stream, a, "tf_grouped_moe_streamed(gate/up)")) return s;
+    if (tf_status s = tf::launch_grouped<2, false, tf::kOutActs, 2816>(ctx, stream, a, false, "tf_grouped_moe_streamed(gate/up)")) return s;
     tf::GroupedArgs b{};
     b.pool_base = lowest; b.expert_stride = 16;
     b.w_off[0] = offsets.down_w_off; b.s_off[0] = offsets.down_s_off; b.b_off[0] = offsets.down_b_off;
@@ -1157,7 +1317,7 @@ tf_status tf_grouped_moe_streamed(tf_context* ctx, void* stream, const void* hid
     b.chunk_start = scratch->chunk_start; b.counters = scratch->counters;
     b.x = reinterpret_cast<const uint16_t*>(acts); b.x_stride = f;
     b.out = tf::byte_ptr(route_partials, route_partials_off); b.out_stride = d; b.rows = d; b.k = f; b.top_k = params->top_k;
-    if (tf_status s = tf::launch_grouped<1, false, tf::kOutPartialF16, 704>(ctx, stream, b, "tf_grouped_moe_streamed(down)")) return s;
+    if (tf_status s = tf::launch_grouped<1, false, tf::kOutPartialF16, 704>(ctx, stream, b, false, "tf_grouped_moe_streamed(down)")) return s;
     if (microbatches_out) *microbatches_out = (params->pair_count + pair_microbatch_rows - 1) / pair_microbatch_rows;
     return TF_OK;
 }
@@ -1214,13 +1374,13 @@ tf_status tf_shared_expert_int4_block(tf_context* ctx, void* stream, const void*
     a.dense[0] = mp[0]; a.dense[1] = mp[1];
     a.x = reinterpret_cast<const uint16_t*>(xp); a.x_stride = x_stride_elements;
     a.out = scratch_act; a.out_stride = fs; a.rows = fs; a.k = d; a.dense_tokens = rows;
-    tf_status s = tf::launch_grouped<2, true, tf::kOutActs, 2816>(ctx, stream, a, "tf_shared_expert_int4_block(gate/up)");
+    tf_status s = tf::launch_grouped<2, true, tf::kOutActs, 2816>(ctx, stream, a, rows > tf::kWideDenseRows, "tf_shared_expert_int4_block(gate/up)");
     if (s) return s;
     tf::GroupedArgs b{};
     b.dense[0] = mp[2];
     b.x = static_cast<const uint16_t*>(scratch_act); b.x_stride = fs;
     b.out = tf::byte_ptr(y, y_off); b.out_stride = y_stride_elements; b.rows = d; b.k = fs; b.dense_tokens = rows;
-    return tf::launch_grouped<1, true, tf::kOutDenseF16, 2112>(ctx, stream, b, "tf_shared_expert_int4_block(down)");
+    return tf::launch_grouped<1, true, tf::kOutDenseF16, 2112>(ctx, stream, b, rows > tf::kWideDenseRows, "tf_shared_expert_int4_block(down)");
 }
 
 // The shared expert for callers that must not allocate. Same kernels as tf_shared_expert_int4_block; the
