@@ -833,6 +833,9 @@ tf_status tf_stack_forward(tf_stack* st, void* stream, void* hidden, uint32_t to
     // launch (combine_residual_rmsnorm_kernel; the values of the separate reduce and norm launches, two launches less).
     const bool fold = !st->layers.empty() && tf::block_keeps_f32_partials(ctx, ws, tokens) && st->layers[0].top_k <= TF_MAX_TOP_K &&
                       tf::aligned(ws->partials, 16) && tf::aligned(ws->shared_y, 16);
+    // Prefill-sized blocks leave expert-sorted fp16 rows instead; the same kernel gathers them through the permutation.
+    const bool fold_rows = !st->layers.empty() && tokens >= ctx->tensorcore_min_tokens && ws->x_sorted != nullptr && st->layers[0].top_k <= TF_MAX_TOP_K &&
+                           tf::aligned(ws->partials, 16) && tf::aligned(ws->shared_y, 16);
     uint32_t fold_threads = ((d / 8 + 31) / 32) * 32;          // one thread per eight columns,
     if (fold_threads < (uint32_t)tf::kRrnThreads) fold_threads = tf::kRrnThreads;      // at least the norm's 128 (its reduction tree)
     const uint16_t* no16 = nullptr;
@@ -845,12 +848,18 @@ tf_status tf_stack_forward(tf_stack* st, void* stream, void* hidden, uint32_t to
             tf::launch_pdl(tf::combine_residual_rmsnorm_kernel<false>, dim3(tokens), dim3(fold_threads), smem, cs, h,
                            static_cast<const void*>(ws->partials), static_cast<const uint16_t*>(ws->weights), no32u,
                            static_cast<const uint16_t*>(ws->shared_y), nw, ws->x_norm, d, st->layers[l - 1].top_k, st->eps, no_wait);
-        else
+        else if (l > 0 && fold_rows) {
+            if (tf_status s = tf::combine_rows_residual_rmsnorm(ctx, stream, h, ws->partials, ws->weights, ws->inverse_perm, ws->shared_y, nw,
+                                                                ws->x_norm, tokens, st->layers[l - 1].top_k, d, st->eps, nullptr)) return s;
+        } else
             tf::launch_pdl(tf::residual_rmsnorm_kernel, dim3(tokens), dim3(tf::kRrnThreads), smem, cs, h,
                            l == 0 ? no16 : static_cast<const uint16_t*>(ws->y_block), nw, ws->x_norm, d, st->eps);
         if (tf_status s = tf::check_launch(ctx, "residual_rmsnorm")) return s;
-        if (tf_status s = tf::block_forward(ctx, stream, &st->layers[l], ws->x_norm, d, fold ? nullptr : ws->y_block, d, tokens, ws)) return s;
+        if (tf_status s = tf::block_forward(ctx, stream, &st->layers[l], ws->x_norm, d, fold || fold_rows ? nullptr : ws->y_block, d, tokens, ws)) return s;
     }
+    if (fold_rows)
+        return tf::combine_rows_residual_rmsnorm(ctx, stream, h, ws->partials, ws->weights, ws->inverse_perm, ws->shared_y, nullptr, nullptr, tokens,
+                                                 st->layers.back().top_k, d, st->eps, nullptr);
     if (fold)
         tf::launch_pdl(tf::combine_residual_rmsnorm_kernel<false>, dim3(tokens), dim3(fold_threads), smem, cs, h,
                        static_cast<const void*>(ws->partials), static_cast<const uint16_t*>(ws->weights), no32u,
