@@ -6,6 +6,7 @@
 // once per block in shared memory; packed weights stream through 128-bit
 // non-allocating loads when the plane is 16-byte aligned, 16-bit loads otherwise.
 #include "rowdot.cuh"
+#include "tile_gemv.cuh"
 
 namespace tf {
 
@@ -120,6 +121,11 @@ static tf_status launch_gemv(tf_context* ctx, void* stream, const void* weights,
                                reinterpret_cast<const uint16_t*>(xp), yp, OUT_F32, m, n, sb_dtype == TF_FP16, name);
     const size_t smem = stage_x_bytes((int)n);
     TF_REQUIRE(ctx, smem <= 96 * 1024, TF_ERR_UNSUPPORTED, "%s: N=%u too large for the staged-x kernel", name, n);
+
+    // Matrices below the streaming kernel's 4096 rows: one launch latency and one memory latency.
+    if (BITS == 4 && m < 4096 && tile_gemv_eligible(W, xp, n))
+        return launch_tile_gemv(ctx, stream, W, reinterpret_cast<const uint16_t*>(S), reinterpret_cast<const uint16_t*>(Bp),
+                                reinterpret_cast<const uint16_t*>(xp), yp, OUT_F32, m, n, sb_dtype == TF_FP16, name);
 
     const size_t row_bytes = BITS == 4 ? n / 2 : n;
     const bool a16 = aligned(W, 16) && row_bytes % 16 == 0;

@@ -6,6 +6,7 @@
 // (moe.metal:62-76); the table is filled on the device from the router's ids,
 // so no id ever crosses to the host.
 #include "rowdot.cuh"
+#include "tile_gemv.cuh"
 
 namespace tf {
 
@@ -152,6 +153,9 @@ static tf_status launch_phase1(tf_context* ctx, void* stream, const void* const*
     if (slots == 0) return TF_OK;
     const size_t smem = stage_x_bytes((int)d);
     TF_REQUIRE(ctx, smem <= 96 * 1024, TF_ERR_UNSUPPORTED, "%s: D too large", name);
+    if (tile_gate_up_eligible(d, x))
+        return launch_tile_gate_up(ctx, stream, blobs, offsets, x, acts, d, f, top_k, slot_map, slots, name);
+    // x off the 16-byte grid: the row kernel loads it element by element
     if (smem > 48 * 1024)
         TF_CUDA(ctx, cudaFuncSetAttribute(moe_phase1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     dim3 grid((f + kP1RowsPerBlock - 1) / kP1RowsPerBlock, slots);
@@ -193,6 +197,8 @@ tf_status tf_moe_phase2_reduce(tf_context* ctx, void* stream, const void* const*
     TF_REQUIRE(ctx, (f / 2) % 16 == 0, TF_ERR_UNSUPPORTED, "%s: F/2 must be a multiple of 16 bytes", name);
     const size_t smem = tf::stage_x_bytes((int)f) * top_k + sizeof(float) * tf::kP2RowsPerBlock * top_k;
     TF_REQUIRE(ctx, smem <= 160 * 1024, TF_ERR_UNSUPPORTED, "%s: F too large", name);
+    if (tf::tile_down_eligible(f, acts))
+        return tf::launch_tile_down(ctx, stream, blobs, offsets, acts, routing_weights, residual, y, d, f, top_k, name);
     if (smem > 48 * 1024)
         TF_CUDA(ctx, cudaFuncSetAttribute(tf::moe_phase2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const uint32_t grid = (d + tf::kP2RowsPerBlock - 1) / tf::kP2RowsPerBlock;
