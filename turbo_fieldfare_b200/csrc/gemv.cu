@@ -13,7 +13,9 @@ namespace tf {
 // gemv_mma.cu: the tensor-core streaming kernel for large, aligned matrices
 bool gemv_mma_eligible(const void* W, const void* S, const void* B, const void* x, uint32_t m, uint32_t n);
 tf_status launch_gemv_mma(tf_context* ctx, void* stream, const uint8_t* W, const uint16_t* S, const uint16_t* B,
-                          const uint16_t* x, void* y, bool out_f32, uint32_t m, uint32_t n, bool sb_fp16, const char* name);
+                          const uint16_t* x, uint16_t* y, uint32_t m, uint32_t n, bool sb_fp16, const char* name);
+tf_status launch_gemv_mma_argmax(tf_context* ctx, void* stream, const uint8_t* W, const uint16_t* S, const uint16_t* B,
+                                 const uint16_t* x, uint32_t m, uint32_t n, unsigned long long* argmax, uint32_t* out_token, const char* name);
 tf_status launch_gemv_mma_batched(tf_context* ctx, void* stream, const uint8_t* W, const uint16_t* S, const uint16_t* B,
                                   uint64_t plane_stride, const uint16_t* x, uint32_t x_stride, uint16_t* y, uint32_t y_stride,
                                   uint32_t m, uint32_t n, uint32_t count, bool sb_fp16, const char* name);
@@ -116,12 +118,11 @@ static tf_status launch_gemv(tf_context* ctx, void* stream, const void* weights,
         TF_REQUIRE(ctx, aligned(W, 2), TF_ERR_ALIGNMENT, "%s: weightsOffset must be even", name);
     TF_REQUIRE(ctx, aligned(S, 2) && aligned(Bp, 2) && aligned(xp, 2) && aligned(yp, OUT_F32 ? 4 : 2), TF_ERR_ALIGNMENT,
                "%s: scale/bias/x/y planes must be 2-byte aligned", name);
-    if (BITS == 4 && gemv_mma_eligible(W, S, Bp, xp, m, n))
+    if (BITS == 4 && !OUT_F32 && gemv_mma_eligible(W, S, Bp, xp, m, n))
         return launch_gemv_mma(ctx, stream, W, reinterpret_cast<const uint16_t*>(S), reinterpret_cast<const uint16_t*>(Bp),
-                               reinterpret_cast<const uint16_t*>(xp), yp, OUT_F32, m, n, sb_dtype == TF_FP16, name);
+                               reinterpret_cast<const uint16_t*>(xp), reinterpret_cast<uint16_t*>(yp), m, n, sb_dtype == TF_FP16, name);
     const size_t smem = stage_x_bytes((int)n);
     TF_REQUIRE(ctx, smem <= 96 * 1024, TF_ERR_UNSUPPORTED, "%s: N=%u too large for the staged-x kernel", name, n);
-
     // Matrices below the streaming kernel's 4096 rows: one launch latency and one memory latency.
     if (BITS == 4 && m < 4096 && tile_gemv_eligible(W, xp, n))
         return launch_tile_gemv(ctx, stream, W, reinterpret_cast<const uint16_t*>(S), reinterpret_cast<const uint16_t*>(Bp),
@@ -157,13 +158,6 @@ static tf_status launch_gemv(tf_context* ctx, void* stream, const void* weights,
 // ---------------------------------------------------------------------------
 // Greedy LM head: argmax over the finite fp32 logits, ties to the lowest row
 // ---------------------------------------------------------------------------
-// A finite float as an unsigned key that orders like the float (every finite value maps above zero).
-__device__ __forceinline__ uint32_t ordered_key(float v) {
-    if (v == 0.0f) v = 0.0f;                        // -0 and +0 compare equal in the reference's reduction
-    const uint32_t b = __float_as_uint(v);
-    return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
-}
-
 constexpr int kArgmaxThreads = 256;
 
 // best = max over rows of (ordered logit << 32 | ~row): the larger logit wins, then the lower row.
@@ -218,21 +212,27 @@ tf_status tf_lm_head_greedy_int4(tf_context* ctx, void* stream, const void* hidd
     TF_REQUIRE(ctx, tf::aligned(out_token, 4), TF_ERR_ALIGNMENT, "%s: outToken must be 4-byte aligned", name);
     // scratch owned by the context; growing it allocates (and so cannot happen inside a stream capture)
     if (ctx->lm_best == nullptr) {
-        TF_CUDA(ctx, cudaMalloc(&ctx->lm_best, sizeof(unsigned long long)));
-        TF_CUDA(ctx, cudaMemset(ctx->lm_best, 0, sizeof(unsigned long long)));
+        TF_CUDA(ctx, cudaMalloc(&ctx->lm_best, 2 * sizeof(unsigned long long)));
+        TF_CUDA(ctx, cudaMemset(ctx->lm_best, 0, 2 * sizeof(unsigned long long)));
     }
     if (d > ctx->lm_x_capacity) {
         if (ctx->lm_x) { TF_CUDA(ctx, cudaFree(ctx->lm_x)); ctx->lm_x = nullptr; ctx->lm_x_capacity = 0; }
         TF_CUDA(ctx, cudaMalloc(&ctx->lm_x, (size_t)d * 2));
         ctx->lm_x_capacity = d;
     }
-    if (vocab > ctx->lm_logits_capacity) {
+    // aligned heads keep only the largest logit; the others store them all
+    const uint8_t *wp = tf::byte_ptr(weights, weights_off), *sp = tf::byte_ptr(scales, scales_off), *bp = tf::byte_ptr(biases, biases_off);
+    const bool streamed = tf::gemv_mma_eligible(wp, sp, bp, ctx->lm_x, vocab, d);
+    if (!streamed && vocab > ctx->lm_logits_capacity) {
         if (ctx->lm_logits) { TF_CUDA(ctx, cudaFree(ctx->lm_logits)); ctx->lm_logits = nullptr; ctx->lm_logits_capacity = 0; }
         TF_CUDA(ctx, cudaMalloc(&ctx->lm_logits, (size_t)vocab * 4));
         ctx->lm_logits_capacity = vocab;
     }
     tf_status st = tf_rmsnorm(ctx, stream, hidden, hidden_off, norm_weight_bf16, norm_off, ctx->lm_x, 0, 1, d, d, rms_eps, TF_FP16);
     if (st != TF_OK) return st;
+    if (streamed)
+        return tf::launch_gemv_mma_argmax(ctx, stream, wp, reinterpret_cast<const uint16_t*>(sp), reinterpret_cast<const uint16_t*>(bp), ctx->lm_x,
+                                          vocab, d, ctx->lm_best, out_token, name);
     st = tf::launch_gemv<4, true>(ctx, stream, weights, weights_off, scales, scales_off, biases, biases_off, ctx->lm_x, 0,
                                   ctx->lm_logits, 0, vocab, d, TF_BF16, name);
     if (st != TF_OK) return st;

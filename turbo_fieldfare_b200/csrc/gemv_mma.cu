@@ -29,10 +29,19 @@ struct GemvBatch {
     uint32_t x_stride, y_stride;
 };
 
-template <bool SB_FP16, bool OUT_F32, int WARPS>
+__device__ __forceinline__ unsigned long long argmax_key(float z, uint32_t row) {
+    return isfinite(z) ? ((unsigned long long)ordered_key(z) << 32) | (unsigned long long)(~row) : 0ull;
+}
+
+// What becomes of the row sums: stored as fp16, or (the greedy LM head) only the largest fp32 one is kept. ARGMAX: the launch
+// follows the call's own norm kernel and nothing else, so weights are requested before that kernel has ended; every block
+// folds its rows into argmax[0] (ordered logit << 32 | ~row) and the last one (argmax[1] counts) decodes the token and
+// clears both. Storing 262144 logits, a second kernel over them and a third to decode took 8 us.
+template <bool SB_FP16, bool ARGMAX, int WARPS>
 __global__ void __launch_bounds__(WARPS * kWarp)
 gemv_mma_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S, const uint16_t* __restrict__ B,
-                const uint16_t* __restrict__ x, void* __restrict__ y, uint32_t m, uint32_t n, const GemvBatch bt) {
+                const uint16_t* __restrict__ x, uint16_t* __restrict__ y, uint32_t m, uint32_t n, const GemvBatch bt,
+                unsigned long long* argmax, uint32_t* out_token) {
     extern __shared__ __align__(16) uint8_t smem[];
     constexpr int kGmRows = WARPS * 16, kGmThreads = WARPS * kWarp;
     {
@@ -41,7 +50,7 @@ gemv_mma_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S, c
         S = reinterpret_cast<const uint16_t*>(reinterpret_cast<const uint8_t*>(S) + b * bt.plane_stride);
         B = reinterpret_cast<const uint16_t*>(reinterpret_cast<const uint8_t*>(B) + b * bt.plane_stride);
         x += b * bt.x_stride;
-        y = static_cast<uint8_t*>(y) + b * bt.y_stride * (OUT_F32 ? 4 : 2);
+        y += b * bt.y_stride;
     }
     const uint32_t ng = n / kGroup;
     uint32_t* xfrag = reinterpret_cast<uint32_t*>(smem);                       // ng * 32 words
@@ -52,6 +61,28 @@ gemv_mma_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S, c
     const int g = lane >> 2, t = lane & 3;
     const uint32_t row_base = blockIdx.x * kGmRows;
 
+    pdl_launch_dependents();
+    if constexpr (!ARGMAX) pdl_wait();
+    // the first groups' codes are on their way while scales, biases and x are staged
+    const uint32_t r0 = row_base + warp * 16 + g, r1 = r0 + 8;
+    const uint32_t row_bytes = n / 2;
+    // rows past the matrix read the last row (their results are not stored)
+    const uint8_t* W0 = W + (size_t)(r0 < m ? r0 : m - 1) * row_bytes + t * 8;
+    const uint8_t* W1 = W + (size_t)(r1 < m ? r1 : m - 1) * row_bytes + t * 8;
+    uint2 wa[kGmBlockGroups], wb[kGmBlockGroups];
+#pragma unroll
+    for (int i = 0; i < kGmBlockGroups; ++i) { wa[i] = gm_ldg64(W0 + i * 32); wb[i] = gm_ldg64(W1 + i * 32); }
+    // ---- scale and bias planes of the block's rows (contiguous in global memory) ----
+    {
+        const uint32_t rows_here = m - row_base < (uint32_t)kGmRows ? m - row_base : (uint32_t)kGmRows;
+        const uint32_t words = rows_here * ng / 2;                             // rows * ng is even (ng % 4 == 0)
+        const uint32_t* gs = reinterpret_cast<const uint32_t*>(S + (size_t)row_base * ng);
+        const uint32_t* gb = reinterpret_cast<const uint32_t*>(B + (size_t)row_base * ng);
+        uint32_t* ds = reinterpret_cast<uint32_t*>(sS);
+        uint32_t* db = reinterpret_cast<uint32_t*>(sB);
+        for (uint32_t i = threadIdx.x; i < words; i += kGmThreads) { ds[i] = __ldg(gs + i); db[i] = __ldg(gb + i); }
+    }
+    if constexpr (ARGMAX) pdl_wait();
     // ---- stage x in MMA operand order: the 16 values x0..x15 at columns 64 G + 16 t feed four MMAs,
     //   j = 0: (x0,x4),(x2,x6)   j = 1: (x1,x5)/16,(x3,x7)/16   j = 2, 3: the same for x8..x15
     // (odd columns are pre-scaled by 1/16 because their codes sit four mantissa bits higher) ----
@@ -82,23 +113,8 @@ gemv_mma_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S, c
             f[4 * h2 + 3] = gm_sixteenth(gm_prmt(r[o + 1], r[o + 3], 0x7632));
         }
     }
-    // ---- scale and bias planes of the block's rows (contiguous in global memory) ----
-    {
-        const uint32_t rows_here = m - row_base < (uint32_t)kGmRows ? m - row_base : (uint32_t)kGmRows;
-        const uint32_t words = rows_here * ng / 2;                             // rows * ng is even (ng % 4 == 0)
-        const uint32_t* gs = reinterpret_cast<const uint32_t*>(S + (size_t)row_base * ng);
-        const uint32_t* gb = reinterpret_cast<const uint32_t*>(B + (size_t)row_base * ng);
-        uint32_t* ds = reinterpret_cast<uint32_t*>(sS);
-        uint32_t* db = reinterpret_cast<uint32_t*>(sB);
-        for (uint32_t i = threadIdx.x; i < words; i += kGmThreads) { ds[i] = __ldg(gs + i); db[i] = __ldg(gb + i); }
-    }
     __syncthreads();
 
-    const uint32_t r0 = row_base + warp * 16 + g, r1 = r0 + 8;
-    const uint32_t row_bytes = n / 2;
-    // rows past the matrix read the last row (their results are not stored)
-    const uint8_t* W0 = W + (size_t)(r0 < m ? r0 : m - 1) * row_bytes + t * 8;
-    const uint8_t* W1 = W + (size_t)(r1 < m ? r1 : m - 1) * row_bytes + t * 8;
     const uint16_t* s0p = sS + (size_t)(warp * 16 + g) * ng;
     const uint16_t* s1p = s0p + 8 * ng;
     const uint16_t* b0p = sB + (size_t)(warp * 16 + g) * ng;
@@ -108,9 +124,6 @@ gemv_mma_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S, c
     for (int j = 0; j < 4; ++j) asm volatile("mov.f32 %0, 0f00000000;" : "=f"(zc[j]));
 
     float acc0 = 0.0f, acc1 = 0.0f;
-    uint2 wa[kGmBlockGroups], wb[kGmBlockGroups];
-#pragma unroll
-    for (int i = 0; i < kGmBlockGroups; ++i) { wa[i] = gm_ldg64(W0 + i * 32); wb[i] = gm_ldg64(W1 + i * 32); }
     for (uint32_t G0 = 0; G0 < ng; G0 += kGmBlockGroups) {
         uint2 ca[kGmBlockGroups], cb[kGmBlockGroups];
 #pragma unroll
@@ -157,14 +170,34 @@ gemv_mma_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S, c
             acc1 = fmaf(s1, c[i][2], fmaf(b1, xsv[i], acc1));
         }
     }
-    if (t == 0) {
-        if constexpr (OUT_F32) {       // unrounded row sums (the greedy LM head compares them as fp32)
-            if (r0 < m) static_cast<float*>(y)[r0] = acc0;
-            if (r1 < m) static_cast<float*>(y)[r1] = acc1;
-        } else {
-            if (r0 < m) static_cast<uint16_t*>(y)[r0] = __half_as_ushort(__float2half_rn(acc0));
-            if (r1 < m) static_cast<uint16_t*>(y)[r1] = __half_as_ushort(__float2half_rn(acc1));
+    if constexpr (ARGMAX) {
+        __shared__ unsigned long long per_warp[WARPS];
+        unsigned long long mine = 0ull;                 // 0 = no finite candidate
+        if (t == 0 && r0 < m) mine = argmax_key(acc0, r0);
+        if (t == 0 && r1 < m) { const unsigned long long k = argmax_key(acc1, r1); mine = k > mine ? k : mine; }
+#pragma unroll
+        for (int o = kWarp / 2; o >= 4; o >>= 1) {
+            const unsigned long long other = __shfl_xor_sync(kFullMask, mine, o);
+            mine = other > mine ? other : mine;
         }
+        if (lane == 0) per_warp[warp] = mine;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+#pragma unroll
+            for (int w = 1; w < WARPS; ++w) mine = per_warp[w] > mine ? per_warp[w] : mine;
+            if (mine) atomicMax(argmax, mine);
+            __threadfence();
+            if (atomicAdd(argmax + 1, 1ull) == gridDim.x - 1) {
+                __threadfence();
+                const unsigned long long k = atomicMax(argmax, 0ull);
+                *out_token = k ? ~(uint32_t)(k & 0xFFFFFFFFull) : 0u;      // 0 when no logit was finite
+                argmax[0] = 0ull;                                        // ready for the next call
+                argmax[1] = 0ull;
+            }
+        }
+    } else if (t == 0) {
+        if (r0 < m) y[r0] = __half_as_ushort(__float2half_rn(acc0));
+        if (r1 < m) y[r1] = __half_as_ushort(__float2half_rn(acc1));
     }
 }
 
@@ -181,14 +214,27 @@ bool gemv_mma_eligible(const void* W, const void* S, const void* B, const void* 
 }
 
 tf_status launch_gemv_mma(tf_context* ctx, void* stream, const uint8_t* W, const uint16_t* S, const uint16_t* B,
-                          const uint16_t* x, void* y, bool out_f32, uint32_t m, uint32_t n, bool sb_fp16, const char* name) {
+                          const uint16_t* x, uint16_t* y, uint32_t m, uint32_t n, bool sb_fp16, const char* name) {
     const size_t smem = gemv_mma_smem_bytes(n);
-    const int which = (sb_fp16 ? 1 : 0) + (out_f32 ? 2 : 0);
-    auto k = which == 0 ? gemv_mma_kernel<false, false, kGmWarps> : which == 1 ? gemv_mma_kernel<true, false, kGmWarps>
-             : which == 2 ? gemv_mma_kernel<false, true, kGmWarps> : gemv_mma_kernel<true, true, kGmWarps>;
-    static DeviceSmemCache configured[4];
-    if (tf_status st = ensure_dynamic_smem(ctx, k, configured[which], smem)) return st;
-    k<<<(m + kGmWarps * 16 - 1) / (kGmWarps * 16), kGmWarps * kWarp, smem, static_cast<cudaStream_t>(stream)>>>(W, S, B, x, y, m, n, GemvBatch{0, 0, 0});
+    auto k = sb_fp16 ? gemv_mma_kernel<true, false, kGmWarps> : gemv_mma_kernel<false, false, kGmWarps>;
+    static DeviceSmemCache configured[2];
+    if (tf_status st = ensure_dynamic_smem(ctx, k, configured[sb_fp16 ? 1 : 0], smem)) return st;
+    launch_pdl(k, dim3((m + kGmWarps * 16 - 1) / (kGmWarps * 16)), dim3(kGmWarps * kWarp), smem, static_cast<cudaStream_t>(stream), W, S, B, x, y,
+               m, n, GemvBatch{0, 0, 0}, nullptr, nullptr);
+    return check_launch(ctx, name);
+}
+
+// The greedy LM head's product: argmax points to two 64-bit words, zero before and after. Must follow, on the stream, the
+// launch that writes x, and that launch must start after everything before it (no programmatic launch of its own).
+// Blocks of 64 rows: 4096 of them for 262144 rows, so that the last round of blocks is a small part of the whole.
+tf_status launch_gemv_mma_argmax(tf_context* ctx, void* stream, const uint8_t* W, const uint16_t* S, const uint16_t* B,
+                                 const uint16_t* x, uint32_t m, uint32_t n, unsigned long long* argmax, uint32_t* out_token, const char* name) {
+    const size_t smem = gemv_mma_smem_bytes_for(n, kGmBatchWarps);
+    auto k = gemv_mma_kernel<false, true, kGmBatchWarps>;
+    static DeviceSmemCache configured;
+    if (tf_status st = ensure_dynamic_smem(ctx, k, configured, smem)) return st;
+    launch_pdl(k, dim3((m + kGmBatchWarps * 16 - 1) / (kGmBatchWarps * 16)), dim3(kGmBatchWarps * kWarp), smem, static_cast<cudaStream_t>(stream),
+               W, S, B, x, nullptr, m, n, GemvBatch{0, 0, 0}, argmax, out_token);
     return check_launch(ctx, name);
 }
 
@@ -204,11 +250,11 @@ tf_status launch_gemv_mma_batched(tf_context* ctx, void* stream, const uint8_t* 
     for (uint32_t first = 0; first < count; first += 65535u) {        // gridDim.y limit
         const uint32_t nb = count - first < 65535u ? count - first : 65535u;
         dim3 grid((m + rows_per_block - 1) / rows_per_block, nb);
-        k<<<grid, kGmBatchWarps * kWarp, smem, static_cast<cudaStream_t>(stream)>>>(
+        launch_pdl(k, grid, dim3(kGmBatchWarps * kWarp), smem, static_cast<cudaStream_t>(stream),
             W + (size_t)first * plane_stride,
             reinterpret_cast<const uint16_t*>(reinterpret_cast<const uint8_t*>(S) + (size_t)first * plane_stride),
             reinterpret_cast<const uint16_t*>(reinterpret_cast<const uint8_t*>(B) + (size_t)first * plane_stride),
-            x + (size_t)first * x_stride, y + (size_t)first * y_stride, m, n, GemvBatch{plane_stride, x_stride, y_stride});
+            x + (size_t)first * x_stride, y + (size_t)first * y_stride, m, n, GemvBatch{plane_stride, x_stride, y_stride}, nullptr, nullptr);
         if (tf_status st = check_launch(ctx, name)) return st;
     }
     return TF_OK;

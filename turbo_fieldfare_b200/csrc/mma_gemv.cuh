@@ -43,4 +43,11 @@ __device__ __forceinline__ void gm_make_frag(const uint32_t (&r)[8], uint32_t* f
     }
 }
 
+// A finite float as an unsigned key that orders like the float (every finite value maps above zero).
+__device__ __forceinline__ uint32_t ordered_key(float v) {
+    if (v == 0.0f) v = 0.0f;                        // -0 and +0 compare equal in the reference's reduction
+    const uint32_t b = __float_as_uint(v);
+    return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+}
+
 }  // namespace tf
