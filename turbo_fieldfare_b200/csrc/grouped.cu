@@ -919,6 +919,187 @@ grouped_ksplit_kernel(const GroupedArgs args) {
     }
 }
 
+// The routed down projection of chunks of 8 tokens for rows short enough that one warp keeps the chunk's fragments of ALL
+// columns in registers (NG = 11 groups: 88 registers, the production width): an item (16 rows) then belongs to one warp, and
+// what the column-split kernel spends on handing partial sums to reducer warps goes away. That kernel had nine compute warps
+// per SM, each waiting on the others twice per item of 6 KB: 550 clocks per item where the SM's share of the HBM rate is 275.
+// Here eleven independent warps take the items in turn, fed by one loader through a ring of stages of four consecutive items
+// (one copy of 64 rows, one of their scales, one of their biases: a loader turn costs several hundred clocks whatever it
+// moves). Sums have the bits of the column-split kernel: parts of four groups, added in order.
+constexpr int kDownWarps = 11;
+constexpr int kDownSub = 4;               // items per stage
+constexpr int kDownStages = 7;
+template <int OUT_MODE, int NG>
+__global__ void __launch_bounds__((kDownWarps + 1) * kWarp, 1)
+grouped_down_kernel(const GroupedArgs args) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    constexpr uint32_t kRowBytes = NG * 32, kCodeBytes = kTileRows * kRowBytes, kPlaneBytes = kTileRows * NG * 2;
+    constexpr uint32_t kStageBytes = kDownSub * (kCodeBytes + 2 * kPlaneBytes);
+    static_assert((kRowBytes / 4) % 32 == 8 || (kRowBytes / 4) % 32 == 24, "unpadded rows must spread over the banks");
+    const int warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
+    const int g = lane >> 2, t = lane & 3;
+    const uint32_t smem_base = (uint32_t)__cvta_generic_to_shared(smem);
+    const uint32_t bar_base = smem_base + kDownStages * kStageBytes;
+    auto bar_full = [&](uint32_t st) { return bar_base + st * 8; };
+    auto bar_empty = [&](uint32_t st) { return bar_base + (kDownStages + st) * 8; };
+    const uint32_t tiles = args.rows / kTileRows;
+    pdl_launch_dependents();
+    if (threadIdx.x == 0) {
+        for (uint32_t st = 0; st < (uint32_t)kDownStages; ++st) { mbar_init(bar_full(st), 1); mbar_init(bar_empty(st), kDownSub); }
+        fence_proxy_async();
+    }
+    __syncthreads();
+    pdl_wait();
+    // contiguous ranges of whole stages (a chunk's tiles are a multiple of four)
+    const uint32_t total_chunks = args.counters[1];
+    const uint32_t total_stages = total_chunks * (tiles / kDownSub);
+    const uint32_t stage_begin = (uint32_t)((uint64_t)total_stages * blockIdx.x / gridDim.x);
+    const uint32_t n_stages = (uint32_t)((uint64_t)total_stages * (blockIdx.x + 1) / gridDim.x) - stage_begin;
+    const uint32_t item_begin = stage_begin * kDownSub, n_items = n_stages * kDownSub;
+    if (n_items == 0) return;
+    ItemCursor<1> cur;
+    uint32_t fail = 0;
+    auto place = [&](uint32_t item) {                         // the cursor's chunk and tile; resolves a new chunk
+        const uint32_t chunk = item / tiles;
+        cur.tile = item - chunk * tiles;
+        if (chunk != cur.chunk) { cur.chunk = chunk; resolve_chunk<1, false, 1>(args, cur, nullptr); return true; }
+        return false;
+    };
+    cur.chunk = 0xFFFFFFFFu;
+    if (warp < kDownWarps) {
+        float zc[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) asm volatile("mov.f32 %0, 0f00000000;" : "=f"(zc[j]));
+        uint2 xb[NG][4];            // B fragments of token g
+        float2 xsum[NG];            // group sums of tokens 2t and 2t + 1, at 2^-24
+        uint32_t idx[2] = {0u, 0u}; // (token * top_k + rank) of tokens 2t and 2t + 1
+        for (uint32_t li = warp; li < n_items; li += kDownWarps) {
+            const uint32_t st = (li / kDownSub) % kDownStages, use = (li / kDownSub) / kDownStages, sub = li % kDownSub;
+            if (place(item_begin + li)) {
+#pragma unroll
+                for (int i = 0; i < NG; ++i) {
+                    uint32_t r[8];
+                    if ((uint32_t)g < cur.ntok) {
+                        const uint4* p = reinterpret_cast<const uint4*>(args.x + (size_t)(cur.row_base + g) * args.x_stride + i * kGroup + t * 16);
+                        const uint4 lo = __ldg(p), hi = __ldg(p + 1);
+                        r[0] = lo.x; r[1] = lo.y; r[2] = lo.z; r[3] = lo.w;
+                        r[4] = hi.x; r[5] = hi.y; r[6] = hi.z; r[7] = hi.w;
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < 8; ++q) r[q] = 0;
+                    }
+                    float sum = 0.0f;
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&r[q]));
+                        sum += v.x + v.y;
+                    }
+                    sum += __shfl_xor_sync(kFullMask, sum, 1);
+                    sum += __shfl_xor_sync(kFullMask, sum, 2);
+                    sum *= 5.9604644775390625e-08f;
+                    xsum[i] = make_float2(__shfl_sync(kFullMask, sum, 8 * t), __shfl_sync(kFullMask, sum, 8 * t + 4));
+#pragma unroll
+                    for (int h2 = 0; h2 < 2; ++h2) {
+                        const int o = 4 * h2;
+                        xb[i][2 * h2] = make_uint2(prmt(r[o], r[o + 2], 0x5410), prmt(r[o + 1], r[o + 3], 0x5410));
+                        xb[i][2 * h2 + 1] = make_uint2(hmul2_sixteenth(prmt(r[o], r[o + 2], 0x7632)),
+                                                       hmul2_sixteenth(prmt(r[o + 1], r[o + 3], 0x7632)));
+                    }
+                }
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    if (2 * t + c < (int)cur.ntok) {
+                        const tf_pair pr = args.sorted_pairs[cur.row_base + 2 * t + c];
+                        idx[c] = pr.token * args.top_k + pr.rank;
+                    }
+                }
+            }
+            if (!mbar_wait(bar_full(st), use & 1)) { fail = kErrTimeoutCodes; break; }
+            const uint32_t codes = smem_base + st * kStageBytes + sub * kCodeBytes + g * kRowBytes + t * 8;
+            const uint32_t scales = smem_base + st * kStageBytes + kDownSub * kCodeBytes + sub * kPlaneBytes + g * (NG * 2);
+            const uint32_t biases = scales + kDownSub * kPlaneBytes;
+            float y[4];
+#pragma unroll
+            for (int h = 0; h < NG; h += kGPW) {
+                constexpr int kMax = kGPW;
+                const int n = NG - h < kMax ? NG - h : kMax;
+                uint2 wa[kMax], wb[kMax];
+                float c[kMax][4];
+#pragma unroll
+                for (int i = 0; i < kMax; ++i)
+                    if (i < n) { wa[i] = lds64(codes + (h + i) * 32); wb[i] = lds64(codes + 8 * kRowBytes + (h + i) * 32); }
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+#pragma unroll
+                    for (int i = 0; i < kMax; ++i) {
+                        if (i < n) {
+                            const uint32_t mask = (j & 1) ? 0x00F000F0u : 0x000F000Fu;
+                            const uint32_t wx = j < 2 ? wa[i].x : wa[i].y, wy = j < 2 ? wb[i].x : wb[i].y;
+                            if (j == 0) mma16816_first(c[i], wx & mask, wy & mask, (wx >> 8) & mask, (wy >> 8) & mask, xb[h + i][0], zc);
+                            else mma16816_acc(c[i], wx & mask, wy & mask, (wx >> 8) & mask, (wy >> 8) & mask, xb[h + i][j]);
+                        }
+                    }
+                }
+                float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+                for (int i = 0; i < kMax; ++i) {
+                    if (i < n) {
+                        const float s0 = bf16_lo(lds16(scales + (h + i) * 2)), s1 = bf16_lo(lds16(scales + 8 * NG * 2 + (h + i) * 2));
+                        const float b0 = bf16_lo(lds16(biases + (h + i) * 2)), b1 = bf16_lo(lds16(biases + 8 * NG * 2 + (h + i) * 2));
+                        acc[0] = fmaf(s0, c[i][0], fmaf(b0, xsum[h + i].x, acc[0]));
+                        acc[1] = fmaf(s0, c[i][1], fmaf(b0, xsum[h + i].y, acc[1]));
+                        acc[2] = fmaf(s1, c[i][2], fmaf(b1, xsum[h + i].x, acc[2]));
+                        acc[3] = fmaf(s1, c[i][3], fmaf(b1, xsum[h + i].y, acc[3]));
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < 4; ++j) y[j] = h == 0 ? acc[j] * 16777216.0f : y[j] + acc[j] * 16777216.0f;
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_empty(st));
+            // y0, y1: row g, tokens 2t, 2t + 1; y2, y3: row g + 8
+            const uint32_t row = cur.tile * kTileRows + g;
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                if (2 * t + c < (int)cur.ntok) {
+                    const size_t o = (size_t)idx[c] * args.out_stride + row;
+                    if constexpr (OUT_MODE == kOutPartialF16) {       // prefill.metal:666-669
+                        static_cast<uint16_t*>(args.out)[o] = __half_as_ushort(__float2half_rn(y[c]));
+                        static_cast<uint16_t*>(args.out)[o + 8] = __half_as_ushort(__float2half_rn(y[2 + c]));
+                    } else {
+                        static_cast<float*>(args.out)[o] = y[c];
+                        static_cast<float*>(args.out)[o + 8] = y[2 + c];
+                    }
+                }
+            }
+        }
+    } else {
+        // loader: lane 0 moves a stage's codes, lane 1 its scales, lane 2 its biases
+        uint32_t st = 0, use = 0, issued = 0;
+        for (uint32_t si = 0; si < n_stages; ++si) {
+            place(item_begin + si * kDownSub);
+            if (use > 0 && !mbar_wait(bar_empty(st), (use - 1) & 1)) { fail = kErrTimeoutStageFree; break; }
+            const uint32_t mbar = bar_full(st), stage = smem_base + st * kStageBytes;
+            if (lane == 0) {
+                fence_proxy_async();          // the stage was last read through the generic proxy
+                mbar_arrive_expect_tx(mbar, kStageBytes);
+            }
+            __syncwarp();
+            const MatPlanes& mp = cur.pl[0];
+            if (lane == 0) bulk_copy_g2s(stage, mp.W + (size_t)cur.tile * kCodeBytes, kDownSub * kCodeBytes, mbar);
+            else if (lane < 3)
+                bulk_copy_g2s(stage + kDownSub * (kCodeBytes + (lane - 1) * kPlaneBytes), (lane == 1 ? mp.S : mp.B) + (size_t)cur.tile * kTileRows * NG,
+                              kDownSub * kPlaneBytes, mbar);
+            ++issued;
+            if (++st == (uint32_t)kDownStages) { st = 0; ++use; }
+        }
+        if (fail)            // the copies already issued land before the CTA's shared memory goes away (bounded)
+            for (uint32_t s2 = 0; s2 < (uint32_t)kDownStages && s2 < issued; ++s2)
+                for (uint32_t par = 0; par < 2; ++par) mbar_wait(bar_full(s2), par);
+    }
+    if (fail && lane == 0) atomicCAS(args.error, 0u, fail);
+}
+
 }  // namespace tf
 
 // ---------------------------------------------------------------------------
@@ -1002,9 +1183,29 @@ static tf_status launch_grouped(tf_context* ctx, void* stream, GroupedArgs& args
     const uint32_t cw = (ng + kGPW - 1) / kGPW;
     TF_REQUIRE(ctx, cw <= (uint32_t)kMaxComputeWarps, TF_ERR_UNSUPPORTED, "%s: K=%u outside the supported range (64..3072)", name, args.k);
     TF_REQUIRE(ctx, args.rows % kTileRows == 0, TF_ERR_UNSUPPORTED, "%s: row count %u must be a multiple of 16", name, args.rows);
-    if (args.k == (uint32_t)KSPEC && wide) return launch_grouped_k<NMAT, DENSE, OUT_MODE, KSPEC, 2>(ctx, stream, args, name);
+    if constexpr (NMAT == 2 || DENSE)        // the routed down projection has a kernel of its own for more tokens
+        if (args.k == (uint32_t)KSPEC && wide) return launch_grouped_k<NMAT, DENSE, OUT_MODE, KSPEC, 2>(ctx, stream, args, name);
     if (args.k == (uint32_t)KSPEC) return launch_grouped_k<NMAT, DENSE, OUT_MODE, KSPEC, 1>(ctx, stream, args, name);
     return launch_grouped_k<NMAT, DENSE, OUT_MODE, 0, 1>(ctx, stream, args, name);
+}
+
+// The routed down projection: the whole-row kernel for the width that it is built for, from 320 (token, expert) pairs on (40
+// tokens of eight experts); with fewer, its deeper pipeline does not pay for the time that it takes to fill. Steps of 30 layers
+// with it and without: 32 tokens 3.27 and 3.23 ms, 48 tokens 3.81 and 3.87, 64 tokens 3.85 and 4.21, 200 tokens 7.45 and 8.26
+// (the latter with 16-token chunks in the column-split kernel).
+constexpr uint32_t kDownMinPairs = 320;
+template <int OUT_MODE>
+static tf_status launch_grouped_down(tf_context* ctx, void* stream, GroupedArgs& args, uint64_t pairs, const char* name) {
+    constexpr int kGroups = 11;
+    if (pairs < kDownMinPairs || args.k != (uint32_t)(kGroups * kGroup) || args.rows % (kTileRows * kDownSub) != 0 || args.rows == 0)
+        return launch_grouped<1, false, OUT_MODE, kGroups * kGroup>(ctx, stream, args, false, name);
+    constexpr size_t smem = (size_t)kDownStages * kDownSub * (kTileRows * kGroups * 36) + 2 * kDownStages * 8;
+    auto kern = grouped_down_kernel<OUT_MODE, kGroups>;
+    static DeviceSmemCache configured;
+    if (tf_status s = ensure_dynamic_smem(ctx, kern, configured, smem)) return s;
+    args.error = ctx->device_error;
+    launch_pdl(kern, dim3((uint32_t)ctx->sm_count), dim3((kDownWarps + 1) * kWarp), smem, static_cast<cudaStream_t>(stream), args);
+    return check_launch(ctx, name);
 }
 
 static tf_status check_blob_alignment(tf_context* ctx, const void* pool, uint64_t stride, const tf_expert_offsets* o, const char* name) {
@@ -1168,8 +1369,8 @@ tf_status grouped_moe_batched(tf_context* ctx, void* stream, const void* hidden,
     b.chunk_start = routes->chunk_start; b.counters = routes->counters;
     b.x = static_cast<const uint16_t*>(acts_scratch); b.x_stride = f;
     b.out = route_partials; b.out_stride = d; b.rows = d; b.k = f; b.top_k = top_k;
-    if (partials_f32) return tf::launch_grouped<1, false, tf::kOutPartialF32, 704>(ctx, stream, b, wide, "tf_grouped_moe_batched(down)");
-    return tf::launch_grouped<1, false, tf::kOutPartialF16, 704>(ctx, stream, b, wide, "tf_grouped_moe_batched(down)");
+    if (partials_f32) return tf::launch_grouped_down<tf::kOutPartialF32>(ctx, stream, b, (uint64_t)query_count * top_k, "tf_grouped_moe_batched(down)");
+    return tf::launch_grouped_down<tf::kOutPartialF16>(ctx, stream, b, (uint64_t)query_count * top_k, "tf_grouped_moe_batched(down)");
 }
 
 }  // namespace tf
@@ -1317,7 +1518,7 @@ tf_status tf_grouped_moe_streamed(tf_context* ctx, void* stream, const void* hid
     b.chunk_start = scratch->chunk_start; b.counters = scratch->counters;
     b.x = reinterpret_cast<const uint16_t*>(acts); b.x_stride = f;
     b.out = tf::byte_ptr(route_partials, route_partials_off); b.out_stride = d; b.rows = d; b.k = f; b.top_k = params->top_k;
-    if (tf_status s = tf::launch_grouped<1, false, tf::kOutPartialF16, 704>(ctx, stream, b, false, "tf_grouped_moe_streamed(down)")) return s;
+    if (tf_status s = tf::launch_grouped_down<tf::kOutPartialF16>(ctx, stream, b, params->pair_count, "tf_grouped_moe_streamed(down)")) return s;
     if (microbatches_out) *microbatches_out = (params->pair_count + pair_microbatch_rows - 1) / pair_microbatch_rows;
     return TF_OK;
 }
