@@ -97,10 +97,11 @@ struct RouterGroupOut {
     uint32_t* counters;
 };
 
+constexpr uint32_t kGroupPrefixWords = 16;           // 512 pairs: what the few-row router groups
 __host__ __device__ inline size_t router_group_smem_bytes(uint32_t n_pairs, uint32_t num_experts) {
     const uint32_t nw = (n_pairs + 31) / 32;
-    // mask, hist + offs, expert ids, warp totals (3 x 32), weights
-    return (size_t)num_experts * nw * 4 + (size_t)num_experts * 2 * 4 + (size_t)n_pairs * 4 + 96 * 4 + (size_t)((n_pairs + 1) / 2) * 4;
+    // mask, its prefix counts, hist + offs, expert ids, warp totals (3 x 32), weights
+    return (size_t)num_experts * nw * 4 + (nw > kGroupPrefixWords ? (size_t)((num_experts * nw + 1) / 2) * 4 : 0) + (size_t)num_experts * 2 * 4 + (size_t)n_pairs * 4 + 96 * 4 + (size_t)((n_pairs + 1) / 2) * 4;
 }
 
 __device__ inline void group_routes_in_block(const uint32_t* __restrict__ idx, const uint16_t* __restrict__ w, uint32_t T, uint32_t K,
@@ -112,6 +113,7 @@ __device__ inline void group_routes_in_block(const uint32_t* __restrict__ idx, c
     uint32_t* exs = offs + E;                                    // [n]
     uint32_t* wtot = exs + n;                                    // [3][32]: per-warp totals of the scan
     uint16_t* wts = reinterpret_cast<uint16_t*>(wtot + 96);      // [n]
+    uint16_t* pre = wts + ((n + 1u) & ~1u);                      // [E][nw]: pairs of the expert in the words before this one
     const uint32_t lane = threadIdx.x % kWarp, warp = threadIdx.x / kWarp, nwarps = blockDim.x / kWarp;
     // ids and weights (written by other blocks of this launch) travel while the bitmaps are cleared
     for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
@@ -130,6 +132,25 @@ __device__ inline void group_routes_in_block(const uint32_t* __restrict__ idx, c
         }
     }
     __syncthreads();
+    // Many words per expert: the counts before every word, a warp per expert (a thread per pair that adds up the words before
+    // its own took 20 us for 1600 pairs). A few words are added up on the spot.
+    const bool counted = nw > kGroupPrefixWords;
+    if (counted) {
+        for (uint32_t ex = warp; ex < E; ex += nwarps) {
+            uint32_t run = 0;
+            for (uint32_t base = 0; base < nw; base += kWarp) {
+                const uint32_t q = base + lane, c = q < nw ? (uint32_t)__popc(mask[(size_t)ex * nw + q]) : 0u;
+                uint32_t incl = c;
+#pragma unroll
+                for (int o = 1; o < kWarp; o <<= 1) {
+                    const uint32_t v = __shfl_up_sync(kFullMask, incl, o);
+                    if ((int)lane >= o) incl += v;
+                }
+                if (q < nw) pre[(size_t)ex * nw + q] = (uint16_t)(run + incl - c);
+                run += __shfl_sync(kFullMask, incl, kWarp - 1);
+            }
+        }
+    }
     // exclusive scans over the experts (pairs, non-empty groups, chunks): every warp scans 32 experts, the warps'
     // totals meet in shared memory, and rounds of nwarps * 32 experts carry the running totals.
     uint32_t off = 0, gi = 0, ch = 0;
@@ -175,9 +196,10 @@ __device__ inline void group_routes_in_block(const uint32_t* __restrict__ idx, c
         const uint32_t ex = exs[i];
         if (ex == 0xFFFFFFFFu) continue;
         const uint32_t* m = mask + (size_t)ex * nw;
-        uint32_t pos = offs[ex];
-        for (uint32_t q = 0; q < i / 32; ++q) pos += __popc(m[q]);
-        pos += __popc(m[i / 32] & ((1u << (i % 32)) - 1u));
+        uint32_t pos = offs[ex] + __popc(m[i / 32] & ((1u << (i % 32)) - 1u));
+        if (counted) pos += pre[(size_t)ex * nw + i / 32];
+        else
+            for (uint32_t q = 0; q < i / 32; ++q) pos += __popc(m[q]);
         out.sorted_pairs[pos] = tf_pair{i / K, ex, i % K, (uint32_t)wts[i]};
     }
 }
