@@ -26,6 +26,8 @@ ep_pack_kernel(const uint16_t* __restrict__ hidden, uint32_t hidden_stride, cons
                uint16_t* __restrict__ send_rows, uint32_t* __restrict__ send_ids, uint32_t* __restrict__ inverse_perm,
                uint32_t* __restrict__ overflow, const uint32_t* __restrict__ grouped_pairs) {
     __shared__ uint32_t dst_base[257], dst_count[256];
+    pdl_launch_dependents();
+    pdl_wait();
     if (n_dst > 1) {
         // pairs are sorted by expert, experts are contiguous per rank: dst_base = prefix of the counts
         if (threadIdx.x == 0) {
@@ -189,7 +191,7 @@ static tf_status pack_rows(tf_context* ctx, void* stream, const void* hidden, ui
     const uint32_t slots = capacity > 0 ? n_dst * capacity : n_pairs;
     const uint32_t per_block = tf::kPackThreads / tf::kWarp;
     auto kern = permute_k8 ? tf::ep_pack_kernel<true> : tf::ep_pack_kernel<false>;
-    kern<<<(slots + per_block - 1) / per_block, tf::kPackThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+    tf::launch_pdl(kern, dim3((slots + per_block - 1) / per_block), dim3(tf::kPackThreads), 0, static_cast<cudaStream_t>(stream),
         reinterpret_cast<const uint16_t*>(hp), hidden_stride_elements, routes->sorted_pairs, routes->per_expert_counts, n_pairs,
         top_k, num_experts, experts_per_rank, n_dst, capacity, d, send_stride, static_cast<uint16_t*>(send_rows), send_expert_ids,
         inverse_perm, ctx->device_error, routes->counters + 3);

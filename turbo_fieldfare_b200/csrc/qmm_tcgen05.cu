@@ -6,25 +6,31 @@
 // prefill_grouped_routed_moe_batched_phase1 / _down (Metal/Prefill/prefill.metal:598-670), which the
 // reference runs as scalar per-thread dot products.
 //
-//   D[128 weight rows x N tokens] += W_tile[128 x 128] . X_tile[N x 128]^T     per step of two 64-column groups, N <= 128
+//   D[128 weight rows x N tokens] += W_tile[128 x 256] . X_tile[N x 256]^T     per stage of four 64-column groups, N <= 128
 //
 // Weights are the A operand (M = 128) and are fed to the MMA from TENSOR MEMORY; tokens are the B operand
 // (N = the tile's token count rounded up to 16, carried in the instruction descriptor) in shared memory,
 // K-major with the 128-byte swizzle. Data path of the weights, which carry nearly all the bytes:
-//   HBM --TMA tile load--> shared memory (packed, 64 bytes per row and step)
+//   HBM --TMA tile load--> shared memory (packed, 128 bytes per row and stage)
 //       --LDS.128--> registers --one HFMA2 per two codes--> w = half(q * s + b)     (tensorops.metal:60-75)
 //       --tcgen05.st--> tensor memory --tcgen05.mma--> fp32 accumulators in tensor memory.
 // The dequantised tile never touches shared memory: an fp16 copy of the weights is four times the packed
 // bytes, and writing it to shared memory and reading it back for the MMA would cost more shared-memory
 // bandwidth than the whole HBM stream.
-// Roles of the 24 warps: warp 0 issues every asynchronous copy (packed codes per step, activation boxes of 16
-// or 128 rows per step, the tile's scale and bias planes as 1-D bulk copies); warp 1 issues the MMAs and commits
-// stages back through mbarriers; warps 4-19 dequantise (four threads per weight row); warps 20-23 read the
-// accumulators with tcgen05.ld and apply GeGLU (gate and up accumulate side by side) or a plain fp16 store,
-// masked to the group's real tokens. Accumulators of tiles with at most 64 tokens (one matrix: any tile)
-// alternate between two buffers so that the epilogue overlaps the next tile's MMAs.
+// A gate/up tile holds 64 gate rows over 64 up rows, so that one accumulator of 128 lanes carries both, 704 rows are eleven
+// whole tiles, and both forms of the kernel have one layout; the epilogue warps of the two halves exchange values.
+// Roles of the 24 warps: warps 0, 2 and 3 issue the copies of packed codes, of activations (boxes of 16 to 128 rows) and of
+// a tile's scale and bias planes (1-D bulk copies), warp 1 the MMAs, and commits stages back through mbarriers; warps 4-19
+// dequantise (a thread takes one group of one row per stage); warps 20-23 read the accumulators with tcgen05.ld, apply
+// GeGLU or nothing, and store through a staging tile as 16-byte words, masked to the group's real tokens.
+// Accumulators alternate between two buffers of 128 columns, so that the epilogue overlaps the next tile's MMAs.
 // A persistent grid walks (group, token tile, weight-row tile) work items derived on the device from the
-// routing metadata. Every mbarrier wait is bounded; on expiry the kernel records a code and leaves.
+// routing metadata. Every mbarrier wait is bounded; on expiry the kernel records a code, waits for its copies and leaves.
+//
+// What bounds it (clock counters around the waits, 4096 x 18944 x 2816, 1.14 PFLOP/s): with 128 tokens per tile the
+// activations, 64 bytes per clock and SM out of L2; with few tokens the dequantisers' integer instructions, about 700 clocks
+// per stage where an SM's share of the HBM rate gives 740. Each single-warp role pays 100 to 150 clocks per wait or commit
+// whatever N is, so a stage is as deep as tensor memory allows.
 //
 // Column order. The cheapest nibble extraction yields the eight codes of a 32-bit word in the order
 // (0,4,1,5,2,6,3,7). A dot product does not care about the order as long as both operands agree, so the
@@ -758,7 +764,20 @@ static uint32_t qmm_dense_per_tile(uint32_t tokens, uint32_t wrow_tiles, uint32_
     return best;
 }
 
-// W[m]: base of matrix m's packed plane for expert 0 (dense: the matrix itself); a.S, a.B likewise.
+// Fills a's group table (a.plan and the groups' source are set). The context has three: one for dense launches, which may run
+// on another stream at the same time, and one for each half of a routed pair, so that both can be filled before the first.
+constexpr int kQmmGateUpTable = 0, kQmmDownTable = 1, kQmmDenseTable = 2;
+static tf_status launch_qmm_prepare(tf_context* ctx, void* stream, QmmArgs& a, int table, const char* name) {
+    TF_REQUIRE(ctx, ctx->qmm_groups != nullptr, TF_ERR_OUT_OF_MEMORY, "%s: context scratch missing", name);
+    a.groups = static_cast<uint4*>(ctx->qmm_groups) + table * (TF_MAX_ROUTER_EXPERTS + 1);
+    a.totals = reinterpret_cast<uint32_t*>(a.groups + TF_MAX_ROUTER_EXPERTS);
+    launch_pdl(qmm_prepare_kernel, dim3(1), dim3(TF_MAX_ROUTER_EXPERTS), 0, static_cast<cudaStream_t>(stream), a.groups, a.totals,
+               a.route_groups, a.route_counters, a.dense_tokens, a.dense_per_tile, a.plan.tok_max);
+    return check_launch(ctx, "qmm_prepare");
+}
+
+// W[m]: base of matrix m's packed plane for expert 0 (dense: the matrix itself); a.S, a.B likewise. A routed launch's table
+// has been filled by the caller.
 template <int NMAT, bool NATURAL_K>
 static tf_status launch_qmm(tf_context* ctx, void* stream, QmmArgs& a, const void* x, uint64_t x_rows, uint32_t x_stride,
                             const uint8_t* const* W, uint64_t experts, uint64_t expert_stride, bool dense, const char* name) {
@@ -791,13 +810,8 @@ static tf_status launch_qmm(tf_context* ctx, void* stream, QmmArgs& a, const voi
     a.expert_stride = dense ? 0 : expert_stride;
     a.out_vec = aligned(a.out, 16) && a.out_stride % 8 == 0 ? 1u : 0u;
     a.error = ctx->device_error;
-    // one table for routed launches and one for dense ones, which may run on two streams at once
-    TF_REQUIRE(ctx, ctx->qmm_groups != nullptr, TF_ERR_OUT_OF_MEMORY, "%s: context scratch missing", name);
-    a.groups = static_cast<uint4*>(ctx->qmm_groups) + (dense ? TF_MAX_ROUTER_EXPERTS + 1 : 0);
-    a.totals = reinterpret_cast<uint32_t*>(a.groups + TF_MAX_ROUTER_EXPERTS);
-    launch_pdl(qmm_prepare_kernel, dim3(1), dim3(TF_MAX_ROUTER_EXPERTS), 0, static_cast<cudaStream_t>(stream), a.groups, a.totals,
-               a.route_groups, a.route_counters, a.dense_tokens, a.dense_per_tile, a.plan.tok_max);
-    if (tf_status s = check_launch(ctx, "qmm_prepare")) return s;
+    if (dense)
+        if (tf_status s = launch_qmm_prepare(ctx, stream, a, kQmmDenseTable, name)) return s;
     auto kern = qmm_tcgen05_kernel<NMAT, NATURAL_K>;
     static DeviceSmemCache configured;
     if (tf_status s = ensure_dynamic_smem(ctx, kern, configured, a.plan.total)) return s;
@@ -839,13 +853,18 @@ tf_status tf_grouped_moe_tensorcore(tf_context* ctx, void* stream, const void* x
     a.S[1] = plane(offsets->up_s_off);   a.B[1] = plane(offsets->up_b_off);
     a.route_groups = routes->groups; a.route_counters = routes->counters;
     a.rows = f; a.k = d; a.out = static_cast<uint16_t*>(acts_scratch); a.out_stride = f; a.round_gate_up = 0;
-    const uint8_t* w_gu[2] = {pool + offsets->gate_w_off, pool + offsets->up_w_off};
-    if (tf_status s = tf::launch_qmm<2, false>(ctx, stream, a, x_sorted, x_rows, d, w_gu, num_experts, expert_stride, false,
-                                                "tf_grouped_moe_tensorcore(gate/up)")) return s;
     tf::QmmArgs b{};
     b.S[0] = plane(offsets->down_s_off); b.B[0] = plane(offsets->down_b_off);
     b.route_groups = routes->groups; b.route_counters = routes->counters;
     b.rows = d; b.k = f; b.out = static_cast<uint16_t*>(out_rows); b.out_stride = d;
+    // both tables first: between the two GEMMs the second one's would wait for the first to end
+    TF_REQUIRE(ctx, tf::qmm_plan(d, 2, &a.plan) && tf::qmm_plan(f, 1, &b.plan), TF_ERR_UNSUPPORTED,
+               "%s: D=%u or F=%u needs more shared memory for the scale planes than there is", name, d, f);
+    if (tf_status s = tf::launch_qmm_prepare(ctx, stream, a, tf::kQmmGateUpTable, name)) return s;
+    if (tf_status s = tf::launch_qmm_prepare(ctx, stream, b, tf::kQmmDownTable, name)) return s;
+    const uint8_t* w_gu[2] = {pool + offsets->gate_w_off, pool + offsets->up_w_off};
+    if (tf_status s = tf::launch_qmm<2, false>(ctx, stream, a, x_sorted, x_rows, d, w_gu, num_experts, expert_stride, false,
+                                                "tf_grouped_moe_tensorcore(gate/up)")) return s;
     const uint8_t* w_dn[2] = {pool + offsets->down_w_off, pool + offsets->down_w_off};
     return tf::launch_qmm<1, false>(ctx, stream, b, acts_scratch, x_rows, f, w_dn, num_experts, expert_stride, false,
                                     "tf_grouped_moe_tensorcore(down)");

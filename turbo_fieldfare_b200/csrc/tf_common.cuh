@@ -65,8 +65,8 @@ struct tf_context {
     uint32_t step_trace_capacity = 0;
     // Per-slice expert histograms and start positions of the grouping of many pairs (grouped.cu): 2 x 256 slices x 256 experts.
     uint32_t* group_scratch = nullptr;
-    // Group tables of the tensor-core grouped GEMM (filled on the device per launch): one for routed launches and one for
-    // dense launches, which may run on two streams at once; each TF_MAX_ROUTER_EXPERTS rows of 16 bytes and a row of totals.
+    // Group tables of the tensor-core grouped GEMM (filled on the device per launch): two for a routed pair of launches and one
+    // for dense ones, which may run on two streams at once; each TF_MAX_ROUTER_EXPERTS rows of 16 bytes and a row of totals.
     void* qmm_groups = nullptr;
     // Side stream and fork/join events: the shared expert of a block runs beside its router and routed experts.
     cudaStream_t side_stream = nullptr;
