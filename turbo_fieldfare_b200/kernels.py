@@ -39,7 +39,8 @@ def _ptr(t) -> int | None:
 
 def _stream(stream) -> int:
     if stream is None:
-        return torch.cuda.current_stream().cuda_stream
+        # the raw handle of the current stream; a Stream object per call costs more than a microsecond
+        return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
     if isinstance(stream, torch.cuda.Stream):
         return stream.cuda_stream
     return int(stream)
@@ -82,7 +83,7 @@ class TurboContext:
 
     def set_router_tensorcore_min_rows(self, rows: int) -> None:
         """Router calls over at least ``rows`` rows compute all logits on the tensor cores and re-check the candidates in
-        the canonical order (default 256; 0xFFFFFFFF keeps the one-launch kernel)."""
+        the canonical order (default 65; 0xFFFFFFFF keeps the one-launch kernel)."""
         self.check(self.lib.tf_context_set_router_tensorcore_min_rows(self.handle, rows))
 
     def set_single_launch_step(self, enabled: bool) -> None:
