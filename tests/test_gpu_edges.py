@@ -1,0 +1,155 @@
+"""Edges of the tiles and of the dispatch rules of the kernels behind the block: token tiles of the tensor-core GEMM, the
+few-row router, chunks of 16 tokens against chunks of 8, and the 16-row tiles of the one-token kernels."""
+import numpy as np
+import pytest
+
+from tests.helpers import config0_matrix, dev_zeros_u16, from_dev, to_dev
+
+pytestmark = pytest.mark.gpu
+
+
+def _dense(o, mat):
+    """The matrix in 64 bits."""
+    q = np.empty((mat.packed.shape[0], mat.packed.shape[1] * 2), np.float64)
+    q[:, 0::2], q[:, 1::2] = mat.packed & 15, mat.packed >> 4
+    s, b = (np.repeat(o.bf16_to_f32(p).astype(np.float64), 64, axis=1) for p in (mat.scales, mat.biases))
+    return q * s + b
+
+
+# K: one group, an odd last group, whole and partial stages of four groups; N: below, at and beyond a 128-row tile; M: tiles of
+# one MMA step, of unequal last steps, exactly full, and several of equal size. y_off = 2 takes the element stores.
+@pytest.mark.parametrize("M,N,K,y_off", [(1, 8, 64, 0), (15, 72, 128, 0), (16, 128, 192, 2), (17, 136, 320, 0), (63, 256, 704, 0), (65, 128, 2112, 2),
+                                         (113, 264, 448, 0), (128, 2112, 256, 0), (129, 128, 2816, 0), (270, 384, 704, 0), (1000, 40, 4096, 0),
+                                         (300, 64, 8192, 0)])
+def test_qmm_token_tiles(tf_ctx, oracle, M, N, K, y_off):
+    import torch
+    from turbo_fieldfare_b200.kernels import MPPPrefillInt4QMM
+    o = oracle
+    rng = np.random.default_rng(M + 3 * N + 7 * K)
+    mat = config0_matrix(o, N, K, rng)
+    x16 = o.f32_to_f16(rng.standard_normal((M, K)).astype(np.float32))
+    y = dev_zeros_u16(M * N + 16, fill=0x7E00)
+    MPPPrefillInt4QMM(tf_ctx).encode(to_dev(mat.packed), to_dev(mat.scales), to_dev(mat.biases), to_dev(x16), y, M, N, K, y_offset=y_off)
+    torch.cuda.synchronize()
+    assert tf_ctx.device_status() == 0
+    out = from_dev(y, np.uint16)
+    got = o.f16_to_f32(out[y_off // 2:y_off // 2 + M * N]).reshape(M, N)
+    assert np.all(out[:y_off // 2] == 0x7E00) and np.all(out[y_off // 2 + M * N:] == 0x7E00)      # nothing beyond the result
+    # weights and results rounded to fp16: 2^-11 each, a third of it in the root mean square
+    assert o.rel_l2(got, o.f16_to_f32(x16).astype(np.float64) @ _dense(oracle, mat).T) < 1e-3
+
+
+@pytest.mark.parametrize("rows", [65, 200, 255, 256, 297, 593, 1184, 1185])
+def test_few_row_router_equals_the_one_launch_kernel(tf_ctx, oracle, rows):
+    """Indices, weights and (up to 255 rows) the grouping tables of the small-tile pass with eight, four, two or one warp per
+    token in the re-check: byte for byte those of the kernel that computes every canonical logit, and of the grouping launch."""
+    import torch
+    from turbo_fieldfare_b200.kernels import DeviceRoutes, PrefillGroupedRoutedMoE, PrefillRouter
+    o = oracle
+    E, D, K = 128, 2816, 8
+    rng = np.random.default_rng(rows)
+    mat = config0_matrix(o, E, D, rng, bits=8)
+    mat.packed[7], mat.scales[7], mat.biases[7] = mat.packed[3], mat.scales[3], mat.biases[3]       # exact ties
+    W, S, B = to_dev(mat.packed), to_dev(mat.scales), to_dev(mat.biases)
+    x = rng.standard_normal((rows, D)).astype(np.float32)
+    x[1, 5] = np.nan
+    x[2] *= 1e-4
+    hid = to_dev(o.f32_to_f16(x))
+    eff, gain = to_dev(o.f32_to_bf16(np.full(D, D ** -0.5, np.float32))), to_dev(o.f32_to_bf16(np.ones(E, np.float32)))
+
+    def run(min_rows):
+        tf_ctx.set_router_tensorcore_min_rows(min_rows)
+        idx, w, routes = torch.full((rows, K), -1, dtype=torch.int32, device="cuda"), dev_zeros_u16(rows * K), DeviceRoutes(rows, K, E)
+        PrefillRouter(tf_ctx).encode_gemma4_block_grouped(W, S, B, hid, eff, gain, idx, w, rows, E, D, K, D, routes)
+        ref = DeviceRoutes(rows, K, E)
+        PrefillGroupedRoutedMoE(tf_ctx).encode_group_routes(idx, w, rows, K, E, ref)
+        torch.cuda.synchronize()
+        assert torch.equal(routes.sorted_pairs, ref.sorted_pairs) and torch.equal(routes.per_expert_counts, ref.per_expert_counts)
+        assert torch.equal(routes.per_expert_offsets, ref.per_expert_offsets) and torch.equal(routes.counters[:2], ref.counters[:2])
+        return from_dev(idx, np.uint32), from_dev(w, np.uint16)
+
+    try:
+        one, two, again = run(0xFFFFFFFF), run(65), run(65)
+    finally:
+        tf_ctx.set_router_tensorcore_min_rows(256)
+    for got in (two, again):
+        assert np.array_equal(got[0], one[0]) and np.array_equal(got[1], one[1])
+
+
+@pytest.fixture(scope="module")
+def layer(tf_ctx):
+    from turbo_fieldfare_b200.stack import ExpertPool, MoEBlockLayer
+    pool = ExpertPool(tf_ctx, 1, 128, 2816, 704)
+    pool.fill_synthetic(11)
+    layer = MoEBlockLayer(tf_ctx, pool, 0, 2816, 704, 2112, 128, 8)
+    layer.fill_synthetic(12)
+    yield layer
+    pool.close()
+
+
+def _forward(tf_ctx, layer, ws, x):
+    import torch
+    from turbo_fieldfare_b200.stack import MoEBlock
+    y = torch.zeros_like(x)
+    MoEBlock(tf_ctx, layer).forward(x, y, x.shape[0], ws)
+    torch.cuda.synchronize()
+    assert tf_ctx.device_status() == 0
+    return y
+
+
+# 103 / 104 tokens lie on either side of the rule for 16-token chunks; a bias towards few experts gives them chunks of every fill
+@pytest.mark.parametrize("tokens,skew", [(103, 0.0), (104, 0.0), (128, 4.0), (255, 0.0), (255, 8.0)])
+def test_wide_chunks_equal_narrow_ones(tf_ctx, layer, tokens, skew):
+    """A token's sums do not depend on the chunk that it sits in: a block of many tokens has the bits of the same tokens in
+    blocks of 40, whose experts' rows (and the shared expert's) are taken eight at a time or in other places."""
+    import torch
+    from turbo_fieldfare_b200.stack import Workspace
+    bias = np.zeros(128, np.float32)
+    bias[[3, 60, 127]] = skew
+    layer.set_logit_bias(bias)
+    try:
+        gen = torch.Generator(device="cuda").manual_seed(tokens)
+        x = torch.randn(tokens, 2816, generator=gen, device="cuda").half()
+        ws = Workspace(tf_ctx, tokens, 2816, 704, 2112, 8, 128)
+        whole = _forward(tf_ctx, layer, ws, x)
+        parts = torch.cat([_forward(tf_ctx, layer, ws, x[i:i + 40].contiguous()) for i in range(0, tokens, 40)])
+        eight = torch.cat([_forward(tf_ctx, layer, ws, x[i:i + 7].contiguous()) for i in range(0, min(tokens, 63), 7)])
+        assert torch.equal(whole, parts)
+        assert torch.equal(whole[:eight.shape[0]], eight)
+    finally:
+        layer.set_logit_bias(None)
+
+
+def test_one_token_block_equals_its_row_in_a_pair(tf_ctx, layer):
+    """The one-token kernels against the grouped ones. Both add exact products in fp32, in an order of their own; the grouped
+    ones hold odd activations at 1/16 (below 2^-10 that costs up to 2^-25 each): within two fp16 roundings of each other."""
+    import torch
+    from turbo_fieldfare_b200.stack import Workspace
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    x = torch.randn(2, 2816, generator=gen, device="cuda").half()
+    ws = Workspace(tf_ctx, 2, 2816, 704, 2112, 8, 128)
+    pair = _forward(tf_ctx, layer, ws, x)
+    for i in range(2):
+        one = _forward(tf_ctx, layer, ws, x[i:i + 1].contiguous())
+        assert (one[0].double() - pair[i].double()).norm() / pair[i].double().norm() < 1e-3
+
+
+@pytest.mark.parametrize("scale", [1.0, 1e-4])
+@pytest.mark.parametrize("m,n", [(1, 64), (15, 128), (16, 192), (17, 2112), (704, 2816), (4095, 320), (33, 16384)])
+def test_tile_gemv(tf_ctx, oracle, m, n, scale):
+    """Remainders of the 16-row tile and of the four-group part; small activations keep their bits."""
+    import torch
+    from turbo_fieldfare_b200.kernels import DequantInt4GEMV
+    o = oracle
+    rng = np.random.default_rng(m * 5 + n)
+    mat = config0_matrix(o, m, n, rng)
+    x16 = o.f32_to_f16((rng.standard_normal(n) * scale).astype(np.float32))
+    y = dev_zeros_u16(m + 8, fill=0x7E00)
+    DequantInt4GEMV(tf_ctx).encode(to_dev(mat.packed), to_dev(mat.scales), to_dev(mat.biases), to_dev(x16), y, m, n)
+    torch.cuda.synchronize()
+    out = from_dev(y, np.uint16)
+    assert np.all(out[m:] == 0x7E00)
+    ref = _dense(o, mat) @ o.f16_to_f32(x16).astype(np.float64)
+    # the result's rounding (2^-11, or half a subnormal step) and fp32 sums of up to 16384 products
+    bound = np.abs(ref) * 2.0 ** -11 + 2.0 ** -25 + (np.abs(_dense(o, mat)) + 0.1) @ np.abs(o.f16_to_f32(x16).astype(np.float64)) * 2.0 ** -20
+    assert np.all(np.abs(o.f16_to_f32(out[:m]) - ref) <= bound)
