@@ -15,7 +15,7 @@ bool gemv_mma_eligible(const void* W, const void* S, const void* B, const void* 
 tf_status launch_gemv_mma(tf_context* ctx, void* stream, const uint8_t* W, const uint16_t* S, const uint16_t* B,
                           const uint16_t* x, uint16_t* y, uint32_t m, uint32_t n, bool sb_fp16, const char* name);
 tf_status launch_gemv_mma_argmax(tf_context* ctx, void* stream, const uint8_t* W, const uint16_t* S, const uint16_t* B,
-                                 const uint16_t* x, uint32_t m, uint32_t n, unsigned long long* argmax, uint32_t* out_token, const char* name);
+                                 const uint16_t* x, uint32_t m, uint32_t n, unsigned long long* argmax, const char* name);
 tf_status launch_gemv_mma_batched(tf_context* ctx, void* stream, const uint8_t* W, const uint16_t* S, const uint16_t* B,
                                   uint64_t plane_stride, const uint16_t* x, uint32_t x_stride, uint16_t* y, uint32_t y_stride,
                                   uint32_t m, uint32_t n, uint32_t count, bool sb_fp16, const char* name);
@@ -188,6 +188,7 @@ lm_head_argmax_kernel(const float* __restrict__ logits, uint32_t vocab, unsigned
 // Decodes the winner (0 when no logit was finite, lm_head_greedy_int4_rows_reduce's fallback) and clears the
 // scratch word for the next call.
 __global__ void lm_head_finish_kernel(unsigned long long* __restrict__ best, uint32_t* __restrict__ out_token) {
+    pdl_wait();
     const unsigned long long k = *best;
     *out_token = k ? ~(uint32_t)(k & 0xFFFFFFFFull) : 0u;
     *best = 0ull;
@@ -212,8 +213,8 @@ tf_status tf_lm_head_greedy_int4(tf_context* ctx, void* stream, const void* hidd
     TF_REQUIRE(ctx, tf::aligned(out_token, 4), TF_ERR_ALIGNMENT, "%s: outToken must be 4-byte aligned", name);
     // scratch owned by the context; growing it allocates (and so cannot happen inside a stream capture)
     if (ctx->lm_best == nullptr) {
-        TF_CUDA(ctx, cudaMalloc(&ctx->lm_best, 2 * sizeof(unsigned long long)));
-        TF_CUDA(ctx, cudaMemset(ctx->lm_best, 0, 2 * sizeof(unsigned long long)));
+        TF_CUDA(ctx, cudaMalloc(&ctx->lm_best, sizeof(unsigned long long)));
+        TF_CUDA(ctx, cudaMemset(ctx->lm_best, 0, sizeof(unsigned long long)));
     }
     if (d > ctx->lm_x_capacity) {
         if (ctx->lm_x) { TF_CUDA(ctx, cudaFree(ctx->lm_x)); ctx->lm_x = nullptr; ctx->lm_x_capacity = 0; }
@@ -230,19 +231,22 @@ tf_status tf_lm_head_greedy_int4(tf_context* ctx, void* stream, const void* hidd
     }
     tf_status st = tf_rmsnorm(ctx, stream, hidden, hidden_off, norm_weight_bf16, norm_off, ctx->lm_x, 0, 1, d, d, rms_eps, TF_FP16);
     if (st != TF_OK) return st;
-    if (streamed)
-        return tf::launch_gemv_mma_argmax(ctx, stream, wp, reinterpret_cast<const uint16_t*>(sp), reinterpret_cast<const uint16_t*>(bp), ctx->lm_x,
-                                          vocab, d, ctx->lm_best, out_token, name);
-    st = tf::launch_gemv<4, true>(ctx, stream, weights, weights_off, scales, scales_off, biases, biases_off, ctx->lm_x, 0,
-                                  ctx->lm_logits, 0, vocab, d, TF_BF16, name);
-    if (st != TF_OK) return st;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const uint32_t want = (vocab + tf::kArgmaxThreads - 1) / tf::kArgmaxThreads;
-    const uint32_t grid = want < (uint32_t)ctx->sm_count ? want : (uint32_t)ctx->sm_count;
-    tf::lm_head_argmax_kernel<<<grid, tf::kArgmaxThreads, 0, s>>>(ctx->lm_logits, vocab, ctx->lm_best);
-    st = tf::check_launch(ctx, name);
-    if (st != TF_OK) return st;
-    tf::lm_head_finish_kernel<<<1, 1, 0, s>>>(ctx->lm_best, out_token);
+    if (streamed) {
+        st = tf::launch_gemv_mma_argmax(ctx, stream, wp, reinterpret_cast<const uint16_t*>(sp), reinterpret_cast<const uint16_t*>(bp), ctx->lm_x,
+                                        vocab, d, ctx->lm_best, name);
+        if (st != TF_OK) return st;
+    } else {
+        st = tf::launch_gemv<4, true>(ctx, stream, weights, weights_off, scales, scales_off, biases, biases_off, ctx->lm_x, 0,
+                                      ctx->lm_logits, 0, vocab, d, TF_BF16, name);
+        if (st != TF_OK) return st;
+        const uint32_t want = (vocab + tf::kArgmaxThreads - 1) / tf::kArgmaxThreads;
+        const uint32_t grid = want < (uint32_t)ctx->sm_count ? want : (uint32_t)ctx->sm_count;
+        tf::lm_head_argmax_kernel<<<grid, tf::kArgmaxThreads, 0, s>>>(ctx->lm_logits, vocab, ctx->lm_best);
+        st = tf::check_launch(ctx, name);
+        if (st != TF_OK) return st;
+    }
+    tf::launch_pdl(tf::lm_head_finish_kernel, dim3(1), dim3(1), 0, s, ctx->lm_best, out_token);
     return tf::check_launch(ctx, name);
 }
 

@@ -34,14 +34,15 @@ __device__ __forceinline__ unsigned long long argmax_key(float z, uint32_t row) 
 }
 
 // What becomes of the row sums: stored as fp16, or (the greedy LM head) only the largest fp32 one is kept. ARGMAX: the launch
-// follows the call's own norm kernel and nothing else, so weights are requested before that kernel has ended; every block
-// folds its rows into argmax[0] (ordered logit << 32 | ~row) and the last one (argmax[1] counts) decodes the token and
-// clears both. Storing 262144 logits, a second kernel over them and a third to decode took 8 us.
+// follows the call's own norm kernel and nothing else, so weights are requested before that kernel has ended, and every block
+// folds its rows into *argmax (ordered logit << 32 | ~row) without waiting for the result. Storing 262144 logits and a second
+// kernel over them took 6 us; a count of finished blocks that lets the last one decode the token held every block up for a
+// fence and an atomic's return, longer than a third launch of one thread.
 template <bool SB_FP16, bool ARGMAX, int WARPS>
 __global__ void __launch_bounds__(WARPS * kWarp)
 gemv_mma_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S, const uint16_t* __restrict__ B,
                 const uint16_t* __restrict__ x, uint16_t* __restrict__ y, uint32_t m, uint32_t n, const GemvBatch bt,
-                unsigned long long* argmax, uint32_t* out_token) {
+                unsigned long long* argmax) {
     extern __shared__ __align__(16) uint8_t smem[];
     constexpr int kGmRows = WARPS * 16, kGmThreads = WARPS * kWarp;
     {
@@ -186,14 +187,6 @@ gemv_mma_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S, c
 #pragma unroll
             for (int w = 1; w < WARPS; ++w) mine = per_warp[w] > mine ? per_warp[w] : mine;
             if (mine) atomicMax(argmax, mine);
-            __threadfence();
-            if (atomicAdd(argmax + 1, 1ull) == gridDim.x - 1) {
-                __threadfence();
-                const unsigned long long k = atomicMax(argmax, 0ull);
-                *out_token = k ? ~(uint32_t)(k & 0xFFFFFFFFull) : 0u;      // 0 when no logit was finite
-                argmax[0] = 0ull;                                        // ready for the next call
-                argmax[1] = 0ull;
-            }
         }
     } else if (t == 0) {
         if (r0 < m) y[r0] = __half_as_ushort(__float2half_rn(acc0));
@@ -220,21 +213,22 @@ tf_status launch_gemv_mma(tf_context* ctx, void* stream, const uint8_t* W, const
     static DeviceSmemCache configured[2];
     if (tf_status st = ensure_dynamic_smem(ctx, k, configured[sb_fp16 ? 1 : 0], smem)) return st;
     launch_pdl(k, dim3((m + kGmWarps * 16 - 1) / (kGmWarps * 16)), dim3(kGmWarps * kWarp), smem, static_cast<cudaStream_t>(stream), W, S, B, x, y,
-               m, n, GemvBatch{0, 0, 0}, nullptr, nullptr);
+               m, n, GemvBatch{0, 0, 0}, nullptr);
     return check_launch(ctx, name);
 }
 
-// The greedy LM head's product: argmax points to two 64-bit words, zero before and after. Must follow, on the stream, the
+// The greedy LM head's product: *argmax is zero before. Must follow, on the stream, the
 // launch that writes x, and that launch must start after everything before it (no programmatic launch of its own).
-// Blocks of 64 rows: 4096 of them for 262144 rows, so that the last round of blocks is a small part of the whole.
+// Blocks of 128 rows, as for the stored form: with 64 rows the staging of x and the scales weighs twice (95 against 89 us for
+// 262144 rows, cold).
 tf_status launch_gemv_mma_argmax(tf_context* ctx, void* stream, const uint8_t* W, const uint16_t* S, const uint16_t* B,
-                                 const uint16_t* x, uint32_t m, uint32_t n, unsigned long long* argmax, uint32_t* out_token, const char* name) {
-    const size_t smem = gemv_mma_smem_bytes_for(n, kGmBatchWarps);
-    auto k = gemv_mma_kernel<false, true, kGmBatchWarps>;
+                                 const uint16_t* x, uint32_t m, uint32_t n, unsigned long long* argmax, const char* name) {
+    const size_t smem = gemv_mma_smem_bytes(n);
+    auto k = gemv_mma_kernel<false, true, kGmWarps>;
     static DeviceSmemCache configured;
     if (tf_status st = ensure_dynamic_smem(ctx, k, configured, smem)) return st;
-    launch_pdl(k, dim3((m + kGmBatchWarps * 16 - 1) / (kGmBatchWarps * 16)), dim3(kGmBatchWarps * kWarp), smem, static_cast<cudaStream_t>(stream),
-               W, S, B, x, nullptr, m, n, GemvBatch{0, 0, 0}, argmax, out_token);
+    launch_pdl(k, dim3((m + kGmWarps * 16 - 1) / (kGmWarps * 16)), dim3(kGmWarps * kWarp), smem, static_cast<cudaStream_t>(stream),
+               W, S, B, x, nullptr, m, n, GemvBatch{0, 0, 0}, argmax);
     return check_launch(ctx, name);
 }
 
@@ -254,7 +248,7 @@ tf_status launch_gemv_mma_batched(tf_context* ctx, void* stream, const uint8_t* 
             W + (size_t)first * plane_stride,
             reinterpret_cast<const uint16_t*>(reinterpret_cast<const uint8_t*>(S) + (size_t)first * plane_stride),
             reinterpret_cast<const uint16_t*>(reinterpret_cast<const uint8_t*>(B) + (size_t)first * plane_stride),
-            x + (size_t)first * x_stride, y + (size_t)first * y_stride, m, n, GemvBatch{plane_stride, x_stride, y_stride}, nullptr, nullptr);
+            x + (size_t)first * x_stride, y + (size_t)first * y_stride, m, n, GemvBatch{plane_stride, x_stride, y_stride}, nullptr);
         if (tf_status st = check_launch(ctx, name)) return st;
     }
     return TF_OK;
