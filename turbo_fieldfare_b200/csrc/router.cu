@@ -182,7 +182,7 @@ router_split_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ 
             }
         }
         if (__syncthreads_or(repeated)) {
-            group_routes_in_block(out_idx, out_w, 1, top_k, num_experts, grp, smem);
+            group_routes_in_block<false>(out_idx, out_w, 1, top_k, num_experts, grp, smem);
             return;
         }
         for (uint32_t e = threadIdx.x; e < num_experts; e += blockDim.x) {
@@ -225,7 +225,7 @@ router_split_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ 
     __syncthreads();
     if (!is_last) return;
     __threadfence();
-    group_routes_in_block(out_idx, out_w, gridDim.x, top_k, num_experts, grp, smem);
+    group_routes_in_block<false>(out_idx, out_w, gridDim.x, top_k, num_experts, grp, smem);
 }
 
 // A handful of rows (batched decode, 2...kRouterSplitRows): grid (rows / R, experts / 8). A block stages R activation
@@ -362,7 +362,7 @@ router_rows_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S
     __syncthreads();
     if (!is_last) return;
     __threadfence();
-    group_routes_in_block(out_idx, out_w, rows, top_k, num_experts, grp, smem);
+    group_routes_in_block<false>(out_idx, out_w, rows, top_k, num_experts, grp, smem);
 }
 
 // Many rows (batched decode, prefill): one block per row.
@@ -574,7 +574,7 @@ static tf_status launch_router(tf_context* ctx, void* stream, const uint8_t* W, 
         RouterGroupOut grp{};
         if (routes) {
             grp = router_group_out(routes);
-            const size_t need = router_group_smem_bytes(rows * top_k, num_experts);
+            const size_t need = router_group_smem_bytes(rows * top_k, num_experts, false);
             if (need > smem_rows) smem_rows = need;
         }
         TF_REQUIRE(ctx, smem_rows <= 200 * 1024, TF_ERR_UNSUPPORTED, "%s: D=%u too large", name, d);
@@ -592,7 +592,7 @@ static tf_status launch_router(tf_context* ctx, void* stream, const uint8_t* W, 
         RouterGroupOut grp{};
         if (routes) {
             grp = router_group_out(routes);
-            const size_t need = router_group_smem_bytes(rows * top_k, num_experts);
+            const size_t need = router_group_smem_bytes(rows * top_k, num_experts, false);
             if (need > smem_split) smem_split = need;
         }
         TF_REQUIRE(ctx, smem_split <= 200 * 1024, TF_ERR_UNSUPPORTED, "%s: D=%u too large", name, d);
@@ -643,7 +643,7 @@ static tf_status launch_router(tf_context* ctx, void* stream, const uint8_t* W, 
         RouterGroupOut grp{};
         if (routes) {
             grp = router_group_out(routes);
-            const size_t need = router_group_smem_bytes(rows * top_k, num_experts);
+            const size_t need = router_group_smem_bytes(rows * top_k, num_experts, true);
             if (need > smem_r) smem_r = need;
         }
         static DeviceSmemCache configured_recheck[4][4];

@@ -21,10 +21,10 @@ __device__ __forceinline__ uint32_t topk_score_key(float v) {
 __device__ __forceinline__ float topk_key_score(uint32_t k) {
     return __uint_as_float((k & 0x80000000u) ? (k & 0x7FFFFFFFu) : ~k);
 }
-__device__ __forceinline__ void warp_select_topk(const float* scores /*shared*/, uint32_t num_experts, uint32_t top_k,
-                                                 const uint16_t* __restrict__ per_expert_scale,
-                                                 uint32_t* __restrict__ out_idx, uint16_t* __restrict__ out_w, int lane) {
-    constexpr int kPerLane = TF_MAX_ROUTER_EXPERTS / kWarp;
+template <int kPerLane>        // experts per lane: num_experts <= 32 * kPerLane
+__device__ __forceinline__ void warp_select_topk_held(const float* scores /*shared*/, uint32_t num_experts, uint32_t top_k,
+                                                      const uint16_t* __restrict__ per_expert_scale,
+                                                      uint32_t* __restrict__ out_idx, uint16_t* __restrict__ out_w, int lane) {
     uint32_t key[kPerLane];
 #pragma unroll
     for (int j = 0; j < kPerLane; ++j) {
@@ -63,6 +63,15 @@ __device__ __forceinline__ void warp_select_topk(const float* scores /*shared*/,
     }
 }
 
+// Half of the comparisons of every round for up to 128 experts.
+__device__ __forceinline__ void warp_select_topk(const float* scores /*shared*/, uint32_t num_experts, uint32_t top_k,
+                                                 const uint16_t* __restrict__ per_expert_scale,
+                                                 uint32_t* __restrict__ out_idx, uint16_t* __restrict__ out_w, int lane) {
+    static_assert(TF_MAX_ROUTER_EXPERTS == 8 * kWarp, "eight experts per lane at the most");
+    if (num_experts <= 4u * kWarp) warp_select_topk_held<4>(scores, num_experts, top_k, per_expert_scale, out_idx, out_w, lane);
+    else warp_select_topk_held<8>(scores, num_experts, top_k, per_expert_scale, out_idx, out_w, lane);
+}
+
 // Canonical logit of one expert row whose bytes, scales and biases sit in shared memory
 // (same arithmetic and order as router_row_logit; only the operand source differs).
 __device__ __forceinline__ float router_row_logit_smem(const uint8_t* Wrow, const uint16_t* s_row, const uint16_t* b_row,
@@ -97,14 +106,16 @@ struct RouterGroupOut {
     uint32_t* counters;
 };
 
-constexpr uint32_t kGroupPrefixWords = 16;           // 512 pairs: what the few-row router groups
-__host__ __device__ inline size_t router_group_smem_bytes(uint32_t n_pairs, uint32_t num_experts) {
+__host__ __device__ inline size_t router_group_smem_bytes(uint32_t n_pairs, uint32_t num_experts, bool counted) {
     const uint32_t nw = (n_pairs + 31) / 32;
     // mask, its prefix counts, hist + offs, expert ids, warp totals (3 x 32), weights
-    return (size_t)num_experts * nw * 4 + (nw > kGroupPrefixWords ? (size_t)((num_experts * nw + 1) / 2) * 4 : 0) + (size_t)num_experts * 2 * 4 + (size_t)n_pairs * 4 + 96 * 4 + (size_t)((n_pairs + 1) / 2) * 4;
+    return (size_t)num_experts * nw * 4 + (counted ? (size_t)((num_experts * nw + 1) / 2) * 4 : 0) + (size_t)num_experts * 2 * 4 + (size_t)n_pairs * 4 + 96 * 4 + (size_t)((n_pairs + 1) / 2) * 4;
 }
 
-__device__ inline void group_routes_in_block(const uint32_t* __restrict__ idx, const uint16_t* __restrict__ w, uint32_t T, uint32_t K,
+// COUNTED (more than 512 pairs): the counts before every bitmap word are taken first, a warp per expert (a thread per pair that
+// adds up the words before its own took 20 us for 1600 pairs); otherwise a few words are added up on the spot.
+template <bool COUNTED>
+__device__ __forceinline__ void group_routes_in_block(const uint32_t* __restrict__ idx, const uint16_t* __restrict__ w, uint32_t T, uint32_t K,
                                       uint32_t E, const RouterGroupOut& out, uint8_t* smem) {
     const uint32_t n = T * K, nw = (n + 31) / 32;
     uint32_t* mask = reinterpret_cast<uint32_t*>(smem);          // [E][nw]
@@ -132,10 +143,7 @@ __device__ inline void group_routes_in_block(const uint32_t* __restrict__ idx, c
         }
     }
     __syncthreads();
-    // Many words per expert: the counts before every word, a warp per expert (a thread per pair that adds up the words before
-    // its own took 20 us for 1600 pairs). A few words are added up on the spot.
-    const bool counted = nw > kGroupPrefixWords;
-    if (counted) {
+    if constexpr (COUNTED) {
         for (uint32_t ex = warp; ex < E; ex += nwarps) {
             uint32_t run = 0;
             for (uint32_t base = 0; base < nw; base += kWarp) {
@@ -197,9 +205,11 @@ __device__ inline void group_routes_in_block(const uint32_t* __restrict__ idx, c
         if (ex == 0xFFFFFFFFu) continue;
         const uint32_t* m = mask + (size_t)ex * nw;
         uint32_t pos = offs[ex] + __popc(m[i / 32] & ((1u << (i % 32)) - 1u));
-        if (counted) pos += pre[(size_t)ex * nw + i / 32];
-        else
+        if constexpr (COUNTED) {
+            pos += pre[(size_t)ex * nw + i / 32];
+        } else {
             for (uint32_t q = 0; q < i / 32; ++q) pos += __popc(m[q]);
+        }
         out.sorted_pairs[pos] = tf_pair{i / K, ex, i % K, (uint32_t)wts[i]};
     }
 }

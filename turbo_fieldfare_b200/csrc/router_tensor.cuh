@@ -604,7 +604,7 @@ router_recheck_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict_
     __syncthreads();
     if (!is_last) return;
     __threadfence();
-    group_routes_in_block(out_idx, out_w, rows, top_k, num_experts, grp, smem);
+    group_routes_in_block<true>(out_idx, out_w, rows, top_k, num_experts, grp, smem);
 }
 
 }  // namespace tf
