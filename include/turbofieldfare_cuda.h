@@ -145,7 +145,7 @@ tf_status tf_context_set_tensorcore_min_tokens(tf_context* ctx, uint32_t tokens)
  * Default 256, like the routed experts: measured at 8, 16, 32 and 64 tokens the streaming kernels were faster
  * (1.07 ms against 1.22 ms for six layers at 64 tokens). */
 tf_status tf_context_set_shared_tensorcore_min_tokens(tf_context* ctx, uint32_t tokens);
-/* Router calls over at least `rows` rows (default 65) take two launches: every logit on the tensor cores with a bound
+/* Router calls over at least `rows` rows (default 256) take two launches: every logit on the tensor cores with a bound
  * on its distance from the canonical fp32 value, then the canonical logit (the reference's order of operations,
  * Metal/MoE/moe.metal:135-185) of the experts that can still reach the top k, typically top_k + 1 or 2 of them.
  * Indices and weights are those of the one-launch kernels bit for bit. UINT32_MAX keeps the one-launch kernel. Calls

@@ -41,8 +41,8 @@ def test_qmm_token_tiles(tf_ctx, oracle, M, N, K, y_off):
 
 @pytest.mark.parametrize("rows", [65, 200, 255, 256, 297, 593, 1184, 1185])
 def test_few_row_router_equals_the_one_launch_kernel(tf_ctx, oracle, rows):
-    """Indices, weights and (up to 255 rows) the grouping tables of the small-tile pass with eight, four, two or one warp per
-    token in the re-check: byte for byte those of the kernel that computes every canonical logit, and of the grouping launch."""
+    """Indices and weights of the small-tile pass with eight, four, two or one warp per token in the re-check: byte for byte
+    those of the kernel that computes every canonical logit."""
     import torch
     from turbo_fieldfare_b200.kernels import DeviceRoutes, PrefillGroupedRoutedMoE, PrefillRouter
     o = oracle
@@ -101,7 +101,8 @@ def _forward(tf_ctx, layer, ws, x):
 @pytest.mark.parametrize("tokens,skew", [(103, 0.0), (104, 0.0), (128, 4.0), (255, 0.0), (255, 8.0)])
 def test_wide_chunks_equal_narrow_ones(tf_ctx, layer, tokens, skew):
     """A token's sums do not depend on the chunk that it sits in: a block of many tokens has the bits of the same tokens in
-    blocks of 40, whose experts' rows (and the shared expert's) are taken eight at a time or in other places."""
+    blocks of 40, whose experts' rows (and the shared expert's) are taken eight at a time or in other places, and which route and
+    group in one launch instead of two."""
     import torch
     from turbo_fieldfare_b200.stack import Workspace
     bias = np.zeros(128, np.float32)

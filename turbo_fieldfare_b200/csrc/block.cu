@@ -403,7 +403,7 @@ tf_status tf_workspace_create(tf_context* ctx, uint32_t max_tokens, uint32_t d, 
                    o_ecnt = take(E * 4), o_groups = take(E * 12), o_cgroup = take((T * K / 8 + E + 1) * 4),
                    o_cstart = take(E * 4), o_counters = take(16), o_acts = take(T * K * f * 2),
                    o_partials = take(T * K * d * (T <= tf::kF32PartialTokens ? 4 : 2)), o_sact = take(T * fs * 2),
-                   o_sy = take(T * d * 2), o_xn = take(T * d * 2), o_yb = take(T * d * 2);
+                   o_sy = take(T * d * 2), o_xn = take(T * d * 2), o_yb = take(T * d * 2), o_ticket = take(4);
     // workspaces that can hold a tensor-core sized block also carry the expert-sorted activation rows
     const bool tensor_path = T >= ctx->tensorcore_min_tokens && d % 64 == 0 && f % 64 == 0 && fs % 64 == 0;
     const uint64_t o_xs = tensor_path ? take(T * K * d * 2) : 0, o_inv = tensor_path ? take(T * K * 4) : 0,
@@ -431,6 +431,7 @@ tf_status tf_workspace_create(tf_context* ctx, uint32_t max_tokens, uint32_t d, 
     w->partials = base + o_partials;
     w->shared_act = reinterpret_cast<uint16_t*>(base + o_sact);
     w->shared_y = reinterpret_cast<uint16_t*>(base + o_sy);
+    w->router_ticket = reinterpret_cast<uint32_t*>(base + o_ticket);
     w->x_norm = reinterpret_cast<uint16_t*>(base + o_xn);
     w->y_block = reinterpret_cast<uint16_t*>(base + o_yb);
     w->x_sorted = tensor_path ? reinterpret_cast<uint16_t*>(base + o_xs) : nullptr;
@@ -465,13 +466,15 @@ namespace tf {
 static tf_status block_routed(tf_context* ctx, void* stream, const tf_moe_layer* layer, const void* x, uint32_t x_stride_elements,
                               uint32_t tokens, tf_workspace* ws, bool tensor_path) {
     const uint32_t d = layer->d, f = layer->f, K = layer->top_k, E = layer->num_experts;
-    // decode-sized blocks route and group in one launch
-    tf_status s = tf_router_gemma4_block_grouped(ctx, stream, layer->router.weights, layer->router.weights_off,
-                                                 layer->router.scales, layer->router.scales_off,
-                                                 layer->router.biases, layer->router.biases_off,
-                                                 x, 0, TF_FP16, layer->effective_scale, 0, layer->per_expert_scale, 0,
-                                                 layer->logit_bias, ws->indices, ws->weights, tokens, E, d, K,
-                                                 x_stride_elements, &ws->routes);
+    // Decode-sized blocks route and group in one launch, blocks of a few hundred tokens in two: their approximate logits lie
+    // where the activations will (they are read before the gate/up phase writes those).
+    void* approx = (uint64_t)K * f * 2 >= (uint64_t)E * 8 ? ws->acts : nullptr;
+    tf_status s = router_block_grouped(ctx, stream, layer->router.weights, layer->router.weights_off,
+                                       layer->router.scales, layer->router.scales_off,
+                                       layer->router.biases, layer->router.biases_off,
+                                       x, 0, TF_FP16, layer->effective_scale, 0, layer->per_expert_scale, 0,
+                                       layer->logit_bias, ws->indices, ws->weights, tokens, E, d, K,
+                                       x_stride_elements, &ws->routes, approx, ws->router_ticket);
     if (s) return s;
     if (tensor_path) {
         // Prefill-sized block: gather the rows into expert order and run gate/up/GeGLU/down as tcgen05 GEMMs; the

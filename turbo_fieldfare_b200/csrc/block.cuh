@@ -24,6 +24,7 @@ struct tf_workspace {
     void* partials;         // [T, K, D] fp32 (T <= f32_tokens) or fp16
     uint16_t* shared_act;   // [T, Fs]
     uint16_t* shared_y;     // [T, D]
+    uint32_t* router_ticket;  // zero between launches
     uint16_t* x_norm;       // [T, D] (stack)
     uint16_t* y_block;      // [T, D] (stack)
     uint16_t* x_sorted;     // [T*K, D] expert-sorted activation rows (tensor-core path; NULL for small workspaces)
@@ -52,6 +53,15 @@ tf_status launch_decode_step(tf_context* ctx, void* stream, tf_stack* st, void* 
 tf_status group_routes_strided(tf_context* ctx, void* stream, const uint32_t* indices, uint32_t idx_stride, uint32_t* ids_out,
                                const void* weights_f16, uint32_t query_count, uint32_t top_k, uint32_t num_experts,
                                const tf_device_routes* routes, const char* name, const struct PeerWait* peer_wait);
+// router.cu: tf_router_gemma4_block_grouped with scratch of the caller's workspace
+tf_status router_block_grouped(tf_context* ctx, void* stream, const void* weights, uint64_t weights_off,
+                               const void* scales, uint64_t scales_off, const void* biases, uint64_t biases_off,
+                               const void* hidden, uint64_t hidden_off, tf_dtype hidden_dtype,
+                               const void* effective_scale, uint64_t effective_scale_off,
+                               const void* per_expert_scale, uint64_t per_expert_scale_off,
+                               const float* logit_bias, uint32_t* out_indices, void* out_weights,
+                               uint32_t query_count, uint32_t num_experts, uint32_t d, uint32_t top_k,
+                               uint32_t hidden_stride_elements, const tf_device_routes* routes, void* approx_scratch, uint32_t* ticket);
 // grouped.cu: tf_grouped_moe_batched for a caller that knows the experts' number (it decides the tokens per chunk)
 tf_status grouped_moe_batched(tf_context* ctx, void* stream, const void* hidden, uint64_t hidden_off,
                               uint32_t hidden_stride_elements, const void* pool_layer_base, uint64_t expert_stride,

@@ -77,7 +77,6 @@ tf_status tf_context_create(int device, tf_context** out) {
     e = cudaMalloc(&ctx->router_logits, sizeof(float) * tf::kRouterSplitRows * TF_MAX_ROUTER_EXPERTS);
     if (e == cudaSuccess) e = cudaMalloc(&ctx->router_tickets, sizeof(unsigned int) * (tf::kRouterSplitRows + 1));   // rows + one for the whole block
     if (e == cudaSuccess) e = cudaMemset(ctx->router_tickets, 0, sizeof(unsigned int) * (tf::kRouterSplitRows + 1));
-    if (e == cudaSuccess) e = cudaMalloc(&ctx->router_approx_few, sizeof(float2) * tf::kRouterFusedGroupRows * TF_MAX_ROUTER_EXPERTS);
     if (e == cudaSuccess) e = cudaMalloc(&ctx->device_error, sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMemset(ctx->device_error, 0, sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMalloc(&ctx->peer_error, sizeof(uint32_t));
@@ -105,7 +104,6 @@ void tf_context_destroy(tf_context* ctx) {
     if (ctx->router_logits) cudaFree(ctx->router_logits);
     if (ctx->router_tickets) cudaFree(ctx->router_tickets);
     if (ctx->router_approx) cudaFree(ctx->router_approx);
-    if (ctx->router_approx_few) cudaFree(ctx->router_approx_few);
     if (ctx->device_error) cudaFree(ctx->device_error);
     if (ctx->peer_error) cudaFree(ctx->peer_error);
     if (ctx->streamed_scratch) cudaFree(ctx->streamed_scratch);

@@ -526,7 +526,6 @@ static int tile_router_rows(uint32_t rows, uint32_t slots) {
 // on demand. Growing allocates, which a stream that is being captured must not do: the caller then takes the
 // one-launch kernel.
 static bool router_scratch(tf_context* ctx, cudaStream_t st, uint32_t rows, uint32_t num_experts) {
-    if (rows <= kRouterFusedGroupRows) return ctx->router_approx_few != nullptr;
     const size_t need = (size_t)rows * num_experts * sizeof(float2);
     if (need <= ctx->router_approx_bytes) return true;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -544,13 +543,20 @@ static RouterGroupOut router_group_out(const tf_device_routes* routes) {
                           static_cast<uint32_t*>(routes->counters)};
 }
 
+// Scratch of the two-launch router that belongs to the caller's workspace: nothing of the context is shared, so such calls may
+// overlap on several streams (the one-launch kernel for more than kRouterSplitRows rows shares nothing either).
+struct RouterScratch {
+    float2* approx;             // [rows, num_experts]
+    unsigned int* ticket;       // zero between calls
+};
+
 // routes: the tables of the grouping, when it is wanted; *grouped (may be NULL) tells whether a launch of this call fills
-// them (always for at most kRouterSplitRows rows).
+// them (always for at most kRouterSplitRows rows, and with own scratch). own: take the two-launch form whatever the row count.
 static tf_status launch_router(tf_context* ctx, void* stream, const uint8_t* W, const uint8_t* S, const uint8_t* B,
                                const uint8_t* hidden, tf_dtype hidden_dtype, const uint8_t* eff, const uint8_t* pes,
                                const float* logit_bias, uint32_t* out_idx, uint8_t* out_w, float* out_logits,
                                uint32_t rows, uint32_t num_experts, uint32_t d, uint32_t top_k, uint32_t stride,
-                               const char* name, const tf_device_routes* routes = nullptr, bool* grouped = nullptr) {
+                               const char* name, const tf_device_routes* routes = nullptr, bool* grouped = nullptr, const RouterScratch* own = nullptr) {
     if (grouped) *grouped = routes != nullptr && rows <= (uint32_t)kRouterSplitRows;
     TF_REQUIRE(ctx, aligned(S, 2) && aligned(B, 2) && aligned(hidden, 2) && aligned(eff, 2) && aligned(pes, 2) &&
                         aligned(out_w, 2) && aligned(out_idx, 4),
@@ -600,11 +606,11 @@ static tf_status launch_router(tf_context* ctx, void* stream, const uint8_t* W, 
         launch_pdl(k, grid, dim3(kSplitThreads), smem_split, st, W, Sp, Bp, hp, stride, ep, pp, logit_bias, out_idx, wp, out_logits,
                    ctx->router_logits, ctx->router_tickets, grp, num_experts, d, top_k, a2);
         return check_launch(ctx, name);
-    } else if (rows >= ctx->router_tensorcore_min_rows && !out_logits && vec16 && d % kApxChunk == 0 && aligned(S, 8) && aligned(B, 8) &&
+    } else if ((own || rows >= ctx->router_tensorcore_min_rows) && !out_logits && vec16 && d % kApxChunk == 0 && aligned(S, 8) && aligned(B, 8) &&
                num_experts <= TF_MAX_ROUTER_EXPERTS && top_k <= (uint32_t)kWarp && top_k <= num_experts &&
-               router_recheck_smem_bytes(d, num_experts, kRecheckWarps) <= 200 * 1024 && router_scratch(ctx, st, rows, num_experts)) {
+               router_recheck_smem_bytes(d, num_experts, kRecheckWarps) <= 200 * 1024 && (own || router_scratch(ctx, st, rows, num_experts))) {
         // logits on the tensor cores, then the canonical logits of the few experts that can reach the top k
-        float2* approx = static_cast<float2*>(rows <= kRouterFusedGroupRows ? ctx->router_approx_few : ctx->router_approx);
+        float2* approx = own ? own->approx : static_cast<float2*>(ctx->router_approx);
         const uint32_t sms = (uint32_t)ctx->sm_count;
         // Few rows: blocks of 8 tokens x 32 experts, all of whose operands are in flight at once, as long as they make at
         // most four rounds of the SMs (100 blocks, 200 rows: 11 us; 168 blocks, 333 rows: 17 us; the 16 x 128 blocks take 25 us there
@@ -642,7 +648,7 @@ static tf_status launch_router(tf_context* ctx, void* stream, const uint8_t* W, 
         const uint32_t per_block = (uint32_t)kRecheckWarps >> which;
         size_t smem_r = router_recheck_smem_bytes(d, num_experts, per_block);
         RouterGroupOut grp{};
-        if (routes) {
+        if (own && routes) {
             grp = router_group_out(routes);
             const size_t need = router_group_smem_bytes(rows * top_k, num_experts, true);
             if (need > smem_r) smem_r = need;
@@ -650,8 +656,8 @@ static tf_status launch_router(tf_context* ctx, void* stream, const uint8_t* W, 
         static DeviceSmemCache configured_recheck[4][4];
         if (tf_status s = ensure_dynamic_smem(ctx, kr, configured_recheck[which][(bf ? 1 : 0) + (fixed ? 2 : 0)], smem_r)) return s;
         launch_pdl(kr, dim3((rows + per_block - 1) / per_block), dim3(kRecheckWarps * kWarp), smem_r, st, W, Sp, Bp, hp, stride,
-                   ep, pp, logit_bias, static_cast<const float2*>(approx), out_idx, wp, ctx->router_tickets, grp, rows, num_experts, d, top_k);
-        if (grouped) *grouped = routes != nullptr;
+                   ep, pp, logit_bias, static_cast<const float2*>(approx), out_idx, wp, own ? own->ticket : nullptr, grp, rows, num_experts, d, top_k);
+        if (grouped) *grouped = own && routes;
     } else if (rows >= 256 && a2 && (size_t)kTileRouterRows * (d + num_experts) * 4 <= 100 * 1024) {
         const int R = tile_router_rows(rows, (uint32_t)ctx->sm_count * 2u);
         void (*k)(const uint8_t*, const uint16_t*, const uint16_t*, const uint16_t*, uint32_t, const uint16_t*, const uint16_t*, const float*,
@@ -671,6 +677,43 @@ static tf_status launch_router(tf_context* ctx, void* stream, const uint8_t* W, 
                    num_experts, d, top_k, a2);
     }
     return check_launch(ctx, name);
+}
+
+// tf_router_gemma4_block_grouped; approx_scratch ([query_count, num_experts] pairs of floats) and ticket (a zero word), when
+// given, belong to the caller's workspace: blocks of 65 to kRouterFusedGroupRows rows then route in two launches, the second of
+// which groups them (the block that finishes the last row does it). One block per row computes every canonical logit there
+// otherwise: 168 + 8 us against 11 + 17 for 200 rows. Larger blocks group with launches of their own, which many SMs share.
+tf_status router_block_grouped(tf_context* ctx, void* stream, const void* weights, uint64_t weights_off,
+                               const void* scales, uint64_t scales_off, const void* biases, uint64_t biases_off,
+                               const void* hidden, uint64_t hidden_off, tf_dtype hidden_dtype,
+                               const void* effective_scale, uint64_t effective_scale_off,
+                               const void* per_expert_scale, uint64_t per_expert_scale_off,
+                               const float* logit_bias, uint32_t* out_indices, void* out_weights,
+                               uint32_t query_count, uint32_t num_experts, uint32_t d, uint32_t top_k,
+                               uint32_t hidden_stride_elements, const tf_device_routes* routes, void* approx_scratch, uint32_t* ticket) {
+    const char* name = "tf_router_gemma4_block_grouped";
+    TF_REQUIRE(ctx, weights && scales && biases && hidden && effective_scale && per_expert_scale && out_indices && out_weights,
+               TF_ERR_INVALID_ARGUMENT, "%s: NULL buffer", name);
+    TF_REQUIRE(ctx, query_count > 0, TF_ERR_INVALID_ARGUMENT, "%s: queryCount must be positive", name);
+    TF_REQUIRE(ctx, num_experts > 0 && num_experts <= TF_MAX_ROUTER_EXPERTS, TF_ERR_INVALID_ARGUMENT,
+               "%s: numExperts > 256 is not supported", name);
+    TF_REQUIRE(ctx, top_k > 0 && top_k <= TF_MAX_TOP_K && num_experts >= top_k, TF_ERR_INVALID_ARGUMENT,
+               "%s: topK must be in 1...%d and at most numExperts, got %u", name, TF_MAX_TOP_K, top_k);
+    TF_REQUIRE(ctx, d > 0 && d % tf::kGroup == 0 && hidden_stride_elements >= d, TF_ERR_INVALID_ARGUMENT,
+               "%s: D must be a multiple of 64 and the stride at least D", name);
+    TF_REQUIRE(ctx, hidden_dtype == TF_FP16 || hidden_dtype == TF_BF16, TF_ERR_INVALID_ARGUMENT, "%s: bad hidden dtype", name);
+    const RouterScratch own{static_cast<float2*>(approx_scratch), ticket};
+    const bool use_own = approx_scratch && ticket && query_count > (uint32_t)kRouterSplitRows && query_count <= kRouterFusedGroupRows &&
+                         ctx->router_tensorcore_min_rows != 0xFFFFFFFFu;
+    bool grouped = false;
+    tf_status s = launch_router(ctx, stream, byte_ptr(weights, weights_off), byte_ptr(scales, scales_off),
+                                byte_ptr(biases, biases_off), byte_ptr(hidden, hidden_off), hidden_dtype,
+                                byte_ptr(effective_scale, effective_scale_off),
+                                byte_ptr(per_expert_scale, per_expert_scale_off), logit_bias, out_indices,
+                                static_cast<uint8_t*>(out_weights), nullptr, query_count, num_experts, d, top_k,
+                                hidden_stride_elements, name, routes, &grouped, use_own ? &own : nullptr);
+    if (s || grouped) return s;
+    return tf_group_routes_device(ctx, stream, out_indices, out_weights, query_count, top_k, num_experts, routes);
 }
 
 }  // namespace tf
@@ -744,27 +787,9 @@ tf_status tf_router_gemma4_block_grouped(tf_context* ctx, void* stream, const vo
     TF_REQUIRE(ctx, routes && routes->sorted_pairs && routes->per_expert_offsets && routes->per_expert_counts && routes->groups &&
                         routes->chunk_group && routes->chunk_start && routes->counters,
                TF_ERR_INVALID_ARGUMENT, "%s: NULL routes buffer", name);
-    TF_REQUIRE(ctx, weights && scales && biases && hidden && effective_scale && per_expert_scale && out_indices && out_weights,
-               TF_ERR_INVALID_ARGUMENT, "%s: NULL buffer", name);
-    TF_REQUIRE(ctx, query_count > 0, TF_ERR_INVALID_ARGUMENT, "%s: queryCount must be positive", name);
-    TF_REQUIRE(ctx, num_experts > 0 && num_experts <= TF_MAX_ROUTER_EXPERTS, TF_ERR_INVALID_ARGUMENT,
-               "%s: numExperts > 256 is not supported", name);
-    TF_REQUIRE(ctx, top_k > 0 && top_k <= TF_MAX_TOP_K && num_experts >= top_k, TF_ERR_INVALID_ARGUMENT,
-               "%s: topK must be in 1...%d and at most numExperts, got %u", name, TF_MAX_TOP_K, top_k);
-    TF_REQUIRE(ctx, d > 0 && d % tf::kGroup == 0 && hidden_stride_elements >= d, TF_ERR_INVALID_ARGUMENT,
-               "%s: D must be a multiple of 64 and the stride at least D", name);
-    TF_REQUIRE(ctx, hidden_dtype == TF_FP16 || hidden_dtype == TF_BF16, TF_ERR_INVALID_ARGUMENT, "%s: bad hidden dtype", name);
-    // Blocks of a few hundred rows group in the router's last launch too (the block that finishes the last row does it);
-    // larger ones group with launches of their own, which many SMs share.
-    bool grouped = false;
-    tf_status s = tf::launch_router(ctx, stream, tf::byte_ptr(weights, weights_off), tf::byte_ptr(scales, scales_off),
-                                    tf::byte_ptr(biases, biases_off), tf::byte_ptr(hidden, hidden_off), hidden_dtype,
-                                    tf::byte_ptr(effective_scale, effective_scale_off),
-                                    tf::byte_ptr(per_expert_scale, per_expert_scale_off), logit_bias, out_indices,
-                                    static_cast<uint8_t*>(out_weights), nullptr, query_count, num_experts, d, top_k,
-                                    hidden_stride_elements, name, query_count <= tf::kRouterFusedGroupRows ? routes : nullptr, &grouped);
-    if (s || grouped) return s;
-    return tf_group_routes_device(ctx, stream, out_indices, out_weights, query_count, top_k, num_experts, routes);
+    return tf::router_block_grouped(ctx, stream, weights, weights_off, scales, scales_off, biases, biases_off, hidden, hidden_off, hidden_dtype,
+                                    effective_scale, effective_scale_off, per_expert_scale, per_expert_scale_off, logit_bias, out_indices,
+                                    out_weights, query_count, num_experts, d, top_k, hidden_stride_elements, routes, nullptr, nullptr);
 }
 
 }  // extern "C"

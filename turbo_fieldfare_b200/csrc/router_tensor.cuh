@@ -447,7 +447,7 @@ __global__ void __launch_bounds__(kRecheckWarps * kWarp, 2)
 router_recheck_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S, const uint16_t* __restrict__ B,
                       const uint16_t* __restrict__ hidden, uint32_t hidden_stride, const uint16_t* __restrict__ eff,
                       const uint16_t* __restrict__ per_expert_scale, const float* __restrict__ logit_bias,
-                      const float2* __restrict__ approx, uint32_t* out_idx, uint16_t* out_w, unsigned int* tickets, const RouterGroupOut grp,
+                      const float2* __restrict__ approx, uint32_t* out_idx, uint16_t* out_w, unsigned int* ticket, const RouterGroupOut grp,
                       uint32_t rows, uint32_t num_experts, uint32_t d, uint32_t top_k) {
     extern __shared__ __align__(16) uint8_t smem[];
     constexpr int kTokens = kRecheckWarps / WPT;                    // tokens per block
@@ -598,8 +598,8 @@ router_recheck_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict_
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
-        is_last = atomicAdd(&tickets[kRouterSplitRows], 1u) == gridDim.x - 1;
-        if (is_last) tickets[kRouterSplitRows] = 0;            // ready for the next launch on this stream
+        is_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+        if (is_last) *ticket = 0;                              // ready for the next launch
     }
     __syncthreads();
     if (!is_last) return;

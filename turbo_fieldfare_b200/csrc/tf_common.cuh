@@ -19,7 +19,7 @@ constexpr int kGroup = TF_GROUP_SIZE;
 constexpr int kWarp = 32;
 constexpr unsigned kFullMask = 0xFFFFFFFFu;
 constexpr int kRouterSplitRows = 64;   // rows served by the multi-block decode router
-constexpr uint32_t kRouterFusedGroupRows = 255;   // with more rows the routes are grouped by launches of their own
+constexpr uint32_t kRouterFusedGroupRows = 255;   // block forwards: with more rows the routes are grouped by launches of their own
 constexpr int kChunkTokens = 8;        // tokens per work chunk of the grouped kernels (the n of m16n8k16)
 
 // ---------------------------------------------------------------------------
@@ -42,13 +42,9 @@ struct tf_context {
     unsigned int* router_tickets = nullptr;  // [kRouterSplitRows], self-resetting
     // Prefill-sized router: (approximate logit, magnitude) per (row, expert) between its two launches; grown on demand.
     void* router_approx = nullptr;
-    // The same for blocks of at most kRouterFusedGroupRows rows, allocated with the context: decode graphs keep its address, so it
-    // must neither move nor need an allocation while a stream is captured.
-    void* router_approx_few = nullptr;
     size_t router_approx_bytes = 0;
-    // Batches of at least this many rows take the two-launch router (tensor-core logits + canonical re-check): all that the
-    // few-row kernels do not take. One block per row computed every canonical logit: 168 us for 200 rows, against 20.
-    uint32_t router_tensorcore_min_rows = tf::kRouterSplitRows + 1;
+    // Batches of at least this many rows take the two-launch router (tensor-core logits + canonical re-check).
+    uint32_t router_tensorcore_min_rows = 256;
     // One device word that kernels with bounded waits set when a wait gives up (0 = healthy).
     uint32_t* device_error = nullptr;
     // The same for the flag barriers of the peer exchange (peer.cu), kept apart so that a code from another kernel

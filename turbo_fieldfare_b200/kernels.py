@@ -83,7 +83,7 @@ class TurboContext:
 
     def set_router_tensorcore_min_rows(self, rows: int) -> None:
         """Router calls over at least ``rows`` rows compute all logits on the tensor cores and re-check the candidates in
-        the canonical order (default 65; 0xFFFFFFFF keeps the one-launch kernel)."""
+        the canonical order (default 256; 0xFFFFFFFF keeps the one-launch kernel)."""
         self.check(self.lib.tf_context_set_router_tensorcore_min_rows(self.handle, rows))
 
     def set_single_launch_step(self, enabled: bool) -> None:
