@@ -626,7 +626,7 @@ def measure_roofline(torch, ctx, stack, ws, h, batch, PrefillRouter, PrefillGrou
     # grouped_ksplit_kernel, routed decode batch 64) read and wrote 435.6 MB for 421.5 MB of touched expert planes,
     # 1.033 bytes per algorithmic byte; traffic grows with the experts touched, so it is scaled by that ratio.
     traffic_ratio = 435.63 / 421.52
-    return {"bound": "hbm", "kernel": "grouped_ksplit_kernel (routed gate/up and down launches of one layer, batch 64)",
+    return {"bound": "hbm", "kernel": "grouped_ksplit_kernel + grouped_down_kernel (routed gate/up and down launches of one layer, batch 64)",
             "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak, "peak_source": peak_src,
             "traffic": bytes_total / launches * traffic_ratio, "traffic_source": "ncu capture at 64 tokens, scaled by experts touched",
             "bytes_per_launch": bytes_total / launches, "us_per_launch": ms * 1e3 / launches,
