@@ -30,6 +30,18 @@ __device__ __forceinline__ bool mbar_wait(uint32_t addr, uint32_t parity) {
     }
     return false;
 }
+// Both waits, the first one polled before the second in every round: what the second returns counts only once the first has
+// passed, so the first may be what makes the second's parity unambiguous. The latencies of the two polls overlap.
+__device__ __forceinline__ bool mbar_wait_both(uint32_t first, uint32_t first_parity, uint32_t second, uint32_t second_parity) {
+    for (uint32_t i = 0; i < kMbarSpinLimit; ++i) {
+        uint32_t ok;
+        asm volatile("{ .reg .pred p, q; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; mbarrier.try_wait.parity.shared::cta.b64 q, [%3], %4; "
+                     "and.pred p, p, q; selp.u32 %0, 1, 0, p; }"
+                     : "=r"(ok) : "r"(first), "r"(first_parity), "r"(second), "r"(second_parity) : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
 __device__ __forceinline__ void bulk_copy_g2s(uint32_t smem_dst, const void* gmem_src, uint32_t bytes, uint32_t mbar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(smem_dst), "l"(gmem_src), "r"(bytes), "r"(mbar) : "memory");

@@ -926,9 +926,17 @@ grouped_ksplit_kernel(const GroupedArgs args) {
 // Here eleven independent warps take the items in turn, fed by one loader through a ring of stages of four consecutive items
 // (one copy of 64 rows, one of their scales, one of their biases: a loader turn costs several hundred clocks whatever it
 // moves). Sums have the bits of the column-split kernel: parts of four groups, added in order.
+//
+// A barrier wait names only a phase's parity, and a warp has no item in most of the stages that pass through a slot, so the wait
+// for stage S alone would also return while the copy of the slot's previous use, S - 7, is still on its way. A warp therefore
+// first waits until that use is released. This wait cannot be taken for another phase: S - 14 was released before the loader
+// issued the warp's own previous stage, and S cannot be released without this warp (a fresh barrier passes it for the first use).
+// It has passed by the time S has landed, so one round of both polls is enough then. (A multiple of four warps would see every use of its slots, but a thirteenth warp on the SM, the loader
+// beside twelve, leaves a thread 128 registers instead of 168, and the fragments spill.)
 constexpr int kDownWarps = 11;
 constexpr int kDownSub = 4;               // items per stage
 constexpr int kDownStages = 7;
+static_assert((kDownWarps + kDownSub - 1) / kDownSub <= kDownStages, "a warp's previous stage is issued after the slot's previous use");
 template <int OUT_MODE, int NG>
 __global__ void __launch_bounds__((kDownWarps + 1) * kWarp, 1)
 grouped_down_kernel(const GroupedArgs args) {
@@ -1014,7 +1022,7 @@ grouped_down_kernel(const GroupedArgs args) {
                     }
                 }
             }
-            if (!mbar_wait(bar_full(st), use & 1)) { fail = kErrTimeoutCodes; break; }
+            if (!mbar_wait_both(bar_empty(st), (use - 1) & 1, bar_full(st), use & 1)) { fail = kErrTimeoutCodes; break; }      // released, landed
             const uint32_t codes = smem_base + st * kStageBytes + sub * kCodeBytes + g * kRowBytes + t * 8;
             const uint32_t scales = smem_base + st * kStageBytes + kDownSub * kCodeBytes + sub * kPlaneBytes + g * (NG * 2);
             const uint32_t biases = scales + kDownSub * kPlaneBytes;
@@ -1191,7 +1199,7 @@ static tf_status launch_grouped(tf_context* ctx, void* stream, GroupedArgs& args
 
 // The routed down projection: the whole-row kernel for the width that it is built for, from 320 (token, expert) pairs on (40
 // tokens of eight experts); with fewer, its deeper pipeline does not pay for the time that it takes to fill. Steps of 30 layers
-// with it and without: 32 tokens 3.27 and 3.23 ms, 48 tokens 3.81 and 3.87, 64 tokens 3.85 and 4.21, 200 tokens 7.45 and 8.26
+// with it and without: 32 tokens 3.27 and 3.23 ms, 48 tokens 3.81 and 3.87, 64 tokens 3.88 and 4.21, 200 tokens 7.50 and 8.26
 // (the latter with 16-token chunks in the column-split kernel).
 constexpr uint32_t kDownMinPairs = 320;
 template <int OUT_MODE>
