@@ -3,7 +3,8 @@ few-row router, chunks of 16 tokens against chunks of 8, and the 16-row tiles of
 import numpy as np
 import pytest
 
-from tests.helpers import config0_matrix, dev_zeros_u16, from_dev, to_dev
+from tests.helpers import blob_table, config0_matrix, dev_zeros_u16, from_dev, to_dev
+from turbo_fieldfare_b200._capi import ExpertOffsets
 
 pytestmark = pytest.mark.gpu
 
@@ -154,3 +155,30 @@ def test_tile_gemv(tf_ctx, oracle, m, n, scale):
     # the result's rounding (2^-11, or half a subnormal step) and fp32 sums of up to 16384 products
     bound = np.abs(ref) * 2.0 ** -11 + 2.0 ** -25 + (np.abs(_dense(o, mat)) + 0.1) @ np.abs(o.f16_to_f32(x16).astype(np.float64)) * 2.0 ** -20
     assert np.all(np.abs(o.f16_to_f32(out[:m]) - ref) <= bound)
+
+
+# Shared memory of the down kernel on either side of what a launch may use unasked (48 KB, the static part included): K * F / 64
+# of 368, then 369 to 372. Smaller sizes first: the limit, once raised, stays raised.
+@pytest.mark.parametrize("K,F", [(8, 2944), (3, 7872), (5, 4736), (7, 3392), (6, 3968), (8, 8192)])
+def test_phase2_shared_memory_limit(tf_ctx, oracle, K, F):
+    import torch
+    from turbo_fieldfare_b200.kernels import MoE
+    o = oracle
+    D = 72
+    rng = np.random.default_rng(K * F)
+    downs = [config0_matrix(o, D, F, rng) for _ in range(K)]
+    blobs = [to_dev(np.concatenate([m.packed.reshape(-1), m.scales.view(np.uint8).reshape(-1), m.biases.view(np.uint8).reshape(-1)])) for m in downs]
+    coff = ExpertOffsets(0, 0, 0, 0, 0, 0, 0, D * F // 2, D * F // 2 + D * (F // 64) * 2)
+    acts16, w16 = o.f32_to_f16(rng.standard_normal((K, F)).astype(np.float32)), o.f32_to_f16(rng.dirichlet(np.ones(K)).astype(np.float32))
+    res16 = o.f32_to_f16(rng.standard_normal(D).astype(np.float32))
+    y = dev_zeros_u16(D + 8, fill=0x7E00)
+    MoE(tf_ctx).encode_routed_phase2_reduce(blob_table(blobs), coff, to_dev(acts16), to_dev(w16), to_dev(res16), y, D, F, K)
+    torch.cuda.synchronize()
+    out = from_dev(y, np.uint16)
+    assert np.all(out[D:] == 0x7E00)
+    x64, w64 = o.f16_to_f32(acts16).astype(np.float64), o.f16_to_f32(w16).astype(np.float64)
+    dense = [_dense(o, m) for m in downs]
+    ref = o.f16_to_f32(res16) + sum(w64[k] * (dense[k] @ x64[k]) for k in range(K))
+    # the result's rounding and fp32 sums of up to 8 x 8192 products
+    bound = np.abs(ref) * 2.0 ** -11 + 2.0 ** -25 + sum(w64[k] * ((np.abs(dense[k]) + 0.1) @ np.abs(x64[k])) for k in range(K)) * 2.0 ** -20
+    assert np.all(np.abs(o.f16_to_f32(out[:D]) - ref) <= bound)

@@ -183,8 +183,8 @@ tf_status launch_tile_down(tf_context* ctx, void* stream, const void* const* blo
     const uint32_t ng = f / kGroup;
     const size_t smem = tile_x_bytes(top_k, ng);
     static DeviceSmemCache configured;
-    if (smem > 48 * 1024)
-        if (tf_status s = ensure_dynamic_smem(ctx, tile_down_kernel, configured, smem)) return s;
+    // whatever the size: the 48 KB that a launch may use unasked include the kernel's static array
+    if (tf_status s = ensure_dynamic_smem(ctx, tile_down_kernel, configured, smem)) return s;
     launch_pdl(tile_down_kernel, dim3((d + kTileRows16 - 1) / kTileRows16), dim3(kTileThreads), smem, static_cast<cudaStream_t>(stream),
                reinterpret_cast<const uint8_t* const*>(blobs), *offsets, static_cast<const uint16_t*>(acts), static_cast<const uint16_t*>(routing_w),
                static_cast<const uint16_t*>(residual), static_cast<uint16_t*>(y), d, ng, top_k);
