@@ -9,6 +9,15 @@ from turbo_fieldfare_b200._capi import ExpertOffsets
 pytestmark = pytest.mark.gpu
 
 
+@pytest.fixture(scope="module")
+def tf_ctx():
+    """A context of this module's own: at its defaults whatever thresholds other modules have set on theirs."""
+    from turbo_fieldfare_b200.kernels import TurboContext
+    ctx = TurboContext(0)
+    yield ctx
+    ctx.close()
+
+
 def _dense(o, mat):
     """The matrix in 64 bits."""
     q = np.empty((mat.packed.shape[0], mat.packed.shape[1] * 2), np.float64)
@@ -182,3 +191,36 @@ def test_phase2_shared_memory_limit(tf_ctx, oracle, K, F):
     # the result's rounding and fp32 sums of up to 8 x 8192 products
     bound = np.abs(ref) * 2.0 ** -11 + 2.0 ** -25 + sum(w64[k] * ((np.abs(dense[k]) + 0.1) @ np.abs(x64[k])) for k in range(K)) * 2.0 ** -20
     assert np.all(np.abs(o.f16_to_f32(out[:D]) - ref) <= bound)
+
+
+def _kernels_of(forward, path):
+    """Text of a captured forward's graph, with the names of its kernels."""
+    import torch
+    from cuda.bindings import runtime
+    forward()                                           # outside the capture: function attributes, side stream
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph, stream=torch.cuda.Stream()):
+        forward()
+    assert runtime.cudaGraphDebugDotPrint(graph.raw_cuda_graph(), str(path).encode(), 1)[0] == runtime.cudaError_t.cudaSuccess
+    return path.read_text()
+
+
+@pytest.mark.parametrize("rows,two_launches", [(None, True), (65, True), (200, True), (201, False), (256, False), (1000, False), (0xFFFFFFFF, False)])
+def test_router_threshold_holds_for_block_forwards(layer, tmp_path, rows, two_launches):
+    """A block forward of 200 rows takes the two-launch router by default, and below a threshold that was set the one-launch one."""
+    import torch
+    from turbo_fieldfare_b200.kernels import TurboContext
+    from turbo_fieldfare_b200.stack import MoEBlock, Workspace
+    ctx = TurboContext(0)
+    try:
+        if rows is not None:
+            ctx.set_router_tensorcore_min_rows(rows)
+        x = torch.randn(200, 2816, device="cuda").half()
+        y, ws, block = torch.zeros_like(x), Workspace(ctx, 200, 2816, 704, 2112, 8, 128), MoEBlock(ctx, layer)
+        text = _kernels_of(lambda: block.forward(x, y, 200, ws), tmp_path / "graph.dot")
+        assert "grouped_ksplit_kernel" in text
+        assert ("router_recheck_kernel" in text) is two_launches
+        ws.close()
+    finally:
+        ctx.close()

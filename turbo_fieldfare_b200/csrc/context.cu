@@ -140,7 +140,7 @@ tf_status tf_context_set_shared_tensorcore_min_tokens(tf_context* ctx, uint32_t 
 
 tf_status tf_context_set_router_tensorcore_min_rows(tf_context* ctx, uint32_t rows) {
     TF_REQUIRE(ctx, ctx != nullptr && rows > 0, TF_ERR_INVALID_ARGUMENT, "tf_context_set_router_tensorcore_min_rows: ctx is NULL or rows is 0");
-    ctx->router_tensorcore_min_rows = rows;
+    ctx->router_tensorcore_min_rows = ctx->router_block_min_rows = rows;
     return TF_OK;
 }
 

@@ -704,7 +704,7 @@ tf_status router_block_grouped(tf_context* ctx, void* stream, const void* weight
     TF_REQUIRE(ctx, hidden_dtype == TF_FP16 || hidden_dtype == TF_BF16, TF_ERR_INVALID_ARGUMENT, "%s: bad hidden dtype", name);
     const RouterScratch own{static_cast<float2*>(approx_scratch), ticket};
     const bool use_own = approx_scratch && ticket && query_count > (uint32_t)kRouterSplitRows && query_count <= kRouterFusedGroupRows &&
-                         ctx->router_tensorcore_min_rows != 0xFFFFFFFFu;
+                         query_count >= ctx->router_block_min_rows;
     bool grouped = false;
     tf_status s = launch_router(ctx, stream, byte_ptr(weights, weights_off), byte_ptr(scales, scales_off),
                                 byte_ptr(biases, biases_off), byte_ptr(hidden, hidden_off), hidden_dtype,

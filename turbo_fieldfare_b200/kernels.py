@@ -82,8 +82,9 @@ class TurboContext:
         self.check(self.lib.tf_context_set_shared_tensorcore_min_tokens(self.handle, tokens))
 
     def set_router_tensorcore_min_rows(self, rows: int) -> None:
-        """Router calls over at least ``rows`` rows compute all logits on the tensor cores and re-check the candidates in
-        the canonical order (default 256; 0xFFFFFFFF keeps the one-launch kernel)."""
+        """Router calls and block forwards over at least ``rows`` rows compute all logits on the tensor cores and re-check the
+        candidates in the canonical order (until set: 256 for router calls, 65 for block forwards; 0xFFFFFFFF keeps the
+        one-launch kernel)."""
         self.check(self.lib.tf_context_set_router_tensorcore_min_rows(self.handle, rows))
 
     def set_single_launch_step(self, enabled: bool) -> None:
