@@ -112,3 +112,15 @@ def test_streamed_params_layout_is_the_reference_one():
     for name, offset in want.items():
         assert getattr(P, name).offset == offset, name
     assert P.local_expert.offset + 15 * 4 == 88           # localExpert15
+
+
+def test_current_stream_handle_with_and_without_the_raw_accessor(monkeypatch):
+    import torch
+    from turbo_fieldfare_b200 import kernels
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 3)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda: type("S", (), {"cuda_stream": 77})())
+    monkeypatch.setattr(kernels, "_raw_current_stream", lambda device: 1000 + device)
+    assert kernels._stream(None) == 1003
+    monkeypatch.setattr(kernels, "_raw_current_stream", None)       # a torch without the private accessor
+    assert kernels._stream(None) == 77
+    assert kernels._stream(5) == 5

@@ -37,10 +37,16 @@ def _ptr(t) -> int | None:
     return int(t)
 
 
+# The raw handle of a device's current stream, where torch has it (the name is not public): a Stream object per call costs more
+# than a microsecond.
+_raw_current_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream(stream) -> int:
     if stream is None:
-        # the raw handle of the current stream; a Stream object per call costs more than a microsecond
-        return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+        if _raw_current_stream is not None:
+            return _raw_current_stream(torch.cuda.current_device())
+        return torch.cuda.current_stream().cuda_stream
     if isinstance(stream, torch.cuda.Stream):
         return stream.cuda_stream
     return int(stream)
