@@ -348,11 +348,12 @@ def test_one_token_stack_equals_layered_path(tf_ctx, oracle):
         stack.close()
 
 
-@pytest.mark.parametrize("T,d", [(7, 256), (40, 2816)])
+@pytest.mark.parametrize("T,d", [(7, 256), (40, 2816), (256, 2816), (300, 256)])
 def test_decode_sized_stack_equals_the_chain_of_entry_points_bit_for_bit(tf_ctx, oracle, T, d):
-    """tf_stack_forward on a decode-sized batch forms the weighted sum of the route partials inside the next norm; the
-    hidden state must equal tf_residual_rmsnorm + tf_moe_block_forward layer by layer, bit for bit (d = 2816: three
-    slices of the norm's sum of squares, the last one partial)."""
+    """tf_stack_forward on a decode-sized batch forms the weighted sum of the route partials inside the next norm, and on a
+    prefill-sized one (from 256 tokens on) that of the expert-sorted rows; the hidden state must equal tf_residual_rmsnorm +
+    tf_moe_block_forward layer by layer, bit for bit (d = 2816: three slices of the norm's sum of squares, the last one
+    partial)."""
     import ctypes as C
     import torch
     from turbo_fieldfare_b200.kernels import _ptr

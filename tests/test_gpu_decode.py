@@ -500,6 +500,36 @@ def test_routed_decode_production_shape_with_device_table(tf_ctx, oracle):
     assert o.rel_error(o.f16_to_f32(from_dev(y, np.uint16)), y_truth) < FP16_CHAINED
 
 
+@pytest.mark.parametrize("D,F", [(128, 64), (2816, 704)])
+@pytest.mark.parametrize("x_shift,acts_shift", [(0, 0), (1, 0), (0, 1), (1, 1)])
+def test_routed_decode_off_the_16_byte_grid(tf_ctx, oracle, D, F, x_shift, acts_shift):
+    """x or acts one fp16 element off the 16-byte grid: the row kernels, which load element by element, against the oracle
+    like the tile kernels that aligned vectors take."""
+    import torch
+    from turbo_fieldfare_b200.kernels import MoE
+    o, K = oracle, 8
+    rng = np.random.default_rng(D + 2 * x_shift + acts_shift)
+    off, _, stride = o.blob_layout(D, F, align=256)
+    blobs = [random_blob(o, D, F, rng, off, stride)[0] for _ in range(K)]
+    dev = [to_dev(b) for b in blobs]
+    table, coff = blob_table(dev), capi_offsets(off)
+    x16 = o.f32_to_f16(rng.standard_normal(D).astype(np.float32))
+    w16 = o.f32_to_f16(rng.dirichlet(np.ones(K)).astype(np.float32))
+    res16 = o.f32_to_f16(rng.standard_normal(D).astype(np.float32))
+    xbuf, abuf, y = dev_zeros_u16(D + 8), dev_zeros_u16(K * F + 8, fill=0x7BFF), dev_zeros_u16(D)
+    x, acts = xbuf[x_shift:x_shift + D], abuf[acts_shift:acts_shift + K * F]
+    x.copy_(to_dev(x16))
+    assert (x.data_ptr() % 16 != 0) == bool(x_shift) and (acts.data_ptr() % 16 != 0) == bool(acts_shift)
+    MoE(tf_ctx).encode_routed_phase1(table, coff, x, acts, D, F, K)
+    MoE(tf_ctx).encode_routed_phase2_reduce(table, coff, acts, to_dev(w16), to_dev(res16), y, D, F, K)
+    torch.cuda.synchronize()
+    _, y_truth, acts_truth = o.moe_routed_decode(blobs, off, x16, w16, res16, D, F, order=0)
+    got = from_dev(abuf, np.uint16)
+    assert np.all(got[:acts_shift] == 0x7BFF) and np.all(got[acts_shift + K * F:] == 0x7BFF)
+    assert o.rel_l2(o.f16_to_f32(got[acts_shift:acts_shift + K * F]), o.f16_to_f32(acts_truth.reshape(-1))) < FP16_CHAINED
+    assert o.rel_l2(o.f16_to_f32(from_dev(y, np.uint16)), y_truth) < FP16_CHAINED
+
+
 # ---------------------------------------------------------------------------
 # shared expert, norms
 # ---------------------------------------------------------------------------
@@ -727,6 +757,35 @@ def test_lm_head_greedy_streaming_shape(tf_ctx, oracle):
         want, logits = o.lm_head_greedy(hidden, norm, mat)
         got = _lm_head_gpu(tf_ctx, o, hidden, norm, mat, d, v)
         assert got == want or abs(float(logits[got]) - float(logits[want])) <= 1e-5 * max(1.0, abs(float(logits[want]))), (got, want)
+    assert tf_ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("d,v", [(256, 4096 + 40), (2816, 4096)])
+def test_lm_head_greedy_streaming_ties_and_non_finite_logits(tf_ctx, oracle, d, v):
+    """The argmax inside the streaming product (128 rows a block, 16 a warp): ties go to the lowest row wherever the tied rows
+    sit, rows without a finite logit are skipped, and a call in which no row has one gives 0 and leaves the next call right."""
+    o = oracle
+    ones = o.f32_to_bf16(np.ones(d, np.float32))
+    hidden = o.f32_to_f16(np.array([0.2 + (i % 5) * 0.02 for i in range(d)], np.float32))
+    two = _constant_rows(o, [-0.25, 1.0], d)
+
+    def head(rows):
+        """Every row -0.25, those of `rows` 1.0."""
+        take = np.zeros(v, np.int64)
+        take[list(rows)] = 1
+        return o.AffineMatrix(np.ascontiguousarray(two.packed[take]), np.ascontiguousarray(two.scales[take]),
+                              np.ascontiguousarray(two.biases[take]), 4, d, two.sb_dtype)
+
+    # one warp (rows g and g + 8, and neighbours), two warps of a block, two blocks, the last block's last row
+    for rows in [(17, 25), (18, 19), (20, 100), (311, 4000), (v - 1,), (v - 5, v - 1), (0, v - 1)]:
+        assert _lm_head_gpu(tf_ctx, o, hidden, ones, head(rows), d, v) == min(rows), rows
+    nan_hidden = np.full(d, 0x7E00, dtype=np.uint16)
+    assert _lm_head_gpu(tf_ctx, o, nan_hidden, ones, head((700,)), d, v) == 0
+    assert _lm_head_gpu(tf_ctx, o, hidden, ones, head((700,)), d, v) == 700
+    for bad in (0x7F80, 0xFF80, 0x7FC0):                    # a scale of +inf, -inf or NaN: no finite logit in the row
+        mat = head((40, 700, 900))
+        mat.scales[40, 0] = bad
+        assert _lm_head_gpu(tf_ctx, o, hidden, ones, mat, d, v) == 700
     assert tf_ctx.device_status() == 0
 
 

@@ -50,11 +50,11 @@ def test_qmm_token_tiles(tf_ctx, oracle, M, N, K, y_off):
 
 
 @pytest.mark.parametrize("rows", [65, 200, 255, 256, 297, 593, 1184, 1185])
-def test_few_row_router_equals_the_one_launch_kernel(tf_ctx, oracle, rows):
+def test_few_row_router_equals_the_one_launch_kernel(oracle, rows):
     """Indices and weights of the small-tile pass with eight, four, two or one warp per token in the re-check: byte for byte
     those of the kernel that computes every canonical logit."""
     import torch
-    from turbo_fieldfare_b200.kernels import DeviceRoutes, PrefillGroupedRoutedMoE, PrefillRouter
+    from turbo_fieldfare_b200.kernels import PrefillRouter, TurboContext
     o = oracle
     E, D, K = 128, 2816, 8
     rng = np.random.default_rng(rows)
@@ -67,21 +67,19 @@ def test_few_row_router_equals_the_one_launch_kernel(tf_ctx, oracle, rows):
     hid = to_dev(o.f32_to_f16(x))
     eff, gain = to_dev(o.f32_to_bf16(np.full(D, D ** -0.5, np.float32))), to_dev(o.f32_to_bf16(np.ones(E, np.float32)))
 
+    ctx = TurboContext(0)               # whose threshold the test sets
+
     def run(min_rows):
-        tf_ctx.set_router_tensorcore_min_rows(min_rows)
-        idx, w, routes = torch.full((rows, K), -1, dtype=torch.int32, device="cuda"), dev_zeros_u16(rows * K), DeviceRoutes(rows, K, E)
-        PrefillRouter(tf_ctx).encode_gemma4_block_grouped(W, S, B, hid, eff, gain, idx, w, rows, E, D, K, D, routes)
-        ref = DeviceRoutes(rows, K, E)
-        PrefillGroupedRoutedMoE(tf_ctx).encode_group_routes(idx, w, rows, K, E, ref)
+        ctx.set_router_tensorcore_min_rows(min_rows)
+        idx, w = torch.full((rows, K), -1, dtype=torch.int32, device="cuda"), dev_zeros_u16(rows * K)
+        PrefillRouter(ctx).encode_gemma4_block(W, S, B, hid, eff, gain, idx, w, rows, E, D, K, D)
         torch.cuda.synchronize()
-        assert torch.equal(routes.sorted_pairs, ref.sorted_pairs) and torch.equal(routes.per_expert_counts, ref.per_expert_counts)
-        assert torch.equal(routes.per_expert_offsets, ref.per_expert_offsets) and torch.equal(routes.counters[:2], ref.counters[:2])
         return from_dev(idx, np.uint32), from_dev(w, np.uint16)
 
     try:
         one, two, again = run(0xFFFFFFFF), run(65), run(65)
     finally:
-        tf_ctx.set_router_tensorcore_min_rows(256)
+        ctx.close()
     for got in (two, again):
         assert np.array_equal(got[0], one[0]) and np.array_equal(got[1], one[1])
 
@@ -105,6 +103,51 @@ def _forward(tf_ctx, layer, ws, x):
     torch.cuda.synchronize()
     assert tf_ctx.device_status() == 0
     return y
+
+
+@pytest.mark.parametrize("tokens,skew", [(65, 0.0), (130, 6.0), (200, 0.0), (255, 0.0), (255, 9.0), (65, -np.inf), (201, -np.inf)])
+def test_block_routing_tables_equal_the_two_calls(tf_ctx, layer, tokens, skew):
+    """Block forwards of 65 to 255 tokens group in the last block of the router's second launch: every table equals what the
+    router and the grouping launch write. With -inf only three experts stay selectable and the selection repeats expert 0.
+    One row has a NaN. Twice, to show that the ticket is reset."""
+    import torch
+    from turbo_fieldfare_b200.kernels import DeviceRoutes, PrefillGroupedRoutedMoE, PrefillRouter
+    from turbo_fieldfare_b200.stack import MoEBlock, Workspace, device_view_u8
+    E, D, K, n = 128, 2816, 8, tokens * 8
+    bias = np.zeros(E, np.float32)
+    bias[[3, E - 1]] = skew, skew / 2
+    if skew == -np.inf:
+        bias[:] = skew
+        bias[[2, 5, E - 1]] = 0.0
+    layer.set_logit_bias(bias)
+    try:
+        gen = torch.Generator(device="cuda").manual_seed(tokens)
+        x = torch.randn(tokens, D, generator=gen, device="cuda").half()
+        x[7, 100] = float("nan")
+        r = layer.router
+        idx, w, ref = torch.full((tokens, K), -1, dtype=torch.int32, device="cuda"), dev_zeros_u16(n), DeviceRoutes(tokens, K, E)
+        PrefillRouter(tf_ctx).encode_gemma4_block(r.buffer, r.buffer, r.buffer, x, layer.effective_scale, layer.per_expert_scale, idx, w, tokens, E,
+                                                  D, K, D, logit_bias=layer.logit_bias, scales_offset=r.s_off, biases_offset=r.b_off)
+        PrefillGroupedRoutedMoE(tf_ctx).encode_group_routes(idx, w, tokens, K, E, ref)
+        torch.cuda.synchronize()
+        ng, nch = ref.counters[:2].tolist()
+        assert ref.counters[2].item() == n and ref.per_expert_counts.sum().item() == n
+        if skew == -np.inf:
+            assert ng == 4 and ref.per_expert_counts[0].item() == (tokens - 1) * (K - 3) + K         # the NaN row has nothing else
+        ws, y = Workspace(tf_ctx, tokens, D, 704, 2112, K, E), torch.zeros_like(x)
+        sizes = dict(sorted_pairs=n * 4, per_expert_offsets=E, per_expert_counts=E, groups=ng * 3, chunk_group=nch, chunk_start=ng, counters=4)
+        for attempt in range(2):
+            MoEBlock(tf_ctx, layer).forward(x, y, tokens, ws)
+            torch.cuda.synchronize()
+            got_idx, got_w = ws.routing(tokens)
+            assert np.array_equal(got_idx.reshape(-1), from_dev(idx, np.uint32).reshape(-1)) and np.array_equal(got_w.reshape(-1), from_dev(w, np.uint16))
+            tables = tf_ctx.lib.tf_workspace_routes(ws.handle).contents
+            for name, words in sizes.items():
+                got = device_view_u8(getattr(tables, name), words * 4).view(torch.int32)
+                assert torch.equal(got, getattr(ref, name)[:words]), (name, attempt)
+        assert tf_ctx.device_status() == 0
+    finally:
+        layer.set_logit_bias(None)
 
 
 # 103 / 104 tokens lie on either side of the rule for 16-token chunks; a bias towards few experts gives them chunks of every fill
