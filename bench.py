@@ -623,9 +623,9 @@ def measure_roofline(torch, ctx, stack, ws, h, batch, PrefillRouter, PrefillGrou
     bytes_total = sum(touched) * EXPERT_BYTES + len(layers) * batch * (D * 2 + K * D * 4)   # weights + activations in/out
     achieved = bytes_total / (ms * 1e-3) / 1e9
     # DRAM traffic per launch: the ncu capture of the same kernel pair at 64 tokens (summary under profiles/, kernel
-    # grouped_ksplit_kernel, routed decode batch 64) read and wrote 435.6 MB for 421.5 MB of touched expert planes,
-    # 1.033 bytes per algorithmic byte; traffic grows with the experts touched, so it is scaled by that ratio.
-    traffic_ratio = 435.63 / 421.52
+    # grouped_ksplit_kernel, routed decode batch 64) read and wrote 429.8 MB for 414.8 MB of touched expert planes and 6.1 MB
+    # of activations and results; traffic grows with the experts touched, so it is scaled by that ratio.
+    traffic_ratio = 429.83 / (414.83 + 6.13)
     return {"bound": "hbm", "kernel": "grouped_ksplit_kernel + grouped_down_kernel (routed gate/up and down launches of one layer, batch 64)",
             "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak, "peak_source": peak_src,
             "traffic": bytes_total / launches * traffic_ratio, "traffic_source": "ncu capture at 64 tokens, scaled by experts touched",
@@ -755,7 +755,7 @@ def case_gemv(args) -> None:
 
 
 def case_lmhead(args) -> None:
-    """Greedy LM head (final RMSNorm, tied int4 head of --rows x 2816, argmax): four launches per token."""
+    """Greedy LM head (final RMSNorm, tied int4 head of --rows x 2816, argmax): three launches per token."""
     import torch
     from turbo_fieldfare_b200.kernels import LMHeadChainInt4, TurboContext
     from turbo_fieldfare_b200.stack import AffineTensor

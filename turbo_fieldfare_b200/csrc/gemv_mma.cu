@@ -219,8 +219,8 @@ tf_status launch_gemv_mma(tf_context* ctx, void* stream, const uint8_t* W, const
 
 // The greedy LM head's product: *argmax is zero before. Must follow, on the stream, the
 // launch that writes x, and that launch must start after everything before it (no programmatic launch of its own).
-// Blocks of 128 rows, as for the stored form (with 64 rows the call takes as long: 103 us either way, before the blocks
-// stopped waiting for their atomics, 96 since).
+// Blocks of 128 rows, as for the stored form (64 rows took as long when both were measured, 103 us; since the blocks stopped
+// waiting for their atomics the call takes 97 to 102 us for 262144 rows, 89 in a loop of nothing else).
 tf_status launch_gemv_mma_argmax(tf_context* ctx, void* stream, const uint8_t* W, const uint16_t* S, const uint16_t* B,
                                  const uint16_t* x, uint32_t m, uint32_t n, unsigned long long* argmax, const char* name) {
     const size_t smem = gemv_mma_smem_bytes(n);

@@ -27,10 +27,11 @@
 // A persistent grid walks (group, token tile, weight-row tile) work items derived on the device from the
 // routing metadata. Every mbarrier wait is bounded; on expiry the kernel records a code, waits for its copies and leaves.
 //
-// What bounds it (clock counters around the waits, 4096 x 18944 x 2816, 1.14 PFLOP/s): with 128 tokens per tile the
-// activations, 64 bytes per clock and SM out of L2; with few tokens the dequantisers' integer instructions, about 700 clocks
-// per stage where an SM's share of the HBM rate gives 740. Each single-warp role pays 100 to 150 clocks per wait or commit
-// whatever N is, so a stage is as deep as tensor memory allows.
+// What bounds it: with 128 tokens per tile the activations, 64 bytes per clock and SM out of L2 (clock counters around the
+// waits, 4096 x 18944 x 2816, 1.14 PFLOP/s). With few tokens no unit: at 21 tokens per expert a stage takes 1480 clocks in the
+// gate/up launch and 1720 in the down launch, of which the dequantisers' integer instructions account for about 700, the MMAs
+// for 250, and an SM's share of the HBM rate for 740; the rest is the hand-over between the roles. Each single-warp role pays
+// 100 to 150 clocks per wait or commit whatever N is, so a stage is as deep as tensor memory allows.
 //
 // Column order. The cheapest nibble extraction yields the eight codes of a 32-bit word in the order
 // (0,4,1,5,2,6,3,7). A dot product does not care about the order as long as both operands agree, so the

@@ -682,7 +682,8 @@ static tf_status launch_router(tf_context* ctx, void* stream, const uint8_t* W, 
 // tf_router_gemma4_block_grouped; approx_scratch ([query_count, num_experts] pairs of floats) and ticket (a zero word), when
 // given, belong to the caller's workspace: blocks of 65 to kRouterFusedGroupRows rows then route in two launches, the second of
 // which groups them (the block that finishes the last row does it). One block per row computes every canonical logit there
-// otherwise: 168 + 8 us against 11 + 17 for 200 rows. Larger blocks group with launches of their own, which many SMs share.
+// otherwise: 168 us and a grouping launch against 11 + 36 for 200 rows (cold; about half of the 36 is the grouping by one
+// block). Larger blocks group with launches of their own, which many SMs share; nothing between the two was measured.
 tf_status router_block_grouped(tf_context* ctx, void* stream, const void* weights, uint64_t weights_off,
                                const void* scales, uint64_t scales_off, const void* biases, uint64_t biases_off,
                                const void* hidden, uint64_t hidden_off, tf_dtype hidden_dtype,

@@ -173,7 +173,8 @@ __device__ __forceinline__ float gelu_tanh(float x) {
 // Programmatic dependent launch: a kernel launched with launch_pdl may start (block scheduling, shared-memory set-up)
 // while its predecessor on the stream is still draining; pdl_wait() returns once the predecessor has completed and its
 // writes are visible, so it comes before the first access to anything another kernel produces (and before any
-// write). Without the launch attribute both instructions do nothing.
+// write). Some kernels request their weights before it: those are written by plain launches and copies only, which never let
+// a dependent start early. Without the launch attribute both instructions do nothing.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

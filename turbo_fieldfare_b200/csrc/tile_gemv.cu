@@ -1,5 +1,6 @@
 // One-token kernels over 16-row tiles (tile_gemv.cuh): the int4 GEMV of matrices too small for the streaming kernel, and the
-// routed experts' gate/up and down phases of a single token. One layer's operators for one token: 80 -> 59 us.
+// routed experts' gate/up and down phases of a single token. One layer's operators for one token as
+// a host calls them one by one: 80 -> 59 us, 44 with the wrappers' cheaper look-up of the stream.
 #include "tile_gemv.cuh"
 
 namespace tf {
