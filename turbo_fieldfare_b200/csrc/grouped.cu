@@ -617,11 +617,7 @@ grouped_ksplit_kernel(const GroupedArgs args) {
 
             const uint32_t ring_item = smem_base + st * lay.stage_bytes() + lane_code_off;
             const uint32_t sb_item = smem_base + st * lay.stage_bytes() + lay.off_sb_in_stage();
-            // partial sums for the reducer: buffer li % kRedStages, 512 bytes per (warp, matrix, 8 tokens)
-            const uint32_t r = li % kRedStages, ruse = li / kRedStages;
-            const uint32_t red_w = red_base + r * lay.red_stage_bytes() + (warp * NMAT * NT) * 512 + (g * 8 + 2 * t) * 4;
             if constexpr (NT == 1) {
-            float y[NMAT][4];
             // All codes of the item first, then the MMAs interleaved over the (matrix, group) pairs: the four
             // MMAs of one group form a dependent chain through its accumulator, so consecutive instructions
             // always belong to different chains and the tensor pipe stays full.
@@ -666,6 +662,7 @@ grouped_ksplit_kernel(const GroupedArgs args) {
                     mma16816_acc(c[m][i], wa[m][i].y & 0x00F000F0u, wb[m][i].y & 0x00F000F0u,
                                  (wa[m][i].y >> 8) & 0x00F000F0u, (wb[m][i].y >> 8) & 0x00F000F0u, xb[0][i][3]);
             }
+            float y[NMAT][4];
 #pragma unroll
             for (int m = 0; m < NMAT; ++m) {
                 const uint32_t sm_s = sb_item + (m * 2) * lay.sb_plane_bytes(), sm_b = sm_s + lay.sb_plane_bytes();
@@ -706,7 +703,10 @@ grouped_ksplit_kernel(const GroupedArgs args) {
             // this warp is done with the stage (codes and scales are in registers or consumed)
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_empty(st));
+            // partial sums for the reducer: buffer li % kRedStages, 512 bytes per (warp, matrix, 8 tokens)
+            const uint32_t r = li % kRedStages, ruse = li / kRedStages;
             if (!mbar_wait(bar_red_free(r), (ruse & 1) ^ 1)) { fail = kErrTimeoutRedFree; break; }
+            const uint32_t red_w = red_base + r * lay.red_stage_bytes() + (warp * NMAT) * 512 + (g * 8 + 2 * t) * 4;
 #pragma unroll
             for (int m = 0; m < NMAT; ++m) {
                 sts_f32x2(red_w + m * 512, y[m][0], y[m][1]);
@@ -714,6 +714,8 @@ grouped_ksplit_kernel(const GroupedArgs args) {
             }
             } else {
             // the reducer's buffer is claimed first, so that a matrix's sums leave the registers before the next matrix begins
+            const uint32_t r = li % kRedStages, ruse = li / kRedStages;
+            const uint32_t red_w = red_base + r * lay.red_stage_bytes() + (warp * NMAT * NT) * 512 + (g * 8 + 2 * t) * 4;
             if (!mbar_wait(bar_red_free(r), (ruse & 1) ^ 1)) { fail = kErrTimeoutRedFree; break; }
 #pragma unroll
             for (int m = 0; m < NMAT; ++m) {
@@ -782,7 +784,7 @@ grouped_ksplit_kernel(const GroupedArgs args) {
             if (lane == 0) mbar_arrive(bar_empty(st));               // this warp is done with the stage
             }
             __syncwarp();
-            if (lane == 0) mbar_arrive(bar_part_full(r));
+            if (lane == 0) mbar_arrive(bar_part_full(li % kRedStages));
             if (li + 1 < n_items) advance(cur);
         }
         if (fail && lane == 0) atomicCAS(args.error, 0u, fail);
