@@ -26,11 +26,13 @@ def _dense(o, mat):
     return q * s + b
 
 
-# K: one group, an odd last group, whole and partial stages of four groups; N: below, at and beyond a 128-row tile; M: tiles of
-# one MMA step, of unequal last steps, exactly full, and several of equal size. y_off = 2 takes the element stores.
+# K: one group, an odd last group, whole and partial stages of four groups, the longest rows (whose scale planes leave room for one
+# buffer: from 7040 on, with one and with two tiles per block); N: below, at and beyond a 128-row tile; M: tiles of one MMA
+# step, of unequal last steps, exactly full, and several of equal size. y_off = 2 takes the element stores.
 @pytest.mark.parametrize("M,N,K,y_off", [(1, 8, 64, 0), (15, 72, 128, 0), (16, 128, 192, 2), (17, 136, 320, 0), (63, 256, 704, 0), (65, 128, 2112, 2),
                                          (113, 264, 448, 0), (128, 2112, 256, 0), (129, 128, 2816, 0), (270, 384, 704, 0), (1000, 40, 4096, 0),
-                                         (300, 64, 8192, 0)])
+                                         (300, 64, 8192, 0), (128, 128, 6976, 0), (129, 136, 7040, 0), (1200, 2112, 7104, 0), (600, 5000, 8256, 0),
+                                         (33, 72, 9024, 0)])
 def test_qmm_token_tiles(tf_ctx, oracle, M, N, K, y_off):
     import torch
     from turbo_fieldfare_b200.kernels import MPPPrefillInt4QMM

@@ -69,7 +69,6 @@ struct QmmPlan {
     uint32_t sc_bufs;       // scale-plane buffers
     uint32_t plane_bytes;   // one scale or bias plane of a tile (128 / NMAT rows)
     uint32_t sc_bytes;      // one buffer: NMAT x (scale plane, bias plane)
-    uint32_t tok_max;       // tokens per tile
     uint32_t off_b, off_sc, off_stage, off_table, off_bars, total;
 };
 
@@ -245,11 +244,11 @@ __device__ __forceinline__ uint4 dequant8_wide(uint32_t w, __half2 s, __half2 b)
 // Position of column k within its eight-column block in the PERMUTED order.
 __device__ __forceinline__ uint32_t permuted_col(uint32_t k) { return (k & ~7u) | ((k & 3u) << 1) | ((k >> 2) & 1u); }
 
-// Tokens per tile of a group: as few tiles as tok_max allows, of equal size (a multiple of 16, the step of the MMA's N).
+// Tokens per tile of a group: as few tiles as kQmmTokMax allows, of equal size (a multiple of 16, the step of the MMA's N).
 // 256 + 14 tokens are three tiles of 96, not 128 + 128 + 14: the weights are dequantised once per tile, and below about
 // 80 tokens that takes longer than the tile's MMAs.
-__host__ __device__ inline uint32_t qmm_tokens_per_tile(uint32_t count, uint32_t tok_max) {
-    const uint32_t tiles = (count + tok_max - 1) / tok_max;
+__host__ __device__ inline uint32_t qmm_tokens_per_tile(uint32_t count) {
+    const uint32_t tiles = (count + kQmmTokMax - 1) / kQmmTokMax;
     return ((count + tiles - 1) / tiles + 15u) & ~15u;
 }
 
@@ -257,7 +256,7 @@ __host__ __device__ inline uint32_t qmm_tokens_per_tile(uint32_t count, uint32_t
 // groups took 29 us for 128 of them, on the critical path before every routed GEMM; this takes about 2.)
 __global__ void __launch_bounds__(TF_MAX_ROUTER_EXPERTS)
 qmm_prepare_kernel(uint4* __restrict__ groups, uint32_t* __restrict__ totals, const tf_group* __restrict__ route_groups,
-                   const uint32_t* __restrict__ route_counters, uint32_t dense_tokens, uint32_t dense_per_tile, uint32_t tok_max) {
+                   const uint32_t* __restrict__ route_counters, uint32_t dense_tokens, uint32_t dense_per_tile) {
     __shared__ uint32_t warp_tiles[TF_MAX_ROUTER_EXPERTS / kWarp], warp_top[TF_MAX_ROUTER_EXPERTS / kWarp];
     const uint32_t warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
     pdl_launch_dependents();
@@ -268,7 +267,7 @@ qmm_prepare_kernel(uint4* __restrict__ groups, uint32_t* __restrict__ totals, co
         if (route_groups) {
             const tf_group rg = route_groups[threadIdx.x];
             row = rg.pair_start; count = rg.pair_count; expert = rg.expert;
-            per = qmm_tokens_per_tile(count > 0 ? count : 1u, tok_max);
+            per = qmm_tokens_per_tile(count > 0 ? count : 1u);
         } else {
             count = dense_tokens; per = dense_per_tile;
         }
@@ -724,22 +723,25 @@ static tf_status make_w_map(tf_context* ctx, CUtensorMap* map, const void* w, ui
 
 // Divides the 227 KB of shared memory for K columns. Packed codes first (four stages keep 48 to 64 KB in flight, what an
 // SM's share of the HBM rate needs at its latency), the activation ring takes what the scale planes leave: three slots of
-// 128 tokens at K = 2816. Long rows give up stages, then tokens per tile.
+// 128 tokens at K = 2816. Long rows give up stages, then (from K = 7040 on) the second buffer of scale planes: the next tile's
+// planes are then copied between two tiles, which costs less than halving the tokens per tile (2000 x 2112 x 8192: 104 us with
+// one buffer, 152 with two and tiles of 64 tokens).
+constexpr uint32_t kQmmMaxK = 9024;
 static bool qmm_plan(uint32_t k, uint32_t nmat, QmmPlan* p) {
+    if (k > kQmmMaxK) return false;
     const uint32_t budget = 227u * 1024u - 1024u;                  // less the alignment slack
     const uint32_t ng = k / kGroup;
     p->plane_bytes = ((kQmmRows / nmat) * ng * 2u + 15u) & ~15u;
     p->sc_bytes = nmat * 2 * p->plane_bytes;
-    p->sc_bufs = 4 * p->sc_bytes <= 48u * 1024u ? 4u : 2u;
-    const uint32_t fixed = p->sc_bufs * p->sc_bytes + kQmmStageBytes + TF_MAX_ROUTER_EXPERTS * 16u + 1024u;
     const uint32_t slot = kQmmTokMax * kQmmHalfK * 2u;              // 32 KB
+    uint32_t fixed = 0;
     p->raw_stages = 0;
-    for (uint32_t raw = kQmmRawMax; raw >= 2 && !p->raw_stages; --raw)
-        if (fixed + raw * kQmmRawBytes + 2 * slot <= budget) { p->raw_stages = raw; p->tok_max = kQmmTokMax; }
-    if (!p->raw_stages) {                                          // very long rows: two slots of 64 tokens
-        if (fixed + 2 * kQmmRawBytes + slot > budget) return false;
-        p->raw_stages = 2;
-        p->tok_max = kQmmTokMax / 2;
+    for (p->sc_bufs = 4 * p->sc_bytes <= 48u * 1024u ? 4u : 2u;; p->sc_bufs = 1) {
+        fixed = p->sc_bufs * p->sc_bytes + kQmmStageBytes + TF_MAX_ROUTER_EXPERTS * 16u + 1024u;
+        for (uint32_t raw = kQmmRawMax; raw >= 2 && !p->raw_stages; --raw)
+            if (fixed + raw * kQmmRawBytes + 2 * slot <= budget) p->raw_stages = raw;
+        if (p->raw_stages) break;
+        if (p->sc_bufs == 1) return false;
     }
     p->b_bytes = (budget - fixed - p->raw_stages * kQmmRawBytes) & ~2047u;
     p->off_b = p->raw_stages * kQmmRawBytes;
@@ -753,10 +755,10 @@ static bool qmm_plan(uint32_t k, uint32_t nmat, QmmPlan* p) {
 
 // Tokens per tile of a dense launch: rounds of the grid x the time of a tile, which is the larger of its MMAs (four clocks
 // per token and 128 columns) and its dequantisation (about 330 clocks per 128 columns), plus a fixed part.
-static uint32_t qmm_dense_per_tile(uint32_t tokens, uint32_t wrow_tiles, uint32_t halves, uint32_t tok_max, uint32_t sms) {
+static uint32_t qmm_dense_per_tile(uint32_t tokens, uint32_t wrow_tiles, uint32_t halves, uint32_t sms) {
     uint32_t best = 16;
     uint64_t best_cost = ~0ull;
-    for (uint32_t per = tok_max; per >= 16; per -= 16) {
+    for (uint32_t per = kQmmTokMax; per >= 16; per -= 16) {
         const uint64_t tiles = (uint64_t)wrow_tiles * ((tokens + per - 1) / per);
         const uint64_t step = 4ull * per > 330 ? 4ull * per : 330;
         const uint64_t cost = ((tiles + sms - 1) / sms) * (halves * step + 1500);
@@ -773,7 +775,7 @@ static tf_status launch_qmm_prepare(tf_context* ctx, void* stream, QmmArgs& a, i
     a.groups = static_cast<uint4*>(ctx->qmm_groups) + table * (TF_MAX_ROUTER_EXPERTS + 1);
     a.totals = reinterpret_cast<uint32_t*>(a.groups + TF_MAX_ROUTER_EXPERTS);
     launch_pdl(qmm_prepare_kernel, dim3(1), dim3(TF_MAX_ROUTER_EXPERTS), 0, static_cast<cudaStream_t>(stream), a.groups, a.totals,
-               a.route_groups, a.route_counters, a.dense_tokens, a.dense_per_tile, a.plan.tok_max);
+               a.route_groups, a.route_counters, a.dense_tokens, a.dense_per_tile);
     return check_launch(ctx, "qmm_prepare");
 }
 
@@ -792,7 +794,7 @@ static tf_status launch_qmm(tf_context* ctx, void* stream, QmmArgs& a, const voi
     uint32_t boxes = 16u | 32u | 64u | 128u;
     if (dense) {
         a.dense_per_tile = qmm_dense_per_tile(a.dense_tokens, (a.rows + kMatRows - 1) / kMatRows, (a.k + kQmmHalfK - 1) / kQmmHalfK,
-                                              a.plan.tok_max, (uint32_t)ctx->sm_count);
+                                              (uint32_t)ctx->sm_count);
         const uint32_t rest = (a.dense_tokens % a.dense_per_tile + 15u) & ~15u;
         boxes = rest | (a.dense_tokens >= a.dense_per_tile ? a.dense_per_tile : 0u);
     }
