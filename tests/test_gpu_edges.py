@@ -191,9 +191,11 @@ def test_one_token_block_equals_its_row_in_a_pair(tf_ctx, layer):
 
 
 @pytest.mark.parametrize("scale", [1.0, 1e-4])
-@pytest.mark.parametrize("m,n", [(1, 64), (15, 128), (16, 192), (17, 2112), (704, 2816), (4095, 320), (33, 16384)])
+@pytest.mark.parametrize("m,n", [(1, 64), (15, 128), (16, 192), (17, 2112), (704, 2816), (4095, 320), (33, 16384), (700, 4160), (2368, 4096),
+                                 (2369, 4160)])
 def test_tile_gemv(tf_ctx, oracle, m, n, scale):
-    """Remainders of the 16-row tile and of the four-group part; small activations keep their bits."""
+    """Remainders of the 16-row tile and of the four-group part, both sides of the rule for sixteen warps (more than 4096
+    columns, a block per SM at most); small activations keep their bits."""
     import torch
     from turbo_fieldfare_b200.kernels import DequantInt4GEMV
     o = oracle

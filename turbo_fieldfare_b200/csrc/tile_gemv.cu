@@ -7,9 +7,9 @@ namespace tf {
 
 constexpr int kTileWarps = 8, kTileThreads = kTileWarps * kWarp;
 
-// y[m] = deq4(W[m, n]) . x[n]: a block per 16 rows; part p of the columns belongs to warp p % 8, two of its parts in flight.
-template <bool SB_FP16, bool OUT_F32>
-__global__ void __launch_bounds__(kTileThreads, 2)
+// y[m] = deq4(W[m, n]) . x[n]: a block per 16 rows; part p of the columns belongs to warp p % WARPS, two of its parts in flight.
+template <bool SB_FP16, bool OUT_F32, int WARPS>
+__global__ void __launch_bounds__(WARPS * kWarp, 16 / WARPS)
 tile_gemv_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S, const uint16_t* __restrict__ B,
                  const uint16_t* __restrict__ x, void* __restrict__ y, uint32_t m, uint32_t ng) {
     extern __shared__ __align__(16) uint8_t smem[];
@@ -22,14 +22,14 @@ tile_gemv_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S, 
     pdl_launch_dependents();
     pdl_wait();
     TileOperands<2> o;
-    tile_load<2>(o, W, S, B, row0, m, ng, warp, kTileWarps);
+    tile_load<2>(o, W, S, B, row0, m, ng, warp, WARPS);
     tile_stage_x(x, 0, 1, ng, frag, xsum);
     __syncthreads();
-    for (uint32_t p0 = warp; p0 < parts; p0 += 2 * kTileWarps) {
-        if (p0 != (uint32_t)warp) tile_load<2>(o, W, S, B, row0, m, ng, p0, kTileWarps);
+    for (uint32_t p0 = warp; p0 < parts; p0 += 2 * WARPS) {
+        if (p0 != (uint32_t)warp) tile_load<2>(o, W, S, B, row0, m, ng, p0, WARPS);
 #pragma unroll
         for (int n = 0; n < 2; ++n) {
-            const uint32_t p = p0 + n * kTileWarps;
+            const uint32_t p = p0 + n * WARPS;
             if (p < parts) {
                 const float2 a = tile_part<SB_FP16, 2>(o, n, frag, xsum, ng, p);
                 if ((lane & 3) == 0) { sums[p * 16 + (lane >> 2)] = a.x; sums[p * 16 + (lane >> 2) + 8] = a.y; }
@@ -149,17 +149,27 @@ static size_t tile_gemv_smem(uint32_t ng, uint32_t mats) {
 // Aligned planes of any row count; vectors up to 16384 columns (shared memory).
 bool tile_gemv_eligible(const void* W, const void* x, uint32_t n) { return aligned(W, 16) && aligned(x, 16) && n % kGroup == 0 && n <= 16384; }
 
-tf_status launch_tile_gemv(tf_context* ctx, void* stream, const uint8_t* W, const uint16_t* S, const uint16_t* B, const uint16_t* x,
-                           void* y, bool out_f32, uint32_t m, uint32_t n, bool sb_fp16, const char* name) {
-    const uint32_t ng = n / kGroup;
+// Two blocks of eight warps fit an SM. Rows of more than 4096 columns take several rounds of loads per warp, one memory latency
+// each; where every block has an SM to itself, sixteen warps halve the rounds (704 x 16384: 22.8 -> 13.2 us a call, 1000 x 8192:
+// 12.6 -> 7.2; the warp-per-row kernel takes 20.5 and 12.3).
+template <int WARPS>
+static tf_status launch_tile_gemv_warps(tf_context* ctx, void* stream, const uint8_t* W, const uint16_t* S, const uint16_t* B, const uint16_t* x,
+                                        void* y, bool out_f32, uint32_t m, uint32_t ng, bool sb_fp16, const char* name) {
     const size_t smem = tile_gemv_smem(ng, 1);
-    auto k = sb_fp16 ? (out_f32 ? tile_gemv_kernel<true, true> : tile_gemv_kernel<true, false>)
-                     : (out_f32 ? tile_gemv_kernel<false, true> : tile_gemv_kernel<false, false>);
+    auto k = sb_fp16 ? (out_f32 ? tile_gemv_kernel<true, true, WARPS> : tile_gemv_kernel<true, false, WARPS>)
+                     : (out_f32 ? tile_gemv_kernel<false, true, WARPS> : tile_gemv_kernel<false, false, WARPS>);
     static DeviceSmemCache configured[4];
     if (smem > 48 * 1024)
         if (tf_status s = ensure_dynamic_smem(ctx, k, configured[(sb_fp16 ? 2 : 0) + (out_f32 ? 1 : 0)], smem)) return s;
-    launch_pdl(k, dim3((m + kTileRows16 - 1) / kTileRows16), dim3(kTileThreads), smem, static_cast<cudaStream_t>(stream), W, S, B, x, y, m, ng);
+    launch_pdl(k, dim3((m + kTileRows16 - 1) / kTileRows16), dim3(WARPS * kWarp), smem, static_cast<cudaStream_t>(stream), W, S, B, x, y, m, ng);
     return check_launch(ctx, name);
+}
+
+tf_status launch_tile_gemv(tf_context* ctx, void* stream, const uint8_t* W, const uint16_t* S, const uint16_t* B, const uint16_t* x,
+                           void* y, bool out_f32, uint32_t m, uint32_t n, bool sb_fp16, const char* name) {
+    const bool alone = (m + kTileRows16 - 1) / kTileRows16 <= (uint32_t)ctx->sm_count;
+    return n > 4096 && alone ? launch_tile_gemv_warps<16>(ctx, stream, W, S, B, x, y, out_f32, m, n / kGroup, sb_fp16, name)
+                             : launch_tile_gemv_warps<8>(ctx, stream, W, S, B, x, y, out_f32, m, n / kGroup, sb_fp16, name);
 }
 
 // Blobs and packed sub-tensor offsets must be 16-byte aligned (checked by the callers).
