@@ -271,3 +271,26 @@ def test_router_threshold_holds_for_block_forwards(layer, tmp_path, rows, two_la
         ws.close()
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("d", [1, 64, 255, 256, 257, 512, 513, 1024, 1025, 2048, 2049, 3072, 3073, 4096, 4097])
+@pytest.mark.parametrize("bf16,weighted", [(False, True), (True, True), (False, False)])
+def test_rmsnorm_row_lengths(tf_ctx, oracle, d, bf16, weighted):
+    """Both sides of every row length at which the norm takes another form; the padding between rows stays as it was."""
+    import torch
+    from turbo_fieldfare_b200.kernels import RMSNorm
+    o, rows, stride = oracle, 5, d + 3
+    rng = np.random.default_rng(d)
+    to_bits, to_float = (o.f32_to_bf16, o.bf16_to_f32) if bf16 else (o.f32_to_f16, o.f16_to_f32)
+    x16, w16 = to_bits(rng.standard_normal((rows, stride)).astype(np.float32)), o.f32_to_bf16(1 + 0.1 * rng.standard_normal(d).astype(np.float32))
+    y = dev_zeros_u16(rows * stride, fill=0x3C01)
+    RMSNorm(tf_ctx).encode(to_dev(x16), to_dev(w16) if weighted else None, y, rows, d, stride, act_dtype=0 if bf16 else 1)
+    torch.cuda.synchronize()
+    out = from_dev(y, np.uint16).reshape(rows, stride)
+    assert np.all(out[:, d:] == 0x3C01)
+    x = to_float(x16)[:, :d].astype(np.float64)
+    ref = x / np.sqrt((x * x).mean(axis=1, keepdims=True) + 1e-6) * (o.bf16_to_f32(w16).astype(np.float64) if weighted else 1.0)
+    # the result's rounding (8 or 11 significant bits), fp32 sums of up to 4097 squares (half of their relative error) and three fp32
+    # roundings
+    bound = np.abs(ref) * ((2.0 ** -8 if bf16 else 2.0 ** -11) + 2.0 ** -18) + 2.0 ** -25
+    assert np.all(np.abs(to_float(out[:, :d]) - ref) <= bound)
