@@ -294,3 +294,32 @@ def test_rmsnorm_row_lengths(tf_ctx, oracle, d, bf16, weighted):
     # roundings
     bound = np.abs(ref) * ((2.0 ** -8 if bf16 else 2.0 ** -11) + 2.0 ** -18) + 2.0 ** -25
     assert np.all(np.abs(to_float(out[:, :d]) - ref) <= bound)
+
+
+# 296 and 376 blocks of 16 rows over all slots, on either side of the rule for rows of more than 3072 columns, and a split call
+@pytest.mark.parametrize("D,F", [(3072, 752), (3136, 592), (3136, 752)])
+def test_phase1_long_rows(tf_ctx, oracle, D, F):
+    import torch
+    from turbo_fieldfare_b200.kernels import MoE
+    o, K = oracle, 8
+    rng = np.random.default_rng(D + F)
+    mats = [(config0_matrix(o, F, D, rng), config0_matrix(o, F, D, rng)) for _ in range(K)]
+    parts = lambda m: [m.packed.reshape(-1), m.scales.view(np.uint8).reshape(-1), m.biases.view(np.uint8).reshape(-1)]
+    blobs = [to_dev(np.concatenate(parts(g) + parts(u))) for g, u in mats]
+    w, s = F * D // 2, F * (D // 64) * 2
+    coff = ExpertOffsets(0, w, w + s, w + 2 * s, 2 * w + 2 * s, 2 * w + 3 * s, 0, 0, 0)
+    x16 = o.f32_to_f16(rng.standard_normal(D).astype(np.float32))
+    table, x, moe = blob_table(blobs), to_dev(x16), MoE(tf_ctx)
+    whole, split = dev_zeros_u16(K * F + 8, fill=0x7E00), dev_zeros_u16(K * F + 8, fill=0x7E00)
+    moe.encode_routed_phase1(table, coff, x, whole, D, F, K)
+    moe.encode_routed_phase1_subset(table, coff, x, split, D, F, K, to_dev(np.array([6, 1], np.uint32)), 2)
+    moe.encode_routed_phase1_subset(table, coff, x, split, D, F, K, to_dev(np.array([0, 2, 3, 4, 5, 7], np.uint32)), 6)
+    torch.cuda.synchronize()
+    assert torch.equal(whole, split)
+    out, x64 = from_dev(whole, np.uint16), o.f16_to_f32(x16).astype(np.float64)
+    assert np.all(out[K * F:] == 0x7E00)
+    for k, (g, u) in enumerate(mats):
+        gt, up = _dense(o, g) @ x64, _dense(o, u) @ x64
+        ref = 0.5 * gt * (1 + np.tanh(np.clip(0.7978845608028654 * (gt + 0.044715 * gt ** 3), -20, 20))) * up
+        # the result's rounding (2^-11, a third of it in the root mean square) and fp32 sums of 3136 products
+        assert o.rel_l2(o.f16_to_f32(out[k * F:(k + 1) * F]), ref) < 5e-4

@@ -153,9 +153,9 @@ static tf_status launch_phase1(tf_context* ctx, void* stream, const void* const*
     if (slots == 0) return TF_OK;
     const size_t smem = stage_x_bytes((int)d);
     TF_REQUIRE(ctx, smem <= 96 * 1024, TF_ERR_UNSUPPORTED, "%s: D too large", name);
-    if (tile_gate_up_eligible(d, x))
+    if (tile_gate_up_eligible(ctx, d, f, top_k, x))
         return launch_tile_gate_up(ctx, stream, blobs, offsets, x, acts, d, f, top_k, slot_map, slots, name);
-    // x off the 16-byte grid: the row kernel loads it element by element
+    // x off the 16-byte grid (the row kernel loads it element by element), or long rows of many blocks
     if (smem > 48 * 1024)
         TF_CUDA(ctx, cudaFuncSetAttribute(moe_phase1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     dim3 grid((f + kP1RowsPerBlock - 1) / kP1RowsPerBlock, slots);

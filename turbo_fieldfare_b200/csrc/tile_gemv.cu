@@ -173,7 +173,13 @@ tf_status launch_tile_gemv(tf_context* ctx, void* stream, const uint8_t* W, cons
 }
 
 // Blobs and packed sub-tensor offsets must be 16-byte aligned (checked by the callers).
-bool tile_gate_up_eligible(uint32_t d, const void* x) { return d % kGroup == 0 && d <= 16384 && aligned(x, 16); }
+// Up to 3072 columns a warp has all of its codes in flight at once; beyond, the tiles win while the blocks of all slots are at most
+// two and a half rounds of one per SM (8 experts, row kernel / tiles: 4096 x 704 19.2 / 18.7 us, 6144 x 704 27.8 / 22.1, 4096 x
+// 1408 28.5 / 29.5, 8192 x 4096 120 / 146). The number of active slots doesn't count: a split call has the bits of a whole one.
+bool tile_gate_up_eligible(tf_context* ctx, uint32_t d, uint32_t f, uint32_t top_k, const void* x) {
+    const uint64_t blocks = (uint64_t)((f + kTileRows16 - 1) / kTileRows16) * top_k;
+    return d % kGroup == 0 && d <= 16384 && aligned(x, 16) && (d <= 3072 || 2 * blocks <= 5ull * (uint32_t)ctx->sm_count);
+}
 bool tile_down_eligible(uint32_t f, const void* acts) { return f % kGroup == 0 && f <= 8192 && aligned(acts, 16); }
 
 tf_status launch_tile_gate_up(tf_context* ctx, void* stream, const void* const* blobs, const tf_expert_offsets* offsets, const void* x,

@@ -116,7 +116,7 @@ __device__ __forceinline__ float2 tile_part(const TileOperands<N>& o, int n, con
 bool tile_gemv_eligible(const void* W, const void* x, uint32_t n);
 tf_status launch_tile_gemv(tf_context* ctx, void* stream, const uint8_t* W, const uint16_t* S, const uint16_t* B, const uint16_t* x,
                            void* y, bool out_f32, uint32_t m, uint32_t n, bool sb_fp16, const char* name);
-bool tile_gate_up_eligible(uint32_t d, const void* x);
+bool tile_gate_up_eligible(tf_context* ctx, uint32_t d, uint32_t f, uint32_t top_k, const void* x);
 bool tile_down_eligible(uint32_t f, const void* acts);
 tf_status launch_tile_gate_up(tf_context* ctx, void* stream, const void* const* blobs, const tf_expert_offsets* offsets, const void* x,
                               void* acts, uint32_t d, uint32_t f, uint32_t top_k, const uint32_t* slot_map, uint32_t slots, const char* name);
