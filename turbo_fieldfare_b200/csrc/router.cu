@@ -635,7 +635,8 @@ static tf_status launch_router(tf_context* ctx, void* stream, const uint8_t* W, 
         const bool fixed = d / kGroup == (uint32_t)kProductionGroups;
         // Warps per token: as many as leave the rows in one round of two blocks per SM. A warp that takes all of a token's
         // candidates one after the other needs about 30 us however few rows there are.
-        const int which = rows <= 2 * sms ? 3 : rows <= 4 * sms ? 2 : rows <= 8 * sms ? 1 : 0;
+        // (Only the form with a token per block can group.)
+        const int which = rows <= 2 * sms || (own && routes) ? 3 : rows <= 4 * sms ? 2 : rows <= 8 * sms ? 1 : 0;
         void (*kr)(const uint8_t*, const uint16_t*, const uint16_t*, const uint16_t*, uint32_t, const uint16_t*, const uint16_t*, const float*,
                    const float2*, uint32_t*, uint16_t*, unsigned int*, RouterGroupOut, uint32_t, uint32_t, uint32_t, uint32_t);
 #define TF_RECHECK(WPT) kr = fixed ? (bf ? router_recheck_kernel<true, kProductionGroups, WPT> : router_recheck_kernel<false, kProductionGroups, WPT>) \

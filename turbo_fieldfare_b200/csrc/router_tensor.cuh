@@ -456,7 +456,7 @@ router_recheck_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict_
     float* xf = reinterpret_cast<float*>(smem) + (size_t)slot * d;
     float* scores = reinterpret_cast<float*>(smem) + (size_t)kTokens * d + (size_t)slot * num_experts;
     const uint32_t groups = d / kGroup;
-    // tokens past the end repeat the last one (the same values are written twice); only the first round counts
+    // tokens past the end repeat the last one (the same values are written twice)
     const uint32_t row = min(blockIdx.x * kTokens + slot, rows - 1);
     pdl_launch_dependents();
     pdl_wait();
@@ -593,18 +593,20 @@ router_recheck_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict_
     if (WPT == 1) __syncwarp(); else __syncthreads();
     if (part == 0)
         warp_select_topk(scores, num_experts, top_k, per_expert_scale, out_idx + (size_t)row * top_k, out_w + (size_t)row * top_k, lane);
-    if (grp.sorted_pairs == nullptr) return;
-    __shared__ bool is_last;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        is_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
-        if (is_last) *ticket = 0;                              // ready for the next launch
+    if constexpr (WPT == kRecheckWarps) {                      // the form of the few rows that are grouped here
+        if (grp.sorted_pairs == nullptr) return;
+        __shared__ bool is_last;
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            is_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+            if (is_last) *ticket = 0;                          // ready for the next launch
+        }
+        __syncthreads();
+        if (!is_last) return;
+        __threadfence();
+        group_routes_in_block<true>(out_idx, out_w, rows, top_k, num_experts, grp, smem);
     }
-    __syncthreads();
-    if (!is_last) return;
-    __threadfence();
-    group_routes_in_block<true>(out_idx, out_w, rows, top_k, num_experts, grp, smem);
 }
 
 }  // namespace tf
