@@ -392,9 +392,10 @@ router_block_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ 
         }
     }
     __syncthreads();
+    // the form for any number of experts: with the choice between two of them this kernel is 0.4 us slower (200 rows of 256: 21.4, 20.9)
     if (warp == 0)
-        warp_select_topk(scores, num_experts, top_k, per_expert_scale, out_idx + (size_t)row * top_k,
-                         out_w + (size_t)row * top_k, lane);
+        warp_select_topk_held<TF_MAX_ROUTER_EXPERTS / kWarp>(scores, num_experts, top_k, per_expert_scale, out_idx + (size_t)row * top_k,
+                                                             out_w + (size_t)row * top_k, lane);
 }
 
 // Prefill-sized batches: one block per R token rows (R = 6, 7 or 8, picked by the host so that the row tiles fill whole
