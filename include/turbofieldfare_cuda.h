@@ -150,8 +150,9 @@ tf_status tf_context_set_shared_tensorcore_min_tokens(tf_context* ctx, uint32_t 
  * Metal/MoE/moe.metal:135-185) of the experts that can still reach the top k, typically top_k + 1 or 2 of them.
  * Indices and weights are those of the one-launch kernels bit for bit. UINT32_MAX keeps the one-launch kernel. Calls
  * that ask for the logits (out_logits) and calls of up to 64 rows always take one launch.
- * Until it is set, the threshold is 256 for the router calls of this header, and 65 for the router inside a block forward
- * (tf_moe_block_forward, tf_stack_forward), whose workspace holds the scratch. A value that is set holds for both. */
+ * Until it is set, the threshold is 256 for the router calls of this header; the router inside a block forward
+ * (tf_moe_block_forward, tf_stack_forward), whose workspace holds the scratch, takes two launches from 65 rows on when its
+ * matrix has more than 65536 codes. A value that is set holds for both. */
 tf_status tf_context_set_router_tensorcore_min_rows(tf_context* ctx, uint32_t rows);
 /* Expert parallelism with fixed-capacity exchanges (decode steps): when ranks * tokens * top_k / (experts of a rank), the
  * expected rows per local expert, reaches `rows`, the owner's expert phase runs on the tensor cores instead of the

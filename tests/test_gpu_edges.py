@@ -296,6 +296,34 @@ def test_rmsnorm_row_lengths(tf_ctx, oracle, d, bf16, weighted):
     assert np.all(np.abs(to_float(out[:, :d]) - ref) <= bound)
 
 
+@pytest.mark.parametrize("E,D,rows,two_launches", [(16, 256, None, False), (128, 512, None, False), (64, 1280, None, True), (16, 256, 65, True)])
+def test_router_size_decides_until_a_threshold_is_set(tmp_path, E, D, rows, two_launches):
+    """Block forwards of 70 tokens with up to 65536 router codes keep the one-launch router, and both routes give the same bits."""
+    import torch
+    from turbo_fieldfare_b200.kernels import TurboContext
+    from turbo_fieldfare_b200.stack import ExpertPool, MoEBlock, MoEBlockLayer, Workspace
+    ctx = TurboContext(0)
+    pool = ExpertPool(ctx, 1, E, D, 64)
+    try:
+        pool.fill_synthetic(3)
+        layer = MoEBlockLayer(ctx, pool, 0, D, 64, 64, E, 8)
+        layer.fill_synthetic(4)
+        if rows is not None:
+            ctx.set_router_tensorcore_min_rows(rows)
+        x = torch.randn(70, D, device="cuda").half()
+        y, z, ws, block = torch.zeros_like(x), torch.zeros_like(x), Workspace(ctx, 70, D, 64, 64, 8, E), MoEBlock(ctx, layer)
+        text = _kernels_of(lambda: block.forward(x, y, 70, ws), tmp_path / "graph.dot")
+        assert ("router_recheck_kernel" in text) is two_launches
+        ctx.set_router_tensorcore_min_rows(1000 if two_launches else 65)         # the other route
+        block.forward(x, z, 70, ws)
+        torch.cuda.synchronize()
+        assert ctx.device_status() == 0 and torch.equal(y, z)
+        ws.close()
+    finally:
+        pool.close()
+        ctx.close()
+
+
 # 296 and 376 blocks of 16 rows over all slots, on either side of the rule for rows of more than 3072 columns, and a split call
 @pytest.mark.parametrize("D,F", [(3072, 752), (3136, 592), (3136, 752)])
 def test_phase1_long_rows(tf_ctx, oracle, D, F):

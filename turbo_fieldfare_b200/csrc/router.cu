@@ -686,6 +686,9 @@ static tf_status launch_router(tf_context* ctx, void* stream, const uint8_t* W, 
 // which groups them (the block that finishes the last row does it). One block per row computes every canonical logit there
 // otherwise: 168 us and a grouping launch against 11 + 36 for 200 rows (cold; about half of the 36 is the grouping by one
 // block). Larger blocks group with launches of their own, which many SMs share; nothing between the two was measured.
+// The one launch grows with experts * D and the two hardly do. Blocks of 65, 130 and 255 tokens gain from two by, in us: 16 x 256 -13,
+// -16, -17; 32 x 1024 -1, -3, -6; 64 x 768 6, 5, 0; 128 x 512 0, -3, -5; 64 x 1024 13, 11, 8; 32 x 2816 20, 20, 18; 128 x 1024 43, 43, 41.
+constexpr uint32_t kRouterTwoLaunchCodes = 65536;
 tf_status router_block_grouped(tf_context* ctx, void* stream, const void* weights, uint64_t weights_off,
                                const void* scales, uint64_t scales_off, const void* biases, uint64_t biases_off,
                                const void* hidden, uint64_t hidden_off, tf_dtype hidden_dtype,
@@ -707,7 +710,7 @@ tf_status router_block_grouped(tf_context* ctx, void* stream, const void* weight
     TF_REQUIRE(ctx, hidden_dtype == TF_FP16 || hidden_dtype == TF_BF16, TF_ERR_INVALID_ARGUMENT, "%s: bad hidden dtype", name);
     const RouterScratch own{static_cast<float2*>(approx_scratch), ticket};
     const bool use_own = approx_scratch && ticket && query_count > (uint32_t)kRouterSplitRows && query_count <= kRouterFusedGroupRows &&
-                         query_count >= ctx->router_block_min_rows;
+                         (ctx->router_block_min_rows ? query_count >= ctx->router_block_min_rows : num_experts * d > kRouterTwoLaunchCodes);
     bool grouped = false;
     tf_status s = launch_router(ctx, stream, byte_ptr(weights, weights_off), byte_ptr(scales, scales_off),
                                 byte_ptr(biases, biases_off), byte_ptr(hidden, hidden_off), hidden_dtype,

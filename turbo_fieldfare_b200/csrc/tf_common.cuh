@@ -45,8 +45,9 @@ struct tf_context {
     size_t router_approx_bytes = 0;
     // Batches of at least this many rows take the two-launch router (tensor-core logits + canonical re-check).
     uint32_t router_tensorcore_min_rows = 256;
-    // The same for block forwards of up to kRouterFusedGroupRows rows, whose workspace holds the scratch of the two launches.
-    uint32_t router_block_min_rows = tf::kRouterSplitRows + 1;
+    // The same for block forwards of up to kRouterFusedGroupRows rows, whose workspace holds the scratch of the two launches; 0
+    // until a caller sets it: the router's size decides (router_block_grouped).
+    uint32_t router_block_min_rows = 0;
     // One device word that kernels with bounded waits set when a wait gives up (0 = healthy).
     uint32_t* device_error = nullptr;
     // The same for the flag barriers of the peer exchange (peer.cu), kept apart so that a code from another kernel

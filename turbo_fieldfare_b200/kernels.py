@@ -89,8 +89,8 @@ class TurboContext:
 
     def set_router_tensorcore_min_rows(self, rows: int) -> None:
         """Router calls and block forwards over at least ``rows`` rows compute all logits on the tensor cores and re-check the
-        candidates in the canonical order (until set: 256 for router calls, 65 for block forwards; 0xFFFFFFFF keeps the
-        one-launch kernel)."""
+        candidates in the canonical order (until set: 256 for router calls, 65 for block forwards with more than 65536
+        router codes; 0xFFFFFFFF keeps the one-launch kernel)."""
         self.check(self.lib.tf_context_set_router_tensorcore_min_rows(self.handle, rows))
 
     def set_single_launch_step(self, enabled: bool) -> None:
