@@ -252,3 +252,17 @@ def test_shared_expert_tensorcore_vs_oracle(tf_ctx, oracle, T, D, Fs):
         _, truth = o.shared_expert_int4(gate, up, down, x16[t], order=0)
         assert o.rel_l2(got[t], truth) < FP16_CHAINED
         assert o.rel_error(got[t], truth) < FP16_CHAINED
+
+
+# Edges of the two forms of the GEMM. One CTA per tile: one stage per tile over more tiles than CTAs (the MMA issuers take whole
+# tiles in turn), three groups in the last stage, rows beyond the last whole tile, one buffer of scale planes. Pairs: an odd number
+# of weight-row tiles (the second CTA's last tile is past the matrix), a last stage of one group, a ragged last token tile.
+@pytest.mark.parametrize("M,N,K", [(16, 20000, 64), (48, 40008, 192), (65, 200, 704), (700, 520, 7104), (9000, 264, 1088), (1000, 2120, 704)])
+def test_int4_qmm_edges_of_both_forms(tf_ctx, oracle, M, N, K):
+    test_int4_qmm_vs_oracle(tf_ctx, oracle, M, N, K)
+
+
+# The same for routed rows: groups on both sides of 64 rows at fewer and at more than 40 rows per expert.
+@pytest.mark.parametrize("T,D,F,E,K,zipf", [(70, 256, 192, 16, 8, True), (2, 64, 64, 256, 8, False), (400, 192, 320, 8, 4, True)])
+def test_grouped_tensorcore_edges_of_both_forms(tf_ctx, oracle, T, D, F, E, K, zipf):
+    test_grouped_tensorcore_vs_oracle_and_cuda_cores(tf_ctx, oracle, T, D, F, E, K, zipf)

@@ -6,11 +6,11 @@
 // prefill_grouped_routed_moe_batched_phase1 / _down (Metal/Prefill/prefill.metal:598-670), which the
 // reference runs as scalar per-thread dot products.
 //
-//   D[128 weight rows x N tokens] += W_tile[128 x 256] . X_tile[N x 256]^T     per stage of four 64-column groups, N <= 128
+//   D[128 or 256 weight rows x N tokens] += W_tile[rows x 256] . X_tile[N x 256]^T     per stage of four 64-column groups
 //
-// Weights are the A operand (M = 128) and are fed to the MMA from TENSOR MEMORY; tokens are the B operand
-// (N = the tile's token count rounded up to 16, carried in the instruction descriptor) in shared memory,
-// K-major with the 128-byte swizzle. Data path of the weights, which carry nearly all the bytes:
+// Weights are the A operand and are fed to the MMA from TENSOR MEMORY; tokens are the B operand (N = the tile's token count
+// rounded up, carried in the instruction descriptor) in shared memory, K-major with the 128-byte swizzle. Data path of the
+// weights, which carry nearly all the bytes:
 //   HBM --TMA tile load--> shared memory (packed, 128 bytes per row and stage)
 //       --LDS.128--> registers --one HFMA2 per two codes--> w = half(q * s + b)     (tensorops.metal:60-75)
 //       --tcgen05.st--> tensor memory --tcgen05.mma--> fp32 accumulators in tensor memory.
@@ -19,19 +19,24 @@
 // bandwidth than the whole HBM stream.
 // A gate/up tile holds 64 gate rows over 64 up rows, so that one accumulator of 128 lanes carries both, 704 rows are eleven
 // whole tiles, and both forms of the kernel have one layout; the epilogue warps of the two halves exchange values.
-// Roles of the 24 warps: warps 0, 2 and 3 issue the copies of packed codes, of activations (boxes of 16 to 128 rows) and of
-// a tile's scale and bias planes (1-D bulk copies), warp 1 the MMAs, and commits stages back through mbarriers; warps 4-19
-// dequantise (a thread takes one group of one row per stage); warps 20-23 read the accumulators with tcgen05.ld, apply
-// GeGLU or nothing, and store through a staging tile as 16-byte words, masked to the group's real tokens.
-// Accumulators alternate between two buffers of 128 columns, so that the epilogue overlaps the next tile's MMAs.
+// Roles of the 24 warps: warp 0 issues the copies of a tile's scale and bias planes (1-D bulk copies) and of packed codes,
+// warp 2 those of activations (one 3-D box of 16 to 64 rows x 256 columns per stage), warps 1 and 3 the MMAs, and commit stages
+// back through mbarriers; warps 4-19 dequantise in two teams that take turns (a thread takes two groups of one row per stage);
+// warps 20-23 read the accumulators with tcgen05.ld, apply GeGLU or nothing, and store through a staging tile as 16-byte words,
+// masked to the group's real tokens. Accumulators are double-buffered, so that the epilogue overlaps the next tile's MMAs.
 // A persistent grid walks (group, token tile, weight-row tile) work items derived on the device from the
 // routing metadata. Every mbarrier wait is bounded; on expiry the kernel records a code, waits for its copies and leaves.
 //
-// What bounds it: with 128 tokens per tile the activations, 64 bytes per clock and SM out of L2 (clock counters around the
-// waits, 4096 x 18944 x 2816, 1.14 PFLOP/s). With few tokens no unit: at 21 tokens per expert a stage takes 1480 clocks in the
-// gate/up launch and 1720 in the down launch, of which the dequantisers' integer instructions account for about 700, the MMAs
-// for 250, and an SM's share of the HBM rate for 740; the rest is the hand-over between the roles. Each single-warp role pays
-// 100 to 150 clocks per wait or commit whatever N is, so a stage is as deep as tensor memory allows.
+// Two forms (clock counters around the waits of each role; 128 experts of 704 x 2816, uniform routing):
+// PAIR, many tokens: with one CTA per tile of 128 rows x 128 tokens a stage took 1700 clocks, 640 of them waits for activations
+// (64 KB per stage and SM out of L2). A pair of CTAs (cta_group::2) shares them: each holds those of half the tokens. 1240 clocks
+// at 104 tokens per tile (MMAs 830), most of the rest the instructions of the one warp that issues them. 4096 tokens: gate/up 281
+// -> 240 us, down 161 -> 141; dense 4096 x 2112 x 2816: 44 us = 1.11 PFLOP/s. (Arrivals on the other CTA's barriers must not
+// be releases at cluster scope: with those a stage took 2150 clocks.)
+// Otherwise, few tokens: the one warp that issued the MMAs bounded the kernel (waits, 16 MMAs and commits: 1250 of 1250 clocks
+// without any copy outstanding at 1170), so two warps take turns, each with an accumulator, and activations come by one copy per
+// stage instead of four. 333 tokens, 21 per expert: 1010 clocks a stage, of which an SM's share of the HBM rate is 790 and the
+// dequantisers' instructions about 550; gate/up 109 -> 74 us, down 70 -> 46.
 //
 // Column order. The cheapest nibble extraction yields the eight codes of a 32-bit word in the order
 // (0,4,1,5,2,6,3,7). A dot product does not care about the order as long as both operands agree, so the
@@ -44,17 +49,17 @@
 
 namespace tf {
 
-constexpr int kQmmTokMax = 128;        // largest N of one MMA: tokens per tile
-constexpr int kQmmRows = 128;          // M of the MMA: weight rows per tile (gate/up: 64 gate rows over 64 up rows)
-constexpr int kQmmRawK = 256;          // columns per packed-code stage: one quantisation group per dequantiser thread
-constexpr int kQmmHalfK = 128;         // half of a stage; the unit of the activation ring for tiles of more than 64 tokens
-constexpr uint32_t kQmmRawBytes = kQmmRows * (kQmmRawK / 2);        // 16 KB
+constexpr int kQmmRows = 128;          // M of a CTA's MMA: weight rows per tile (gate/up: 64 gate rows over 64 up rows)
+constexpr int kQmmBoxMax = 64;         // activation rows that a CTA holds per tile: tokens of a tile, or half of them (PAIR)
+constexpr int kQmmStageK = 256;        // columns per stage: four quantisation groups
+constexpr uint32_t kQmmRawBytes = kQmmRows * (kQmmStageK / 2);      // 16 KB of packed codes
+constexpr uint32_t kQmmRowBytes = kQmmStageK * 2;                   // one activation row of a stage
 constexpr int kQmmRawMax = 4, kQmmBMax = 12, kQmmScMax = 4;         // ring depths (the launch picks them to fit, see QmmPlan)
-constexpr int kQmmASlots = 2;          // TMEM ring of dequantised stages, 128 TMEM columns each
-constexpr int kQmmFirstDequantWarp = 4, kQmmDequantWarps = 16;      // four threads per weight row
+constexpr int kQmmTeams = 2;           // teams of dequantisers, each with its slot of a dequantised stage (128 TMEM columns)
+constexpr int kQmmFirstDequantWarp = 4, kQmmDequantWarps = 16, kQmmTeamWarps = kQmmDequantWarps / kQmmTeams;
 constexpr int kQmmFirstEpilogueWarp = 20, kQmmEpilogueWarps = 4;
 constexpr int kQmmThreads = (kQmmFirstEpilogueWarp + kQmmEpilogueWarps) * 32;
-constexpr int kQmmTmemCols = 512;      // columns 0..255: two accumulator buffers; 256..511: the ring of dequantised slots
+constexpr int kQmmTmemCols = 512;      // columns 0..255: accumulators; 256..511: the teams' slots of dequantised weights
 constexpr int kQmmAccCols = 256;
 constexpr uint32_t kQmmStageBytes = 16384;    // output staging of the epilogue
 constexpr uint32_t kQmmSpin = 1u << 22;
@@ -85,6 +90,7 @@ struct QmmArgs {
     const tf_group* route_groups;
     const uint32_t* route_counters;
     uint32_t dense_tokens, dense_per_tile;
+    uint32_t ctas;          // CTAs of a tile: 2 for pairs
     // problem
     uint32_t rows;          // weight rows (output features)
     uint32_t k;             // columns (input features)
@@ -116,9 +122,30 @@ __device__ __forceinline__ bool q_mbar_wait(uint32_t addr, uint32_t parity) {
     }
     return false;
 }
-__device__ __forceinline__ void tma_load_2d(uint32_t smem_dst, const CUtensorMap* map, int c0, int c1, uint32_t mbar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                 ::"r"(smem_dst), "l"(map), "r"(c0), "r"(c1), "r"(mbar) : "memory");
+// One look at a barrier, without waiting.
+__device__ __forceinline__ bool q_mbar_test(uint32_t addr, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{ .reg .pred p; mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+                 : "=r"(ok) : "r"(addr), "r"(parity) : "memory");
+    return ok != 0;
+}
+// The same shared-memory address in the first CTA of the pair.
+__device__ __forceinline__ uint32_t q_in_leader(uint32_t addr) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
+    return r;
+}
+// Relaxed: what these arrivals publish is tensor memory, whose accesses the tcgen05 waits and fences order, not memory.
+__device__ __forceinline__ void q_mbar_arrive_cluster(uint32_t addr) {
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
+}
+__device__ __forceinline__ void q_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Into this CTA's shared memory, counted on a barrier of the pair's first CTA.
+__device__ __forceinline__ void tma_load_3d_pair(uint32_t smem_dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t mbar) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3, %4}], [%5];"
+                 ::"r"(smem_dst), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(mbar) : "memory");
 }
 __device__ __forceinline__ void tma_load_3d(uint32_t smem_dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t mbar) {
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
@@ -138,14 +165,26 @@ __device__ __forceinline__ bool elect_one() {
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void q_fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+// Arrives at mbar (PAIR: at this address in both CTAs) once the MMAs issued so far have completed.
+template <bool PAIR>
 __device__ __forceinline__ void tc_commit(uint32_t mbar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
+    if constexpr (PAIR)
+        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                     ::"r"(mbar), "h"((uint16_t)3) : "memory");
+    else
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
 }
-// D[tmem] (+)= A[tmem] * B[smem descriptor]
+// D[tmem] (+)= A[tmem] * B[smem descriptor]; PAIR: 128 rows of A and D in each CTA, half of B's rows in each.
+template <bool PAIR>
 __device__ __forceinline__ void tc_mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-                 ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+    if constexpr (PAIR)
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                     "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+                     ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+    else
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                     "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+                     ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
 __device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
@@ -181,9 +220,9 @@ __device__ __forceinline__ uint32_t q_lds16(uint32_t addr) {
 __device__ __forceinline__ uint64_t umma_smem_desc(uint32_t smem_addr) {
     return (uint64_t)((smem_addr & 0x3FFFFu) >> 4) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }
-// kind::f16, fp16 x fp16 -> fp32, both operands K-major, M = 128, N = n (a multiple of 16, at most 256).
-__device__ __forceinline__ uint32_t qmm_idesc(uint32_t n) {
-    return (1u << 4) | ((n >> 3) << 17) | ((uint32_t)(kQmmRows >> 4) << 24);
+// kind::f16, fp16 x fp16 -> fp32, both operands K-major, M = m, N = n (a multiple of 16, of 32 for M = 256).
+__device__ __forceinline__ uint32_t qmm_idesc(uint32_t m, uint32_t n) {
+    return (1u << 4) | ((n >> 3) << 17) | ((m >> 4) << 24);
 }
 
 // Eight packed codes (one 32-bit word) -> eight fp16 weights w = half(q * s + b).
@@ -244,30 +283,32 @@ __device__ __forceinline__ uint4 dequant8_wide(uint32_t w, __half2 s, __half2 b)
 // Position of column k within its eight-column block in the PERMUTED order.
 __device__ __forceinline__ uint32_t permuted_col(uint32_t k) { return (k & ~7u) | ((k & 3u) << 1) | ((k >> 2) & 1u); }
 
-// Tokens per tile of a group: as few tiles as kQmmTokMax allows, of equal size (a multiple of 16, the step of the MMA's N).
-// 256 + 14 tokens are three tiles of 96, not 128 + 128 + 14: the weights are dequantised once per tile, and below about
-// 80 tokens that takes longer than the tile's MMAs.
-__host__ __device__ inline uint32_t qmm_tokens_per_tile(uint32_t count) {
-    const uint32_t tiles = (count + kQmmTokMax - 1) / kQmmTokMax;
-    return ((count + tiles - 1) / tiles + 15u) & ~15u;
+// Tokens per tile of a group: as few tiles as 64 * ctas tokens each allow, of equal size (a multiple of 16 per CTA, the step
+// of the MMA's N). 256 + 14 tokens are three tiles of 96, not 128 + 128 + 14: the weights are dequantised once per tile, and
+// below about 80 tokens that takes longer than the tile's MMAs.
+__host__ __device__ inline uint32_t qmm_tokens_per_tile(uint32_t count, uint32_t ctas) {
+    const uint32_t most = ctas * kQmmBoxMax, step = ctas * 16u;
+    const uint32_t tiles = (count + most - 1) / most;
+    return ((count + tiles - 1) / tiles + step - 1) / step * step;
 }
 
 // The group table of a launch: one thread per group, the tile counts scanned over the block. (One thread that walked the
 // groups took 29 us for 128 of them, on the critical path before every routed GEMM; this takes about 2.)
 __global__ void __launch_bounds__(TF_MAX_ROUTER_EXPERTS)
 qmm_prepare_kernel(uint4* __restrict__ groups, uint32_t* __restrict__ totals, const tf_group* __restrict__ route_groups,
-                   const uint32_t* __restrict__ route_counters, uint32_t dense_tokens, uint32_t dense_per_tile) {
+                   const uint32_t* __restrict__ route_counters, uint32_t dense_tokens, uint32_t dense_per_tile, uint32_t ctas) {
     __shared__ uint32_t warp_tiles[TF_MAX_ROUTER_EXPERTS / kWarp], warp_top[TF_MAX_ROUTER_EXPERTS / kWarp];
     const uint32_t warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
     pdl_launch_dependents();
     pdl_wait();
     const uint32_t ngroups = route_groups ? min(route_counters[0], (uint32_t)TF_MAX_ROUTER_EXPERTS) : 1u;
-    uint32_t row = 0, count = 0, expert = 0, per = 16;
+    const uint32_t step = ctas * 16u;
+    uint32_t row = 0, count = 0, expert = 0, per = step;
     if (threadIdx.x < ngroups) {
         if (route_groups) {
             const tf_group rg = route_groups[threadIdx.x];
             row = rg.pair_start; count = rg.pair_count; expert = rg.expert;
-            per = qmm_tokens_per_tile(count > 0 ? count : 1u);
+            per = qmm_tokens_per_tile(count > 0 ? count : 1u, ctas);
         } else {
             count = dense_tokens; per = dense_per_tile;
         }
@@ -279,10 +320,10 @@ qmm_prepare_kernel(uint4* __restrict__ groups, uint32_t* __restrict__ totals, co
         const uint32_t v = __shfl_up_sync(kFullMask, incl, o);
         if (lane >= (uint32_t)o) incl += v;
     }
-    const uint32_t top = __reduce_max_sync(kFullMask, min((count + 15u) & ~15u, per));
+    const uint32_t top = __reduce_max_sync(kFullMask, min((count + step - 1) / step * step, per));
     if (lane == kWarp - 1) { warp_tiles[warp] = incl; warp_top[warp] = top; }
     __syncthreads();
-    uint32_t before = 0, all = 0, n_top = 16;
+    uint32_t before = 0, all = 0, n_top = step;
 #pragma unroll
     for (uint32_t w = 0; w < TF_MAX_ROUTER_EXPERTS / kWarp; ++w) {
         before += w < warp ? warp_tiles[w] : 0u;
@@ -293,268 +334,317 @@ qmm_prepare_kernel(uint4* __restrict__ groups, uint32_t* __restrict__ totals, co
     if (threadIdx.x == 0) { totals[0] = ngroups; totals[1] = all; totals[2] = n_top; }
 }
 
-// A role's place in the CTA's sequence of tiles. Tiles only move forward, so the group is found by stepping through the
-// table in shared memory, not by searching it.
+// A role's place in its CTA's (or pair's) sequence of tiles, which is tile first, first + step, ... Tiles only move forward: the
+// group is found by stepping through the table in shared memory, 32 entries to a look, without a division.
 struct QmmTile {
+    uint32_t tglob, wt;         // token tile over all groups; weight-row tile (of a pair: the two CTAs' tiles 2 wt, 2 wt + 1)
+    uint32_t dt, dw;            // their step
+    uint32_t wrow_tiles;
     uint32_t gi = 0;            // group
-    uint32_t wt = 0;            // weight-row tile
     uint32_t row0 = 0;          // first activation / output row
     uint32_t ntok = 0;          // real tokens
     uint32_t expert = 0;
-    __device__ __forceinline__ void locate(const uint4* table, uint32_t ngroups, uint32_t wrow_tiles, uint32_t tile) {
-        const uint32_t tglob = tile / wrow_tiles;
-        wt = tile - tglob * wrow_tiles;
-        while (gi + 1 < ngroups && table[gi + 1].x <= tglob) ++gi;
+    __device__ __forceinline__ QmmTile(uint32_t first, uint32_t step, uint32_t tiles)
+        : tglob(first / tiles), wt(first % tiles), dt(step / tiles), dw(step % tiles), wrow_tiles(tiles) {}
+    __device__ __forceinline__ void locate(const uint4* table, uint32_t ngroups, uint32_t lane) {
+        for (uint32_t ahead = kWarp; ahead == kWarp;) {              // group starts grow: the votes are a prefix of the lanes
+            const uint32_t g = gi + 1 + lane;
+            ahead = __popc(__ballot_sync(kFullMask, g < ngroups && table[g].x <= tglob));
+            gi += ahead;
+        }
         const uint4 g = table[gi];                                  // tile start, first row, tokens, expert | tokens per tile << 16
         const uint32_t per = g.w >> 16, done = (tglob - g.x) * per;
         expert = g.w & 0xFFFFu;
         row0 = g.y + done;
         ntok = g.z - done < per ? g.z - done : per;
     }
-    __device__ __forceinline__ uint32_t n() const { return (ntok + 15u) & ~15u; }
+    __device__ __forceinline__ void next() {
+        tglob += dt; wt += dw;
+        if (wt >= wrow_tiles) { wt -= wrow_tiles; ++tglob; }
+    }
 };
 
-template <int NMAT, bool NATURAL_K>
+// PAIR: two CTAs of a cluster (two SMs that share their tensor cores' operands, cta_group::2) take one tile of 2 x 128 weight
+// rows x up to 128 tokens. Each dequantises its own 128 rows and holds half of the tokens' activations, the first one issues the
+// MMAs. Otherwise a CTA takes 128 rows x up to 64 tokens, and two warps issue MMAs, one for each team of dequantisers.
+template <int NMAT, bool NATURAL_K, bool PAIR>
 __global__ void __launch_bounds__(kQmmThreads, 1)
 qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map16, const __grid_constant__ CUtensorMap x_map32,
-                   const __grid_constant__ CUtensorMap x_map64, const __grid_constant__ CUtensorMap x_map128,
+                   const __grid_constant__ CUtensorMap x_map48, const __grid_constant__ CUtensorMap x_map64,
                    const __grid_constant__ CUtensorMap w_map0, const __grid_constant__ CUtensorMap w_map1, const QmmArgs args) {
     extern __shared__ uint8_t smem_raw[];
     constexpr uint32_t kMatRows = kQmmRows / NMAT;                     // rows of one matrix in a tile
+    constexpr uint32_t kCtas = PAIR ? 2 : 1;                           // CTAs of a tile
+    constexpr uint32_t kStep = 16 * kCtas;                             // N of an MMA is a multiple of it
+    constexpr uint32_t kAccTok = PAIR ? 128 : 64;                      // columns of an accumulator
     const QmmPlan& plan = args.plan;
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;                      // swizzle atoms need 1024-byte alignment
     uint8_t* base_ptr = smem_raw + (base - raw);
     const uint32_t bars = base + plan.off_bars;
-    // barrier map (8 bytes each)
+    // barrier map (8 bytes each); L: in a pair only the first CTA's are used
     auto bar_full_raw = [&](uint32_t s) { return bars + s * 8; };                            // 4: TMA tx
-    auto bar_empty_raw = [&](uint32_t s) { return bars + (4 + s) * 8; };                     // 4: dequant warps
-    auto bar_full_b = [&](uint32_t s) { return bars + (8 + s) * 8; };                        // 12: TMA tx
+    auto bar_empty_raw = [&](uint32_t s) { return bars + (4 + s) * 8; };                     // 4: the team's warps
+    auto bar_full_b = [&](uint32_t s) { return bars + (8 + s) * 8; };                        // 12 L: TMA tx
     auto bar_empty_b = [&](uint32_t s) { return bars + (20 + s) * 8; };                      // 12: tcgen05.commit
-    auto bar_full_a = [&](uint32_t s) { return bars + (32 + s) * 8; };                       // 2: dequant warps
-    auto bar_empty_a = [&](uint32_t s) { return bars + (36 + s) * 8; };                      // 2: tcgen05.commit
+    auto bar_full_a = [&](uint32_t t) { return bars + (32 + t) * 8; };                       // 2 L: the team's warps, of both CTAs
+    auto bar_empty_a = [&](uint32_t t) { return bars + (34 + t) * 8; };                      // 2: tcgen05.commit
     auto bar_full_sc = [&](uint32_t b) { return bars + (40 + b) * 8; };                      // 4: bulk-copy tx
     auto bar_empty_sc = [&](uint32_t b) { return bars + (44 + b) * 8; };                     // 4: dequant warps
-    auto bar_acc_full = [&](uint32_t b) { return bars + (48 + b) * 8; };                     // 2: tcgen05.commit
-    auto bar_acc_empty = [&](uint32_t b) { return bars + (50 + b) * 8; };                    // 2: epilogue warps
-    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(base_ptr + plan.off_bars + 52 * 8);   // TMEM base
+    auto bar_acc_full = [&](uint32_t i, uint32_t b) { return bars + (48 + 2 * i + b) * 8; }; // 4: tcgen05.commit
+    auto bar_acc_empty = [&](uint32_t b) { return bars + (52 + b) * 8; };                    // 2 L: epilogue warps, of both CTAs
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(base_ptr + plan.off_bars + 54 * 8);   // TMEM base
     uint4* table = reinterpret_cast<uint4*>(base_ptr + plan.off_table);
 
     // The shuffle makes the warp index uniform for the compiler: the roles' branches and their operands then stay in uniform
     // registers, where the MMA and copy instructions want them (the MMA issuer's loop was 10 to 15 % slower without).
     const int warp = __shfl_sync(kFullMask, (int)(threadIdx.x / kWarp), 0), lane = threadIdx.x % kWarp;
+    const uint32_t rank = PAIR ? blockIdx.x & 1 : 0;                   // CTA within the pair
     const uint32_t ng = args.k / kGroup;
-    const uint32_t ksteps = (ng + 3) / 4;                              // packed-code stages per tile
-    const uint32_t wrow_tiles = (args.rows + kMatRows - 1) / kMatRows;
+    const uint32_t ksteps = (ng + 3) / 4;                              // stages per tile
+    const uint32_t wrow_tiles = (args.rows + kCtas * kMatRows - 1) / (kCtas * kMatRows);
 
     pdl_launch_dependents();
     if (threadIdx.x == 0) {
-        for (uint32_t s = 0; s < (uint32_t)kQmmRawMax; ++s) { q_mbar_init(bar_full_raw(s), 1); q_mbar_init(bar_empty_raw(s), kQmmDequantWarps); }
+        for (uint32_t s = 0; s < (uint32_t)kQmmRawMax; ++s) { q_mbar_init(bar_full_raw(s), 1); q_mbar_init(bar_empty_raw(s), kQmmTeamWarps); }
         for (uint32_t s = 0; s < (uint32_t)kQmmBMax; ++s) { q_mbar_init(bar_full_b(s), 1); q_mbar_init(bar_empty_b(s), 1); }
-        for (uint32_t s = 0; s < (uint32_t)kQmmASlots; ++s) { q_mbar_init(bar_full_a(s), kQmmDequantWarps); q_mbar_init(bar_empty_a(s), 1); }
+        for (uint32_t t = 0; t < (uint32_t)kQmmTeams; ++t) { q_mbar_init(bar_full_a(t), kCtas * kQmmTeamWarps); q_mbar_init(bar_empty_a(t), 1); }
         for (uint32_t b = 0; b < (uint32_t)kQmmScMax; ++b) { q_mbar_init(bar_full_sc(b), 1); q_mbar_init(bar_empty_sc(b), kQmmDequantWarps); }
-        for (uint32_t b = 0; b < 2; ++b) { q_mbar_init(bar_acc_full(b), 1); q_mbar_init(bar_acc_empty(b), kQmmEpilogueWarps); }
+        for (uint32_t b = 0; b < 2; ++b) {
+            for (uint32_t i = 0; i < 2; ++i) q_mbar_init(bar_acc_full(i, b), 1);
+            q_mbar_init(bar_acc_empty(b), kCtas * kQmmEpilogueWarps);
+        }
+        if constexpr (PAIR) asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         q_fence_async_smem();
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                     ::"r"(smem_u32(const_cast<uint32_t*>(tmem_slot))), "r"((uint32_t)kQmmTmemCols) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        const uint32_t slot = smem_u32(const_cast<uint32_t*>(tmem_slot));
+        if constexpr (PAIR) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"((uint32_t)kQmmTmemCols) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"((uint32_t)kQmmTmemCols) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
     }
     pdl_wait();                                                        // routes and activations come from the kernels before this one
     const uint32_t ngroups = args.totals[0], total_tiles = args.totals[1] * wrow_tiles, n_top = args.totals[2];
     if (threadIdx.x < ngroups) table[threadIdx.x] = args.groups[threadIdx.x];
     tc_fence_before();
     __syncthreads();
+    if constexpr (PAIR) q_cluster_sync();                              // the other CTA's barriers are initialised, too
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    // Activation ring: slots of the launch's largest tile, as many as fit. A slot holds a whole stage's columns when two or
-    // more of those fit beside each other with at most 64 tokens (fewer waits and commits per MMA), otherwise half of them.
-    const uint32_t b_block = n_top * 128;                             // 64 columns of a slot
-    const uint32_t b_halves = n_top <= 64 && plan.b_bytes >= 8 * b_block ? 2u : 1u;
-    const uint32_t b_slot = b_halves * 2 * b_block;
-    const uint32_t b_fit = plan.b_bytes / b_slot;
+    // Activation ring: slots of a whole stage of the launch's largest tile, as many as fit. With two MMA issuers an even number,
+    // as for the packed codes, so that a slot always belongs to the same one and a wait never sees the phase of another use.
+    // Where only two slots of 64 tokens would fit beside four stages of packed codes, those make do with two.
+    const uint32_t b_slot = n_top / kCtas * kQmmRowBytes;
+    const uint32_t raw_stages = !PAIR && plan.b_bytes < 4 * b_slot ? 2u : plan.raw_stages;
+    const uint32_t off_b = raw_stages * kQmmRawBytes, b_bytes = plan.off_b + plan.b_bytes - off_b;
+    const uint32_t b_fit = PAIR ? b_bytes / b_slot : b_bytes / b_slot & ~1u;
     const uint32_t b_stages = b_fit < (uint32_t)kQmmBMax ? b_fit : (uint32_t)kQmmBMax;
     const uint32_t a_ring = tmem_base + kQmmAccCols;
+    const uint32_t first_tile = blockIdx.x / kCtas, tile_step = gridDim.x / kCtas;
 
     uint32_t fail = 0;
-    QmmTile tl;
+    QmmTile tl(first_tile, tile_step, wrow_tiles);
 
     if (warp == 0) {
-        // ===================== copy issuer: packed codes =====================
-        uint32_t sr = 0, ur = 0;
-        for (uint32_t tile = blockIdx.x; tile < total_tiles && !fail; tile += gridDim.x) {
-            tl.locate(table, ngroups, wrow_tiles, tile);
+        // ===================== copy issuer: scale and bias planes of a tile, packed codes =====================
+        uint32_t sr = 0, ur = 0, sc = 0, uc = 0;
+        for (uint32_t tile = first_tile; tile < total_tiles && !fail; tile += tile_step, tl.next()) {
+            tl.locate(table, ngroups, lane);
+            const uint32_t first = (tl.wt * kCtas + rank) * kMatRows;
+            // (the dequantisers of the tile that used this buffer last are as far as the ring of codes asks for below, or one tile
+            // ahead of it where the planes have one buffer)
+            if (uc > 0 && !q_mbar_wait(bar_empty_sc(sc), (uc - 1) & 1)) { fail = kErrQmmTimeout | 6; break; }
+            if (elect_one()) {
+                const uint32_t left = first < args.rows ? args.rows - first : 0;      // a pair's second tile may be past the matrix
+                const uint32_t bytes = (left < kMatRows ? left : kMatRows) * ng * 2;  // a multiple of 16: rows are a multiple of 8
+                const size_t off = (size_t)tl.expert * args.expert_stride + (size_t)first * ng * 2;
+                q_mbar_expect_tx(bar_full_sc(sc), NMAT * 2 * bytes);
+                if (bytes > 0) {
+#pragma unroll
+                    for (int m = 0; m < NMAT; ++m) {
+                        const uint32_t dst = base + plan.off_sc + sc * plan.sc_bytes + m * 2 * plan.plane_bytes;
+                        q_bulk_g2s(dst, reinterpret_cast<const uint8_t*>(args.S[m]) + off, bytes, bar_full_sc(sc));
+                        q_bulk_g2s(dst + plan.plane_bytes, reinterpret_cast<const uint8_t*>(args.B[m]) + off, bytes, bar_full_sc(sc));
+                    }
+                }
+            }
+            __syncwarp();
+            if (++sc == plan.sc_bufs) { sc = 0; ++uc; }
             for (uint32_t ks = 0; ks < ksteps; ++ks) {
                 if (ur > 0 && !q_mbar_wait(bar_empty_raw(sr), (ur - 1) & 1)) { fail = kErrQmmTimeout | 1; break; }
                 if (elect_one()) {
                     const uint32_t dst = base + sr * kQmmRawBytes;
                     q_mbar_expect_tx(bar_full_raw(sr), kQmmRawBytes);
-                    tma_load_3d(dst, &w_map0, (int)(ks * (kQmmRawK / 2)), (int)(tl.wt * kMatRows), (int)tl.expert, bar_full_raw(sr));
+                    tma_load_3d(dst, &w_map0, (int)(ks * (kQmmStageK / 2)), (int)first, (int)tl.expert, bar_full_raw(sr));
                     if (NMAT == 2)
-                        tma_load_3d(dst + kQmmRawBytes / 2, &w_map1, (int)(ks * (kQmmRawK / 2)), (int)(tl.wt * kMatRows), (int)tl.expert, bar_full_raw(sr));
+                        tma_load_3d(dst + kQmmRawBytes / 2, &w_map1, (int)(ks * (kQmmStageK / 2)), (int)first, (int)tl.expert, bar_full_raw(sr));
                 }
                 __syncwarp();
-                if (++sr == plan.raw_stages) { sr = 0; ++ur; }
+                if (++sr == raw_stages) { sr = 0; ++ur; }
             }
         }
-        if (fail)            // the copies already issued land before the CTA's shared memory goes away (bounded)
-            for (uint32_t s = 0; s < plan.raw_stages; ++s) q_mbar_wait(bar_full_raw(s), (s < sr ? ur : ur + 1) & 1);
+        if (fail) {          // the copies already issued land before the CTA's shared memory goes away (bounded)
+            for (uint32_t s = 0; s < raw_stages; ++s) q_mbar_wait(bar_full_raw(s), (s < sr ? ur : ur + 1) & 1);
+            for (uint32_t s = 0; s < plan.sc_bufs; ++s) q_mbar_wait(bar_full_sc(s), (s < sc ? uc : uc + 1) & 1);
+        }
     } else if (warp == 2) {
-        // ===================== copy issuer: activations =====================
+        // ===================== copy issuer: activations, one copy per stage =====================
         uint32_t sb = 0, ub = 0;
-        for (uint32_t tile = blockIdx.x; tile < total_tiles && !fail; tile += gridDim.x) {
-            tl.locate(table, ngroups, wrow_tiles, tile);
-            const uint32_t n = tl.n();
-            for (uint32_t g0 = 0; g0 < ng; g0 += 2 * b_halves) {
+        for (uint32_t tile = first_tile; tile < total_tiles && !fail; tile += tile_step, tl.next()) {
+            tl.locate(table, ngroups, lane);
+            const uint32_t box = (tl.ntok + kStep - 1) / kStep * 16;  // rows per CTA
+            const CUtensorMap* map = box == 64 ? &x_map64 : box == 48 ? &x_map48 : box == 32 ? &x_map32 : &x_map16;
+            const int row = (int)(tl.row0 + rank * box);
+            for (uint32_t ks = 0; ks < ksteps; ++ks) {
                 if (ub > 0 && !q_mbar_wait(bar_empty_b(sb), (ub - 1) & 1)) { fail = kErrQmmTimeout | 7; break; }
-                if (elect_one()) {
-                    const uint32_t left = ng - g0, blocks = left < 2 * b_halves ? left : 2 * b_halves;
-                    q_mbar_expect_tx(bar_full_b(sb), blocks * n * 128);
-                    for (uint32_t h = 0; h < blocks; ++h) {
-                        uint32_t dst = base + plan.off_b + sb * b_slot + h * b_block;
-                        const int col = (int)((g0 + h) * kGroup);
-                        int row = (int)tl.row0;
-                        if (n == 128) {
-                            tma_load_2d(dst, &x_map128, col, row, bar_full_b(sb));
-                        } else {                                  // 16 to 112 rows: boxes of 64, 32 and 16
-                            if (n & 64) { tma_load_2d(dst, &x_map64, col, row, bar_full_b(sb)); dst += 64 * 128; row += 64; }
-                            if (n & 32) { tma_load_2d(dst, &x_map32, col, row, bar_full_b(sb)); dst += 32 * 128; row += 32; }
-                            if (n & 16) tma_load_2d(dst, &x_map16, col, row, bar_full_b(sb));
-                        }
-                    }
+                if (elect_one()) {                                    // groups past K arrive as zeros and are not multiplied
+                    const uint32_t dst = base + off_b + sb * b_slot;
+                    if (rank == 0) q_mbar_expect_tx(bar_full_b(sb), kCtas * box * kQmmRowBytes);
+                    if constexpr (PAIR) tma_load_3d_pair(dst, map, 0, row, (int)(4 * ks), q_in_leader(bar_full_b(sb)));
+                    else tma_load_3d(dst, map, 0, row, (int)(4 * ks), bar_full_b(sb));
                 }
                 __syncwarp();
                 if (++sb == b_stages) { sb = 0; ++ub; }
             }
         }
-        if (fail)
+        if (fail && rank == 0)       // counts the copies of both CTAs, which leave together
             for (uint32_t s = 0; s < b_stages; ++s) q_mbar_wait(bar_full_b(s), (s < sb ? ub : ub + 1) & 1);
-    } else if (warp == 3) {
-        // ===================== copy issuer: scale and bias planes of a tile =====================
-        uint32_t sc = 0, uc = 0;
-        for (uint32_t tile = blockIdx.x; tile < total_tiles && !fail; tile += gridDim.x) {
-            tl.locate(table, ngroups, wrow_tiles, tile);
-            if (uc > 0 && !q_mbar_wait(bar_empty_sc(sc), (uc - 1) & 1)) { fail = kErrQmmTimeout | 6; break; }
-            if (elect_one()) {
-                const uint32_t first = tl.wt * kMatRows;
-                const uint32_t nrows = args.rows - first < kMatRows ? args.rows - first : kMatRows;
-                const uint32_t bytes = nrows * ng * 2;                // a multiple of 16: rows are a multiple of 8
-                const size_t off = (size_t)tl.expert * args.expert_stride + (size_t)first * ng * 2;
-                q_mbar_expect_tx(bar_full_sc(sc), NMAT * 2 * bytes);
-#pragma unroll
-                for (int m = 0; m < NMAT; ++m) {
-                    const uint32_t dst = base + plan.off_sc + sc * plan.sc_bytes + m * 2 * plan.plane_bytes;
-                    q_bulk_g2s(dst, reinterpret_cast<const uint8_t*>(args.S[m]) + off, bytes, bar_full_sc(sc));
-                    q_bulk_g2s(dst + plan.plane_bytes, reinterpret_cast<const uint8_t*>(args.B[m]) + off, bytes, bar_full_sc(sc));
-                }
-            }
-            __syncwarp();
-            if (++sc == plan.sc_bufs) { sc = 0; ++uc; }
-        }
-        if (fail)
-            for (uint32_t s = 0; s < plan.sc_bufs; ++s) q_mbar_wait(bar_full_sc(s), (s < sc ? uc : uc + 1) & 1);
-    } else if (warp == 1) {
-        // ===================== MMA issuer =====================
-        uint32_t sb = 0, ub = 0, sa = 0, ua = 0, buf = 0, uacc = 0;
-        const uint64_t b_desc0 = umma_smem_desc(base + plan.off_b);
-        for (uint32_t tile = blockIdx.x; tile < total_tiles && !fail; tile += gridDim.x) {
-            tl.locate(table, ngroups, wrow_tiles, tile);
-            const uint32_t idesc = qmm_idesc(tl.n());
+    } else if (warp == 1 || warp == 3) {
+        // ===================== MMA issuers =====================
+        // PAIR: warp 1 of the first CTA issues every stage. Otherwise the two warps take turns, each with an accumulator of its
+        // own (the epilogue adds them).
+        const uint32_t who = warp == 1 ? 0 : 1;
+        const bool mine = PAIR ? rank == 0 && who == 0 : true;
+        uint32_t sb = 0, ub = 0, count = 0, buf = 0, uacc = 0;        // count: stages so far; stage c is the (c / 2)-th use of its team's slot
+        const uint64_t b_desc0 = umma_smem_desc(base + off_b);
+        bool ready = false;                                           // the next stage's operands were there at the last look
+        for (uint32_t tile = first_tile; mine && tile < total_tiles && !fail; tile += tile_step, tl.next()) {
+            tl.locate(table, ngroups, lane);
+            const uint32_t n = (tl.ntok + kStep - 1) / kStep * kStep;
+            const uint32_t idesc = qmm_idesc(kCtas * kQmmRows, n);
+            const uint32_t b_block = (n / kCtas * 128) >> 4;         // 64 columns of a slot, in units of the descriptor
             if (uacc > 0 && !q_mbar_wait(bar_acc_empty(buf), (uacc - 1) & 1)) { fail = kErrQmmTimeout | 2; break; }
             tc_fence_after();
-            const uint32_t acc = tmem_base + buf * 128;
+            const uint32_t acc = tmem_base + (PAIR ? buf * kAccTok : (2 * buf + who) * kAccTok);
+            uint32_t accumulate = 0;
             for (uint32_t ks = 0; ks < ksteps; ++ks) {
-                if (!q_mbar_wait(bar_full_b(sb), ub & 1) || !q_mbar_wait(bar_full_a(sa), ua & 1)) { fail = kErrQmmTimeout | 3; break; }
-                tc_fence_after();
-                const uint32_t a_slot = a_ring + sa * 128;
-                const uint32_t groups = ng - 4 * ks;                  // groups left; those past K are skipped
-                const bool leader = elect_one();
-#pragma unroll
-                for (uint32_t h = 0; h < 2; ++h) {
-                    if (h == 1) {
-                        if (groups <= 2) break;
-                        if (b_halves == 1) {                          // the other half has a slot of its own
-                            if (leader) tc_commit(bar_empty_b(sb));
-                            __syncwarp();
-                            if (++sb == b_stages) { sb = 0; ++ub; }
-                            if (!q_mbar_wait(bar_full_b(sb), ub & 1)) { fail = kErrQmmTimeout | 3; break; }
-                        }
+                if (PAIR || (count & 1) == who) {
+                    const uint32_t t = count & 1;
+                    if (!ready && (!q_mbar_wait(bar_full_b(sb), ub & 1) || !q_mbar_wait(bar_full_a(t), (count >> 1) & 1))) {
+                        fail = kErrQmmTimeout | 3;
+                        break;
                     }
-                    if (leader) {                                     // 16 columns of K per MMA: 8 TMEM columns of A, 32 bytes of B
-                        const uint64_t b_desc = b_desc0 + (uint64_t)((sb * b_slot + (b_halves == 2 ? h * 2 * b_block : 0u)) >> 4);
-                        const uint32_t a = a_slot + h * 64;
-                        tc_mma_f16_ts(acc, a, b_desc, idesc, (ks > 0 || h > 0) ? 1u : 0u);
+                    tc_fence_after();
+                    const uint32_t a = a_ring + t * 128;
+                    const uint32_t groups = ng - 4 * ks;              // groups left; those past K are skipped
+                    const uint64_t b_desc = b_desc0 + (uint64_t)((sb * b_slot) >> 4);
+                    auto multiply = [&](uint32_t g) {                 // one group: 16 columns of K per MMA, 8 TMEM columns of A, 32 bytes of B
+                        if (g > 0 && groups <= g) return;
 #pragma unroll
-                        for (int j = 1; j < 4; ++j) tc_mma_f16_ts(acc, a + j * 8, b_desc + (uint64_t)(j * 2), idesc, 1u);
-                        if (groups > 2 * h + 1) {
-                            const uint64_t b_desc2 = b_desc + (uint64_t)(b_block >> 4);
+                        for (uint32_t j = 0; j < 4; ++j)
+                            tc_mma_f16_ts<PAIR>(acc, a + g * 32 + j * 8, b_desc + (uint64_t)(g * b_block + j * 2), idesc, g + j > 0 ? 1u : accumulate);
+                    };
+                    const bool leader = elect_one();
+                    if (leader) {
 #pragma unroll
-                            for (int j = 0; j < 4; ++j) tc_mma_f16_ts(acc, a + 32 + j * 8, b_desc2 + (uint64_t)(j * 2), idesc, 1u);
-                        }
+                        for (uint32_t g = 0; g < 3; ++g) multiply(g);
                     }
+                    if constexpr (PAIR) {
+                        // A look at the next stage while these MMAs run: a wait on a barrier that is ready takes about 100 clocks,
+                        // in which the tensor cores would run dry. (With few tokens the next operands are never there this early.)
+                        __syncwarp();
+                        const uint32_t nsb = sb + 1 < b_stages ? sb + 1 : 0;
+                        ready = __all_sync(kFullMask, q_mbar_test(bar_full_b(nsb), (nsb > sb ? ub : ub + 1) & 1) &&
+                                                          q_mbar_test(bar_full_a(t ^ 1), ((count + 1) >> 1) & 1));
+                    }
+                    if (leader) {
+                        multiply(3);
+                        tc_commit<PAIR>(bar_empty_a(t));              // both slots are free once these MMAs have read them
+                        tc_commit<PAIR>(bar_empty_b(sb));
+                        if (ks + (PAIR ? 1 : 2) >= ksteps) tc_commit<PAIR>(bar_acc_full(who, buf));
+                    }
+                    __syncwarp();
+                    accumulate = 1;
                 }
-                if (fail) break;
-                if (leader) {
-                    tc_commit(bar_empty_a(sa));                       // both slots are free once these MMAs have read them
-                    tc_commit(bar_empty_b(sb));
-                    if (ks + 1 == ksteps) tc_commit(bar_acc_full(buf));
-                }
-                __syncwarp();
+                ++count;
                 if (++sb == b_stages) { sb = 0; ++ub; }
-                if (++sa == (uint32_t)kQmmASlots) { sa = 0; ++ua; }
             }
             if (++buf == 2) { buf = 0; ++uacc; }
         }
     } else if (warp < kQmmFirstEpilogueWarp) {
-        // ===================== dequantisers: a thread takes one quantisation group of one weight row per stage =====================
+        // ===================== dequantisers: two teams of eight warps, each takes every other stage =====================
+        // A thread takes two quantisation groups of one weight row. While a team waits for codes, for its slot or for its stores,
+        // the other one computes.
         const uint32_t dw = warp - kQmmFirstDequantWarp;
-        const uint32_t q = dw & 3, gc = dw >> 2;                 // TMEM lane quarter; group within the stage
+        const uint32_t q = dw & 3, gc = ((dw >> 2) & 1) * 2;     // TMEM lane quarter; first group within the stage
+        const uint32_t team = dw >> 3;
         const uint32_t r = q * kWarp + lane;                     // row within the tile = TMEM lane
         // packed codes of the row: 128 bytes whose 16-byte chunks sit at chunk ^ (row % 8) (128-byte TMA swizzle)
-        const uint32_t raw_off0 = r * 128 + (((2 * gc) ^ (r & 7u)) << 4), raw_off1 = r * 128 + (((2 * gc + 1) ^ (r & 7u)) << 4);
-        const uint32_t sc_off = base + plan.off_sc + (r / kMatRows) * 2 * plan.plane_bytes + (r % kMatRows) * ng * 2;
-        const uint32_t a_lane = a_ring + ((q * kWarp) << 16) + gc * 32;
-        uint32_t sr = 0, ur = 0, sc = 0, uc = 0, sa = 0, ua = 0;
-        for (uint32_t tile = blockIdx.x; tile < total_tiles && !fail; tile += gridDim.x) {
+        const uint32_t raw_off = base + r * 128 + (((2 * gc) ^ (r & 7u)) << 4);
+        const uint32_t sc_off = base + plan.off_sc + (r / kMatRows) * 2 * plan.plane_bytes + (r % kMatRows) * ng * 2 + gc * 2;
+        const uint32_t a_slot = a_ring + ((q * kWarp) << 16) + team * 128 + gc * 32;      // the team's slot
+        uint32_t sr = 0, ur = 0, sc = 0, uc = 0, ua = 0, turn = 0;
+        for (uint32_t tile = first_tile; tile < total_tiles && !fail; tile += tile_step) {
             if (!q_mbar_wait(bar_full_sc(sc), uc & 1)) { fail = kErrQmmTimeout | 8; break; }
             const uint32_t sc_base = sc_off + sc * plan.sc_bytes;
             for (uint32_t ks = 0; ks < ksteps; ++ks) {
-                const uint32_t grp = 4 * ks + gc;
-                const bool real = grp < ng;                       // a group past K is neither dequantised nor multiplied
-                const float sf = real ? bf16_bits_to_float((uint16_t)q_lds16(sc_base + grp * 2)) : 0.0f;
-                const float bf = real ? bf16_bits_to_float((uint16_t)q_lds16(sc_base + plan.plane_bytes + grp * 2)) : 0.0f;
-                const bool fast = __all_sync(kFullMask, fabsf(sf) < FastScale<NATURAL_K>::kLimit);
-                if (!q_mbar_wait(bar_full_raw(sr), ur & 1)) { fail = kErrQmmTimeout | 4; break; }
-                const uint4 c0 = q_lds128(base + sr * kQmmRawBytes + raw_off0), c1 = q_lds128(base + sr * kQmmRawBytes + raw_off1);
-                uint4 out[8];
-                if (fast) {                                       // one branch per warp and stage, both arms straight-line
-                    const FastScale<NATURAL_K> s2(sf);
-                    const __half2 b2 = __float2half2_rn(bf);
-                    out[0] = dequant8_fast<NATURAL_K>(c0.x, s2, b2); out[1] = dequant8_fast<NATURAL_K>(c0.y, s2, b2);
-                    out[2] = dequant8_fast<NATURAL_K>(c0.z, s2, b2); out[3] = dequant8_fast<NATURAL_K>(c0.w, s2, b2);
-                    out[4] = dequant8_fast<NATURAL_K>(c1.x, s2, b2); out[5] = dequant8_fast<NATURAL_K>(c1.y, s2, b2);
-                    out[6] = dequant8_fast<NATURAL_K>(c1.z, s2, b2); out[7] = dequant8_fast<NATURAL_K>(c1.w, s2, b2);
-                } else {
-                    const __half2 s2 = __float2half2_rn(sf), b2 = __float2half2_rn(bf);
-                    out[0] = dequant8_wide<NATURAL_K>(c0.x, s2, b2); out[1] = dequant8_wide<NATURAL_K>(c0.y, s2, b2);
-                    out[2] = dequant8_wide<NATURAL_K>(c0.z, s2, b2); out[3] = dequant8_wide<NATURAL_K>(c0.w, s2, b2);
-                    out[4] = dequant8_wide<NATURAL_K>(c1.x, s2, b2); out[5] = dequant8_wide<NATURAL_K>(c1.y, s2, b2);
-                    out[6] = dequant8_wide<NATURAL_K>(c1.z, s2, b2); out[7] = dequant8_wide<NATURAL_K>(c1.w, s2, b2);
-                }
-                __syncwarp();
-                if (lane == 0) q_mbar_arrive(bar_empty_raw(sr));  // the codes are in registers
-                if (++sr == plan.raw_stages) { sr = 0; ++ur; }
-                if (ua > 0 && !q_mbar_wait(bar_empty_a(sa), (ua - 1) & 1)) { fail = kErrQmmTimeout | 5; break; }
-                tc_fence_after();
-                if (real) {
-                    tc_st32(a_lane + sa * 128, out);
+                if (turn == team) {
+                    const uint32_t left = ng - 4 * ks > gc ? ng - 4 * ks - gc : 0;         // groups past K are neither dequantised nor multiplied
+                    float sf[2], bf[2];
+#pragma unroll
+                    for (uint32_t h = 0; h < 2; ++h) {
+                        sf[h] = left > h ? bf16_bits_to_float((uint16_t)q_lds16(sc_base + ks * 8 + h * 2)) : 0.0f;
+                        bf[h] = left > h ? bf16_bits_to_float((uint16_t)q_lds16(sc_base + plan.plane_bytes + ks * 8 + h * 2)) : 0.0f;
+                    }
+                    const bool fast[2] = {(bool)__all_sync(kFullMask, fabsf(sf[0]) < FastScale<NATURAL_K>::kLimit),
+                                          (bool)__all_sync(kFullMask, fabsf(sf[1]) < FastScale<NATURAL_K>::kLimit)};
+                    if (!q_mbar_wait(bar_full_raw(sr), ur & 1)) { fail = kErrQmmTimeout | 4; break; }
+                    const uint32_t src = raw_off + sr * kQmmRawBytes;
+                    uint4 c[4];
+#pragma unroll
+                    for (uint32_t i = 0; i < 4; ++i) c[i] = q_lds128(src ^ (i << 4));
+#pragma unroll
+                    for (uint32_t h = 0; h < 2; ++h) {
+                        const uint4 c0 = c[2 * h], c1 = c[2 * h + 1];
+                        uint4 out[8];
+                        if (fast[h]) {                            // one branch per warp and group, both arms straight-line
+                            const FastScale<NATURAL_K> s2(sf[h]);
+                            const __half2 b2 = __float2half2_rn(bf[h]);
+                            out[0] = dequant8_fast<NATURAL_K>(c0.x, s2, b2); out[1] = dequant8_fast<NATURAL_K>(c0.y, s2, b2);
+                            out[2] = dequant8_fast<NATURAL_K>(c0.z, s2, b2); out[3] = dequant8_fast<NATURAL_K>(c0.w, s2, b2);
+                            out[4] = dequant8_fast<NATURAL_K>(c1.x, s2, b2); out[5] = dequant8_fast<NATURAL_K>(c1.y, s2, b2);
+                            out[6] = dequant8_fast<NATURAL_K>(c1.z, s2, b2); out[7] = dequant8_fast<NATURAL_K>(c1.w, s2, b2);
+                        } else {
+                            const __half2 s2 = __float2half2_rn(sf[h]), b2 = __float2half2_rn(bf[h]);
+                            out[0] = dequant8_wide<NATURAL_K>(c0.x, s2, b2); out[1] = dequant8_wide<NATURAL_K>(c0.y, s2, b2);
+                            out[2] = dequant8_wide<NATURAL_K>(c0.z, s2, b2); out[3] = dequant8_wide<NATURAL_K>(c0.w, s2, b2);
+                            out[4] = dequant8_wide<NATURAL_K>(c1.x, s2, b2); out[5] = dequant8_wide<NATURAL_K>(c1.y, s2, b2);
+                            out[6] = dequant8_wide<NATURAL_K>(c1.z, s2, b2); out[7] = dequant8_wide<NATURAL_K>(c1.w, s2, b2);
+                        }
+                        if (h == 0) {
+                            __syncwarp();
+                            if (lane == 0) q_mbar_arrive(bar_empty_raw(sr));      // the codes are in registers
+                            if (ua > 0 && !q_mbar_wait(bar_empty_a(team), (ua - 1) & 1)) { fail = kErrQmmTimeout | 5; break; }
+                            tc_fence_after();
+                        }
+                        if (left > h) tc_st32(a_slot + h * 32, out);
+                    }
+                    if (fail) break;
                     tc_wait_st();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) {
+                        if constexpr (PAIR) q_mbar_arrive_cluster(q_in_leader(bar_full_a(team)));
+                        else q_mbar_arrive(bar_full_a(team));
+                    }
+                    ++ua;
                 }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) q_mbar_arrive(bar_full_a(sa));
-                if (++sa == (uint32_t)kQmmASlots) { sa = 0; ++ua; }
+                turn ^= 1;
+                if (++sr == raw_stages) { sr = 0; ++ur; }
             }
             __syncwarp();
             if (lane == 0) q_mbar_arrive(bar_empty_sc(sc));       // done with this tile's scale planes
@@ -572,28 +662,49 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map16, const __grid_con
         const uint32_t stage0 = NMAT == 2 ? xch + 8192 : xch;     // two staging tiles of 32 tokens
         const uint32_t mrow = r % kMatRows;
         const uint32_t pos = (NMAT == 2 && !NATURAL_K) ? permuted_col(mrow) : mrow;      // the GeGLU output feeds the down GEMM
-        uint32_t buf = 0, uacc = 0, flip = 0;
-        for (uint32_t tile = blockIdx.x; tile < total_tiles && !fail; tile += gridDim.x) {
-            tl.locate(table, ngroups, wrow_tiles, tile);
-            const uint32_t first = tl.wt * kMatRows;
-            const uint32_t nrows = args.rows - first < kMatRows ? args.rows - first : kMatRows;
-            if (!q_mbar_wait(bar_acc_full(buf), uacc & 1)) fail = kErrQmmTimeout | 9;
+        uint32_t buf = 0, uacc = 0, flip = 0, turn = 0;
+        for (uint32_t tile = first_tile; tile < total_tiles && !fail; tile += tile_step, tl.next()) {
+            tl.locate(table, ngroups, lane);
+            const uint32_t first = (tl.wt * kCtas + rank) * kMatRows;
+            const uint32_t left = first < args.rows ? args.rows - first : 0, nrows = left < kMatRows ? left : kMatRows;
+            const bool two = !PAIR && ksteps > 1;                     // both issuers had stages of the tile
+            const uint32_t one = PAIR ? 0 : turn;                     // the issuer of its first stage
+            if (!q_mbar_wait(bar_acc_full(one, buf), uacc & 1)) fail = kErrQmmTimeout | 9;
+            if (two && !q_mbar_wait(bar_acc_full(one ^ 1, buf), uacc & 1)) fail = kErrQmmTimeout | 9;
+            turn ^= ksteps & 1;
             // every warp of the role leaves together: the barriers below count all four
             asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbarrier.red.or.pred q, 1, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
                          : "=r"(flip) : "r"(fail) : "memory");
             if (flip) { if (!fail) fail = kErrQmmTimeout | 9; break; }
             tc_fence_after();
-            const uint32_t acc = tmem_base + ((q * kWarp) << 16) + buf * 128;
+            const uint32_t acc = tmem_base + ((q * kWarp) << 16) + (PAIR ? buf : 2 * buf + one) * kAccTok;
+            const uint32_t acc2 = tmem_base + ((q * kWarp) << 16) + (2 * buf + (one ^ 1)) * kAccTok;      // the other issuer's
             uint32_t which = 0;
             for (uint32_t c0 = 0; c0 < tl.ntok; c0 += 32, which ^= 1) {
                 uint32_t va[16], vb[16];
                 tc_ld16(acc + c0, va);
                 tc_ld16(acc + c0 + 16, vb);                       // past the tile's tokens: stale columns of the buffer, never stored
                 tc_wait_ld();
+                if constexpr (!PAIR) {
+                    if (two) {
+                        uint32_t v2[16];
+                        tc_ld16(acc2 + c0, v2);
+                        tc_wait_ld();
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) va[j] = __float_as_uint(__uint_as_float(va[j]) + __uint_as_float(v2[j]));
+                        tc_ld16(acc2 + c0 + 16, v2);
+                        tc_wait_ld();
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) vb[j] = __float_as_uint(__uint_as_float(vb[j]) + __uint_as_float(v2[j]));
+                    }
+                }
                 if (c0 + 32 >= tl.ntok) {                         // the accumulators are in registers
                     tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) q_mbar_arrive(bar_acc_empty(buf));
+                    if (lane == 0) {
+                        if constexpr (PAIR) q_mbar_arrive_cluster(q_in_leader(bar_acc_empty(buf)));
+                        else q_mbar_arrive(bar_acc_empty(buf));
+                    }
                 }
                 const uint32_t stage = stage0 + which * (32 * kTokBytes) + pos * 2;
                 if constexpr (NMAT == 2) {
@@ -665,9 +776,11 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map16, const __grid_con
     if (fail && lane == 0) atomicCAS(args.error, 0u, fail);
     tc_fence_before();
     __syncthreads();
+    if constexpr (PAIR) q_cluster_sync();      // the other CTA's MMAs, copies and arrivals no longer need this one
     if (warp == 1) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)kQmmTmemCols) : "memory");
+        if constexpr (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)kQmmTmemCols) : "memory");
+        else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)kQmmTmemCols) : "memory");
     }
 }
 
@@ -687,16 +800,17 @@ static EncodeTiledFn encode_tiled_fn() {
     return fn;
 }
 
-// fp16 matrix [rows, k] with a row stride: box = 64 columns x box_rows rows, 128-byte swizzle, zero fill outside.
+// fp16 matrix [rows, k] with a row stride, seen as [k / 64][rows][64]: one copy brings a stage, four blocks of 64 columns x
+// box_rows rows, each block laid out as the MMA wants it (128-byte swizzle, rows of 128 bytes); zero fill outside.
 static tf_status make_x_map(tf_context* ctx, CUtensorMap* map, const void* x, uint64_t rows, uint32_t k, uint32_t stride_elems,
                             uint32_t box_rows, const char* name) {
     EncodeTiledFn fn = encode_tiled_fn();
     TF_REQUIRE(ctx, fn != nullptr, TF_ERR_UNSUPPORTED, "%s: cuTensorMapEncodeTiled is not available in this driver", name);
-    const cuuint64_t dims[2] = {k, rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)stride_elems * 2};
-    const cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
-    const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(x), dims, strides, box, estr,
+    const cuuint64_t dims[3] = {64, rows, k / 64};
+    const cuuint64_t strides[2] = {(cuuint64_t)stride_elems * 2, 128};
+    const cuuint32_t box[3] = {64, (cuuint32_t)box_rows, kQmmStageK / 64};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(x), dims, strides, box, estr,
                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     TF_REQUIRE(ctx, r == CUDA_SUCCESS, TF_ERR_CUDA, "%s: cuTensorMapEncodeTiled(activations) failed (%d)", name, (int)r);
@@ -712,7 +826,7 @@ static tf_status make_w_map(tf_context* ctx, CUtensorMap* map, const void* w, ui
     TF_REQUIRE(ctx, fn != nullptr, TF_ERR_UNSUPPORTED, "%s: cuTensorMapEncodeTiled is not available in this driver", name);
     const cuuint64_t dims[3] = {k / 2, rows, experts};
     const cuuint64_t strides[2] = {(cuuint64_t)(k / 2), expert_stride};
-    const cuuint32_t box[3] = {(cuuint32_t)(kQmmRawK / 2), (cuuint32_t)box_rows, 1};
+    const cuuint32_t box[3] = {(cuuint32_t)(kQmmStageK / 2), (cuuint32_t)box_rows, 1};
     const cuuint32_t estr[3] = {1, 1, 1};
     const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(w), dims, strides, box, estr,
                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -723,7 +837,7 @@ static tf_status make_w_map(tf_context* ctx, CUtensorMap* map, const void* w, ui
 
 // Divides the 227 KB of shared memory for K columns. Packed codes first (four stages keep 48 to 64 KB in flight, what an
 // SM's share of the HBM rate needs at its latency), the activation ring takes what the scale planes leave: three slots of
-// 128 tokens at K = 2816. Long rows give up stages, then (from K = 7040 on) the second buffer of scale planes: the next tile's
+// 64 rows at K = 2816. Long rows give up stages, then (from K = 7040 on) the second buffer of scale planes: the next tile's
 // planes are then copied between two tiles, which costs less than halving the tokens per tile (2000 x 2112 x 8192: 104 us with
 // one buffer, 152 with two and tiles of 64 tokens).
 constexpr uint32_t kQmmMaxK = 9024;
@@ -733,12 +847,12 @@ static bool qmm_plan(uint32_t k, uint32_t nmat, QmmPlan* p) {
     const uint32_t ng = k / kGroup;
     p->plane_bytes = ((kQmmRows / nmat) * ng * 2u + 15u) & ~15u;
     p->sc_bytes = nmat * 2 * p->plane_bytes;
-    const uint32_t slot = kQmmTokMax * kQmmHalfK * 2u;              // 32 KB
+    const uint32_t slot = kQmmBoxMax * kQmmRowBytes;                // 32 KB
     uint32_t fixed = 0;
     p->raw_stages = 0;
     for (p->sc_bufs = 4 * p->sc_bytes <= 48u * 1024u ? 4u : 2u;; p->sc_bufs = 1) {
         fixed = p->sc_bufs * p->sc_bytes + kQmmStageBytes + TF_MAX_ROUTER_EXPERTS * 16u + 1024u;
-        for (uint32_t raw = kQmmRawMax; raw >= 2 && !p->raw_stages; --raw)
+        for (uint32_t raw = kQmmRawMax; raw >= 2 && !p->raw_stages; raw -= 2)         // even: a slot belongs to one team of dequantisers
             if (fixed + raw * kQmmRawBytes + 2 * slot <= budget) p->raw_stages = raw;
         if (p->raw_stages) break;
         if (p->sc_bufs == 1) return false;
@@ -753,17 +867,23 @@ static bool qmm_plan(uint32_t k, uint32_t nmat, QmmPlan* p) {
     return true;
 }
 
-// Tokens per tile of a dense launch: rounds of the grid x the time of a tile, which is the larger of its MMAs (four clocks
-// per token and 128 columns) and its dequantisation (about 330 clocks per 128 columns), plus a fixed part.
-static uint32_t qmm_dense_per_tile(uint32_t tokens, uint32_t wrow_tiles, uint32_t halves, uint32_t sms) {
-    uint32_t best = 16;
+// Tokens per tile of a dense launch, by one CTA or by pairs: rounds of the grid x the clocks of a tile's stages, and what start
+// and last epilogue take. The clocks of a stage are fitted to launches of 16 to 64 and of 32 to 128 tokens per tile (us, 1000 x 2112
+// x 2816: 50, 28, 25, 20 and 36, 23, 24, 17; 333 x 2112 x 2816: 22, 16, 12, 13 and 21, 14, 14, 15; 200 x 512 x 1024: 6.8, 6.9, 7.5,
+// 7.5 and 8.5, 8.7, 9.2, 10).
+struct QmmDense {
+    uint32_t ctas, per_tile;
+};
+static QmmDense qmm_dense_tiles(uint32_t tokens, uint32_t rows, uint32_t mat_rows, uint32_t stages, uint32_t sms) {
+    QmmDense best{1, 16};
     uint64_t best_cost = ~0ull;
-    for (uint32_t per = kQmmTokMax; per >= 16; per -= 16) {
-        const uint64_t tiles = (uint64_t)wrow_tiles * ((tokens + per - 1) / per);
-        const uint64_t step = 4ull * per > 330 ? 4ull * per : 330;
-        const uint64_t cost = ((tiles + sms - 1) / sms) * (halves * step + 1500);
-        if (cost < best_cost) { best_cost = cost; best = per; }
-    }
+    for (uint32_t ctas = 1; ctas <= 2 && ctas <= sms; ++ctas)
+        for (uint32_t per = ctas * kQmmBoxMax; per >= ctas * 16u; per -= ctas * 16u) {
+            const uint64_t tiles = (uint64_t)((rows + ctas * mat_rows - 1) / (ctas * mat_rows)) * ((tokens + per - 1) / per);
+            const uint64_t rounds = (tiles + sms / ctas - 1) / (sms / ctas);
+            const uint64_t cost = ctas == 1 ? rounds * stages * (1000 + 5 * per) + 9500 : rounds * stages * (1250 + 3 * per) + 11400;
+            if (cost < best_cost) { best_cost = cost; best = {ctas, per}; }
+        }
     return best;
 }
 
@@ -775,38 +895,38 @@ static tf_status launch_qmm_prepare(tf_context* ctx, void* stream, QmmArgs& a, i
     a.groups = static_cast<uint4*>(ctx->qmm_groups) + table * (TF_MAX_ROUTER_EXPERTS + 1);
     a.totals = reinterpret_cast<uint32_t*>(a.groups + TF_MAX_ROUTER_EXPERTS);
     launch_pdl(qmm_prepare_kernel, dim3(1), dim3(TF_MAX_ROUTER_EXPERTS), 0, static_cast<cudaStream_t>(stream), a.groups, a.totals,
-               a.route_groups, a.route_counters, a.dense_tokens, a.dense_per_tile);
+               a.route_groups, a.route_counters, a.dense_tokens, a.dense_per_tile, a.ctas);
     return check_launch(ctx, "qmm_prepare");
 }
 
 // W[m]: base of matrix m's packed plane for expert 0 (dense: the matrix itself); a.S, a.B likewise. A routed launch's table
 // has been filled by the caller.
-template <int NMAT, bool NATURAL_K>
-static tf_status launch_qmm(tf_context* ctx, void* stream, QmmArgs& a, const void* x, uint64_t x_rows, uint32_t x_stride,
+template <int NMAT, bool NATURAL_K, bool PAIR>
+static tf_status launch_qmm_kernel(tf_context* ctx, void* stream, QmmArgs& a, const void* x, uint64_t x_rows, uint32_t x_stride,
                             const uint8_t* const* W, uint64_t experts, uint64_t expert_stride, bool dense, const char* name) {
     TF_REQUIRE(ctx, a.k % kGroup == 0 && a.k >= (uint32_t)kGroup, TF_ERR_INVALID_ARGUMENT, "%s: K must be a positive multiple of 64", name);
     TF_REQUIRE(ctx, a.rows % 8 == 0 && a.rows > 0, TF_ERR_INVALID_ARGUMENT, "%s: the weight rows must be a positive multiple of 8", name);
     TF_REQUIRE(ctx, aligned(x, 16) && (x_stride * 2) % 16 == 0, TF_ERR_ALIGNMENT, "%s: activation rows must be 16-byte aligned", name);
     TF_REQUIRE(ctx, qmm_plan(a.k, NMAT, &a.plan), TF_ERR_UNSUPPORTED, "%s: K=%u needs more shared memory for the scale planes than there is", name, a.k);
     constexpr uint32_t kMatRows = kQmmRows / NMAT;
-    // Activation boxes of 16, 32, 64 and 128 rows. A dense launch knows its tiles (full ones and a last one) and encodes only
-    // the boxes that those are made of: an encode is most of a microsecond of host time, and small products are bound by it.
-    uint32_t boxes = 16u | 32u | 64u | 128u;
+    // Activation boxes of 16, 32, 48 and 64 rows. A dense launch knows its tiles (full ones and a last one) and encodes only
+    // the boxes of those: an encode is most of a microsecond of host time, and small products are bound by it.
+    constexpr uint32_t kCtas = PAIR ? 2 : 1;
+    uint32_t boxes = 15u;
     if (dense) {
-        a.dense_per_tile = qmm_dense_per_tile(a.dense_tokens, (a.rows + kMatRows - 1) / kMatRows, (a.k + kQmmHalfK - 1) / kQmmHalfK,
-                                              (uint32_t)ctx->sm_count);
-        const uint32_t rest = (a.dense_tokens % a.dense_per_tile + 15u) & ~15u;
-        boxes = rest | (a.dense_tokens >= a.dense_per_tile ? a.dense_per_tile : 0u);
+        const uint32_t rest = a.dense_tokens % a.dense_per_tile;
+        boxes = (a.dense_tokens >= a.dense_per_tile ? 1u << (a.dense_per_tile / kCtas / 16 - 1) : 0u) |
+                (rest ? 1u << ((rest + 16 * kCtas - 1) / (16 * kCtas) - 1) : 0u);
     }
     CUtensorMap xmap[4], wmap[2];
     int some = -1;
     for (int i = 0; i < 4; ++i) {
-        if (!(boxes & (16u << i))) continue;
-        if (tf_status s = make_x_map(ctx, &xmap[i], x, x_rows, a.k, x_stride, 16u << i, name)) return s;
+        if (!(boxes & (1u << i))) continue;
+        if (tf_status s = make_x_map(ctx, &xmap[i], x, x_rows, a.k, x_stride, 16u * (i + 1), name)) return s;
         some = i;
     }
     for (int i = 0; i < 4; ++i)
-        if (!(boxes & (16u << i))) xmap[i] = xmap[some];
+        if (!(boxes & (1u << i))) xmap[i] = xmap[some];
     for (int m = 0; m < NMAT; ++m)
         if (tf_status s = make_w_map(ctx, &wmap[m], W[m], a.rows, a.k, experts, dense ? (uint64_t)a.rows * (a.k / 2) : expert_stride, kMatRows, name)) return s;
     if (NMAT == 1) wmap[1] = wmap[0];
@@ -815,17 +935,27 @@ static tf_status launch_qmm(tf_context* ctx, void* stream, QmmArgs& a, const voi
     a.error = ctx->device_error;
     if (dense)
         if (tf_status s = launch_qmm_prepare(ctx, stream, a, kQmmDenseTable, name)) return s;
-    auto kern = qmm_tcgen05_kernel<NMAT, NATURAL_K>;
+    auto kern = qmm_tcgen05_kernel<NMAT, NATURAL_K, PAIR>;
     static DeviceSmemCache configured;
     if (tf_status s = ensure_dynamic_smem(ctx, kern, configured, a.plan.total)) return s;
-    uint32_t grid = (uint32_t)ctx->sm_count;
+    uint32_t grid = (uint32_t)ctx->sm_count / kCtas;
     if (dense) {
-        const uint64_t tiles = (uint64_t)((a.rows + kMatRows - 1) / kMatRows) * ((a.dense_tokens + a.dense_per_tile - 1) / a.dense_per_tile);
+        const uint64_t tiles = (uint64_t)((a.rows + kCtas * kMatRows - 1) / (kCtas * kMatRows)) * ((a.dense_tokens + a.dense_per_tile - 1) / a.dense_per_tile);
         if (tiles < grid) grid = (uint32_t)tiles;
     }
-    launch_pdl(kern, dim3(grid), dim3(kQmmThreads), a.plan.total, static_cast<cudaStream_t>(stream), xmap[0], xmap[1], xmap[2], xmap[3],
-               wmap[0], wmap[1], a);
+    launch_pdl_cluster(kern, dim3(grid * kCtas), dim3(kQmmThreads), a.plan.total, static_cast<cudaStream_t>(stream), kCtas, xmap[0], xmap[1],
+                       xmap[2], xmap[3], wmap[0], wmap[1], a);
     return check_launch(ctx, name);
+}
+template <int NMAT, bool NATURAL_K>
+static tf_status launch_qmm(tf_context* ctx, void* stream, QmmArgs& a, const void* x, uint64_t x_rows, uint32_t x_stride,
+                            const uint8_t* const* W, uint64_t experts, uint64_t expert_stride, bool dense, const char* name) {
+    if (dense) {
+        const QmmDense t = qmm_dense_tiles(a.dense_tokens, a.rows, kQmmRows / NMAT, (a.k + kQmmStageK - 1) / kQmmStageK, (uint32_t)ctx->sm_count);
+        a.ctas = t.ctas; a.dense_per_tile = t.per_tile;
+    }
+    return a.ctas == 2 ? launch_qmm_kernel<NMAT, NATURAL_K, true>(ctx, stream, a, x, x_rows, x_stride, W, experts, expert_stride, dense, name)
+                       : launch_qmm_kernel<NMAT, NATURAL_K, false>(ctx, stream, a, x, x_rows, x_stride, W, experts, expert_stride, dense, name);
 }
 
 tf_status launch_qmm_generic(tf_context* ctx, void* stream, const uint8_t* W, const uint16_t* S, const uint16_t* B,
@@ -860,6 +990,9 @@ tf_status tf_grouped_moe_tensorcore(tf_context* ctx, void* stream, const void* x
     b.S[0] = plane(offsets->down_s_off); b.B[0] = plane(offsets->down_b_off);
     b.route_groups = routes->groups; b.route_counters = routes->counters;
     b.rows = d; b.k = f; b.out = static_cast<uint16_t*>(out_rows); b.out_stride = d;
+    // Pairs of CTAs from 40 rows per expert on. Both GEMMs of a layer of 128 experts, one CTA / pairs: 333 tokens (21 rows) 126 / 150
+    // us with uniform and 70 / 62 with Zipf routing, 700 (44 rows) 159 / 157 and 105 / 94, 1000 190 / 165, 4096 518 / 385.
+    a.ctas = b.ctas = (uint64_t)x_rows >= 40ull * num_experts ? 2 : 1;
     // both tables first: between the two GEMMs the second one's would wait for the first to end
     TF_REQUIRE(ctx, tf::qmm_plan(d, 2, &a.plan) && tf::qmm_plan(f, 1, &b.plan), TF_ERR_UNSUPPORTED,
                "%s: D=%u or F=%u needs more shared memory for the scale planes than there is", name, d, f);
