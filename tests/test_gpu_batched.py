@@ -213,6 +213,12 @@ def test_grouped_moe_random_vs_oracle(tf_ctx, oracle, T, D, F, E, K):
             assert o.rel_error(y_batched, y32) < FP16_CHAINED
 
 
+# The line between the two kernels of the routed down projection (64 pairs), and chunks of one to a few tokens on both sides.
+@pytest.mark.parametrize("T,E", [(7, 48), (8, 48), (9, 16), (20, 128)])
+def test_grouped_moe_few_tokens_of_the_production_width(tf_ctx, oracle, T, E):
+    test_grouped_moe_random_vs_oracle(tf_ctx, oracle, T, 2816, 704, E, 8)
+
+
 def test_reduce_token_major(tf_ctx, oracle):
     # Tests/TurboFieldfare/Core/Kernels/Prefill/PrefillMoETests.swift:8-64
     import torch

@@ -275,7 +275,7 @@ constexpr int kWStages = 3;             // ring depth (items) of the tile ring (
 // Narrow single-matrix tiles (the routed down projection: 16 rows x 352 bytes) are a few KB each, so three of them in
 // flight per CTA leave the memory system idle; their ring is deeper.
 template <int NMAT, int KC>
-__host__ __device__ constexpr uint32_t ring_stages() { return (NMAT == 1 && KC > 0 && KC <= 1024) ? 8u : (uint32_t)kWStages; }
+__host__ __device__ constexpr uint32_t ring_stages() { return (NMAT == 1 && KC > 0 && KC <= 1024) ? 7u : (uint32_t)kWStages; }
 constexpr int kReducers = 2;            // reducer warps; reducer q owns the items and the partial buffer of parity q
 constexpr int kRedStages = kReducers;   // partial-sum buffers
 constexpr int kTileRows = 16;           // weight rows per MMA tile (the m of m16n8k16)
@@ -321,6 +321,7 @@ struct GroupedArgs {
     uint32_t k;                // columns (D for gate/up, F for down)
     uint32_t top_k;
     uint32_t dense_tokens;     // dense mode: number of tokens
+    uint32_t after_gate_up;    // down launch whose predecessor on the stream is the gate/up launch of the same call
     uint32_t* error;           // device word: 0, or the code of the wait that gave up
 };
 
@@ -488,8 +489,18 @@ grouped_ksplit_kernel(const GroupedArgs args) {
     auto bar_red_free = [&](uint32_t r) { return bar_base + (2 * kSt + kRedStages + r) * 8; };
 
     const uint32_t tiles = args.rows / kTileRows;
-    pdl_launch_dependents();
-    pdl_wait();              // routing metadata and activations come from the kernels before this one
+    // A down launch asks for its weights while the last gate/up blocks still run: a block that finds a place on an SM fills its
+    // ring, and only the compute warps wait. What it reads early, the routing metadata, is complete then, because the routed
+    // gate/up launch lets its dependent start only after its own wait. With this and the router's later release (see
+    // router_split_kernel) a 30-layer step of 1 token took 994 -> 895 us, of 4 tokens 1532 -> 1254, of 8 tokens 1875 -> 1655.
+    const bool early = NMAT == 1 && args.after_gate_up;
+    if (NMAT == 2 && !DENSE) {
+        pdl_wait();
+        pdl_launch_dependents();
+    } else {
+        pdl_launch_dependents();
+        if (!early) pdl_wait();          // routing metadata and activations come from the kernels before this one
+    }
     constexpr uint32_t kTokens = (uint32_t)kChunkTokens * NT;
     uint32_t* chunk_first = reinterpret_cast<uint32_t*>(smem + lay.off_chunks());
     uint32_t total_chunks;
@@ -521,7 +532,10 @@ grouped_ksplit_kernel(const GroupedArgs args) {
     // contiguous item range per CTA: consecutive items share the chunk, whose activations stay in registers
     const uint32_t item_begin = (uint32_t)((uint64_t)total_items * blockIdx.x / gridDim.x);
     const uint32_t item_end = (uint32_t)((uint64_t)total_items * (blockIdx.x + 1) / gridDim.x);
-    if (item_begin >= item_end) return;
+    if (item_begin >= item_end) {
+        if (early) pdl_wait();
+        return;
+    }
     const uint32_t n_items = item_end - item_begin;
 
     if (threadIdx.x == 0) {
@@ -558,6 +572,7 @@ grouped_ksplit_kernel(const GroupedArgs args) {
         cur.tile = item_begin % tiles;
         cur.group = !DENSE && NT > 1 ? find_group(chunk_first, args.counters[0], cur.chunk) : 0u;
         resolve_chunk<NMAT, DENSE, NT>(args, cur, chunk_first);
+        if (early) pdl_wait();           // the activations
 
         // Four registers that stay zero: the accumulator input of every group's first MMA (a literal zero makes the
         // compiler clear four fresh registers per MMA).
@@ -959,14 +974,18 @@ grouped_down_kernel(const GroupedArgs args) {
         fence_proxy_async();
     }
     __syncthreads();
-    pdl_wait();
+    const bool early = args.after_gate_up;      // as in grouped_ksplit_kernel: the ring fills as soon as a gate/up block has left the SM
+    if (!early) pdl_wait();
     // contiguous ranges of whole stages (a chunk's tiles are a multiple of four)
     const uint32_t total_chunks = args.counters[1];
     const uint32_t total_stages = total_chunks * (tiles / kDownSub);
     const uint32_t stage_begin = (uint32_t)((uint64_t)total_stages * blockIdx.x / gridDim.x);
     const uint32_t n_stages = (uint32_t)((uint64_t)total_stages * (blockIdx.x + 1) / gridDim.x) - stage_begin;
     const uint32_t item_begin = stage_begin * kDownSub, n_items = n_stages * kDownSub;
-    if (n_items == 0) return;
+    if (n_items == 0) {
+        if (early) pdl_wait();
+        return;
+    }
     ItemCursor<1> cur;
     uint32_t fail = 0;
     auto place = [&](uint32_t item) {                         // the cursor's chunk and tile; resolves a new chunk
@@ -977,6 +996,7 @@ grouped_down_kernel(const GroupedArgs args) {
     };
     cur.chunk = 0xFFFFFFFFu;
     if (warp < kDownWarps) {
+        if (early) pdl_wait();           // the activations
         float zc[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) asm volatile("mov.f32 %0, 0f00000000;" : "=f"(zc[j]));
@@ -1199,11 +1219,11 @@ static tf_status launch_grouped(tf_context* ctx, void* stream, GroupedArgs& args
     return launch_grouped_k<NMAT, DENSE, OUT_MODE, 0, 1>(ctx, stream, args, name);
 }
 
-// The routed down projection: the whole-row kernel for the width that it is built for, from 320 (token, expert) pairs on (40
-// tokens of eight experts); with fewer, its deeper pipeline does not pay for the time that it takes to fill. Steps of 30 layers
-// with it and without: 32 tokens 3.27 and 3.23 ms, 48 tokens 3.81 and 3.87, 64 tokens 3.88 and 4.21, 200 tokens 7.50 and 8.26
-// (the latter with 16-token chunks in the column-split kernel).
-constexpr uint32_t kDownMinPairs = 320;
+// The routed down projection: the whole-row kernel for the width that it is built for, from 64 (token, expert) pairs on (8 tokens
+// of eight experts); with fewer, its deeper pipeline does not pay for the time that it takes to fill. Steps of 30 layers with it
+// and without, us: 4 tokens 1285 and 1254, 8 tokens 1631 and 1655, 16 tokens 2128 and 2176, 32 tokens 2918 and 3062, 64 tokens 3880
+// and 4210, 200 tokens 7500 and 8260 (the latter with 16-token chunks in the column-split kernel).
+constexpr uint32_t kDownMinPairs = 64;
 template <int OUT_MODE>
 static tf_status launch_grouped_down(tf_context* ctx, void* stream, GroupedArgs& args, uint64_t pairs, const char* name) {
     constexpr int kGroups = 11;
@@ -1379,6 +1399,7 @@ tf_status grouped_moe_batched(tf_context* ctx, void* stream, const void* hidden,
     b.chunk_start = routes->chunk_start; b.counters = routes->counters;
     b.x = static_cast<const uint16_t*>(acts_scratch); b.x_stride = f;
     b.out = route_partials; b.out_stride = d; b.rows = d; b.k = f; b.top_k = top_k;
+    b.after_gate_up = 1;
     if (partials_f32) return tf::launch_grouped_down<tf::kOutPartialF32>(ctx, stream, b, (uint64_t)query_count * top_k, "tf_grouped_moe_batched(down)");
     return tf::launch_grouped_down<tf::kOutPartialF16>(ctx, stream, b, (uint64_t)query_count * top_k, "tf_grouped_moe_batched(down)");
 }
@@ -1528,6 +1549,7 @@ tf_status tf_grouped_moe_streamed(tf_context* ctx, void* stream, const void* hid
     b.chunk_start = scratch->chunk_start; b.counters = scratch->counters;
     b.x = reinterpret_cast<const uint16_t*>(acts); b.x_stride = f;
     b.out = tf::byte_ptr(route_partials, route_partials_off); b.out_stride = d; b.rows = d; b.k = f; b.top_k = params->top_k;
+    b.after_gate_up = 1;
     if (tf_status s = tf::launch_grouped_down<tf::kOutPartialF16>(ctx, stream, b, params->pair_count, "tf_grouped_moe_streamed(down)")) return s;
     if (microbatches_out) *microbatches_out = (params->pair_count + pair_microbatch_rows - 1) / pair_microbatch_rows;
     return TF_OK;
@@ -1591,6 +1613,7 @@ tf_status tf_shared_expert_int4_block(tf_context* ctx, void* stream, const void*
     b.dense[0] = mp[2];
     b.x = static_cast<const uint16_t*>(scratch_act); b.x_stride = fs;
     b.out = tf::byte_ptr(y, y_off); b.out_stride = y_stride_elements; b.rows = d; b.k = fs; b.dense_tokens = rows;
+    b.after_gate_up = 1;
     return tf::launch_grouped<1, true, tf::kOutDenseF16, 2112>(ctx, stream, b, rows > tf::kWideDenseRows, "tf_shared_expert_int4_block(down)");
 }
 

@@ -91,6 +91,7 @@ struct QmmArgs {
     const uint32_t* route_counters;
     uint32_t dense_tokens, dense_per_tile;
     uint32_t ctas;          // CTAs of a tile: 2 for pairs
+    uint32_t after_gate_up; // down launch whose predecessor on the stream is the gate/up launch of the same call
     // problem
     uint32_t rows;          // weight rows (output features)
     uint32_t k;             // columns (input features)
@@ -404,7 +405,8 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map16, const __grid_con
     const uint32_t ksteps = (ng + 3) / 4;                              // stages per tile
     const uint32_t wrow_tiles = (args.rows + kCtas * kMatRows - 1) / (kCtas * kMatRows);
 
-    pdl_launch_dependents();
+    constexpr bool kRoutedGateUp = NMAT == 2 && !NATURAL_K;
+    if (!kRoutedGateUp) pdl_launch_dependents();
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < (uint32_t)kQmmRawMax; ++s) { q_mbar_init(bar_full_raw(s), 1); q_mbar_init(bar_empty_raw(s), kQmmTeamWarps); }
         for (uint32_t s = 0; s < (uint32_t)kQmmBMax; ++s) { q_mbar_init(bar_full_b(s), 1); q_mbar_init(bar_empty_b(s), 1); }
@@ -427,7 +429,11 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map16, const __grid_con
             asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
         }
     }
-    pdl_wait();                                                        // routes and activations come from the kernels before this one
+    // The routed down launch takes its tables and weights while the last gate/up tiles are still being computed elsewhere; only the
+    // copies of its activations wait. The tables are complete: gate/up lets its dependent start after its own wait.
+    const bool early = NMAT == 1 && args.after_gate_up;
+    if (!early) pdl_wait();                                             // routes and activations come from the kernels before this one
+    if (kRoutedGateUp) pdl_launch_dependents();
     const uint32_t ngroups = args.totals[0], total_tiles = args.totals[1] * wrow_tiles, n_top = args.totals[2];
     if (threadIdx.x < ngroups) table[threadIdx.x] = args.groups[threadIdx.x];
     tc_fence_before();
@@ -494,6 +500,7 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map16, const __grid_con
     } else if (warp == 2) {
         // ===================== copy issuer: activations, one copy per stage =====================
         uint32_t sb = 0, ub = 0;
+        if (early) pdl_wait();
         for (uint32_t tile = first_tile; tile < total_tiles && !fail; tile += tile_step, tl.next()) {
             tl.locate(table, ngroups, lane);
             const uint32_t box = (tl.ntok + kStep - 1) / kStep * 16;  // rows per CTA
@@ -990,6 +997,7 @@ tf_status tf_grouped_moe_tensorcore(tf_context* ctx, void* stream, const void* x
     b.S[0] = plane(offsets->down_s_off); b.B[0] = plane(offsets->down_b_off);
     b.route_groups = routes->groups; b.route_counters = routes->counters;
     b.rows = d; b.k = f; b.out = static_cast<uint16_t*>(out_rows); b.out_stride = d;
+    b.after_gate_up = 1;
     // Pairs of CTAs from 40 rows per expert on. Both GEMMs of a layer of 128 experts, one CTA / pairs: 333 tokens (21 rows) 126 / 150
     // us with uniform and 70 / 62 with Zipf routing, 700 (44 rows) 159 / 157 and 105 / 94, 1000 190 / 165, 4096 518 / 385.
     a.ctas = b.ctas = (uint64_t)x_rows >= 40ull * num_experts ? 2 : 1;

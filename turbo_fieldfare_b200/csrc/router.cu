@@ -79,7 +79,6 @@ router_split_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ 
     const uint16_t* hrow = hidden + (size_t)row * hidden_stride;
     const bool a16 = (reinterpret_cast<uintptr_t>(wsrc) & 15) == 0 && (d & 15) == 0;
     const bool x16 = (reinterpret_cast<uintptr_t>(hrow) & 15) == 0 && (reinterpret_cast<uintptr_t>(eff) & 15) == 0 && (d & 7) == 0;
-    pdl_launch_dependents();
     if (a16 && x16 && ne * d <= kSplitThreads * 16 * 6 && d <= kSplitThreads * 8 * 3) {
         // latency path: every load of the block is issued before the first one is consumed
         uint4 wv[6], hv[3], ev[3];
@@ -146,6 +145,9 @@ router_split_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ 
         if (logit_bias) logit = __fadd_rn(logit, logit_bias[e]);
         if (lane == 0) scratch_logits[(size_t)row * TF_MAX_ROUTER_EXPERTS + e] = logit;
     }
+    // Only now: the routed gate/up launch would otherwise sit on the SMs, waiting, from the first microsecond on, and keep the
+    // shared expert's blocks, which could run beside this kernel, until it has ended.
+    pdl_launch_dependents();
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -235,6 +237,7 @@ router_split_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ 
 // (ticket) selects the top-k of its R rows, one warp per row; the block that completes the last row group builds the
 // grouping tables.
 constexpr int kRowsThreads = 256;
+constexpr uint32_t kRowsLateRelease = 52;
 constexpr int kRowsExpertsPerBlock = kRowsThreads / kWarp;
 template <bool X_BF16, int R>
 __global__ void __launch_bounds__(kRowsThreads)
@@ -257,7 +260,11 @@ router_rows_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S
     const uint32_t row0 = blockIdx.x * R;
     const uint32_t e0 = blockIdx.y * kRowsExpertsPerBlock;
     const uint32_t ne = num_experts - e0 < (uint32_t)kRowsExpertsPerBlock ? num_experts - e0 : (uint32_t)kRowsExpertsPerBlock;
-    pdl_launch_dependents();
+    // As in router_split_kernel the routed launch is let in after the logits, as long as all blocks of this one are resident (six
+    // per SM at the production width): 12 rows 1953 -> 1808 us per 30-layer step, 48 rows 3735 -> 3468. With more rows the shared
+    // expert's blocks get in before the routed ones anyhow, and a late release costs 0.2 % (64 rows: 3859 and 3866).
+    const bool late = gridDim.x <= kRowsLateRelease;
+    if (!late) pdl_launch_dependents();
     // expert rows (contiguous in every plane; d is a multiple of 64 and the planes are 16-byte aligned by contract)
     {
         const uint8_t* wsrc = W + (size_t)e0 * d;
@@ -328,6 +335,7 @@ router_rows_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S
             if (lane == 0 && row0 + r < rows) scratch_logits[(size_t)(row0 + r) * TF_MAX_ROUTER_EXPERTS + e] = logit;
         }
     }
+    if (late) pdl_launch_dependents();
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
