@@ -213,6 +213,33 @@ def test_tile_gemv(tf_ctx, oracle, m, n, scale):
     assert np.all(np.abs(o.f16_to_f32(out[:m]) - ref) <= bound)
 
 
+# The streaming product: remainders of the 16-row tile (the last tile repeats rows), fewer tiles than blocks and than slots, rows of 1024
+# columns up to those that leave two teams, and what stays with the other kernels (1023 columns' side of the line, odd planes).
+@pytest.mark.parametrize("m,n", [(4096, 1024), (4104, 1280), (4100, 2816), (5002, 2816), (4112, 4096), (40008, 1024), (4096, 5632), (4096, 6144),
+                                 (4099, 1280), (4098, 768)])
+def test_streaming_gemv(tf_ctx, oracle, m, n):
+    test_tile_gemv(tf_ctx, oracle, m, n, 1.0)
+
+
+# The greedy head on both sides of the streaming form's line (2^27 weights), ragged vocabularies.
+@pytest.mark.parametrize("v", [47660, 47664, 47666, 50008])
+def test_lm_head_rows_around_the_streaming_line(tf_ctx, oracle, v):
+    from tests.test_gpu_decode import _lm_head_gpu
+    o, d = oracle, 2816
+    rng = np.random.default_rng(v)
+    mat = config0_matrix(o, v, d, rng)
+    norm = o.f32_to_bf16((1.0 + 0.02 * rng.standard_normal(d)).astype(np.float32))
+    hidden = o.f32_to_f16(rng.standard_normal(d).astype(np.float32))
+    want, logits = o.lm_head_greedy(hidden, norm, mat)
+    got = _lm_head_gpu(tf_ctx, o, hidden, norm, mat, d, v)
+    assert got == want or abs(float(logits[got]) - float(logits[want])) <= 1e-5 * max(1.0, abs(float(logits[want])))
+
+
+def test_lm_head_ties_and_non_finite_logits_of_the_streaming_form(tf_ctx, oracle):
+    from tests.test_gpu_decode import test_lm_head_greedy_streaming_ties_and_non_finite_logits as ties
+    ties(tf_ctx, oracle, 2816, 47680)
+
+
 # Shared memory of the down kernel on either side of what a launch may use unasked (48 KB, the static part included): K * F / 64
 # of 368, then 369 to 372. Smaller sizes first: the limit, once raised, stays raised.
 @pytest.mark.parametrize("K,F", [(8, 2944), (3, 7872), (5, 4736), (7, 3392), (6, 3968), (8, 8192)])
