@@ -385,6 +385,12 @@ def test_decode_sized_stack_equals_the_chain_of_entry_points_bit_for_bit(tf_ctx,
         stack.close()
 
 
+# Blocks whose combine takes several tokens per thread block: one round and a part of the next, two and a part, an exact multiple.
+@pytest.mark.parametrize("T", [445, 889, 592])
+def test_stack_of_many_tokens_equals_the_chain_of_entry_points_bit_for_bit(tf_ctx, oracle, T):
+    test_decode_sized_stack_equals_the_chain_of_entry_points_bit_for_bit(tf_ctx, oracle, T, 256)
+
+
 @pytest.mark.parametrize("T", [1, 40])
 def test_block_forward_with_8bit_shared_expert(tf_ctx, oracle, T):
     """A layer whose shared expert is 8-bit affine (tf_moe_layer.shared_bits = 8; SharedExpertInt8.swift:55-210): the
