@@ -41,8 +41,10 @@ __host__ __device__ inline size_t router_approx_smem_bytes() {
     return 2 * (size_t)kApxExperts * kApxWPitch + 2 * (size_t)kApxTokens * kApxXPitch + 2 * 4 * kApxTokens * sizeof(float);
 }
 __host__ __device__ inline size_t router_recheck_smem_bytes(uint32_t d, uint32_t num_experts, uint32_t tokens_per_block) {
-    return (size_t)tokens_per_block * ((size_t)d + num_experts) * sizeof(float);
+    return ((size_t)tokens_per_block * (((size_t)d + num_experts) * sizeof(float) + num_experts * sizeof(uint16_t)) + 15) & ~(size_t)15;
 }
+// Two expert rows per warp, where the re-check stages them (see router_logit_staged).
+__host__ __device__ inline size_t router_recheck_code_bytes(uint32_t d) { return (size_t)kRecheckWarps * 2 * d; }
 
 __device__ __forceinline__ void cp_async_16(void* smem_dst, const void* global_src) {
     const uint32_t dst = (uint32_t)__cvta_generic_to_shared(smem_dst);
@@ -386,21 +388,6 @@ __device__ __forceinline__ float router_logit_chunk(float acc, const uint32_t (&
     }
     return acc;
 }
-// The lowest expert of the candidate masks (32 experts per word), removed from them; 0xFFFFFFFF when none is left.
-template <int N>
-__device__ __forceinline__ uint32_t pop_candidate(uint32_t (&masks)[N]) {
-    uint32_t e = 0xFFFFFFFFu;
-#pragma unroll
-    for (int j = N - 1; j >= 0; --j)
-        if (masks[j]) e = (uint32_t)(__ffs((int)masks[j]) - 1) + j * kWarp;
-    if (e != 0xFFFFFFFFu) {
-#pragma unroll
-        for (int j = 0; j < N; ++j)
-            if ((uint32_t)j == e / kWarp) masks[j] &= masks[j] - 1u;
-    }
-    return e;
-}
-
 // The same for a group count known at compile time (the production width): all of an expert's codes are requested at
 // once, lane l holds the scale and bias of groups l and l + 32, and nothing in the loop is guarded.
 template <int GROUPS>
@@ -438,10 +425,102 @@ __device__ __forceinline__ float router_logit_all(const LogitOperands<GROUPS>& r
     return warp_sum(acc);
 }
 
+// The same for two experts whose rows are staged in shared memory, in a loop of a few dozen instructions; activations and their sums
+// are shared. For the forms with several warps per token, whose warps have one to three candidates: with the unrolled form above,
+// some ten KB of instructions executed once or twice, that phase took 35 900 clocks at 333 rows, 20 500 with this one (10 200
+// since the candidates are a list). With a warp per token and 16 warps per SM the unrolled form stays ahead (4096 rows, 30
+// layers: 22.1 ms against 22.5 with two warps per token and this form).
+template <int GROUPS>
+__device__ __forceinline__ float2 router_logits_staged(const uint8_t* codes_a, const uint8_t* codes_b, uint32_t a0, uint32_t a1, uint32_t b0,
+                                                       uint32_t b1, const float* xf, int lane) {
+    static_assert(GROUPS <= 2 * kWarp, "two scale words per lane");
+    const uint8_t *wa = codes_a + lane * 2, *wb = codes_b + lane * 2;
+    const float* xl = xf + lane * 2;
+    float acc_a = 0.0f, acc_b = 0.0f;
+#pragma unroll 4
+    for (int g = 0; g < GROUPS; ++g) {
+        const uint32_t va = __shfl_sync(kFullMask, g < kWarp ? a0 : a1, g % kWarp), vb = __shfl_sync(kFullMask, g < kWarp ? b0 : b1, g % kWarp);
+        const uint32_t qa = *reinterpret_cast<const uint16_t*>(wa + g * kGroup), qb = *reinterpret_cast<const uint16_t*>(wb + g * kGroup);
+        const float2 xv = *reinterpret_cast<const float2*>(xl + g * kGroup);
+        const float sum = __fadd_rn(xv.x, xv.y);
+        // byte -> float through the 2^23 mantissa trick (exact for 0...255)
+        const float pa = __fmaf_rn(__uint_as_float(0x4B000000u | (qa >> 8)) - 8388608.0f, xv.y,
+                                   __fmul_rn(__uint_as_float(0x4B000000u | (qa & 0xFFu)) - 8388608.0f, xv.x));
+        const float pb = __fmaf_rn(__uint_as_float(0x4B000000u | (qb >> 8)) - 8388608.0f, xv.y,
+                                   __fmul_rn(__uint_as_float(0x4B000000u | (qb & 0xFFu)) - 8388608.0f, xv.x));
+        acc_a = __fmaf_rn(__uint_as_float(va << 16), pa, acc_a);
+        acc_b = __fmaf_rn(__uint_as_float(vb << 16), pb, acc_b);
+        acc_a = __fmaf_rn(__uint_as_float(va & 0xFFFF0000u), sum, acc_a);
+        acc_b = __fmaf_rn(__uint_as_float(vb & 0xFFFF0000u), sum, acc_b);
+    }
+    return make_float2(warp_sum(acc_a), warp_sum(acc_b));
+}
+
+// The experts that can reach the top k, in list (ascending), and their number: those whose upper bound is not below the top_k-th
+// largest lower bound. N: experts per lane. (A list: warps that took their candidates off bit masks, each skipping those of the token's
+// other warps, spent up to 20 000 clocks on that at eight warps per token.)
+template <int N>
+__device__ __forceinline__ uint32_t router_candidates(const float2* __restrict__ approx_row, const float* __restrict__ logit_bias,
+                                                      uint32_t num_experts, uint32_t top_k, int lane, uint16_t* list /* shared */) {
+    float upper[N];
+    uint32_t key[N];
+    bool bad = false;
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+        const uint32_t e = lane + j * kWarp;
+        upper[j] = -INFINITY;
+        key[j] = 0u;
+        if (e < num_experts) {
+            const float2 am = approx_row[e];
+            float v = am.x;
+            if (!isfinite(am.x) || !isfinite(am.y)) bad = true;
+            if (logit_bias) v = __fadd_rn(v, logit_bias[e]);
+            if (v == -INFINITY) {
+                key[j] = topk_score_key(-INFINITY);             // a -inf bias: the canonical logit is -inf as well
+            } else if (!isfinite(v)) {
+                bad = true;
+            } else {
+                const float eps = fmaf(kApxRelError, am.y, fabsf(v) * 2.384185791015625e-07f);    // + 2^-22 |v|: the bias add
+                upper[j] = v + eps;
+                key[j] = topk_score_key(v - eps);
+            }
+        }
+    }
+    // the top_k-th largest lower bound
+    uint32_t lb_key = 0u;
+#pragma unroll 1
+    for (uint32_t r = 0; r < top_k; ++r) {
+        uint32_t best = 0u;
+#pragma unroll
+        for (int j = 0; j < N; ++j) best = max(best, key[j]);
+        lb_key = __reduce_max_sync(kFullMask, best);
+        const uint32_t who = __reduce_min_sync(kFullMask, (best == lb_key && lb_key != 0u) ? (uint32_t)lane : 32u);
+        if ((uint32_t)lane == who) {
+            bool done = false;
+#pragma unroll
+            for (int j = 0; j < N; ++j)
+                if (!done && key[j] == lb_key) { key[j] = 0u; done = true; }
+        }
+    }
+    if (lb_key == 0u) bad = true;                 // fewer than top_k comparable experts
+    bad = __any_sync(kFullMask, bad);
+    const float lb = bad ? -INFINITY : topk_key_score(lb_key);
+    uint32_t count = 0;
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+        const uint32_t e = lane + j * kWarp;
+        const bool cand = e < num_experts && (bad || upper[j] >= lb);
+        const uint32_t mask = __ballot_sync(kFullMask, cand);
+        if (cand) list[count + __popc(mask & ((1u << lane) - 1u))] = (uint16_t)e;
+        count += __popc(mask);
+    }
+    return count;
+}
+
 // WPT warps per token: candidates from the approximate logits and their bounds (every warp of the token finds them), canonical
 // logits of the candidates (dealt out to the warps), top-k and softmax as in every other router kernel (one warp). A
 // canonical logit is one long dependent chain, so with few rows a token's eight or nine must not follow one another: one
-// warp per token took 30 us at 333 rows. With grp.sorted_pairs the block that finishes the last row groups all of them.
+// warp per token took 30 us at 333 rows; four take 15. With grp.sorted_pairs the block that finishes the last row groups all of them.
 template <bool X_BF16, int GROUPS, int WPT>          // GROUPS: d / 64 when known at compile time, 0 for any width
 __global__ void __launch_bounds__(kRecheckWarps * kWarp, 2)
 router_recheck_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S, const uint16_t* __restrict__ B,
@@ -479,68 +558,48 @@ router_recheck_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict_
             if (c < d) *reinterpret_cast<float2*>(xf + c) = make_float2(x0, x1);
         }
     }
-    constexpr int kPerLane = TF_MAX_ROUTER_EXPERTS / kWarp;
-    float upper[kPerLane];
-    uint32_t key[kPerLane];
-    bool bad = false;
-#pragma unroll
-    for (int j = 0; j < kPerLane; ++j) {
-        const uint32_t e = lane + j * kWarp;
-        upper[j] = -INFINITY;
-        key[j] = 0u;
-        if (e < num_experts) {
-            const float2 am = approx[(size_t)row * num_experts + e];
-            float v = am.x;
-            if (!isfinite(am.x) || !isfinite(am.y)) bad = true;
-            if (logit_bias) v = __fadd_rn(v, logit_bias[e]);
-            if (v == -INFINITY) {
-                key[j] = topk_score_key(-INFINITY);             // a -inf bias: the canonical logit is -inf as well
-            } else if (!isfinite(v)) {
-                bad = true;
-            } else {
-                const float eps = fmaf(kApxRelError, am.y, fabsf(v) * 2.384185791015625e-07f);    // + 2^-22 |v|: the bias add
-                upper[j] = v + eps;
-                key[j] = topk_score_key(v - eps);
-            }
-        }
-    }
-    // the top_k-th largest lower bound
-    uint32_t lb_key = 0u;
-    for (uint32_t r = 0; r < top_k; ++r) {
-        uint32_t best = 0u;
-#pragma unroll
-        for (int j = 0; j < kPerLane; ++j) best = max(best, key[j]);
-        lb_key = __reduce_max_sync(kFullMask, best);
-        const uint32_t who = __reduce_min_sync(kFullMask, (best == lb_key && lb_key != 0u) ? (uint32_t)lane : 32u);
-        if ((uint32_t)lane == who) {
-            bool done = false;
-#pragma unroll
-            for (int j = 0; j < kPerLane; ++j)
-                if (!done && key[j] == lb_key) { key[j] = 0u; done = true; }
-        }
-    }
-    if (lb_key == 0u) bad = true;                 // fewer than top_k comparable experts
-    bad = __any_sync(kFullMask, bad);
-    const float lb = bad ? -INFINITY : topk_key_score(lb_key);
-    uint32_t masks[kPerLane];
-#pragma unroll
-    for (int j = 0; j < kPerLane; ++j) {
-        const uint32_t e = lane + j * kWarp;
-        const bool cand = e < num_experts && (bad || upper[j] >= lb);
-        masks[j] = __ballot_sync(kFullMask, cand);
-    }
+    // (every warp of a token writes the same list)
+    uint16_t* list = reinterpret_cast<uint16_t*>(reinterpret_cast<float*>(smem) + (size_t)kTokens * (d + num_experts)) + (size_t)slot * num_experts;
+    const float2* approx_row = approx + (size_t)row * num_experts;
+    const uint32_t candidates = num_experts <= 4u * kWarp ? router_candidates<4>(approx_row, logit_bias, num_experts, top_k, lane, list)
+                                                          : router_candidates<TF_MAX_ROUTER_EXPERTS / kWarp>(approx_row, logit_bias, num_experts, top_k, lane, list);
     if (WPT == 1) __syncwarp(); else __syncthreads();             // the row's activations and the cleared scores
     // this warp's candidates: every WPT-th one
+    uint32_t next = part;
     auto next_candidate = [&]() {
-        const uint32_t e = pop_candidate(masks);
-#pragma unroll
-        for (int i = 1; i < WPT; ++i) pop_candidate(masks);
+        const uint32_t e = next < candidates ? (uint32_t)list[next] : 0xFFFFFFFFu;
+        next += WPT;
         return e;
     };
-    for (int i = 0; i < part; ++i) pop_candidate(masks);
     // (expert, chunk) pairs in one software pipeline: the next pair's loads are issued before the current pair is multiplied
     uint32_t ld_e = next_candidate(), ld_g = 0u;
-    if constexpr (GROUPS > 0) {
+    if constexpr (GROUPS > 0 && WPT > 1) {
+        // two candidates at a time (a last one alone is computed twice)
+        uint8_t* codes = smem + router_recheck_smem_bytes(d, num_experts, kTokens) + (size_t)warp * 2 * d;
+        auto request = [&](uint32_t e, uint8_t* dst, uint32_t& s0, uint32_t& s1) {
+            const uint8_t* src = W + (size_t)e * d;
+            for (uint32_t i = lane; i < d / 16; i += kWarp) cp_async_16(dst + i * 16, src + i * 16);
+            const uint16_t *sr = S + (size_t)e * GROUPS, *br = B + (size_t)e * GROUPS;
+            s0 = lane < GROUPS ? (uint32_t)__ldg(sr + lane) | ((uint32_t)__ldg(br + lane) << 16) : 0u;
+            s1 = lane + kWarp < GROUPS ? (uint32_t)__ldg(sr + lane + kWarp) | ((uint32_t)__ldg(br + lane + kWarp) << 16) : 0u;
+        };
+#pragma unroll 1
+        for (uint32_t ea = ld_e; ea != 0xFFFFFFFFu; ea = next_candidate()) {
+            const uint32_t eb = next_candidate();
+            uint32_t a0, a1, b0, b1;
+            request(ea, codes, a0, a1);
+            if (eb != 0xFFFFFFFFu) request(eb, codes + d, b0, b1);
+            else { b0 = a0; b1 = a1; }
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncwarp();
+            const float2 l = router_logits_staged<GROUPS>(codes, eb != 0xFFFFFFFFu ? codes + d : codes, a0, a1, b0, b1, xf, lane);
+            if (lane == 0) {
+                scores[ea] = logit_bias ? __fadd_rn(l.x, logit_bias[ea]) : l.x;
+                if (eb != 0xFFFFFFFFu) scores[eb] = logit_bias ? __fadd_rn(l.y, logit_bias[eb]) : l.y;
+            }
+            __syncwarp();                                         // the rows have been read
+        }
+    } else if constexpr (GROUPS > 0) {
         // two operand sets used in turns: the next candidate's loads are in flight while the current one is multiplied
         LogitOperands<GROUPS> ra, rb;
         auto finish = [&](uint32_t e, float l) {
