@@ -145,9 +145,6 @@ router_split_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ 
         if (logit_bias) logit = __fadd_rn(logit, logit_bias[e]);
         if (lane == 0) scratch_logits[(size_t)row * TF_MAX_ROUTER_EXPERTS + e] = logit;
     }
-    // Only now: the routed gate/up launch would otherwise sit on the SMs, waiting, from the first microsecond on, and keep the
-    // shared expert's blocks, which could run beside this kernel, until it has ended.
-    pdl_launch_dependents();
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -167,6 +164,10 @@ router_split_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ 
     if (warp == 0)
         warp_select_topk(scores, num_experts, top_k, per_expert_scale, out_idx + (size_t)row * top_k,
                          out_w + (size_t)row * top_k, lane);
+    // Only now: the routed gate/up launch would otherwise sit on the SMs, waiting, from the first microsecond on, and keep both launches
+    // of the shared expert, which run beside this kernel, until it has ended. One token, 30 layers: released at the start 994
+    // us, after the logits 895 (863 with the faster selection), here 860; one block called eagerly 32.8, 28.6 and 26.9.
+    pdl_launch_dependents();
     if (grp.sorted_pairs == nullptr) return;
     if (gridDim.x == 1) {
         // One token: a pair's place is the number of selected experts with a smaller id; every group holds one pair
@@ -237,7 +238,6 @@ router_split_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ 
 // (ticket) selects the top-k of its R rows, one warp per row; the block that completes the last row group builds the
 // grouping tables.
 constexpr int kRowsThreads = 256;
-constexpr uint32_t kRowsLateRelease = 52;
 constexpr int kRowsExpertsPerBlock = kRowsThreads / kWarp;
 template <bool X_BF16, int R>
 __global__ void __launch_bounds__(kRowsThreads)
@@ -260,11 +260,6 @@ router_rows_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S
     const uint32_t row0 = blockIdx.x * R;
     const uint32_t e0 = blockIdx.y * kRowsExpertsPerBlock;
     const uint32_t ne = num_experts - e0 < (uint32_t)kRowsExpertsPerBlock ? num_experts - e0 : (uint32_t)kRowsExpertsPerBlock;
-    // As in router_split_kernel the routed launch is let in after the logits, as long as all blocks of this one are resident (six
-    // per SM at the production width): 12 rows 1953 -> 1808 us per 30-layer step, 48 rows 3735 -> 3468. With more rows the shared
-    // expert's blocks get in before the routed ones anyhow, and a late release costs 0.2 % (64 rows: 3859 and 3866).
-    const bool late = gridDim.x <= kRowsLateRelease;
-    if (!late) pdl_launch_dependents();
     // expert rows (contiguous in every plane; d is a multiple of 64 and the planes are 16-byte aligned by contract)
     {
         const uint8_t* wsrc = W + (size_t)e0 * d;
@@ -335,7 +330,6 @@ router_rows_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S
             if (lane == 0 && row0 + r < rows) scratch_logits[(size_t)(row0 + r) * TF_MAX_ROUTER_EXPERTS + e] = logit;
         }
     }
-    if (late) pdl_launch_dependents();
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -369,8 +363,12 @@ router_rows_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S
     }
     __syncthreads();
     if (!is_last) return;
+    // Only now, as in router_split_kernel. 30 layers, us, released at the start, after the logits and here: 4 rows 1532, 1284 and 1222,
+    // 8 rows 1875, 1684 and 1575, 11 rows 1877, 1734 and 1686, 32 rows 3131, 2839 and 2784, 48 rows 3748, 3329 and 3317, 64 rows 3859,
+    // 3866 and 3836.
+    pdl_launch_dependents();
     __threadfence();
-    group_routes_in_block<false>(out_idx, out_w, rows, top_k, num_experts, grp, smem);
+    group_routes_in_block<true>(out_idx, out_w, rows, top_k, num_experts, grp, smem);
 }
 
 // Many rows (batched decode, prefill): one block per row.
@@ -589,7 +587,7 @@ static tf_status launch_router(tf_context* ctx, void* stream, const uint8_t* W, 
         RouterGroupOut grp{};
         if (routes) {
             grp = router_group_out(routes);
-            const size_t need = router_group_smem_bytes(rows * top_k, num_experts, false);
+            const size_t need = router_group_smem_bytes(rows * top_k, num_experts, true);
             if (need > smem_rows) smem_rows = need;
         }
         TF_REQUIRE(ctx, smem_rows <= 200 * 1024, TF_ERR_UNSUPPORTED, "%s: D=%u too large", name, d);

@@ -8,11 +8,13 @@ namespace tf {
 
 // Top-k of a row of scores (highest first, ties to the lower expert index) and the softmax over the selected scores
 // times the per-expert gain, rounded to fp16: the first k entries of the order (score desc, index asc), which is the
-// result of the reference's insertion scan (Metal/MoE/moe.metal:152-184). Every lane keeps its experts' scores in registers as
-// order-preserving integer keys; a round is one warp-wide integer maximum followed by a warp-wide minimum over the
-// indices that hold it; a selected expert drops to -inf, so it can only come back when nothing greater is left (fewer
-// comparable candidates than top_k). NaN scores never win. The exponentials are taken by top_k lanes at once and summed
-// in rank order. `scores` is only read.
+// result of the reference's insertion scan (Metal/MoE/moe.metal:152-184). Every lane holds its experts' scores as
+// order-preserving integer keys, sorted; a round is one warp-wide integer maximum over the lanes' greatest keys (lanes that tie
+// compare indices), and the winner's lane moves on to its next key. When nothing above -inf is left (fewer comparable candidates
+// than top_k), the remaining ranks repeat the lowest expert that is selected or at -inf, expert 0 if there is none. NaN scores never
+// win. The per-expert gains travel during the rounds; the exponentials are taken by top_k lanes at once and summed in rank
+// order. `scores` is only read. (With two reductions and a scan of the lane's keys per round and the gains loaded at the end, 3300
+// to 6000 clocks for 8 of 128 in a step; 2700 to 3600 with this.)
 __device__ __forceinline__ uint32_t topk_score_key(float v) {
     if (v != v) return 0u;
     const uint32_t b = __float_as_uint(v + 0.0f);             // -0 and +0 compare equal: one key for both
@@ -25,39 +27,65 @@ template <int kPerLane>        // experts per lane: num_experts <= 32 * kPerLane
 __device__ __forceinline__ void warp_select_topk_held(const float* scores /*shared*/, uint32_t num_experts, uint32_t top_k,
                                                       const uint16_t* __restrict__ per_expert_scale,
                                                       uint32_t* __restrict__ out_idx, uint16_t* __restrict__ out_w, int lane) {
-    uint32_t key[kPerLane];
+    constexpr uint32_t kNegInfKey = 0x007FFFFFu;
+    uint32_t key[kPerLane], idx[kPerLane];
+    uint16_t gain[kPerLane];
+    uint32_t low = 0xFFFFFFFFu;                  // this lane's lowest expert that is selected or at -inf
 #pragma unroll
     for (int j = 0; j < kPerLane; ++j) {
         const uint32_t e = lane + j * kWarp;
+        idx[j] = e;
         key[j] = e < num_experts ? topk_score_key(scores[e]) : 0u;
+        gain[j] = e < num_experts ? __ldg(per_expert_scale + e) : (uint16_t)0;
+        if (key[j] == kNegInfKey) low = min(low, e);
     }
-    const uint32_t neg_inf_key = 0x007FFFFFu;
-    float my_score = 0.0f, max_s = 0.0f;
-    uint32_t my_idx = 0;
-    for (uint32_t r = 0; r < top_k; ++r) {
-        uint32_t best = 0u, best_e = 0xFFFFFFFFu;
+    // descending by key; equal keys keep their order, which is ascending by expert
 #pragma unroll
-        for (int j = 0; j < kPerLane; ++j) {
-            const uint32_t e = lane + j * kWarp;
-            if (e < num_experts && key[j] > best) { best = key[j]; best_e = e; }      // ascending e: ties keep the lower index
+    for (int i = 1; i < kPerLane; ++i) {
+#pragma unroll
+        for (int j = i; j > 0; --j) {
+            const bool swap = key[j] > key[j - 1];
+            const uint32_t k0 = swap ? key[j] : key[j - 1], k1 = swap ? key[j - 1] : key[j];
+            const uint32_t i0 = swap ? idx[j] : idx[j - 1], i1 = swap ? idx[j - 1] : idx[j];
+            key[j - 1] = k0; key[j] = k1; idx[j - 1] = i0; idx[j] = i1;
         }
-        const uint32_t top = __reduce_max_sync(kFullMask, best);
-        uint32_t winner = __reduce_min_sync(kFullMask, (best == top && top != 0u) ? best_e : 0xFFFFFFFFu);
-        float top_score = topk_key_score(top);
-        if (winner == 0xFFFFFFFFu) { winner = 0u; top_score = -INFINITY; }            // no comparable candidate at all
+    }
+    float my_score = 0.0f, max_s = 0.0f;
+    uint32_t my_idx = 0, r = 0;
+    for (; r < top_k; ++r) {
+        const uint32_t top = __reduce_max_sync(kFullMask, key[0]);
+        if (top <= kNegInfKey) break;
+        const uint32_t holders = __ballot_sync(kFullMask, key[0] == top);
+        uint32_t winner;
+        if (holders & (holders - 1u)) winner = __reduce_min_sync(kFullMask, key[0] == top ? idx[0] : 0xFFFFFFFFu);
+        else winner = __shfl_sync(kFullMask, idx[0], __ffs((int)holders) - 1);
+        const float top_score = topk_key_score(top);
         if (r == 0) max_s = top_score;
         if ((uint32_t)lane == r) { my_score = top_score; my_idx = winner; }
-        if (winner < num_experts && (winner % kWarp) == (uint32_t)lane) {
+        if (key[0] == top && idx[0] == winner) {
+            low = min(low, winner);
 #pragma unroll
-            for (int j = 0; j < kPerLane; ++j)
-                if ((uint32_t)j == winner / kWarp) key[j] = neg_inf_key;
+            for (int j = 1; j < kPerLane; ++j) { key[j - 1] = key[j]; idx[j - 1] = idx[j]; }
+            key[kPerLane - 1] = 0u;
         }
+    }
+    if (r < top_k) {
+        const uint32_t lowest = __reduce_min_sync(kFullMask, low), winner = lowest == 0xFFFFFFFFu ? 0u : lowest;
+        if (r == 0) max_s = -INFINITY;
+        if ((uint32_t)lane >= r) { my_score = -INFINITY; my_idx = winner; }
+    }
+    uint32_t my_gain = 0;
+#pragma unroll
+    for (int j = 0; j < kPerLane; ++j) {
+        const uint32_t v = __shfl_sync(kFullMask, (uint32_t)gain[j], (int)(my_idx % kWarp));
+        if (my_idx / kWarp == (uint32_t)j) my_gain = v;
     }
     const float ex = (uint32_t)lane < top_k ? expf(my_score - max_s) : 0.0f;
     float sum_exp = 0.0f;
-    for (uint32_t r = 0; r < top_k; ++r) sum_exp += __shfl_sync(kFullMask, ex, (int)r);
+#pragma unroll 4
+    for (uint32_t k = 0; k < top_k; ++k) sum_exp += __shfl_sync(kFullMask, ex, (int)k);
     if ((uint32_t)lane < top_k) {
-        const float w = ex / sum_exp * bf16_bits_to_float(per_expert_scale[my_idx]);
+        const float w = ex / sum_exp * bf16_bits_to_float((uint16_t)my_gain);
         out_idx[lane] = my_idx;
         out_w[lane] = __half_as_ushort(__float2half_rn(w));
     }
