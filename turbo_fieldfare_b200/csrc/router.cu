@@ -238,6 +238,7 @@ router_split_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ 
 // (ticket) selects the top-k of its R rows, one warp per row; the block that completes the last row group builds the
 // grouping tables.
 constexpr int kRowsThreads = 256;
+constexpr uint32_t kRowsLateRelease = 52;
 constexpr int kRowsExpertsPerBlock = kRowsThreads / kWarp;
 template <bool X_BF16, int R>
 __global__ void __launch_bounds__(kRowsThreads)
@@ -260,6 +261,13 @@ router_rows_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S
     const uint32_t row0 = blockIdx.x * R;
     const uint32_t e0 = blockIdx.y * kRowsExpertsPerBlock;
     const uint32_t ne = num_experts - e0 < (uint32_t)kRowsExpertsPerBlock ? num_experts - e0 : (uint32_t)kRowsExpertsPerBlock;
+    // As in router_split_kernel the routed launch is let in before the grouping, as long as all blocks of this one are resident (six
+    // per SM at the production width). 30 layers, us, released at the start, after the logits and there: 4 rows 1532, 1284 and
+    // 1222, 8 rows 1875, 1684 and 1575, 11 rows 1877, 1734 and 1686, 32 rows 3131, 2839 and 2784, 48 rows 3748, 3329 and 3317. With
+    // more rows the shared expert's gate/up blocks get in before the routed ones anyhow, and its down projection, 17 us by then,
+    // must not (64 rows: 3868 at the start; late 3836 or, when it got in, 3970).
+    const bool late = gridDim.x <= kRowsLateRelease;
+    if (!late) pdl_launch_dependents();
     // expert rows (contiguous in every plane; d is a multiple of 64 and the planes are 16-byte aligned by contract)
     {
         const uint8_t* wsrc = W + (size_t)e0 * d;
@@ -363,10 +371,7 @@ router_rows_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S
     }
     __syncthreads();
     if (!is_last) return;
-    // Only now, as in router_split_kernel. 30 layers, us, released at the start, after the logits and here: 4 rows 1532, 1284 and 1222,
-    // 8 rows 1875, 1684 and 1575, 11 rows 1877, 1734 and 1686, 32 rows 3131, 2839 and 2784, 48 rows 3748, 3329 and 3317, 64 rows 3859,
-    // 3866 and 3836.
-    pdl_launch_dependents();
+    if (late) pdl_launch_dependents();
     __threadfence();
     group_routes_in_block<true>(out_idx, out_w, rows, top_k, num_experts, grp, smem);
 }
