@@ -620,7 +620,7 @@ static tf_status launch_router(tf_context* ctx, void* stream, const uint8_t* W, 
         return check_launch(ctx, name);
     } else if ((own || rows >= ctx->router_tensorcore_min_rows) && !out_logits && vec16 && d % kApxChunk == 0 && aligned(S, 8) && aligned(B, 8) &&
                num_experts <= TF_MAX_ROUTER_EXPERTS && top_k <= (uint32_t)kWarp && top_k <= num_experts &&
-               router_recheck_smem_bytes(d, num_experts, kRecheckWarps) <= 200 * 1024 && (own || router_scratch(ctx, st, rows, num_experts))) {
+               router_recheck_smem_bytes(d, num_experts, kRecheckWarps) <= 205 * 1024 && (own || router_scratch(ctx, st, rows, num_experts))) {
         // logits on the tensor cores, then the canonical logits of the few experts that can reach the top k
         float2* approx = own ? own->approx : static_cast<float2*>(ctx->router_approx);
         const uint32_t sms = (uint32_t)ctx->sm_count;
