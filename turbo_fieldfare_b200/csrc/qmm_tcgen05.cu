@@ -534,7 +534,10 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map16, const __grid_con
             const uint32_t n = (tl.ntok + kStep - 1) / kStep * kStep;
             const uint32_t idesc = qmm_idesc(kCtas * kQmmRows, n);
             const uint32_t b_block = (n / kCtas * 128) >> 4;         // 64 columns of a slot, in units of the descriptor
-            if (uacc > 0 && !q_mbar_wait(bar_acc_empty(buf), (uacc - 1) & 1)) { fail = kErrQmmTimeout | 2; break; }
+            // Only for a tile that this warp has a stage of: the parity tells phases apart only while the barrier is at most one
+            // phase ahead of the wait, and a tile of one stage can be multiplied and emptied without the other issuer.
+            const bool takes_part = PAIR || ksteps > 1 || (count & 1) == who;
+            if (takes_part && uacc > 0 && !q_mbar_wait(bar_acc_empty(buf), (uacc - 1) & 1)) { fail = kErrQmmTimeout | 2; break; }
             tc_fence_after();
             const uint32_t acc = tmem_base + (PAIR ? buf * kAccTok : (2 * buf + who) * kAccTok);
             uint32_t accumulate = 0;
