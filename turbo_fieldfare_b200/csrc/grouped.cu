@@ -30,6 +30,8 @@
 // (deterministic), apply the epilogue and store. No warp ever meets another at a
 // block-wide barrier in the steady state. Every mbarrier wait is bounded: on expiry
 // the kernel records an error code and returns.
+#include <type_traits>
+
 #include "async_copy.cuh"
 #include "peer.cuh"
 
@@ -306,11 +308,11 @@ struct GroupedArgs {
     // dense mode (one matrix set for all tokens)
     MatPlanes dense[2];
     // routing metadata (routed mode)
-    const tf_pair* sorted_pairs;
-    const tf_group* groups;
-    const uint32_t* chunk_group;
-    const uint32_t* chunk_start;
-    const uint32_t* counters;
+    EarlyTable<tf_pair> sorted_pairs;
+    EarlyTable<tf_group> groups;
+    EarlyTable<uint32_t> chunk_group;
+    EarlyTable<uint32_t> chunk_start;
+    EarlyTable<uint32_t> counters;
     // activations in: row r of the chunk's tokens at x + row_index * x_stride (elements)
     const uint16_t* x;
     uint32_t x_stride;
@@ -426,7 +428,8 @@ __device__ __forceinline__ uint32_t find_group(const uint32_t* chunk_first, uint
     return lo;
 }
 // chunk_first: NT = 2, the groups' first chunks of 16 tokens in shared memory (the global tables hold chunks of 8)
-template <int NMAT, bool DENSE, int NT>
+// EARLY: the caller may not have waited for the previous launch (see EarlyTable).
+template <int NMAT, bool DENSE, int NT, bool EARLY = NMAT == 1>
 __device__ __forceinline__ void resolve_chunk(const GroupedArgs& args, ItemCursor<NMAT>& c, const uint32_t* chunk_first) {
     constexpr uint32_t kTokens = (uint32_t)kChunkTokens * NT;
     if constexpr (DENSE) {
@@ -442,10 +445,10 @@ __device__ __forceinline__ void resolve_chunk(const GroupedArgs& args, ItemCurso
             gi = c.group;
             first = chunk_first[gi];
         } else {
-            gi = args.chunk_group[c.chunk];
-            first = args.chunk_start[gi];
+            gi = args.chunk_group.at<EARLY>(c.chunk);
+            first = args.chunk_start.at<EARLY>(gi);
         }
-        const tf_group grp = args.groups[gi];
+        const tf_group grp = args.groups.at<EARLY>(gi);
         const uint32_t cin = c.chunk - first;
         const uint8_t* blob = args.pool_base + (uint64_t)grp.expert * args.expert_stride;
 #pragma unroll
@@ -490,9 +493,10 @@ grouped_ksplit_kernel(const GroupedArgs args) {
 
     const uint32_t tiles = args.rows / kTileRows;
     // A down launch asks for its weights while the last gate/up blocks still run: a block that finds a place on an SM fills its
-    // ring, and only the compute warps wait. What it reads early, the routing metadata, is complete then, because the routed
-    // gate/up launch lets its dependent start only after its own wait. With this and the router's later release (see
+    // ring, and only the compute warps wait. What it reads early, the routing metadata, is complete then (see EarlyTable), because
+    // the routed gate/up launch lets its dependent start only after its own wait. With this and the router's later release (see
     // router_split_kernel) a 30-layer step of 1 token took 994 -> 895 us, of 4 tokens 1532 -> 1254, of 8 tokens 1875 -> 1655.
+    // (Waiting before the tables instead costs 46 us of a step of 1 token, 62 at 4, 16 at 8, 35 to 55 at 11 to 32, nothing from 48 on.)
     const bool early = NMAT == 1 && args.after_gate_up;
     if (NMAT == 2 && !DENSE) {
         pdl_wait();
@@ -508,11 +512,11 @@ grouped_ksplit_kernel(const GroupedArgs args) {
         total_chunks = (args.dense_tokens + kTokens - 1) / kTokens;
     } else if constexpr (NT > 1) {
         // one warp scans the groups' chunk counts, 32 groups at a time
-        const uint32_t ngroups = args.counters[0];
+        const uint32_t ngroups = args.counters.at<NMAT == 1>(0);
         if (warp == 0) {
             uint32_t run = 0;
             for (uint32_t base = 0; base < ngroups; base += kWarp) {
-                uint32_t incl = base + lane < ngroups ? (args.groups[base + lane].pair_count + kTokens - 1) / kTokens : 0u;
+                uint32_t incl = base + lane < ngroups ? (args.groups.field<NMAT == 1>(base + lane, &tf_group::pair_count) + kTokens - 1) / kTokens : 0u;
 #pragma unroll
                 for (int o = 1; o < kWarp; o <<= 1) {
                     const uint32_t v = __shfl_up_sync(kFullMask, incl, o);
@@ -526,7 +530,7 @@ grouped_ksplit_kernel(const GroupedArgs args) {
         __syncthreads();
         total_chunks = chunk_first[ngroups];
     } else {
-        total_chunks = args.counters[1];
+        total_chunks = args.counters.at<NMAT == 1>(1);
     }
     const uint32_t total_items = total_chunks * tiles;
     // contiguous item range per CTA: consecutive items share the chunk, whose activations stay in registers
@@ -570,7 +574,7 @@ grouped_ksplit_kernel(const GroupedArgs args) {
         ItemCursor<NMAT> cur;
         cur.chunk = item_begin / tiles;
         cur.tile = item_begin % tiles;
-        cur.group = !DENSE && NT > 1 ? find_group(chunk_first, args.counters[0], cur.chunk) : 0u;
+        cur.group = !DENSE && NT > 1 ? find_group(chunk_first, args.counters.at<NMAT == 1>(0), cur.chunk) : 0u;
         resolve_chunk<NMAT, DENSE, NT>(args, cur, chunk_first);
         if (early) pdl_wait();           // the activations
 
@@ -598,7 +602,7 @@ grouped_ksplit_kernel(const GroupedArgs args) {
                 for (int i = 0; i < kGPW; ++i) {
                     uint32_t r[8];
                     if ((uint32_t)i < ngw && (uint32_t)(n * 8 + g) < cur.ntok) {
-                        const uint32_t rr = (DENSE || NMAT == 1) ? cur.row_base + n * 8 + g : args.sorted_pairs[cur.row_base + n * 8 + g].token;
+                        const uint32_t rr = (DENSE || NMAT == 1) ? cur.row_base + n * 8 + g : args.sorted_pairs.field<NMAT == 1>(cur.row_base + n * 8 + g, &tf_pair::token);
                         const uint4* p = reinterpret_cast<const uint4*>(args.x + (size_t)rr * args.x_stride + (g0 + i) * kGroup + t * 16);
                         const uint4 lo = __ldg(p), hi = __ldg(p + 1);
                         r[0] = lo.x; r[1] = lo.y; r[2] = lo.z; r[3] = lo.w;
@@ -808,7 +812,7 @@ grouped_ksplit_kernel(const GroupedArgs args) {
         ItemCursor<NMAT> iss;
         iss.chunk = item_begin / tiles;
         iss.tile = item_begin % tiles;
-        iss.group = !DENSE && NT > 1 ? find_group(chunk_first, args.counters[0], iss.chunk) : 0u;
+        iss.group = !DENSE && NT > 1 ? find_group(chunk_first, args.counters.at<NMAT == 1>(0), iss.chunk) : 0u;
         resolve_chunk<NMAT, DENSE, NT>(args, iss, chunk_first);
         const uint32_t plane_bytes = lay.sb_plane_bytes();
         const uint32_t rpc = lay.rows_per_copy();                    // 16: the rows of a tile land as one copy
@@ -853,7 +857,7 @@ grouped_ksplit_kernel(const GroupedArgs args) {
         ItemCursor<NMAT> cur;
         cur.chunk = item_begin / tiles;
         cur.tile = item_begin % tiles;
-        cur.group = !DENSE && NT > 1 ? find_group(chunk_first, args.counters[0], cur.chunk) : 0u;
+        cur.group = !DENSE && NT > 1 ? find_group(chunk_first, args.counters.at<NMAT == 1>(0), cur.chunk) : 0u;
         resolve_chunk<NMAT, DENSE, NT>(args, cur, chunk_first);
         if (q < n_items) advance_by(cur, q);
         uint32_t fail = 0;
@@ -871,8 +875,8 @@ grouped_ksplit_kernel(const GroupedArgs args) {
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
                             if (n * 8 + tok4 + j < cur.ntok) {
-                                const tf_pair pr = args.sorted_pairs[cur.row_base + n * 8 + tok4 + j];
-                                pair_base[n][j] = pr.token * args.top_k + pr.rank;
+                                const uint32_t at = cur.row_base + n * 8 + tok4 + j;
+                                pair_base[n][j] = args.sorted_pairs.field<NMAT == 1>(at, &tf_pair::token) * args.top_k + args.sorted_pairs.field<NMAT == 1>(at, &tf_pair::rank);
                             }
                         }
                     }
@@ -977,7 +981,7 @@ grouped_down_kernel(const GroupedArgs args) {
     const bool early = args.after_gate_up;      // as in grouped_ksplit_kernel: the ring fills as soon as a gate/up block has left the SM
     if (!early) pdl_wait();
     // contiguous ranges of whole stages (a chunk's tiles are a multiple of four)
-    const uint32_t total_chunks = args.counters[1];
+    const uint32_t total_chunks = args.counters.at<true>(1);
     const uint32_t total_stages = total_chunks * (tiles / kDownSub);
     const uint32_t stage_begin = (uint32_t)((uint64_t)total_stages * blockIdx.x / gridDim.x);
     const uint32_t n_stages = (uint32_t)((uint64_t)total_stages * (blockIdx.x + 1) / gridDim.x) - stage_begin;
@@ -988,10 +992,10 @@ grouped_down_kernel(const GroupedArgs args) {
     }
     ItemCursor<1> cur;
     uint32_t fail = 0;
-    auto place = [&](uint32_t item) {                         // the cursor's chunk and tile; resolves a new chunk
+    auto place = [&](uint32_t item, auto before_wait) {      // the cursor's chunk and tile; resolves a new chunk
         const uint32_t chunk = item / tiles;
         cur.tile = item - chunk * tiles;
-        if (chunk != cur.chunk) { cur.chunk = chunk; resolve_chunk<1, false, 1>(args, cur, nullptr); return true; }
+        if (chunk != cur.chunk) { cur.chunk = chunk; resolve_chunk<1, false, 1, before_wait.value>(args, cur, nullptr); return true; }
         return false;
     };
     cur.chunk = 0xFFFFFFFFu;
@@ -1005,7 +1009,7 @@ grouped_down_kernel(const GroupedArgs args) {
         uint32_t idx[2] = {0u, 0u}; // (token * top_k + rank) of tokens 2t and 2t + 1
         for (uint32_t li = warp; li < n_items; li += kDownWarps) {
             const uint32_t st = (li / kDownSub) % kDownStages, use = (li / kDownSub) / kDownStages, sub = li % kDownSub;
-            if (place(item_begin + li)) {
+            if (place(item_begin + li, std::false_type{})) {
 #pragma unroll
                 for (int i = 0; i < NG; ++i) {
                     uint32_t r[8];
@@ -1039,8 +1043,8 @@ grouped_down_kernel(const GroupedArgs args) {
 #pragma unroll
                 for (int c = 0; c < 2; ++c) {
                     if (2 * t + c < (int)cur.ntok) {
-                        const tf_pair pr = args.sorted_pairs[cur.row_base + 2 * t + c];
-                        idx[c] = pr.token * args.top_k + pr.rank;
+                        const uint32_t at = cur.row_base + 2 * t + c;
+                        idx[c] = args.sorted_pairs.field<false>(at, &tf_pair::token) * args.top_k + args.sorted_pairs.field<false>(at, &tf_pair::rank);
                     }
                 }
             }
@@ -1107,7 +1111,7 @@ grouped_down_kernel(const GroupedArgs args) {
         // loader: lane 0 moves a stage's codes, lane 1 its scales, lane 2 its biases
         uint32_t st = 0, use = 0, issued = 0;
         for (uint32_t si = 0; si < n_stages; ++si) {
-            place(item_begin + si * kDownSub);
+            place(item_begin + si * kDownSub, std::true_type{});
             if (use > 0 && !mbar_wait(bar_empty(st), (use - 1) & 1)) { fail = kErrTimeoutStageFree; break; }
             const uint32_t mbar = bar_full(st), stage = smem_base + st * kStageBytes;
             if (lane == 0) {
@@ -1385,8 +1389,8 @@ tf_status grouped_moe_batched(tf_context* ctx, void* stream, const void* hidden,
     a.expert_stride = expert_stride;
     a.w_off[0] = offsets->gate_w_off; a.s_off[0] = offsets->gate_s_off; a.b_off[0] = offsets->gate_b_off;
     a.w_off[1] = offsets->up_w_off;   a.s_off[1] = offsets->up_s_off;   a.b_off[1] = offsets->up_b_off;
-    a.sorted_pairs = routes->sorted_pairs; a.groups = routes->groups; a.chunk_group = routes->chunk_group;
-    a.chunk_start = routes->chunk_start; a.counters = routes->counters;
+    a.sorted_pairs = {routes->sorted_pairs}; a.groups = {routes->groups}; a.chunk_group = {routes->chunk_group};
+    a.chunk_start = {routes->chunk_start}; a.counters = {routes->counters};
     a.x = reinterpret_cast<const uint16_t*>(hp); a.x_stride = hidden_stride_elements;
     a.out = acts_scratch; a.out_stride = f; a.rows = f; a.k = d; a.top_k = top_k;
     tf_status s = tf::launch_grouped<2, false, tf::kOutActs, 2816>(ctx, stream, a, wide, "tf_grouped_moe_batched(gate/up)");
@@ -1395,8 +1399,8 @@ tf_status grouped_moe_batched(tf_context* ctx, void* stream, const void* hidden,
     tf::GroupedArgs b{};
     b.pool_base = a.pool_base; b.expert_stride = expert_stride;
     b.w_off[0] = offsets->down_w_off; b.s_off[0] = offsets->down_s_off; b.b_off[0] = offsets->down_b_off;
-    b.sorted_pairs = routes->sorted_pairs; b.groups = routes->groups; b.chunk_group = routes->chunk_group;
-    b.chunk_start = routes->chunk_start; b.counters = routes->counters;
+    b.sorted_pairs = {routes->sorted_pairs}; b.groups = {routes->groups}; b.chunk_group = {routes->chunk_group};
+    b.chunk_start = {routes->chunk_start}; b.counters = {routes->counters};
     b.x = static_cast<const uint16_t*>(acts_scratch); b.x_stride = f;
     b.out = route_partials; b.out_stride = d; b.rows = d; b.k = f; b.top_k = top_k;
     b.after_gate_up = 1;
@@ -1537,16 +1541,16 @@ tf_status tf_grouped_moe_streamed(tf_context* ctx, void* stream, const void* hid
     a.pool_base = lowest; a.expert_stride = 16;
     a.w_off[0] = offsets.gate_w_off; a.s_off[0] = offsets.gate_s_off; a.b_off[0] = offsets.gate_b_off;
     a.w_off[1] = offsets.up_w_off;   a.s_off[1] = offsets.up_s_off;   a.b_off[1] = offsets.up_b_off;
-    a.sorted_pairs = pairs; a.groups = scratch->groups; a.chunk_group = scratch->chunk_group;
-    a.chunk_start = scratch->chunk_start; a.counters = scratch->counters;
+    a.sorted_pairs = {pairs}; a.groups = {scratch->groups}; a.chunk_group = {scratch->chunk_group};
+    a.chunk_start = {scratch->chunk_start}; a.counters = {scratch->counters};
     a.x = reinterpret_cast<const uint16_t*>(hp); a.x_stride = params->hidden_stride_elements;
     a.out = acts; a.out_stride = f; a.rows = f; a.k = d; a.top_k = params->top_k;
     if (tf_status s = tf::launch_grouped<2, false, tf::kOutActs, 2816>(ctx, stream, a, false, "tf_grouped_moe_streamed(gate/up)")) return s;
     tf::GroupedArgs b{};
     b.pool_base = lowest; b.expert_stride = 16;
     b.w_off[0] = offsets.down_w_off; b.s_off[0] = offsets.down_s_off; b.b_off[0] = offsets.down_b_off;
-    b.sorted_pairs = pairs; b.groups = scratch->groups; b.chunk_group = scratch->chunk_group;
-    b.chunk_start = scratch->chunk_start; b.counters = scratch->counters;
+    b.sorted_pairs = {pairs}; b.groups = {scratch->groups}; b.chunk_group = {scratch->chunk_group};
+    b.chunk_start = {scratch->chunk_start}; b.counters = {scratch->counters};
     b.x = reinterpret_cast<const uint16_t*>(acts); b.x_stride = f;
     b.out = tf::byte_ptr(route_partials, route_partials_off); b.out_stride = d; b.rows = d; b.k = f; b.top_k = params->top_k;
     b.after_gate_up = 1;

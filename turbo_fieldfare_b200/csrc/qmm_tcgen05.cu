@@ -84,8 +84,8 @@ struct QmmArgs {
     uint64_t expert_stride;
     // groups of the launch, filled by qmm_prepare_kernel: {first token tile, first row, tokens, expert | tokens per tile << 16},
     // and {groups, token tiles, largest N}
-    uint4* groups;
-    uint32_t* totals;
+    EarlyTable<uint4> groups;
+    EarlyTable<uint32_t> totals;
     // their source; routed: what the grouping kernels left on the device; dense (NULL): one group
     const tf_group* route_groups;
     const uint32_t* route_counters;
@@ -430,12 +430,12 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map16, const __grid_con
         }
     }
     // The routed down launch takes its tables and weights while the last gate/up tiles are still being computed elsewhere; only the
-    // copies of its activations wait. The tables are complete: gate/up lets its dependent start after its own wait.
+    // copies of its activations wait. The tables are complete (see EarlyTable): gate/up lets its dependent start after its own wait.
     const bool early = NMAT == 1 && args.after_gate_up;
     if (!early) pdl_wait();                                             // routes and activations come from the kernels before this one
     if (kRoutedGateUp) pdl_launch_dependents();
-    const uint32_t ngroups = args.totals[0], total_tiles = args.totals[1] * wrow_tiles, n_top = args.totals[2];
-    if (threadIdx.x < ngroups) table[threadIdx.x] = args.groups[threadIdx.x];
+    const uint32_t ngroups = args.totals.at<NMAT == 1>(0), total_tiles = args.totals.at<NMAT == 1>(1) * wrow_tiles, n_top = args.totals.at<NMAT == 1>(2);
+    if (threadIdx.x < ngroups) table[threadIdx.x] = args.groups.at<NMAT == 1>(threadIdx.x);
     tc_fence_before();
     __syncthreads();
     if constexpr (PAIR) q_cluster_sync();                              // the other CTA's barriers are initialised, too
@@ -902,9 +902,11 @@ static QmmDense qmm_dense_tiles(uint32_t tokens, uint32_t rows, uint32_t mat_row
 constexpr int kQmmGateUpTable = 0, kQmmDownTable = 1, kQmmDenseTable = 2;
 static tf_status launch_qmm_prepare(tf_context* ctx, void* stream, QmmArgs& a, int table, const char* name) {
     TF_REQUIRE(ctx, ctx->qmm_groups != nullptr, TF_ERR_OUT_OF_MEMORY, "%s: context scratch missing", name);
-    a.groups = static_cast<uint4*>(ctx->qmm_groups) + table * (TF_MAX_ROUTER_EXPERTS + 1);
-    a.totals = reinterpret_cast<uint32_t*>(a.groups + TF_MAX_ROUTER_EXPERTS);
-    launch_pdl(qmm_prepare_kernel, dim3(1), dim3(TF_MAX_ROUTER_EXPERTS), 0, static_cast<cudaStream_t>(stream), a.groups, a.totals,
+    uint4* groups = static_cast<uint4*>(ctx->qmm_groups) + table * (TF_MAX_ROUTER_EXPERTS + 1);
+    uint32_t* totals = reinterpret_cast<uint32_t*>(groups + TF_MAX_ROUTER_EXPERTS);
+    a.groups = {groups};
+    a.totals = {totals};
+    launch_pdl(qmm_prepare_kernel, dim3(1), dim3(TF_MAX_ROUTER_EXPERTS), 0, static_cast<cudaStream_t>(stream), groups, totals,
                a.route_groups, a.route_counters, a.dense_tokens, a.dense_per_tile, a.ctas);
     return check_launch(ctx, "qmm_prepare");
 }

@@ -8,6 +8,7 @@
 
 #include <cstdarg>
 #include <cstdio>
+#include <cstring>
 #include <mutex>
 #include <string>
 
@@ -186,6 +187,47 @@ __device__ __forceinline__ float gelu_tanh(float x) {
 // a dependent start early. Without the launch attribute both instructions do nothing.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// A table that a gate/up launch reads after its pdl_wait and the down launch that follows it before its own. What holds for the latter:
+// the launches that wrote the table had completed, and their writes were visible, when gate/up returned from its wait, and
+// only after that did gate/up let the down launch start. Nothing is promised to a grid that has not waited itself about lines
+// that its SM's L1 may hold, so it reads with relaxed loads at GPU scope, which L2 serves, where the writes are. (Gate/up keeps
+// plain ones: every warp of the chip reads the same few lines there, and without L1 a one-token layer took 1 us longer.)
+template <typename T>
+struct EarlyTable {
+    const T* p;
+    template <bool BEFORE_WAIT>
+    __device__ __forceinline__ T at(size_t i) const {
+        if constexpr (!BEFORE_WAIT) {
+            return p[i];
+        } else if constexpr (alignof(T) == 16) {
+            static_assert(sizeof(T) == 16, "one vector load");
+            T v;
+            asm volatile("ld.relaxed.gpu.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p + i));
+            return v;
+        } else {
+            static_assert(sizeof(T) % 4 == 0 && alignof(T) == 4, "by 32-bit words: the pairs of a streamed call are aligned to four bytes");
+            uint32_t w[sizeof(T) / 4];
+#pragma unroll
+            for (size_t j = 0; j < sizeof(T) / 4; ++j) w[j] = word(reinterpret_cast<const uint32_t*>(p + i) + j);
+            T v;
+            memcpy(&v, w, sizeof(T));
+            return v;
+        }
+    }
+    template <bool BEFORE_WAIT, typename S>           // S is T, spelled so that a table of words compiles
+    __device__ __forceinline__ uint32_t field(size_t i, uint32_t S::*member) const {
+        if constexpr (!BEFORE_WAIT) return static_cast<const S*>(p)[i].*member;
+        else return word(&(static_cast<const S*>(p)[i].*member));
+    }
+
+private:
+    static __device__ __forceinline__ uint32_t word(const uint32_t* a) {
+        uint32_t v;
+        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a));
+        return v;
+    }
+};
 
 __device__ __forceinline__ uint4 ldg_nc_u4(const void* p) {
     uint4 v;
