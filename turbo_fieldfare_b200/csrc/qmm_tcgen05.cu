@@ -396,6 +396,7 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map16, const __grid_con
     auto bar_acc_empty = [&](uint32_t b) { return bars + (52 + b) * 8; };                    // 2 L: epilogue warps, of both CTAs
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(base_ptr + plan.off_bars + 54 * 8);   // TMEM base
     uint4* table = reinterpret_cast<uint4*>(base_ptr + plan.off_table);
+    uint32_t* totals = reinterpret_cast<uint32_t*>(base_ptr + plan.off_bars + 55 * 8);
 
     // The shuffle makes the warp index uniform for the compiler: the roles' branches and their operands then stay in uniform
     // registers, where the MMA and copy instructions want them (the MMA issuer's loop was 10 to 15 % slower without).
@@ -434,12 +435,14 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map16, const __grid_con
     const bool early = NMAT == 1 && args.after_gate_up;
     if (!early) pdl_wait();                                             // routes and activations come from the kernels before this one
     if (kRoutedGateUp) pdl_launch_dependents();
-    const uint32_t ngroups = args.totals.at<NMAT == 1>(0), total_tiles = args.totals.at<NMAT == 1>(1) * wrow_tiles, n_top = args.totals.at<NMAT == 1>(2);
-    if (threadIdx.x < ngroups) table[threadIdx.x] = args.groups.at<NMAT == 1>(threadIdx.x);
+    // The whole table and the totals in one round trip, a thread per entry (rows past the groups are copied and never used).
+    if (threadIdx.x < (args.route_groups ? (uint32_t)TF_MAX_ROUTER_EXPERTS : 1u)) table[threadIdx.x] = args.groups.at<NMAT == 1>(threadIdx.x);
+    else if (threadIdx.x - TF_MAX_ROUTER_EXPERTS < 3u) totals[threadIdx.x - TF_MAX_ROUTER_EXPERTS] = args.totals.at<NMAT == 1>(threadIdx.x - TF_MAX_ROUTER_EXPERTS);
     tc_fence_before();
     __syncthreads();
     if constexpr (PAIR) q_cluster_sync();                              // the other CTA's barriers are initialised, too
     tc_fence_after();
+    const uint32_t ngroups = totals[0], total_tiles = totals[1] * wrow_tiles, n_top = totals[2];
     const uint32_t tmem_base = *tmem_slot;
     // Activation ring: slots of a whole stage of the launch's largest tile, as many as fit. With two MMA issuers an even number,
     // as for the packed codes, so that a slot always belongs to the same one and a wait never sees the phase of another use.
