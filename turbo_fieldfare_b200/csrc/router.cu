@@ -79,6 +79,8 @@ router_split_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ 
     const uint16_t* hrow = hidden + (size_t)row * hidden_stride;
     const bool a16 = (reinterpret_cast<uintptr_t>(wsrc) & 15) == 0 && (d & 15) == 0;
     const bool x16 = (reinterpret_cast<uintptr_t>(hrow) & 15) == 0 && (reinterpret_cast<uintptr_t>(eff) & 15) == 0 && (d & 7) == 0;
+    const bool late = grp.sorted_pairs != nullptr;        // see below
+    if (!late) pdl_launch_dependents();
     if (a16 && x16 && ne * d <= kSplitThreads * 16 * 6 && d <= kSplitThreads * 8 * 3) {
         // latency path: every load of the block is issued before the first one is consumed
         uint4 wv[6], hv[3], ev[3];
@@ -164,11 +166,11 @@ router_split_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ 
     if (warp == 0)
         warp_select_topk(scores, num_experts, top_k, per_expert_scale, out_idx + (size_t)row * top_k,
                          out_w + (size_t)row * top_k, lane);
-    // Only now: the routed gate/up launch would otherwise sit on the SMs, waiting, from the first microsecond on, and keep both launches
-    // of the shared expert, which run beside this kernel, until it has ended. One token, 30 layers: released at the start 994
-    // us, after the logits 895 (863 with the faster selection), here 860; one block called eagerly 32.8, 28.6 and 26.9.
+    // With grouping (a block forward) the next launch is let in only now, while warp 0 selects: the routed gate/up launch would otherwise
+    // sit on the SMs, waiting, from the first microsecond on, and keep both launches of the shared expert, which run beside this
+    // kernel, until it has ended. One token, 30 layers: released at the start 994 us, after the logits 860.
+    if (!late) return;
     pdl_launch_dependents();
-    if (grp.sorted_pairs == nullptr) return;
     if (gridDim.x == 1) {
         // One token: a pair's place is the number of selected experts with a smaller id; every group holds one pair
         // and one chunk. That needs distinct experts: a row with fewer than top_k selectable logits (NaN, -inf)
@@ -238,7 +240,7 @@ router_split_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ 
 // (ticket) selects the top-k of its R rows, one warp per row; the block that completes the last row group builds the
 // grouping tables.
 constexpr int kRowsThreads = 256;
-constexpr uint32_t kRowsLateRelease = 52;
+constexpr uint32_t kRowsLateRows = 52;
 constexpr int kRowsExpertsPerBlock = kRowsThreads / kWarp;
 template <bool X_BF16, int R>
 __global__ void __launch_bounds__(kRowsThreads)
@@ -248,7 +250,7 @@ router_rows_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S
                    const float* __restrict__ logit_bias,
                    uint32_t* __restrict__ out_idx, uint16_t* __restrict__ out_w, float* __restrict__ out_logits,
                    float* scratch_logits, unsigned int* tickets, const RouterGroupOut grp,
-                   uint32_t rows, uint32_t num_experts, uint32_t d, uint32_t top_k) {
+                   uint32_t rows, uint32_t num_experts, uint32_t d, uint32_t top_k, bool resident) {
     extern __shared__ __align__(16) uint8_t smem[];
     const uint32_t groups = d / kGroup;
     float* xf = reinterpret_cast<float*>(smem);                                        // [R][d]
@@ -261,13 +263,16 @@ router_rows_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S
     const uint32_t row0 = blockIdx.x * R;
     const uint32_t e0 = blockIdx.y * kRowsExpertsPerBlock;
     const uint32_t ne = num_experts - e0 < (uint32_t)kRowsExpertsPerBlock ? num_experts - e0 : (uint32_t)kRowsExpertsPerBlock;
-    // As in router_split_kernel the routed launch is let in before the grouping, as long as all blocks of this one are resident (six
-    // per SM at the production width). 30 layers, us, released at the start, after the logits and there: 4 rows 1532, 1284 and
-    // 1222, 8 rows 1875, 1684 and 1575, 11 rows 1877, 1734 and 1686, 32 rows 3131, 2839 and 2784, 48 rows 3748, 3329 and 3317. With
-    // more rows the shared expert's gate/up blocks get in before the routed ones anyhow, and its down projection, 17 us by then,
-    // must not (64 rows: 3868 at the start; late 3836 or, when it got in, 3970).
-    const bool late = gridDim.x <= kRowsLateRelease;
-    if (!late) pdl_launch_dependents();
+    // As in router_split_kernel the routed launch is let in late, by the block that groups, before it does: released at the start, the
+    // routed blocks take every SM that a router block leaves and wait there, ahead of the shared expert. Blocks that are not
+    // all resident let it in late by themselves, when the last of them starts; what is left then are the microseconds of selection
+    // and grouping, and with many rows those let the shared expert's down projection in before the routed blocks, too, which
+    // must not be. us a layer, at the start and late. All resident: 128 experts of 2816, 40 rows 119.9 and 110.7; 16 experts of
+    // 2816, 64 rows 73.2 and 64.8; 64 experts of 1024, 64 rows 56.1 and 51.1. Not all: 256 experts of 2816, 32 rows 138.8 and 135.2, 52
+    // rows 176.3 and 174.1, 64 rows 189.7 and 190.5; 128 experts, 56 rows 123.8 and 125.4, 64 rows 129.3 and 132.2. A call without
+    // grouping has no such launch behind it.
+    const bool late = gridDim.x <= kRowsLateRows || resident;
+    if (!late || grp.sorted_pairs == nullptr) pdl_launch_dependents();
     // expert rows (contiguous in every plane; d is a multiple of 64 and the planes are 16-byte aligned by contract)
     {
         const uint8_t* wsrc = W + (size_t)e0 * d;
@@ -599,8 +604,12 @@ static tf_status launch_router(tf_context* ctx, void* stream, const uint8_t* W, 
         static DeviceSmemCache configured_rows[2];
         if (tf_status s2 = ensure_dynamic_smem(ctx, k, configured_rows[bf ? 1 : 0], smem_rows)) return s2;
         dim3 grid((rows + R - 1) / R, (num_experts + kRowsExpertsPerBlock - 1) / kRowsExpertsPerBlock);
+        // While all blocks are resident (five per SM at the production width: up to 46 rows of 128 experts), and up to kRowsLateRows rows in
+        // any case, the next launch is let in late, see the kernel.
+        static ResidentBlocksCache held[2];
+        const bool resident = grid.x * grid.y <= resident_blocks(ctx, k, held[bf ? 1 : 0], kRowsThreads, smem_rows);
         launch_pdl(k, grid, dim3(kRowsThreads), smem_rows, st, W, Sp, Bp, hp, stride, ep, pp, logit_bias, out_idx, wp, out_logits,
-                   ctx->router_logits, ctx->router_tickets, grp, rows, num_experts, d, top_k);
+                   ctx->router_logits, ctx->router_tickets, grp, rows, num_experts, d, top_k, resident);
         return check_launch(ctx, name);
     }
     if (rows <= (uint32_t)kRouterSplitRows) {

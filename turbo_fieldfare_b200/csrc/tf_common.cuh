@@ -143,6 +143,29 @@ inline tf_status ensure_dynamic_smem(tf_context* ctx, Kernel kernel, DeviceSmemC
     return TF_OK;
 }
 
+// Blocks of a kernel that ctx's device holds at once, at a block size and dynamic shared memory within the limit set before; 0 if the
+// query fails. The last few answers per device are kept.
+struct ResidentBlocksCache {
+    std::mutex mu;
+    struct Entry { uint32_t threads, smem, per_sm; } entry[kMaxDevices][4] = {};
+    uint8_t next[kMaxDevices] = {};
+};
+template <typename Kernel>
+inline uint32_t resident_blocks(tf_context* ctx, Kernel kernel, ResidentBlocksCache& cache, uint32_t threads, size_t smem) {
+    const int dev = ctx->device >= 0 && ctx->device < kMaxDevices ? ctx->device : -1;
+    std::lock_guard<std::mutex> lock(cache.mu);
+    if (dev >= 0)
+        for (const auto& e : cache.entry[dev])
+            if (e.threads == threads && e.smem == (uint32_t)smem) return e.per_sm * (uint32_t)ctx->sm_count;
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, (int)threads, smem) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    if (dev >= 0) cache.entry[dev][cache.next[dev]++ % 4] = {threads, (uint32_t)smem, (uint32_t)per_sm};
+    return (uint32_t)per_sm * (uint32_t)ctx->sm_count;
+}
+
 inline bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }
 inline const uint8_t* byte_ptr(const void* p, uint64_t off) { return static_cast<const uint8_t*>(p) + off; }
 inline uint8_t* byte_ptr(void* p, uint64_t off) { return static_cast<uint8_t*>(p) + off; }
