@@ -385,10 +385,15 @@ def test_decode_sized_stack_equals_the_chain_of_entry_points_bit_for_bit(tf_ctx,
         stack.close()
 
 
-# Blocks whose combine takes several tokens per thread block: one round and a part of the next, two and a part, an exact multiple.
-@pytest.mark.parametrize("T", [445, 889, 592])
-def test_stack_of_many_tokens_equals_the_chain_of_entry_points_bit_for_bit(tf_ctx, oracle, T):
-    test_decode_sized_stack_equals_the_chain_of_entry_points_bit_for_bit(tf_ctx, oracle, T, 256)
+# Blocks whose combine takes several tokens per thread block, in tokens per SM and beyond: one round and a part of the next, two and a
+# part, an exact multiple. Rows of one slice of the sum of squares, of two (the last warp partly idle), of three (production), the
+# widest of this form and one beyond it.
+@pytest.mark.parametrize("d", [256, 1088, 2816, 3072, 3136])
+@pytest.mark.parametrize("per_sm,more", [(3, 1), (6, 1), (4, 0), (12, 5)])
+def test_stack_of_many_tokens_equals_the_chain_of_entry_points_bit_for_bit(tf_ctx, oracle, d, per_sm, more):
+    import torch
+    T = per_sm * torch.cuda.get_device_properties(0).multi_processor_count + more
+    test_decode_sized_stack_equals_the_chain_of_entry_points_bit_for_bit(tf_ctx, oracle, T, d)
 
 
 @pytest.mark.parametrize("T", [1, 40])

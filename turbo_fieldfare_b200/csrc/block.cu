@@ -265,7 +265,7 @@ combine_residual_rmsnorm_kernel(uint16_t* __restrict__ h, const void* __restrict
 // combine_residual_rmsnorm_kernel<true> for blocks of many tokens, with its bits: a persistent block requests the rows of its next
 // token as soon as the current one's are summed, so that they travel while the sum of squares, the norm and the stores run. 4096
 // tokens x 8 rows of 2816, 277 MB: 71 to 74 us with a block per token, 49 to 51 here, 42 at the HBM rate.
-constexpr int kCrpThreads = 384;         // d <= 3072; two blocks per SM (wider rows keep the other form)
+constexpr int kCrpThreads = 384;         // d <= 3072; two blocks per SM and more (wider rows keep the other form)
 __global__ void __launch_bounds__(kCrpThreads, 2)
 combine_rows_pipelined_kernel(uint16_t* __restrict__ h, const uint16_t* __restrict__ rows, const uint16_t* __restrict__ route_weights,
                               const uint32_t* __restrict__ inverse_perm, const uint16_t* __restrict__ shared_y,
@@ -685,8 +685,14 @@ tf_status combine_rows_residual_rmsnorm(tf_context* ctx, void* stream, void* hid
     uint32_t threads = ((d / 8 + 31) / 32) * 32;
     if (threads < (uint32_t)kRrnThreads) threads = kRrnThreads;
     const PeerWait wait = peer_wait ? *peer_wait : PeerWait{nullptr, nullptr, nullptr, 0u};
-    if (threads <= (uint32_t)kCrpThreads && tokens > 3u * (uint32_t)ctx->sm_count) {       // up to there, three resident blocks per SM of the other form
-        launch_pdl(combine_rows_pipelined_kernel, dim3(2u * (uint32_t)ctx->sm_count), dim3(threads), 0, static_cast<cudaStream_t>(stream),
+    // As many blocks as the device holds: two per SM at 2816 columns, more for narrower rows, whose few threads would leave the SMs idle
+    // otherwise (a layer of 4000 tokens: 256 columns 105.5 us with two blocks per SM, 96.5 here, 99.0 in the other form; 1024 columns
+    // 171.5, 157.6, 162.8; 2816 columns 318, 318, 335). Up to three tokens per SM every block of the other form is resident.
+    static ResidentBlocksCache cache;
+    const uint32_t held = threads <= (uint32_t)kCrpThreads && tokens > 3u * (uint32_t)ctx->sm_count
+                              ? resident_blocks(ctx, combine_rows_pipelined_kernel, cache, threads, 0) : 0u;
+    if (held > 0) {
+        launch_pdl(combine_rows_pipelined_kernel, dim3(held < tokens ? held : tokens), dim3(threads), 0, static_cast<cudaStream_t>(stream),
                    static_cast<uint16_t*>(hidden), static_cast<const uint16_t*>(rows), static_cast<const uint16_t*>(route_weights), inverse_perm,
                    static_cast<const uint16_t*>(shared_y), static_cast<const uint16_t*>(norm_weight_bf16), static_cast<uint16_t*>(x), d, top_k, eps,
                    tokens, wait);
