@@ -213,19 +213,22 @@ def test_tile_gemv(tf_ctx, oracle, m, n, scale):
     assert np.all(np.abs(o.f16_to_f32(out[:m]) - ref) <= bound)
 
 
-# The streaming product: remainders of the 16-row tile (the last tile repeats rows), fewer tiles than blocks and than slots, rows of 1024
-# columns up to those that leave two teams, and what stays with the other kernels (1023 columns' side of the line, odd planes).
-@pytest.mark.parametrize("m,n", [(4096, 1024), (4104, 1280), (4100, 2816), (5002, 2816), (4112, 4096), (40008, 1024), (4096, 5632), (4096, 6144),
-                                 (4099, 1280), (4098, 768)])
+# The streaming product: remainders of the 16-row tile (the last tile repeats rows), fewer tiles than teams and than slots, rows of 1024
+# columns up to the widest that leave two teams (5888), and what stays with the other kernels (fewer or more columns, planes of
+# the last tile off the 16-byte grid).
+@pytest.mark.parametrize("m,n", [(4096, 1024), (4104, 1280), (4100, 2816), (5002, 2816), (4112, 4096), (40008, 1024), (4096, 5632), (4104, 5888),
+                                 (4096, 6144), (4099, 1280), (4098, 768)])
 def test_streaming_gemv(tf_ctx, oracle, m, n):
     test_tile_gemv(tf_ctx, oracle, m, n, 1.0)
 
 
-# The greedy head on both sides of the streaming form's line (2^27 weights), ragged vocabularies.
-@pytest.mark.parametrize("v", [47660, 47664, 47666, 50008])
-def test_lm_head_rows_around_the_streaming_line(tf_ctx, oracle, v):
+# The greedy head on both sides of the streaming form's lines (2^27 weights; fewer than 1536 columns; 2^28 weights of more than 4096
+# columns), ragged vocabularies.
+@pytest.mark.parametrize("d,v", [(2816, 47660), (2816, 47664), (2816, 47666), (2816, 50008), (1280, 104872), (1536, 87376), (1536, 87390),
+                                 (4096, 32776), (5120, 52424), (5120, 52434)])
+def test_lm_head_rows_around_the_streaming_line(tf_ctx, oracle, d, v):
     from tests.test_gpu_decode import _lm_head_gpu
-    o, d = oracle, 2816
+    o = oracle
     rng = np.random.default_rng(v)
     mat = config0_matrix(o, v, d, rng)
     norm = o.f32_to_bf16((1.0 + 0.02 * rng.standard_normal(d)).astype(np.float32))

@@ -37,8 +37,8 @@ __device__ __forceinline__ unsigned long long argmax_key(float z, uint32_t row) 
 // x in MMA operand order and its group sums, by the whole block: the 16 values x0..x15 at columns 64 G + 16 t feed four MMAs,
 //   j = 0: (x0,x4),(x2,x6)   j = 1: (x1,x5)/16,(x3,x7)/16   j = 2, 3: the same for x8..x15
 // (odd columns are pre-scaled by 1/16 because their codes sit four mantissa bits higher)
-__device__ __forceinline__ void gm_stage_x(const uint16_t* __restrict__ x, uint32_t ng, uint32_t* xfrag, float* xsum) {
-    for (uint32_t idx = threadIdx.x; idx < ((ng * 4 + 31u) & ~31u); idx += blockDim.x) {   // whole warps: the sums use shuffles
+__device__ __forceinline__ void gm_stage_x(const uint16_t* __restrict__ x, uint32_t ng, uint32_t* xfrag, float* xsum, uint32_t threads) {
+    for (uint32_t idx = threadIdx.x; idx < ((ng * 4 + 31u) & ~31u); idx += threads) {   // whole warps: the sums use shuffles
         const bool ok = idx < ng * 4;
         const uint32_t G = idx >> 2, tt = idx & 3;
         const uint4* p = reinterpret_cast<const uint4*>(x + G * kGroup + tt * 16);
@@ -166,7 +166,7 @@ gemv_mma_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S, c
         for (uint32_t i = threadIdx.x; i < words; i += kGmThreads) { ds[i] = __ldg(gs + i); db[i] = __ldg(gb + i); }
     }
     if constexpr (ARGMAX) pdl_wait();
-    gm_stage_x(x, ng, xfrag, xsum);
+    gm_stage_x(x, ng, xfrag, xsum, kGmThreads);
     __syncthreads();
 
     const uint16_t* s0p = sS + (size_t)(warp * 16 + g) * ng;
@@ -263,7 +263,7 @@ gemv_stream_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S
         if (tile + step < tiles) request(tile + step, 1);
     }
     if constexpr (ARGMAX) pdl_wait();
-    gm_stage_x(x, ng, xfrag, xsum);
+    gm_stage_x(x, ng, xfrag, xsum, blockDim.x);
     __syncthreads();
     float zc[4];
 #pragma unroll
@@ -320,14 +320,18 @@ gemv_stream_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S
     if constexpr (ARGMAX) gm_fold_argmax(best, per_warp, argmax);
 }
 // Teams of a block, 0 where the kernel does not apply: two slots of whole rows for at least two teams, planes of the last tile (which
-// may repeat rows) on a 16-byte boundary, rows of 1024 columns and more (a team's slots hold too little otherwise; us, with
-// gemv_mma_kernel and here: 65536 x 512 7.1 and 8.3, 65536 x 1024 12.1 and 11.7, 32768 x 1024 8.2 and 6.8, 8192 x 2816 9.8 and
-// 5.9). The greedy LM head waits for its norm at the start, which a block of many small tiles hides better: from 2^27 weights
-// on (2816 columns, 32000 rows 18.2 and 20.6, 65536 rows 31.9 and 28.5, 131072 rows 49.9 and 43.1).
-constexpr uint32_t kGsMinColumns = 1024;
-constexpr uint64_t kGsMinArgmaxWeights = 1ull << 27;
+// may repeat rows; callers have 4096 and more) on a 16-byte boundary, rows of 1024 columns and more (a team's slots hold too
+// little otherwise; us, with gemv_mma_kernel and here: 65536 x 512 7.1 and 8.3, 65536 x 1024 12.2 and 11.3, 32768 x 1024 8.5 and 7.0,
+// 8192 x 2816 11.8 and 5.7). The greedy LM head waits for its norm at the start, which a block of many small tiles hides
+// better: from 1536 columns and 2^27 weights on (262144 rows of 1024 columns 38.2 and 41.6, of 1280 45.8 and 46.7, of 1536 52.0
+// and 47.4; 2816 columns, 32000 rows out of L2 18.2 and 20.6, 65536 rows 30.5 and 26.8, 131072 rows 48.4 and 41.3), for rows of more
+// than 4096 columns, whose few large slots start and end slowly, from 2^28 (5120 columns, 32000 rows 34.6 and 37.4, 48000 rows
+// 45.6 and 51.6, 65536 rows 59.5 and 58.9, 262144 rows 178.7 and 158.9).
+constexpr uint32_t kGsMinColumns = 1024, kGsMinArgmaxColumns = 1536, kGsLongColumns = 4096;
+constexpr uint64_t kGsMinArgmaxWeights = 1ull << 27, kGsMinArgmaxWeightsLong = 1ull << 28;
 static uint32_t gs_teams(uint32_t m, uint32_t n, bool greedy) {
-    if (m < 16 || n < kGsMinColumns || (greedy && (uint64_t)m * n < kGsMinArgmaxWeights)) return 0;
+    if (n < (greedy ? kGsMinArgmaxColumns : kGsMinColumns)) return 0;
+    if (greedy && (uint64_t)m * n < (n > kGsLongColumns ? kGsMinArgmaxWeightsLong : kGsMinArgmaxWeights)) return 0;
     if (m % 16 != 0 && ((uint64_t)m * (n / kGroup)) % 8 != 0) return 0;
     const uint32_t x_bytes = gs_x_bytes(n), two = 2 * gs_stage_bytes(n), budget = 220u * 1024u;
     const uint32_t fit = x_bytes < budget ? (budget - x_bytes) / two : 0u, teams = fit < (uint32_t)kGsTeams ? fit : (uint32_t)kGsTeams;
@@ -373,7 +377,7 @@ tf_status launch_gemv_mma(tf_context* ctx, void* stream, const uint8_t* W, const
 
 // The greedy LM head's product: *argmax is zero before. Must follow, on the stream, the
 // launch that writes x, and that launch must start after everything before it (no programmatic launch of its own).
-// Blocks of 128 rows, as for the stored form (64 rows took as long when both were measured, 103 us for 262144 rows).
+// Short of gs_teams' line blocks of 128 rows, as for the stored form (64 rows took as long when both were measured).
 tf_status launch_gemv_mma_argmax(tf_context* ctx, void* stream, const uint8_t* W, const uint16_t* S, const uint16_t* B,
                                  const uint16_t* x, uint32_t m, uint32_t n, unsigned long long* argmax, const char* name) {
     if (const uint32_t teams = gs_teams(m, n, true))
