@@ -266,3 +266,21 @@ def test_int4_qmm_edges_of_both_forms(tf_ctx, oracle, M, N, K):
 @pytest.mark.parametrize("T,D,F,E,K,zipf", [(70, 256, 192, 16, 8, True), (2, 64, 64, 256, 8, False), (400, 192, 320, 8, 4, True)])
 def test_grouped_tensorcore_edges_of_both_forms(tf_ctx, oracle, T, D, F, E, K, zipf):
     test_grouped_tensorcore_vs_oracle_and_cuda_cores(tf_ctx, oracle, T, D, F, E, K, zipf)
+
+
+# The form with one issuer and up to 128 tokens per tile. A last stage of one group and rows beyond the last whole tile, with a last token tile
+# of its own box and one of the full tile's; fewer tokens than a tile; one stage; a last stage of three groups.
+@pytest.mark.parametrize("M,N,K", [(1000, 4104, 320), (1016, 4104, 320), (90, 18000, 256), (2049, 1040, 64), (513, 5000, 1088), (700, 2816, 704)])
+def test_int4_qmm_edges_of_wide_tiles(tf_ctx, oracle, M, N, K):
+    test_int4_qmm_vs_oracle(tf_ctx, oracle, M, N, K)
+
+
+# The same for a shared expert's gate/up, and pairs with an odd number of weight-row tiles for plain rows.
+@pytest.mark.parametrize("T,D,Fs", [(700, 512, 1024), (333, 576, 4096)])
+def test_shared_expert_tensorcore_wide_tiles(tf_ctx, oracle, T, D, Fs):
+    test_shared_expert_tensorcore_vs_oracle(tf_ctx, oracle, T, D, Fs)
+
+
+@pytest.mark.parametrize("M,N,K", [(600, 2824, 2112), (1000, 2112, 2816)])
+def test_int4_qmm_pairs_past_the_matrix(tf_ctx, oracle, M, N, K):
+    test_int4_qmm_vs_oracle(tf_ctx, oracle, M, N, K)

@@ -17,7 +17,7 @@ def _waits_only_with_a_stage():
     """Whether the source's issuers skip the wait for the accumulator of a tile that they have no stage of."""
     text = SOURCE.read_text()
     issuers = text[text.index("// ===================== MMA issuers"):text.index("// ===================== dequantisers")]
-    return ("const bool takes_part = PAIR || ksteps > 1 || (count & 1) == who;" in issuers and
+    return ("const bool takes_part = !kTwoIssuers || ksteps > 1 || (count & 1) == who;" in issuers and
             "if (takes_part && uacc > 0 && !q_mbar_wait(bar_acc_empty(buf)" in issuers)
 
 

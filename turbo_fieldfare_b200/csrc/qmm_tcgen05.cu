@@ -18,25 +18,29 @@
 // bytes, and writing it to shared memory and reading it back for the MMA would cost more shared-memory
 // bandwidth than the whole HBM stream.
 // A gate/up tile holds 64 gate rows over 64 up rows, so that one accumulator of 128 lanes carries both, 704 rows are eleven
-// whole tiles, and both forms of the kernel have one layout; the epilogue warps of the two halves exchange values.
-// Roles of the 24 warps: warp 0 issues the copies of a tile's scale and bias planes (1-D bulk copies) and of packed codes,
-// warp 2 those of activations (one 3-D box of 16 to 64 rows x 256 columns per stage), warps 1 and 3 the MMAs, and commit stages
-// back through mbarriers; warps 4-19 dequantise in two teams that take turns (a thread takes two groups of one row per stage);
+// whole tiles, and all forms of the kernel have one layout; the epilogue warps of the two halves exchange values.
+// Roles of the 24 warps: warp 0 issues the copies of packed codes and of a tile's scale and bias planes (1-D bulk copies; kQmmWide:
+// warp 3), warp 2 those of activations (one 3-D box of 16 to 128 rows x 256 columns per stage), warp 1 the MMAs (kQmmFew: in turn
+// with warp 3), and commits stages back through mbarriers; warps 4-19 dequantise in two teams that take turns, a thread two
+// groups of one row per stage (kQmmWide: in one, a thread one group);
 // warps 20-23 read the accumulators with tcgen05.ld, apply GeGLU or nothing, and store through a staging tile as 16-byte words,
 // masked to the group's real tokens. Accumulators are double-buffered, so that the epilogue overlaps the next tile's MMAs.
 // A persistent grid walks (group, token tile, weight-row tile) work items derived on the device from the
 // routing metadata. Every mbarrier wait is bounded; on expiry the kernel records a code, waits for its copies and leaves.
 //
-// Two forms (clock counters around the waits of each role; 128 experts of 704 x 2816, uniform routing):
-// PAIR, many tokens: with one CTA per tile of 128 rows x 128 tokens a stage took 1700 clocks, 640 of them waits for activations
+// Three forms (clock counters around the waits of each role; 128 experts of 704 x 2816, uniform routing):
+// kQmmPair, many tokens: with one CTA per tile of 128 rows x 128 tokens a stage took 1700 clocks, 640 of them waits for activations
 // (64 KB per stage and SM out of L2). A pair of CTAs (cta_group::2) shares them: each holds those of half the tokens. 1240 clocks
 // at 104 tokens per tile (MMAs 830), most of the rest the instructions of the one warp that issues them. 4096 tokens: gate/up 281
 // -> 240 us, down 161 -> 141; dense 4096 x 2112 x 2816: 44 us = 1.11 PFLOP/s. (Arrivals on the other CTA's barriers must not
 // be releases at cluster scope: with those a stage took 2150 clocks.)
-// Otherwise, few tokens: the one warp that issued the MMAs bounded the kernel (waits, 16 MMAs and commits: 1250 of 1250 clocks
+// kQmmFew: the one warp that issued the MMAs bounded the kernel (waits, 16 MMAs and commits: 1250 of 1250 clocks
 // without any copy outstanding at 1170), so two warps take turns, each with an accumulator, and activations come by one copy per
 // stage instead of four. 333 tokens, 21 per expert: 1010 clocks a stage, of which an SM's share of the HBM rate is 790 and the
 // dequantisers' instructions about 550; gate/up 109 -> 74 us, down 70 -> 46.
+// kQmmWide, dense launches of more than 64 tokens per tile whose tiles have few stages: there start and end count, which take a pair
+// about 1 us longer, and tiles of 64 tokens would be twice as many. 2000 x 1024 x 512: 8.5 us in the better of the other two, 7.5
+// here; 500 x 4096 x 512 8.5 and 7.7; 500 x 8192 x 256 9.1 and 8.2. (Activations by half stages: up to 7 % slower.)
 //
 // Column order. The cheapest nibble extraction yields the eight codes of a 32-bit word in the order
 // (0,4,1,5,2,6,3,7). A dot product does not care about the order as long as both operands agree, so the
@@ -50,13 +54,13 @@
 namespace tf {
 
 constexpr int kQmmRows = 128;          // M of a CTA's MMA: weight rows per tile (gate/up: 64 gate rows over 64 up rows)
-constexpr int kQmmBoxMax = 64;         // activation rows that a CTA holds per tile: tokens of a tile, or half of them (PAIR)
+constexpr int kQmmBoxMax = 64;         // activation rows that a CTA holds per tile: tokens of a tile (kQmmPair: half of them; kQmmWide: up to 128)
 constexpr int kQmmStageK = 256;        // columns per stage: four quantisation groups
 constexpr uint32_t kQmmRawBytes = kQmmRows * (kQmmStageK / 2);      // 16 KB of packed codes
 constexpr uint32_t kQmmRowBytes = kQmmStageK * 2;                   // one activation row of a stage
 constexpr int kQmmRawMax = 4, kQmmBMax = 12, kQmmScMax = 4;         // ring depths (the launch picks them to fit, see QmmPlan)
-constexpr int kQmmTeams = 2;           // teams of dequantisers, each with its slot of a dequantised stage (128 TMEM columns)
-constexpr int kQmmFirstDequantWarp = 4, kQmmDequantWarps = 16, kQmmTeamWarps = kQmmDequantWarps / kQmmTeams;
+constexpr int kQmmASlots = 2;          // slots of a dequantised stage (128 TMEM columns), used in turn
+constexpr int kQmmFirstDequantWarp = 4, kQmmDequantWarps = 16;
 constexpr int kQmmFirstEpilogueWarp = 20, kQmmEpilogueWarps = 4;
 constexpr int kQmmThreads = (kQmmFirstEpilogueWarp + kQmmEpilogueWarps) * 32;
 constexpr int kQmmTmemCols = 512;      // columns 0..255: accumulators; 256..511: the teams' slots of dequantised weights
@@ -91,6 +95,7 @@ struct QmmArgs {
     const uint32_t* route_counters;
     uint32_t dense_tokens, dense_per_tile;
     uint32_t ctas;          // CTAs of a tile: 2 for pairs
+    uint32_t step_tok, step_row;      // what the grid's number of tiles is in whole token tiles and weight-row tiles
     uint32_t after_gate_up; // down launch whose predecessor on the stream is the gate/up launch of the same call
     // problem
     uint32_t rows;          // weight rows (output features)
@@ -345,10 +350,10 @@ struct QmmTile {
     uint32_t row0 = 0;          // first activation / output row
     uint32_t ntok = 0;          // real tokens
     uint32_t expert = 0;
-    __device__ __forceinline__ QmmTile(uint32_t first, uint32_t step, uint32_t tiles)
-        : tglob(first / tiles), wt(first % tiles), dt(step / tiles), dw(step % tiles), wrow_tiles(tiles) {}
+    __device__ __forceinline__ QmmTile(uint32_t first, uint32_t step_tok, uint32_t step_row, uint32_t tiles)
+        : tglob(first / tiles), wt(first - tglob * tiles), dt(step_tok), dw(step_row), wrow_tiles(tiles) {}
     __device__ __forceinline__ void locate(const uint4* table, uint32_t ngroups, uint32_t lane) {
-        for (uint32_t ahead = kWarp; ahead == kWarp;) {              // group starts grow: the votes are a prefix of the lanes
+        for (uint32_t ahead = ngroups > 1 ? kWarp : 0; ahead == kWarp;) {      // group starts grow: the votes are a prefix of the lanes
             const uint32_t g = gi + 1 + lane;
             ahead = __popc(__ballot_sync(kFullMask, g < ngroups && table[g].x <= tglob));
             gi += ahead;
@@ -365,19 +370,26 @@ struct QmmTile {
     }
 };
 
-// PAIR: two CTAs of a cluster (two SMs that share their tensor cores' operands, cta_group::2) take one tile of 2 x 128 weight
+// kQmmPair: two CTAs of a cluster (two SMs that share their tensor cores' operands, cta_group::2) take one tile of 2 x 128 weight
 // rows x up to 128 tokens. Each dequantises its own 128 rows and holds half of the tokens' activations, the first one issues the
-// MMAs. Otherwise a CTA takes 128 rows x up to 64 tokens, and two warps issue MMAs, one for each team of dequantisers.
-template <int NMAT, bool NATURAL_K, bool PAIR>
+// MMAs. kQmmFew: a CTA takes 128 rows x up to 64 tokens, and two warps issue MMAs, one for each team of dequantisers. kQmmWide:
+// a CTA takes 128 rows x up to 128 tokens, one warp issues.
+// x_map0 ... x_map3: boxes of 16, 32, 48 and 64 activation rows; kQmmWide: of a full tile's and of the last tile's rows.
+enum QmmForm { kQmmFew, kQmmWide, kQmmPair };
+template <int NMAT, bool NATURAL_K, QmmForm FORM>
 __global__ void __launch_bounds__(kQmmThreads, 1)
-qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map16, const __grid_constant__ CUtensorMap x_map32,
-                   const __grid_constant__ CUtensorMap x_map48, const __grid_constant__ CUtensorMap x_map64,
+qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map0, const __grid_constant__ CUtensorMap x_map1,
+                   const __grid_constant__ CUtensorMap x_map2, const __grid_constant__ CUtensorMap x_map3,
                    const __grid_constant__ CUtensorMap w_map0, const __grid_constant__ CUtensorMap w_map1, const QmmArgs args) {
     extern __shared__ uint8_t smem_raw[];
+    constexpr bool PAIR = FORM == kQmmPair, kTwoIssuers = FORM == kQmmFew;
     constexpr uint32_t kMatRows = kQmmRows / NMAT;                     // rows of one matrix in a tile
     constexpr uint32_t kCtas = PAIR ? 2 : 1;                           // CTAs of a tile
+    // One team of dequantisers, a group of a row per thread and stage, or two that take turns, two groups per thread: the latter
+    // hide one another's waits, the former has a tile's first stage ready sooner, which is what counts for tiles of few stages.
+    constexpr uint32_t kTeams = FORM == kQmmWide ? 1 : 2, kTeamWarps = kQmmDequantWarps / kTeams;
     constexpr uint32_t kStep = 16 * kCtas;                             // N of an MMA is a multiple of it
-    constexpr uint32_t kAccTok = PAIR ? 128 : 64;                      // columns of an accumulator
+    constexpr uint32_t kAccTok = kTwoIssuers ? 64 : 128;               // columns of an accumulator
     const QmmPlan& plan = args.plan;
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;                      // swizzle atoms need 1024-byte alignment
@@ -409,9 +421,9 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map16, const __grid_con
     constexpr bool kRoutedGateUp = NMAT == 2 && !NATURAL_K;
     if (!kRoutedGateUp) pdl_launch_dependents();
     if (threadIdx.x == 0) {
-        for (uint32_t s = 0; s < (uint32_t)kQmmRawMax; ++s) { q_mbar_init(bar_full_raw(s), 1); q_mbar_init(bar_empty_raw(s), kQmmTeamWarps); }
+        for (uint32_t s = 0; s < (uint32_t)kQmmRawMax; ++s) { q_mbar_init(bar_full_raw(s), 1); q_mbar_init(bar_empty_raw(s), kTeamWarps); }
         for (uint32_t s = 0; s < (uint32_t)kQmmBMax; ++s) { q_mbar_init(bar_full_b(s), 1); q_mbar_init(bar_empty_b(s), 1); }
-        for (uint32_t t = 0; t < (uint32_t)kQmmTeams; ++t) { q_mbar_init(bar_full_a(t), kCtas * kQmmTeamWarps); q_mbar_init(bar_empty_a(t), 1); }
+        for (uint32_t t = 0; t < (uint32_t)kQmmASlots; ++t) { q_mbar_init(bar_full_a(t), kCtas * kTeamWarps); q_mbar_init(bar_empty_a(t), 1); }
         for (uint32_t b = 0; b < (uint32_t)kQmmScMax; ++b) { q_mbar_init(bar_full_sc(b), 1); q_mbar_init(bar_empty_sc(b), kQmmDequantWarps); }
         for (uint32_t b = 0; b < 2; ++b) {
             for (uint32_t i = 0; i < 2; ++i) q_mbar_init(bar_acc_full(i, b), 1);
@@ -446,43 +458,53 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map16, const __grid_con
     const uint32_t tmem_base = *tmem_slot;
     // Activation ring: slots of a whole stage of the launch's largest tile, as many as fit. With two MMA issuers an even number,
     // as for the packed codes, so that a slot always belongs to the same one and a wait never sees the phase of another use.
-    // Where only two slots of 64 tokens would fit beside four stages of packed codes, those make do with two.
+    // Where too few slots would fit beside four stages of packed codes, those make do with two.
     const uint32_t b_slot = n_top / kCtas * kQmmRowBytes;
-    const uint32_t raw_stages = !PAIR && plan.b_bytes < 4 * b_slot ? 2u : plan.raw_stages;
+    const uint32_t raw_stages = !PAIR && plan.b_bytes < (kTwoIssuers ? 4 : 3) * b_slot ? 2u : plan.raw_stages;
     const uint32_t off_b = raw_stages * kQmmRawBytes, b_bytes = plan.off_b + plan.b_bytes - off_b;
-    const uint32_t b_fit = PAIR ? b_bytes / b_slot : b_bytes / b_slot & ~1u;
+    const uint32_t b_fit = kTwoIssuers ? b_bytes / b_slot & ~1u : b_bytes / b_slot;
     const uint32_t b_stages = b_fit < (uint32_t)kQmmBMax ? b_fit : (uint32_t)kQmmBMax;
     const uint32_t a_ring = tmem_base + kQmmAccCols;
     const uint32_t first_tile = blockIdx.x / kCtas, tile_step = gridDim.x / kCtas;
 
     uint32_t fail = 0;
-    QmmTile tl(first_tile, tile_step, wrow_tiles);
+    QmmTile tl(first_tile, args.step_tok, args.step_row, wrow_tiles);
 
+    // Scale and bias planes of tile tl; false when the wait for the buffer ran out.
+    uint32_t pl_buf = 0, pl_use = 0;
+    auto copy_planes = [&]() {
+        const uint32_t first = (tl.wt * kCtas + rank) * kMatRows;
+        if (pl_use > 0 && !q_mbar_wait(bar_empty_sc(pl_buf), (pl_use - 1) & 1)) return false;
+        if (elect_one()) {
+            const uint32_t left = first < args.rows ? args.rows - first : 0;      // a pair's second tile may be past the matrix
+            const uint32_t bytes = (left < kMatRows ? left : kMatRows) * ng * 2;  // a multiple of 16: rows are a multiple of 8
+            const size_t off = (size_t)tl.expert * args.expert_stride + (size_t)first * ng * 2;
+            q_mbar_expect_tx(bar_full_sc(pl_buf), NMAT * 2 * bytes);
+            if (bytes > 0) {
+#pragma unroll
+                for (int m = 0; m < NMAT; ++m) {
+                    const uint32_t dst = base + plan.off_sc + pl_buf * plan.sc_bytes + m * 2 * plan.plane_bytes;
+                    q_bulk_g2s(dst, reinterpret_cast<const uint8_t*>(args.S[m]) + off, bytes, bar_full_sc(pl_buf));
+                    q_bulk_g2s(dst + plan.plane_bytes, reinterpret_cast<const uint8_t*>(args.B[m]) + off, bytes, bar_full_sc(pl_buf));
+                }
+            }
+        }
+        __syncwarp();
+        if (++pl_buf == plan.sc_bufs) { pl_buf = 0; ++pl_use; }
+        return true;
+    };
+    auto drain_planes = [&]() {
+        for (uint32_t s = 0; s < plan.sc_bufs; ++s) q_mbar_wait(bar_full_sc(s), (s < pl_buf ? pl_use : pl_use + 1) & 1);
+    };
     if (warp == 0) {
         // ===================== copy issuer: scale and bias planes of a tile, packed codes =====================
-        uint32_t sr = 0, ur = 0, sc = 0, uc = 0;
+        uint32_t sr = 0, ur = 0;
         for (uint32_t tile = first_tile; tile < total_tiles && !fail; tile += tile_step, tl.next()) {
             tl.locate(table, ngroups, lane);
             const uint32_t first = (tl.wt * kCtas + rank) * kMatRows;
             // (the dequantisers of the tile that used this buffer last are as far as the ring of codes asks for below, or one tile
             // ahead of it where the planes have one buffer)
-            if (uc > 0 && !q_mbar_wait(bar_empty_sc(sc), (uc - 1) & 1)) { fail = kErrQmmTimeout | 6; break; }
-            if (elect_one()) {
-                const uint32_t left = first < args.rows ? args.rows - first : 0;      // a pair's second tile may be past the matrix
-                const uint32_t bytes = (left < kMatRows ? left : kMatRows) * ng * 2;  // a multiple of 16: rows are a multiple of 8
-                const size_t off = (size_t)tl.expert * args.expert_stride + (size_t)first * ng * 2;
-                q_mbar_expect_tx(bar_full_sc(sc), NMAT * 2 * bytes);
-                if (bytes > 0) {
-#pragma unroll
-                    for (int m = 0; m < NMAT; ++m) {
-                        const uint32_t dst = base + plan.off_sc + sc * plan.sc_bytes + m * 2 * plan.plane_bytes;
-                        q_bulk_g2s(dst, reinterpret_cast<const uint8_t*>(args.S[m]) + off, bytes, bar_full_sc(sc));
-                        q_bulk_g2s(dst + plan.plane_bytes, reinterpret_cast<const uint8_t*>(args.B[m]) + off, bytes, bar_full_sc(sc));
-                    }
-                }
-            }
-            __syncwarp();
-            if (++sc == plan.sc_bufs) { sc = 0; ++uc; }
+            if (FORM != kQmmWide && !copy_planes()) { fail = kErrQmmTimeout | 6; break; }
             for (uint32_t ks = 0; ks < ksteps; ++ks) {
                 if (ur > 0 && !q_mbar_wait(bar_empty_raw(sr), (ur - 1) & 1)) { fail = kErrQmmTimeout | 1; break; }
                 if (elect_one()) {
@@ -498,8 +520,15 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map16, const __grid_con
         }
         if (fail) {          // the copies already issued land before the CTA's shared memory goes away (bounded)
             for (uint32_t s = 0; s < raw_stages; ++s) q_mbar_wait(bar_full_raw(s), (s < sr ? ur : ur + 1) & 1);
-            for (uint32_t s = 0; s < plan.sc_bufs; ++s) q_mbar_wait(bar_full_sc(s), (s < sc ? uc : uc + 1) & 1);
+            if (FORM != kQmmWide) drain_planes();
         }
+    } else if (FORM == kQmmWide && warp == 3) {
+        // ===================== copy issuer: scale and bias planes, beside the codes =====================
+        for (uint32_t tile = first_tile; tile < total_tiles && !fail; tile += tile_step, tl.next()) {
+            tl.locate(table, ngroups, lane);
+            if (!copy_planes()) fail = kErrQmmTimeout | 6;
+        }
+        if (fail) drain_planes();
     } else if (warp == 2) {
         // ===================== copy issuer: activations, one copy per stage =====================
         uint32_t sb = 0, ub = 0;
@@ -507,7 +536,8 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map16, const __grid_con
         for (uint32_t tile = first_tile; tile < total_tiles && !fail; tile += tile_step, tl.next()) {
             tl.locate(table, ngroups, lane);
             const uint32_t box = (tl.ntok + kStep - 1) / kStep * 16;  // rows per CTA
-            const CUtensorMap* map = box == 64 ? &x_map64 : box == 48 ? &x_map48 : box == 32 ? &x_map32 : &x_map16;
+            const CUtensorMap* map = FORM == kQmmWide ? (box == args.dense_per_tile ? &x_map0 : &x_map1)
+                                                      : box == 64 ? &x_map3 : box == 48 ? &x_map2 : box == 32 ? &x_map1 : &x_map0;
             const int row = (int)(tl.row0 + rank * box);
             for (uint32_t ks = 0; ks < ksteps; ++ks) {
                 if (ub > 0 && !q_mbar_wait(bar_empty_b(sb), (ub - 1) & 1)) { fail = kErrQmmTimeout | 7; break; }
@@ -525,10 +555,10 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map16, const __grid_con
             for (uint32_t s = 0; s < b_stages; ++s) q_mbar_wait(bar_full_b(s), (s < sb ? ub : ub + 1) & 1);
     } else if (warp == 1 || warp == 3) {
         // ===================== MMA issuers =====================
-        // PAIR: warp 1 of the first CTA issues every stage. Otherwise the two warps take turns, each with an accumulator of its
-        // own (the epilogue adds them).
+        // One issuer: warp 1 of the (first) CTA issues every stage. Two: the warps take turns, each with an accumulator of its own
+        // (the epilogue adds them).
         const uint32_t who = warp == 1 ? 0 : 1;
-        const bool mine = PAIR ? rank == 0 && who == 0 : true;
+        const bool mine = kTwoIssuers || (rank == 0 && who == 0);
         uint32_t sb = 0, ub = 0, count = 0, buf = 0, uacc = 0;        // count: stages so far; stage c is the (c / 2)-th use of its team's slot
         const uint64_t b_desc0 = umma_smem_desc(base + off_b);
         bool ready = false;                                           // the next stage's operands were there at the last look
@@ -539,13 +569,13 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map16, const __grid_con
             const uint32_t b_block = (n / kCtas * 128) >> 4;         // 64 columns of a slot, in units of the descriptor
             // Only for a tile that this warp has a stage of: the parity tells phases apart only while the barrier is at most one
             // phase ahead of the wait, and a tile of one stage can be multiplied and emptied without the other issuer.
-            const bool takes_part = PAIR || ksteps > 1 || (count & 1) == who;
+            const bool takes_part = !kTwoIssuers || ksteps > 1 || (count & 1) == who;
             if (takes_part && uacc > 0 && !q_mbar_wait(bar_acc_empty(buf), (uacc - 1) & 1)) { fail = kErrQmmTimeout | 2; break; }
             tc_fence_after();
-            const uint32_t acc = tmem_base + (PAIR ? buf * kAccTok : (2 * buf + who) * kAccTok);
+            const uint32_t acc = tmem_base + (kTwoIssuers ? 2 * buf + who : buf) * kAccTok;
             uint32_t accumulate = 0;
             for (uint32_t ks = 0; ks < ksteps; ++ks) {
-                if (PAIR || (count & 1) == who) {
+                if (!kTwoIssuers || (count & 1) == who) {
                     const uint32_t t = count & 1;
                     if (!ready && (!q_mbar_wait(bar_full_b(sb), ub & 1) || !q_mbar_wait(bar_full_a(t), (count >> 1) & 1))) {
                         fail = kErrQmmTimeout | 3;
@@ -566,7 +596,7 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map16, const __grid_con
 #pragma unroll
                         for (uint32_t g = 0; g < 3; ++g) multiply(g);
                     }
-                    if constexpr (PAIR) {
+                    if constexpr (!kTwoIssuers) {
                         // A look at the next stage while these MMAs run: a wait on a barrier that is ready takes about 100 clocks,
                         // in which the tensor cores would run dry. (With few tokens the next operands are never there this early.)
                         __syncwarp();
@@ -578,7 +608,7 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map16, const __grid_con
                         multiply(3);
                         tc_commit<PAIR>(bar_empty_a(t));              // both slots are free once these MMAs have read them
                         tc_commit<PAIR>(bar_empty_b(sb));
-                        if (ks + (PAIR ? 1 : 2) >= ksteps) tc_commit<PAIR>(bar_acc_full(who, buf));
+                        if (ks + (kTwoIssuers ? 2 : 1) >= ksteps) tc_commit<PAIR>(bar_acc_full(who, buf));
                     }
                     __syncwarp();
                     accumulate = 1;
@@ -589,39 +619,40 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map16, const __grid_con
             if (++buf == 2) { buf = 0; ++uacc; }
         }
     } else if (warp < kQmmFirstEpilogueWarp) {
-        // ===================== dequantisers: two teams of eight warps, each takes every other stage =====================
-        // A thread takes two quantisation groups of one weight row. While a team waits for codes, for its slot or for its stores,
-        // the other one computes.
+        // ===================== dequantisers =====================
+        // Two teams of eight warps: each takes every other stage, a thread two quantisation groups of one weight row. While a team
+        // waits for codes, for its slot or for its stores, the other one computes. One team: every stage, a group per thread.
         const uint32_t dw = warp - kQmmFirstDequantWarp;
-        const uint32_t q = dw & 3, gc = ((dw >> 2) & 1) * 2;     // TMEM lane quarter; first group within the stage
-        const uint32_t team = dw >> 3;
+        const uint32_t q = dw & 3, gc = (dw >> 2) % (4 / kTeams) * kTeams;       // TMEM lane quarter; first group within the stage
+        const uint32_t team = dw / kTeamWarps;
         const uint32_t r = q * kWarp + lane;                     // row within the tile = TMEM lane
         // packed codes of the row: 128 bytes whose 16-byte chunks sit at chunk ^ (row % 8) (128-byte TMA swizzle)
         const uint32_t raw_off = base + r * 128 + (((2 * gc) ^ (r & 7u)) << 4);
         const uint32_t sc_off = base + plan.off_sc + (r / kMatRows) * 2 * plan.plane_bytes + (r % kMatRows) * ng * 2 + gc * 2;
-        const uint32_t a_slot = a_ring + ((q * kWarp) << 16) + team * 128 + gc * 32;      // the team's slot
-        uint32_t sr = 0, ur = 0, sc = 0, uc = 0, ua = 0, turn = 0;
+        const uint32_t a_lane = a_ring + ((q * kWarp) << 16) + gc * 32;
+        uint32_t sr = 0, ur = 0, sc = 0, uc = 0, count = 0;      // count: stages so far; stage c is the (c / 2)-th use of slot c % 2
         for (uint32_t tile = first_tile; tile < total_tiles && !fail; tile += tile_step) {
             if (!q_mbar_wait(bar_full_sc(sc), uc & 1)) { fail = kErrQmmTimeout | 8; break; }
             const uint32_t sc_base = sc_off + sc * plan.sc_bytes;
             for (uint32_t ks = 0; ks < ksteps; ++ks) {
-                if (turn == team) {
+                const uint32_t slot = count & 1, ua = count >> 1;
+                if (kTeams == 1 || slot == team) {
                     const uint32_t left = ng - 4 * ks > gc ? ng - 4 * ks - gc : 0;         // groups past K are neither dequantised nor multiplied
-                    float sf[2], bf[2];
+                    float sf[kTeams], bf[kTeams];
+                    bool fast[kTeams];
 #pragma unroll
-                    for (uint32_t h = 0; h < 2; ++h) {
+                    for (uint32_t h = 0; h < kTeams; ++h) {
                         sf[h] = left > h ? bf16_bits_to_float((uint16_t)q_lds16(sc_base + ks * 8 + h * 2)) : 0.0f;
                         bf[h] = left > h ? bf16_bits_to_float((uint16_t)q_lds16(sc_base + plan.plane_bytes + ks * 8 + h * 2)) : 0.0f;
+                        fast[h] = __all_sync(kFullMask, fabsf(sf[h]) < FastScale<NATURAL_K>::kLimit);
                     }
-                    const bool fast[2] = {(bool)__all_sync(kFullMask, fabsf(sf[0]) < FastScale<NATURAL_K>::kLimit),
-                                          (bool)__all_sync(kFullMask, fabsf(sf[1]) < FastScale<NATURAL_K>::kLimit)};
                     if (!q_mbar_wait(bar_full_raw(sr), ur & 1)) { fail = kErrQmmTimeout | 4; break; }
                     const uint32_t src = raw_off + sr * kQmmRawBytes;
-                    uint4 c[4];
+                    uint4 c[2 * kTeams];
 #pragma unroll
-                    for (uint32_t i = 0; i < 4; ++i) c[i] = q_lds128(src ^ (i << 4));
+                    for (uint32_t i = 0; i < 2 * kTeams; ++i) c[i] = q_lds128(src ^ (i << 4));
 #pragma unroll
-                    for (uint32_t h = 0; h < 2; ++h) {
+                    for (uint32_t h = 0; h < kTeams; ++h) {
                         const uint4 c0 = c[2 * h], c1 = c[2 * h + 1];
                         uint4 out[8];
                         if (fast[h]) {                            // one branch per warp and group, both arms straight-line
@@ -641,22 +672,21 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map16, const __grid_con
                         if (h == 0) {
                             __syncwarp();
                             if (lane == 0) q_mbar_arrive(bar_empty_raw(sr));      // the codes are in registers
-                            if (ua > 0 && !q_mbar_wait(bar_empty_a(team), (ua - 1) & 1)) { fail = kErrQmmTimeout | 5; break; }
+                            if (ua > 0 && !q_mbar_wait(bar_empty_a(slot), (ua - 1) & 1)) { fail = kErrQmmTimeout | 5; break; }
                             tc_fence_after();
                         }
-                        if (left > h) tc_st32(a_slot + h * 32, out);
+                        if (left > h) tc_st32(a_lane + slot * 128 + h * 32, out);
                     }
                     if (fail) break;
                     tc_wait_st();
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) {
-                        if constexpr (PAIR) q_mbar_arrive_cluster(q_in_leader(bar_full_a(team)));
-                        else q_mbar_arrive(bar_full_a(team));
+                        if constexpr (PAIR) q_mbar_arrive_cluster(q_in_leader(bar_full_a(slot)));
+                        else q_mbar_arrive(bar_full_a(slot));
                     }
-                    ++ua;
                 }
-                turn ^= 1;
+                ++count;
                 if (++sr == raw_stages) { sr = 0; ++ur; }
             }
             __syncwarp();
@@ -680,8 +710,8 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map16, const __grid_con
             tl.locate(table, ngroups, lane);
             const uint32_t first = (tl.wt * kCtas + rank) * kMatRows;
             const uint32_t left = first < args.rows ? args.rows - first : 0, nrows = left < kMatRows ? left : kMatRows;
-            const bool two = !PAIR && ksteps > 1;                     // both issuers had stages of the tile
-            const uint32_t one = PAIR ? 0 : turn;                     // the issuer of its first stage
+            const bool two = kTwoIssuers && ksteps > 1;                     // both issuers had stages of the tile
+            const uint32_t one = kTwoIssuers ? turn : 0;                     // the issuer of its first stage
             if (!q_mbar_wait(bar_acc_full(one, buf), uacc & 1)) fail = kErrQmmTimeout | 9;
             if (two && !q_mbar_wait(bar_acc_full(one ^ 1, buf), uacc & 1)) fail = kErrQmmTimeout | 9;
             turn ^= ksteps & 1;
@@ -690,7 +720,7 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map16, const __grid_con
                          : "=r"(flip) : "r"(fail) : "memory");
             if (flip) { if (!fail) fail = kErrQmmTimeout | 9; break; }
             tc_fence_after();
-            const uint32_t acc = tmem_base + ((q * kWarp) << 16) + (PAIR ? buf : 2 * buf + one) * kAccTok;
+            const uint32_t acc = tmem_base + ((q * kWarp) << 16) + (kTwoIssuers ? 2 * buf + one : buf) * kAccTok;
             const uint32_t acc2 = tmem_base + ((q * kWarp) << 16) + (2 * buf + (one ^ 1)) * kAccTok;      // the other issuer's
             uint32_t which = 0;
             for (uint32_t c0 = 0; c0 < tl.ntok; c0 += 32, which ^= 1) {
@@ -698,7 +728,7 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map16, const __grid_con
                 tc_ld16(acc + c0, va);
                 tc_ld16(acc + c0 + 16, vb);                       // past the tile's tokens: stale columns of the buffer, never stored
                 tc_wait_ld();
-                if constexpr (!PAIR) {
+                if constexpr (kTwoIssuers) {
                     if (two) {
                         uint32_t v2[16];
                         tc_ld16(acc2 + c0, v2);
@@ -880,24 +910,38 @@ static bool qmm_plan(uint32_t k, uint32_t nmat, QmmPlan* p) {
     return true;
 }
 
-// Tokens per tile of a dense launch, by one CTA or by pairs: rounds of the grid x the clocks of a tile's stages, and what start
-// and last epilogue take. The clocks of a stage are fitted to launches of 16 to 64 and of 32 to 128 tokens per tile (us, 1000 x 2112
-// x 2816: 50, 28, 25, 20 and 36, 23, 24, 17; 333 x 2112 x 2816: 22, 16, 12, 13 and 21, 14, 14, 15; 200 x 512 x 1024: 6.8, 6.9, 7.5,
-// 7.5 and 8.5, 8.7, 9.2, 10).
+// Form and tokens per tile of a dense launch: the least of rounds of the grid x (a tile's stages + what a tile takes besides) + what
+// the call takes besides. Fitted to 1500 launches of 13 matrices (256 x 256 to 8192 x 768 and 4096 x 2816) x 65 to 4096 tokens in every
+// form and tile size; what it picks takes 0.3 % longer than the best of them on average, 6 % at the most. us, kQmmFew, kQmmWide and
+// kQmmPair at their best sizes: 333 x 2112 x 2816 11.8, 13.1, 13.4; 1000 x 4096 x 512 11.1, 9.8, 10.6; 700 x 2816 x 704 9.2, 8.8, 9.6;
+// 1000 x 2112 x 2816 19.2, 16.0, 15.4; 4096 x 4096 x 2816 102, 81, 70.
 struct QmmDense {
-    uint32_t ctas, per_tile;
+    QmmForm form;
+    uint32_t per_tile;
 };
-static QmmDense qmm_dense_tiles(uint32_t tokens, uint32_t rows, uint32_t mat_rows, uint32_t stages, uint32_t sms) {
-    QmmDense best{1, 16};
+static QmmDense qmm_dense_tiles(uint32_t tokens, uint32_t rows, uint32_t mat_rows, uint32_t stages, uint32_t sms, uint32_t most_wide) {
+    struct Cost { uint32_t stage, token, tile, call; };               // in units of 50 ps; token: per token of the tile and stage
+    constexpr Cost kCost[3] = {{7800, 65, 7400, 94800}, {6000, 98, 9800, 91200}, {9800, 44, 10400, 118600}};      // by form
+    QmmDense best{kQmmFew, 16};
     uint64_t best_cost = ~0ull;
-    for (uint32_t ctas = 1; ctas <= 2 && ctas <= sms; ++ctas)
-        for (uint32_t per = ctas * kQmmBoxMax; per >= ctas * 16u; per -= ctas * 16u) {
+    for (const QmmForm form : {kQmmFew, kQmmWide, kQmmPair}) {
+        const uint32_t ctas = form == kQmmPair ? 2 : 1, step = ctas * 16u;
+        if (ctas > sms) continue;
+        const uint32_t least = form == kQmmWide ? kQmmBoxMax + step : step;
+        for (uint32_t per = form == kQmmWide ? most_wide : ctas * kQmmBoxMax; per >= least; per -= step) {
             const uint64_t tiles = (uint64_t)((rows + ctas * mat_rows - 1) / (ctas * mat_rows)) * ((tokens + per - 1) / per);
             const uint64_t rounds = (tiles + sms / ctas - 1) / (sms / ctas);
-            const uint64_t cost = ctas == 1 ? rounds * stages * (1000 + 5 * per) + 9500 : rounds * stages * (1250 + 3 * per) + 11400;
-            if (cost < best_cost) { best_cost = cost; best = {ctas, per}; }
+            const Cost& c = kCost[form];
+            const uint64_t cost = rounds * ((uint64_t)stages * (c.stage + c.token * per) + c.tile) + c.call;
+            if (cost < best_cost) { best_cost = cost; best = {form, per}; }
         }
+    }
     return best;
+}
+// Tokens of a kQmmWide tile: two slots of the activation ring have to fit beside two stages of packed codes.
+static uint32_t qmm_most_wide(const QmmPlan& p) {
+    const uint32_t fit = (p.off_b + p.b_bytes - 2 * kQmmRawBytes) / (2 * kQmmRowBytes) & ~15u;
+    return fit < 128u ? fit : 128u;
 }
 
 // Fills a's group table (a.plan and the groups' source are set). The context has three: one for dense launches, which may run
@@ -916,7 +960,7 @@ static tf_status launch_qmm_prepare(tf_context* ctx, void* stream, QmmArgs& a, i
 
 // W[m]: base of matrix m's packed plane for expert 0 (dense: the matrix itself); a.S, a.B likewise. A routed launch's table
 // has been filled by the caller.
-template <int NMAT, bool NATURAL_K, bool PAIR>
+template <int NMAT, bool NATURAL_K, QmmForm FORM>
 static tf_status launch_qmm_kernel(tf_context* ctx, void* stream, QmmArgs& a, const void* x, uint64_t x_rows, uint32_t x_stride,
                             const uint8_t* const* W, uint64_t experts, uint64_t expert_stride, bool dense, const char* name) {
     TF_REQUIRE(ctx, a.k % kGroup == 0 && a.k >= (uint32_t)kGroup, TF_ERR_INVALID_ARGUMENT, "%s: K must be a positive multiple of 64", name);
@@ -924,24 +968,31 @@ static tf_status launch_qmm_kernel(tf_context* ctx, void* stream, QmmArgs& a, co
     TF_REQUIRE(ctx, aligned(x, 16) && (x_stride * 2) % 16 == 0, TF_ERR_ALIGNMENT, "%s: activation rows must be 16-byte aligned", name);
     TF_REQUIRE(ctx, qmm_plan(a.k, NMAT, &a.plan), TF_ERR_UNSUPPORTED, "%s: K=%u needs more shared memory for the scale planes than there is", name, a.k);
     constexpr uint32_t kMatRows = kQmmRows / NMAT;
-    // Activation boxes of 16, 32, 48 and 64 rows. A dense launch knows its tiles (full ones and a last one) and encodes only
-    // the boxes of those: an encode is most of a microsecond of host time, and small products are bound by it.
-    constexpr uint32_t kCtas = PAIR ? 2 : 1;
-    uint32_t boxes = 15u;
+    // Activation boxes: see the kernel. A dense launch knows its tiles (full ones and a last one) and encodes only the boxes of
+    // those: an encode is most of a microsecond of host time, and small products are bound by it.
+    constexpr uint32_t kCtas = FORM == kQmmPair ? 2 : 1;
+    uint32_t box[4] = {16, 32, 48, 64};           // 0: not wanted
     if (dense) {
         const uint32_t rest = a.dense_tokens % a.dense_per_tile;
-        boxes = (a.dense_tokens >= a.dense_per_tile ? 1u << (a.dense_per_tile / kCtas / 16 - 1) : 0u) |
-                (rest ? 1u << ((rest + 16 * kCtas - 1) / (16 * kCtas) - 1) : 0u);
+        const uint32_t full_box = a.dense_tokens >= a.dense_per_tile ? a.dense_per_tile / kCtas : 0u;
+        const uint32_t rest_box = (rest + 16 * kCtas - 1) / (16 * kCtas) * 16;
+        if (FORM == kQmmWide) {
+            box[0] = full_box ? full_box : rest_box == a.dense_per_tile ? rest_box : 0u;
+            box[1] = rest_box == a.dense_per_tile ? 0u : rest_box;
+            box[2] = box[3] = 0;
+        } else {
+            for (uint32_t& b : box) b = b == full_box || b == rest_box ? b : 0u;
+        }
     }
     CUtensorMap xmap[4], wmap[2];
     int some = -1;
     for (int i = 0; i < 4; ++i) {
-        if (!(boxes & (1u << i))) continue;
-        if (tf_status s = make_x_map(ctx, &xmap[i], x, x_rows, a.k, x_stride, 16u * (i + 1), name)) return s;
+        if (box[i] == 0) continue;
+        if (tf_status s = make_x_map(ctx, &xmap[i], x, x_rows, a.k, x_stride, box[i], name)) return s;
         some = i;
     }
     for (int i = 0; i < 4; ++i)
-        if (!(boxes & (1u << i))) xmap[i] = xmap[some];
+        if (box[i] == 0) xmap[i] = xmap[some];
     for (int m = 0; m < NMAT; ++m)
         if (tf_status s = make_w_map(ctx, &wmap[m], W[m], a.rows, a.k, experts, dense ? (uint64_t)a.rows * (a.k / 2) : expert_stride, kMatRows, name)) return s;
     if (NMAT == 1) wmap[1] = wmap[0];
@@ -950,14 +1001,16 @@ static tf_status launch_qmm_kernel(tf_context* ctx, void* stream, QmmArgs& a, co
     a.error = ctx->device_error;
     if (dense)
         if (tf_status s = launch_qmm_prepare(ctx, stream, a, kQmmDenseTable, name)) return s;
-    auto kern = qmm_tcgen05_kernel<NMAT, NATURAL_K, PAIR>;
+    auto kern = qmm_tcgen05_kernel<NMAT, NATURAL_K, FORM>;
     static DeviceSmemCache configured;
     if (tf_status s = ensure_dynamic_smem(ctx, kern, configured, a.plan.total)) return s;
     uint32_t grid = (uint32_t)ctx->sm_count / kCtas;
+    const uint32_t wrow_tiles = (a.rows + kCtas * kMatRows - 1) / (kCtas * kMatRows);
     if (dense) {
-        const uint64_t tiles = (uint64_t)((a.rows + kCtas * kMatRows - 1) / (kCtas * kMatRows)) * ((a.dense_tokens + a.dense_per_tile - 1) / a.dense_per_tile);
+        const uint64_t tiles = (uint64_t)wrow_tiles * ((a.dense_tokens + a.dense_per_tile - 1) / a.dense_per_tile);
         if (tiles < grid) grid = (uint32_t)tiles;
     }
+    a.step_tok = grid / wrow_tiles; a.step_row = grid % wrow_tiles;
     launch_pdl_cluster(kern, dim3(grid * kCtas), dim3(kQmmThreads), a.plan.total, static_cast<cudaStream_t>(stream), kCtas, xmap[0], xmap[1],
                        xmap[2], xmap[3], wmap[0], wmap[1], a);
     return check_launch(ctx, name);
@@ -965,12 +1018,15 @@ static tf_status launch_qmm_kernel(tf_context* ctx, void* stream, QmmArgs& a, co
 template <int NMAT, bool NATURAL_K>
 static tf_status launch_qmm(tf_context* ctx, void* stream, QmmArgs& a, const void* x, uint64_t x_rows, uint32_t x_stride,
                             const uint8_t* const* W, uint64_t experts, uint64_t expert_stride, bool dense, const char* name) {
-    if (dense) {
-        const QmmDense t = qmm_dense_tiles(a.dense_tokens, a.rows, kQmmRows / NMAT, (a.k + kQmmStageK - 1) / kQmmStageK, (uint32_t)ctx->sm_count);
-        a.ctas = t.ctas; a.dense_per_tile = t.per_tile;
+    if constexpr (NATURAL_K) {             // the dense launches
+        const QmmDense t = qmm_dense_tiles(a.dense_tokens, a.rows, kQmmRows / NMAT, (a.k + kQmmStageK - 1) / kQmmStageK, (uint32_t)ctx->sm_count,
+                                           qmm_plan(a.k, NMAT, &a.plan) ? qmm_most_wide(a.plan) : 0u);
+        a.ctas = t.form == kQmmPair ? 2 : 1; a.dense_per_tile = t.per_tile;
+        if (t.form == kQmmWide)
+            return launch_qmm_kernel<NMAT, NATURAL_K, kQmmWide>(ctx, stream, a, x, x_rows, x_stride, W, experts, expert_stride, dense, name);
     }
-    return a.ctas == 2 ? launch_qmm_kernel<NMAT, NATURAL_K, true>(ctx, stream, a, x, x_rows, x_stride, W, experts, expert_stride, dense, name)
-                       : launch_qmm_kernel<NMAT, NATURAL_K, false>(ctx, stream, a, x, x_rows, x_stride, W, experts, expert_stride, dense, name);
+    return a.ctas == 2 ? launch_qmm_kernel<NMAT, NATURAL_K, kQmmPair>(ctx, stream, a, x, x_rows, x_stride, W, experts, expert_stride, dense, name)
+                       : launch_qmm_kernel<NMAT, NATURAL_K, kQmmFew>(ctx, stream, a, x, x_rows, x_stride, W, experts, expert_stride, dense, name);
 }
 
 tf_status launch_qmm_generic(tf_context* ctx, void* stream, const uint8_t* W, const uint16_t* S, const uint16_t* B,
