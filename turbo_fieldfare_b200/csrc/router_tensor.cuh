@@ -569,7 +569,9 @@ router_recheck_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict_
     auto next_candidate = [&]() {
         const uint32_t e = next < candidates ? (uint32_t)list[next] : 0xFFFFFFFFu;
         next += WPT;
-        return e;
+        // The shuffle tells the compiler that the warp has one expert, and its guards in the chunked loop one outcome: 1200 rows of 128
+        // experts x 2048, 87 -> 82 us, 4096 rows x 4096 312 -> 297. (Nothing is guarded in the other loops.)
+        return GROUPS > 0 ? e : __shfl_sync(kFullMask, e, 0);
     };
     // (expert, chunk) pairs in one software pipeline: the next pair's loads are issued before the current pair is multiplied
     uint32_t ld_e = next_candidate(), ld_g = 0u;
