@@ -194,6 +194,12 @@ def test_single_rank_peer_exchange_matches_fused_stack_and_replays_in_a_graph(tf
     ep_stack.close()
 
 
+# More than three tokens per SM: the combine that starts with the wait for the return flags takes several tokens per thread block.
+@pytest.mark.parametrize("T,tensor_rows", [(600, 0), (1801, 1)])
+def test_single_rank_peer_exchange_of_many_tokens(tf_ctx, oracle, T, tensor_rows):
+    test_single_rank_peer_exchange_matches_fused_stack_and_replays_in_a_graph(tf_ctx, oracle, T, tensor_rows)
+
+
 def test_peer_barrier_wait_runs_out_and_reports(oracle):
     """A barrier whose second participant never arrives (its flag is a word that nothing sets): the bounded wait gives
     up after about two seconds, the kernel returns, the context reports the device code and stays usable, and a later

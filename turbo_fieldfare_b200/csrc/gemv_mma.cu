@@ -1,4 +1,4 @@
-// Streaming int4 GEMV for large matrices: y[m] = deq4(W[m,n]) . x[n] at HBM speed.
+// Streaming int4 GEMVs for large matrices: y[m] = deq4(W[m,n]) . x[n] at HBM speed.
 // Second implementation of dequant_int4_gemv_simd (Metal/Quant/dequant_int4.metal:93-191) for the sizes where
 // the warp-per-row kernel of gemv.cu is bound by its instruction count (about three CUDA-core instructions per
 // weight: extract, convert, multiply-add), e.g. the LM-head-sized instance 262144 x 2816.
@@ -11,6 +11,8 @@
 // memory in fragment order. Scale and bias are applied per group to the fp32 accumulator, acc += s * (q . x)
 // + b * sum(x), the reference's algebra (dequant_int4.metal:132-170). Four groups are in flight as
 // independent MMA chains, and the next four groups' codes are loaded before the current ones are consumed.
+// That is gemv_mma_kernel: batches of small matrices, rows of few columns, smaller greedy heads. gemv_stream_kernel below does the
+// same arithmetic on whole rows that bulk copies bring to shared memory; gs_teams says which one a product takes.
 #include "async_copy.cuh"
 #include "mma_gemv.cuh"
 
