@@ -483,7 +483,7 @@ def measure_gemv(torch, ctx, peak, peak_src):
     ms = s.elapsed_time(e) / reps
     nbytes = mat.w_bytes + 2 * mat.sb_bytes
     achieved = nbytes / (ms * 1e-3) / 1e9
-    return {"bound": "hbm", "kernel": "gemv_mma_kernel (tf_int4_gemv, 262144 x 2816)", "achieved": achieved, "peak": peak, "unit": "GB/s",
+    return {"bound": "hbm", "kernel": "gemv_stream_kernel (tf_int4_gemv, 262144 x 2816)", "achieved": achieved, "peak": peak, "unit": "GB/s",
             "frac": achieved / peak, "peak_source": peak_src, "bytes_per_launch": nbytes, "us_per_launch": ms * 1e3}
 
 
