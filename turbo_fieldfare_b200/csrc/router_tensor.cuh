@@ -537,7 +537,12 @@ router_recheck_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict_
     const uint32_t groups = d / kGroup;
     // tokens past the end repeat the last one (the same values are written twice)
     const uint32_t row = min(blockIdx.x * kTokens + slot, rows - 1);
-    pdl_launch_dependents();
+    // With grouping the routed gate/up launch comes next and is let in only before the grouping, as in router_rows_kernel: let in at the
+    // start it takes the SMs that the shared expert's gate/up, which no longer fits beside a block of this kernel since that holds
+    // staged rows, could use meanwhile. 30 layers, us, at the start and late: 65 tokens 4819 and 4112, 100 tokens 5623 and 4952, 128
+    // tokens 6583 and 6088, 150 tokens 6998 and 6190, 175 tokens 7427 and 6634, 190 to 255 tokens the same.
+    const bool late = WPT == kRecheckWarps && grp.sorted_pairs != nullptr;
+    if (!late) pdl_launch_dependents();
     pdl_wait();
     const uint16_t* hrow = hidden + (size_t)row * hidden_stride;
     for (uint32_t e = part * kWarp + lane; e < num_experts; e += WPT * kWarp) scores[e] = -INFINITY;
@@ -665,6 +670,7 @@ router_recheck_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict_
         }
         __syncthreads();
         if (!is_last) return;
+        pdl_launch_dependents();
         __threadfence();
         group_routes_in_block<true>(out_idx, out_w, rows, top_k, num_experts, grp, smem);
     }
