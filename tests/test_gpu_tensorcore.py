@@ -254,9 +254,9 @@ def test_shared_expert_tensorcore_vs_oracle(tf_ctx, oracle, T, D, Fs):
         assert o.rel_error(got[t], truth) < FP16_CHAINED
 
 
-# Edges of the two forms of the GEMM. One CTA per tile: one stage per tile over more tiles than CTAs (the MMA issuers take whole
-# tiles in turn), three groups in the last stage, rows beyond the last whole tile, one buffer of scale planes. Pairs: an odd number
-# of weight-row tiles (the second CTA's last tile is past the matrix), a last stage of one group, a ragged last token tile.
+# Edges of tiles by one CTA: one stage per tile over more tiles than CTAs (the two MMA issuers take whole tiles in turn), three groups in
+# the last stage, rows beyond the last whole tile, one buffer of scale planes; with one issuer many tokens for few rows, an odd
+# number of weight-row tiles, a last stage of one group, a ragged last token tile.
 @pytest.mark.parametrize("M,N,K", [(16, 20000, 64), (48, 40008, 192), (65, 200, 704), (700, 520, 7104), (9000, 264, 1088), (1000, 2120, 704)])
 def test_int4_qmm_edges_of_both_forms(tf_ctx, oracle, M, N, K):
     test_int4_qmm_vs_oracle(tf_ctx, oracle, M, N, K)
@@ -275,12 +275,14 @@ def test_int4_qmm_edges_of_wide_tiles(tf_ctx, oracle, M, N, K):
     test_int4_qmm_vs_oracle(tf_ctx, oracle, M, N, K)
 
 
-# The same for a shared expert's gate/up, and pairs with an odd number of weight-row tiles for plain rows.
+# The same for a shared expert's gate/up.
 @pytest.mark.parametrize("T,D,Fs", [(700, 512, 1024), (333, 576, 4096)])
 def test_shared_expert_tensorcore_wide_tiles(tf_ctx, oracle, T, D, Fs):
     test_shared_expert_tensorcore_vs_oracle(tf_ctx, oracle, T, D, Fs)
 
 
-@pytest.mark.parametrize("M,N,K", [(600, 2824, 2112), (1000, 2112, 2816)])
+# Pairs: an odd number of weight-row tiles (the second CTA's last tile is past the matrix), a last stage of one group, a ragged last
+# token tile.
+@pytest.mark.parametrize("M,N,K", [(900, 2120, 2112), (2000, 2120, 1344), (1000, 2112, 2816)])
 def test_int4_qmm_pairs_past_the_matrix(tf_ctx, oracle, M, N, K):
     test_int4_qmm_vs_oracle(tf_ctx, oracle, M, N, K)
