@@ -515,7 +515,7 @@ tf_status tf_workspace_create(tf_context* ctx, uint32_t max_tokens, uint32_t d, 
                    o_ecnt = take(E * 4), o_groups = take(E * 12), o_cgroup = take((T * K / 8 + E + 1) * 4),
                    o_cstart = take(E * 4), o_counters = take(16), o_acts = take(T * K * f * 2),
                    o_partials = take(T * K * d * (T <= tf::kF32PartialTokens ? 4 : 2)), o_sact = take(T * fs * 2),
-                   o_sy = take(T * d * 2), o_xn = take(T * d * 2), o_yb = take(T * d * 2), o_ticket = take(4);
+                   o_sy = take(T * d * 2), o_xn = take(T * d * 2), o_yb = take(T * d * 2), o_ticket = take(4), o_logits = take(TF_MAX_ROUTER_EXPERTS * 4);
     // workspaces that can hold a tensor-core sized block also carry the expert-sorted activation rows
     const bool tensor_path = T >= ctx->tensorcore_min_tokens && d % 64 == 0 && f % 64 == 0 && fs % 64 == 0;
     const uint64_t o_xs = tensor_path ? take(T * K * d * 2) : 0, o_inv = tensor_path ? take(T * K * 4) : 0,
@@ -544,6 +544,7 @@ tf_status tf_workspace_create(tf_context* ctx, uint32_t max_tokens, uint32_t d, 
     w->shared_act = reinterpret_cast<uint16_t*>(base + o_sact);
     w->shared_y = reinterpret_cast<uint16_t*>(base + o_sy);
     w->router_ticket = reinterpret_cast<uint32_t*>(base + o_ticket);
+    w->one_token_logits = reinterpret_cast<float*>(base + o_logits);
     w->x_norm = reinterpret_cast<uint16_t*>(base + o_xn);
     w->y_block = reinterpret_cast<uint16_t*>(base + o_yb);
     w->x_sorted = tensor_path ? reinterpret_cast<uint16_t*>(base + o_xs) : nullptr;
@@ -634,6 +635,8 @@ static tf_status block_forward(tf_context* ctx, void* stream, const tf_moe_layer
                "%s: router is (%u,%u), expected (%u,%u)", name, layer->router.rows, layer->router.cols, layer->num_experts, layer->d);
     if (tokens == 0) return TF_OK;
     const uint32_t d = layer->d, K = layer->top_k;
+    if (tokens == 1 && y != nullptr && aligned(x, 16) && aligned(y, 2) && one_token_eligible(ctx, layer, ws))
+        return one_token_block(ctx, stream, layer, x, y, ws);
     // The shared expert needs only x, so it runs on the context's side stream beside the router and the routed
     // experts and joins before the combine (inside a stream capture this becomes a fork and a join of the graph).
     cudaStream_t main_st = static_cast<cudaStream_t>(stream);
@@ -956,6 +959,17 @@ tf_status tf_stack_forward(tf_stack* st, void* stream, void* hidden, uint32_t to
     TF_REQUIRE(ctx, tf::aligned(hidden, 16), TF_ERR_ALIGNMENT, "%s: hidden must be 16-byte aligned", name);
     // one token: the whole step is one persistent launch (decode_step.cu)
     if (tokens == 1 && ctx->single_launch_step && tf::decode_step_eligible(st, ws)) return tf::launch_decode_step(ctx, stream, st, hidden, ws);
+    if (tokens == 1) {
+        bool fused = !st->layers.empty();
+        for (size_t l = 0; l < st->layers.size() && fused; ++l) {
+            const tf_moe_layer& m = st->layers[l];
+            fused = m.d == d && m.f == ws->f && m.fs == ws->fs && m.top_k == ws->top_k && m.num_experts == ws->num_experts &&
+                    st->norm_weights[l] && tf::aligned(st->norm_weights[l], 16) && tf::one_token_eligible(ctx, &m, ws);
+        }
+        for (size_t l = 0; l < st->layers.size() && fused; ++l)
+            if (tf_status s = tf::one_token_layer(ctx, stream, &st->layers[l], st->norm_weights[l], hidden, st->eps, ws)) return s;
+        if (fused) return TF_OK;
+    }
     cudaStream_t cs = static_cast<cudaStream_t>(stream);
     uint16_t* h = static_cast<uint16_t*>(hidden);
     // Decode-sized steps: the weighted sum of a layer's route partials, the residual add and the next norm are one

@@ -30,6 +30,7 @@ struct tf_workspace {
     uint16_t* x_sorted;     // [T*K, D] expert-sorted activation rows (tensor-core path; NULL for small workspaces)
     uint32_t* inverse_perm; // [T*K] sorted row of every (token, rank)
     uint32_t* pack_ids;     // [T*K]
+    float* one_token_logits;  // [TF_MAX_ROUTER_EXPERTS] (one_token.cu)
     uint64_t bytes;
 };
 
@@ -49,6 +50,10 @@ struct PeerWait;
 bool decode_step_eligible(const tf_stack* st, const tf_workspace* ws);
 tf_status decode_step_prepare(tf_context* ctx, tf_stack* st);
 tf_status launch_decode_step(tf_context* ctx, void* stream, tf_stack* st, void* hidden, tf_workspace* ws);
+// one_token.cu: a layer of a stack (hidden row updated in place), or a block forward, for one token
+bool one_token_eligible(const tf_context* ctx, const tf_moe_layer* layer, const tf_workspace* ws);
+tf_status one_token_layer(tf_context* ctx, void* stream, const tf_moe_layer* layer, const void* norm_weight_bf16, void* hidden, float eps, tf_workspace* ws);
+tf_status one_token_block(tf_context* ctx, void* stream, const tf_moe_layer* layer, const void* x, void* y, tf_workspace* ws);
 // grouped.cu: tf_group_routes_device over ids read at a stride (and optionally written out densely)
 tf_status group_routes_strided(tf_context* ctx, void* stream, const uint32_t* indices, uint32_t idx_stride, uint32_t* ids_out,
                                const void* weights_f16, uint32_t query_count, uint32_t top_k, uint32_t num_experts,

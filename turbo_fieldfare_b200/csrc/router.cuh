@@ -241,4 +241,52 @@ __device__ __forceinline__ void group_routes_in_block(const uint32_t* __restrict
     }
 }
 
+// The tables of one token: a pair's place is the number of selected experts with a smaller id; every group holds one pair and one
+// chunk. That needs distinct experts: a row with fewer than top_k selectable logits (NaN, -inf) repeats an expert, and then the general
+// grouping merges the repeats into one group. All threads of the block, after a barrier behind the writes of out_idx and out_w.
+__device__ __forceinline__ void group_one_token(const uint32_t* out_idx, const uint16_t* out_w, uint32_t top_k, uint32_t num_experts,
+                                                const RouterGroupOut& grp, uint8_t* smem) {
+    int repeated = 0;
+    if (threadIdx.x < top_k) {
+        uint32_t mine = out_idx[threadIdx.x];
+        if (mine >= num_experts) mine = num_experts - 1;
+        for (uint32_t r = 0; r < top_k; ++r) {
+            uint32_t other = out_idx[r];
+            if (other >= num_experts) other = num_experts - 1;
+            repeated |= (r != threadIdx.x && other == mine) ? 1 : 0;
+        }
+    }
+    if (__syncthreads_or(repeated)) {
+        group_routes_in_block<false>(out_idx, out_w, 1, top_k, num_experts, grp, smem);
+        return;
+    }
+    for (uint32_t e = threadIdx.x; e < num_experts; e += blockDim.x) {
+        grp.per_expert_counts[e] = 0u;
+        grp.per_expert_offsets[e] = 0xFFFFFFFFu;
+    }
+    __syncthreads();
+    if (threadIdx.x < top_k) {
+        uint32_t mine = out_idx[threadIdx.x];
+        if (mine >= num_experts) mine = num_experts - 1;
+        uint32_t pos = 0;
+        for (uint32_t r = 0; r < top_k; ++r) {
+            uint32_t other = out_idx[r];
+            if (other >= num_experts) other = num_experts - 1;
+            pos += other < mine ? 1u : 0u;
+        }
+        grp.sorted_pairs[pos] = tf_pair{0u, mine, threadIdx.x, (uint32_t)out_w[threadIdx.x]};
+        grp.per_expert_counts[mine] = 1u;
+        grp.per_expert_offsets[mine] = pos;
+        grp.groups[pos] = tf_group{mine, pos, 1u};
+        grp.chunk_start[pos] = pos;
+        grp.chunk_group[pos] = pos;
+    }
+    if (threadIdx.x == 0) {
+        grp.counters[0] = top_k;
+        grp.counters[1] = top_k;
+        grp.counters[2] = top_k;
+        grp.counters[3] = top_k;
+    }
+}
+
 }  // namespace tf
