@@ -597,7 +597,7 @@ static tf_status block_routed(tf_context* ctx, void* stream, const tf_moe_layer*
                                        layer->router.biases, layer->router.biases_off,
                                        x, 0, TF_FP16, layer->effective_scale, 0, layer->per_expert_scale, 0,
                                        layer->logit_bias, ws->indices, ws->weights, tokens, E, d, K,
-                                       x_stride_elements, &ws->routes, approx, ws->router_ticket);
+                                       x_stride_elements, &ws->routes, approx, (size_t)ws->max_tokens * K * f * 2, ws->router_ticket);
     if (s) return s;
     if (tensor_path) {
         // Prefill-sized block: gather the rows into expert order and run gate/up/GeGLU/down as tcgen05 GEMMs; the
@@ -646,8 +646,14 @@ static bool block_exact(const tf_context* ctx, const tf_moe_layer* l, const tf_w
     return l->d == ws->d && l->f == ws->f && l->fs == ws->fs && l->top_k == ws->top_k && l->num_experts == ws->num_experts && l->pool_layer_base &&
            aligned(l->pool_layer_base, 16) && l->expert_stride % 16 == 0 && l->top_k <= TF_MAX_TOP_K && l->num_experts <= TF_MAX_ROUTER_EXPERTS;
 }
-static bool shared_exact(const tf_context* ctx, const tf_moe_layer* l, uint32_t tokens) {
-    if (ctx->shared_tensorcore_min_set || l->shared_bits == 8 || tokens >= ctx->shared_tensorcore_min_tokens || l->fs > kExactMaxK) return false;
+// The shared expert of a stack's layer for 65 to 255 tokens, whatever the routed experts run on: on the CUDA cores its two launches hold the SMs
+// until 55 us of a layer of 100 tokens, here until 50, and the routed gate/up waits for them. Steps of 30 layers, us: 75 tokens 4122 -> 4027,
+// 90: 4510 -> 4390, 100: 4824 -> 4752, 110: 5512 -> 5374. (The size: as for the routed experts.)
+static bool shared_exact(const tf_context* ctx, const tf_moe_layer* l, const tf_workspace* ws, uint32_t tokens) {
+    if (!ws->x_ext || ctx->tensorcore_min_set || ctx->shared_tensorcore_min_set || l->shared_bits == 8 || tokens <= kF32PartialTokens ||
+        tokens > kExactMaxTokens || tokens >= ctx->shared_tensorcore_min_tokens || (uint64_t)tokens * l->d * l->fs < 1ull << 28 || l->d > kExactMaxK ||
+        l->fs > kExactMaxK)
+        return false;
     const tf_projection* ps[3] = {&l->shared_gate, &l->shared_up, &l->shared_down};
     const uint32_t rows[3] = {l->fs, l->fs, l->d}, cols[3] = {l->d, l->d, l->fs};
     for (int i = 0; i < 3; ++i)
@@ -668,7 +674,7 @@ static bool block_keeps_f32_partials(const tf_context* ctx, const tf_workspace* 
 // is left to the caller, which finds the partials, weights and shared output in the workspace.
 static tf_status block_forward(tf_context* ctx, void* stream, const tf_moe_layer* layer,
                                const void* x, uint32_t x_stride_elements,
-                               void* y, uint32_t y_stride_elements, uint32_t tokens, tf_workspace* ws, bool exact = false) {
+                               void* y, uint32_t y_stride_elements, uint32_t tokens, tf_workspace* ws, bool exact = false, bool exact_shared = false) {
     const char* name = "tf_moe_block_forward";
     TF_REQUIRE(ctx, ctx != nullptr, TF_ERR_INVALID_ARGUMENT, "%s: ctx is NULL", name);
     TF_REQUIRE(ctx, layer && x && ws, TF_ERR_INVALID_ARGUMENT, "%s: NULL argument", name);
@@ -689,7 +695,7 @@ static tf_status block_forward(tf_context* ctx, void* stream, const tf_moe_layer
     TF_CUDA(ctx, cudaStreamWaitEvent(ctx->side_stream, ctx->fork_event, 0));
     const bool tensor_path = tokens >= ctx->tensorcore_min_tokens && ws->tensor_path;
     tf_status s;
-    if (exact && shared_exact(ctx, layer, tokens))
+    if (exact_shared && shared_exact(ctx, layer, ws, tokens))
         s = shared_expert_exact(ctx, ctx->side_stream, x, x_stride_elements, &layer->shared_gate, &layer->shared_up, &layer->shared_down, ws->x_ext,
                                 ws->shared_act, ws->shared_y, tokens);
     else if (layer->shared_bits == 8)
@@ -1049,7 +1055,7 @@ tf_status tf_stack_forward(tf_stack* st, void* stream, void* hidden, uint32_t to
             tf::launch_pdl(tf::residual_rmsnorm_kernel, dim3(tokens), dim3(tf::kRrnThreads), smem, cs, h,
                            l == 0 ? no16 : static_cast<const uint16_t*>(ws->y_block), nw, ws->x_norm, d, st->eps);
         if (tf_status s = tf::check_launch(ctx, "residual_rmsnorm")) return s;
-        if (tf_status s = tf::block_forward(ctx, stream, &st->layers[l], ws->x_norm, d, fold || fold_rows ? nullptr : ws->y_block, d, tokens, ws, exact)) return s;
+        if (tf_status s = tf::block_forward(ctx, stream, &st->layers[l], ws->x_norm, d, fold || fold_rows ? nullptr : ws->y_block, d, tokens, ws, exact, true)) return s;
     }
     if (fold_rows)
         return tf::combine_rows_residual_rmsnorm(ctx, stream, h, ws->partials, ws->weights, ws->inverse_perm, ws->shared_y, nullptr, nullptr, tokens,

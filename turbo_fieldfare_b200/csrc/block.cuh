@@ -75,7 +75,7 @@ tf_status router_block_grouped(tf_context* ctx, void* stream, const void* weight
                                const void* per_expert_scale, uint64_t per_expert_scale_off,
                                const float* logit_bias, uint32_t* out_indices, void* out_weights,
                                uint32_t query_count, uint32_t num_experts, uint32_t d, uint32_t top_k,
-                               uint32_t hidden_stride_elements, const tf_device_routes* routes, void* approx_scratch, uint32_t* ticket);
+                               uint32_t hidden_stride_elements, const tf_device_routes* routes, void* approx_scratch, size_t approx_bytes, uint32_t* ticket);
 // grouped.cu: tf_grouped_moe_batched for a caller that knows the experts' number (it decides the tokens per chunk)
 tf_status grouped_moe_batched(tf_context* ctx, void* stream, const void* hidden, uint64_t hidden_off,
                               uint32_t hidden_stride_elements, const void* pool_layer_base, uint64_t expert_stride,

@@ -11,6 +11,8 @@
 //   logit = xor-butterfly sum over the 32 lanes (offsets 16, 8, 4, 2, 1)
 // which is the reference kernel's per-lane element assignment with the
 // contraction and reduction order fixed.
+#include <algorithm>
+
 #include "router.cuh"
 #include "router_tensor.cuh"
 
@@ -498,12 +500,16 @@ static int tile_router_rows(uint32_t rows, uint32_t slots) {
 
 // Scratch of the two-launch router: (approximate logit, magnitude) per (row, expert), owned by the context and grown
 // on demand. Growing allocates, which a stream that is being captured must not do: the caller then takes the
-// one-launch kernel.
-static bool router_scratch(tf_context* ctx, cudaStream_t st, uint32_t rows, uint32_t num_experts) {
-    const size_t need = (size_t)rows * num_experts * sizeof(float2);
+// one-launch kernel; where it holds fewer planes than `parts`, that is the number of parts.
+static bool router_scratch(tf_context* ctx, cudaStream_t st, uint32_t rows, uint32_t num_experts, uint32_t& parts) {
+    const size_t plane = (size_t)rows * num_experts * sizeof(float2), need = plane * parts;
     if (need <= ctx->router_approx_bytes) return true;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) { cudaGetLastError(); return false; }
+    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        parts = (uint32_t)(ctx->router_approx_bytes / plane);
+        return parts > 0;
+    }
     if (ctx->router_approx) { cudaFree(ctx->router_approx); ctx->router_approx = nullptr; ctx->router_approx_bytes = 0; }
     if (cudaMalloc(&ctx->router_approx, need) != cudaSuccess) { cudaGetLastError(); return false; }
     ctx->router_approx_bytes = need;
@@ -520,7 +526,8 @@ static RouterGroupOut router_group_out(const tf_device_routes* routes) {
 // Scratch of the two-launch router that belongs to the caller's workspace: nothing of the context is shared, so such calls may
 // overlap on several streams (the one-launch kernel for more than kRouterSplitRows rows shares nothing either).
 struct RouterScratch {
-    float2* approx;             // [rows, num_experts]
+    float2* approx;             // [parts][rows, num_experts]
+    size_t bytes;
     unsigned int* ticket;       // zero between calls
 };
 
@@ -547,6 +554,11 @@ static tf_status launch_router(tf_context* ctx, void* stream, const uint8_t* W, 
     auto pp = reinterpret_cast<const uint16_t*>(pes);
     auto wp = reinterpret_cast<uint16_t*>(out_w);
     const bool vec16 = aligned(W, 16) && aligned(hp, 16) && aligned(ep, 16) && d % 16 == 0 && stride % 8 == 0;
+    // Parts of the approximate logits: a chunk of columns each while two rounds of two blocks per SM hold them all, three chunks, whose loads
+    // overlap, beyond that. One chunk, three, all eleven (us): 333 rows 7.5, 17.9, 37.9; 512 rows 14.9, 18.0, 39.0; 800 rows 14.9, 16.9, 38.8;
+    // 1500 rows 23.7, 22.4, 45.6; 4096 rows 47.8, 41.0, 48.5 (and adding the planes takes the re-check 9 us less with three).
+    const uint32_t apx_blocks = (rows + kApxTokens - 1) / kApxTokens * ((num_experts + kApxExperts - 1) / kApxExperts) * (d / kApxChunk);
+    uint32_t parts = apx_blocks <= 4u * (uint32_t)ctx->sm_count ? d / kApxChunk : (d / kApxChunk + 2) / 3;
     if (rows >= 2 && rows <= (uint32_t)kRouterSplitRows && vec16) {
         constexpr int R = 1;          // latency bound: a 64-token step took 4.35 ms with four rows per block, 4.28 with two, 4.16 with one
         auto k = bf ? router_rows_kernel<true, R> : router_rows_kernel<false, R>;
@@ -586,27 +598,30 @@ static tf_status launch_router(tf_context* ctx, void* stream, const uint8_t* W, 
         return check_launch(ctx, name);
     } else if ((own || rows >= ctx->router_tensorcore_min_rows) && !out_logits && vec16 && d % kApxChunk == 0 && aligned(S, 8) && aligned(B, 8) &&
                num_experts <= TF_MAX_ROUTER_EXPERTS && top_k <= (uint32_t)kWarp && top_k <= num_experts &&
-               router_recheck_smem_bytes(d, num_experts, kRecheckWarps) <= 205 * 1024 && (own || router_scratch(ctx, st, rows, num_experts))) {
+               router_recheck_smem_bytes(d, num_experts, kRecheckWarps) <= 205 * 1024 && (own || router_scratch(ctx, st, rows, num_experts, parts))) {
         // logits on the tensor cores, then the canonical logits of the few experts that can reach the top k
         float2* approx = own ? own->approx : static_cast<float2*>(ctx->router_approx);
         const uint32_t sms = (uint32_t)ctx->sm_count;
-        // Few rows: blocks of 8 tokens x 32 experts, all of whose operands are in flight at once, as long as they make at
-        // most four rounds of the SMs (100 blocks, 200 rows: 11 us; 168 blocks, 333 rows: 17 us; the 16 x 128 blocks take 25 us there
-        // and 41 us at 4096 rows).
+        // Few rows: blocks of 8 tokens x 32 experts with all of their operands in flight at once, while they make one round of the SMs: 200 rows,
+        // 100 blocks, 9.8 us. Two rounds (333 rows, 168 blocks) take 16.6, the parts of the other kernel 7.5. (Those take 6.2 us at 200 rows,
+        // but steps of 66 to 255 tokens gained nothing or lost 0.5 %, and prefills of 256 took 2.7 % longer.)
         const size_t smem_few = router_approx_few_smem_bytes(d);
         const dim3 grid_few((rows + kFewTokens - 1) / kFewTokens, (num_experts + kFewExperts - 1) / kFewExperts);
-        if (smem_few <= 224 * 1024 && grid_few.x * grid_few.y <= 4 * sms) {
+        if (smem_few <= 224 * 1024 && grid_few.x * grid_few.y <= sms) {
+            parts = 1;
             auto ka = bf ? router_approx_few_kernel<true> : router_approx_few_kernel<false>;
             static DeviceSmemCache configured_few[2];
             if (tf_status s = ensure_dynamic_smem(ctx, ka, configured_few[bf ? 1 : 0], smem_few)) return s;
             launch_pdl(ka, grid_few, dim3(kFewThreads), smem_few, st, W, Sp, Bp, hp, stride, ep, approx, rows, num_experts, d);
         } else {
+            if (own) parts = std::max(1u, std::min(parts, (uint32_t)(own->bytes / ((size_t)rows * num_experts * sizeof(float2)))));
+            const uint32_t chunks = (d / kApxChunk + parts - 1) / parts;
+            parts = (d / kApxChunk + chunks - 1) / chunks;
             auto ka = bf ? router_approx_kernel<true> : router_approx_kernel<false>;
             static DeviceSmemCache configured_approx[2];
-            const size_t smem_a = router_approx_smem_bytes();
-            if (tf_status s = ensure_dynamic_smem(ctx, ka, configured_approx[bf ? 1 : 0], smem_a)) return s;
-            launch_pdl(ka, dim3((rows + kApxTokens - 1) / kApxTokens, (num_experts + kApxExperts - 1) / kApxExperts), dim3(kApxThreads),
-                       smem_a, st, W, Sp, Bp, hp, stride, ep, approx, rows, num_experts, d);
+            if (tf_status s = ensure_dynamic_smem(ctx, ka, configured_approx[bf ? 1 : 0], router_approx_smem_bytes(2))) return s;
+            launch_pdl(ka, dim3((rows + kApxTokens - 1) / kApxTokens, (num_experts + kApxExperts - 1) / kApxExperts, parts), dim3(kApxThreads),
+                       router_approx_smem_bytes(chunks), st, W, Sp, Bp, hp, stride, ep, approx, rows, num_experts, d, chunks);
         }
         if (tf_status s = check_launch(ctx, name)) return s;
         constexpr int kProductionGroups = 2816 / kGroup;          // the recheck keeps an expert's 44 code words in registers
@@ -616,7 +631,7 @@ static tf_status launch_router(tf_context* ctx, void* stream, const uint8_t* W, 
         // (Only the form with a token per block can group.)
         const int which = rows <= 2 * sms || (own && routes) ? 3 : rows <= 4 * sms ? 2 : rows <= 8 * sms ? 1 : 0;
         void (*kr)(const uint8_t*, const uint16_t*, const uint16_t*, const uint16_t*, uint32_t, const uint16_t*, const uint16_t*, const float*,
-                   const float2*, uint32_t*, uint16_t*, unsigned int*, RouterGroupOut, uint32_t, uint32_t, uint32_t, uint32_t);
+                   const float2*, uint32_t, uint32_t*, uint16_t*, unsigned int*, RouterGroupOut, uint32_t, uint32_t, uint32_t, uint32_t);
 #define TF_RECHECK(WPT) kr = fixed ? (bf ? router_recheck_kernel<true, kProductionGroups, WPT> : router_recheck_kernel<false, kProductionGroups, WPT>) \
                                    : (bf ? router_recheck_kernel<true, 0, WPT> : router_recheck_kernel<false, 0, WPT>)
         if (which == 3) TF_RECHECK(8);
@@ -635,7 +650,7 @@ static tf_status launch_router(tf_context* ctx, void* stream, const uint8_t* W, 
         static DeviceSmemCache configured_recheck[4][4];
         if (tf_status s = ensure_dynamic_smem(ctx, kr, configured_recheck[which][(bf ? 1 : 0) + (fixed ? 2 : 0)], smem_r)) return s;
         launch_pdl(kr, dim3((rows + per_block - 1) / per_block), dim3(kRecheckWarps * kWarp), smem_r, st, W, Sp, Bp, hp, stride,
-                   ep, pp, logit_bias, static_cast<const float2*>(approx), out_idx, wp, own ? own->ticket : nullptr, grp, rows, num_experts, d, top_k);
+                   ep, pp, logit_bias, static_cast<const float2*>(approx), parts, out_idx, wp, own ? own->ticket : nullptr, grp, rows, num_experts, d, top_k);
         if (grouped) *grouped = own && routes;
     } else if (rows >= 256 && a2 && (size_t)kTileRouterRows * (d + num_experts) * 4 <= 100 * 1024) {
         const int R = tile_router_rows(rows, (uint32_t)ctx->sm_count * 2u);
@@ -673,7 +688,7 @@ tf_status router_block_grouped(tf_context* ctx, void* stream, const void* weight
                                const void* per_expert_scale, uint64_t per_expert_scale_off,
                                const float* logit_bias, uint32_t* out_indices, void* out_weights,
                                uint32_t query_count, uint32_t num_experts, uint32_t d, uint32_t top_k,
-                               uint32_t hidden_stride_elements, const tf_device_routes* routes, void* approx_scratch, uint32_t* ticket) {
+                               uint32_t hidden_stride_elements, const tf_device_routes* routes, void* approx_scratch, size_t approx_bytes, uint32_t* ticket) {
     const char* name = "tf_router_gemma4_block_grouped";
     TF_REQUIRE(ctx, weights && scales && biases && hidden && effective_scale && per_expert_scale && out_indices && out_weights,
                TF_ERR_INVALID_ARGUMENT, "%s: NULL buffer", name);
@@ -685,7 +700,7 @@ tf_status router_block_grouped(tf_context* ctx, void* stream, const void* weight
     TF_REQUIRE(ctx, d > 0 && d % tf::kGroup == 0 && hidden_stride_elements >= d, TF_ERR_INVALID_ARGUMENT,
                "%s: D must be a multiple of 64 and the stride at least D", name);
     TF_REQUIRE(ctx, hidden_dtype == TF_FP16 || hidden_dtype == TF_BF16, TF_ERR_INVALID_ARGUMENT, "%s: bad hidden dtype", name);
-    const RouterScratch own{static_cast<float2*>(approx_scratch), ticket};
+    const RouterScratch own{static_cast<float2*>(approx_scratch), approx_bytes, ticket};
     const bool use_own = approx_scratch && ticket && query_count > (uint32_t)kRouterSplitRows && query_count <= kRouterFusedGroupRows &&
                          (ctx->router_block_min_rows ? query_count >= ctx->router_block_min_rows : num_experts * d > kRouterTwoLaunchCodes);
     bool grouped = false;
@@ -772,7 +787,7 @@ tf_status tf_router_gemma4_block_grouped(tf_context* ctx, void* stream, const vo
                TF_ERR_INVALID_ARGUMENT, "%s: NULL routes buffer", name);
     return tf::router_block_grouped(ctx, stream, weights, weights_off, scales, scales_off, biases, biases_off, hidden, hidden_off, hidden_dtype,
                                     effective_scale, effective_scale_off, per_expert_scale, per_expert_scale_off, logit_bias, out_indices,
-                                    out_weights, query_count, num_experts, d, top_k, hidden_stride_elements, routes, nullptr, nullptr);
+                                    out_weights, query_count, num_experts, d, top_k, hidden_stride_elements, routes, nullptr, 0, nullptr);
 }
 
 }  // extern "C"

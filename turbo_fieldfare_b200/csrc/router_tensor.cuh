@@ -37,8 +37,8 @@ constexpr float kApxPrescale = 1024.0f;            // activations are split as x
 constexpr float kApxRelError = 1.220703125e-04f;   // 2^-13
 constexpr int kRecheckWarps = 8;                   // warps per block of router_recheck_kernel
 
-__host__ __device__ inline size_t router_approx_smem_bytes() {
-    return 2 * (size_t)kApxExperts * kApxWPitch + 2 * (size_t)kApxTokens * kApxXPitch + 2 * 4 * kApxTokens * sizeof(float);
+__host__ __device__ inline size_t router_approx_smem_bytes(uint32_t chunks) {        // one weight buffer for parts of one chunk
+    return (chunks > 1 ? 2 : 1) * (size_t)kApxExperts * kApxWPitch + 2 * (size_t)kApxTokens * kApxXPitch + 2 * 4 * kApxTokens * sizeof(float);
 }
 __host__ __device__ inline size_t router_recheck_smem_bytes(uint32_t d, uint32_t num_experts, uint32_t tokens_per_block) {
     return ((size_t)tokens_per_block * (((size_t)d + num_experts) * sizeof(float) + num_experts * sizeof(uint16_t)) + 15) & ~(size_t)15;
@@ -65,18 +65,28 @@ __device__ __forceinline__ uint32_t bytes_to_half2(uint32_t word, uint32_t sel) 
     return *reinterpret_cast<const uint32_t*>(&v);
 }
 
+// Activations behind a wait in the middle of a kernel: a plain load through a const __restrict__ pointer counts as invariant and may be moved
+// ahead of the wait (rows of the layer before were read).
+__device__ __forceinline__ uint4 load_row_words(const uint16_t* p) {
+    uint4 v;
+    asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    return v;
+}
+
 // out[token][expert] = (approximate logit without the logit bias, magnitude), both in units of x (not x * 2^10).
-// Grid: (ceil(rows / 16), ceil(num_experts / 128)). Column k of an MMA step is mapped to the matrix column
+// Grid: (ceil(rows / 16), ceil(num_experts / 128), parts); a part sums `chunks` chunks of 256 columns into its own plane of out, and the
+// re-check adds the planes. A chunk alone is a chain of latencies (rows, conversion, MMAs, store), eleven in a row took 41 us at 512 rows
+// with 32 blocks; see launch_router for the split. The weights, scales and biases are requested before the previous kernel has ended. Column k of an MMA step is mapped to the matrix column
 // 16 t + 4 step + {0, 1} (k = 2 t + {0, 1}) and 16 t + 4 step + {2, 3} (k = 2 t + 8 + {0, 1}) of the group, for both
 // operands, so a thread's 16 weight bytes and 16 activation values of a group are contiguous.
 template <bool X_BF16>
 __global__ void __launch_bounds__(kApxThreads, 2)
 router_approx_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S, const uint16_t* __restrict__ B,
                      const uint16_t* __restrict__ hidden, uint32_t hidden_stride, const uint16_t* __restrict__ eff,
-                     float2* __restrict__ out, uint32_t rows, uint32_t num_experts, uint32_t d) {
+                     float2* __restrict__ out, uint32_t rows, uint32_t num_experts, uint32_t d, uint32_t chunks) {
     extern __shared__ __align__(16) uint8_t smem[];
-    uint8_t* Wc0 = smem;                                                   // [2][128][kApxWPitch]
-    uint8_t* Hi = Wc0 + 2 * (size_t)kApxExperts * kApxWPitch;             // [16][kApxXPitch]
+    uint8_t* Wc0 = smem;                                                   // [2 or 1][128][kApxWPitch]
+    uint8_t* Hi = Wc0 + (chunks > 1 ? 2 : 1) * (size_t)kApxExperts * kApxWPitch;             // [16][kApxXPitch]
     uint8_t* Lo = Hi + (size_t)kApxTokens * kApxXPitch;
     float* XS = reinterpret_cast<float*>(Lo + (size_t)kApxTokens * kApxXPitch);   // [4 groups][16 tokens]: sum of x * 2^10
     float* XA = XS + 4 * kApxTokens;                                       // the same of |x * 2^10| (+ the split's absolute part)
@@ -85,8 +95,9 @@ router_approx_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__
     const uint32_t groups = d / kGroup;
     const uint32_t last = num_experts - 1;
     const uint32_t e_lo = min(e0 + warp * 16 + g, last), e_hi = min(e0 + warp * 16 + g + 8, last);   // rows past the end repeat the last one
+    const uint32_t c_first = blockIdx.z * chunks * kApxChunk, c_end = min(c_first + chunks * kApxChunk, d);
+    out += (size_t)blockIdx.z * rows * num_experts;
     pdl_launch_dependents();
-    pdl_wait();
     float acc[2][4] = {}, mag[2][4] = {};
     // The next chunk's weight codes (cp.async into the other buffer) and activation rows (registers) are requested
     // before the current chunk is multiplied.
@@ -105,13 +116,24 @@ router_approx_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const uint32_t tok = tok0 + warp + 8 * h;
-            hreg[h] = tok < rows ? *reinterpret_cast<const uint4*>(hidden + (size_t)tok * hidden_stride + c0 + lane * 8) : make_uint4(0u, 0u, 0u, 0u);
+            hreg[h] = tok < rows ? load_row_words(hidden + (size_t)tok * hidden_stride + c0 + lane * 8) : make_uint4(0u, 0u, 0u, 0u);
         }
     };
-    request_weights(0, Wc0);
-    request_rows(0);
+    // scales and biases of a chunk's four groups for this thread's two expert rows (8-byte aligned: groups % 4 == 0)
+    uint2 s_lo, s_hi, b_lo, b_hi;
+    auto request_scales = [&](uint32_t c0) {
+        const uint32_t gq = c0 / kGroup;
+        s_lo = __ldg(reinterpret_cast<const uint2*>(S + (size_t)e_lo * groups + gq));
+        s_hi = __ldg(reinterpret_cast<const uint2*>(S + (size_t)e_hi * groups + gq));
+        b_lo = __ldg(reinterpret_cast<const uint2*>(B + (size_t)e_lo * groups + gq));
+        b_hi = __ldg(reinterpret_cast<const uint2*>(B + (size_t)e_hi * groups + gq));
+    };
+    request_weights(c_first, Wc0);
+    request_scales(c_first);
+    pdl_wait();                                  // the activations
+    request_rows(c_first);
     uint32_t ci = 0;
-    for (uint32_t c0 = 0; c0 < d; c0 += kApxChunk, ++ci) {
+    for (uint32_t c0 = c_first; c0 < c_end; c0 += kApxChunk, ++ci) {
         uint8_t* Wc = Wc0 + (size_t)(ci & 1u) * kApxExperts * kApxWPitch;
         __syncthreads();                         // the previous chunk's fragments have been read
         // activations: a warp stages the 256 columns of tokens `warp` and `warp + 8`, eight columns per lane (zero bits
@@ -155,18 +177,13 @@ router_approx_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__
         }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
-        if (c0 + kApxChunk < d) {
+        if (c0 + kApxChunk < c_end) {
             request_weights(c0 + kApxChunk, Wc0 + (size_t)((ci + 1u) & 1u) * kApxExperts * kApxWPitch);
             request_rows(c0 + kApxChunk);
         }
-        // scales and biases of the chunk's four groups for this thread's two expert rows (8-byte aligned: groups % 4 == 0)
-        const uint32_t gq = c0 / kGroup;
-        const uint2 s_lo = *reinterpret_cast<const uint2*>(S + (size_t)e_lo * groups + gq);
-        const uint2 s_hi = *reinterpret_cast<const uint2*>(S + (size_t)e_hi * groups + gq);
-        const uint2 b_lo = *reinterpret_cast<const uint2*>(B + (size_t)e_lo * groups + gq);
-        const uint2 b_hi = *reinterpret_cast<const uint2*>(B + (size_t)e_hi * groups + gq);
-        const uint32_t slw[2] = {s_lo.x, s_lo.y}, shw[2] = {s_hi.x, s_hi.y}, blw[2] = {b_lo.x, b_lo.y}, bhw[2] = {b_hi.x, b_hi.y};
-#pragma unroll
+        const uint2 sc_lo = s_lo, sc_hi = s_hi, bc_lo = b_lo, bc_hi = b_hi;
+        if (c0 + kApxChunk < c_end) request_scales(c0 + kApxChunk);
+#pragma unroll 1
         for (int gi = 0; gi < 4; ++gi) {
             const uint4 a_lo = *reinterpret_cast<const uint4*>(Wc + (size_t)(warp * 16 + g) * kApxWPitch + gi * 64 + t * 16);
             const uint4 a_hi = *reinterpret_cast<const uint4*>(Wc + (size_t)(warp * 16 + g + 8) * kApxWPitch + gi * 64 + t * 16);
@@ -177,9 +194,13 @@ router_approx_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__
                 af[s][0] = bytes_to_half2(alw[s], 0x5140u); af[s][1] = bytes_to_half2(ahw[s], 0x5140u);
                 af[s][2] = bytes_to_half2(alw[s], 0x7362u); af[s][3] = bytes_to_half2(ahw[s], 0x7362u);
             }
-            float P[2][4] = {};
+            const uint32_t sh = (gi & 1) * 16;
+            const float sl = bf16_bits_to_float((uint16_t)((gi < 2 ? sc_lo.x : sc_lo.y) >> sh)), sH = bf16_bits_to_float((uint16_t)((gi < 2 ? sc_hi.x : sc_hi.y) >> sh));
+            const float bL = bf16_bits_to_float((uint16_t)((gi < 2 ? bc_lo.x : bc_lo.y) >> sh)), bH = bf16_bits_to_float((uint16_t)((gi < 2 ? bc_hi.x : bc_hi.y) >> sh));
+            const float ml = fmaf(255.0f, fabsf(sl), fabsf(bL)), mh = fmaf(255.0f, fabsf(sH), fabsf(bH));
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt) {
+                float P[4] = {};
                 const size_t off = (size_t)(nt * 8 + g) * kApxXPitch + (size_t)(gi * 64 + t * 16) * 2;
                 const uint4 h0 = *reinterpret_cast<const uint4*>(Hi + off), h1 = *reinterpret_cast<const uint4*>(Hi + off + 16);
                 const uint4 l0 = *reinterpret_cast<const uint4*>(Lo + off), l1 = *reinterpret_cast<const uint4*>(Lo + off + 16);
@@ -187,22 +208,15 @@ router_approx_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__
                 const uint32_t bl[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
 #pragma unroll
                 for (int s = 0; s < 4; ++s) {
-                    mma_f16_f32(P[nt], af[s][0], af[s][1], af[s][2], af[s][3], bh[2 * s], bh[2 * s + 1]);
-                    mma_f16_f32(P[nt], af[s][0], af[s][1], af[s][2], af[s][3], bl[2 * s], bl[2 * s + 1]);
+                    mma_f16_f32(P, af[s][0], af[s][1], af[s][2], af[s][3], bh[2 * s], bh[2 * s + 1]);
+                    mma_f16_f32(P, af[s][0], af[s][1], af[s][2], af[s][3], bl[2 * s], bl[2 * s + 1]);
                 }
-            }
-            const uint32_t sh = (gi & 1) * 16;
-            const float sl = bf16_bits_to_float((uint16_t)(slw[gi >> 1] >> sh)), sH = bf16_bits_to_float((uint16_t)(shw[gi >> 1] >> sh));
-            const float bL = bf16_bits_to_float((uint16_t)(blw[gi >> 1] >> sh)), bH = bf16_bits_to_float((uint16_t)(bhw[gi >> 1] >> sh));
-            const float ml = fmaf(255.0f, fabsf(sl), fabsf(bL)), mh = fmaf(255.0f, fabsf(sH), fabsf(bH));
-#pragma unroll
-            for (int nt = 0; nt < 2; ++nt) {
                 const float2 xs = *reinterpret_cast<const float2*>(XS + gi * kApxTokens + nt * 8 + 2 * t);
                 const float2 xa = *reinterpret_cast<const float2*>(XA + gi * kApxTokens + nt * 8 + 2 * t);
-                acc[nt][0] = fmaf(sl, P[nt][0], fmaf(bL, xs.x, acc[nt][0]));
-                acc[nt][1] = fmaf(sl, P[nt][1], fmaf(bL, xs.y, acc[nt][1]));
-                acc[nt][2] = fmaf(sH, P[nt][2], fmaf(bH, xs.x, acc[nt][2]));
-                acc[nt][3] = fmaf(sH, P[nt][3], fmaf(bH, xs.y, acc[nt][3]));
+                acc[nt][0] = fmaf(sl, P[0], fmaf(bL, xs.x, acc[nt][0]));
+                acc[nt][1] = fmaf(sl, P[1], fmaf(bL, xs.y, acc[nt][1]));
+                acc[nt][2] = fmaf(sH, P[2], fmaf(bH, xs.x, acc[nt][2]));
+                acc[nt][3] = fmaf(sH, P[3], fmaf(bH, xs.y, acc[nt][3]));
                 mag[nt][0] = fmaf(ml, xa.x, mag[nt][0]);
                 mag[nt][1] = fmaf(ml, xa.y, mag[nt][1]);
                 mag[nt][2] = fmaf(mh, xa.x, mag[nt][2]);
@@ -460,18 +474,33 @@ __device__ __forceinline__ float2 router_logits_staged(const uint8_t* codes_a, c
 // largest lower bound. N: experts per lane. (A list: warps that took their candidates off bit masks, each skipping those of the token's
 // other warps, spent up to 20 000 clocks on that at eight warps per token.)
 template <int N>
-__device__ __forceinline__ uint32_t router_candidates(const float2* __restrict__ approx_row, const float* __restrict__ logit_bias,
+__device__ __forceinline__ uint32_t router_candidates(const float2* __restrict__ approx_row, uint32_t parts, size_t part_stride, const float* __restrict__ logit_bias,
                                                       uint32_t num_experts, uint32_t top_k, int lane, uint16_t* list /* shared */) {
     float upper[N];
     uint32_t key[N];
     bool bad = false;
+    float2 sum[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) sum[j] = (uint32_t)(lane + j * kWarp) < num_experts ? approx_row[lane + j * kWarp] : make_float2(0.0f, 0.0f);
+    if (parts > 1) {
+#pragma unroll 5
+        for (uint32_t p = 1; p < parts; ++p) {
+#pragma unroll
+            for (int j = 0; j < N; ++j) {
+                if ((uint32_t)(lane + j * kWarp) < num_experts) {
+                    const float2 more = approx_row[p * part_stride + lane + j * kWarp];
+                    sum[j].x += more.x; sum[j].y += more.y;
+                }
+            }
+        }
+    }
 #pragma unroll
     for (int j = 0; j < N; ++j) {
         const uint32_t e = lane + j * kWarp;
         upper[j] = -INFINITY;
         key[j] = 0u;
         if (e < num_experts) {
-            const float2 am = approx_row[e];
+            const float2 am = sum[j];
             float v = am.x;
             if (!isfinite(am.x) || !isfinite(am.y)) bad = true;
             if (logit_bias) v = __fadd_rn(v, logit_bias[e]);
@@ -526,7 +555,7 @@ __global__ void __launch_bounds__(kRecheckWarps * kWarp, 2)
 router_recheck_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S, const uint16_t* __restrict__ B,
                       const uint16_t* __restrict__ hidden, uint32_t hidden_stride, const uint16_t* __restrict__ eff,
                       const uint16_t* __restrict__ per_expert_scale, const float* __restrict__ logit_bias,
-                      const float2* __restrict__ approx, uint32_t* out_idx, uint16_t* out_w, unsigned int* ticket, const RouterGroupOut grp,
+                      const float2* __restrict__ approx, uint32_t parts, uint32_t* out_idx, uint16_t* out_w, unsigned int* ticket, const RouterGroupOut grp,
                       uint32_t rows, uint32_t num_experts, uint32_t d, uint32_t top_k) {
     extern __shared__ __align__(16) uint8_t smem[];
     constexpr int kTokens = kRecheckWarps / WPT;                    // tokens per block
@@ -566,8 +595,8 @@ router_recheck_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict_
     // (every warp of a token writes the same list)
     uint16_t* list = reinterpret_cast<uint16_t*>(reinterpret_cast<float*>(smem) + (size_t)kTokens * (d + num_experts)) + (size_t)slot * num_experts;
     const float2* approx_row = approx + (size_t)row * num_experts;
-    const uint32_t candidates = num_experts <= 4u * kWarp ? router_candidates<4>(approx_row, logit_bias, num_experts, top_k, lane, list)
-                                                          : router_candidates<TF_MAX_ROUTER_EXPERTS / kWarp>(approx_row, logit_bias, num_experts, top_k, lane, list);
+    const uint32_t candidates = num_experts <= 4u * kWarp ? router_candidates<4>(approx_row, parts, (size_t)rows * num_experts, logit_bias, num_experts, top_k, lane, list)
+                                                          : router_candidates<TF_MAX_ROUTER_EXPERTS / kWarp>(approx_row, parts, (size_t)rows * num_experts, logit_bias, num_experts, top_k, lane, list);
     if (WPT == 1) __syncwarp(); else __syncthreads();             // the row's activations and the cleared scores
     // this warp's candidates: every WPT-th one
     uint32_t next = part;
