@@ -47,8 +47,9 @@ def test_router_in_parts_equals_the_one_launch_router(tf_ctx, rows, experts, d, 
     assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
 
 
-@pytest.mark.parametrize("tokens", [300, 880])
-def test_stacks_route_on_the_rows_of_their_own_layer(tf_ctx, tokens):
+# up to 255 tokens the re-check groups, too: pairs that fill no round of 32 to a warp, and all of its counters
+@pytest.mark.parametrize("tokens,experts", [(66, 256), (131, 200), (255, 20), (255, 256), (300, 64), (880, 64)])
+def test_stacks_route_on_the_rows_of_their_own_layer(tf_ctx, tokens, experts):
     import torch
     from turbo_fieldfare_b200.kernels import TurboContext
     from turbo_fieldfare_b200.stack import MoEStack
@@ -57,7 +58,7 @@ def test_stacks_route_on_the_rows_of_their_own_layer(tf_ctx, tokens):
     for threshold in (65, 0xFFFFFFFF):
         ctx = TurboContext(0)
         ctx.set_router_tensorcore_min_rows(threshold)
-        stack = MoEStack(ctx, layers=4, d=2816, f=128, fs=128, num_experts=64, top_k=8, seed=3, align=256)
+        stack = MoEStack(ctx, layers=4, d=2816, f=128, fs=128, num_experts=experts, top_k=8, seed=3, align=256)
         try:
             ws = stack.workspace(tokens)
             for _ in range(1 if out else 20):

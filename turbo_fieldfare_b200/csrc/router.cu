@@ -644,7 +644,7 @@ static tf_status launch_router(tf_context* ctx, void* stream, const uint8_t* W, 
         RouterGroupOut grp{};
         if (own && routes) {
             grp = router_group_out(routes);
-            const size_t need = router_group_smem_bytes(rows * top_k, num_experts, true);
+            const size_t need = router_group_rows_smem_bytes(rows * top_k, num_experts);
             if (need > smem_r) smem_r = need;
         }
         static DeviceSmemCache configured_recheck[4][4];
@@ -676,8 +676,7 @@ static tf_status launch_router(tf_context* ctx, void* stream, const uint8_t* W, 
 // tf_router_gemma4_block_grouped; approx_scratch ([query_count, num_experts] pairs of floats) and ticket (a zero word), when
 // given, belong to the caller's workspace: blocks of 65 to kRouterFusedGroupRows rows then route in two launches, the second of
 // which groups them (the block that finishes the last row does it). One block per row computes every canonical logit there
-// otherwise: 168 us and a grouping launch against 11 + 27 for 200 rows (15 of the 27 are the re-check, the rest its last block's
-// grouping; 11 + 36 before the candidate list and the grouping's thread per expert). Larger blocks group with launches of their own, which many SMs share; nothing between the two was measured.
+// otherwise: 168 us and a grouping launch against 10 + 27 for 200 rows. Larger blocks group with launches of their own, which many SMs share; nothing between the two was measured.
 // The one launch grows with experts * D and the two hardly do. Blocks of 65, 130 and 255 tokens gain from two by, in us: 16 x 256 -13,
 // -16, -17; 32 x 1024 -1, -3, -6; 64 x 768 6, 5, 0; 128 x 512 0, -3, -5; 64 x 1024 13, 11, 8; 32 x 2816 20, 20, 18; 128 x 1024 43, 43, 41.
 constexpr uint32_t kRouterTwoLaunchCodes = 65536;

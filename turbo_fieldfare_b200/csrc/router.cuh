@@ -140,7 +140,7 @@ __host__ __device__ inline size_t router_group_smem_bytes(uint32_t n_pairs, uint
     return (size_t)num_experts * nw * 4 + (counted ? (size_t)((num_experts * nw + 1) / 2) * 4 : 0) + (size_t)num_experts * 2 * 4 + (size_t)n_pairs * 4 + 96 * 4 + (size_t)((n_pairs + 1) / 2) * 4;
 }
 
-// COUNTED (the few-row router and the re-check): the counts before every bitmap word are taken first, a thread per expert (a thread
+// COUNTED (the few-row router): the counts before every bitmap word are taken first, a thread per expert (a thread
 // per pair that adds up the words before its own took 20 us for 1600 pairs). Otherwise (one block per row) the words before a
 // pair's own are added up on the spot.
 template <bool COUNTED>

@@ -546,6 +546,113 @@ __device__ __forceinline__ uint32_t router_candidates(const float2* __restrict__
     return count;
 }
 
+// The grouping of the re-check's last block, up to a few thousand pairs: a warp takes consecutive pairs, 32 to a round, whose lanes find their
+// rank among the round's pairs of the same expert with match.any; the first of them adds their number to the warp's count of the expert. A
+// thread per expert then turns the counts into starts. Latency bounds it. (group_routes_in_block, whose bitmaps have rows of 64 words at 255
+// tokens of top 8, all in one bank: 255 rows 42 -> 30 us for the launch, 200 rows 31 -> 27, 70 rows 19 -> 16.5; a step of 255 tokens
+// 6177 -> 5955. The few-row router stays with those: up to 11 tokens it took 1 to 3 % longer with this.)
+constexpr uint32_t kGroupRowsWarps = kRecheckWarps;
+__host__ __device__ inline size_t router_group_rows_smem_bytes(uint32_t n_pairs, uint32_t num_experts) {
+    return (size_t)num_experts * (kGroupRowsWarps + 1) * 4 + (size_t)n_pairs * 4 + 3 * kGroupRowsWarps * 4 + (size_t)((n_pairs + 1) / 2) * 4;
+}
+__device__ __forceinline__ void group_rows_in_block(const uint32_t* __restrict__ idx, const uint16_t* __restrict__ w, uint32_t T, uint32_t K,
+                                                    uint32_t E, const RouterGroupOut& out, uint8_t* smem) {
+    constexpr uint32_t kAtOnce = 8;                              // rounds whose ids are requested together
+    const uint32_t n = T * K, rounds = (n + kGroupRowsWarps * kWarp - 1) / (kGroupRowsWarps * kWarp);
+    uint32_t* counts = reinterpret_cast<uint32_t*>(smem);        // [warp][E]: the warp's pairs of the expert, then where they start
+    uint32_t* offs = counts + (size_t)kGroupRowsWarps * E;       // [E]
+    uint32_t* exs = offs + E;                                    // [n]: expert | rank among the warp's pairs of it << 16
+    uint32_t* wtot = exs + n;                                    // [3][warps]
+    uint16_t* wts = reinterpret_cast<uint16_t*>(wtot + 3 * kGroupRowsWarps);      // [n]
+    const uint32_t lane = threadIdx.x % kWarp, warp = threadIdx.x / kWarp, first = warp * rounds * kWarp + lane;
+    uint32_t* mine = counts + (size_t)warp * E;
+    for (uint32_t i = lane; i < E; i += kWarp) mine[i] = 0;
+    __syncwarp();
+    for (uint32_t r0 = 0; r0 < rounds; r0 += kAtOnce) {
+        uint32_t ids[kAtOnce], wt[kAtOnce];
+#pragma unroll
+        for (uint32_t j = 0; j < kAtOnce; ++j) {                 // written by other blocks of this launch
+            const uint32_t i = first + (r0 + j) * kWarp;
+            const bool in = r0 + j < rounds && i < n;
+            ids[j] = in ? __ldcg(idx + i) : 0xFFFFFFFFu;
+            wt[j] = in ? (uint32_t)__ldcg(w + i) : 0u;
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < kAtOnce; ++j) {
+            if (r0 + j < rounds) {
+                const uint32_t i = first + (r0 + j) * kWarp;
+                uint32_t ex = ids[j];
+                if (ex != 0xFFFFFFFFu && ex >= E) ex = E - 1;    // min(id, E-1): Runtime/Inference/RealForwardRunner.swift:955
+                const uint32_t peers = __match_any_sync(kFullMask, ex);
+                const uint32_t rank = __popc(peers & ((1u << lane) - 1u));
+                uint32_t before = 0;
+                if (ex != 0xFFFFFFFFu && rank == 0) {
+                    before = mine[ex];
+                    mine[ex] = before + __popc(peers);
+                }
+                before = __shfl_sync(kFullMask, before, __ffs(peers) - 1);
+                if (i < n) {
+                    exs[i] = ex == 0xFFFFFFFFu ? ex : ex | (before + rank) << 16;
+                    wts[i] = (uint16_t)wt[j];
+                }
+                __syncwarp();
+            }
+        }
+    }
+    __syncthreads();
+    // a thread per expert: the warps' counts to starts, exclusive scans over the experts (pairs, non-empty groups, chunks) of 32 to a warp
+    static_assert(TF_MAX_ROUTER_EXPERTS <= kGroupRowsWarps * kWarp, "a thread per expert");
+    const uint32_t e = threadIdx.x;
+    uint32_t cnt = 0;
+    if (e < E) {
+        uint32_t c[kGroupRowsWarps];
+#pragma unroll
+        for (uint32_t v = 0; v < kGroupRowsWarps; ++v) c[v] = counts[(size_t)v * E + e];
+#pragma unroll
+        for (uint32_t v = 0; v < kGroupRowsWarps; ++v) {
+            counts[(size_t)v * E + e] = cnt;
+            cnt += c[v];
+        }
+    }
+    const uint32_t nch = (cnt + (uint32_t)kChunkTokens - 1) / (uint32_t)kChunkTokens;
+    uint32_t i_off = cnt, i_g = cnt ? 1u : 0u, i_ch = nch;
+#pragma unroll
+    for (int o = 1; o < kWarp; o <<= 1) {
+        const uint32_t a = __shfl_up_sync(kFullMask, i_off, o), b2 = __shfl_up_sync(kFullMask, i_g, o), c = __shfl_up_sync(kFullMask, i_ch, o);
+        if ((int)lane >= o) { i_off += a; i_g += b2; i_ch += c; }
+    }
+    if (lane == kWarp - 1) { wtot[warp] = i_off; wtot[kGroupRowsWarps + warp] = i_g; wtot[2 * kGroupRowsWarps + warp] = i_ch; }
+    __syncthreads();
+    uint32_t off = i_off - cnt, gi = i_g - (cnt ? 1u : 0u), ch = i_ch - nch;
+#pragma unroll
+    for (uint32_t v = 0; v < kGroupRowsWarps; ++v)
+        if (v < warp) { off += wtot[v]; gi += wtot[kGroupRowsWarps + v]; ch += wtot[2 * kGroupRowsWarps + v]; }
+    if (e < E) {
+        offs[e] = off;
+        out.per_expert_counts[e] = cnt;
+        out.per_expert_offsets[e] = cnt ? off : 0xFFFFFFFFu;
+        if (cnt) {
+            out.groups[gi] = tf_group{e, off, cnt};
+            out.chunk_start[gi] = ch;
+            for (uint32_t j = 0; j < nch; ++j) out.chunk_group[ch + j] = gi;
+        }
+    }
+    if (e == E - 1) {
+        out.counters[0] = gi + (cnt ? 1u : 0u);
+        out.counters[1] = ch + nch;
+        out.counters[2] = n;
+        out.counters[3] = off + cnt;
+    }
+    __syncthreads();
+    for (uint32_t r = 0; r < rounds; ++r) {
+        const uint32_t i = first + r * kWarp;
+        if (i >= n) break;
+        const uint32_t v = exs[i], ex = v & 0xFFFFu;
+        if (v == 0xFFFFFFFFu) continue;
+        out.sorted_pairs[offs[ex] + mine[ex] + (v >> 16)] = tf_pair{i / K, ex, i % K, (uint32_t)wts[i]};
+    }
+}
+
 // WPT warps per token: candidates from the approximate logits and their bounds (every warp of the token finds them), canonical
 // logits of the candidates (dealt out to the warps), top-k and softmax as in every other router kernel (one warp). A
 // canonical logit is one long dependent chain, so with few rows a token's eight or nine must not follow one another: one
@@ -701,7 +808,7 @@ router_recheck_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict_
         if (!is_last) return;
         pdl_launch_dependents();
         __threadfence();
-        group_routes_in_block<true>(out_idx, out_w, rows, top_k, num_experts, grp, smem);
+        group_rows_in_block(out_idx, out_w, rows, top_k, num_experts, grp, smem);
     }
 }
 
