@@ -16,7 +16,7 @@ namespace tf {
 
 constexpr uint32_t kF32PartialTokens = 64;   // decode-sized batches keep fp32 partials (decode kernel semantics)
 constexpr uint32_t kExactMaxK = 3072;        // columns up to which its kernels have two buffers of scale planes, which they need
-constexpr uint32_t kExactMaxTokens = 255;    // most tokens of a block on the tensor cores with exact weights (block_exact)
+constexpr uint32_t kExactMaxTokens = 255;    // most tokens of a stack on the tensor cores with exact weights (block_exact)
 
 __device__ __forceinline__ uint64_t mix64(uint64_t z) {
     z += 0x9E3779B97F4A7C15ull;
@@ -524,7 +524,7 @@ tf_status tf_workspace_create(tf_context* ctx, uint32_t max_tokens, uint32_t d, 
                    o_sy = take(T * d * 2), o_xn = take(T * d * 2), o_yb = take(T * d * 2), o_ticket = take(4), o_logits = take(TF_MAX_ROUTER_EXPERTS * 4);
     // workspaces that can hold a tensor-core sized block also carry the expert-sorted activation rows
     const bool tensor_path = T >= ctx->tensorcore_min_tokens && d % 64 == 0 && f % 64 == 0 && fs % 64 == 0;
-    // and those for 65 tokens and more, whose blocks of up to kExactMaxTokens run there with exact weights, rows with extra columns
+    // and those for 65 tokens and more, in which stacks of up to kExactMaxTokens run there with exact weights, rows with extra columns
     const uint64_t o_xs = off, sorted = tensor_path ? T * K * d : 0, sorted_exact = X * K * dx;
     take((sorted > sorted_exact ? sorted : sorted_exact) * 2);
     const uint64_t R = tensor_path ? T : X, o_inv = take(R * K * 4), o_pid = take(R * K * 4), o_xe = take(X * dx * 2);
