@@ -396,6 +396,39 @@ def test_stack_of_many_tokens_equals_the_chain_of_entry_points_bit_for_bit(tf_ct
     test_decode_sized_stack_equals_the_chain_of_entry_points_bit_for_bit(tf_ctx, oracle, T, d)
 
 
+# Between the decode-sized batches and the tensor-core threshold: few rows per expert and many (four to sixteen).
+@pytest.mark.parametrize("T,d", [(65, 2816), (112, 2816), (255, 2816), (255, 1088)])
+def test_stack_of_65_to_255_tokens_equals_the_chain_of_entry_points_bit_for_bit(tf_ctx, oracle, T, d):
+    test_decode_sized_stack_equals_the_chain_of_entry_points_bit_for_bit(tf_ctx, oracle, T, d)
+
+
+def test_a_threshold_set_to_its_default_changes_nothing(tf_ctx, oracle):
+    import torch
+    from turbo_fieldfare_b200.kernels import TurboContext
+    from turbo_fieldfare_b200.stack import MoEStack
+    h16 = oracle.f32_to_f16(np.random.default_rng(9).standard_normal((200, 2816)).astype(np.float32))
+    out = []
+    for set_thresholds in (False, True):
+        ctx = TurboContext(0)
+        if set_thresholds:
+            ctx.set_tensorcore_min_tokens(256)
+            ctx.set_shared_tensorcore_min_tokens(256)
+        stack = MoEStack(ctx, layers=2, d=2816, f=256, fs=512, num_experts=16, top_k=8, seed=5, align=256)
+        try:
+            h = to_dev(h16.copy())
+            before = ctx.launch_count
+            stack.forward(h, 200, stack.workspace(200))
+            count = ctx.launch_count - before
+            torch.cuda.synchronize()
+            assert ctx.device_status() == 0
+            out.append((count, from_dev(h, np.uint16)))
+        finally:
+            torch.cuda.synchronize()
+            stack.close()
+            ctx.close()
+    assert out[0][0] == out[1][0] and np.array_equal(out[0][1], out[1][1])
+
+
 @pytest.mark.parametrize("T", [1, 40])
 def test_block_forward_with_8bit_shared_expert(tf_ctx, oracle, T):
     """A layer whose shared expert is 8-bit affine (tf_moe_layer.shared_bits = 8; SharedExpertInt8.swift:55-210): the

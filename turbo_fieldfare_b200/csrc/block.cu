@@ -15,8 +15,6 @@
 namespace tf {
 
 constexpr uint32_t kF32PartialTokens = 64;   // decode-sized batches keep fp32 partials (decode kernel semantics)
-constexpr uint32_t kExactMaxK = 3072;        // columns up to which its kernels have two buffers of scale planes, which they need
-constexpr uint32_t kExactMaxTokens = 255;    // most tokens of a stack on the tensor cores with exact weights (block_exact)
 
 __device__ __forceinline__ uint64_t mix64(uint64_t z) {
     z += 0x9E3779B97F4A7C15ull;
@@ -513,21 +511,15 @@ tf_status tf_workspace_create(tf_context* ctx, uint32_t max_tokens, uint32_t d, 
     auto up = [](uint64_t v) { return (v + 255) / 256 * 256; };
     uint64_t off = 0;
     auto take = [&](uint64_t bytes) { uint64_t o = off; off += up(bytes); return o; };
-    const bool exact = T > tf::kF32PartialTokens && !ctx->tensorcore_min_set && d % 64 == 0 && f % 64 == 0 && fs % 64 == 0;
-    const uint64_t X = !exact ? 0 : T < tf::kExactMaxTokens ? T : tf::kExactMaxTokens;
-    const uint64_t dx = tf::qmm_exact_columns(d), fx = tf::qmm_exact_columns(f), fsx = tf::qmm_exact_columns(fs);
-    const uint64_t acts = T * f > X * fx ? T * f : X * fx, sact = T * fs > X * fsx ? T * fs : X * fsx;
     const uint64_t o_idx = take(T * K * 4), o_w = take(T * K * 2), o_pairs = take(T * K * 16), o_eoff = take(E * 4),
                    o_ecnt = take(E * 4), o_groups = take(E * 12), o_cgroup = take((T * K / 8 + E + 1) * 4),
-                   o_cstart = take(E * 4), o_counters = take(16), o_acts = take(K * acts * 2),
-                   o_partials = take(T * K * d * (T <= tf::kF32PartialTokens ? 4 : 2)), o_sact = take(sact * 2),
+                   o_cstart = take(E * 4), o_counters = take(16), o_acts = take(T * K * f * 2),
+                   o_partials = take(T * K * d * (T <= tf::kF32PartialTokens ? 4 : 2)), o_sact = take(T * fs * 2),
                    o_sy = take(T * d * 2), o_xn = take(T * d * 2), o_yb = take(T * d * 2), o_ticket = take(4), o_logits = take(TF_MAX_ROUTER_EXPERTS * 4);
     // workspaces that can hold a tensor-core sized block also carry the expert-sorted activation rows
     const bool tensor_path = T >= ctx->tensorcore_min_tokens && d % 64 == 0 && f % 64 == 0 && fs % 64 == 0;
-    // and those for 65 tokens and more, in which stacks of up to kExactMaxTokens run there with exact weights, rows with extra columns
-    const uint64_t o_xs = off, sorted = tensor_path ? T * K * d : 0, sorted_exact = X * K * dx;
-    take((sorted > sorted_exact ? sorted : sorted_exact) * 2);
-    const uint64_t R = tensor_path ? T : X, o_inv = take(R * K * 4), o_pid = take(R * K * 4), o_xe = take(X * dx * 2);
+    const uint64_t o_xs = tensor_path ? take(T * K * d * 2) : 0, o_inv = tensor_path ? take(T * K * 4) : 0,
+                   o_pid = tensor_path ? take(T * K * 4) : 0;
     uint8_t* base = nullptr;
     cudaError_t e = cudaMalloc(&base, off);
     if (e != cudaSuccess) {
@@ -555,11 +547,9 @@ tf_status tf_workspace_create(tf_context* ctx, uint32_t max_tokens, uint32_t d, 
     w->one_token_logits = reinterpret_cast<float*>(base + o_logits);
     w->x_norm = reinterpret_cast<uint16_t*>(base + o_xn);
     w->y_block = reinterpret_cast<uint16_t*>(base + o_yb);
-    w->tensor_path = tensor_path;
-    w->x_sorted = R ? reinterpret_cast<uint16_t*>(base + o_xs) : nullptr;
-    w->inverse_perm = R ? reinterpret_cast<uint32_t*>(base + o_inv) : nullptr;
-    w->pack_ids = R ? reinterpret_cast<uint32_t*>(base + o_pid) : nullptr;
-    w->x_ext = exact ? reinterpret_cast<uint16_t*>(base + o_xe) : nullptr;
+    w->x_sorted = tensor_path ? reinterpret_cast<uint16_t*>(base + o_xs) : nullptr;
+    w->inverse_perm = tensor_path ? reinterpret_cast<uint32_t*>(base + o_inv) : nullptr;
+    w->pack_ids = tensor_path ? reinterpret_cast<uint32_t*>(base + o_pid) : nullptr;
     *out = w;
     return TF_OK;
 }
@@ -587,7 +577,7 @@ namespace tf {
 
 // Router, device grouping and the routed experts of one block, on the caller's stream.
 static tf_status block_routed(tf_context* ctx, void* stream, const tf_moe_layer* layer, const void* x, uint32_t x_stride_elements,
-                              uint32_t tokens, tf_workspace* ws, bool tensor_path, bool exact) {
+                              uint32_t tokens, tf_workspace* ws, bool tensor_path) {
     const uint32_t d = layer->d, f = layer->f, K = layer->top_k, E = layer->num_experts;
     // Decode-sized blocks route and group in one launch, blocks of a few hundred tokens in two: their approximate logits lie
     // where the activations will (they are read before the gate/up phase writes those).
@@ -608,9 +598,6 @@ static tf_status block_routed(tf_context* ctx, void* stream, const tf_moe_layer*
         return tf_grouped_moe_tensorcore(ctx, stream, ws->x_sorted, tokens * K, layer->pool_layer_base, layer->expert_stride, E,
                                          &layer->offsets, &ws->routes, ws->acts, ws->partials, d, f);
     }
-    if (exact)
-        return grouped_moe_exact(ctx, stream, x, x_stride_elements, tokens, K, ws->x_sorted, ws->inverse_perm, layer->pool_layer_base, layer->expert_stride,
-                                 E, &layer->offsets, &ws->routes, ws->acts, ws->partials, d, f);
     // The partial dtype follows the workspace's capacity so that one workspace
     // always runs the same arithmetic whatever the call's token count.
     const int f32 = ws->max_tokens <= kF32PartialTokens ? 1 : 0;
@@ -626,47 +613,9 @@ extern "C" {
 
 namespace tf {
 
-// Layers of a stack for 65 to 255 tokens whose experts run on the tensor cores with exact weights: the precision of the CUDA-core kernels (fp32
-// sums of exact products, the same roundings of activations and partials), but sums of another order, so that single blocks, which have the bits
-// of their tokens in blocks of any size below tensorcore_min_tokens, stay on those.
-// From 7 rows per expert on: the CUDA-core kernels read an expert's weights again for every eight of its tokens, this path once. A layer of
-// 2816 x 704 x 128 experts, top 8 (us, these kernels / those): 66 tokens 156 / 133, 100: 175 / 160, 110: 180 / 184, 130: 184 / 196,
-// 200: 194 / 239, 255: 210 / 280; 64 experts, top 4 alike, 128 experts, top 4 even at 200 tokens. And only where the products outweigh the
-// tensor maps and the two launches more (a layer, tokens * top_k * d * f: 2^26.7 at 512 x 256 x 16 experts 47 / 43, 2^27.8 at
-// 1024 x 512 x 32 60 / 61, 2^28.3 61 / 71).
-static bool block_exact(const tf_context* ctx, const tf_moe_layer* l, const tf_workspace* ws, uint32_t tokens) {
-    if (!ws->x_ext || ctx->tensorcore_min_set || ws->max_tokens <= kF32PartialTokens || tokens > kExactMaxTokens ||
-        tokens >= ctx->tensorcore_min_tokens || l->d > kExactMaxK || l->f > kExactMaxK)
-        return false;
-    if ((uint64_t)tokens * l->top_k < 7ull * l->num_experts || (uint64_t)tokens * l->top_k * l->d * l->f < 1ull << 28) return false;
-    const tf_expert_offsets& o = l->offsets;
-    const uint32_t all[9] = {o.gate_w_off, o.gate_s_off, o.gate_b_off, o.up_w_off, o.up_s_off, o.up_b_off, o.down_w_off, o.down_s_off, o.down_b_off};
-    for (uint32_t v : all)
-        if (v % 16 != 0) return false;
-    return l->d == ws->d && l->f == ws->f && l->fs == ws->fs && l->top_k == ws->top_k && l->num_experts == ws->num_experts && l->pool_layer_base &&
-           aligned(l->pool_layer_base, 16) && l->expert_stride % 16 == 0 && l->top_k <= TF_MAX_TOP_K && l->num_experts <= TF_MAX_ROUTER_EXPERTS;
-}
-// The shared expert of a stack's layer for 65 to 255 tokens, whatever the routed experts run on: on the CUDA cores its two launches hold the SMs
-// until 55 us of a layer of 100 tokens, here until 50, and the routed gate/up waits for them. Steps of 30 layers, us: 75 tokens 4122 -> 4027,
-// 90: 4510 -> 4390, 100: 4824 -> 4752, 110: 5512 -> 5374. (The size: as for the routed experts.)
-static bool shared_exact(const tf_context* ctx, const tf_moe_layer* l, const tf_workspace* ws, uint32_t tokens) {
-    if (!ws->x_ext || ctx->tensorcore_min_set || ctx->shared_tensorcore_min_set || l->shared_bits == 8 || tokens <= kF32PartialTokens ||
-        tokens > kExactMaxTokens || tokens >= ctx->shared_tensorcore_min_tokens || (uint64_t)tokens * l->d * l->fs < 1ull << 28 || l->d > kExactMaxK ||
-        l->fs > kExactMaxK)
-        return false;
-    const tf_projection* ps[3] = {&l->shared_gate, &l->shared_up, &l->shared_down};
-    const uint32_t rows[3] = {l->fs, l->fs, l->d}, cols[3] = {l->d, l->d, l->fs};
-    for (int i = 0; i < 3; ++i)
-        if (!ps[i]->weights || !ps[i]->scales || !ps[i]->biases || ps[i]->rows != rows[i] || ps[i]->cols != cols[i] ||
-            !aligned(byte_ptr(ps[i]->weights, ps[i]->weights_off), 16) || !aligned(byte_ptr(ps[i]->scales, ps[i]->scales_off), 16) ||
-            !aligned(byte_ptr(ps[i]->biases, ps[i]->biases_off), 16))
-            return false;
-    return true;
-}
-
 // Decode-sized blocks leave fp32 route partials that the next layer's norm can fold in (combine_residual_rmsnorm_kernel).
 static bool block_keeps_f32_partials(const tf_context* ctx, const tf_workspace* ws, uint32_t tokens) {
-    const bool tensor_path = tokens >= ctx->tensorcore_min_tokens && ws->tensor_path;
+    const bool tensor_path = tokens >= ctx->tensorcore_min_tokens && ws->x_sorted != nullptr;
     return !tensor_path && ws->max_tokens <= kF32PartialTokens;
 }
 
@@ -674,7 +623,7 @@ static bool block_keeps_f32_partials(const tf_context* ctx, const tf_workspace* 
 // is left to the caller, which finds the partials, weights and shared output in the workspace.
 static tf_status block_forward(tf_context* ctx, void* stream, const tf_moe_layer* layer,
                                const void* x, uint32_t x_stride_elements,
-                               void* y, uint32_t y_stride_elements, uint32_t tokens, tf_workspace* ws, bool exact = false, bool exact_shared = false) {
+                               void* y, uint32_t y_stride_elements, uint32_t tokens, tf_workspace* ws) {
     const char* name = "tf_moe_block_forward";
     TF_REQUIRE(ctx, ctx != nullptr, TF_ERR_INVALID_ARGUMENT, "%s: ctx is NULL", name);
     TF_REQUIRE(ctx, layer && x && ws, TF_ERR_INVALID_ARGUMENT, "%s: NULL argument", name);
@@ -693,12 +642,9 @@ static tf_status block_forward(tf_context* ctx, void* stream, const tf_moe_layer
     cudaStream_t main_st = static_cast<cudaStream_t>(stream);
     TF_CUDA(ctx, cudaEventRecord(ctx->fork_event, main_st));
     TF_CUDA(ctx, cudaStreamWaitEvent(ctx->side_stream, ctx->fork_event, 0));
-    const bool tensor_path = tokens >= ctx->tensorcore_min_tokens && ws->tensor_path;
+    const bool tensor_path = tokens >= ctx->tensorcore_min_tokens && ws->x_sorted != nullptr;
     tf_status s;
-    if (exact_shared && shared_exact(ctx, layer, ws, tokens))
-        s = shared_expert_exact(ctx, ctx->side_stream, x, x_stride_elements, &layer->shared_gate, &layer->shared_up, &layer->shared_down, ws->x_ext,
-                                ws->shared_act, ws->shared_y, tokens);
-    else if (layer->shared_bits == 8)
+    if (layer->shared_bits == 8)
         s = tf_shared_expert_int8_block(ctx, ctx->side_stream, x, 0, x_stride_elements, &layer->shared_gate, &layer->shared_up,
                                         &layer->shared_down, ws->shared_y, 0, d, ws->shared_act, tokens);
     else if (tensor_path || (tokens >= ctx->shared_tensorcore_min_tokens && d % 64 == 0 && layer->fs % 64 == 0))
@@ -710,7 +656,7 @@ static tf_status block_forward(tf_context* ctx, void* stream, const tf_moe_layer
     // the join is recorded even after a failure so that a capture in progress stays well formed
     cudaEventRecord(ctx->join_event, ctx->side_stream);
     if (s) { cudaStreamWaitEvent(main_st, ctx->join_event, 0); return s; }
-    s = tf::block_routed(ctx, stream, layer, x, x_stride_elements, tokens, ws, tensor_path, exact);
+    s = tf::block_routed(ctx, stream, layer, x, x_stride_elements, tokens, ws, tensor_path);
     TF_CUDA(ctx, cudaStreamWaitEvent(main_st, ctx->join_event, 0));
     if (s) return s;
     if (y == nullptr) return TF_OK;
@@ -1031,10 +977,7 @@ tf_status tf_stack_forward(tf_stack* st, void* stream, void* hidden, uint32_t to
     const bool fold = !st->layers.empty() && tf::block_keeps_f32_partials(ctx, ws, tokens) && st->layers[0].top_k <= TF_MAX_TOP_K &&
                       tf::aligned(ws->partials, 16) && tf::aligned(ws->shared_y, 16);
     // Prefill-sized blocks leave expert-sorted fp16 rows instead; the same kernel gathers them through the permutation.
-    const bool tensor_path = tokens >= ctx->tensorcore_min_tokens && ws->tensor_path;
-    bool exact = !st->layers.empty() && !tensor_path;          // so do stacks whose layers are all of the sizes for exact weights
-    for (size_t l = 0; l < st->layers.size() && exact; ++l) exact = tf::block_exact(ctx, &st->layers[l], ws, tokens);
-    const bool fold_rows = !st->layers.empty() && (tensor_path || exact) && st->layers[0].top_k <= TF_MAX_TOP_K &&
+    const bool fold_rows = !st->layers.empty() && tokens >= ctx->tensorcore_min_tokens && ws->x_sorted != nullptr && st->layers[0].top_k <= TF_MAX_TOP_K &&
                            tf::aligned(ws->partials, 16) && tf::aligned(ws->shared_y, 16);
     uint32_t fold_threads = ((d / 8 + 31) / 32) * 32;          // one thread per eight columns,
     if (fold_threads < (uint32_t)tf::kRrnThreads) fold_threads = tf::kRrnThreads;      // at least the norm's 128 (its reduction tree)
@@ -1055,7 +998,7 @@ tf_status tf_stack_forward(tf_stack* st, void* stream, void* hidden, uint32_t to
             tf::launch_pdl(tf::residual_rmsnorm_kernel, dim3(tokens), dim3(tf::kRrnThreads), smem, cs, h,
                            l == 0 ? no16 : static_cast<const uint16_t*>(ws->y_block), nw, ws->x_norm, d, st->eps);
         if (tf_status s = tf::check_launch(ctx, "residual_rmsnorm")) return s;
-        if (tf_status s = tf::block_forward(ctx, stream, &st->layers[l], ws->x_norm, d, fold || fold_rows ? nullptr : ws->y_block, d, tokens, ws, exact, true)) return s;
+        if (tf_status s = tf::block_forward(ctx, stream, &st->layers[l], ws->x_norm, d, fold || fold_rows ? nullptr : ws->y_block, d, tokens, ws)) return s;
     }
     if (fold_rows)
         return tf::combine_rows_residual_rmsnorm(ctx, stream, h, ws->partials, ws->weights, ws->inverse_perm, ws->shared_y, nullptr, nullptr, tokens,

@@ -27,11 +27,9 @@ struct tf_workspace {
     uint32_t* router_ticket;  // zero between launches
     uint16_t* x_norm;       // [T, D] (stack)
     uint16_t* y_block;      // [T, D] (stack)
-    bool tensor_path;       // holds a tensor-core sized block
     uint16_t* x_sorted;     // [T*K, D] expert-sorted activation rows (tensor-core path; NULL for small workspaces)
     uint32_t* inverse_perm; // [T*K] sorted row of every (token, rank)
     uint32_t* pack_ids;     // [T*K]
-    uint16_t* x_ext;        // rows with extra columns (qmm_exact_columns) of blocks that run on the tensor cores with exact weights; NULL: none do
     float* one_token_logits;  // [TF_MAX_ROUTER_EXPERTS] (one_token.cu)
     uint64_t bytes;
 };
@@ -52,13 +50,6 @@ struct PeerWait;
 bool decode_step_eligible(const tf_stack* st, const tf_workspace* ws);
 tf_status decode_step_prepare(tf_context* ctx, tf_stack* st);
 tf_status launch_decode_step(tf_context* ctx, void* stream, tf_stack* st, void* hidden, tf_workspace* ws);
-// qmm_tcgen05.cu: the routed and the shared experts on the tensor cores with exact weights
-uint32_t qmm_exact_columns(uint32_t k);
-tf_status grouped_moe_exact(tf_context* ctx, void* stream, const void* x, uint32_t x_stride_elements, uint32_t tokens, uint32_t top_k, void* x_sorted,
-                            uint32_t* inverse_perm, const void* pool_layer_base, uint64_t expert_stride, uint32_t num_experts,
-                            const tf_expert_offsets* offsets, const tf_device_routes* routes, void* acts_scratch, void* out_rows, uint32_t d, uint32_t f);
-tf_status shared_expert_exact(tf_context* ctx, void* stream, const void* x, uint32_t x_stride_elements, const tf_projection* gate, const tf_projection* up,
-                              const tf_projection* down, void* x_ext, void* scratch_act, void* y, uint32_t rows);
 // one_token.cu: a layer of a stack (hidden row updated in place), or a block forward, for one token
 bool one_token_eligible(const tf_context* ctx, const tf_moe_layer* layer, const tf_workspace* ws);
 tf_status one_token_layer(tf_context* ctx, void* stream, const tf_moe_layer* layer, const void* norm_weight_bf16, void* hidden, float eps, tf_workspace* ws);

@@ -129,14 +129,12 @@ uint64_t tf_launch_count(tf_context* ctx) { return ctx ? ctx->launches : 0; }
 tf_status tf_context_set_tensorcore_min_tokens(tf_context* ctx, uint32_t tokens) {
     TF_REQUIRE(ctx, ctx != nullptr && tokens > 0, TF_ERR_INVALID_ARGUMENT, "tf_context_set_tensorcore_min_tokens: ctx is NULL or tokens is 0");
     ctx->tensorcore_min_tokens = tokens;
-    ctx->tensorcore_min_set = true;
     return TF_OK;
 }
 
 tf_status tf_context_set_shared_tensorcore_min_tokens(tf_context* ctx, uint32_t tokens) {
     TF_REQUIRE(ctx, ctx != nullptr && tokens > 0, TF_ERR_INVALID_ARGUMENT, "tf_context_set_shared_tensorcore_min_tokens: ctx is NULL or tokens is 0");
     ctx->shared_tensorcore_min_tokens = tokens;
-    ctx->shared_tensorcore_min_set = true;
     return TF_OK;
 }
 

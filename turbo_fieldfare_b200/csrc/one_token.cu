@@ -719,7 +719,7 @@ bool one_token_eligible(const tf_context* ctx, const tf_moe_layer* l, const tf_w
                        l->d <= kOneMaxGroups * kGroup && l->f <= kOneMaxGroups * kGroup && l->fs <= kOneMaxGroups * kGroup &&
                        l->top_k > 0 && l->top_k <= TF_MAX_TOP_K && l->top_k <= l->num_experts && l->num_experts <= TF_MAX_ROUTER_EXPERTS;
     if (!shape || l->shared_bits == 8 || ws->max_tokens > 64 || ctx->shared_tensorcore_min_tokens <= 1 ||
-        (ctx->tensorcore_min_tokens <= 1 && ws->tensor_path))
+        (ctx->tensorcore_min_tokens <= 1 && ws->x_sorted != nullptr))
         return false;
     const tf_projection* ps[4] = {&l->router, &l->shared_gate, &l->shared_up, &l->shared_down};
     const uint32_t rows[4] = {l->num_experts, l->fs, l->fs, l->d}, cols[4] = {l->d, l->d, l->d, l->fs};

@@ -28,7 +28,7 @@
 // A persistent grid walks (group, token tile, weight-row tile) work items derived on the device from the
 // routing metadata. Every mbarrier wait is bounded; on expiry the kernel records a code, waits for its copies and leaves.
 //
-// Four forms (clock counters around the waits of each role; 128 experts of 704 x 2816, uniform routing):
+// Three forms (clock counters around the waits of each role; 128 experts of 704 x 2816, uniform routing):
 // kQmmPair, many tokens: with one CTA per tile of 128 rows x 128 tokens a stage took 1700 clocks, 640 of them waits for activations
 // (64 KB per stage and SM out of L2). A pair of CTAs (cta_group::2) shares them: each holds those of half the tokens. 1240 clocks
 // at 104 tokens per tile (MMAs 830), most of the rest the instructions of the one warp that issues them. 4096 tokens: gate/up 281
@@ -41,9 +41,6 @@
 // kQmmWide, dense launches of more than 64 tokens per tile whose tiles have few stages: there start and end count, which take a pair
 // about 1 us longer, and tiles of 64 tokens would be twice as many. 2000 x 1024 x 512: 8.5 us in the better of the other two, 7.5
 // here; 500 x 4096 x 512 8.5 and 7.7; 500 x 8192 x 256 9.1 and 8.2. (Activations by half stages: up to 7 % slower.)
-// kQmmExact, blocks of up to 255 tokens with 7 rows per expert and more: kQmmFew with weights that are not rounded (below). Instructions
-// bound it, those of a stage with the extra groups' beside them (stalls for instructions 1.0 per issued one, kQmmFew 0.4). 200 tokens:
-// gate/up 106 -> 89 us, down 72 -> 53 (the CUDA-core kernels, whose loads of an expert serve eight tokens, and these).
 //
 // Column order. The cheapest nibble extraction yields the eight codes of a 32-bit word in the order
 // (0,4,1,5,2,6,3,7). A dot product does not care about the order as long as both operands agree, so the
@@ -81,7 +78,7 @@ struct QmmPlan {
     uint32_t sc_bufs;       // scale-plane buffers
     uint32_t plane_bytes;   // one scale or bias plane of a tile (128 / NMAT rows)
     uint32_t sc_bytes;      // one buffer: NMAT x (scale plane, bias plane)
-    uint32_t off_b, off_sc, off_stage, off_table, off_bars, off_exact, total;
+    uint32_t off_b, off_sc, off_stage, off_table, off_bars, total;
 };
 
 struct QmmArgs {
@@ -93,8 +90,7 @@ struct QmmArgs {
     // and {groups, token tiles, largest N}
     EarlyTable<uint4> groups;
     EarlyTable<uint32_t> totals;
-    // their source; routed: what the grouping kernels left on the device; dense (NULL): one group (kQmmExact: every CTA forms its tables
-    // from it, without a launch of its own for that)
+    // their source; routed: what the grouping kernels left on the device; dense (NULL): one group
     const tf_group* route_groups;
     const uint32_t* route_counters;
     uint32_t dense_tokens, dense_per_tile;
@@ -108,24 +104,9 @@ struct QmmArgs {
     uint32_t out_stride;
     uint32_t out_vec;       // rows of out start on 16-byte boundaries
     uint32_t round_gate_up; // shared expert: gate and up rounded to fp16 before the activation
-    uint32_t extra;         // kQmmExact: groups that follow the K columns of an activation row (see qmm_extra_groups)
     uint32_t* error;
     QmmPlan plan;
 };
-
-// kQmmExact: what the weights' products leave out, sum over the groups of (b + 8 s) * (sum of the group's activations), is 64-column groups
-// more of the same GEMM: a group of the row takes three columns, half(c'), half(c') * 2^-11 and half(c' - half(c')) of the weights'
-// c' = (b + 8 s) * 2^6 against half(x'), half((x' - half(x')) * 2^11) and half(x') of the activations' x' = sum * 2^-6: 22 bits of either, for sums of
-// up to 64 * 65504 and small ones alike. Twelve groups to 64 columns (12 of each kind, 28 of zeros), which spreads the production width's 44
-// over a stage's four groups, whose columns different threads make.
-constexpr uint32_t kQmmPerExtra = 12;
-__host__ __device__ constexpr uint32_t qmm_extra_groups(uint32_t k) { return (k / kGroup + kQmmPerExtra - 1) / kQmmPerExtra; }
-// The m-th of the three columns for a sum.
-__device__ __forceinline__ uint16_t qmm_extra_value(float sum, uint32_t m) {
-    const float x = sum * 0.015625f;
-    const __half hi = __float2half_rn(x);
-    return __half_as_ushort(m == 1 ? __float2half_rn((x - __half2float(hi)) * 2048.0f) : hi);
-}
 
 // ---- PTX wrappers ----
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -134,12 +115,6 @@ __device__ __forceinline__ void q_mbar_init(uint32_t addr, uint32_t count) {
 }
 __device__ __forceinline__ void q_mbar_arrive(uint32_t addr) {
     asm volatile("{ .reg .b64 st; mbarrier.arrive.shared::cta.b64 st, [%0]; }" ::"r"(addr) : "memory");
-}
-// Arrives once a and b are in registers: both arms arrive, but which one takes their values. For loads whose source the next bulk copy
-// overwrites: a plain arrival after them does not wait for their data (kQmmExact then had single rows with the codes of two stages later).
-__device__ __forceinline__ void q_mbar_arrive_after(uint32_t addr, uint32_t a, uint32_t b) {
-    asm volatile("{ .reg .b64 st; .reg .pred p; setp.eq.u32 p, %1, %2;\n\t"
-                 "@p mbarrier.arrive.shared::cta.b64 st, [%0];\n\t@!p mbarrier.arrive.shared::cta.b64 st, [%0], 1; }" ::"r"(addr), "r"(a), "r"(b) : "memory");
 }
 __device__ __forceinline__ void q_mbar_expect_tx(uint32_t addr, uint32_t bytes) {
     asm volatile("{ .reg .b64 st; mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1; }" ::"r"(addr), "r"(bytes) : "memory");
@@ -324,21 +299,20 @@ __host__ __device__ inline uint32_t qmm_tokens_per_tile(uint32_t count, uint32_t
 }
 
 // The group table of a launch: one thread per group, the tile counts scanned over the block. (One thread that walked the
-// groups took 29 us for 128 of them, on the critical path before every routed GEMM; this takes about 2.) All threads of the block; the
-// tables are complete after a barrier. IN_GEMM: of a block with more threads; EARLY: which may not have waited (see EarlyTable).
-template <bool IN_GEMM, bool EARLY>
-__device__ __forceinline__ void qmm_group_table(uint4* __restrict__ groups, uint32_t* __restrict__ totals, const tf_group* __restrict__ route_groups,
-                                                const uint32_t* __restrict__ route_counters, uint32_t dense_tokens, uint32_t dense_per_tile, uint32_t ctas) {
+// groups took 29 us for 128 of them, on the critical path before every routed GEMM; this takes about 2.)
+__global__ void __launch_bounds__(TF_MAX_ROUTER_EXPERTS)
+qmm_prepare_kernel(uint4* __restrict__ groups, uint32_t* __restrict__ totals, const tf_group* __restrict__ route_groups,
+                   const uint32_t* __restrict__ route_counters, uint32_t dense_tokens, uint32_t dense_per_tile, uint32_t ctas) {
     __shared__ uint32_t warp_tiles[TF_MAX_ROUTER_EXPERTS / kWarp], warp_top[TF_MAX_ROUTER_EXPERTS / kWarp];
     const uint32_t warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
-    const bool scans = !IN_GEMM || threadIdx.x < TF_MAX_ROUTER_EXPERTS;            // whole warps
-    const uint32_t counted = !route_groups ? 1u : IN_GEMM ? EarlyTable<uint32_t>{route_counters}.at<EARLY>(0) : route_counters[0];
-    const uint32_t ngroups = scans ? min(counted, (uint32_t)TF_MAX_ROUTER_EXPERTS) : 0u;
+    pdl_launch_dependents();
+    pdl_wait();
+    const uint32_t ngroups = route_groups ? min(route_counters[0], (uint32_t)TF_MAX_ROUTER_EXPERTS) : 1u;
     const uint32_t step = ctas * 16u;
     uint32_t row = 0, count = 0, expert = 0, per = step;
     if (threadIdx.x < ngroups) {
         if (route_groups) {
-            const tf_group rg = IN_GEMM ? EarlyTable<tf_group>{route_groups}.at<EARLY>(threadIdx.x) : route_groups[threadIdx.x];
+            const tf_group rg = route_groups[threadIdx.x];
             row = rg.pair_start; count = rg.pair_count; expert = rg.expert;
             per = qmm_tokens_per_tile(count > 0 ? count : 1u, ctas);
         } else {
@@ -347,15 +321,13 @@ __device__ __forceinline__ void qmm_group_table(uint4* __restrict__ groups, uint
     }
     const uint32_t tiles = (count + per - 1) / per;
     uint32_t incl = tiles;
-    if (scans) {
 #pragma unroll
-        for (int o = 1; o < kWarp; o <<= 1) {
-            const uint32_t v = __shfl_up_sync(kFullMask, incl, o);
-            if (lane >= (uint32_t)o) incl += v;
-        }
-        const uint32_t top = __reduce_max_sync(kFullMask, min((count + step - 1) / step * step, per));
-        if (lane == kWarp - 1) { warp_tiles[warp] = incl; warp_top[warp] = top; }
+    for (int o = 1; o < kWarp; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(kFullMask, incl, o);
+        if (lane >= (uint32_t)o) incl += v;
     }
+    const uint32_t top = __reduce_max_sync(kFullMask, min((count + step - 1) / step * step, per));
+    if (lane == kWarp - 1) { warp_tiles[warp] = incl; warp_top[warp] = top; }
     __syncthreads();
     uint32_t before = 0, all = 0, n_top = step;
 #pragma unroll
@@ -366,67 +338,6 @@ __device__ __forceinline__ void qmm_group_table(uint4* __restrict__ groups, uint
     }
     if (threadIdx.x < ngroups) groups[threadIdx.x] = make_uint4(before + incl - tiles, row, count, expert | (per << 16));
     if (threadIdx.x == 0) { totals[0] = ngroups; totals[1] = all; totals[2] = n_top; }
-}
-__global__ void __launch_bounds__(TF_MAX_ROUTER_EXPERTS)
-qmm_prepare_kernel(uint4* __restrict__ groups, uint32_t* __restrict__ totals, const tf_group* __restrict__ route_groups,
-                   const uint32_t* __restrict__ route_counters, uint32_t dense_tokens, uint32_t dense_per_tile, uint32_t ctas) {
-    pdl_launch_dependents();
-    pdl_wait();
-    qmm_group_table<false, false>(groups, totals, route_groups, route_counters, dense_tokens, dense_per_tile, ctas);
-}
-
-// Rows for kQmmExact: out[row] = the row and its extra columns, one warp per row. PACK: row = token of sorted pair `row`, every eight columns in
-// the order of the routed GEMM; ids and inverse permutation as ep_pack_kernel leaves them.
-constexpr int kExtendThreads = 256;
-template <bool PACK>
-__global__ void __launch_bounds__(kExtendThreads)
-qmm_extend_rows_kernel(const uint16_t* __restrict__ x, uint32_t stride, uint32_t rows, uint32_t d, uint16_t* __restrict__ out, uint32_t out_stride,
-                       const tf_pair* __restrict__ pairs, const uint32_t* __restrict__ grouped, uint32_t top_k, uint32_t* __restrict__ inverse_perm) {
-    __shared__ float sums[kExtendThreads / kWarp][48 + 16];
-    const uint32_t warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp, row = blockIdx.x * (kExtendThreads / kWarp) + warp;
-    pdl_launch_dependents();
-    pdl_wait();
-    if (row >= (PACK ? min(rows, *grouped) : rows)) return;
-    uint32_t src_row = row;
-    if constexpr (PACK) {
-        const tf_pair pr = pairs[row];
-        src_row = pr.token;
-        if (lane == 0) inverse_perm[pr.token * top_k + pr.rank] = row;
-    }
-    const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)src_row * stride);
-    uint4* dst = reinterpret_cast<uint4*>(out + (size_t)row * out_stride);
-    const uint32_t vecs = d / 8, ng = d / kGroup;
-    for (uint32_t base = 0; base < vecs; base += kWarp) {              // whole warps
-        const uint32_t i = base + lane;
-        const bool ok = i < vecs;
-        uint4 v = ok ? __ldg(src + i) : make_uint4(0u, 0u, 0u, 0u);
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-        float sum = 0.0f;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[q]));
-            sum += f.x + f.y;
-        }
-#pragma unroll
-        for (int o = 1; o < 8; o <<= 1) sum += __shfl_xor_sync(kFullMask, sum, o);
-        if (!ok) continue;
-        if ((lane & 7) == 0) sums[warp][i / 8] = sum;
-        if constexpr (PACK) {
-            uint4 o;
-            asm("prmt.b32 %0, %1, %2, 0x5410;" : "=r"(o.x) : "r"(v.x), "r"(v.z));   // (k0, k4)
-            asm("prmt.b32 %0, %1, %2, 0x7632;" : "=r"(o.y) : "r"(v.x), "r"(v.z));   // (k1, k5)
-            asm("prmt.b32 %0, %1, %2, 0x5410;" : "=r"(o.z) : "r"(v.y), "r"(v.w));   // (k2, k6)
-            asm("prmt.b32 %0, %1, %2, 0x7632;" : "=r"(o.w) : "r"(v.y), "r"(v.w));   // (k3, k7)
-            v = o;
-        }
-        dst[i] = v;
-    }
-    __syncwarp();
-    uint16_t* extra = out + (size_t)row * out_stride + d;
-    for (uint32_t p = lane; p < qmm_extra_groups(d) * kGroup; p += kWarp) {
-        const uint32_t q = p % kGroup, g = p / kGroup * kQmmPerExtra + q % kQmmPerExtra;
-        extra[p] = q < 3 * kQmmPerExtra && g < ng ? qmm_extra_value(sums[warp][g], q / kQmmPerExtra) : (uint16_t)0;
-    }
 }
 
 // A role's place in its CTA's (or pair's) sequence of tiles, which is tile first, first + step, ... Tiles only move forward: the
@@ -464,19 +375,14 @@ struct QmmTile {
 // MMAs. kQmmFew: a CTA takes 128 rows x up to 64 tokens, and two warps issue MMAs, one for each team of dequantisers. kQmmWide:
 // a CTA takes 128 rows x up to 128 tokens, one warp issues.
 // x_map0 ... x_map3: boxes of 16, 32, 48 and 64 activation rows; kQmmWide: of a full tile's and of the last tile's rows.
-// kQmmExact: kQmmFew without a rounding of the weights, for batches that the CUDA-core kernels would take otherwise. (q - 8) * s, with s brought
-// into [.., 2^-6) by a power of two per row, is exact in fp16 (eight significant bits of s times three), so the MMAs sum exact products; the rest of
-// the bias, (b + 8 s) * sum of the group's activations, takes extra columns of the same GEMM (qmm_extra_groups). (With that rest as fp32
-// FMAs of the epilogue the kernel took twice as long as kQmmFew. The epilogue warps find each row's power of two; where the dequantisers did, a
-// layer of 200 tokens took 11 us more.)
-enum QmmForm { kQmmFew, kQmmWide, kQmmPair, kQmmExact };
+enum QmmForm { kQmmFew, kQmmWide, kQmmPair };
 template <int NMAT, bool NATURAL_K, QmmForm FORM>
 __global__ void __launch_bounds__(kQmmThreads, 1)
 qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map0, const __grid_constant__ CUtensorMap x_map1,
                    const __grid_constant__ CUtensorMap x_map2, const __grid_constant__ CUtensorMap x_map3,
                    const __grid_constant__ CUtensorMap w_map0, const __grid_constant__ CUtensorMap w_map1, const QmmArgs args) {
     extern __shared__ uint8_t smem_raw[];
-    constexpr bool PAIR = FORM == kQmmPair, EXACT = FORM == kQmmExact, kTwoIssuers = FORM == kQmmFew || EXACT;
+    constexpr bool PAIR = FORM == kQmmPair, kTwoIssuers = FORM == kQmmFew;
     constexpr uint32_t kMatRows = kQmmRows / NMAT;                     // rows of one matrix in a tile
     constexpr uint32_t kCtas = PAIR ? 2 : 1;                           // CTAs of a tile
     // One team of dequantisers, a group of a row per thread and stage, or two that take turns, two groups per thread: the latter
@@ -496,7 +402,6 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map0, const __grid_cons
     auto bar_empty_b = [&](uint32_t s) { return bars + (20 + s) * 8; };                      // 12: tcgen05.commit
     auto bar_full_a = [&](uint32_t t) { return bars + (32 + t) * 8; };                       // 2 L: the team's warps, of both CTAs
     auto bar_empty_a = [&](uint32_t t) { return bars + (34 + t) * 8; };                      // 2: tcgen05.commit
-    auto bar_scaled = [&](uint32_t b) { return bars + (36 + b) * 8; };                       // 4: kQmmExact: epilogue warps
     auto bar_full_sc = [&](uint32_t b) { return bars + (40 + b) * 8; };                      // 4: bulk-copy tx
     auto bar_empty_sc = [&](uint32_t b) { return bars + (44 + b) * 8; };                     // 4: dequant warps
     auto bar_acc_full = [&](uint32_t i, uint32_t b) { return bars + (48 + 2 * i + b) * 8; }; // 4: tcgen05.commit
@@ -510,8 +415,7 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map0, const __grid_cons
     const int warp = __shfl_sync(kFullMask, (int)(threadIdx.x / kWarp), 0), lane = threadIdx.x % kWarp;
     const uint32_t rank = PAIR ? blockIdx.x & 1 : 0;                   // CTA within the pair
     const uint32_t ng = args.k / kGroup;
-    const uint32_t ngx = EXACT ? ng + args.extra : ng;                 // with the extra groups
-    const uint32_t ksteps = (ngx + 3) / 4;                             // stages per tile
+    const uint32_t ksteps = (ng + 3) / 4;                              // stages per tile
     const uint32_t wrow_tiles = (args.rows + kCtas * kMatRows - 1) / (kCtas * kMatRows);
 
     constexpr bool kRoutedGateUp = NMAT == 2 && !NATURAL_K;
@@ -520,7 +424,7 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map0, const __grid_cons
         for (uint32_t s = 0; s < (uint32_t)kQmmRawMax; ++s) { q_mbar_init(bar_full_raw(s), 1); q_mbar_init(bar_empty_raw(s), kTeamWarps); }
         for (uint32_t s = 0; s < (uint32_t)kQmmBMax; ++s) { q_mbar_init(bar_full_b(s), 1); q_mbar_init(bar_empty_b(s), 1); }
         for (uint32_t t = 0; t < (uint32_t)kQmmASlots; ++t) { q_mbar_init(bar_full_a(t), kCtas * kTeamWarps); q_mbar_init(bar_empty_a(t), 1); }
-        for (uint32_t b = 0; b < (uint32_t)kQmmScMax; ++b) { q_mbar_init(bar_full_sc(b), 1); q_mbar_init(bar_empty_sc(b), kQmmDequantWarps); q_mbar_init(bar_scaled(b), kQmmEpilogueWarps); }
+        for (uint32_t b = 0; b < (uint32_t)kQmmScMax; ++b) { q_mbar_init(bar_full_sc(b), 1); q_mbar_init(bar_empty_sc(b), kQmmDequantWarps); }
         for (uint32_t b = 0; b < 2; ++b) {
             for (uint32_t i = 0; i < 2; ++i) q_mbar_init(bar_acc_full(i, b), 1);
             q_mbar_init(bar_acc_empty(b), kCtas * kQmmEpilogueWarps);
@@ -543,9 +447,6 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map0, const __grid_cons
     const bool early = NMAT == 1 && args.after_gate_up;
     if (!early) pdl_wait();                                             // routes and activations come from the kernels before this one
     if (kRoutedGateUp) pdl_launch_dependents();
-    if constexpr (EXACT) {
-        qmm_group_table<true, NMAT == 1>(table, totals, args.route_groups, args.route_counters, args.dense_tokens, args.dense_per_tile, 1);
-    } else
     // The whole table and the totals in one round trip, a thread per entry (rows past the groups are copied and never used).
     if (threadIdx.x < (args.route_groups ? (uint32_t)TF_MAX_ROUTER_EXPERTS : 1u)) table[threadIdx.x] = args.groups.at<NMAT == 1>(threadIdx.x);
     else if (threadIdx.x - TF_MAX_ROUTER_EXPERTS < 3u) totals[threadIdx.x - TF_MAX_ROUTER_EXPERTS] = args.totals.at<NMAT == 1>(threadIdx.x - TF_MAX_ROUTER_EXPERTS);
@@ -566,19 +467,18 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map0, const __grid_cons
     const uint32_t a_ring = tmem_base + kQmmAccCols;
     const uint32_t first_tile = blockIdx.x / kCtas, tile_step = gridDim.x / kCtas;
 
-    float* row_scales = reinterpret_cast<float*>(base_ptr + plan.off_exact);       // kQmmExact: [scale buffer][row]
     uint32_t fail = 0;
     QmmTile tl(first_tile, args.step_tok, args.step_row, wrow_tiles);
 
-    // Scale and bias planes of a tile; false when the wait for the buffer ran out.
+    // Scale and bias planes of tile tl; false when the wait for the buffer ran out.
     uint32_t pl_buf = 0, pl_use = 0;
-    auto copy_planes = [&](const QmmTile& of) {
-        const uint32_t first = (of.wt * kCtas + rank) * kMatRows;
+    auto copy_planes = [&]() {
+        const uint32_t first = (tl.wt * kCtas + rank) * kMatRows;
         if (pl_use > 0 && !q_mbar_wait(bar_empty_sc(pl_buf), (pl_use - 1) & 1)) return false;
         if (elect_one()) {
             const uint32_t left = first < args.rows ? args.rows - first : 0;      // a pair's second tile may be past the matrix
             const uint32_t bytes = (left < kMatRows ? left : kMatRows) * ng * 2;  // a multiple of 16: rows are a multiple of 8
-            const size_t off = (size_t)of.expert * args.expert_stride + (size_t)first * ng * 2;
+            const size_t off = (size_t)tl.expert * args.expert_stride + (size_t)first * ng * 2;
             q_mbar_expect_tx(bar_full_sc(pl_buf), NMAT * 2 * bytes);
             if (bytes > 0) {
 #pragma unroll
@@ -599,28 +499,13 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map0, const __grid_cons
     if (warp == 0) {
         // ===================== copy issuer: scale and bias planes of a tile, packed codes =====================
         uint32_t sr = 0, ur = 0;
-        QmmTile ptl = tl;
-        uint32_t ptile = first_tile;
-        auto next_planes = [&]() {
-            if (ptile >= total_tiles) return true;
-            ptl.locate(table, ngroups, lane);
-            const bool ok = copy_planes(ptl);
-            ptile += tile_step;
-            ptl.next();
-            return ok;
-        };
-        if constexpr (EXACT) {
-            if (!next_planes()) fail = kErrQmmTimeout | 6;
-        }
         for (uint32_t tile = first_tile; tile < total_tiles && !fail; tile += tile_step, tl.next()) {
             tl.locate(table, ngroups, lane);
             const uint32_t first = (tl.wt * kCtas + rank) * kMatRows;
             // (the dequantisers of the tile that used this buffer last are as far as the ring of codes asks for below, or one tile
             // ahead of it where the planes have one buffer)
-            if (FORM != kQmmWide && !EXACT && !copy_planes(tl)) { fail = kErrQmmTimeout | 6; break; }
+            if (FORM != kQmmWide && !copy_planes()) { fail = kErrQmmTimeout | 6; break; }
             for (uint32_t ks = 0; ks < ksteps; ++ks) {
-                // kQmmExact: the planes a tile earlier, since the epilogue warps look at them before the dequantisers
-                if (EXACT && ks + 1 == ksteps && !next_planes()) { fail = kErrQmmTimeout | 6; break; }
                 if (ur > 0 && !q_mbar_wait(bar_empty_raw(sr), (ur - 1) & 1)) { fail = kErrQmmTimeout | 1; break; }
                 if (elect_one()) {
                     const uint32_t dst = base + sr * kQmmRawBytes;
@@ -641,7 +526,7 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map0, const __grid_cons
         // ===================== copy issuer: scale and bias planes, beside the codes =====================
         for (uint32_t tile = first_tile; tile < total_tiles && !fail; tile += tile_step, tl.next()) {
             tl.locate(table, ngroups, lane);
-            if (!copy_planes(tl)) fail = kErrQmmTimeout | 6;
+            if (!copy_planes()) fail = kErrQmmTimeout | 6;
         }
         if (fail) drain_planes();
     } else if (warp == 2) {
@@ -698,7 +583,7 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map0, const __grid_cons
                     }
                     tc_fence_after();
                     const uint32_t a = a_ring + t * 128;
-                    const uint32_t groups = ngx - 4 * ks;             // groups left; those past K are skipped
+                    const uint32_t groups = ng - 4 * ks;              // groups left; those past K are skipped
                     const uint64_t b_desc = b_desc0 + (uint64_t)((sb * b_slot) >> 4);
                     auto multiply = [&](uint32_t g) {                 // one group: 16 columns of K per MMA, 8 TMEM columns of A, 32 bytes of B
                         if (g > 0 && groups <= g) return;
@@ -744,101 +629,22 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map0, const __grid_cons
         // packed codes of the row: 128 bytes whose 16-byte chunks sit at chunk ^ (row % 8) (128-byte TMA swizzle)
         const uint32_t raw_off = base + r * 128 + (((2 * gc) ^ (r & 7u)) << 4);
         const uint32_t sc_off = base + plan.off_sc + (r / kMatRows) * 2 * plan.plane_bytes + (r % kMatRows) * ng * 2 + gc * 2;
-        const uint32_t row_planes = sc_off - gc * 2;             // the row's scales from group 0 on
         const uint32_t a_lane = a_ring + ((q * kWarp) << 16) + gc * 32;
         uint32_t sr = 0, ur = 0, sc = 0, uc = 0, count = 0;      // count: stages so far; stage c is the (c / 2)-th use of slot c % 2
         for (uint32_t tile = first_tile; tile < total_tiles && !fail; tile += tile_step) {
-            // kQmmExact: scaled, and by then landed: the epilogue warps read the planes first
-            if (!q_mbar_wait(EXACT ? bar_scaled(sc) : bar_full_sc(sc), uc & 1)) { fail = kErrQmmTimeout | 8; break; }
+            if (!q_mbar_wait(bar_full_sc(sc), uc & 1)) { fail = kErrQmmTimeout | 8; break; }
             const uint32_t sc_base = sc_off + sc * plan.sc_bytes;
-            float row_scale = 1.0f;
-            if constexpr (EXACT) row_scale = row_scales[sc * kQmmRows + r];
             for (uint32_t ks = 0; ks < ksteps; ++ks) {
                 const uint32_t slot = count & 1, ua = count >> 1;
-                if (EXACT && (kTeams == 1 || slot == team) && 4 * ks + gc + kTeams > ng) {
-                    // A stage with extra groups, apart from the others' code, which was slower with these branches in it.
-                    if (!q_mbar_wait(bar_full_raw(sr), ur & 1)) { fail = kErrQmmTimeout | 4; break; }
-                    const uint32_t src = raw_off + sr * kQmmRawBytes;
-                    uint4 c0 = q_lds128(src), c1 = q_lds128(src ^ 16u);           // the first group's codes, if it is one of the weights'
-                    __syncwarp();
-                    if (lane == 0) q_mbar_arrive_after(bar_empty_raw(sr), c0.x, c1.x);
-                    if (ua > 0 && !q_mbar_wait(bar_empty_a(slot), (ua - 1) & 1)) { fail = kErrQmmTimeout | 5; break; }
-                    tc_fence_after();
-#pragma unroll 1
-                    for (uint32_t h = 0; h < kTeams; ++h) {
-                        const uint32_t G = 4 * ks + gc + h;
-                        if (G >= ngx) break;
-                        uint4 out[8];
-                        if (G < ng) {                             // one group of the weights at the most: ng % 4 == 1 or 3
-                            const float sf = bf16_bits_to_float((uint16_t)q_lds16(sc_base + ks * 8 + h * 2)) * row_scale;
-                            const FastScale<NATURAL_K> s2(sf);
-                            const __half2 b2 = __float2half2_rn(-8.0f * sf);
-                            out[0] = dequant8_fast<NATURAL_K>(c0.x, s2, b2); out[1] = dequant8_fast<NATURAL_K>(c0.y, s2, b2);
-                            out[2] = dequant8_fast<NATURAL_K>(c0.z, s2, b2); out[3] = dequant8_fast<NATURAL_K>(c0.w, s2, b2);
-                            out[4] = dequant8_fast<NATURAL_K>(c1.x, s2, b2); out[5] = dequant8_fast<NATURAL_K>(c1.y, s2, b2);
-                            out[6] = dequant8_fast<NATURAL_K>(c1.z, s2, b2); out[7] = dequant8_fast<NATURAL_K>(c1.w, s2, b2);
-                        } else {                                  // see qmm_extra_groups
-                            const uint32_t g0 = (G - ng) * kQmmPerExtra, at = row_planes + sc * plan.sc_bytes + g0 * 2;
-                            const float up = row_scale * 64.0f;
-                            uint32_t w[32];
-#pragma unroll
-                            for (int i = 3 * (int)kQmmPerExtra / 2; i < 32; ++i) w[i] = 0u;
-#pragma unroll
-                            for (int j = 0; j < (int)kQmmPerExtra; j += 4) {
-                                uint2 s4 = make_uint2(0u, 0u), b4 = s4;
-                                if (ng % 4 == 0) {
-                                    if (g0 + j < ng) {
-                                        asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(s4.x), "=r"(s4.y) : "r"(at + j * 2));
-                                        asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(b4.x), "=r"(b4.y) : "r"(at + plan.plane_bytes + j * 2));
-                                    }
-                                } else {
-                                    uint32_t v[8];
-#pragma unroll
-                                    for (int i = 0; i < 4; ++i) {
-                                        const bool in = g0 + j + i < ng;
-                                        v[i] = in ? q_lds16(at + (j + i) * 2) : 0u;
-                                        v[4 + i] = in ? q_lds16(at + plan.plane_bytes + (j + i) * 2) : 0u;
-                                    }
-                                    s4 = make_uint2(v[0] | v[1] << 16, v[2] | v[3] << 16);
-                                    b4 = make_uint2(v[4] | v[5] << 16, v[6] | v[7] << 16);
-                                }
-#pragma unroll
-                                for (int i = 0; i < 2; ++i) {
-                                    const uint32_t sp = i ? s4.y : s4.x, bp = i ? b4.y : b4.x;
-                                    const float c0 = fmaf(8.0f, __uint_as_float(sp << 16), __uint_as_float(bp << 16)) * up;
-                                    const float c1 = fmaf(8.0f, __uint_as_float(sp & 0xFFFF0000u), __uint_as_float(bp & 0xFFFF0000u)) * up;
-                                    const __half2 hi = __floats2half2_rn(c0, c1), low = __hmul2(hi, __half2half2(__ushort_as_half(0x1000)));      // 2^-11
-                                    const float2 hf = __half22float2(hi);
-                                    const __half2 lo = __floats2half2_rn(c0 - hf.x, c1 - hf.y);
-                                    w[j / 2 + i] = *reinterpret_cast<const uint32_t*>(&hi);
-                                    w[kQmmPerExtra / 2 + j / 2 + i] = *reinterpret_cast<const uint32_t*>(&low);
-                                    w[kQmmPerExtra + j / 2 + i] = *reinterpret_cast<const uint32_t*>(&lo);
-                                }
-                            }
-#pragma unroll
-                            for (int i = 0; i < 8; ++i) out[i] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
-                        }
-                        __syncwarp();
-                        tc_st32(a_lane + slot * 128 + h * 32, out);
-                    }
-                    tc_wait_st();
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) q_mbar_arrive(bar_full_a(slot));
-                } else if (kTeams == 1 || slot == team) {
+                if (kTeams == 1 || slot == team) {
                     const uint32_t left = ng - 4 * ks > gc ? ng - 4 * ks - gc : 0;         // groups past K are neither dequantised nor multiplied
                     float sf[kTeams], bf[kTeams];
                     bool fast[kTeams];
 #pragma unroll
                     for (uint32_t h = 0; h < kTeams; ++h) {
                         sf[h] = left > h ? bf16_bits_to_float((uint16_t)q_lds16(sc_base + ks * 8 + h * 2)) : 0.0f;
-                        if constexpr (EXACT) {
-                            sf[h] *= row_scale;
-                            bf[h] = -8.0f * sf[h];
-                        } else {
-                            bf[h] = left > h ? bf16_bits_to_float((uint16_t)q_lds16(sc_base + plan.plane_bytes + ks * 8 + h * 2)) : 0.0f;
-                        }
-                        fast[h] = EXACT || __all_sync(kFullMask, fabsf(sf[h]) < FastScale<NATURAL_K>::kLimit);       // kQmmExact: by its power of two
+                        bf[h] = left > h ? bf16_bits_to_float((uint16_t)q_lds16(sc_base + plan.plane_bytes + ks * 8 + h * 2)) : 0.0f;
+                        fast[h] = __all_sync(kFullMask, fabsf(sf[h]) < FastScale<NATURAL_K>::kLimit);
                     }
                     if (!q_mbar_wait(bar_full_raw(sr), ur & 1)) { fail = kErrQmmTimeout | 4; break; }
                     const uint32_t src = raw_off + sr * kQmmRawBytes;
@@ -865,10 +671,7 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map0, const __grid_cons
                         }
                         if (h == 0) {
                             __syncwarp();
-                            if (lane == 0) {                      // the codes are in registers
-                                if constexpr (EXACT) q_mbar_arrive_after(bar_empty_raw(sr), out[0].x ^ c[2 * kTeams - 2].x, out[7].w ^ c[2 * kTeams - 1].x);
-                                else q_mbar_arrive(bar_empty_raw(sr));
-                            }
+                            if (lane == 0) q_mbar_arrive(bar_empty_raw(sr));      // the codes are in registers
                             if (ua > 0 && !q_mbar_wait(bar_empty_a(slot), (ua - 1) & 1)) { fail = kErrQmmTimeout | 5; break; }
                             tc_fence_after();
                         }
@@ -903,50 +706,9 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map0, const __grid_cons
         const uint32_t mrow = r % kMatRows;
         const uint32_t pos = (NMAT == 2 && !NATURAL_K) ? permuted_col(mrow) : mrow;      // the GeGLU output feeds the down GEMM
         uint32_t buf = 0, uacc = 0, flip = 0, turn = 0;
-        // kQmmExact: the power of two for this row of a tile, found ahead of the dequantisers: the greatest |s| below 2^-6, the
-        // greatest |b| below 2^8 (pairs of magnitudes compare as integers)
-        const uint32_t row_sc = base + plan.off_sc + (r / kMatRows) * 2 * plan.plane_bytes + (r % kMatRows) * ng * 2;
-        uint32_t psc = 0, puc = 0, esc = 0;
-        auto greatest = [&](uint32_t at) {
-            uint32_t top = 0;
-            if (ng % 4 == 0) {
-#pragma unroll 4
-                for (uint32_t g = 0; g < ng; g += 4) {
-                    uint2 v;
-                    asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(at + g * 2));
-                    top = __vmaxu2(top, __vmaxu2(v.x & 0x7FFF7FFFu, v.y & 0x7FFF7FFFu));
-                }
-            } else {                                              // whole words around the row's halves
-                const uint32_t end = at + ng * 2;
-#pragma unroll 4
-                for (uint32_t a = at & ~3u; a < end; a += 4) {
-                    uint32_t v;
-                    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
-                    v &= (a < at ? 0x7FFF0000u : 0x7FFF7FFFu) & (a + 4 > end ? 0x7FFFu : 0x7FFF7FFFu);
-                    top = __vmaxu2(top, v);
-                }
-            }
-            return (int)(max(top & 0xFFFFu, top >> 16) >> 7);     // biased exponent
-        };
-        auto scale_rows = [&]() {
-            if (!q_mbar_wait(bar_full_sc(psc), puc & 1)) { fail = kErrQmmTimeout | 10; return; }
-            const uint32_t at = row_sc + psc * plan.sc_bytes;
-            const int e = min(max(max(greatest(at), greatest(at + plan.plane_bytes) - 14), 1), 246);
-            row_scales[psc * kQmmRows + r] = __uint_as_float((uint32_t)(247 - e) << 23);
-            __syncwarp();
-            if (lane == 0) q_mbar_arrive(bar_scaled(psc));
-            if (++psc == plan.sc_bufs) { psc = 0; ++puc; }
-        };
-        uint32_t stile = first_tile;
-        if constexpr (EXACT) {
-            if (stile < total_tiles) { scale_rows(); stile += tile_step; }
-        }
         for (uint32_t tile = first_tile; tile < total_tiles && !fail; tile += tile_step, tl.next()) {
             tl.locate(table, ngroups, lane);
             const uint32_t first = (tl.wt * kCtas + rank) * kMatRows;
-            if constexpr (EXACT) {
-                if (stile < total_tiles && !fail) { scale_rows(); stile += tile_step; }
-            }
             const uint32_t left = first < args.rows ? args.rows - first : 0, nrows = left < kMatRows ? left : kMatRows;
             const bool two = kTwoIssuers && ksteps > 1;                     // both issuers had stages of the tile
             const uint32_t one = kTwoIssuers ? turn : 0;                     // the issuer of its first stage
@@ -960,94 +722,7 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map0, const __grid_cons
             tc_fence_after();
             const uint32_t acc = tmem_base + ((q * kWarp) << 16) + (kTwoIssuers ? 2 * buf + one : buf) * kAccTok;
             const uint32_t acc2 = tmem_base + ((q * kWarp) << 16) + (2 * buf + (one ^ 1)) * kAccTok;      // the other issuer's
-            float unscale = 1.0f;
-            if constexpr (EXACT) unscale = __uint_as_float((254u << 23) - __float_as_uint(row_scales[esc * kQmmRows + r]));
             uint32_t which = 0;
-            if constexpr (EXACT) {
-                // 16 tokens at a time: most tiles have no more, and the code of 32 (below) next to the dequantisers' exceeds what the SM's
-                // instruction cache holds (warps stalled for instructions 2.2 per issued one in the down launch instead of 0.5)
-#pragma unroll 1
-                for (uint32_t c0 = 0; c0 < tl.ntok; c0 += 16, which ^= 1) {
-                    uint32_t v[16];
-                    __syncwarp();                                 // the lanes part in the stores at the end of a turn
-                    tc_ld16(acc + c0, v);
-                    tc_wait_ld();
-                    if (two) {
-                        uint32_t v2[16];
-                        tc_ld16(acc2 + c0, v2);
-                        tc_wait_ld();
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(v2[j]));
-                    }
-                    if (c0 + 16 >= tl.ntok) {                     // the accumulators are in registers
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) q_mbar_arrive(bar_acc_empty(buf));
-                    }
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * unscale);
-                    const uint32_t stage = stage0 + which * (32 * kTokBytes);
-                    constexpr uint32_t kVecs = kTokBytes / 16;
-                    if constexpr (NMAT == 2) {
-                        // each side hands half of the tokens to the other, as below
-                        const bool gate_side = q < 2;
-                        const uint32_t xrow = xch + mrow * 4, give = xrow + (gate_side ? 8 * 256 : 0), take = xrow + (gate_side ? 0 : 8 * 256);
-                        uint32_t own[8], other[8];
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) {
-                            own[j] = gate_side ? v[j] : v[8 + j];
-                            asm volatile("st.shared.b32 [%0], %1;" ::"r"(give + j * 256), "r"(gate_side ? v[8 + j] : v[j]) : "memory");
-                        }
-                        asm volatile("barrier.sync 1, 128;" ::: "memory");
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) asm volatile("ld.shared.b32 %0, [%1];" : "=r"(other[j]) : "r"(take + j * 256));
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) {
-                            float gt = __uint_as_float(gate_side ? own[j] : other[j]), up = __uint_as_float(gate_side ? other[j] : own[j]);
-                            if (args.round_gate_up) {             // Kernels/MoE/SharedExpertInt4.swift:62-93
-                                gt = __half2float(__float2half_rn(gt));
-                                up = __half2float(__float2half_rn(up));
-                            }
-                            const uint16_t a = __half_as_ushort(__float2half_rn(gelu_tanh(gt) * up));        // prefill.metal:634-636
-                            asm volatile("st.shared.b16 [%0], %1;" ::"r"(stage + pos * 2 + ((gate_side ? 0 : 8) + j) * kTokBytes), "h"(a) : "memory");
-                        }
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 16; ++j)
-                            asm volatile("st.shared.b16 [%0], %1;" ::"r"(stage + pos * 2 + j * kTokBytes), "h"(__half_as_ushort(__float2half_rn(__uint_as_float(v[j])))) : "memory");
-                    }
-                    asm volatile("barrier.sync 1, 128;" ::: "memory");
-#pragma unroll
-                    for (int i = 0; i < (int)(16 * kVecs / 128); ++i) {
-                        const uint32_t w = et + i * 128, tok = w / kVecs, c = w % kVecs;
-                        const uint4 d = q_lds128(stage + tok * kTokBytes + c * 16);
-                        uint16_t* o = args.out + (size_t)(tl.row0 + c0 + tok) * args.out_stride;
-                        if constexpr (NMAT == 2) {                // a tile's 64 outputs of a token are one group of the down projection
-                            const uint32_t dw4[4] = {d.x, d.y, d.z, d.w};
-                            float sum = 0.0f;
-#pragma unroll
-                            for (int e = 0; e < 4; ++e) {
-                                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&dw4[e]));
-                                sum += f.x + f.y;
-                            }
-#pragma unroll
-                            for (int s2 = 1; s2 < (int)kVecs; s2 <<= 1) sum += __shfl_xor_sync(kFullMask, sum, s2);
-                            if (c0 + tok < tl.ntok) {
-                                uint16_t* x = o + args.rows + tl.wt / kQmmPerExtra * kGroup;
-                                const uint32_t j = tl.wt % kQmmPerExtra;
-                                if (c < 3) {
-                                    x[c * kQmmPerExtra + j] = qmm_extra_value(sum, c);
-                                    if (tl.wt + 1 == wrow_tiles)              // what the last of the 64 columns does not fill is zero
-                                        for (uint32_t z = j + 1; z < kQmmPerExtra; ++z) x[c * kQmmPerExtra + z] = 0;
-                                }
-                                if (j == 0)
-                                    for (uint32_t z = 3 * kQmmPerExtra + c; z < (uint32_t)kGroup; z += kVecs) x[z] = 0;
-                            }
-                        }
-                        if (c0 + tok < tl.ntok && c * 8 < nrows) *reinterpret_cast<uint4*>(o + first + c * 8) = d;
-                    }
-                }
-            } else
             for (uint32_t c0 = 0; c0 < tl.ntok; c0 += 32, which ^= 1) {
                 uint32_t va[16], vb[16];
                 tc_ld16(acc + c0, va);
@@ -1139,7 +814,6 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map0, const __grid_cons
                 }
             }
             if (++buf == 2) { buf = 0; ++uacc; }
-            if constexpr (EXACT) { if (++esc == plan.sc_bufs) esc = 0; }
         }
     }
     if (fail && lane == 0) atomicCAS(args.error, 0u, fail);
@@ -1210,19 +884,17 @@ static tf_status make_w_map(tf_context* ctx, CUtensorMap* map, const void* w, ui
 // planes are then copied between two tiles, which costs less than halving the tokens per tile (2000 x 2112 x 8192: 104 us with
 // one buffer, 152 with two and tiles of 64 tokens).
 constexpr uint32_t kQmmMaxK = 9024;
-static bool qmm_plan(uint32_t k, uint32_t nmat, QmmPlan* p, bool exact = false) {
+static bool qmm_plan(uint32_t k, uint32_t nmat, QmmPlan* p) {
     if (k > kQmmMaxK) return false;
     const uint32_t budget = 227u * 1024u - 1024u;                  // less the alignment slack
     const uint32_t ng = k / kGroup;
-    const uint32_t exact_bytes = exact ? 4u * kQmmRows * 4u + 256u : 0u;      // rows' scales; static shared memory
     p->plane_bytes = ((kQmmRows / nmat) * ng * 2u + 15u) & ~15u;
     p->sc_bytes = nmat * 2 * p->plane_bytes;
     const uint32_t slot = kQmmBoxMax * kQmmRowBytes;                // 32 KB
     uint32_t fixed = 0;
     p->raw_stages = 0;
-    for (p->sc_bufs = 4 * p->sc_bytes <= 48u * 1024u ? 4u : 2u;; p->sc_bufs = 1) {      // exact: the next tile's planes beside this one's
-        if (exact && p->sc_bufs == 1) return false;
-        fixed = p->sc_bufs * p->sc_bytes + kQmmStageBytes + TF_MAX_ROUTER_EXPERTS * 16u + 1024u + exact_bytes;
+    for (p->sc_bufs = 4 * p->sc_bytes <= 48u * 1024u ? 4u : 2u;; p->sc_bufs = 1) {
+        fixed = p->sc_bufs * p->sc_bytes + kQmmStageBytes + TF_MAX_ROUTER_EXPERTS * 16u + 1024u;
         for (uint32_t raw = kQmmRawMax; raw >= 2 && !p->raw_stages; raw -= 2)         // even: a slot belongs to one team of dequantisers
             if (fixed + raw * kQmmRawBytes + 2 * slot <= budget) p->raw_stages = raw;
         if (p->raw_stages) break;
@@ -1234,9 +906,7 @@ static bool qmm_plan(uint32_t k, uint32_t nmat, QmmPlan* p, bool exact = false) 
     p->off_stage = p->off_sc + p->sc_bufs * p->sc_bytes;
     p->off_table = p->off_stage + kQmmStageBytes;
     p->off_bars = p->off_table + TF_MAX_ROUTER_EXPERTS * 16u;
-    p->off_exact = p->off_bars + 1024u;
     p->total = p->off_bars + 1024u + 1024u;
-    p->total += exact_bytes;
     return true;
 }
 
@@ -1296,7 +966,7 @@ static tf_status launch_qmm_kernel(tf_context* ctx, void* stream, QmmArgs& a, co
     TF_REQUIRE(ctx, a.k % kGroup == 0 && a.k >= (uint32_t)kGroup, TF_ERR_INVALID_ARGUMENT, "%s: K must be a positive multiple of 64", name);
     TF_REQUIRE(ctx, a.rows % 8 == 0 && a.rows > 0, TF_ERR_INVALID_ARGUMENT, "%s: the weight rows must be a positive multiple of 8", name);
     TF_REQUIRE(ctx, aligned(x, 16) && (x_stride * 2) % 16 == 0, TF_ERR_ALIGNMENT, "%s: activation rows must be 16-byte aligned", name);
-    TF_REQUIRE(ctx, qmm_plan(a.k, NMAT, &a.plan, FORM == kQmmExact), TF_ERR_UNSUPPORTED, "%s: K=%u needs more shared memory for the scale planes than there is", name, a.k);
+    TF_REQUIRE(ctx, qmm_plan(a.k, NMAT, &a.plan), TF_ERR_UNSUPPORTED, "%s: K=%u needs more shared memory for the scale planes than there is", name, a.k);
     constexpr uint32_t kMatRows = kQmmRows / NMAT;
     // Activation boxes: see the kernel. A dense launch knows its tiles (full ones and a last one) and encodes only the boxes of
     // those: an encode is most of a microsecond of host time, and small products are bound by it.
@@ -1318,7 +988,7 @@ static tf_status launch_qmm_kernel(tf_context* ctx, void* stream, QmmArgs& a, co
     int some = -1;
     for (int i = 0; i < 4; ++i) {
         if (box[i] == 0) continue;
-        if (tf_status s = make_x_map(ctx, &xmap[i], x, x_rows, a.k + a.extra * kGroup, x_stride, box[i], name)) return s;
+        if (tf_status s = make_x_map(ctx, &xmap[i], x, x_rows, a.k, x_stride, box[i], name)) return s;
         some = i;
     }
     for (int i = 0; i < 4; ++i)
@@ -1329,9 +999,8 @@ static tf_status launch_qmm_kernel(tf_context* ctx, void* stream, QmmArgs& a, co
     a.expert_stride = dense ? 0 : expert_stride;
     a.out_vec = aligned(a.out, 16) && a.out_stride % 8 == 0 ? 1u : 0u;
     a.error = ctx->device_error;
-    if (dense && FORM != kQmmExact) {
+    if (dense)
         if (tf_status s = launch_qmm_prepare(ctx, stream, a, kQmmDenseTable, name)) return s;
-    }
     auto kern = qmm_tcgen05_kernel<NMAT, NATURAL_K, FORM>;
     static DeviceSmemCache configured;
     if (tf_status s = ensure_dynamic_smem(ctx, kern, configured, a.plan.total)) return s;
@@ -1362,81 +1031,6 @@ static tf_status launch_qmm(tf_context* ctx, void* stream, QmmArgs& a, const voi
 
 tf_status launch_qmm_generic(tf_context* ctx, void* stream, const uint8_t* W, const uint16_t* S, const uint16_t* B,
                              const uint16_t* X, uint16_t* Y, uint32_t m, uint32_t n, uint32_t k, const char* name);   // qmm_generic.cu
-
-}  // namespace tf
-
-namespace tf {
-
-uint32_t qmm_exact_columns(uint32_t k) { return k + qmm_extra_groups(k) * kGroup; }
-
-// The routed experts of a block without a rounding of the weights (kQmmExact). x_sorted: rows of qmm_exact_columns(d) for the sorted pairs, filled
-// here, as is inverse_perm; acts: rows of qmm_exact_columns(f).
-tf_status grouped_moe_exact(tf_context* ctx, void* stream, const void* x, uint32_t x_stride_elements, uint32_t tokens, uint32_t top_k, void* x_sorted,
-                            uint32_t* inverse_perm, const void* pool_layer_base, uint64_t expert_stride, uint32_t num_experts,
-                            const tf_expert_offsets* offsets, const tf_device_routes* routes, void* acts_scratch, void* out_rows, uint32_t d, uint32_t f) {
-    const uint32_t rows = tokens * top_k, per_block = kExtendThreads / kWarp;
-    launch_pdl(qmm_extend_rows_kernel<true>, dim3((rows + per_block - 1) / per_block), dim3(kExtendThreads), 0, static_cast<cudaStream_t>(stream),
-               static_cast<const uint16_t*>(x), x_stride_elements, rows, d, static_cast<uint16_t*>(x_sorted), qmm_exact_columns(d),
-               static_cast<const tf_pair*>(routes->sorted_pairs), static_cast<const uint32_t*>(routes->counters) + 3, top_k, inverse_perm);
-    if (tf_status s = check_launch(ctx, "qmm_extend_rows")) return s;
-    const uint8_t* pool = static_cast<const uint8_t*>(pool_layer_base);
-    auto plane = [&](uint32_t off) { return reinterpret_cast<const uint16_t*>(pool + off); };
-    QmmArgs a{}, b{};
-    a.S[0] = plane(offsets->gate_s_off); a.B[0] = plane(offsets->gate_b_off);
-    a.S[1] = plane(offsets->up_s_off);   a.B[1] = plane(offsets->up_b_off);
-    b.S[0] = plane(offsets->down_s_off); b.B[0] = plane(offsets->down_b_off);
-    a.route_groups = b.route_groups = routes->groups; a.route_counters = b.route_counters = routes->counters;
-    a.ctas = b.ctas = 1;
-    a.rows = f; a.k = d; a.out = static_cast<uint16_t*>(acts_scratch); a.out_stride = qmm_exact_columns(f); a.extra = qmm_extra_groups(d);
-    b.rows = d; b.k = f; b.out = static_cast<uint16_t*>(out_rows); b.out_stride = d; b.extra = qmm_extra_groups(f);
-    b.after_gate_up = 1;
-    const uint8_t* w_gu[2] = {pool + offsets->gate_w_off, pool + offsets->up_w_off};
-    if (tf_status s = launch_qmm_kernel<2, false, kQmmExact>(ctx, stream, a, x_sorted, rows, qmm_exact_columns(d), w_gu, num_experts, expert_stride, false,
-                                                             "grouped_moe_exact(gate/up)")) return s;
-    const uint8_t* w_dn[2] = {pool + offsets->down_w_off, pool + offsets->down_w_off};
-    return launch_qmm_kernel<1, false, kQmmExact>(ctx, stream, b, acts_scratch, rows, qmm_exact_columns(f), w_dn, num_experts, expert_stride, false,
-                                                  "grouped_moe_exact(down)");
-}
-
-// The shared expert of such a block. x_ext: rows of qmm_exact_columns(d), filled here; act: rows of qmm_exact_columns(fs).
-tf_status shared_expert_exact(tf_context* ctx, void* stream, const void* x, uint32_t x_stride_elements, const tf_projection* gate, const tf_projection* up,
-                              const tf_projection* down, void* x_ext, void* scratch_act, void* y, uint32_t rows) {
-    const uint32_t fs = gate->rows, d = gate->cols, per_block = kExtendThreads / kWarp;
-    const uint8_t* W[3]; const uint16_t* S[3]; const uint16_t* B[3];
-    const tf_projection* ps[3] = {gate, up, down};
-    for (int i = 0; i < 3; ++i) {
-        W[i] = byte_ptr(ps[i]->weights, ps[i]->weights_off);
-        S[i] = reinterpret_cast<const uint16_t*>(byte_ptr(ps[i]->scales, ps[i]->scales_off));
-        B[i] = reinterpret_cast<const uint16_t*>(byte_ptr(ps[i]->biases, ps[i]->biases_off));
-    }
-    launch_pdl(qmm_extend_rows_kernel<false>, dim3((rows + per_block - 1) / per_block), dim3(kExtendThreads), 0, static_cast<cudaStream_t>(stream),
-               static_cast<const uint16_t*>(x), x_stride_elements, rows, d, static_cast<uint16_t*>(x_ext), qmm_exact_columns(d),
-               static_cast<const tf_pair*>(nullptr), static_cast<const uint32_t*>(nullptr), 1u, static_cast<uint32_t*>(nullptr));
-    if (tf_status s = check_launch(ctx, "qmm_extend_rows")) return s;
-    auto per_tile = [&](uint32_t n, uint32_t mat_rows, uint32_t stages) {           // the cost of kQmmFew in qmm_dense_tiles
-        uint32_t best = 16;
-        uint64_t best_cost = ~0ull;
-        for (uint32_t per = kQmmBoxMax; per >= 16; per -= 16) {
-            const uint64_t tiles = (uint64_t)((n + mat_rows - 1) / mat_rows) * ((rows + per - 1) / per);
-            const uint64_t cost = (tiles + ctx->sm_count - 1) / ctx->sm_count * ((uint64_t)stages * (7800 + 65 * per) + 7400);
-            if (cost < best_cost) { best_cost = cost; best = per; }
-        }
-        return best;
-    };
-    QmmArgs a{}, b{};
-    a.S[0] = S[0]; a.B[0] = B[0]; a.S[1] = S[1]; a.B[1] = B[1];
-    b.S[0] = S[2]; b.B[0] = B[2];
-    a.ctas = b.ctas = 1;
-    a.dense_tokens = b.dense_tokens = rows;
-    a.dense_per_tile = per_tile(fs, kQmmRows / 2, (qmm_exact_columns(d) + kQmmStageK - 1) / kQmmStageK);
-    b.dense_per_tile = per_tile(d, kQmmRows, (qmm_exact_columns(fs) + kQmmStageK - 1) / kQmmStageK);
-    a.rows = fs; a.k = d; a.out = static_cast<uint16_t*>(scratch_act); a.out_stride = qmm_exact_columns(fs); a.round_gate_up = 1; a.extra = qmm_extra_groups(d);
-    b.rows = d; b.k = fs; b.out = static_cast<uint16_t*>(y); b.out_stride = d; b.extra = qmm_extra_groups(fs);
-    const uint8_t* w_gu[2] = {W[0], W[1]};
-    if (tf_status s = launch_qmm_kernel<2, true, kQmmExact>(ctx, stream, a, x_ext, rows, qmm_exact_columns(d), w_gu, 1, 0, true, "shared_expert_exact(gate/up)")) return s;
-    const uint8_t* w_dn[2] = {W[2], W[2]};
-    return launch_qmm_kernel<1, true, kQmmExact>(ctx, stream, b, scratch_act, rows, qmm_exact_columns(fs), w_dn, 1, 0, true, "shared_expert_exact(down)");
-}
 
 }  // namespace tf
 

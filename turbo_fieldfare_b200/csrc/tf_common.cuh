@@ -73,11 +73,8 @@ struct tf_context {
     cudaEvent_t fork_event = nullptr, join_event = nullptr;
     // Block forwards of at least this many tokens run their expert GEMMs on the tcgen05 tensor cores.
     uint32_t tensorcore_min_tokens = 256;
-    // Set by a caller: the blocks below it then keep to the CUDA-core kernels (block_exact).
-    bool tensorcore_min_set = false;
     // The same for the shared expert alone (a dense GEMM over all tokens of the block).
     uint32_t shared_tensorcore_min_tokens = 256;
-    bool shared_tensorcore_min_set = false;
     // Fixed-capacity expert-parallel exchanges whose expected rows per local expert (ranks x tokens x top_k / experts of
     // a rank) reach this number run the owner's expert phase on the tensor cores. Off by default (measured slower at eight
     // ranks x 64 tokens, 32 rows per expert: 6.62 ms against 5.98 ms per step).
