@@ -286,3 +286,26 @@ def test_shared_expert_tensorcore_wide_tiles(tf_ctx, oracle, T, D, Fs):
 @pytest.mark.parametrize("M,N,K", [(900, 2120, 2112), (2000, 2120, 1344), (1000, 2112, 2816)])
 def test_int4_qmm_pairs_past_the_matrix(tf_ctx, oracle, M, N, K):
     test_int4_qmm_vs_oracle(tf_ctx, oracle, M, N, K)
+
+
+# Every form over many stages per CTA, so that each ring slot of codes is refilled many times: forty dispatches give the same bytes, and the first
+# agrees with the oracle. Tiles by one CTA of up to 64 tokens, of more, pairs.
+@pytest.mark.parametrize("M,N,K", [(64, 20000, 1088), (700, 5000, 704), (3000, 2120, 2816)])
+def test_int4_qmm_forms_repeat_byte_for_byte(tf_ctx, oracle, M, N, K):
+    import torch
+    from turbo_fieldfare_b200.kernels import MPPPrefillInt4QMM
+    o = oracle
+    rng = np.random.default_rng(M + N + K)
+    mat = config0_matrix(o, N, K, rng)
+    x16 = o.f32_to_f16(rng.standard_normal((M, K)).astype(np.float32))
+    W, S, B, X = to_dev(mat.packed), to_dev(mat.scales), to_dev(mat.biases), to_dev(x16)
+    first = None
+    for _ in range(40):
+        y = dev_zeros_u16(M * N, fill=0x7E00)
+        MPPPrefillInt4QMM(tf_ctx).encode(W, S, B, X, y, M, N, K)
+        first = y if first is None else first
+        assert torch.equal(first, y)
+    _status_ok(tf_ctx)
+    rows = [0, M // 2, M - 1]
+    got = o.f16_to_f32(from_dev(first, np.uint16).reshape(M, N)[rows])
+    assert o.rel_l2(got, o.int4_qmm_ref(mat, np.ascontiguousarray(x16[rows]))) < QMM_TOL

@@ -18,6 +18,15 @@ __device__ __forceinline__ void mbar_init(uint32_t addr, uint32_t count) {
 __device__ __forceinline__ void mbar_arrive(uint32_t addr) {
     asm volatile("{ .reg .b64 st; mbarrier.arrive.shared::cta.b64 st, [%0]; }" ::"r"(addr) : "memory");
 }
+// Hands a slot back after loads from it, once a and b are in registers: both arms arrive, but which one takes their values. A plain arrival
+// waits for no load: neither for data that is still on its way nor for one that the compiler has moved to its first use behind the arrival
+// (a tensor-core GEMM whose use was behind it had single rows with the weights of two stages later). a and b together depend on every
+// load from the slot.
+__device__ __forceinline__ void mbar_arrive_after(uint32_t addr, uint32_t a, uint32_t b) {
+    asm volatile("{ .reg .b64 st; .reg .pred p; setp.eq.u32 p, %1, %2;\n\t"
+                 "@p mbarrier.arrive.shared::cta.b64 st, [%0];\n\t@!p mbarrier.arrive.shared::cta.b64 st, [%0], 1; }" ::"r"(addr), "r"(a), "r"(b) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_after(uint32_t addr, float a, float b) { mbar_arrive_after(addr, __float_as_uint(a), __float_as_uint(b)); }
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t addr, uint32_t bytes) {
     asm volatile("{ .reg .b64 st; mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1; }" ::"r"(addr), "r"(bytes) : "memory");
 }

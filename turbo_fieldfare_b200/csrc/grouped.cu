@@ -720,9 +720,14 @@ grouped_ksplit_kernel(const GroupedArgs args) {
 #pragma unroll
                 for (int j = 0; j < 4; ++j) y[m][j] = acc[j] * 16777216.0f;
             }
-            // this warp is done with the stage (codes and scales are in registers or consumed)
+            // this warp is done with the stage: the sums of rows g and g + 8 of the matrices come of all of its loads
             __syncwarp();
-            if (lane == 0) mbar_arrive(bar_empty(st));
+            if (lane == 0) {
+                if constexpr (NMAT == 2)
+                    mbar_arrive_after(bar_empty(st), __float_as_uint(y[0][0]) ^ __float_as_uint(y[0][2]) ^ __float_as_uint(y[1][0]), __float_as_uint(y[1][2]));
+                else
+                    mbar_arrive_after(bar_empty(st), y[0][0], y[0][2]);
+            }
             // partial sums for the reducer: buffer li % kRedStages, 512 bytes per (warp, matrix, 8 tokens)
             const uint32_t r = li % kRedStages, ruse = li / kRedStages;
             if (!mbar_wait(bar_red_free(r), (ruse & 1) ^ 1)) { fail = kErrTimeoutRedFree; break; }
@@ -801,7 +806,7 @@ grouped_ksplit_kernel(const GroupedArgs args) {
                 }
             }
             __syncwarp();
-            if (lane == 0) mbar_arrive(bar_empty(st));               // this warp is done with the stage
+            if (lane == 0) mbar_arrive(bar_empty(st));               // this warp is done with the stage: its sums, of all loads, have been stored
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_part_full(li % kRedStages));
@@ -903,7 +908,7 @@ grouped_ksplit_kernel(const GroupedArgs args) {
                 }
                 if (n == NT - 1) {
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(bar_red_free(q));
+                    if (lane == 0) mbar_arrive_after(bar_red_free(q), acc[0].x, acc[NMAT - 1].y);
                 }
                 const float o0[4] = {acc[0].x, acc[0].y, acc[0].z, acc[0].w};
                 const float o1[4] = {acc[NMAT - 1].x, acc[NMAT - 1].y, acc[NMAT - 1].z, acc[NMAT - 1].w};
@@ -1091,7 +1096,7 @@ grouped_down_kernel(const GroupedArgs args) {
                 for (int j = 0; j < 4; ++j) y[j] = h == 0 ? acc[j] * 16777216.0f : y[j] + acc[j] * 16777216.0f;
             }
             __syncwarp();
-            if (lane == 0) mbar_arrive(bar_empty(st));
+            if (lane == 0) mbar_arrive_after(bar_empty(st), y[0], y[2]);      // sums of rows g and g + 8
             // y0, y1: row g, tokens 2t, 2t + 1; y2, y3: row g + 8
             const uint32_t row = cur.tile * kTileRows + g;
 #pragma unroll
