@@ -52,7 +52,7 @@ __global__ void fill_affine_kernel(uint8_t* W, uint16_t* S, uint16_t* B, uint64_
 constexpr int kRrnThreads = 128;
 constexpr int kRrnMaxSlices = 4;          // d <= 128 * 8 * 4 = 4096
 __global__ void __launch_bounds__(kRrnThreads)
-residual_rmsnorm_kernel(uint16_t* __restrict__ h, const uint16_t* __restrict__ y, const uint16_t* __restrict__ w,
+residual_rmsnorm_kernel(uint16_t* h, const uint16_t* y, const uint16_t* __restrict__ w,
                         uint16_t* __restrict__ x, uint32_t d, float eps) {
     __shared__ float red[kRrnThreads / kWarp];
     pdl_launch_dependents();
@@ -61,17 +61,21 @@ residual_rmsnorm_kernel(uint16_t* __restrict__ h, const uint16_t* __restrict__ y
     const uint32_t vecs = d / 8;
     float v[kRrnMaxSlices][8];
     float acc = 0.0f;
+    uint4 hv[kRrnMaxSlices], yv[kRrnMaxSlices];          // all loads before the first store
+#pragma unroll
+    for (int s = 0; s < kRrnMaxSlices; ++s) {
+        const uint32_t i = threadIdx.x + s * kRrnThreads;
+        hv[s] = yv[s] = make_uint4(0u, 0u, 0u, 0u);
+        if (i < vecs) {
+            hv[s] = *reinterpret_cast<const uint4*>(hr + i * 8);
+            if (y) yv[s] = *reinterpret_cast<const uint4*>(y + (size_t)blockIdx.x * d + i * 8);
+        }
+    }
 #pragma unroll
     for (int s = 0; s < kRrnMaxSlices; ++s) {
         const uint32_t i = threadIdx.x + s * kRrnThreads;
         if (i < vecs) {
-            const uint4 hv = *reinterpret_cast<const uint4*>(hr + i * 8);
-            const uint32_t hw[4] = {hv.x, hv.y, hv.z, hv.w};
-            uint32_t yw[4] = {0u, 0u, 0u, 0u};
-            if (y) {
-                const uint4 yv = __ldg(reinterpret_cast<const uint4*>(y + (size_t)blockIdx.x * d + i * 8));
-                yw[0] = yv.x; yw[1] = yv.y; yw[2] = yv.z; yw[3] = yv.w;
-            }
+            const uint32_t hw[4] = {hv[s].x, hv[s].y, hv[s].z, hv[s].w}, yw[4] = {yv[s].x, yv[s].y, yv[s].z, yv[s].w};
             uint32_t ow[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
@@ -117,7 +121,7 @@ residual_rmsnorm_kernel(uint16_t* __restrict__ h, const uint16_t* __restrict__ y
 // magnitude is zero or within fp16's normal range, since bf16 carries 8 significant bits and fp16 11; TO_BF16 = true:
 // fp16 -> bf16, round to nearest even). Eight elements per thread.
 template <bool TO_BF16>
-__global__ void convert_rows_kernel(const uint16_t* __restrict__ src, uint32_t src_stride, uint16_t* __restrict__ dst, uint32_t dst_stride,
+__global__ void convert_rows_kernel(const uint16_t* src, uint32_t src_stride, uint16_t* __restrict__ dst, uint32_t dst_stride,
                                     uint32_t rows, uint32_t d) {
     pdl_launch_dependents();
     pdl_wait();
@@ -155,8 +159,8 @@ __global__ void convert_rows_kernel(const uint16_t* __restrict__ src, uint32_t s
 constexpr int kCrnMaxThreads = kRrnThreads * kRrnMaxSlices;      // 512: d <= 4096
 template <bool ROWS>
 __global__ void __launch_bounds__(kCrnMaxThreads)
-combine_residual_rmsnorm_kernel(uint16_t* __restrict__ h, const void* __restrict__ results, const uint16_t* __restrict__ route_weights,
-                                const uint32_t* __restrict__ inverse_perm, const uint16_t* __restrict__ shared_y,
+combine_residual_rmsnorm_kernel(uint16_t* h, const void* results, const uint16_t* route_weights,
+                                const uint32_t* inverse_perm, const uint16_t* shared_y,
                                 const uint16_t* __restrict__ w, uint16_t* __restrict__ x, uint32_t d, uint32_t top_k, float eps,
                                 const PeerWait peer_wait) {
     __shared__ float chain[kRrnThreads];
@@ -174,21 +178,21 @@ combine_residual_rmsnorm_kernel(uint16_t* __restrict__ h, const void* __restrict
         for (int r = 0; r < TF_MAX_TOP_K; ++r) {
             if ((uint32_t)r < top_k) {
                 if constexpr (ROWS) {
-                    const uint32_t slot = __ldg(inverse_perm + (size_t)token * top_k + r);
+                    const uint32_t slot = inverse_perm[(size_t)token * top_k + r];
                     const uint4 rv = *reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(results) + (size_t)slot * d + i * 8);
                     p[r][0] = make_float4(__uint_as_float(rv.x), __uint_as_float(rv.y), __uint_as_float(rv.z), __uint_as_float(rv.w));
                 } else {
                     const float4* src = reinterpret_cast<const float4*>(static_cast<const float*>(results) + ((size_t)token * top_k + r) * d + i * 8);
-                    p[r][0] = __ldg(src); p[r][1] = __ldg(src + 1);
+                    p[r][0] = src[0]; p[r][1] = src[1];
                 }
-                rw[r] = f16_bits_to_float(__ldg(route_weights + (size_t)token * top_k + r));
+                rw[r] = f16_bits_to_float(route_weights[(size_t)token * top_k + r]);
             } else {
                 p[r][0] = make_float4(0.0f, 0.0f, 0.0f, 0.0f); p[r][1] = p[r][0]; rw[r] = 0.0f;
             }
         }
         const uint4 hv = *reinterpret_cast<const uint4*>(h + (size_t)token * d + i * 8);
         uint4 sv = make_uint4(0u, 0u, 0u, 0u);
-        if (shared_y) sv = __ldg(reinterpret_cast<const uint4*>(shared_y + (size_t)token * d + i * 8));
+        if (shared_y) sv = *reinterpret_cast<const uint4*>(shared_y + (size_t)token * d + i * 8);
         const uint32_t hw[4] = {hv.x, hv.y, hv.z, hv.w}, sw[4] = {sv.x, sv.y, sv.z, sv.w};
         uint32_t ow[4];
 #pragma unroll
@@ -267,8 +271,8 @@ combine_residual_rmsnorm_kernel(uint16_t* __restrict__ h, const void* __restrict
 // tokens x 8 rows of 2816, 277 MB: 71 to 74 us with a block per token, 49 to 51 here, 42 at the HBM rate.
 constexpr int kCrpThreads = 384;         // d <= 3072; two blocks per SM and more (wider rows keep the other form)
 __global__ void __launch_bounds__(kCrpThreads, 2)
-combine_rows_pipelined_kernel(uint16_t* __restrict__ h, const uint16_t* __restrict__ rows, const uint16_t* __restrict__ route_weights,
-                              const uint32_t* __restrict__ inverse_perm, const uint16_t* __restrict__ shared_y,
+combine_rows_pipelined_kernel(uint16_t* h, const uint16_t* rows, const uint16_t* route_weights,
+                              const uint32_t* inverse_perm, const uint16_t* shared_y,
                               const uint16_t* __restrict__ w, uint16_t* __restrict__ x, uint32_t d, uint32_t top_k, float eps, uint32_t tokens,
                               const PeerWait peer_wait) {
     __shared__ float chain[kRrnThreads];
@@ -297,7 +301,7 @@ combine_rows_pipelined_kernel(uint16_t* __restrict__ h, const uint16_t* __restri
         for (int r = 0; r < TF_MAX_TOP_K; ++r)
             if ((uint32_t)r < top_k) p[r] = *reinterpret_cast<const uint4*>(rows + (size_t)slot_of[buf][r] * d + i * 8);
         hv = *reinterpret_cast<const uint4*>(h + (size_t)tk * d + i * 8);
-        if (shared_y) sv = __ldg(reinterpret_cast<const uint4*>(shared_y + (size_t)tk * d + i * 8));
+        if (shared_y) sv = *reinterpret_cast<const uint4*>(shared_y + (size_t)tk * d + i * 8);
     };
     if (mine && token < tokens) request(token, 0);
     for (uint32_t buf = 0; token < tokens; token += gridDim.x, buf ^= 1) {

@@ -20,11 +20,11 @@ constexpr int kPackThreads = 256;
 // activation layout of the tensor-core grouped GEMM.
 template <bool PERMUTE_K8>
 __global__ void __launch_bounds__(kPackThreads)
-ep_pack_kernel(const uint16_t* __restrict__ hidden, uint32_t hidden_stride, const tf_pair* __restrict__ sorted_pairs,
-               const uint32_t* __restrict__ per_expert_counts, uint32_t n_pairs, uint32_t top_k, uint32_t num_experts,
+ep_pack_kernel(const uint16_t* hidden, uint32_t hidden_stride, const tf_pair* sorted_pairs,
+               const uint32_t* per_expert_counts, uint32_t n_pairs, uint32_t top_k, uint32_t num_experts,
                uint32_t experts_per_rank, uint32_t n_dst, uint32_t capacity, uint32_t d, uint32_t send_stride,
                uint16_t* __restrict__ send_rows, uint32_t* __restrict__ send_ids, uint32_t* __restrict__ inverse_perm,
-               uint32_t* __restrict__ overflow, const uint32_t* __restrict__ grouped_pairs) {
+               uint32_t* __restrict__ overflow, const uint32_t* grouped_pairs) {
     __shared__ uint32_t dst_base[257], dst_count[256];
     pdl_launch_dependents();
     pdl_wait();
@@ -71,22 +71,30 @@ ep_pack_kernel(const uint16_t* __restrict__ hidden, uint32_t hidden_stride, cons
     }
     const uint4* src = reinterpret_cast<const uint4*>(hidden + (size_t)pr.token * hidden_stride);
     uint4* dst_row = reinterpret_cast<uint4*>(send_rows + (size_t)slot * send_stride);
-    for (uint32_t i = lane; i < d / 8; i += kWarp) {
-        uint4 v = __ldg(src + i);
-        if (PERMUTE_K8) {
-            uint4 o;
-            asm("prmt.b32 %0, %1, %2, 0x5410;" : "=r"(o.x) : "r"(v.x), "r"(v.z));   // (k0, k4)
-            asm("prmt.b32 %0, %1, %2, 0x7632;" : "=r"(o.y) : "r"(v.x), "r"(v.z));   // (k1, k5)
-            asm("prmt.b32 %0, %1, %2, 0x5410;" : "=r"(o.z) : "r"(v.y), "r"(v.w));   // (k2, k6)
-            asm("prmt.b32 %0, %1, %2, 0x7632;" : "=r"(o.w) : "r"(v.y), "r"(v.w));   // (k3, k7)
-            v = o;
+    constexpr int kAtOnce = 4;                       // loads before the first store
+    for (uint32_t i0 = lane; i0 < d / 8; i0 += kAtOnce * kWarp) {
+        uint4 v[kAtOnce];
+#pragma unroll
+        for (int j = 0; j < kAtOnce; ++j)
+            if (i0 + j * kWarp < d / 8) v[j] = src[i0 + j * kWarp];
+#pragma unroll
+        for (int j = 0; j < kAtOnce; ++j) {
+            if (i0 + j * kWarp >= d / 8) break;
+            if (PERMUTE_K8) {
+                uint4 o;
+                asm("prmt.b32 %0, %1, %2, 0x5410;" : "=r"(o.x) : "r"(v[j].x), "r"(v[j].z));   // (k0, k4)
+                asm("prmt.b32 %0, %1, %2, 0x7632;" : "=r"(o.y) : "r"(v[j].x), "r"(v[j].z));   // (k1, k5)
+                asm("prmt.b32 %0, %1, %2, 0x5410;" : "=r"(o.z) : "r"(v[j].y), "r"(v[j].w));   // (k2, k6)
+                asm("prmt.b32 %0, %1, %2, 0x7632;" : "=r"(o.w) : "r"(v[j].y), "r"(v[j].w));   // (k3, k7)
+                v[j] = o;
+            }
+            dst_row[i0 + j * kWarp] = v[j];
         }
-        dst_row[i] = v;
     }
 }
 
 // ids[slot] = the id a row of `stride` > d elements carries in its tail (see ep_pack_kernel).
-__global__ void ep_extract_ids_kernel(const uint16_t* __restrict__ rows, uint32_t stride, uint32_t d, uint32_t slots,
+__global__ void ep_extract_ids_kernel(const uint16_t* rows, uint32_t stride, uint32_t d, uint32_t slots,
                                       uint32_t* __restrict__ ids) {
     const uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
     pdl_launch_dependents();
@@ -97,10 +105,10 @@ __global__ void ep_extract_ids_kernel(const uint16_t* __restrict__ rows, uint32_
 // y[t,d] = half(sum_r fma(w[t,r], partial[inverse[t*K+r]][d], acc) + residual[t,d]), rank order.
 // VEC: a thread owns eight consecutive columns (16-byte loads and stores; D a multiple of 8, rows 16-byte aligned).
 template <bool VEC>
-__global__ void ep_combine_kernel(const uint16_t* __restrict__ rows, const uint16_t* __restrict__ weights,
-                                  const uint32_t* __restrict__ inverse_perm, const uint16_t* __restrict__ residual,
+__global__ void ep_combine_kernel(const uint16_t* rows, const uint16_t* weights,
+                                  const uint32_t* inverse_perm, const uint16_t* residual,
                                   uint32_t residual_stride, uint16_t* __restrict__ out, uint32_t out_stride,
-                                  uint32_t T, uint32_t K, uint32_t D, const PeerWait peer_wait, const uint32_t* __restrict__ skip_ids) {
+                                  uint32_t T, uint32_t K, uint32_t D, const PeerWait peer_wait, const uint32_t* skip_ids) {
     peer_wait_in_block(peer_wait);      // the rows may come from peers that are still writing them
     // rows in grid.x (up to 2^31 - 1 blocks), column blocks in grid.y: an expert-parallel rank can hold more than 65535 rows
     const uint32_t t = blockIdx.x;

@@ -187,7 +187,7 @@ lm_head_argmax_kernel(const float* __restrict__ logits, uint32_t vocab, unsigned
 
 // Decodes the winner (0 when no logit was finite, lm_head_greedy_int4_rows_reduce's fallback) and clears the
 // scratch word for the next call.
-__global__ void lm_head_finish_kernel(unsigned long long* __restrict__ best, uint32_t* __restrict__ out_token) {
+__global__ void lm_head_finish_kernel(unsigned long long* best, uint32_t* __restrict__ out_token) {
     pdl_wait();
     const unsigned long long k = *best;
     *out_token = k ? ~(uint32_t)(k & 0xFFFFFFFFull) : 0u;

@@ -39,13 +39,13 @@ __device__ __forceinline__ unsigned long long argmax_key(float z, uint32_t row) 
 // x in MMA operand order and its group sums, by the whole block: the 16 values x0..x15 at columns 64 G + 16 t feed four MMAs,
 //   j = 0: (x0,x4),(x2,x6)   j = 1: (x1,x5)/16,(x3,x7)/16   j = 2, 3: the same for x8..x15
 // (odd columns are pre-scaled by 1/16 because their codes sit four mantissa bits higher)
-__device__ __forceinline__ void gm_stage_x(const uint16_t* __restrict__ x, uint32_t ng, uint32_t* xfrag, float* xsum, uint32_t threads) {
+__device__ __forceinline__ void gm_stage_x(const uint16_t* x, uint32_t ng, uint32_t* xfrag, float* xsum, uint32_t threads) {
     for (uint32_t idx = threadIdx.x; idx < ((ng * 4 + 31u) & ~31u); idx += threads) {   // whole warps: the sums use shuffles
         const bool ok = idx < ng * 4;
         const uint32_t G = idx >> 2, tt = idx & 3;
         const uint4* p = reinterpret_cast<const uint4*>(x + G * kGroup + tt * 16);
         uint4 lo = make_uint4(0u, 0u, 0u, 0u), hi = lo;
-        if (ok) { lo = __ldg(p); hi = __ldg(p + 1); }
+        if (ok) { lo = p[0]; hi = p[1]; }
         const uint32_t r[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
         float sum = 0.0f;
 #pragma unroll
@@ -125,7 +125,7 @@ __device__ __forceinline__ void gm_fold_argmax(unsigned long long mine, unsigned
 template <bool SB_FP16, bool ARGMAX, int WARPS>
 __global__ void __launch_bounds__(WARPS * kWarp)
 gemv_mma_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S, const uint16_t* __restrict__ B,
-                const uint16_t* __restrict__ x, uint16_t* __restrict__ y, uint32_t m, uint32_t n, const GemvBatch bt,
+                const uint16_t* x, uint16_t* __restrict__ y, uint32_t m, uint32_t n, const GemvBatch bt,
                 unsigned long long* argmax) {
     extern __shared__ __align__(16) uint8_t smem[];
     constexpr int kGmRows = WARPS * 16, kGmThreads = WARPS * kWarp;
@@ -225,7 +225,7 @@ constexpr uint32_t kErrGemvTimeout = 0x7B000001u;
 template <bool SB_FP16, bool ARGMAX>
 __global__ void __launch_bounds__(kGsTeams * kGsTeamWarps * kWarp, 1)
 gemv_stream_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S, const uint16_t* __restrict__ B,
-                   const uint16_t* __restrict__ x, uint16_t* __restrict__ y, uint32_t m, uint32_t n, unsigned long long* argmax, uint32_t* error) {
+                   const uint16_t* x, uint16_t* __restrict__ y, uint32_t m, uint32_t n, unsigned long long* argmax, uint32_t* error) {
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ __align__(8) unsigned long long bars[kGsTeams][2];
     __shared__ unsigned long long per_warp[kGsTeams * kGsTeamWarps];

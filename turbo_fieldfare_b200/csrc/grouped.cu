@@ -46,8 +46,8 @@ constexpr int kGroupPerThread = 4;
 
 // counters: [0] group count, [1] total chunks (sum over groups of ceil(count/8)), [2] pair count
 __global__ void __launch_bounds__(kGroupThreads)
-group_routes_kernel(const uint32_t* __restrict__ indices, uint32_t idx_stride, uint32_t* __restrict__ ids_out,
-                    const uint16_t* __restrict__ weights, uint32_t T, uint32_t K, uint32_t E,
+group_routes_kernel(const uint32_t* indices, uint32_t idx_stride, uint32_t* __restrict__ ids_out,
+                    const uint16_t* weights, uint32_t T, uint32_t K, uint32_t E,
                     tf_pair* __restrict__ sorted_pairs, uint32_t* __restrict__ per_expert_offsets,
                     uint32_t* __restrict__ per_expert_counts, tf_group* __restrict__ groups,
                     uint32_t* __restrict__ chunk_group, uint32_t* __restrict__ chunk_start,
@@ -62,13 +62,23 @@ group_routes_kernel(const uint32_t* __restrict__ indices, uint32_t idx_stride, u
     pdl_wait();
     peer_wait_in_block(peer_wait);      // the ids may sit in rows that peers are still writing (ends with a block barrier)
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-        // idx_stride > 1: the ids sit in the tails of exchanged rows; the first block also writes them out densely
-        uint32_t ex = indices[(size_t)i * idx_stride];
-        if (ids_out && e == 0) ids_out[i] = ex;
-        if (ex == 0xFFFFFFFFu) continue;    // empty slot of a fixed-capacity exchange buffer
-        if (ex >= E) ex = E - 1;            // min(id, E-1): Runtime/Inference/RealForwardRunner.swift:955
-        atomicAdd(&hist[ex], 1u);
+    for (uint32_t i0 = threadIdx.x; i0 < n; i0 += kGroupPerThread * kGroupThreads) {
+        uint32_t ids[kGroupPerThread];              // loads before the first store
+#pragma unroll
+        for (int j = 0; j < kGroupPerThread; ++j) {
+            const uint32_t i = i0 + j * kGroupThreads;
+            ids[j] = i < n ? indices[(size_t)i * idx_stride] : 0xFFFFFFFFu;
+        }
+#pragma unroll
+        for (int j = 0; j < kGroupPerThread; ++j) {
+            // idx_stride > 1: the ids sit in the tails of exchanged rows; the first block also writes them out densely
+            const uint32_t i = i0 + j * kGroupThreads;
+            uint32_t ex = ids[j];
+            if (ids_out && e == 0 && i < n) ids_out[i] = ex;
+            if (ex == 0xFFFFFFFFu) continue;    // empty slot of a fixed-capacity exchange buffer
+            if (ex >= E) ex = E - 1;            // min(id, E-1): Runtime/Inference/RealForwardRunner.swift:955
+            atomicAdd(&hist[ex], 1u);
+        }
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -154,7 +164,7 @@ __host__ __device__ inline uint32_t grp_slice_len(uint32_t n, uint32_t slices) {
 }
 
 __global__ void __launch_bounds__(kGrpSliceThreads)
-group_count_kernel(const uint32_t* __restrict__ indices, uint32_t idx_stride, uint32_t* __restrict__ ids_out, uint32_t n, uint32_t E,
+group_count_kernel(const uint32_t* indices, uint32_t idx_stride, uint32_t* __restrict__ ids_out, uint32_t n, uint32_t E,
                    uint32_t slice_len, uint32_t* __restrict__ slice_hist, const PeerWait peer_wait) {
     __shared__ uint32_t hist[TF_MAX_ROUTER_EXPERTS];
     pdl_launch_dependents();
@@ -163,19 +173,29 @@ group_count_kernel(const uint32_t* __restrict__ indices, uint32_t idx_stride, ui
     peer_wait_in_block(peer_wait);
     __syncthreads();
     const uint32_t lo = blockIdx.x * slice_len, hi = lo + slice_len < n ? lo + slice_len : n;
-    for (uint32_t i = lo + threadIdx.x; i < hi; i += blockDim.x) {
-        uint32_t ex = indices[(size_t)i * idx_stride];
-        if (ids_out) ids_out[i] = ex;
-        if (ex == 0xFFFFFFFFu) continue;
-        if (ex >= E) ex = E - 1;
-        atomicAdd(&hist[ex], 1u);
+    for (uint32_t i0 = lo + threadIdx.x; i0 < hi; i0 += kGroupPerThread * kGrpSliceThreads) {
+        uint32_t ids[kGroupPerThread];              // loads before the first store
+#pragma unroll
+        for (int j = 0; j < kGroupPerThread; ++j) {
+            const uint32_t i = i0 + j * kGrpSliceThreads;
+            ids[j] = i < hi ? indices[(size_t)i * idx_stride] : 0xFFFFFFFFu;
+        }
+#pragma unroll
+        for (int j = 0; j < kGroupPerThread; ++j) {
+            const uint32_t i = i0 + j * kGrpSliceThreads;
+            uint32_t ex = ids[j];
+            if (ids_out && i < hi) ids_out[i] = ex;
+            if (ex == 0xFFFFFFFFu) continue;
+            if (ex >= E) ex = E - 1;
+            atomicAdd(&hist[ex], 1u);
+        }
     }
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < E; i += blockDim.x) slice_hist[(size_t)blockIdx.x * E + i] = hist[i];
 }
 
 __global__ void __launch_bounds__(TF_MAX_ROUTER_EXPERTS)
-group_scan_kernel(const uint32_t* __restrict__ slice_hist, uint32_t* __restrict__ slice_start, uint32_t slices, uint32_t n, uint32_t E,
+group_scan_kernel(const uint32_t* slice_hist, uint32_t* __restrict__ slice_start, uint32_t slices, uint32_t n, uint32_t E,
                   uint32_t* __restrict__ per_expert_offsets, uint32_t* __restrict__ per_expert_counts, tf_group* __restrict__ groups,
                   uint32_t* __restrict__ chunk_group, uint32_t* __restrict__ chunk_start, uint32_t* __restrict__ counters) {
     __shared__ uint32_t wtot[3][TF_MAX_ROUTER_EXPERTS / kWarp];
@@ -213,18 +233,24 @@ group_scan_kernel(const uint32_t* __restrict__ slice_hist, uint32_t* __restrict_
         }
         // where each slice's pairs of this expert start
         uint32_t running = my_off;
-#pragma unroll 8
-        for (uint32_t b = 0; b < slices; ++b) {
-            slice_start[(size_t)b * E + e] = running;
-            running += slice_hist[(size_t)b * E + e];
+        constexpr uint32_t kAtOnce = 8;
+        for (uint32_t b0 = 0; b0 < slices; b0 += kAtOnce) {
+            uint32_t c[kAtOnce];                    // loads before the first store
+#pragma unroll
+            for (uint32_t j = 0; j < kAtOnce; ++j) c[j] = b0 + j < slices ? slice_hist[(size_t)(b0 + j) * E + e] : 0u;
+#pragma unroll
+            for (uint32_t j = 0; j < kAtOnce; ++j) {
+                if (b0 + j < slices) slice_start[(size_t)(b0 + j) * E + e] = running;
+                running += c[j];
+            }
         }
     }
     if (threadIdx.x == 0) { counters[0] = t_g; counters[1] = t_ch; counters[2] = n; counters[3] = t_off; }
 }
 
 __global__ void __launch_bounds__(kGrpSliceThreads)
-group_place_kernel(const uint32_t* __restrict__ indices, uint32_t idx_stride, const uint16_t* __restrict__ weights, uint32_t n, uint32_t K,
-                   uint32_t E, uint32_t slice_len, const uint32_t* __restrict__ slice_start, tf_pair* __restrict__ sorted_pairs) {
+group_place_kernel(const uint32_t* indices, uint32_t idx_stride, const uint16_t* weights, uint32_t n, uint32_t K,
+                   uint32_t E, uint32_t slice_len, const uint32_t* slice_start, tf_pair* __restrict__ sorted_pairs) {
     __shared__ uint32_t wcnt[kGrpSliceThreads / kWarp][TF_MAX_ROUTER_EXPERTS];     // per warp and expert: count, then start
     __shared__ uint32_t run[TF_MAX_ROUTER_EXPERTS];                                // next free position per expert
     pdl_launch_dependents();
@@ -605,7 +631,7 @@ grouped_ksplit_kernel(const GroupedArgs args) {
                     if ((uint32_t)i < ngw && (uint32_t)(n * 8 + g) < cur.ntok) {
                         const uint32_t rr = (DENSE || NMAT == 1) ? cur.row_base + n * 8 + g : args.sorted_pairs.field<NMAT == 1>(cur.row_base + n * 8 + g, &tf_pair::token);
                         const uint4* p = reinterpret_cast<const uint4*>(args.x + (size_t)rr * args.x_stride + (g0 + i) * kGroup + t * 16);
-                        const uint4 lo = __ldg(p), hi = __ldg(p + 1);
+                        const uint4 lo = p[0], hi = p[1];
                         r[0] = lo.x; r[1] = lo.y; r[2] = lo.z; r[3] = lo.w;
                         r[4] = hi.x; r[5] = hi.y; r[6] = hi.z; r[7] = hi.w;
                     } else {
@@ -1021,7 +1047,7 @@ grouped_down_kernel(const GroupedArgs args) {
                     uint32_t r[8];
                     if ((uint32_t)g < cur.ntok) {
                         const uint4* p = reinterpret_cast<const uint4*>(args.x + (size_t)(cur.row_base + g) * args.x_stride + i * kGroup + t * 16);
-                        const uint4 lo = __ldg(p), hi = __ldg(p + 1);
+                        const uint4 lo = p[0], hi = p[1];
                         r[0] = lo.x; r[1] = lo.y; r[2] = lo.z; r[3] = lo.w;
                         r[4] = hi.x; r[5] = hi.y; r[6] = hi.z; r[7] = hi.w;
                     } else {
@@ -1152,8 +1178,8 @@ namespace tf {
 // PARTIAL_F32 = true: the decode kernel's order (Metal/MoE/moe.metal:473-480):
 //     acc = float(residual[d]); acc += float(w_r) * partial_r, r = 0..K-1; y = half(acc)
 template <bool PARTIAL_F32>
-__global__ void reduce_token_major_kernel(const void* __restrict__ partials, const uint16_t* __restrict__ weights,
-                                          const uint16_t* __restrict__ residual, uint32_t residual_stride,
+__global__ void reduce_token_major_kernel(const void* partials, const uint16_t* weights,
+                                          const uint16_t* residual, uint32_t residual_stride,
                                           uint16_t* __restrict__ out, uint32_t out_stride,
                                           uint32_t T, uint32_t K, uint32_t D) {
     const uint32_t d = blockIdx.y * blockDim.x + threadIdx.x;      // rows in grid.x: no 65535 limit on the token count

@@ -301,8 +301,8 @@ __host__ __device__ inline uint32_t qmm_tokens_per_tile(uint32_t count, uint32_t
 // The group table of a launch: one thread per group, the tile counts scanned over the block. (One thread that walked the
 // groups took 29 us for 128 of them, on the critical path before every routed GEMM; this takes about 2.)
 __global__ void __launch_bounds__(TF_MAX_ROUTER_EXPERTS)
-qmm_prepare_kernel(uint4* __restrict__ groups, uint32_t* __restrict__ totals, const tf_group* __restrict__ route_groups,
-                   const uint32_t* __restrict__ route_counters, uint32_t dense_tokens, uint32_t dense_per_tile, uint32_t ctas) {
+qmm_prepare_kernel(uint4* __restrict__ groups, uint32_t* __restrict__ totals, const tf_group* route_groups,
+                   const uint32_t* route_counters, uint32_t dense_tokens, uint32_t dense_per_tile, uint32_t ctas) {
     __shared__ uint32_t warp_tiles[TF_MAX_ROUTER_EXPERTS / kWarp], warp_top[TF_MAX_ROUTER_EXPERTS / kWarp];
     const uint32_t warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
     pdl_launch_dependents();

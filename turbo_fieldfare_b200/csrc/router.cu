@@ -23,7 +23,7 @@ constexpr int kSplitThreads = kSplitExpertsPerBlock * kWarp;
 constexpr int kBlockRouterThreads = 256;
 
 template <bool X_BF16>
-__device__ __forceinline__ void stage_router_x(const uint16_t* __restrict__ hidden, const uint16_t* __restrict__ eff,
+__device__ __forceinline__ void stage_router_x(const uint16_t* hidden, const uint16_t* __restrict__ eff,
                                                float* xf, uint32_t d) {
     for (uint32_t i = threadIdx.x; i < d; i += blockDim.x) {
         const float h = X_BF16 ? bf16_bits_to_float(hidden[i]) : f16_bits_to_float(hidden[i]);
@@ -59,7 +59,7 @@ __device__ __forceinline__ float router_row_logit(const uint8_t* __restrict__ Wr
 template <bool X_BF16>
 __global__ void __launch_bounds__(kSplitThreads)
 router_split_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S, const uint16_t* __restrict__ B,
-                    const uint16_t* __restrict__ hidden, uint32_t hidden_stride,
+                    const uint16_t* hidden, uint32_t hidden_stride,
                     const uint16_t* __restrict__ eff, const uint16_t* __restrict__ per_expert_scale,
                     const float* __restrict__ logit_bias,
                     uint32_t* __restrict__ out_idx, uint16_t* __restrict__ out_w, float* __restrict__ out_logits,
@@ -96,7 +96,7 @@ router_split_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ 
         for (int j = 0; j < 3; ++j) {
             const uint32_t i = threadIdx.x + j * kSplitThreads;
             const bool ok = i < d / 8;
-            hv[j] = ok ? __ldg(reinterpret_cast<const uint4*>(hrow) + i) : make_uint4(0u, 0u, 0u, 0u);
+            hv[j] = ok ? reinterpret_cast<const uint4*>(hrow)[i] : make_uint4(0u, 0u, 0u, 0u);
             ev[j] = ok ? __ldg(reinterpret_cast<const uint4*>(eff) + i) : make_uint4(0u, 0u, 0u, 0u);
         }
         for (uint32_t i = threadIdx.x; i < ne * groups; i += blockDim.x) {
@@ -204,7 +204,7 @@ constexpr int kRowsExpertsPerBlock = kRowsThreads / kWarp;
 template <bool X_BF16, int R>
 __global__ void __launch_bounds__(kRowsThreads)
 router_rows_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S, const uint16_t* __restrict__ B,
-                   const uint16_t* __restrict__ hidden, uint32_t hidden_stride,
+                   const uint16_t* hidden, uint32_t hidden_stride,
                    const uint16_t* __restrict__ eff, const uint16_t* __restrict__ per_expert_scale,
                    const float* __restrict__ logit_bias,
                    uint32_t* __restrict__ out_idx, uint16_t* __restrict__ out_w, float* __restrict__ out_logits,
@@ -249,7 +249,7 @@ router_rows_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S
         uint4 hv[R];
 #pragma unroll
         for (int r = 0; r < R; ++r)
-            hv[r] = row0 + r < rows ? __ldg(reinterpret_cast<const uint4*>(hidden + (size_t)(row0 + r) * hidden_stride) + i)
+            hv[r] = row0 + r < rows ? reinterpret_cast<const uint4*>(hidden + (size_t)(row0 + r) * hidden_stride)[i]
                                     : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
         for (int r = 0; r < R; ++r) {
@@ -344,7 +344,7 @@ router_rows_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S
 template <bool X_BF16>
 __global__ void __launch_bounds__(kBlockRouterThreads)
 router_block_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S, const uint16_t* __restrict__ B,
-                    const uint16_t* __restrict__ hidden, uint32_t hidden_stride,
+                    const uint16_t* hidden, uint32_t hidden_stride,
                     const uint16_t* __restrict__ eff, const uint16_t* __restrict__ per_expert_scale,
                     const float* __restrict__ logit_bias,
                     uint32_t* __restrict__ out_idx, uint16_t* __restrict__ out_w, float* __restrict__ out_logits,
@@ -382,7 +382,7 @@ constexpr int kTileExperts = 4;             // experts per warp iteration
 template <bool X_BF16, int R>
 __global__ void __launch_bounds__(kBlockRouterThreads, 2)
 router_tile_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S, const uint16_t* __restrict__ B,
-                   const uint16_t* __restrict__ hidden, uint32_t hidden_stride,
+                   const uint16_t* hidden, uint32_t hidden_stride,
                    const uint16_t* __restrict__ eff, const uint16_t* __restrict__ per_expert_scale,
                    const float* __restrict__ logit_bias,
                    uint32_t* __restrict__ out_idx, uint16_t* __restrict__ out_w, float* __restrict__ out_logits,

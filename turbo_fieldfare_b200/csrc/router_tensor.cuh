@@ -65,14 +65,6 @@ __device__ __forceinline__ uint32_t bytes_to_half2(uint32_t word, uint32_t sel) 
     return *reinterpret_cast<const uint32_t*>(&v);
 }
 
-// Activations behind a wait in the middle of a kernel: a plain load through a const __restrict__ pointer counts as invariant and may be moved
-// ahead of the wait (rows of the layer before were read).
-__device__ __forceinline__ uint4 load_row_words(const uint16_t* p) {
-    uint4 v;
-    asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
-    return v;
-}
-
 // out[token][expert] = (approximate logit without the logit bias, magnitude), both in units of x (not x * 2^10).
 // Grid: (ceil(rows / 16), ceil(num_experts / 128), parts); a part sums `chunks` chunks of 256 columns into its own plane of out, and the
 // re-check adds the planes. A chunk alone is a chain of latencies (rows, conversion, MMAs, store), eleven in a row took 41 us at 512 rows
@@ -82,7 +74,7 @@ __device__ __forceinline__ uint4 load_row_words(const uint16_t* p) {
 template <bool X_BF16>
 __global__ void __launch_bounds__(kApxThreads, 2)
 router_approx_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S, const uint16_t* __restrict__ B,
-                     const uint16_t* __restrict__ hidden, uint32_t hidden_stride, const uint16_t* __restrict__ eff,
+                     const uint16_t* hidden, uint32_t hidden_stride, const uint16_t* __restrict__ eff,
                      float2* __restrict__ out, uint32_t rows, uint32_t num_experts, uint32_t d, uint32_t chunks) {
     extern __shared__ __align__(16) uint8_t smem[];
     uint8_t* Wc0 = smem;                                                   // [2 or 1][128][kApxWPitch]
@@ -116,7 +108,7 @@ router_approx_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const uint32_t tok = tok0 + warp + 8 * h;
-            hreg[h] = tok < rows ? load_row_words(hidden + (size_t)tok * hidden_stride + c0 + lane * 8) : make_uint4(0u, 0u, 0u, 0u);
+            hreg[h] = tok < rows ? *reinterpret_cast<const uint4*>(hidden + (size_t)tok * hidden_stride + c0 + lane * 8) : make_uint4(0u, 0u, 0u, 0u);
         }
     };
     // scales and biases of a chunk's four groups for this thread's two expert rows (8-byte aligned: groups % 4 == 0)
@@ -250,7 +242,7 @@ __host__ __device__ inline size_t router_approx_few_smem_bytes(uint32_t d) {
 template <bool X_BF16>
 __global__ void __launch_bounds__(kFewThreads, 1)
 router_approx_few_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S, const uint16_t* __restrict__ B,
-                         const uint16_t* __restrict__ hidden, uint32_t hidden_stride, const uint16_t* __restrict__ eff,
+                         const uint16_t* hidden, uint32_t hidden_stride, const uint16_t* __restrict__ eff,
                          float2* __restrict__ out, uint32_t rows, uint32_t num_experts, uint32_t d) {
     extern __shared__ __align__(16) uint8_t smem[];
     const uint32_t w_pitch = d + 64, x_pitch = 2 * d + 16;                 // bank-conflict free, as kApxWPitch and kApxXPitch
@@ -474,7 +466,7 @@ __device__ __forceinline__ float2 router_logits_staged(const uint8_t* codes_a, c
 // largest lower bound. N: experts per lane. (A list: warps that took their candidates off bit masks, each skipping those of the token's
 // other warps, spent up to 20 000 clocks on that at eight warps per token.)
 template <int N>
-__device__ __forceinline__ uint32_t router_candidates(const float2* __restrict__ approx_row, uint32_t parts, size_t part_stride, const float* __restrict__ logit_bias,
+__device__ __forceinline__ uint32_t router_candidates(const float2* approx_row, uint32_t parts, size_t part_stride, const float* __restrict__ logit_bias,
                                                       uint32_t num_experts, uint32_t top_k, int lane, uint16_t* list /* shared */) {
     float upper[N];
     uint32_t key[N];
@@ -660,9 +652,9 @@ __device__ __forceinline__ void group_rows_in_block(const uint32_t* __restrict__
 template <bool X_BF16, int GROUPS, int WPT>          // GROUPS: d / 64 when known at compile time, 0 for any width
 __global__ void __launch_bounds__(kRecheckWarps * kWarp, 2)
 router_recheck_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S, const uint16_t* __restrict__ B,
-                      const uint16_t* __restrict__ hidden, uint32_t hidden_stride, const uint16_t* __restrict__ eff,
+                      const uint16_t* hidden, uint32_t hidden_stride, const uint16_t* __restrict__ eff,
                       const uint16_t* __restrict__ per_expert_scale, const float* __restrict__ logit_bias,
-                      const float2* __restrict__ approx, uint32_t parts, uint32_t* out_idx, uint16_t* out_w, unsigned int* ticket, const RouterGroupOut grp,
+                      const float2* approx, uint32_t parts, uint32_t* out_idx, uint16_t* out_w, unsigned int* ticket, const RouterGroupOut grp,
                       uint32_t rows, uint32_t num_experts, uint32_t d, uint32_t top_k) {
     extern __shared__ __align__(16) uint8_t smem[];
     constexpr int kTokens = kRecheckWarps / WPT;                    // tokens per block

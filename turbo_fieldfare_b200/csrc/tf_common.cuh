@@ -208,6 +208,9 @@ __device__ __forceinline__ float gelu_tanh(float x) {
 // writes are visible, so it comes before the first access to anything another kernel produces (and before any
 // write). Some kernels request their weights before it: those are written by plain launches and copies only, which never let
 // a dependent start early. Without the launch attribute both instructions do nothing.
+// Pointers to what other kernels write are plain ones, without __restrict__, and their loads plain loads, without __ldg: a load
+// through a const __restrict__ parameter of a kernel and an __ldg count as invariant, which the wait does not keep from being moved ahead of it (a
+// router then read the rows of the layer before). Weights and scales, which no such kernel writes, keep both.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

@@ -11,7 +11,7 @@ constexpr int kTileWarps = 8, kTileThreads = kTileWarps * kWarp;
 template <bool SB_FP16, bool OUT_F32, int WARPS>
 __global__ void __launch_bounds__(WARPS * kWarp, 16 / WARPS)
 tile_gemv_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S, const uint16_t* __restrict__ B,
-                 const uint16_t* __restrict__ x, void* __restrict__ y, uint32_t m, uint32_t ng) {
+                 const uint16_t* x, void* __restrict__ y, uint32_t m, uint32_t ng) {
     extern __shared__ __align__(16) uint8_t smem[];
     const uint32_t parts = (ng + kTilePart - 1) / kTilePart;
     uint32_t* frag = reinterpret_cast<uint32_t*>(smem);
@@ -48,8 +48,8 @@ tile_gemv_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S, 
 // acts[slot][row] = half(gelu(gate) * up): grid (F / 16, slots). Warp w takes matrix w % 2 and the parts w / 2, w / 2 + 4, ...,
 // three of them in flight (the production width has eleven parts).
 __global__ void __launch_bounds__(kTileThreads, 2)
-tile_gate_up_kernel(const uint8_t* const* __restrict__ blobs, const tf_expert_offsets off, const uint16_t* __restrict__ x, uint16_t* __restrict__ acts,
-                    uint32_t ng, uint32_t f, uint32_t top_k, const uint32_t* __restrict__ slot_map) {
+tile_gate_up_kernel(const uint8_t* const* blobs, const tf_expert_offsets off, const uint16_t* x, uint16_t* __restrict__ acts,
+                    uint32_t ng, uint32_t f, uint32_t top_k, const uint32_t* slot_map) {
     extern __shared__ __align__(16) uint8_t smem[];
     const uint32_t parts = (ng + kTilePart - 1) / kTilePart;
     uint32_t* frag = reinterpret_cast<uint32_t*>(smem);
@@ -97,8 +97,8 @@ tile_gate_up_kernel(const uint8_t* const* __restrict__ blobs, const tf_expert_of
 // The down projection of every slot for 16 output rows: a warp per slot, three parts in flight (all of the production width).
 // y = half(residual + sum over the slots, in order, of w_s * sum_s) (moe.metal:473-480).
 __global__ void __launch_bounds__(kTileThreads, 2)
-tile_down_kernel(const uint8_t* const* __restrict__ blobs, const tf_expert_offsets off, const uint16_t* __restrict__ acts, const uint16_t* __restrict__ routing_w,
-                 const uint16_t* __restrict__ residual, uint16_t* __restrict__ y, uint32_t d, uint32_t ng, uint32_t top_k) {
+tile_down_kernel(const uint8_t* const* blobs, const tf_expert_offsets off, const uint16_t* acts, const uint16_t* routing_w,
+                 const uint16_t* residual, uint16_t* __restrict__ y, uint32_t d, uint32_t ng, uint32_t top_k) {
     extern __shared__ __align__(16) uint8_t smem[];
     uint32_t* frag = reinterpret_cast<uint32_t*>(smem);                 // [top_k][ng] groups
     float* xsum = reinterpret_cast<float*>(smem + (size_t)top_k * ng * 128);

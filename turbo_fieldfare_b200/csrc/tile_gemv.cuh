@@ -17,7 +17,7 @@ constexpr int kTilePart = 4;               // groups per part
 
 // x as B fragments ([groups][4 lanes t][8 words]) and group sums scaled by 2^-24 (the codes enter the MMA as q * 2^-24).
 // Called by whole warps; `count` vectors of `ng` groups, x_stride elements apart, 16-byte aligned.
-__device__ __forceinline__ void tile_stage_x(const uint16_t* __restrict__ x, uint32_t x_stride, uint32_t count, uint32_t ng,
+__device__ __forceinline__ void tile_stage_x(const uint16_t* x, uint32_t x_stride, uint32_t count, uint32_t ng,
                                              uint32_t* frag, float* xsum) {
     const uint32_t items = count * ng * 4;
     for (uint32_t idx = threadIdx.x; idx < ((items + 31u) & ~31u); idx += blockDim.x) {
