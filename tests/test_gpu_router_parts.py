@@ -72,3 +72,64 @@ def test_stacks_route_on_the_rows_of_their_own_layer(tf_ctx, tokens, experts):
             stack.close()
             ctx.close()
     assert all(torch.equal(out[0], h) for h in out[1:])
+
+
+# Calls of fewer rows may need more scratch (more parts): 600 and 848 rows outgrow what 1024 rows left. A graph that was captured before keeps its
+# buffer; under capture a call takes as many parts as the buffer holds, or, where there is none yet, one launch.
+@pytest.mark.parametrize("before,captured,after", [([1024], 1024, [600, 848]), ([1500], 600, [848, 4096]), ([333], 1024, [848]), ([], 700, [700, 1500])])
+def test_a_captured_router_keeps_its_scratch(before, captured, after):
+    import torch
+    from turbo_fieldfare_b200.kernels import TurboContext
+    from turbo_fieldfare_b200.stack import AffineTensor, _ptr
+    d, experts = 2816, 128
+    ctx, plain = TurboContext(0), TurboContext(0)
+    try:
+        plain.set_router_tensorcore_min_rows(0xFFFFFFFF)
+        gen = torch.Generator(device="cuda").manual_seed(captured)
+        most = max(before + [captured] + after)
+        x = torch.randn(most, d, generator=gen, device="cuda").half()
+        eff = (1.0 + 0.1 * torch.randn(d, generator=gen, device="cuda")).to(torch.bfloat16)
+        gain = (0.5 + torch.rand(experts, generator=gen, device="cuda")).to(torch.bfloat16)
+        w = AffineTensor(experts, d, 8)
+        w.fill_synthetic(ctx, 7)
+        p = w.projection()
+        torch.cuda.synchronize()
+
+        def route(c, rows, idx, wt, stream=0):
+            c.check(c.lib.tf_router_gemma4_block(c.handle, stream, p.weights, p.weights_off, p.scales, p.scales_off, p.biases, p.biases_off, _ptr(x), 0, 1,
+                                                 _ptr(eff), 0, _ptr(gain), 0, None, _ptr(idx), 0, _ptr(wt), 0, None, rows, experts, d, 8, d))
+
+        def outputs(rows):
+            return torch.zeros(rows * 8, dtype=torch.int32, device="cuda"), torch.zeros(rows * 8, dtype=torch.int16, device="cuda")
+
+        def expected(rows):
+            idx, wt = outputs(rows)
+            route(plain, rows, idx, wt)
+            torch.cuda.synchronize()
+            return idx, wt
+
+        for rows in before:
+            route(ctx, rows, *outputs(rows))
+        torch.cuda.synchronize()
+        idx, wt = outputs(captured)
+        graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+        with torch.cuda.graph(graph, stream=stream):
+            route(ctx, captured, idx, wt, stream.cuda_stream)
+        for rows in after:
+            got, want = outputs(rows), expected(rows)
+            route(ctx, rows, *got)
+            torch.cuda.synchronize()
+            assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+        want = expected(captured)
+        for _ in range(3):
+            idx.zero_()
+            wt.zero_()
+            graph.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(idx, want[0]) and torch.equal(wt, want[1])
+        assert ctx.device_status() == 0
+        del graph
+    finally:
+        torch.cuda.synchronize()
+        ctx.close()
+        plain.close()

@@ -104,6 +104,7 @@ void tf_context_destroy(tf_context* ctx) {
     if (ctx->router_logits) cudaFree(ctx->router_logits);
     if (ctx->router_tickets) cudaFree(ctx->router_tickets);
     if (ctx->router_approx) cudaFree(ctx->router_approx);
+    for (uint32_t i = 0; i < ctx->router_approx_replaced_count; ++i) cudaFree(ctx->router_approx_replaced[i]);
     if (ctx->device_error) cudaFree(ctx->device_error);
     if (ctx->peer_error) cudaFree(ctx->peer_error);
     if (ctx->streamed_scratch) cudaFree(ctx->streamed_scratch);

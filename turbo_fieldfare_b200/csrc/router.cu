@@ -498,22 +498,32 @@ static int tile_router_rows(uint32_t rows, uint32_t slots) {
     return best;
 }
 
-// Scratch of the two-launch router: (approximate logit, magnitude) per (row, expert), owned by the context and grown
-// on demand. Growing allocates, which a stream that is being captured must not do: the caller then takes the
-// one-launch kernel; where it holds fewer planes than `parts`, that is the number of parts.
+// Scratch of the two-launch router: `parts` planes of (approximate logit, magnitude) per (row, expert), owned by the context and grown
+// on demand, to twice its size at least. A buffer that was outgrown stays (see router_approx_replaced): more rows do not always take more
+// scratch, since the number of parts falls, so a call of fewer rows than a captured one may be what outgrows it. Growing allocates, which a stream
+// that is being captured must not do. There, and where memory runs out, the parts are as many as the buffer holds; false if that is
+// none (the caller then takes the one-launch kernel).
 static bool router_scratch(tf_context* ctx, cudaStream_t st, uint32_t rows, uint32_t num_experts, uint32_t& parts) {
     const size_t plane = (size_t)rows * num_experts * sizeof(float2), need = plane * parts;
     if (need <= ctx->router_approx_bytes) return true;
+    const uint32_t held = (uint32_t)(ctx->router_approx_bytes / plane);       // planes, fewer than `parts`
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
-        cudaGetLastError();
-        parts = (uint32_t)(ctx->router_approx_bytes / plane);
-        return parts > 0;
+    if (cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) {
+        for (uint32_t want : {parts, 1u}) {                   // one plane where there is no memory for all
+            if (want <= held) break;
+            const size_t bytes = std::max(plane * want, 2 * ctx->router_approx_bytes);
+            void* grown = nullptr;
+            if (cudaMalloc(&grown, bytes) != cudaSuccess) { cudaGetLastError(); continue; }
+            if (ctx->router_approx) ctx->router_approx_replaced[ctx->router_approx_replaced_count++] = ctx->router_approx;
+            ctx->router_approx = grown;
+            ctx->router_approx_bytes = bytes;
+            parts = want;
+            return true;
+        }
     }
-    if (ctx->router_approx) { cudaFree(ctx->router_approx); ctx->router_approx = nullptr; ctx->router_approx_bytes = 0; }
-    if (cudaMalloc(&ctx->router_approx, need) != cudaSuccess) { cudaGetLastError(); return false; }
-    ctx->router_approx_bytes = need;
-    return true;
+    cudaGetLastError();
+    parts = held;
+    return held > 0;
 }
 
 static RouterGroupOut router_group_out(const tf_device_routes* routes) {
@@ -558,7 +568,13 @@ static tf_status launch_router(tf_context* ctx, void* stream, const uint8_t* W, 
     // overlap, beyond that. One chunk, three, all eleven (us): 333 rows 7.5, 17.9, 37.9; 512 rows 14.9, 18.0, 39.0; 800 rows 14.9, 16.9, 38.8;
     // 1500 rows 23.7, 22.4, 45.6; 4096 rows 47.8, 41.0, 48.5 (and adding the planes takes the re-check 9 us less with three).
     const uint32_t apx_blocks = (rows + kApxTokens - 1) / kApxTokens * ((num_experts + kApxExperts - 1) / kApxExperts) * (d / kApxChunk);
-    uint32_t parts = apx_blocks <= 4u * (uint32_t)ctx->sm_count ? d / kApxChunk : (d / kApxChunk + 2) / 3;
+    // Few rows: blocks of 8 tokens x 32 experts with all of their operands in flight at once, while they make one round of the SMs: 200 rows,
+    // 100 blocks, 9.8 us. Two rounds (333 rows, 168 blocks) take 16.6, the parts of the other kernel 7.5. (Those take 6.2 us at 200 rows,
+    // but steps of 66 to 255 tokens gained nothing or lost 0.5 %, and prefills of 256 took 2.7 % longer.)
+    const size_t smem_few = router_approx_few_smem_bytes(d);
+    const dim3 grid_few((rows + kFewTokens - 1) / kFewTokens, (num_experts + kFewExperts - 1) / kFewExperts);
+    const bool few = smem_few <= 224 * 1024 && grid_few.x * grid_few.y <= (uint32_t)ctx->sm_count;
+    uint32_t parts = few ? 1u : apx_blocks <= 4u * (uint32_t)ctx->sm_count ? d / kApxChunk : (d / kApxChunk + 2) / 3;
     if (rows >= 2 && rows <= (uint32_t)kRouterSplitRows && vec16) {
         constexpr int R = 1;          // latency bound: a 64-token step took 4.35 ms with four rows per block, 4.28 with two, 4.16 with one
         auto k = bf ? router_rows_kernel<true, R> : router_rows_kernel<false, R>;
@@ -602,13 +618,7 @@ static tf_status launch_router(tf_context* ctx, void* stream, const uint8_t* W, 
         // logits on the tensor cores, then the canonical logits of the few experts that can reach the top k
         float2* approx = own ? own->approx : static_cast<float2*>(ctx->router_approx);
         const uint32_t sms = (uint32_t)ctx->sm_count;
-        // Few rows: blocks of 8 tokens x 32 experts with all of their operands in flight at once, while they make one round of the SMs: 200 rows,
-        // 100 blocks, 9.8 us. Two rounds (333 rows, 168 blocks) take 16.6, the parts of the other kernel 7.5. (Those take 6.2 us at 200 rows,
-        // but steps of 66 to 255 tokens gained nothing or lost 0.5 %, and prefills of 256 took 2.7 % longer.)
-        const size_t smem_few = router_approx_few_smem_bytes(d);
-        const dim3 grid_few((rows + kFewTokens - 1) / kFewTokens, (num_experts + kFewExperts - 1) / kFewExperts);
-        if (smem_few <= 224 * 1024 && grid_few.x * grid_few.y <= sms) {
-            parts = 1;
+        if (few) {
             auto ka = bf ? router_approx_few_kernel<true> : router_approx_few_kernel<false>;
             static DeviceSmemCache configured_few[2];
             if (tf_status s = ensure_dynamic_smem(ctx, ka, configured_few[bf ? 1 : 0], smem_few)) return s;

@@ -44,6 +44,10 @@ struct tf_context {
     // Prefill-sized router: (approximate logit, magnitude) per (row, expert) between its two launches; grown on demand.
     void* router_approx = nullptr;
     size_t router_approx_bytes = 0;
+    // Smaller buffers that it replaced. Captured graphs may hold their addresses, so they live as long as the context; each was at most half of
+    // its successor, so this many are never reached.
+    void* router_approx_replaced[48] = {};
+    uint32_t router_approx_replaced_count = 0;
     // Batches of at least this many rows take the two-launch router (tensor-core logits + canonical re-check).
     uint32_t router_tensorcore_min_rows = 256;
     // The same for block forwards of up to kRouterFusedGroupRows rows, whose workspace holds the scratch of the two launches; 0
