@@ -8,9 +8,10 @@ from helpers import from_dev, to_dev
 pytestmark = pytest.mark.gpu
 
 # (d, f, fs, experts, top_k): production; parts of four groups full and partial in d, f and fs; one tile per block, several and more than are in
-# flight at once; few and most experts; shared memory at its limit, and beyond it (there one token takes the layered launches, too)
+# flight at once; few and most experts; shared memory near its limit, and beyond it (there one token takes the layered launches, too)
 SIZES = [(2816, 704, 2112, 128, 8), (256, 128, 192, 16, 8), (320, 64, 64, 9, 8), (64, 64, 64, 4, 2), (1088, 192, 448, 256, 7),
-         (2752, 1024, 576, 24, 8), (3072, 1280, 1152, 16, 6), (3072, 1536, 3072, 16, 8)]
+         (2752, 1024, 576, 24, 8), (3072, 1280, 1152, 16, 6), (3072, 1536, 3072, 16, 8), (3072, 3072, 3072, 9, 8)]
+BEYOND = SIZES[-1]
 
 
 def _rows(o, rng, d):
@@ -46,6 +47,30 @@ def test_one_token_block_and_stack_have_the_bits_of_two_equal_tokens(tf_ctx, ora
         assert tf_ctx.device_status() == 0
         assert np.array_equal(from_dev(y1, np.uint16), from_dev(y2, np.uint16)[:d])
         assert np.array_equal(ws1.routing(1)[0][0], ws2.routing(2)[0][0])
+    finally:
+        stack.close()
+
+
+@pytest.mark.parametrize("d,f,fs,experts,top_k", SIZES)
+def test_one_token_takes_its_own_launches(tf_ctx, oracle, tmp_path, d, f, fs, experts, top_k):
+    """Three a layer of a stack and, in a block, kernels of their own; the layered ones beyond the shared memory."""
+    import torch
+    from test_gpu_edges import _kernels_of
+    from turbo_fieldfare_b200.stack import MoEBlock, MoEStack
+    stack = MoEStack(tf_ctx, layers=2, d=d, f=f, fs=fs, num_experts=experts, top_k=top_k, seed=7, align=256)
+    try:
+        h = to_dev(_rows(oracle, np.random.default_rng(d), d))
+        y = torch.zeros(d, dtype=torch.int16, device="cuda")
+        ws = stack.workspace(1)
+        before = tf_ctx.launch_count
+        stack.forward(h, 1, ws)
+        launches = tf_ctx.launch_count - before
+        text = _kernels_of(lambda: MoEBlock(tf_ctx, stack.layers[1]).forward(h, y, 1, ws), tmp_path / "graph.dot")
+        torch.cuda.synchronize()
+        assert tf_ctx.device_status() == 0
+        own = (d, f, fs, experts, top_k) != BEYOND
+        assert (launches == 3 * 2) is own
+        assert all((k in text) is own for k in ("one_token_front_kernel", "one_token_gate_up_kernel", "one_token_down_kernel"))
     finally:
         stack.close()
 

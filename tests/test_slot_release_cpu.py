@@ -54,3 +54,16 @@ def test_a_dependent_arrival_takes_its_values():
     body = body[body.index("void mbar_arrive_after(uint32_t addr, uint32_t a, uint32_t b) {"):]
     body = body[:body.index("\n}")]
     assert "setp.eq.u32 p, %1, %2" in body and "@p mbarrier.arrive" in body and "@!p mbarrier.arrive" in body and '"memory"' in body
+
+
+def test_one_token_kernels_wait_again_for_copies_in_flight():
+    """A wait for a landing copy that runs out is recorded, and the copies under way get one more bounded wait before the block, and with it
+    their destination, goes away."""
+    text = re.sub(r"//[^\n]*", "", (CSRC / "one_token.cu").read_text())
+    first = [m for m in re.finditer(r"(?:!mbar_wait\(|= mbar_wait\()(bars? ?\+?[^,]*|bar), ", text) if "slots + slot" not in m.group(1)]
+    assert len(first) == 4                            # front: tiles, router's codes; gate/up: tiles; down: both phases
+    for m in first:
+        after = text[m.end():]
+        after = after[:after.index("__syncthreads();") if "__syncthreads();" in after else None]
+        again = re.search(r"(?<![!= ]) mbar_wait\(|\n\s*mbar_wait\(|\) mbar_wait\(", after)
+        assert again, text[m.start():m.start() + 80]

@@ -365,7 +365,10 @@ one_token_front_kernel(const OneTokenArgs a, uint32_t most) {
             landed = mbar_wait(bar + i * 8, 0) && landed;
             for (uint32_t p = warp; p < parts; p += kOneWarps) one_tile_part<FOURS>(lay, smem, i, i, p);
         }
-        if (!landed && lane == 0) atomicCAS(a.error, 0u, kErrTimeoutOneToken);
+        if (!landed) {
+            if (lane == 0) atomicCAS(a.error, 0u, kErrTimeoutOneToken);
+            for (uint32_t i = 0; i < count; ++i) mbar_wait(bar + i * 8, 0);           // once more (bounded) for the copies in flight
+        }
         __syncthreads();
         one_tiles_finish<true>(lay, smem, count, resolve, true);
         if (a.behind_router) pdl_wait();
@@ -383,7 +386,10 @@ one_token_front_kernel(const OneTokenArgs a, uint32_t most) {
     }
     __syncthreads();
     if (!scores) return;
-    if (!mbar_wait(bar, 0) && lane == 0) atomicCAS(a.error, 0u, kErrTimeoutOneToken);
+    if (!mbar_wait(bar, 0)) {
+        if (lane == 0) atomicCAS(a.error, 0u, kErrTimeoutOneToken);
+        mbar_wait(bar, 0);                              // once more (bounded) for the copy in flight
+    }
     // the canonical logit (router.cu)
     float acc = 0.0f;
     const uint8_t* codes = smem + rlay.off_codes() + warp * a.d + lane * 2;
@@ -525,7 +531,13 @@ one_token_gate_up_kernel(const OneTokenArgs a, uint32_t slots, uint32_t most) {
         uint32_t slot = 0, use = 0;
         if (warp < (uint32_t)kOneWarps) {
             for (uint32_t i = 0; i < n && warp < parts; ++i) {
-                if (live && !mbar_wait(bars + slot * 8, use & 1)) { landed = false; break; }
+                if (live && !mbar_wait(bars + slot * 8, use & 1)) {
+                    landed = false;
+                    // once more (bounded) for the copies in flight: this tile's and those of the other slots, no others have been requested
+                    // since this slot is not free
+                    for (uint32_t k = i; k < n && k < i + slots; ++k) mbar_wait(bars + k % slots * 8, (k / slots) & 1);
+                    break;
+                }
                 for (uint32_t p = warp; p < parts; p += kOneWarps) one_tile_part<FOURS>(lay, smem, slot, i, p);
                 __syncwarp();
                 if (live && lane == 0) mbar_arrive(bars + (slots + slot) * 8);
