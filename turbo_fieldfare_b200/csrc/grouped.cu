@@ -746,14 +746,6 @@ grouped_ksplit_kernel(const GroupedArgs args) {
 #pragma unroll
                 for (int j = 0; j < 4; ++j) y[m][j] = acc[j] * 16777216.0f;
             }
-            // this warp is done with the stage: the sums of rows g and g + 8 of the matrices come of all of its loads
-            __syncwarp();
-            if (lane == 0) {
-                if constexpr (NMAT == 2)
-                    mbar_arrive_after(bar_empty(st), __float_as_uint(y[0][0]) ^ __float_as_uint(y[0][2]) ^ __float_as_uint(y[1][0]), __float_as_uint(y[1][2]));
-                else
-                    mbar_arrive_after(bar_empty(st), y[0][0], y[0][2]);
-            }
             // partial sums for the reducer: buffer li % kRedStages, 512 bytes per (warp, matrix, 8 tokens)
             const uint32_t r = li % kRedStages, ruse = li / kRedStages;
             if (!mbar_wait(bar_red_free(r), (ruse & 1) ^ 1)) { fail = kErrTimeoutRedFree; break; }
@@ -763,6 +755,10 @@ grouped_ksplit_kernel(const GroupedArgs args) {
                 sts_f32x2(red_w + m * 512, y[m][0], y[m][1]);
                 sts_f32x2(red_w + m * 512 + 256, y[m][2], y[m][3]);      // weight row g + 8: index (g + 8) * 8 + 2t
             }
+            // This warp is done with the stage: its sums, of all loads, have been stored. (Handed back in front of the wait for the reducer, by an
+            // arrival that takes the sums, steps of 11 to 100 tokens took 1 % longer, 4 and 200 tokens the same.)
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_empty(st));
             } else {
             // the reducer's buffer is claimed first, so that a matrix's sums leave the registers before the next matrix begins
             const uint32_t r = li % kRedStages, ruse = li / kRedStages;
@@ -934,7 +930,7 @@ grouped_ksplit_kernel(const GroupedArgs args) {
                 }
                 if (n == NT - 1) {
                     __syncwarp();
-                    if (lane == 0) mbar_arrive_after(bar_red_free(q), acc[0].x, acc[NMAT - 1].y);
+                    if (lane == 0) mbar_arrive_after(bar_red_free(q), acc[0].x, acc[NMAT - 1].x);
                 }
                 const float o0[4] = {acc[0].x, acc[0].y, acc[0].z, acc[0].w};
                 const float o1[4] = {acc[NMAT - 1].x, acc[NMAT - 1].y, acc[NMAT - 1].z, acc[NMAT - 1].w};

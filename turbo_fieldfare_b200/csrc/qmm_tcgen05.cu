@@ -672,8 +672,8 @@ qmm_tcgen05_kernel(const __grid_constant__ CUtensorMap x_map0, const __grid_cons
                         if (h == 0) {
                             __syncwarp();
                             if (lane == 0) {                      // the codes are in registers
-                                if constexpr (kTeams == 2) mbar_arrive_after(bar_empty_raw(sr), c[0].x ^ c[1].x ^ c[2].x, c[3].x);
-                                else mbar_arrive_after(bar_empty_raw(sr), c[0].x, c[1].x);
+                                if constexpr (kTeams == 2) mbar_arrive_after(bar_empty_raw(sr), c[0].x | c[1].x | c[2].x | c[3].x);
+                                else mbar_arrive_after(bar_empty_raw(sr), c[0].x | c[1].x);
                             }
                             if (ua > 0 && !q_mbar_wait(bar_empty_a(slot), (ua - 1) & 1)) { fail = kErrQmmTimeout | 5; break; }
                             tc_fence_after();
