@@ -48,7 +48,7 @@ def test_router_in_parts_equals_the_one_launch_router(tf_ctx, rows, experts, d, 
 
 
 # up to 255 tokens the re-check groups, too: pairs that fill no round of 32 to a warp, and all of its counters
-@pytest.mark.parametrize("tokens,experts", [(66, 256), (131, 200), (255, 20), (255, 256), (300, 64), (880, 64)])
+@pytest.mark.parametrize("tokens,experts", [(66, 256), (112, 128), (113, 128), (131, 200), (255, 20), (255, 256), (300, 64), (880, 64)])
 def test_stacks_route_on_the_rows_of_their_own_layer(tf_ctx, tokens, experts):
     import torch
     from turbo_fieldfare_b200.kernels import TurboContext

@@ -533,6 +533,9 @@ static RouterGroupOut router_group_out(const tf_device_routes* routes) {
                           static_cast<uint32_t*>(routes->counters)};
 }
 
+// See as_used in launch_router.
+constexpr uint32_t kRecheckAsUsedRows = 112, kRecheckAsUsedCodes = 262144;
+
 // Scratch of the two-launch router that belongs to the caller's workspace: nothing of the context is shared, so such calls may
 // overlap on several streams (the one-launch kernel for more than kRouterSplitRows rows shares nothing either).
 struct RouterScratch {
@@ -640,11 +643,19 @@ static tf_status launch_router(tf_context* ctx, void* stream, const uint8_t* W, 
         // candidates one after the other needs about 30 us however few rows there are.
         // (Only the form with a token per block can group.)
         const int which = rows <= 2 * sms || (own && routes) ? 3 : rows <= 4 * sms ? 2 : rows <= 8 * sms ? 1 : 0;
+        // Blocks of few rows and many experts read the approximate logits where they are used: a re-check that requests them ahead ends earlier, and
+        // the routed gate/up launch that it lets in then takes the SMs on which the shared expert's down launch would run beside it. Steps of
+        // 30 layers of 128 experts x 2816, us, as used and ahead: 75 tokens 4129, 4129; 90: 4525, 4566; 98: 4820, 4992; 105: 5443, 5650; 112: 5545,
+        // 5654; 115: 5655, 5636; 120: 5691, 5657; 150: 6258, 6135. Blocks of 128 x 1024, 90 to 110 tokens: 67 to 69, 63 to 66; of 64 x 2816 the same.
+        const bool as_used = own && routes && parts == 1 && rows <= kRecheckAsUsedRows && num_experts * d > kRecheckAsUsedCodes;
         void (*kr)(const uint8_t*, const uint16_t*, const uint16_t*, const uint16_t*, uint32_t, const uint16_t*, const uint16_t*, const float*,
                    const float2*, uint32_t, uint32_t*, uint16_t*, unsigned int*, RouterGroupOut, uint32_t, uint32_t, uint32_t, uint32_t);
 #define TF_RECHECK(WPT) kr = fixed ? (bf ? router_recheck_kernel<true, kProductionGroups, WPT> : router_recheck_kernel<false, kProductionGroups, WPT>) \
                                    : (bf ? router_recheck_kernel<true, 0, WPT> : router_recheck_kernel<false, 0, WPT>)
-        if (which == 3) TF_RECHECK(8);
+        if (as_used)
+            kr = fixed ? (bf ? router_recheck_kernel<true, kProductionGroups, 8, false> : router_recheck_kernel<false, kProductionGroups, 8, false>)
+                       : (bf ? router_recheck_kernel<true, 0, 8, false> : router_recheck_kernel<false, 0, 8, false>);
+        else if (which == 3) TF_RECHECK(8);
         else if (which == 2) TF_RECHECK(4);
         else if (which == 1) TF_RECHECK(2);
         else TF_RECHECK(1);
@@ -657,8 +668,8 @@ static tf_status launch_router(tf_context* ctx, void* stream, const uint8_t* W, 
             const size_t need = router_group_rows_smem_bytes(rows * top_k, num_experts);
             if (need > smem_r) smem_r = need;
         }
-        static DeviceSmemCache configured_recheck[4][4];
-        if (tf_status s = ensure_dynamic_smem(ctx, kr, configured_recheck[which][(bf ? 1 : 0) + (fixed ? 2 : 0)], smem_r)) return s;
+        static DeviceSmemCache configured_recheck[5][4];
+        if (tf_status s = ensure_dynamic_smem(ctx, kr, configured_recheck[as_used ? 4 : which][(bf ? 1 : 0) + (fixed ? 2 : 0)], smem_r)) return s;
         launch_pdl(kr, dim3((rows + per_block - 1) / per_block), dim3(kRecheckWarps * kWarp), smem_r, st, W, Sp, Bp, hp, stride,
                    ep, pp, logit_bias, static_cast<const float2*>(approx), parts, out_idx, wp, own ? own->ticket : nullptr, grp, rows, num_experts, d, top_k);
         if (grouped) *grouped = own && routes;

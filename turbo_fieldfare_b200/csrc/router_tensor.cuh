@@ -465,23 +465,25 @@ __device__ __forceinline__ float2 router_logits_staged(const uint8_t* codes_a, c
 // The experts that can reach the top k, in list (ascending), and their number: those whose upper bound is not below the top_k-th
 // largest lower bound. N: experts per lane. (A list: warps that took their candidates off bit masks, each skipping those of the token's
 // other warps, spent up to 20 000 clocks on that at eight warps per token.)
-template <int N>
+template <int N, bool AHEAD>
 __device__ __forceinline__ uint32_t router_candidates(const float2* approx_row, uint32_t parts, size_t part_stride, const float* __restrict__ logit_bias,
                                                       uint32_t num_experts, uint32_t top_k, int lane, uint16_t* list /* shared */) {
     float upper[N];
     uint32_t key[N];
     bool bad = false;
     float2 sum[N];
+    if constexpr (AHEAD) {
 #pragma unroll
-    for (int j = 0; j < N; ++j) sum[j] = (uint32_t)(lane + j * kWarp) < num_experts ? approx_row[lane + j * kWarp] : make_float2(0.0f, 0.0f);
-    if (parts > 1) {
+        for (int j = 0; j < N; ++j) sum[j] = (uint32_t)(lane + j * kWarp) < num_experts ? approx_row[lane + j * kWarp] : make_float2(0.0f, 0.0f);
+        if (parts > 1) {
 #pragma unroll 5
-        for (uint32_t p = 1; p < parts; ++p) {
+            for (uint32_t p = 1; p < parts; ++p) {
 #pragma unroll
-            for (int j = 0; j < N; ++j) {
-                if ((uint32_t)(lane + j * kWarp) < num_experts) {
-                    const float2 more = approx_row[p * part_stride + lane + j * kWarp];
-                    sum[j].x += more.x; sum[j].y += more.y;
+                for (int j = 0; j < N; ++j) {
+                    if ((uint32_t)(lane + j * kWarp) < num_experts) {
+                        const float2 more = approx_row[p * part_stride + lane + j * kWarp];
+                        sum[j].x += more.x; sum[j].y += more.y;
+                    }
                 }
             }
         }
@@ -492,7 +494,7 @@ __device__ __forceinline__ uint32_t router_candidates(const float2* approx_row, 
         upper[j] = -INFINITY;
         key[j] = 0u;
         if (e < num_experts) {
-            const float2 am = sum[j];
+            const float2 am = AHEAD ? sum[j] : approx_row[e];
             float v = am.x;
             if (!isfinite(am.x) || !isfinite(am.y)) bad = true;
             if (logit_bias) v = __fadd_rn(v, logit_bias[e]);
@@ -649,7 +651,8 @@ __device__ __forceinline__ void group_rows_in_block(const uint32_t* __restrict__
 // logits of the candidates (dealt out to the warps), top-k and softmax as in every other router kernel (one warp). A
 // canonical logit is one long dependent chain, so with few rows a token's eight or nine must not follow one another: one
 // warp per token took 30 us at 333 rows; four take 15. With grp.sorted_pairs the block that finishes the last row groups all of them.
-template <bool X_BF16, int GROUPS, int WPT>          // GROUPS: d / 64 when known at compile time, 0 for any width
+// AHEAD: the planes' values are requested before the first is looked at; otherwise (one plane) each where it is used, see launch_router.
+template <bool X_BF16, int GROUPS, int WPT, bool AHEAD = true>          // GROUPS: d / 64 when known at compile time, 0 for any width
 __global__ void __launch_bounds__(kRecheckWarps * kWarp, 2)
 router_recheck_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict__ S, const uint16_t* __restrict__ B,
                       const uint16_t* hidden, uint32_t hidden_stride, const uint16_t* __restrict__ eff,
@@ -694,8 +697,8 @@ router_recheck_kernel(const uint8_t* __restrict__ W, const uint16_t* __restrict_
     // (every warp of a token writes the same list)
     uint16_t* list = reinterpret_cast<uint16_t*>(reinterpret_cast<float*>(smem) + (size_t)kTokens * (d + num_experts)) + (size_t)slot * num_experts;
     const float2* approx_row = approx + (size_t)row * num_experts;
-    const uint32_t candidates = num_experts <= 4u * kWarp ? router_candidates<4>(approx_row, parts, (size_t)rows * num_experts, logit_bias, num_experts, top_k, lane, list)
-                                                          : router_candidates<TF_MAX_ROUTER_EXPERTS / kWarp>(approx_row, parts, (size_t)rows * num_experts, logit_bias, num_experts, top_k, lane, list);
+    const uint32_t candidates = num_experts <= 4u * kWarp ? router_candidates<4, AHEAD>(approx_row, parts, (size_t)rows * num_experts, logit_bias, num_experts, top_k, lane, list)
+                                                          : router_candidates<TF_MAX_ROUTER_EXPERTS / kWarp, AHEAD>(approx_row, parts, (size_t)rows * num_experts, logit_bias, num_experts, top_k, lane, list);
     if (WPT == 1) __syncwarp(); else __syncthreads();             // the row's activations and the cleared scores
     // this warp's candidates: every WPT-th one
     uint32_t next = part;
