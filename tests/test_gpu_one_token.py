@@ -8,10 +8,12 @@ from helpers import from_dev, to_dev
 pytestmark = pytest.mark.gpu
 
 # (d, f, fs, experts, top_k): production; parts of four groups full and partial in d, f and fs; one tile per block, several and more than are in
-# flight at once; few and most experts; shared memory near its limit, and beyond it (there one token takes the layered launches, too)
+# flight at once; few and most experts; down blocks near the shared memory that they have beside a gate/up block, and beyond it (there a
+# stack takes the layered launches; a block, too, for few columns, long experts or still larger blocks)
 SIZES = [(2816, 704, 2112, 128, 8), (256, 128, 192, 16, 8), (320, 64, 64, 9, 8), (64, 64, 64, 4, 2), (1088, 192, 448, 256, 7),
-         (2752, 1024, 576, 24, 8), (3072, 1280, 1152, 16, 6), (3072, 1536, 3072, 16, 8), (3072, 3072, 3072, 9, 8)]
-BEYOND = SIZES[-1]
+         (2752, 1024, 576, 24, 8), (3072, 1280, 1152, 16, 6), (1088, 1408, 2816, 16, 6), (512, 1536, 1536, 16, 8), (1024, 2816, 704, 9, 4),
+         (3072, 1536, 3072, 16, 8), (3072, 3072, 3072, 9, 8)]
+LAYERED_STACKS, LAYERED_BLOCKS = SIZES[-5:], SIZES[-4:]
 
 
 def _rows(o, rng, d):
@@ -53,7 +55,7 @@ def test_one_token_block_and_stack_have_the_bits_of_two_equal_tokens(tf_ctx, ora
 
 @pytest.mark.parametrize("d,f,fs,experts,top_k", SIZES)
 def test_one_token_takes_its_own_launches(tf_ctx, oracle, tmp_path, d, f, fs, experts, top_k):
-    """Three a layer of a stack and, in a block, kernels of their own; the layered ones beyond the shared memory."""
+    """Three a layer of a stack and, in a block, kernels of their own; the layered ones for sizes that those take less time for."""
     import torch
     from test_gpu_edges import _kernels_of
     from turbo_fieldfare_b200.stack import MoEBlock, MoEStack
@@ -68,9 +70,10 @@ def test_one_token_takes_its_own_launches(tf_ctx, oracle, tmp_path, d, f, fs, ex
         text = _kernels_of(lambda: MoEBlock(tf_ctx, stack.layers[1]).forward(h, y, 1, ws), tmp_path / "graph.dot")
         torch.cuda.synchronize()
         assert tf_ctx.device_status() == 0
-        own = (d, f, fs, experts, top_k) != BEYOND
-        assert (launches == 3 * 2) is own
-        assert all((k in text) is own for k in ("one_token_front_kernel", "one_token_gate_up_kernel", "one_token_down_kernel"))
+        size = (d, f, fs, experts, top_k)
+        assert (launches == 3 * 2) is (size not in LAYERED_STACKS)
+        kernels = ("one_token_front_kernel", "one_token_gate_up_kernel", "one_token_down_kernel")
+        assert [k in text for k in kernels] == [size not in LAYERED_BLOCKS] * 3
     finally:
         stack.close()
 

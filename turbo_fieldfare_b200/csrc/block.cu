@@ -639,7 +639,7 @@ static tf_status block_forward(tf_context* ctx, void* stream, const tf_moe_layer
                "%s: router is (%u,%u), expected (%u,%u)", name, layer->router.rows, layer->router.cols, layer->num_experts, layer->d);
     if (tokens == 0) return TF_OK;
     const uint32_t d = layer->d, K = layer->top_k;
-    if (tokens == 1 && y != nullptr && aligned(x, 16) && aligned(y, 2) && one_token_eligible(ctx, layer, ws))
+    if (tokens == 1 && y != nullptr && aligned(x, 16) && aligned(y, 2) && one_token_eligible(ctx, layer, ws, false))
         return one_token_block(ctx, stream, layer, x, y, ws);
     // The shared expert needs only x, so it runs on the context's side stream beside the router and the routed
     // experts and joins before the combine (inside a stream capture this becomes a fork and a join of the graph).
@@ -968,7 +968,7 @@ tf_status tf_stack_forward(tf_stack* st, void* stream, void* hidden, uint32_t to
         for (size_t l = 0; l < st->layers.size() && fused; ++l) {
             const tf_moe_layer& m = st->layers[l];
             fused = m.d == d && m.f == ws->f && m.fs == ws->fs && m.top_k == ws->top_k && m.num_experts == ws->num_experts &&
-                    st->norm_weights[l] && tf::aligned(st->norm_weights[l], 16) && tf::one_token_eligible(ctx, &m, ws);
+                    st->norm_weights[l] && tf::aligned(st->norm_weights[l], 16) && tf::one_token_eligible(ctx, &m, ws, true);
         }
         for (size_t l = 0; l < st->layers.size() && fused; ++l)
             if (tf_status s = tf::one_token_layer(ctx, stream, &st->layers[l], st->norm_weights[l], hidden, st->eps, ws)) return s;

@@ -51,7 +51,7 @@ bool decode_step_eligible(const tf_stack* st, const tf_workspace* ws);
 tf_status decode_step_prepare(tf_context* ctx, tf_stack* st);
 tf_status launch_decode_step(tf_context* ctx, void* stream, tf_stack* st, void* hidden, tf_workspace* ws);
 // one_token.cu: a layer of a stack (hidden row updated in place), or a block forward, for one token
-bool one_token_eligible(const tf_context* ctx, const tf_moe_layer* layer, const tf_workspace* ws);
+bool one_token_eligible(const tf_context* ctx, const tf_moe_layer* layer, const tf_workspace* ws, bool stack);
 tf_status one_token_layer(tf_context* ctx, void* stream, const tf_moe_layer* layer, const void* norm_weight_bf16, void* hidden, float eps, tf_workspace* ws);
 tf_status one_token_block(tf_context* ctx, void* stream, const tf_moe_layer* layer, const void* x, void* y, tf_workspace* ws);
 // grouped.cu: tf_group_routes_device over ids read at a stride (and optionally written out densely)

@@ -35,6 +35,7 @@ constexpr uint32_t kOneSlots = 4;                   // gate/up tiles in flight p
 // a down block leaves.
 constexpr uint32_t kOneAloneBytes = 114 * 1024, kOneFrontBytes = 61 * 1024;
 constexpr uint32_t kOneDownBytes = 108 * 1024;      // a block of the down launch beside a gate/up block
+constexpr uint32_t kOneBlockDownBytes = 160 * 1024, kOneBlockMinD = 1024, kOneBlockMaxF = 2048;      // see one_token_size
 constexpr uint32_t kErrTimeoutOneToken = 0x7F000041u;
 static_assert(TF_MAX_ROUTER_EXPERTS <= kOneThreads, "a thread per expert");
 
@@ -715,18 +716,29 @@ one_token_down_kernel(const OneTokenArgs a, uint32_t rows) {
 
 // ---- host ----
 
-// What the layered launches accept and these do not: other shapes, an 8-bit shared expert, workspaces of more tokens (fp16 partials), a
-// tensor-core threshold of one token. Arguments that the layered launches refuse go there, too, and are refused.
-// Blocks of the down launch, one per SM at the most, and their most rows; 0 rows if those do not fit an SM.
-struct OneDownGrid { uint32_t blocks, rows; };
+// Blocks of the down launch, one per SM at the most or 16 rows each, their most rows and the shared memory of one (of the launch of both parts).
+struct OneDownGrid { uint32_t blocks, rows; size_t bytes; };
 static OneDownGrid one_down_grid(const tf_context* ctx, uint32_t d, uint32_t f, uint32_t fs, uint32_t top_k) {
     const uint32_t quads = d / 4, sixteens = d / kTileRows16;
     auto rows = [&](uint32_t blocks) { const uint32_t r = (quads + blocks - 1) / blocks * 4; return r < (uint32_t)kTileRows16 ? (uint32_t)kTileRows16 : r; };
     uint32_t blocks = sixteens < (uint32_t)ctx->sm_count ? sixteens : (uint32_t)ctx->sm_count;
     if (rows(blocks) > 2 * kTileRows16 || OneDownSmem{fs / kGroup, f / kGroup, top_k, rows(blocks)}.total() > kOneDownBytes) blocks = sixteens;
-    return {blocks, OneDownSmem{fs / kGroup, f / kGroup, top_k, rows(blocks)}.total() <= 200 * 1024 ? rows(blocks) : 0u};
+    return {blocks, rows(blocks), OneDownSmem{fs / kGroup, f / kGroup, top_k, rows(blocks)}.total()};
 }
-bool one_token_eligible(const tf_context* ctx, const tf_moe_layer* l, const tf_workspace* ws) {
+// Sizes that these launches take. A stack's layer: a block of the down launch has a place beside one of the gate/up launch (kOneDownBytes); a larger one
+// requests its weights only when that has ended. us a layer, layered and here (d x f x fs, top_k; KB of a down block): 2816 x 704 x 2112, 8
+// (105) 22.8, 19.5; 3072 x 1280 x 1152, 6 (98) 32.3, 27.3; 1024 x 2048 x 1024, 4 (101) 20.2, 18.6; 2816 x 960 x 2112, 8 (110) 31.1, 27.6;
+// 2816 x 1088 x 1024, 8 (111) 22 to 31, 33; 2048 x 1408 x 2816, 6 (126) 24.8, 24.2; 2816 x 2816 x 704, 4 (132) 31.7, 35.6;
+// 2048 x 1536 x 1536, 8 (153) 21.6, 27.6; 256 x 1024 x 2048, 8 (113) 18.7, 19.5; 3072 x 1536 x 3072, 8 (169) 29, 44.
+// A block's two down launches have such a place up to larger sizes, and no side stream: 2048 x 1408 x 2816, 6 33.4, 28.0; 2048 x 1536 x 1536, 8
+// 33.0, 29.2; 1024 x 1536 x 1536, 8 27.6, 26.4; but 512 x 1536 x 1536, 8 24.6, 25.0; 2816 x 2816 x 704, 4 31.0, 34.5; 3072 x 1536 x 3072, 8 42.5, 43.
+static bool one_token_size(const tf_context* ctx, const tf_moe_layer* l, bool stack) {
+    const size_t bytes = one_down_grid(ctx, l->d, l->f, l->fs, l->top_k).bytes;
+    return bytes <= kOneDownBytes || (!stack && bytes <= kOneBlockDownBytes && l->d >= kOneBlockMinD && l->f <= kOneBlockMaxF);
+}
+// What the layered launches accept and these do not: other shapes, an 8-bit shared expert, workspaces of more tokens (fp16 partials), a
+// tensor-core threshold of one token. Arguments that the layered launches refuse go there, too, and are refused.
+bool one_token_eligible(const tf_context* ctx, const tf_moe_layer* l, const tf_workspace* ws, bool stack) {
     const bool shape = l->d % kGroup == 0 && l->f % kGroup == 0 && l->fs % kGroup == 0 && l->d > 0 && l->f > 0 && l->fs > 0 &&
                        l->d <= kOneMaxGroups * kGroup && l->f <= kOneMaxGroups * kGroup && l->fs <= kOneMaxGroups * kGroup &&
                        l->top_k > 0 && l->top_k <= TF_MAX_TOP_K && l->top_k <= l->num_experts && l->num_experts <= TF_MAX_ROUTER_EXPERTS;
@@ -747,7 +759,7 @@ bool one_token_eligible(const tf_context* ctx, const tf_moe_layer* l, const tf_w
         if (v % 16 != 0) return false;
     return l->pool_layer_base && aligned(l->pool_layer_base, 16) && l->expert_stride % 16 == 0 && l->effective_scale && aligned(l->effective_scale, 16) &&
            l->per_expert_scale && aligned(l->per_expert_scale, 2) && aligned(l->logit_bias, 4) &&
-           one_down_grid(ctx, l->d, l->f, l->fs, l->top_k).rows > 0;
+           one_token_size(ctx, l, stack);
 }
 
 static OneTokenArgs one_token_args(const tf_context* ctx, const tf_moe_layer* l, tf_workspace* ws) {
