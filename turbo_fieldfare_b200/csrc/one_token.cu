@@ -540,7 +540,7 @@ one_token_gate_up_kernel(const OneTokenArgs a, uint32_t slots, uint32_t most) {
                     break;
                 }
                 for (uint32_t p = warp; p < parts; p += kOneWarps) one_tile_part<FOURS>(lay, smem, slot, i, p);
-                __syncwarp();
+                __syncwarp();                // the sums, of all loads from the slot, have been stored
                 if (live && lane == 0) mbar_arrive(bars + (slots + slot) * 8);
                 if (++slot == slots) { slot = 0; ++use; }
             }

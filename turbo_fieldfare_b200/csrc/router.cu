@@ -572,8 +572,9 @@ static tf_status launch_router(tf_context* ctx, void* stream, const uint8_t* W, 
     // 1500 rows 23.7, 22.4, 45.6; 4096 rows 47.8, 41.0, 48.5 (and adding the planes takes the re-check 9 us less with three).
     const uint32_t apx_blocks = (rows + kApxTokens - 1) / kApxTokens * ((num_experts + kApxExperts - 1) / kApxExperts) * (d / kApxChunk);
     // Few rows: blocks of 8 tokens x 32 experts with all of their operands in flight at once, while they make one round of the SMs: 200 rows,
-    // 100 blocks, 9.8 us. Two rounds (333 rows, 168 blocks) take 16.6, the parts of the other kernel 7.5. (Those take 6.2 us at 200 rows,
-    // but steps of 66 to 255 tokens gained nothing or lost 0.5 %, and prefills of 256 took 2.7 % longer.)
+    // 100 blocks, 9.8 us. Two rounds (333 rows, 168 blocks) take 16.6, the parts of the other kernel 7.5. (Those take 6.2 us at 200 rows. Steps of
+    // 30 layers, us, here and with those: 80 tokens 4232, 4253; 100: 4839, 4933; 110: 5517, 5640; 120: 5693, 5463; 150: 6118, 5999; 200: 7001, 6932;
+    // 255: 8139, 8111; prefills of 256 5513, 5453, of 290 the same.)
     const size_t smem_few = router_approx_few_smem_bytes(d);
     const dim3 grid_few((rows + kFewTokens - 1) / kFewTokens, (num_experts + kFewExperts - 1) / kFewExperts);
     const bool few = smem_few <= 224 * 1024 && grid_few.x * grid_few.y <= (uint32_t)ctx->sm_count;

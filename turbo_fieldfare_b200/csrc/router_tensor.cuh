@@ -543,8 +543,9 @@ __device__ __forceinline__ uint32_t router_candidates(const float2* approx_row, 
 // The grouping of the re-check's last block, up to a few thousand pairs: a warp takes consecutive pairs, 32 to a round, whose lanes find their
 // rank among the round's pairs of the same expert with match.any; the first of them adds their number to the warp's count of the expert. A
 // thread per expert then turns the counts into starts. Latency bounds it. (group_routes_in_block, whose bitmaps have rows of 64 words at 255
-// tokens of top 8, all in one bank: 255 rows 42 -> 30 us for the launch, 200 rows 31 -> 27, 70 rows 19 -> 16.5; a step of 255 tokens
-// 6177 -> 5955. The few-row router stays with those: up to 11 tokens it took 1 to 3 % longer with this.)
+// tokens of top 8, all in one bank: 255 rows 42 -> 30 us for the launch, 200 rows 31 -> 27, 70 rows 19 -> 16.5; steps of 30 layers, 255
+// tokens 8446 -> 8139, 200 tokens 7076 -> 7001, 130 tokens 5869 -> 5810, up to 120 tokens the same. The few-row router stays with those: up to 11
+// tokens it took 1 to 3 % longer with this.)
 constexpr uint32_t kGroupRowsWarps = kRecheckWarps;
 __host__ __device__ inline size_t router_group_rows_smem_bytes(uint32_t n_pairs, uint32_t num_experts) {
     return (size_t)num_experts * (kGroupRowsWarps + 1) * 4 + (size_t)n_pairs * 4 + 3 * kGroupRowsWarps * 4 + (size_t)((n_pairs + 1) / 2) * 4;
